@@ -1,0 +1,652 @@
+// Scaled-dot-product attention in one kernel per pass for head dim 64: scores, mask, softmax, dropout and the product with the values
+// stay on the SM, so no [Tq, Tk] matrix is written to memory.
+//
+//   flash_fwd     one CTA per (batch entry, head, 128 queries): a loop over tiles of 64 keys, online softmax
+//   flash_bwd_q   the same split: recomputes the scores from the saved log-sum, dS = P * (dP - delta), dQ = scale * dS K
+//   flash_bwd_kv  one CTA per (batch entry, head, 128 keys): a loop over tiles of 64 queries, transposed scores, dK and dV
+//
+// A CTA has 128 threads = the 128 lanes of tensor memory: a thread owns one row of the score tile (a query; in flash_bwd_kv a key) and
+// needs no exchange with others for maximum and sum. Thread 0 also issues the TMA loads (two stages) and the tcgen05.mma. The chain load ->
+// product -> softmax -> product of one CTA is serial; three (backward: two) CTAs per SM fill each other's gaps. That is why the tiles are
+// 64 wide: 128 TMEM columns and 66 KB of shared memory per CTA (backward 256 columns and 82 / 98 KB). The two-pass backward (dQ apart from
+// dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
+// The kernels are bound by the per-row exponentials and that chain, not by memory.
+//
+// Visible keys, dropout and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per score.
+#include "tcgen05.cuh"
+
+using namespace rbt;
+
+namespace {
+
+constexpr int kRows = 128;   // rows of a CTA
+constexpr int kTile = 64;    // width of a score tile, and the head dim
+constexpr int kBig = kRows * 128;   // bytes of a [128, 64] bf16 tile
+constexpr int kSmall = kTile * 128;  // ... [64, 64]
+constexpr int kThreads = 128;
+constexpr float kLog2e = 1.4426950408889634f;
+
+struct Flash {
+  const int* k_lens;
+  float* lse;    // [B*H, tq] log2 of the softmax denominator, maximum included; +inf: no visible key
+  float* delta;  // [B*H, tq] sum_d dO * O
+  uint32_t* keep;  // [B*H, tq, words] dropout: bit j of word w = key 32 w + j is kept
+  const long long* seed;
+  const long long* offset;
+  int* status;
+  int heads, tq, tk, causal, shift, tiles, hq, hk, hv, hdo, words, tqp, tkp;
+  float scale, p_drop;
+};
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ void tmem_ld64(uint32_t addr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  tmem_ld32(addr, r);
+  tmem_ld32(addr + 32, r + 32);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// 64 values -> row `row` of a swizzled [rows, 64] bf16 tile
+__device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float* v) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    *reinterpret_cast<uint4*>(tile + row * 128 + ((c ^ (row & 7)) << 4)) =
+        make_uint4(pack2(v[8 * c], v[8 * c + 1]), pack2(v[8 * c + 2], v[8 * c + 3]), pack2(v[8 * c + 4], v[8 * c + 5]), pack2(v[8 * c + 6], v[8 * c + 7]));
+  }
+}
+
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
+  const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    s = fmaf(__uint_as_float(x[e] << 16), __uint_as_float(y[e] << 16), s);
+    s = fmaf(__uint_as_float(x[e] & 0xffff0000u), __uint_as_float(y[e] & 0xffff0000u), s);
+  }
+  return s;
+}
+
+// D[128, 64] (+)= A[128, 64] B: A K-major; B K-major [n, k] or, `b_mn`, stored [k, n]
+template <bool B_MN>
+__device__ __forceinline__ void mma64(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    umma_f16(d, make_desc(sa + kk * 32, 16, 1024), B_MN ? make_desc(sb + kk * 2048, 8192, 1024) : make_desc(sb + kk * 32, 16, 1024), idesc,
+             (accumulate || kk > 0) ? 1u : 0u);
+  }
+}
+
+__device__ __forceinline__ int visible(const Flash& p, int i, int klen) {
+  int n = klen;
+  if (p.causal) n = min(n, i + p.shift + 1);
+  return max(n, 0);
+}
+
+// the part that the three kernels share: barriers, tensor memory, the abort flag
+struct Cta {
+  uint64_t* full;    // [2] loads of a stage
+  uint64_t* done;    // products of an iteration
+  uint64_t* extra;   // one more load
+  uint32_t tmem;
+  volatile int* abort_flag;
+};
+
+template <uint32_t COLS>
+__device__ __forceinline__ Cta cta_begin(uint8_t* tail) {
+  Cta c;
+  c.full = reinterpret_cast<uint64_t*>(tail);
+  c.done = c.full + 2;
+  c.extra = c.full + 3;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(c.full + 4);
+  c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(c.full + i, 1);
+    *c.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  c.tmem = *slot;
+  return c;
+}
+
+template <uint32_t COLS>
+__device__ __forceinline__ void cta_end(const Cta& c) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*c.abort_flag && threadIdx.x == 0) {
+    for (uint32_t i = 0; i < (1u << 12); ++i) __nanosleep(256);  // copies still in flight land before the shared memory goes away
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "r"(COLS) : "memory");
+  }
+}
+
+// bounded wait; a wait that gives up marks the CTA and the status word
+__device__ __forceinline__ bool wait_or_abort(const Cta& c, uint64_t* bar, uint32_t parity, int* status, int code) {
+  const bool ok = mbar_wait(bar, parity, c.abort_flag);
+  if (!ok) {
+    *c.abort_flag = 1;
+    if (status) atomicCAS(status, 0, (8 << 24) | code);
+  }
+  return ok;
+}
+
+template <bool DROP>
+__global__ void __launch_bounds__(kThreads, 3)
+flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                 const __grid_constant__ CUtensorMap tm_o, const Flash p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sk = sq + kBig;
+  uint8_t* sv = sk + 2 * kSmall;
+  uint8_t* sp = sv + 2 * kSmall;
+  const Cta c = cta_begin<128>(sp + kBig);
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const int tid = threadIdx.x;
+  const int z = blockIdx.x / p.tiles;
+  const int q0 = (p.tiles - 1 - (int)(blockIdx.x % p.tiles)) * kRows;  // causal: the long rows first
+  const int b = z / p.heads, h = z - b * p.heads;
+  const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
+  const int row = q0 + tid;
+  const int n = row < p.tq ? visible(p, row, klen) : 0;
+  const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
+  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+  const uint32_t t_s = c.tmem, t_o = c.tmem + 64;
+  auto load_kv = [&](int t) {
+    const int s = t & 1;
+    tma_load_3d(sk + s * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[s]);
+    tma_load_3d(sv + s * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[s]);
+  };
+  bool ok = true;
+  if (tid == 0 && n_tiles > 0) {
+    mbar_expect_tx(&c.full[0], kBig + 2 * kSmall);
+    tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
+    load_kv(0);
+    if (n_tiles > 1) {
+      mbar_expect_tx(&c.full[1], 2 * kSmall);
+      load_kv(1);
+    }
+    ok = wait_or_abort(c, &c.full[0], 0, p.status, 1);
+    if (ok) {
+      mma64<false>(t_s, sq, sk, false);
+      umma_commit(c.done);
+    }
+  }
+  const float cs = p.scale * kLog2e;
+  const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
+  const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
+  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+  float m = -INFINITY, l = 0.f;
+  float acc[64];
+#pragma unroll
+  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+  int it = 0;
+  for (; it < n_tiles; ++it) {
+    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 2);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {  // the products of the previous iteration are complete: its stage is free
+      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
+      load_kv(it + 1);
+    }
+    __syncwarp();
+    float s[64];
+    if (it > 0) {
+      tmem_ld64(t_row + 64, s);
+#pragma unroll
+      for (int j = 0; j < 64; ++j) acc[j] += s[j];
+    }
+    tmem_ld64(t_row, s);
+    const int left = n - it * kTile;  // visible keys of this row in this tile
+    float mx = m;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      s[j] = j < left ? s[j] * cs : -INFINITY;
+      mx = fmaxf(mx, s[j]);
+    }
+    const float mu = mx == -INFINITY ? 0.f : mx;
+    const float corr = ex2(m - mu);
+    m = mx;
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      s[j] = ex2(s[j] - mu);
+      sum += s[j];
+    }
+    l = l * corr + sum;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] *= corr;
+    if constexpr (DROP) {
+      const uint64_t base = off + ((uint64_t)z * p.tqp + row) * p.tkp + it * kTile;
+      uint32_t bits[2] = {0u, 0u};
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) {
+        const uint64_t ctr = base + j;
+        const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x51u, 0u));
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool k = w[e] >= thresh;
+          s[j + e] = k ? s[j + e] * keep_scale : 0.f;
+          if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        }
+      }
+      if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
+    }
+    store_row64(sp, tid, s);
+    fence_proxy_async_smem();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      mma64<true>(t_o, sp, sv + (it & 1) * kSmall, false);
+      if (it + 1 < n_tiles) {
+        ok = wait_or_abort(c, &c.full[(it + 1) & 1], ((it + 1) >> 1) & 1, p.status, 3);
+        if (ok) mma64<false>(t_s, sq, sk + ((it + 1) & 1) * kSmall, false);
+      }
+      if (ok) umma_commit(c.done);
+    }
+  }
+  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 4);
+  if (!__syncthreads_or(ok ? 0 : 1)) {
+    if (n_tiles > 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float s[64];
+      tmem_ld64(t_row + 64, s);
+      const float inv = n > 0 ? 1.f / l : 0.f;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) acc[j] = n > 0 ? (acc[j] + s[j]) * inv : 0.f;
+    }
+    store_row64(sq, tid, acc);
+    if (row < p.tq) p.lse[(long long)z * p.tq + row] = n > 0 ? m + __log2f(l) : INFINITY;
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&tm_o, h * kTile, q0, b, sq);
+      tma_store_commit();
+      tma_store_wait_all();
+    }
+  }
+  cta_end<128>(c);
+}
+
+template <bool DROP>
+__global__ void __launch_bounds__(kThreads, 2)
+flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                   const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
+                   const Flash p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sdo = sq + kBig;
+  uint8_t* sk = sdo + kBig;
+  uint8_t* sv = sk + 2 * kSmall;
+  uint8_t* sds = sv + 2 * kSmall;  // first the tile of O
+  const Cta c = cta_begin<256>(sds + kBig);
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const int tid = threadIdx.x;
+  const int z = blockIdx.x / p.tiles;
+  const int q0 = (p.tiles - 1 - (int)(blockIdx.x % p.tiles)) * kRows;
+  const int b = z / p.heads, h = z - b * p.heads;
+  const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
+  const int row = q0 + tid;
+  const int n = row < p.tq ? visible(p, row, klen) : 0;
+  const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
+  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+  const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dq = c.tmem + 128;
+  auto load_kv = [&](int t) {
+    const int s = t & 1;
+    tma_load_3d(sk + s * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[s]);
+    tma_load_3d(sv + s * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[s]);
+  };
+  bool ok = true;
+  if (tid == 0 && n_tiles > 0) {
+    mbar_expect_tx(&c.full[0], 2 * kBig + 2 * kSmall);
+    tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
+    tma_load_3d(sdo, &tm_do, h * p.hdo, q0, b, &c.full[0]);
+    load_kv(0);
+    mbar_expect_tx(c.extra, kBig);
+    tma_load_3d(sds, &tm_o, h * kTile, q0, b, c.extra);
+    if (n_tiles > 1) {
+      mbar_expect_tx(&c.full[1], 2 * kSmall);
+      load_kv(1);
+    }
+    ok = wait_or_abort(c, &c.full[0], 0, p.status, 5);
+    if (ok) {
+      mma64<false>(t_s, sq, sk, false);
+      mma64<false>(t_dp, sdo, sv, false);
+      umma_commit(c.done);
+    }
+  }
+  float lse = INFINITY, delta = 0.f;
+  if (n_tiles > 0) {
+    ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 6) && wait_or_abort(c, c.extra, 0, p.status, 6);
+    if (ok) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int at = tid * 128 + ((j ^ (tid & 7)) << 4);
+        delta += dot8(*reinterpret_cast<const uint4*>(sds + at), *reinterpret_cast<const uint4*>(sdo + at));
+      }
+      if (row < p.tq) {
+        lse = p.lse[(long long)z * p.tq + row];
+        p.delta[(long long)z * p.tq + row] = delta;
+      }
+    }
+  }
+  const float cs = p.scale * kLog2e;
+  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+  int it = 0;
+  for (; it < n_tiles; ++it) {
+    uint2 bits = make_uint2(0u, 0u);
+    if (DROP && row < p.tq) bits = *reinterpret_cast<const uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2);
+    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 7);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
+      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
+      load_kv(it + 1);
+    }
+    __syncwarp();
+    float s[64], dp[64];
+    tmem_ld64(t_row, s);
+    tmem_ld64(t_row + 64, dp);
+    const int left = n - it * kTile;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      float d = dp[j];
+      if (DROP) d = (((j < 32 ? bits.x : bits.y) >> (j & 31)) & 1u) ? d * keep_scale : 0.f;
+      s[j] = j < left ? ex2(fmaf(s[j], cs, -lse)) * (d - delta) : 0.f;
+    }
+    store_row64(sds, tid, s);
+    fence_proxy_async_smem();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      mma64<true>(t_dq, sds, sk + (it & 1) * kSmall, it > 0);
+      if (it + 1 < n_tiles) {
+        const int st = (it + 1) & 1;
+        ok = wait_or_abort(c, &c.full[st], ((it + 1) >> 1) & 1, p.status, 8);
+        if (ok) {
+          mma64<false>(t_s, sq, sk + st * kSmall, false);
+          mma64<false>(t_dp, sdo, sv + st * kSmall, false);
+        }
+      }
+      if (ok) umma_commit(c.done);
+    }
+  }
+  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 9);
+  if (!__syncthreads_or(ok ? 0 : 1)) {
+    float s[64];
+    if (n_tiles > 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_ld64(t_row + 128, s);
+    }
+#pragma unroll
+    for (int j = 0; j < 64; ++j) s[j] = n_tiles > 0 ? s[j] * p.scale : 0.f;
+    store_row64(sq, tid, s);
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&tm_dq, h * kTile, q0, b, sq);
+      tma_store_commit();
+      tma_store_wait_all();
+    }
+  }
+  cta_end<256>(c);
+}
+
+template <bool DROP>
+__global__ void __launch_bounds__(kThreads, 2)
+flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                    const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
+                    const Flash p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sk = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sv = sk + kBig;
+  uint8_t* sq = sv + kBig;
+  uint8_t* sdo = sq + 2 * kSmall;
+  uint8_t* sp = sdo + 2 * kSmall;
+  uint8_t* sds = sp + kBig;
+  float2* stat = reinterpret_cast<float2*>(sds + kBig);        // [2][64] (log-sum, delta) of the queries of a tile
+  uint4* kept = reinterpret_cast<uint4*>(sds + kBig + 1024);   // [2][64] dropout bits of this CTA's 128 keys
+  const Cta c = cta_begin<256>(sds + kBig + 1024 + 2048);
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const int tid = threadIdx.x;
+  const int z = blockIdx.x / p.tiles;
+  const int k0 = (int)(blockIdx.x % p.tiles) * kRows;
+  const int b = z / p.heads, h = z - b * p.heads;
+  const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
+  const int key = k0 + tid;
+  const int first = p.causal ? max(0, k0 - p.shift) / kTile : 0;  // queries before cannot see the first key of the tile
+  const int n_tiles = k0 < klen ? max(0, (p.tq + kTile - 1) / kTile - first) : 0;
+  // queries that see this key: [lo, tq)
+  const int lo = key < klen ? (p.causal ? max(0, key - p.shift) : 0) : p.tq;
+  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+  const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dv = c.tmem + 128, t_dk = c.tmem + 192;
+  auto load_q = [&](int t) {
+    const int s = t & 1;
+    tma_load_3d(sq + s * kSmall, &tm_q, h * p.hq, (first + t) * kTile, b, &c.full[s]);
+    tma_load_3d(sdo + s * kSmall, &tm_do, h * p.hdo, (first + t) * kTile, b, &c.full[s]);
+  };
+  auto load_stat = [&](int t) {
+    const int q = (first + t) * kTile + (tid & 63);
+    if (tid < 64) {
+      float2 v = make_float2(INFINITY, 0.f);
+      if (q < p.tq) v = make_float2(p.lse[(long long)z * p.tq + q], p.delta[(long long)z * p.tq + q]);
+      stat[(t & 1) * 64 + tid] = v;
+    } else if (DROP) {
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (q < p.tq) v = *reinterpret_cast<const uint4*>(p.keep + ((long long)z * p.tq + q) * p.words + k0 / 32);
+      kept[(t & 1) * 64 + (tid & 63)] = v;
+    }
+  };
+  bool ok = true;
+  if (n_tiles > 0) load_stat(0);
+  __syncthreads();
+  if (tid == 0 && n_tiles > 0) {
+    mbar_expect_tx(&c.full[0], 2 * kBig + 2 * kSmall);
+    tma_load_3d(sk, &tm_k, h * p.hk, k0, b, &c.full[0]);
+    tma_load_3d(sv, &tm_v, h * p.hv, k0, b, &c.full[0]);
+    load_q(0);
+    if (n_tiles > 1) {
+      mbar_expect_tx(&c.full[1], 2 * kSmall);
+      load_q(1);
+    }
+    ok = wait_or_abort(c, &c.full[0], 0, p.status, 10);
+    if (ok) {
+      mma64<false>(t_s, sk, sq, false);
+      mma64<false>(t_dp, sv, sdo, false);
+      umma_commit(c.done);
+    }
+  }
+  const float cs = p.scale * kLog2e;
+  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+  int it = 0;
+  for (; it < n_tiles; ++it) {
+    if (it + 1 < n_tiles) load_stat(it + 1);  // seen by all after this iteration's barrier
+    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 11);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
+      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
+      load_q(it + 1);
+    }
+    __syncwarp();
+    float s[64], dp[64];
+    tmem_ld64(t_row, s);
+    tmem_ld64(t_row + 64, dp);
+    const int q_base = (first + it) * kTile;
+    const float2* st = stat + (it & 1) * 64;
+    const uint32_t* kp = reinterpret_cast<const uint32_t*>(kept + (it & 1) * 64) + (tid >> 5);
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      const float2 ld = st[j];
+      const bool vis = q_base + j >= lo && q_base + j < p.tq;
+      float pr = vis ? ex2(fmaf(s[j], cs, -ld.x)) : 0.f;
+      float d = dp[j];
+      float pd = pr;
+      if (DROP) {
+        const bool k = (kp[j * 4] >> (tid & 31)) & 1u;
+        d = k ? d * keep_scale : 0.f;
+        pd = k ? pr * keep_scale : 0.f;
+      }
+      dp[j] = vis ? pr * (d - ld.y) : 0.f;
+      s[j] = pd;
+    }
+    store_row64(sp, tid, s);
+    store_row64(sds, tid, dp);
+    fence_proxy_async_smem();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      mma64<true>(t_dv, sp, sdo + (it & 1) * kSmall, it > 0);
+      mma64<true>(t_dk, sds, sq + (it & 1) * kSmall, it > 0);
+      if (it + 1 < n_tiles) {
+        const int sn = (it + 1) & 1;
+        ok = wait_or_abort(c, &c.full[sn], ((it + 1) >> 1) & 1, p.status, 12);
+        if (ok) {
+          mma64<false>(t_s, sk, sq + sn * kSmall, false);
+          mma64<false>(t_dp, sv, sdo + sn * kSmall, false);
+        }
+      }
+      if (ok) umma_commit(c.done);
+    }
+  }
+  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 13);
+  if (!__syncthreads_or(ok ? 0 : 1)) {
+    float s[64], dp[64];
+    if (n_tiles > 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_ld64(t_row + 128, s);
+      tmem_ld64(t_row + 192, dp);
+    }
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      s[j] = n_tiles > 0 ? s[j] : 0.f;
+      dp[j] = n_tiles > 0 ? dp[j] * p.scale : 0.f;
+    }
+    store_row64(sv, tid, s);
+    store_row64(sk, tid, dp);
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&tm_dv, h * kTile, k0, b, sv);
+      tma_store_3d(&tm_dk, h * kTile, k0, b, sk);
+      tma_store_commit();
+      tma_store_wait_all();
+    }
+  }
+  cta_end<256>(c);
+}
+
+constexpr int kFwdSmem = 2 * kBig + 4 * kSmall + 64 + 1024;
+constexpr int kBwdQSmem = 3 * kBig + 4 * kSmall + 64 + 1024;
+constexpr int kBwdKvSmem = 4 * kBig + 4 * kSmall + 1024 + 2048 + 64 + 1024;
+
+int launch_failed(const char* what, cudaError_t e) {
+  rb_set_error("%s: %s", what, cudaGetErrorString(e));
+  return RB_ERR_LAUNCH;
+}
+
+// geom: B, H, Tq, Tk, causal, causal shift, then row and head pitch (elements) of q, k, v, dO, Tqp, Tkp, dropout words per row
+enum { G_B, G_H, G_TQ, G_TK, G_CAUSAL, G_SHIFT, G_RQ, G_HQ, G_RK, G_HK, G_RV, G_HV, G_RDO, G_HDO, G_TQP, G_TKP, G_WORDS };
+
+Flash make_params(const int* g, const int* k_lens, float* lse, float* delta, void* keep, float scale, float p_drop, const long long* seed,
+                  const long long* offset, int* status) {
+  Flash p = {};
+  p.k_lens = k_lens; p.lse = lse; p.delta = delta; p.keep = (uint32_t*)keep; p.seed = seed; p.offset = offset; p.status = status;
+  p.heads = g[G_H]; p.tq = g[G_TQ]; p.tk = g[G_TK]; p.causal = g[G_CAUSAL]; p.shift = g[G_SHIFT];
+  p.hq = g[G_HQ]; p.hk = g[G_HK]; p.hv = g[G_HV]; p.hdo = g[G_HDO]; p.words = g[G_WORDS]; p.tqp = g[G_TQP]; p.tkp = g[G_TKP];
+  p.scale = scale; p.p_drop = p_drop;
+  return p;
+}
+
+int map_of(CUtensorMap* m, const void* base, const int* g, int t, int row_pitch, int head_pitch, int box_rows) {
+  return make_map_3d(m, base, (long long)(g[G_H] - 1) * head_pitch + kTile, t, g[G_B], row_pitch, (long long)t * row_pitch, box_rows);
+}
+
+}  // namespace
+
+RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse, void* keep, const int* k_lens, const int* g, float scale,
+                              float p_drop, const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
+  if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0 || g[G_TK] <= 0) return RB_OK;
+  Flash p = make_params(g, k_lens, lse, nullptr, keep, scale, p_drop, seed, offset, status);
+  p.tiles = (p.tq + kRows - 1) / kRows;
+  const long long ctas = (long long)p.tiles * g[G_B] * g[G_H];
+  if (ctas > 0x7fffffffLL) {
+    rb_set_error("flash_fwd: too many tiles");
+    return RB_ERR_ARG;
+  }
+  const int hd = g[G_H] * kTile;
+  CUtensorMap tq, tk, tv, to;
+  int st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kRows);
+  if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kTile);
+  if (!st) st = map_of(&tv, v, g, p.tk, g[G_RV], g[G_HV], kTile);
+  if (!st) st = map_of(&to, o, g, p.tq, hd, kTile, kRows);
+  if (st) return st;
+  auto kernel = p_drop > 0.f ? flash_fwd_kernel<true> : flash_fwd_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
+  if (e != cudaSuccess) return launch_failed("flash_fwd", e);
+  rb_launch_pdl(kernel, dim3((unsigned)ctas), dim3(kThreads), kFwdSmem, stream, tq, tk, tv, to, p);
+  return rb_check_launch("flash_fwd");
+}
+
+RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, void* dq, void* dk, void* dv, float* lse,
+                              float* delta, void* keep, const int* k_lens, const int* g, float scale, float p_drop, int* status, cudaStream_t stream) {
+  if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0 || g[G_TK] <= 0) return RB_OK;
+  Flash p = make_params(g, k_lens, lse, delta, keep, scale, p_drop, nullptr, nullptr, status);
+  const int hd = g[G_H] * kTile;
+  const int tiles_q = (p.tq + kRows - 1) / kRows, tiles_k = (p.tk + kRows - 1) / kRows;
+  const long long bh = (long long)g[G_B] * g[G_H];
+  if (bh * tiles_q > 0x7fffffffLL || bh * tiles_k > 0x7fffffffLL) {
+    rb_set_error("flash_bwd: too many tiles");
+    return RB_ERR_ARG;
+  }
+  CUtensorMap tq, tk, tv, to, td, tg, tg2;
+  int st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kRows);
+  if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kTile);
+  if (!st) st = map_of(&tv, v, g, p.tk, g[G_RV], g[G_HV], kTile);
+  if (!st) st = map_of(&to, o, g, p.tq, hd, kTile, kRows);
+  if (!st) st = map_of(&td, d_o, g, p.tq, g[G_RDO], g[G_HDO], kRows);
+  if (!st) st = map_of(&tg, dq, g, p.tq, hd, kTile, kRows);
+  if (st) return st;
+  auto kq = p_drop > 0.f ? flash_bwd_q_kernel<true> : flash_bwd_q_kernel<false>;
+  auto kkv = p_drop > 0.f ? flash_bwd_kv_kernel<true> : flash_bwd_kv_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdQSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdKvSmem);
+  if (e != cudaSuccess) return launch_failed("flash_bwd", e);
+  p.tiles = tiles_q;
+  rb_launch_pdl(kq, dim3((unsigned)(bh * tiles_q)), dim3(kThreads), kBwdQSmem, stream, tq, tk, tv, to, td, tg, p);
+  st = rb_check_launch("flash_bwd_q");
+  if (!st) st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kTile);
+  if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kRows);
+  if (!st) st = map_of(&tv, v, g, p.tk, g[G_RV], g[G_HV], kRows);
+  if (!st) st = map_of(&td, d_o, g, p.tq, g[G_RDO], g[G_HDO], kTile);
+  if (!st) st = map_of(&tg, dk, g, p.tk, hd, kTile, kRows);
+  if (!st) st = map_of(&tg2, dv, g, p.tk, hd, kTile, kRows);
+  if (st) return st;
+  p.tiles = tiles_k;
+  rb_launch_pdl(kkv, dim3((unsigned)(bh * tiles_k)), dim3(kThreads), kBwdKvSmem, stream, tq, tk, tv, td, tg, tg2, p);
+  return rb_check_launch("flash_bwd_kv");
+}

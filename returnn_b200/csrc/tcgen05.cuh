@@ -43,6 +43,13 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
 // shared memory matrix descriptor (sm_100 format): 128-byte swizzle
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   uint64_t d = 0;
@@ -97,6 +104,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(smem_src))
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z, const void* smem_src) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(smem_src))
+               : "memory");
+}
 // element-wise add of the box into global memory (performed at the L2, so concurrent adds to the same element are safe)
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, const void* smem_src) {
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
@@ -138,6 +150,45 @@ inline EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// encodes with `encode` (a callable that returns a CUresult)
+template <typename Encode>
+inline CUresult encode_in_context(Encode encode) {
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread that has made no runtime call yet (a worker thread of the autograd engine) has no current context for the driver
+    // API: cudaFree(0) binds the device's primary context to this thread
+    cudaFree(0);
+    r = encode();
+  }
+  return r;
+}
+
+// 3-D bf16 tensor map with the 128-byte swizzle: `rows` rows of `inner` contiguous elements, `row_pitch` elements apart, in each of
+// `batch` entries that are `batch_pitch` elements apart; boxes of 64 x box_rows within one entry, so that a tile that reaches past an
+// entry's last row reads zeros and writes nothing there
+inline int make_map_3d(CUtensorMap* map, const void* base, long long inner, long long rows, long long batch, long long row_pitch,
+                       long long batch_pitch, int box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) {
+    rb_set_error("cuTensorMapEncodeTiled not available");
+    return RB_ERR_UNSUPPORTED;
+  }
+  cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[2] = {(cuuint64_t)row_pitch * 2, (cuuint64_t)batch_pitch * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  cuuint32_t elem[3] = {1, 1, 1};
+  const CUresult r = encode_in_context([&]() {
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
+  if (r != CUDA_SUCCESS) {
+    rb_set_error("cuTensorMapEncodeTiled failed (%d): base %p inner %lld rows %lld batch %lld pitches %lld %lld", (int)r, base, inner, rows, batch,
+                 row_pitch, batch_pitch);
+    return RB_ERR_ARG;
+  }
+  return RB_OK;
+}
+
 // 2-D tensor map: inner (contiguous) extent `inner`, outer extent `outer`, row pitch in elements; bf16 elements with the 128-byte
 // swizzle unless said otherwise (fp32 = true: 4-byte elements; swizzle64 = true: boxes whose rows are 64 bytes long)
 inline int make_map(CUtensorMap* map, const void* base, long long inner, long long outer, long long pitch_elems, int box_inner, int box_outer,
@@ -151,18 +202,11 @@ inline int make_map(CUtensorMap* map, const void* base, long long inner, long lo
   cuuint64_t strides[1] = {(cuuint64_t)pitch_elems * (fp32 ? 4 : 2)};
   cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
   cuuint32_t elem[2] = {1, 1};
-  auto encode = [&]() {
+  const CUresult r = encode_in_context([&]() {
     return fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  };
-  CUresult r = encode();
-  if (r == CUDA_ERROR_INVALID_CONTEXT) {
-    // a thread that has made no runtime call yet (a worker thread of the autograd engine) has no current context for the driver
-    // API: cudaFree(0) binds the device's primary context to this thread
-    cudaFree(0);
-    r = encode();
-  }
+  });
   if (r != CUDA_SUCCESS) {
     rb_set_error("gemm: cuTensorMapEncodeTiled failed (%d): base %p inner %lld outer %lld pitch %lld", (int)r, base, inner, outer, pitch_elems);
     return RB_ERR_ARG;

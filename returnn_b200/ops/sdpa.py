@@ -158,6 +158,63 @@ class _SdpaFn(torch.autograd.Function):
         return (dq.view(B, Tq, H, D).to(in_dtype), dk.view(B, Tk, H, D).to(in_dtype), dv.view(B, Tk, H, D).to(in_dtype), None, None, None, None, None)
 
 
+class _FlashFn(torch.autograd.Function):
+    """head dim 64: one kernel forward, two backward (``csrc/sdpa_flash.cu``); nothing of size Tq x Tk is kept but the dropout bits"""
+
+    @staticmethod
+    def forward(ctx, q, k, v, k_lens, H, causal, scale, p_drop):
+        B, Tq, _, D = q.shape
+        Tk = k.shape[1]
+        dev = q.device
+        q2, rq, hq = _rows(q)
+        k2, rk, hk = _rows(k)
+        v2, rv, hv = _rows(v)
+        Tqp, Tkp = _r64(Tq), _r64(Tk)
+        words = (Tk + 127) // 128 * 4
+        o = torch.empty(B, Tq, H, D, dtype=torch.bfloat16, device=dev)
+        lse = torch.empty(B * H * Tq, dtype=torch.float32, device=dev)
+        drop = p_drop > 0.0
+        keep = seed = off = None
+        if drop:
+            keep = torch.empty(B * H * Tq * words, dtype=torch.int32, device=dev)
+            seed = _seed_tensor(dev)
+            off = seed[1:2].clone()
+            seed[1] += B * H * Tqp * Tkp
+        geom = (B, H, Tq, Tk, int(causal), Tk - Tq, rq, hq, rk, hk, rv, hv, 0, 0, Tqp, Tkp, words)
+        st = _gemm.status_tensor(dev)
+        fn = _lib.bind("rb200_flash_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp, _vp, _vp])
+        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), scale,
+                      p_drop, _p(seed), _p(off), st.data_ptr(), _lib.stream_ptr()), "flash_fwd")
+        _lib.count_launch()
+        ctx.save_for_backward(q2, k2, v2, o, lse, keep, k_lens)
+        ctx.geom, ctx.scale, ctx.p_drop, ctx.in_dtype = geom, scale, p_drop, q.dtype
+        return o if q.dtype == torch.bfloat16 else o.to(q.dtype)
+
+    @staticmethod
+    def backward(ctx, d_out):
+        q2, k2, v2, o, lse, keep, k_lens = ctx.saved_tensors
+        B, H, Tq, Tk = ctx.geom[:4]
+        dev, bf = d_out.device, torch.bfloat16
+        do2, rdo, hdo = _rows(d_out)
+        geom = ctx.geom[:12] + (rdo, hdo) + ctx.geom[14:]
+        delta = torch.empty_like(lse)
+        dq = torch.empty(B, Tq, H, 64, dtype=bf, device=dev)
+        dk = torch.empty(B, Tk, H, 64, dtype=bf, device=dev)
+        dv = torch.empty(B, Tk, H, 64, dtype=bf, device=dev)
+        st = _gemm.status_tensor(dev)
+        fn = _lib.bind("rb200_flash_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp])
+        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o.data_ptr(), do2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                      lse.data_ptr(), delta.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), ctx.scale, ctx.p_drop, st.data_ptr(),
+                      _lib.stream_ptr()), "flash_bwd")
+        _lib.count_launch(2)
+        dt = ctx.in_dtype
+        return dq.to(dt), dk.to(dt), dv.to(dt), None, None, None, None, None
+
+
+def _p(t: Optional[torch.Tensor]):
+    return None if t is None else t.data_ptr()
+
+
 def sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, num_heads: int, k_lens: Optional[torch.Tensor] = None, causal: bool = False,
          scale: Optional[float] = None, dropout_p: float = 0.0) -> torch.Tensor:
     """
@@ -190,7 +247,10 @@ def sdpa_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, k_lens: Opt
         scale = 1.0 / math.sqrt(d)
     if k_lens is not None:
         k_lens = host_to_device(k_lens.to(torch.int32), q.device).contiguous()
-    return _SdpaFn.apply(q, k, v, k_lens, int(num_heads), bool(causal), float(scale), float(dropout_p))
+    # the fused kernels are written for one 64-column tile per head, the head dim of all configurations here; other dims take the products
+    # with a softmax kernel in between
+    fn = _FlashFn if d == 64 and hasattr(_lib.get_lib(), "rb200_flash_fwd") else _SdpaFn
+    return fn.apply(q, k, v, k_lens, int(num_heads), bool(causal), float(scale), float(dropout_p))
 
 
 def sdpa_reference(q, k, v, *, num_heads: int, k_lens=None, causal: bool = False, scale: Optional[float] = None) -> torch.Tensor:

@@ -98,3 +98,43 @@ def test_sdpa_heads_reads_slices_of_a_fused_projection_in_place(layout):
     torch.testing.assert_close(out.float(), ref, atol=2e-2, rtol=2e-2)
     scale = float(qkv.grad.abs().max())
     assert float((got.float() - qkv.grad.float()).abs().max()) / scale < 3e-2
+
+
+@pytest.mark.parametrize("Tq,Tk,causal,with_lens", [
+    (1, 1, False, False),       # one score
+    (63, 65, False, True),      # a key into the second tile of 64
+    (65, 64, False, False),
+    (128, 128, True, False),    # whole tiles
+    (129, 257, True, True),     # one row into the second tile of queries; causal with more keys than queries
+    (200, 70, True, False),     # more queries than keys: the first queries see no key and get zeros
+])
+def test_sdpa_head_dim_64_tile_edges(Tq, Tk, causal, with_lens):
+    _case(2, 3, 64, Tq, Tk, causal, with_lens, seed=Tq)
+
+
+@pytest.mark.parametrize("T", [64, 50])
+def test_sdpa_head_dim_64_dropout_gradients(T):
+    """with the identity as values the output is the dropped probabilities: they give the mask, which the backward pass has to use as well"""
+    from returnn_b200.ops import sdpa as S
+    from returnn_b200.ops.elementwise import _seed_tensor
+
+    torch.manual_seed(5)
+    dev, B, H, D, p = torch.device("cuda"), 2, 2, 64, 0.3
+    q, k, v = ((torch.randn(B, T, H, D, device=dev) * 0.7).to(torch.bfloat16).requires_grad_(True) for _ in range(3))
+    eye = torch.eye(T, D, device=dev, dtype=torch.bfloat16)[None, :, None].expand(B, T, H, D).contiguous()
+    seed = _seed_tensor(q.device)
+    state = seed.clone()
+    probs = S.sdpa_heads(q, k, eye, dropout_p=p)
+    mask = (probs.detach().float()[..., :T] > 0).transpose(1, 2).float()  # [B, H, T, T]
+    assert abs(mask.mean().item() - (1 - p)) < 0.03
+    seed.copy_(state)
+    out = S.sdpa_heads(q, k, v, dropout_p=p)
+    w = torch.randn_like(out, dtype=torch.float32)
+    (out.float() * w).sum().backward()
+    qr, kr, vr = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+    att = torch.softmax(torch.einsum("bihd,bjhd->bhij", qr, kr) * D ** -0.5, -1) * mask / (1 - p)
+    ref = torch.einsum("bhij,bjhd->bihd", att, vr)
+    (ref * w).sum().backward()
+    torch.testing.assert_close(out.float(), ref, atol=2e-2, rtol=2e-2)
+    for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
+        assert (got.float() - want).norm() / want.norm() < 1e-2  # bf16 probabilities and results: 2^-9 each per element
