@@ -131,18 +131,43 @@ def _act_grad(z: torch.Tensor, dy: torch.Tensor, act: str) -> torch.Tensor:
     raise ValueError(act)
 
 
+def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], db: Optional[torch.Tensor]) -> torch.Tensor:
+    """
+    gradient before the activation, ``dy * act'(z)``, with its column sums added to ``db`` (fp32, None: not wanted), in one kernel
+
+    :param dy: [m, n] bf16, contiguous
+    """
+    if act is None and db is None:
+        return dy
+    m, n = dy.shape
+    # 16-byte accesses: a gradient that starts off that alignment takes the elementwise form
+    if dy.dtype == torch.bfloat16 and n % 8 == 0 and dy.data_ptr() % 16 == 0 and (z is None or z.data_ptr() % 16 == 0):
+        dz = torch.empty_like(dy) if act is not None else dy
+        fn = _lib.bind("rb200_act_grad_colsum", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        _lib.check(fn(z.data_ptr() if act is not None else None, dy.data_ptr(), dz.data_ptr() if act is not None else None,
+                      db.data_ptr() if db is not None else None, m, n, _ACT[act], _lib.stream_ptr()), "act_grad_colsum")
+        _lib.count_launch()
+        return dz
+    dz = _act_grad(z, dy, act) if act is not None else dy
+    if db is not None:
+        db += dz.float().sum(dim=0)
+    return dz
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x2, w, bias, act):
+    def forward(ctx, x2, weight, bias, act):
+        w = weight.to(torch.bfloat16).contiguous()
         m, k = x2.shape
         n = w.shape[1]
-        need_z = act is not None and (x2.requires_grad or w.requires_grad)
+        need_z = act is not None and (x2.requires_grad or weight.requires_grad)
         if need_z:
             z, y = gemm(x2, w, m=m, n=n, k=k, a_mn_major=False, b_mn_major=True, bias=bias, act=act, want_act_output=True)
         else:
             z, y = None, gemm(x2, w, m=m, n=n, k=k, a_mn_major=False, b_mn_major=True, bias=bias, act=act)
         ctx.save_for_backward(x2, w, z)
         ctx.act = act
+        ctx.w_dtype = weight.dtype
         ctx.has_bias = bias is not None
         ctx.bias_dtype = bias.dtype if bias is not None else None
         return y
@@ -153,18 +178,22 @@ class _LinearFn(torch.autograd.Function):
         m, k = x2.shape
         n = w.shape[1]
         dy = dy.contiguous()
-        if ctx.act is not None:
-            dy = _act_grad(z, dy, ctx.act)
         dx = dw = db = None
+        if ctx.has_bias and ctx.needs_input_grad[2]:
+            db = torch.zeros(n, dtype=torch.float32, device=dy.device)
+        dy = _grad_pre(dy, z, ctx.act, db)
         if ctx.needs_input_grad[0]:
             # dX[m,k] = dY[m,n] · W[k,n]^T : contraction over n, W rows are contiguous in n -> "K-major" B
             dx = gemm(dy, w, m=m, n=k, k=n, a_mn_major=False, b_mn_major=False)
         if ctx.needs_input_grad[1]:
             # dW[k,n] = X[m,k]^T · dY[m,n] : contraction over m, both operands contiguous in their output dim
-            dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy.float().sum(dim=0).to(ctx.bias_dtype)
-        return dx, dw, db, None
+            if ctx.w_dtype == torch.float32:
+                # few output tiles and a long contraction: the sum over the rows is split over the SMs into the fp32 gradient of the
+                # fp32 weight (one slice per tile is the plain product)
+                dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out=torch.zeros(k, n, dtype=torch.float32, device=dy.device), atomic=True)
+            else:
+                dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True).to(ctx.w_dtype)
+        return dx, dw, db.to(ctx.bias_dtype) if db is not None else None, None
 
 
 class _ArenaLinearFn(torch.autograd.Function):
@@ -192,15 +221,10 @@ class _ArenaLinearFn(torch.autograd.Function):
         m, k = x2.shape
         n = w16.shape[1]
         dy = dy.contiguous()
-        if ctx.act is not None:
-            dy = _act_grad(z, dy, ctx.act)
+        dy = _grad_pre(dy, z, ctx.act, ctx.gb32)
         dx = gemm(dy, w16, m=m, n=k, k=n, a_mn_major=False, b_mn_major=False) if ctx.needs_input_grad[0] else None
         if ctx.gw32 is not None:
             gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out=ctx.gw32, atomic=True)
-        if ctx.gb32 is not None:
-            fn = _lib.bind("rb200_colsum_bf16", [_vp, _vp, _i32, _i32, _vp])
-            _lib.check(fn(dy.data_ptr(), ctx.gb32.data_ptr(), m, n, _lib.stream_ptr()), "colsum")
-            _lib.count_launch()
         from ..parallel import grad_reducer as _gr
 
         _gr.notify_grads_written([ctx.gw32, ctx.gb32])
@@ -336,13 +360,10 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     """``x[..., in] @ weight[in, out] (+ bias) (activation)`` with bf16 operands"""
     if x.dtype != torch.bfloat16:
         x = x.to(torch.bfloat16)
-    w = weight if weight.dtype == torch.bfloat16 else weight.to(torch.bfloat16)
     if bias is not None and bias.dtype not in (torch.bfloat16, torch.float32):
         bias = bias.float()
-    if not w.is_contiguous():
-        w = w.contiguous()
     x2 = x.reshape(-1, x.shape[-1])
     if not x2.is_contiguous():
         x2 = x2.contiguous()
-    y = _LinearFn.apply(x2, w, bias, activation)
-    return y.reshape(*x.shape[:-1], w.shape[1])
+    y = _LinearFn.apply(x2, weight, bias, activation)
+    return y.reshape(*x.shape[:-1], weight.shape[1])

@@ -165,3 +165,26 @@ def test_linear_arena_padded_out():
         s = by_name[name]
         got = arena.flat_grad[s.offset: s.offset + s.numel].view(ref.shape)
         torch.testing.assert_close(got, ref, atol=3e-2, rtol=5e-2)
+
+
+@gpu
+@pytest.mark.parametrize("m,n,act", [(1, 8, "silu"), (31, 72, "relu"), (65, 64, "gelu"), (300, 136, "silu"), (5000, 1032, None)])
+def test_linear_backward_before_the_products(m, n, act):
+    """activation gradient and bias gradient in one kernel: rows and columns off its tiles, fp32 weight (its gradient stays fp32)"""
+    from returnn_b200.ops.linear import linear
+
+    torch.manual_seed(m)
+    dev, k = "cuda", 64
+    x = torch.randn(m, k, device=dev).to(torch.bfloat16).requires_grad_(True)
+    w = (torch.randn(k, n, device=dev) * 0.125).requires_grad_(True)
+    b = torch.randn(n, device=dev).requires_grad_(True)
+    dy = torch.randn(m, n, device=dev).to(torch.bfloat16)
+    got = torch.autograd.grad(linear(x, w, b, act), [x, w, b], dy)
+    assert got[1].dtype == torch.float32 and got[2].dtype == torch.float32
+    xr, wr, br = x.detach().double().requires_grad_(True), w.detach().bfloat16().double().requires_grad_(True), b.detach().double().requires_grad_(True)
+    z = xr @ wr + br
+    y = {"silu": torch.nn.functional.silu, "relu": torch.relu, "gelu": torch.nn.functional.gelu, None: lambda t: t}[act](z)
+    want = torch.autograd.grad(y, [xr, wr, br], dy.double())
+    for g, r in zip(got, want):
+        # z and dz are rounded to bf16 (2^-9 each), and dx again
+        assert (g.double() - r).norm() <= 8e-3 * r.norm() + 1e-6
