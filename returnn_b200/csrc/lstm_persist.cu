@@ -1,5 +1,5 @@
 // Persistent LSTM recurrence: ONE kernel runs all T steps of a direction. The recurrent matrix never leaves the chip: CTA c
-// keeps the rows of W_rec that produce the four gates of its kUnits hidden units in shared memory (forward), or the columns
+// keeps the rows of W_rec that produce the four gates of its hidden units in shared memory (forward), or the columns
 // that those units feed (backward), for the whole sequence. Per step a CTA multiplies the small [B, K] activation matrix (read
 // from L2, where the other CTAs wrote it in the previous step) with its resident slice on the tensor cores, applies the cell
 // for its units, publishes its slice of h_t (or dz_t) and meets the other CTAs at a grid barrier. The per-step executor in
@@ -23,44 +23,64 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kUnits = 8;      // hidden units per CTA (H = 1024 -> 128 CTAs)
 constexpr int kMaxRows = 48;   // batch rows (three m16 tiles)
-constexpr int kThreads = 256;  // eight warps: each takes one eighth of the contraction
 constexpr int kPad = 32;       // row padding of the resident slice: pitch = 64 bytes mod 128 (conflict-free 16-byte fragment loads)
 constexpr int kRedPad = 8;      // row padding of the partial-sum slots
+constexpr int kMaxCtas = 160;   // CTAs of one direction
 constexpr uint32_t kSpinLimit = 1u << 22;
+
+// How a direction is spread over the GPU: U hidden units per CTA, W warps that split the contraction, room for 16 * MT batch rows.
+// Narrow: two CTAs per SM for the two directions of a layer (one direction: one per SM). Wide: one CTA per SM with twice the units. All
+// CTAs read the whole exchanged matrix in every step, so half the CTAs halve that L2 traffic (H = 1024, 16 rows, backward: 17 instead of
+// 34 MB per step) and the flags of a barrier, and with 16 warps a warp has all of its operand loads in flight at once. Three row tiles do
+// not fit the 128 registers of a 512-thread CTA: batches above 32 rows take the narrow form.
+template <int UNITS, int WARPS, int TILES, int PF_FWD, int PF_BWD>
+struct Shape {
+  static constexpr int U = UNITS, W = WARPS, MT = TILES, Threads = 32 * WARPS, Rows = 16 * TILES, Slots = WARPS / 2;
+  static constexpr int PrefetchFwd = PF_FWD, PrefetchBwd = PF_BWD;  // blocks of 32 k whose loads a warp has in flight
+  static constexpr int PerThread = (Rows * UNITS + Threads - 1) / Threads;  // (row, unit) pairs of a thread
+};
+using Narrow = Shape<8, 8, 3, 4, 4>;
+using NarrowPair = Shape<8, 8, 3, 2, 2>;
+using Wide1 = Shape<16, 16, 1, 2, 8>;
+using Wide2 = Shape<16, 16, 2, 2, 4>;
 
 __device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + __expf(-x)); }
 
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
+__device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
   uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
-// all CTAs of the grid; false (for every thread of every CTA, eventually) when someone timed out
-__device__ bool grid_barrier(uint32_t* counter, uint32_t target, int* abort_word, int* status) {
-  __shared__ int sh_ok;
+// Barrier of the CTAs of one direction, in two halves: a CTA announces that its slice of the exchanged matrix is written by storing the
+// step number into its own flag word (no atomic: adds of all CTAs onto one counter are served one after the other), does what the others
+// need not wait for, and then waits for all flags, one thread per flag. Only the exchanged slice is stored before the announcement, so the
+// fence in it does not wait for the tensors that are kept for the backward pass.
+__device__ __forceinline__ void barrier_arrive(uint32_t* flags, int cta, uint32_t step) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(counter, 1u);
-    int ok = 1;
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flags + cta), "r"(step) : "memory");
+  }
+}
+// false (for every thread of every CTA, eventually) when someone timed out
+__device__ __forceinline__ bool barrier_wait(uint32_t* flags, int n_cta, uint32_t step, int* abort_word, int* status) {
+  int ok = 1;
+  if ((int)threadIdx.x < n_cta) {
     uint32_t spins = 0;
-    while ((int32_t)(ld_acquire_gpu(counter) - target) < 0) {
-      if (++spins > kSpinLimit || *reinterpret_cast<volatile int*>(abort_word)) {
+    while ((int32_t)(ld_relaxed_gpu(flags + threadIdx.x) - step) < 0) {
+      ++spins;
+      if (spins > kSpinLimit || ((spins & 255u) == 0 && *reinterpret_cast<volatile int*>(abort_word))) {
         ok = 0;
         atomicExch(abort_word, 1);
         if (status) atomicCAS(status, 0, (5 << 24) | (int)(blockIdx.x & 0xFFFF));
         break;
       }
-      __nanosleep(64);
     }
     __threadfence();
-    sh_ok = ok;
   }
-  __syncthreads();
-  return sh_ok != 0;
+  return __syncthreads_and(ok) != 0;
 }
 
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -70,42 +90,41 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 // red[row][n] += sum_k A[row][k] * Bs[n][k] for rows < n_rows; A in global (written by other CTAs: read through L2), Bs resident
-// in shared memory with row pitch K + kPad. The contraction is cut into blocks of 32 k; the warp w takes the blocks
-// [w*nblk/8, (w+1)*nblk/8).
+// in shared memory with row pitch K + kPad. The contraction is cut into blocks of 32 k; the warp w of S::W takes the blocks
+// [w*nblk/W, (w+1)*nblk/W).
 //
 // Operand fetch: all CTAs read the same small A matrix at the same time, so the number of L2 requests, not the bytes, sets the
 // step time. A lane therefore fetches 16 contiguous bytes (8 k) per row and block instead of four 4-byte fragment words: the
 // order of the k inside a block is free as long as A and B agree, so the lane t of a quad owns k [8t, 8t+8) of the block, its
 // words 0/1 feed the first m16n8k16 (as the fragment halves "k 2t.." and "k 2t+8..") and its words 2/3 the second one. The B
 // fragments come from shared memory with the same 16-byte pattern (row pitch = 64 bytes mod 128: conflict-free quarter warps).
-template <int NOUT, int kPrefetch>
+template <typename S, int NOUT, int kPrefetch>
 __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_rows, int K, const bf16* __restrict__ Bs, float* __restrict__ red) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int pitch = K + kPad;
-  float acc[3][NOUT / 8][4];
+  float acc[S::MT][NOUT / 8][4];
 #pragma unroll
-  for (int m = 0; m < 3; ++m)
+  for (int m = 0; m < S::MT; ++m)
 #pragma unroll
     for (int n = 0; n < NOUT / 8; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
   const int m_tiles = (n_rows + 15) / 16;
-  auto load_a = [&](int k0, uint4 (&a)[3][2]) {
+  auto load_a = [&](int k0, uint4 (&a)[S::MT][2]) {
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m < S::MT; ++m) {
       const int r0 = m * 16 + g, r1 = r0 + 8;
       a[m][0] = r0 < n_rows ? __ldcg(reinterpret_cast<const uint4*>(A + (size_t)r0 * K + k0 + 8 * t)) : make_uint4(0u, 0u, 0u, 0u);
       a[m][1] = r1 < n_rows ? __ldcg(reinterpret_cast<const uint4*>(A + (size_t)r1 * K + k0 + 8 * t)) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
   // chunks of kPrefetch blocks: all operand loads of a chunk are issued before its first multiply, so a chunk costs one L2 round
-  // trip (kPrefetch = 4: the forward contraction of H = 1024 is a single chunk per warp; the two-direction kernels use 2 to stay
-  // within 128 registers, so that two CTAs share an SM and cover each other's round trips)
+  // trip (as many as the registers hold: wide, 16 rows: one trip at H = 1024 in both passes; narrow with two CTAs per SM: 2 and 8 trips)
   const int nblk = K >> 5;
-  const int b_begin = warp * nblk / 8, b_end = (warp + 1) * nblk / 8;
+  const int b_begin = warp * nblk / S::W, b_end = (warp + 1) * nblk / S::W;
   for (int bc = b_begin; bc < b_end; bc += kPrefetch) {
-    uint4 a[kPrefetch][3][2];
+    uint4 a[kPrefetch][S::MT][2];
 #pragma unroll
     for (int i = 0; i < kPrefetch; ++i)
       if (bc + i < b_end) load_a((bc + i) << 5, a[i]);
@@ -117,7 +136,7 @@ __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_ro
       for (int n = 0; n < NOUT / 8; ++n) {
         const uint4 b = *reinterpret_cast<const uint4*>(Bs + (size_t)(n * 8 + g) * pitch + k0 + 8 * t);
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
+        for (int m = 0; m < S::MT; ++m) {
           if (m >= m_tiles) continue;
           const uint32_t f0[4] = {a[i][m][0].x, a[i][m][1].x, a[i][m][0].y, a[i][m][1].y};
           mma16816(acc[m][n], f0, b.x, b.y);
@@ -127,15 +146,15 @@ __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_ro
       }
     }
   }
-  // The partial sums of the eight warps meet in shared memory without atomics (eight warps adding 48 values per lane onto the
-  // same words was the largest batch-dependent part of a forward step): warps 4..7 store theirs into slot (warp - 4), warps
-  // 0..3 add their own onto that slot, the caller sums the four slots (red_sum). Row pitch NOUT + 8 floats: the 8-byte accesses
+  // The partial sums of the warps meet in shared memory without atomics (warps adding 48 values per lane onto the
+  // same words was the largest batch-dependent part of a forward step): the upper half of the warps store theirs into slot warp - W/2, the
+  // lower half add their own onto that slot, the caller sums the W/2 slots (red_sum). Row pitch NOUT + 8 floats: the 8-byte accesses
   // of a half warp fall on distinct banks.
   constexpr int RP = NOUT + kRedPad;
-  float* slot = red + (warp & 3) * (kMaxRows * RP);
-  if (warp >= 4) {
+  float* slot = red + (warp & (S::Slots - 1)) * (S::Rows * RP);
+  if (warp >= S::Slots) {
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m < S::MT; ++m) {
       if (m >= m_tiles) continue;
       const int r0 = m * 16 + g, r1 = r0 + 8;
 #pragma unroll
@@ -147,9 +166,9 @@ __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_ro
     }
   }
   __syncthreads();
-  if (warp < 4) {
+  if (warp < S::Slots) {
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m < S::MT; ++m) {
       if (m >= m_tiles) continue;
       const int r0 = m * 16 + g, r1 = r0 + 8;
 #pragma unroll
@@ -165,12 +184,19 @@ __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_ro
   }
 }
 
-// sum over the four slots that step_matmul leaves (after a __syncthreads)
-template <int NOUT>
+// sum over the slots that step_matmul leaves (after a __syncthreads)
+template <typename S, int NOUT>
 __device__ __forceinline__ float red_sum(const float* __restrict__ red, int row, int col) {
   constexpr int RP = NOUT + kRedPad;
   const float* q = red + row * RP + col;
-  return (q[0] + q[kMaxRows * RP]) + (q[2 * kMaxRows * RP] + q[3 * kMaxRows * RP]);
+  float v[S::Slots];
+#pragma unroll
+  for (int i = 0; i < S::Slots; ++i) v[i] = q[i * S::Rows * RP];
+#pragma unroll
+  for (int d = S::Slots / 2; d > 0; d >>= 1)
+#pragma unroll
+    for (int i = 0; i < d; ++i) v[i] += v[i + d];
+  return v[0];
 }
 
 struct FwdArgs {
@@ -185,119 +211,130 @@ struct FwdArgs {
   bf16* hprev_all;      // [T,B,H]
   float *h_final, *c_final;
   bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state
-  uint32_t* counter;    // zeroed before the launch
+  uint32_t* flags;      // one word per CTA, zeroed before the launch
   int* abort_word;      // zeroed before the launch
   int* status;          // receives (5 << 24) | cta when a barrier wait ran out
 };
 
-template <int kPrefetch>
-__device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const uint32_t n_cta) {
+template <typename S>
+__device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const int n_cta) {
+  constexpr int U = S::U, kThreads = S::Threads, NOUT = 4 * U;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int H = p.H, B = p.B;
   const int pitch = H + kPad;
-  bf16* Ws = reinterpret_cast<bf16*>(smem_raw);                                 // [4*kUnits][H+kPad]: row q*kUnits+u = W_rec[q*H + j0 + u]
-  float* red = reinterpret_cast<float*>(Ws + (size_t)4 * kUnits * pitch);       // [4 slots][48][4*kUnits + kRedPad]
-  float* cst = red + 4 * kMaxRows * (4 * kUnits + kRedPad);                                     // [48][kUnits] cell state
-  float* hst = cst + kMaxRows * kUnits;                                         // [48][kUnits] own slice of h (fp32)
-  const int j0 = cta * kUnits;
-  // resident slice: 4*kUnits rows of H elements, 16-byte copies
-  for (int idx = threadIdx.x; idx < 4 * kUnits * (H / 8); idx += kThreads) {
+  bf16* Ws = reinterpret_cast<bf16*>(smem_raw);                           // [4*U][H+kPad]: row q*U+u = W_rec[q*H + j0 + u]
+  float* red = reinterpret_cast<float*>(Ws + (size_t)NOUT * pitch);       // [slots][rows][4*U + kRedPad]
+  const int j0 = cta * U;
+  // resident slice: 4*U rows of H elements, 16-byte copies
+  for (int idx = threadIdx.x; idx < NOUT * (H / 8); idx += kThreads) {
     const int r = idx / (H / 8), v = idx % (H / 8);
-    const int q = r / kUnits, u = r % kUnits;
+    const int q = r / U, u = r % U;
     *reinterpret_cast<uint4*>(Ws + (size_t)r * pitch + v * 8) = *reinterpret_cast<const uint4*>(p.w_rec + ((size_t)q * H + j0 + u) * H + v * 8);
   }
-  for (int idx = threadIdx.x; idx < kMaxRows * kUnits; idx += kThreads) {
-    const int b = idx / kUnits, u = idx % kUnits;
-    float c = 0.f, h = 0.f;
-    if (b < B) {
-      c = p.c0[(size_t)b * H + j0 + u];
-      h = p.h0[(size_t)b * H + j0 + u];
-      p.hbuf[(size_t)b * H + j0 + u] = __float2bfloat16(h);
+  // every thread owns up to PerThread (row, unit) pairs: their state stays in registers, and their input projections z_in[t] are fetched
+  // one step ahead (they come from DRAM) so that the cell does not wait for them after the barrier
+  constexpr int N = S::PerThread;
+  float cst[N], hst[N];
+  bf16 zin[N][4];  // as loaded: a conversion next to the load would wait for it
+  int len[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int idx = threadIdx.x + i * kThreads;
+    const int b = idx / U, u = idx % U;
+    cst[i] = hst[i] = 0.f;
+    len[i] = p.T;
+    if (idx < B * U) {
+      const float h = p.h0[(size_t)b * H + j0 + u];
+      const bf16 hb = __float2bfloat16(h);
+      cst[i] = p.c0[(size_t)b * H + j0 + u];
+      hst[i] = __bfloat162float(hb);
+      if (p.lens) len[i] = p.lens[b];
+      p.hbuf[(size_t)b * H + j0 + u] = hb;
     }
-    cst[idx] = c;
-    hst[idx] = __bfloat162float(__float2bfloat16(h));
   }
-  // every thread owns up to kSlots (row, unit) pairs; their input projections z_in[t] are fetched one step ahead (they come from
-  // DRAM) so that the cell does not wait for them after the barrier
-  constexpr int kSlots = (kMaxRows * kUnits + kThreads - 1) / kThreads;
-  float zin[kSlots][4];
   auto fetch_zin = [&](int t) {
 #pragma unroll
-    for (int i = 0; i < kSlots; ++i) {
+    for (int i = 0; i < N; ++i) {
       const int idx = threadIdx.x + i * kThreads;
-      if (idx < B * kUnits) {
-        const int b = idx / kUnits, u = idx % kUnits;
+      if (idx < B * U) {
+        const int b = idx / U, u = idx % U;
         const bf16* z = p.z_in + ((size_t)t * B + b) * 4 * H + j0 + u;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) zin[i][q] = __bfloat162float(z[(size_t)q * H]);
+        for (int q = 0; q < 4; ++q) zin[i][q] = z[(size_t)q * H];
       }
     }
   };
+  uint32_t n_bar = 1;
+  barrier_arrive(p.flags, cta, n_bar);
   if (p.T > 0) fetch_zin(p.reverse ? p.T - 1 : 0);
-  uint32_t n_bar = 0;
-  bool ok = grid_barrier(p.counter, (++n_bar) * n_cta, p.abort_word, p.status);
+  bool ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);
   for (int s = 0; s < p.T && ok; ++s) {
     const int t = p.reverse ? p.T - 1 - s : s;
     const bf16* h_cur = p.hbuf + (size_t)(s & 1) * B * H;
     bf16* h_nxt = p.hbuf + (size_t)((s + 1) & 1) * B * H;
-    step_matmul<4 * kUnits, kPrefetch>(h_cur, B, H, Ws, red);
+    step_matmul<S, NOUT, S::PrefetchFwd>(h_cur, B, H, Ws, red);
     __syncthreads();
+    float gates[N][4], hp[N];
 #pragma unroll
-    for (int i = 0; i < kSlots; ++i) {
+    for (int i = 0; i < N; ++i) {
       const int idx = threadIdx.x + i * kThreads;
-      if (idx >= B * kUnits) continue;
-      const int b = idx / kUnits, u = idx % kUnits;
+      if (idx >= B * U) continue;
+      const int b = idx / U, u = idx % U;
+      hp[i] = hst[i];
+      gates[i][0] = gates[i][1] = gates[i][2] = gates[i][3] = 0.f;
+      if (t < len[i]) {
+        const float gi = sigm(red_sum<S, NOUT>(red, b, u) + __bfloat162float(zin[i][0]));
+        const float gf = sigm(red_sum<S, NOUT>(red, b, U + u) + __bfloat162float(zin[i][1]));
+        const float gg = tanhf(red_sum<S, NOUT>(red, b, 2 * U + u) + __bfloat162float(zin[i][2]));
+        const float go = sigm(red_sum<S, NOUT>(red, b, 3 * U + u) + __bfloat162float(zin[i][3]));
+        const float c = gf * cst[i] + gi * gg;
+        cst[i] = c;
+        hst[i] = __bfloat162float(__float2bfloat16(go * tanhf(c)));
+        gates[i][0] = gi; gates[i][1] = gf; gates[i][2] = gg; gates[i][3] = go;
+      }
+      h_nxt[(size_t)b * H + j0 + u] = __float2bfloat16(hst[i]);
+    }
+    barrier_arrive(p.flags, cta, ++n_bar);
+    if (s + 1 < p.T) fetch_zin(p.reverse ? p.T - 2 - s : s + 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int idx = threadIdx.x + i * kThreads;
+      if (idx >= B * U) continue;
+      const int b = idx / U, u = idx % U;
       const size_t o = ((size_t)t * B + b) * H + j0 + u;
       const size_t zo = ((size_t)t * B + b) * 4 * H + j0 + u;
-      const bool valid = !p.lens || t < p.lens[b];
-      const float hp = hst[idx], cp = cst[idx];
-      p.hprev_all[o] = __float2bfloat16(hp);
-      if (!valid) {
-        p.y[o] = __float2bfloat16(0.f);
-        p.c_all[o] = cp;
-        p.gates[zo] = p.gates[zo + H] = p.gates[zo + 2 * H] = p.gates[zo + 3 * H] = __float2bfloat16(0.f);
-        h_nxt[(size_t)b * H + j0 + u] = __float2bfloat16(hp);
-        continue;
-      }
-      const float gi = sigm(red_sum<4 * kUnits>(red, b, u) + zin[i][0]);
-      const float gf = sigm(red_sum<4 * kUnits>(red, b, kUnits + u) + zin[i][1]);
-      const float gg = tanhf(red_sum<4 * kUnits>(red, b, 2 * kUnits + u) + zin[i][2]);
-      const float go = sigm(red_sum<4 * kUnits>(red, b, 3 * kUnits + u) + zin[i][3]);
-      const float c = gf * cp + gi * gg;
-      const bf16 hb = __float2bfloat16(go * tanhf(c));
-      cst[idx] = c;
-      hst[idx] = __bfloat162float(hb);
-      p.c_all[o] = c;
-      p.y[o] = hb;
-      h_nxt[(size_t)b * H + j0 + u] = hb;
-      p.gates[zo] = __float2bfloat16(gi);
-      p.gates[zo + H] = __float2bfloat16(gf);
-      p.gates[zo + 2 * H] = __float2bfloat16(gg);
-      p.gates[zo + 3 * H] = __float2bfloat16(go);
+      p.hprev_all[o] = __float2bfloat16(hp[i]);
+      p.y[o] = __float2bfloat16(t < len[i] ? hst[i] : 0.f);
+      p.c_all[o] = cst[i];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) p.gates[zo + (size_t)q * H] = __float2bfloat16(gates[i][q]);
     }
-    if (s + 1 < p.T) fetch_zin(p.reverse ? p.T - 2 - s : s + 1);
-    ok = grid_barrier(p.counter, (++n_bar) * n_cta, p.abort_word, p.status);
+    ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);
   }
-  for (int idx = threadIdx.x; idx < B * kUnits; idx += kThreads) {
-    const int b = idx / kUnits, u = idx % kUnits;
-    p.h_final[(size_t)b * H + j0 + u] = hst[idx];
-    p.c_final[(size_t)b * H + j0 + u] = cst[idx];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int idx = threadIdx.x + i * kThreads;
+    if (idx >= B * U) continue;
+    const size_t o = (size_t)(idx / U) * H + j0 + idx % U;
+    p.h_final[o] = hst[i];
+    p.c_final[o] = cst[i];
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) lstm_persist_fwd_kernel(FwdArgs p) { fwd_body<4>(p, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(Narrow::Threads, 1) lstm_persist_fwd_kernel(FwdArgs p) { fwd_body<Narrow>(p, blockIdx.x, gridDim.x); }
 
-// Both directions of a bidirectional layer in one launch: the first half of the grid runs d[0], the second half d[1], each with
-// its own barrier words. Two CTAs share an SM (128 registers per thread), so the two recurrences, each bound by the latency of
-// its grid barrier and L2 round trip per step, overlap instead of running one after the other.
+// Both directions of a bidirectional layer in one launch: the first half of the grid runs d[0], the second half d[1], each with its own
+// flags: two recurrences, each bound by the latency of its barrier and L2 round trips per step, overlap instead of running one after the
+// other. Narrow: two CTAs per SM (128 registers per thread); wide: one.
 struct FwdPair {
   FwdArgs d[2];
 };
 
-__global__ void __launch_bounds__(kThreads, 2) lstm_persist_fwd_pair_kernel(const __grid_constant__ FwdPair pp) {
+template <typename S>
+__global__ void __launch_bounds__(S::Threads, S::U == 8 ? 2 : 1) lstm_persist_fwd_pair_kernel(const __grid_constant__ FwdPair pp) {
   const int half = gridDim.x / 2;
-  if ((int)blockIdx.x < half) fwd_body<2>(pp.d[0], blockIdx.x, half);
-  else fwd_body<2>(pp.d[1], blockIdx.x - half, half);
+  if ((int)blockIdx.x < half) fwd_body<S>(pp.d[0], blockIdx.x, half);
+  else fwd_body<S>(pp.d[1], blockIdx.x - half, half);
 }
 
 struct BwdArgs {
@@ -310,92 +347,130 @@ struct BwdArgs {
   int T, B, H, reverse;
   bf16* dz;              // [T,B,4H]: output and per-step exchange buffer
   float *dh0, *dc0;      // [B,H] outputs
-  uint32_t* counter;
+  uint32_t* flags;
   int* abort_word;
   int* status;
 };
 
-template <int kPrefetch>
-__device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const uint32_t n_cta) {
+template <typename S>
+__device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const int n_cta) {
+  constexpr int U = S::U, kThreads = S::Threads;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int H = p.H, B = p.B, K = 4 * p.H;
   const int pitch = K + kPad;
-  bf16* Wt = reinterpret_cast<bf16*>(smem_raw);                      // [kUnits][4H+kPad]: Wt[u][n] = W_rec[n][j0+u]
-  float* red = reinterpret_cast<float*>(Wt + (size_t)kUnits * pitch);  // [4 slots][48][kUnits + kRedPad]
-  float* dhs = red + 4 * kMaxRows * (kUnits + kRedPad);                              // [48][16] gradient arriving at h_t
-  float* dcs = dhs + kMaxRows * kUnits;                              // [48][16] gradient arriving at c_t
-  const int j0 = cta * kUnits;
-  for (int idx = threadIdx.x; idx < K * (kUnits / 8); idx += kThreads) {
-    // row n of W_rec, units j0 .. j0 + kUnits - 1, in 16-byte pieces
-    const int n = idx / (kUnits / 8), piece = idx % (kUnits / 8);
+  bf16* Wt = reinterpret_cast<bf16*>(smem_raw);                    // [U][4H+kPad]: Wt[u][n] = W_rec[n][j0+u]
+  float* red = reinterpret_cast<float*>(Wt + (size_t)U * pitch);   // [slots][rows][U + kRedPad]
+  const int j0 = cta * U;
+  for (int idx = threadIdx.x; idx < K * (U / 8); idx += kThreads) {
+    // row n of W_rec, units j0 .. j0 + U - 1, in 16-byte pieces
+    const int n = idx / (U / 8), piece = idx % (U / 8);
     const uint4 v = *reinterpret_cast<const uint4*>(p.w_rec + (size_t)n * H + j0 + piece * 8);
     const bf16* e = reinterpret_cast<const bf16*>(&v);
 #pragma unroll
     for (int i = 0; i < 8; ++i) Wt[(size_t)(piece * 8 + i) * pitch + n] = e[i];
   }
-  for (int idx = threadIdx.x; idx < kMaxRows * kUnits; idx += kThreads) {
-    const int b = idx / kUnits, u = idx % kUnits;
-    dhs[idx] = (b < B && p.dh_final) ? p.dh_final[(size_t)b * H + j0 + u] : 0.f;
-    dcs[idx] = (b < B && p.dc_final) ? p.dc_final[(size_t)b * H + j0 + u] : 0.f;
+  // a thread's (row, unit) pairs: gradients arriving at h_t and c_t, and what the forward pass kept, fetched one step ahead (DRAM)
+  constexpr int N = S::PerThread;
+  float dhs[N], dcs[N], c_t[N], c_p[N];
+  bf16 kept[N][4], dy[N];  // as loaded: a conversion next to the load would wait for it
+  int len[N];
+  auto fetch = [&](int s) {  // gates, dy and the cell state before step s; (the state after it is that of the step after)
+    const int t = p.reverse ? p.T - 1 - s : s;
+    const int t_prev = p.reverse ? t + 1 : t - 1;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int idx = threadIdx.x + i * kThreads;
+      if (idx >= B * U) continue;
+      const int b = idx / U, u = idx % U;
+      const bf16* gt = p.gates + ((size_t)t * B + b) * K + j0 + u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) kept[i][q] = gt[(size_t)q * H];
+      dy[i] = p.dy ? p.dy[((size_t)t * B + b) * H + j0 + u] : __float2bfloat16(0.f);
+      c_p[i] = s > 0 ? p.c_all[((size_t)t_prev * B + b) * H + j0 + u] : p.c0[(size_t)b * H + j0 + u];
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int idx = threadIdx.x + i * kThreads;
+    dhs[i] = dcs[i] = c_t[i] = 0.f;
+    len[i] = p.T;
+    if (idx >= B * U) continue;
+    const int b = idx / U, u = idx % U;
+    if (p.dh_final) dhs[i] = p.dh_final[(size_t)b * H + j0 + u];
+    if (p.dc_final) dcs[i] = p.dc_final[(size_t)b * H + j0 + u];
+    if (p.lens) len[i] = p.lens[b];
+    if (p.T > 0) c_t[i] = p.c_all[((size_t)(p.reverse ? 0 : p.T - 1) * B + b) * H + j0 + u];
   }
+  if (p.T > 0) fetch(p.T - 1);
   __syncthreads();
   uint32_t n_bar = 0;
   bool ok = true;
   for (int s = p.T - 1; s >= 0 && ok; --s) {
     const int t = p.reverse ? p.T - 1 - s : s;
-    const int t_prev = p.reverse ? t + 1 : t - 1;
     bf16* dz_t = p.dz + (size_t)t * B * K;
-    for (int idx = threadIdx.x; idx < B * kUnits; idx += kThreads) {
-      const int b = idx / kUnits, u = idx % kUnits;
-      const size_t o = ((size_t)t * B + b) * H + j0 + u;
-      const size_t zo = (size_t)b * K + j0 + u;
-      const bool valid = !p.lens || t < p.lens[b];
-      if (!valid) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int idx = threadIdx.x + i * kThreads;
+      if (idx >= B * U) continue;
+      const size_t zo = (size_t)(idx / U) * K + j0 + idx % U;
+      if (t >= len[i]) {
         dz_t[zo] = dz_t[zo + H] = dz_t[zo + 2 * H] = dz_t[zo + 3 * H] = __float2bfloat16(0.f);
         continue;  // state was carried: dh and dc pass through
       }
-      const float dh = dhs[idx] + (p.dy ? __bfloat162float(p.dy[o]) : 0.f);
-      const bf16* gt = p.gates + ((size_t)t * B + b) * K + j0 + u;
-      const float gi = __bfloat162float(gt[0]), gf = __bfloat162float(gt[H]), gg = __bfloat162float(gt[2 * H]), go = __bfloat162float(gt[3 * H]);
-      const float tc = tanhf(p.c_all[o]);
-      const float cprev = s > 0 ? p.c_all[((size_t)t_prev * B + b) * H + j0 + u] : p.c0[(size_t)b * H + j0 + u];
-      const float dc = dcs[idx] + dh * go * (1.f - tc * tc);
+      const float dh = dhs[i] + __bfloat162float(dy[i]);
+      const float gi = __bfloat162float(kept[i][0]), gf = __bfloat162float(kept[i][1]), gg = __bfloat162float(kept[i][2]),
+                  go = __bfloat162float(kept[i][3]);
+      const float tc = tanhf(c_t[i]);
+      const float dc = dcs[i] + dh * go * (1.f - tc * tc);
       dz_t[zo] = __float2bfloat16(dc * gg * gi * (1.f - gi));
-      dz_t[zo + H] = __float2bfloat16(dc * cprev * gf * (1.f - gf));
+      dz_t[zo + H] = __float2bfloat16(dc * c_p[i] * gf * (1.f - gf));
       dz_t[zo + 2 * H] = __float2bfloat16(dc * gi * (1.f - gg * gg));
       dz_t[zo + 3 * H] = __float2bfloat16(dh * tc * go * (1.f - go));
-      dcs[idx] = dc * gf;
-      dhs[idx] = 0.f;
+      dcs[i] = dc * gf;
+      dhs[i] = 0.f;
     }
-    ok = grid_barrier(p.counter, (++n_bar) * n_cta, p.abort_word, p.status);  // all slices of dz_t are written
+    barrier_arrive(p.flags, cta, ++n_bar);
+#pragma unroll
+    for (int i = 0; i < N; ++i) c_t[i] = c_p[i];
+    if (s > 0) fetch(s - 1);
+    ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);  // all slices of dz_t are written
     if (!ok) break;
-    step_matmul<kUnits, kPrefetch>(dz_t, B, K, Wt, red);
+    step_matmul<S, U, S::PrefetchBwd>(dz_t, B, K, Wt, red);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < B * kUnits; idx += kThreads) dhs[idx] += red_sum<kUnits>(red, idx / kUnits, idx % kUnits);
-    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int idx = threadIdx.x + i * kThreads;
+      if (idx < B * U) dhs[i] += red_sum<S, U>(red, idx / U, idx % U);
+    }
+    // (the slots are written again after the next barrier only)
   }
-  for (int idx = threadIdx.x; idx < B * kUnits; idx += kThreads) {
-    const int b = idx / kUnits, u = idx % kUnits;
-    p.dh0[(size_t)b * H + j0 + u] = dhs[idx];
-    p.dc0[(size_t)b * H + j0 + u] = dcs[idx];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int idx = threadIdx.x + i * kThreads;
+    if (idx >= B * U) continue;
+    const size_t o = (size_t)(idx / U) * H + j0 + idx % U;
+    p.dh0[o] = dhs[i];
+    p.dc0[o] = dcs[i];
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) lstm_persist_bwd_kernel(BwdArgs p) { bwd_body<4>(p, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(Narrow::Threads, 1) lstm_persist_bwd_kernel(BwdArgs p) { bwd_body<Narrow>(p, blockIdx.x, gridDim.x); }
 
 struct BwdPair {
   BwdArgs d[2];
 };
 
-__global__ void __launch_bounds__(kThreads, 2) lstm_persist_bwd_pair_kernel(const __grid_constant__ BwdPair pp) {
+template <typename S>
+__global__ void __launch_bounds__(S::Threads, S::U == 8 ? 2 : 1) lstm_persist_bwd_pair_kernel(const __grid_constant__ BwdPair pp) {
   const int half = gridDim.x / 2;
-  if ((int)blockIdx.x < half) bwd_body<2>(pp.d[0], blockIdx.x, half);
-  else bwd_body<2>(pp.d[1], blockIdx.x - half, half);
+  if ((int)blockIdx.x < half) bwd_body<S>(pp.d[0], blockIdx.x, half);
+  else bwd_body<S>(pp.d[1], blockIdx.x - half, half);
 }
 
-// barrier words of the calls in flight: 64 slots of (counter, abort word), handed out round robin
+// barrier words of the calls in flight: 64 slots of (abort word, flags), handed out round robin
 constexpr int kSyncSlots = 64;
-static __device__ unsigned int g_lstm_sync[kSyncSlots * 2];
+constexpr int kSyncWords = 32 + kMaxCtas;  // the flags start on a line of their own
+static __device__ __align__(128) unsigned int g_lstm_sync[kSyncSlots * kSyncWords];
 
 unsigned int* sync_slot() {
   static unsigned int* base[64] = {nullptr};
@@ -407,14 +482,16 @@ unsigned int* sync_slot() {
     if (cudaGetSymbolAddress((void**)&ptr, g_lstm_sync) != cudaSuccess) return nullptr;
     base[dev] = ptr;
   }
-  return base[dev] + 2 * (next++ % kSyncSlots);
+  return base[dev] + kSyncWords * (next++ % kSyncSlots);
 }
 
+template <typename S>
 size_t fwd_smem(int H) {
-  return (size_t)4 * kUnits * (H + kPad) * sizeof(bf16) + (size_t)kMaxRows * (4 * (4 * kUnits + kRedPad) + 2 * kUnits) * sizeof(float);
+  return (size_t)4 * S::U * (H + kPad) * sizeof(bf16) + (size_t)S::Slots * S::Rows * (4 * S::U + kRedPad) * sizeof(float);
 }
+template <typename S>
 size_t bwd_smem(int H) {
-  return (size_t)kUnits * (4 * H + kPad) * sizeof(bf16) + (size_t)kMaxRows * (4 * (kUnits + kRedPad) + 2 * kUnits) * sizeof(float);
+  return (size_t)S::U * (4 * H + kPad) * sizeof(bf16) + (size_t)S::Slots * S::Rows * (S::U + kRedPad) * sizeof(float);
 }
 
 bool enabled() {
@@ -429,8 +506,8 @@ bool enabled() {
 
 // whether the persistent kernels take this problem (else the per-step executor runs)
 bool rb_lstm_persist_supported(int T, int B, int H) {
-  if (!enabled() || T <= 0 || B <= 0 || B > kMaxRows || H % 128 || H / kUnits > 148) return false;
-  return fwd_smem(H) <= 220 * 1024 && bwd_smem(H) <= 220 * 1024;
+  if (!enabled() || T <= 0 || B <= 0 || B > kMaxRows || H % 128 || H / Narrow::U > 148) return false;
+  return fwd_smem<Narrow>(H) <= 220 * 1024 && bwd_smem<Narrow>(H) <= 220 * 1024;
 }
 
 // scratch: hbuf 2*B*H bf16 provided by the caller, contents arbitrary
@@ -446,12 +523,12 @@ int rb_lstm_persist_fwd(const void* z_in, const void* w_rec, const int* lens, co
   a.z_in = (const bf16*)z_in; a.w_rec = (const bf16*)w_rec; a.lens = lens; a.h0 = h0; a.c0 = c0;
   a.T = T; a.B = B; a.H = H; a.reverse = reverse;
   a.y = (bf16*)y; a.c_all = c_all; a.gates = (bf16*)gates; a.hprev_all = (bf16*)hprev_all; a.h_final = h_final; a.c_final = c_final;
-  a.hbuf = (bf16*)hbuf; a.counter = sync_words; a.abort_word = reinterpret_cast<int*>(sync_words + 1); a.status = status;
-  cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), stream);
-  const size_t smem = fwd_smem(H);
+  a.hbuf = (bf16*)hbuf; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+  cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
+  const size_t smem = fwd_smem<Narrow>(H);
   cudaError_t e = cudaFuncSetAttribute(lstm_persist_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   void* args[] = {&a};
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)lstm_persist_fwd_kernel, dim3(H / kUnits), dim3(kThreads), args, smem, stream);
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)lstm_persist_fwd_kernel, dim3(H / Narrow::U), dim3(Narrow::Threads), args, smem, stream);
   if (e != cudaSuccess) {
     rb_set_error("lstm_persist_fwd: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -471,12 +548,12 @@ int rb_lstm_persist_bwd(const void* dy, const float* dh_final, const float* dc_f
   BwdArgs a;
   a.dy = (const bf16*)dy; a.dh_final = dh_final; a.dc_final = dc_final; a.w_rec = (const bf16*)w_rec; a.lens = lens; a.gates = (const bf16*)gates;
   a.c_all = c_all; a.c0 = c0; a.T = T; a.B = B; a.H = H; a.reverse = reverse; a.dz = (bf16*)dz; a.dh0 = dh0; a.dc0 = dc0;
-  a.counter = sync_words; a.abort_word = reinterpret_cast<int*>(sync_words + 1); a.status = status;
-  cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), stream);
-  const size_t smem = bwd_smem(H);
+  a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+  cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
+  const size_t smem = bwd_smem<Narrow>(H);
   cudaError_t e = cudaFuncSetAttribute(lstm_persist_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   void* args[] = {&a};
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)lstm_persist_bwd_kernel, dim3(H / kUnits), dim3(kThreads), args, smem, stream);
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)lstm_persist_bwd_kernel, dim3(H / Narrow::U), dim3(Narrow::Threads), args, smem, stream);
   if (e != cudaSuccess) {
     rb_set_error("lstm_persist_bwd: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -487,35 +564,64 @@ int rb_lstm_persist_bwd(const void* dy, const float* dh_final, const float* dc_f
 
 // ---- both directions of a bidirectional layer in one cooperative launch -------------------------------------------------
 
-// whether the two-direction kernels take this problem: the single-direction conditions, and both grids co-resident (two CTAs
-// per SM: checked through the occupancy of the pair kernels on the current device)
-RB_EXPORT int rb200_blstm_supported(int T, int B, int H) {
-  if (!rb_lstm_persist_supported(T, B, H)) return 0;
-  static int sm_count = 0, occ_fwd[2] = {-1, 0}, occ_bwd[2] = {-1, 0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (!sm_count && cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (occ_fwd[0] != H) {
-    const size_t sf = fwd_smem(H), sb = bwd_smem(H);
-    if (cudaFuncSetAttribute(lstm_persist_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf) != cudaSuccess ||
-        cudaFuncSetAttribute(lstm_persist_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_fwd[1], lstm_persist_fwd_pair_kernel, kThreads, sf) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_bwd[1], lstm_persist_bwd_pair_kernel, kThreads, sb) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    occ_fwd[0] = occ_bwd[0] = H;
-  }
-  const int need = 2 * (H / kUnits);
-  return occ_fwd[1] * sm_count >= need && occ_bwd[1] * sm_count >= need;
+namespace {
+
+// whether both grids of a pair of kernels of this shape are co-resident on the current device; raises their shared-memory limits
+template <typename S>
+bool pair_fits(int H) {
+  static thread_local int last_dev = -1, last_h = 0;
+  static thread_local bool last_ok = false;
+  const size_t sf = fwd_smem<S>(H), sb = bwd_smem<S>(H);
+  constexpr int kLimit = 220 * 1024;
+  int dev = 0, sm_count = 0, of = 0, ob = 0;
+  if (sf > kLimit || sb > kLimit || H % S::U || H / S::U > kMaxCtas || cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev == last_dev && H == last_h) return last_ok;
+  bool ok = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+            cudaFuncSetAttribute(lstm_persist_fwd_pair_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit) == cudaSuccess &&
+            cudaFuncSetAttribute(lstm_persist_bwd_pair_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&of, lstm_persist_fwd_pair_kernel<S>, S::Threads, sf) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, lstm_persist_bwd_pair_kernel<S>, S::Threads, sb) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  ok = ok && of * sm_count >= 2 * (H / S::U) && ob * sm_count >= 2 * (H / S::U);
+  last_dev = dev;
+  last_h = H;
+  last_ok = ok;
+  return ok;
 }
+
+enum { kNoPair = 0, kNarrow = 1, kWide1 = 2, kWide2 = 3 };
+
+// the shape that runs a bidirectional layer
+int pair_shape(int T, int B, int H) {
+  if (!rb_lstm_persist_supported(T, B, H)) return kNoPair;
+  if (B <= 16 && pair_fits<Wide1>(H)) return kWide1;
+  if (B <= 32 && pair_fits<Wide2>(H)) return kWide2;
+  return pair_fits<NarrowPair>(H) ? kNarrow : kNoPair;
+}
+
+template <typename S>
+cudaError_t launch_fwd_pair(FwdPair& pp, int H, cudaStream_t stream) {
+  void* args[] = {&pp};
+  return cudaLaunchCooperativeKernel((const void*)lstm_persist_fwd_pair_kernel<S>, dim3(2 * (H / S::U)), dim3(S::Threads), args, fwd_smem<S>(H), stream);
+}
+template <typename S>
+cudaError_t launch_bwd_pair(BwdPair& pp, int H, cudaStream_t stream) {
+  void* args[] = {&pp};
+  return cudaLaunchCooperativeKernel((const void*)lstm_persist_bwd_pair_kernel<S>, dim3(2 * (H / S::U)), dim3(S::Threads), args, bwd_smem<S>(H), stream);
+}
+
+}  // namespace
+
+// whether the two-direction kernels take this problem: the single-direction conditions, and both grids co-resident
+RB_EXPORT int rb200_blstm_supported(int T, int B, int H) { return pair_shape(T, B, H) != kNoPair ? 1 : 0; }
 
 // ptrs[d * 11 + i] for direction d (0: forward in time, 1: reversed):
 //   0 z_in [T,B,4H] bf16, 1 w_rec [4H,H] bf16, 2 h0, 3 c0 [B,H] fp32, 4 y [T,B,H] bf16, 5 c_all [T,B,H] fp32, 6 gates [T,B,4H] bf16,
 //   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 hbuf (scratch, 2*B*H bf16)
 RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, int H, int* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return RB_OK;
-  if (!rb200_blstm_supported(T, B, H)) {
+  const int shape = pair_shape(T, B, H);
+  if (shape == kNoPair) {
     rb_set_error("blstm_fwd: shape T=%d B=%d H=%d is not supported by the two-direction kernel", T, B, H);
     return RB_ERR_UNSUPPORTED;
   }
@@ -531,12 +637,12 @@ RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, 
     a.z_in = (const bf16*)q[0]; a.w_rec = (const bf16*)q[1]; a.lens = lens; a.h0 = (const float*)q[2]; a.c0 = (const float*)q[3];
     a.T = T; a.B = B; a.H = H; a.reverse = d;
     a.y = (bf16*)q[4]; a.c_all = (float*)q[5]; a.gates = (bf16*)q[6]; a.hprev_all = (bf16*)q[7]; a.h_final = (float*)q[8]; a.c_final = (float*)q[9];
-    a.hbuf = (bf16*)q[10]; a.counter = sync_words; a.abort_word = reinterpret_cast<int*>(sync_words + 1); a.status = status;
-    cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), stream);
+    a.hbuf = (bf16*)q[10]; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+    cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   }
-  const size_t smem = fwd_smem(H);
-  void* args[] = {&pp};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)lstm_persist_fwd_pair_kernel, dim3(2 * (H / kUnits)), dim3(kThreads), args, smem, stream);
+  const cudaError_t e = shape == kWide1   ? launch_fwd_pair<Wide1>(pp, H, stream)
+                        : shape == kWide2 ? launch_fwd_pair<Wide2>(pp, H, stream)
+                                          : launch_fwd_pair<NarrowPair>(pp, H, stream);
   if (e != cudaSuccess) {
     rb_set_error("blstm_fwd: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -549,7 +655,8 @@ RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, 
 //   8 dz [T,B,4H] bf16 (out), 9 dw_rec [4H,H] fp32 (accumulated into; may be null), 10 dh0, 11 dc0 [B,H] fp32 (out)
 RB_EXPORT int rb200_blstm_bwd(void* const* ptrs, const int* lens, int T, int B, int H, int* status, int* n_launch, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return RB_OK;
-  if (!rb200_blstm_supported(T, B, H)) {
+  const int shape = pair_shape(T, B, H);
+  if (shape == kNoPair) {
     rb_set_error("blstm_bwd: shape T=%d B=%d H=%d is not supported by the two-direction kernel", T, B, H);
     return RB_ERR_UNSUPPORTED;
   }
@@ -565,12 +672,12 @@ RB_EXPORT int rb200_blstm_bwd(void* const* ptrs, const int* lens, int T, int B, 
     a.dy = (const bf16*)q[0]; a.dh_final = (const float*)q[1]; a.dc_final = (const float*)q[2]; a.w_rec = (const bf16*)q[3]; a.lens = lens;
     a.gates = (const bf16*)q[4]; a.c_all = (const float*)q[5]; a.c0 = (const float*)q[6]; a.T = T; a.B = B; a.H = H; a.reverse = d;
     a.dz = (bf16*)q[8]; a.dh0 = (float*)q[10]; a.dc0 = (float*)q[11];
-    a.counter = sync_words; a.abort_word = reinterpret_cast<int*>(sync_words + 1); a.status = status;
-    cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), stream);
+    a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+    cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   }
-  const size_t smem = bwd_smem(H);
-  void* args[] = {&pp};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)lstm_persist_bwd_pair_kernel, dim3(2 * (H / kUnits)), dim3(kThreads), args, smem, stream);
+  const cudaError_t e = shape == kWide1   ? launch_bwd_pair<Wide1>(pp, H, stream)
+                        : shape == kWide2 ? launch_bwd_pair<Wide2>(pp, H, stream)
+                                          : launch_bwd_pair<NarrowPair>(pp, H, stream);
   if (e != cudaSuccess) {
     rb_set_error("blstm_bwd: %s", cudaGetErrorString(e));
     cudaGetLastError();

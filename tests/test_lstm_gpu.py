@@ -194,3 +194,29 @@ def test_lstm_input_width_off_the_pitch_rule_and_training_through_the_fallback()
         torch.testing.assert_close(y.float(), yr, atol=0.05, rtol=0.03)
         for g, t in zip(got, (x, w_ff, w_rec, bias)):
             assert float((g.float() - t.grad).abs().max()) / (float(t.grad.abs().max()) + 1e-6) < 0.06
+
+
+@pytest.mark.parametrize("T,B,H", [(1, 1, 128), (7, 16, 256), (6, 17, 128), (9, 32, 384), (5, 33, 128)])
+def test_blstm_batch_sizes_around_the_row_tiles(T, B, H):
+    """16 and 32 rows are the capacities of the two wide forms of the recurrence, 33 takes the narrow one; ragged lengths, initial states"""
+    from returnn_b200.ops import lstm as L, gemm
+
+    torch.manual_seed(B)
+    dev, I = "cuda", 32
+    x = (torch.randn(T, B, I, device=dev) * 0.5).requires_grad_(True)
+    par = [(torch.randn(*s, device=dev) * 0.1).requires_grad_(True) for s in ((4 * H, I), (4 * H, H), (4 * H,)) * 2]
+    st = [(torch.randn(B, H, device=dev) * 0.3).requires_grad_(True) for _ in range(4)]
+    lens = torch.randint(1, T + 1, (B,), dtype=torch.int32)
+    w = [torch.randn(T, B, H, device=dev), torch.randn(T, B, H, device=dev)]
+
+    def loss(fw, bw):
+        return (fw[0].float() * w[0]).sum() + (bw[0].float() * w[1]).sum() + fw[1].sum() + (bw[2] * 0.5).sum()
+
+    got = L.blstm(x, lens, tuple(par[:3]), tuple(par[3:]), *st)
+    g = torch.autograd.grad(loss(*got), [x, *par, *st])
+    gemm.check_status()
+    ref = (L.lstm_reference(x, lens, *par[:3], st[0], st[1], reverse=False), L.lstm_reference(x, lens, *par[3:], st[2], st[3], reverse=True))
+    r = torch.autograd.grad(loss(*ref), [x, *par, *st])
+    for a, b in zip([t for d in got for t in d] + list(g), [t for d in ref for t in d] + list(r)):
+        # bf16 operands, states and gates: 2^-9 per factor, a few of them per step
+        assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-4
