@@ -34,6 +34,9 @@ struct RbGemm {
   long long a_rows = 0, a_cols = 0, b_rows = 0, b_cols = 0;
   const int* lens = nullptr;
   int m_from_lens = 0, n_from_lens = 0, k_from_lens = 0;
+  // split operands (CTA-pair kernel only): A and B are sums hi + lo whose parts lie in ONE stored matrix each, the rows of lo seg_a / seg_b
+  // rows after those of hi (seg_a > 0). The contraction runs over hi*lo, lo*hi and hi*hi into one accumulator. B is stored [k][n].
+  int seg_a = 0, seg_b = 0;
   int* status = nullptr;         // device word: 0 fine, else (role << 24 | detail) of the wait that gave up
 };
 

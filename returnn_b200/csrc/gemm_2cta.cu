@@ -143,9 +143,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           uint8_t* sb = sa + kTileBytesA;
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);  // the leader's barrier collects both CTAs' bytes
           if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
-          const int k0 = kb * BK;
+          // split operands: block kb belongs to hi*lo, lo*hi or hi*hi (columns of A past k read zeros, so the rows of B there do not
+          // count). The small products come first: additions to a large accumulator are what the tensor core rounds
+          const int seg = p.seg_kb ? kb / p.seg_kb : 0;
+          const int k0 = (kb - seg * p.seg_kb) * BK;
+          const int a_row = p.seg_kb && seg == 1 ? g.seg_a : 0, b_row = p.seg_kb && seg == 0 ? g.seg_b : 0;
           if (!g.a_mn_major) {
-            tma_load_2d_pair(sa, &tm_a, k0, m0, bar);
+            tma_load_2d_pair(sa, &tm_a, k0, a_row + m0, bar);
           } else {
 #pragma unroll
             for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * 8192, &tm_a, m0 + 64 * j, k0, bar);
@@ -154,7 +158,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             tma_load_2d_pair(sb, &tm_b, k0, n0, bar);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tm_b, n0 + 64 * j, k0, bar);
+            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tm_b, n0 + 64 * j, b_row + k0, bar);
           }
         }
       }
@@ -290,6 +294,8 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   p.tiles_m = (g.m + BM - 1) / BM;
   p.tiles_n = (g.n + BN - 1) / BN;
   p.num_kb = (g.k + BK - 1) / BK;
+  p.seg_kb = g.seg_a > 0 ? p.num_kb : 0;
+  if (p.seg_kb) p.num_kb *= 3;
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs_max = num_sms() / 2;
   int split = 1;
@@ -328,8 +334,8 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
     }
     if (st) return st;
   }
-  const long long a_rows = g.a_mn_major ? g.k : g.m, a_cols = g.a_mn_major ? g.m : g.k;
-  const long long b_rows = g.b_mn_major ? g.k : g.n, b_cols = g.b_mn_major ? g.n : g.k;
+  const long long a_rows = (g.a_mn_major ? g.k : g.m) + (long long)g.seg_a, a_cols = g.a_mn_major ? g.m : g.k;
+  const long long b_rows = (g.b_mn_major ? g.k : g.n) + (long long)g.seg_b, b_cols = g.b_mn_major ? g.n : g.k;
   st = g.a_mn_major ? make_map(&tm_a, g.a, a_cols, a_rows, g.lda, 64, BK) : make_map(&tm_a, g.a, a_cols, a_rows, g.lda, BK, 128);
   if (st) return st;
   st = g.b_mn_major ? make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, 64, BK) : make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, BK, BN / 2);

@@ -307,6 +307,10 @@ int rb_gemm(const RbGemm& g, cudaStream_t stream) {
     rb_set_error("gemm: split_k needs accumulate == 2");
     return RB_ERR_ARG;
   }
+  if (g.seg_a > 0 && (!rb_gemm_pair_wanted(g) || g.a_mn_major || !g.b_mn_major || g.accumulate == 2)) {
+    rb_set_error("gemm: split operands need the CTA-pair kernel, A stored [m][k] and B stored [k][n]");
+    return RB_ERR_UNSUPPORTED;
+  }
   if (rb_gemm_pair_wanted(g)) return rb_gemm_pair(g, stream);
   if (g.n > 128) return launch<256>(g, stream);
   return launch<128>(g, stream);
@@ -343,4 +347,19 @@ RB_EXPORT int rb200_gemm_fp16_ex(const void* a, const void* b, void* c, void* c2
                                  cudaStream_t stream) {
   return gemm_ex(a, b, c, c2, bias, m, n, k, lda, ldb, ldc, a_mn_major, b_mn_major, bias_bf16, act, out_fp32, accumulate, alpha, dact_z, drop_p, seed,
                  offset, drop_site, resid, res_scale, split_k, status, 1, stream);
+}
+
+// c[m,n] (fp32) = A·B with fp16 operands split in two: A = hi + lo, hi stored [m][k] at `a` and lo a_lo_rows rows further on, B likewise
+// stored [k][n]; the product of the two lo parts (2^-22 of the result) is left out. RB_ERR_UNSUPPORTED: not a shape of the CTA-pair kernel.
+RB_EXPORT int rb200_gemm_fp16_split(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc, int a_lo_rows, int b_lo_rows,
+                                    int* status, cudaStream_t stream) {
+  RbGemm g;
+  g.a = a; g.b = b; g.c = c; g.m = m; g.n = n; g.k = k; g.lda = lda; g.ldb = ldb; g.ldc = ldc;
+  g.b_mn_major = 1; g.ab_fp16 = 1; g.out_fp32 = 1; g.status = status;
+  g.seg_a = a_lo_rows; g.seg_b = b_lo_rows;
+  if (a_lo_rows < m || b_lo_rows < k) {
+    rb_set_error("gemm_fp16_split: the lo rows overlap the hi rows");
+    return RB_ERR_ARG;
+  }
+  return rb_gemm(g, stream);
 }

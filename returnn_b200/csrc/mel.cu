@@ -76,65 +76,91 @@ log_mel_kernel(const float* __restrict__ audio, const int* __restrict__ lens, lo
 // The tensor-core form: the DFT of all frames is ONE matrix product, frames [rows * slots, window] x table [window, n_fft], on the
 // tcgen05 GEMM. The frames are never materialised: the A operand is a strided view of the audio (row pitch = step samples, so
 // consecutive rows overlap by window - step samples), which a TMA tensor map expresses directly. fp32 audio and table are split into
-// fp16 high and low parts and three products (hi*hi + hi*lo + lo*hi) accumulate in fp32, which keeps 22 mantissa bits per factor
+// fp16 high and low parts and three products (hi*lo + lo*hi + hi*hi) accumulate in fp32, which keeps 22 mantissa bits per factor
 // (bf16 parts would keep 16: an error floor 96 dB under a frame's strongest component, audible in the weakest mel bands).
 // Audio is expected within fp16's range (|x| < 65504; samples scaled to [-1, 1] or raw 16-bit PCM values both are).
 // The two kernels here are the ends of that pipeline: the split of the audio, and power spectrum -> mel -> log.
 
 // audio [rows, T] fp32 -> hi, lo [rows * Tp + tail] fp16 with audio[r][c] at r * Tp + c, zeros elsewhere (Tp = slots * step)
+// Eight samples per thread: two 16-byte loads where the row's start allows them, two 16-byte stores (Tp is a multiple of 8, so a group
+// lies in one row). Bound by memory, 8 bytes per sample.
 __global__ void __launch_bounds__(256)
 split_hi_lo_kernel(const float* __restrict__ audio, int rows, long long T, long long Tp, long long total, __half* __restrict__ hi,
                    __half* __restrict__ lo) {
+  const long long groups = total / 8, per_row = Tp / 8;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const long long r = i / Tp, c = i - r * Tp;
-    float x = 0.f;
-    if (r < rows && c < T) x = audio[r * T + c];
-    const __half h = __float2half_rn(x);
-    hi[i] = h;
-    lo[i] = __float2half_rn(x - __half2float(h));
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += stride) {
+    const long long r = i / per_row, c = (i - r * per_row) * 8;
+    const float* src = audio + r * T + c;
+    float x[8];
+    if (r < rows && c + 8 <= T && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+      const float4 u = reinterpret_cast<const float4*>(src)[0], v = reinterpret_cast<const float4*>(src)[1];
+      x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+      x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = r < rows && c + e < T ? src[e] : 0.f;
+    }
+    __align__(16) __half h[8], l[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      h[e] = __float2half_rn(x[e]);
+      l[e] = __float2half_rn(x[e] - __half2float(h[e]));
+    }
+    *reinterpret_cast<uint4*>(hi + 8 * i) = *reinterpret_cast<const uint4*>(h);
+    *reinterpret_cast<uint4*>(lo + 8 * i) = *reinterpret_cast<const uint4*>(l);
   }
 }
 
 // spec [rows * slots, ld] fp32: column 2j = Re X_j, 2j + 1 = Im X_j for 0 < j < n_fft / 2; column 0 = X_0 and column 1 = X_{n_fft/2}
 // (both real). One warp per frame: power spectrum into shared memory, then every lane sums the bins of its mel filters, which are
-// contiguous ranges [fb_start[m], fb_start[m] + fb_len[m]) of the filterbank matrix fbank [n_bins, n_mel].
+// contiguous ranges [fb_start[m], fb_start[m] + fb_len[m]). The filter weights come as a table [max_len, n_mel], entry i of filter m at
+// [i][m], held in shared memory for the kMelFrames frames of every warp: read from the filterbank matrix, where the lanes' filters lie in
+// different rows, each load took 32 cache accesses, which was the time of the kernel.
 constexpr int kMelWarps = 8;
+constexpr int kMelFrames = 4;
 
 __global__ void __launch_bounds__(kMelWarps * 32)
 mel_from_spectrum_kernel(const float* __restrict__ spec, int ld, int slots, int n_frames_max, const int* __restrict__ lens, long long T, int window,
-                         int step, int n_fft, const float* __restrict__ fbank, const int* __restrict__ fb_start, const int* __restrict__ fb_len,
-                         int n_mel, float log_scale, float eps, float* __restrict__ out) {
-  extern __shared__ float spow[];  // [kMelWarps][n_bins]
+                         int step, int n_fft, const float* __restrict__ weights, int max_len, const int* __restrict__ fb_start,
+                         const int* __restrict__ fb_len, int n_mel, float log_scale, float eps, float* __restrict__ out) {
+  extern __shared__ float shm[];  // [kMelWarps][n_bins], then [max_len][n_mel]
   const int n_bins = n_fft / 2 + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* ws = shm + kMelWarps * n_bins;
+  for (int i = threadIdx.x; i < max_len * n_mel; i += kMelWarps * 32) ws[i] = weights[i];
+  __syncthreads();
   const int row = blockIdx.y;
-  const int fr = blockIdx.x * kMelWarps + warp;
-  if (fr >= n_frames_max) return;
   const long long len = lens ? (long long)lens[row] : T;
   const int n_frames = len >= window ? (int)((len - window) / step + 1) : 0;
-  float* o = out + ((size_t)row * n_frames_max + fr) * n_mel;
-  if (fr >= n_frames) {
-    for (int m = lane; m < n_mel; m += 32) o[m] = 0.f;
-    return;
-  }
-  const float2* sp = reinterpret_cast<const float2*>(spec + ((size_t)row * slots + fr) * ld);
-  float* pw = spow + warp * n_bins;
-  for (int j = lane; j < n_fft / 2; j += 32) {
-    const float2 v = sp[j];
-    if (j == 0) {
-      pw[0] = v.x * v.x;
-      pw[n_fft / 2] = v.y * v.y;
-    } else {
-      pw[j] = v.x * v.x + v.y * v.y;
+  float* pw = shm + warp * n_bins;
+  for (int f = 0; f < kMelFrames; ++f) {
+    const int fr = (blockIdx.x * kMelFrames + f) * kMelWarps + warp;
+    if (fr >= n_frames_max) return;
+    float* o = out + ((size_t)row * n_frames_max + fr) * n_mel;
+    if (fr >= n_frames) {
+      for (int m = lane; m < n_mel; m += 32) o[m] = 0.f;
+      continue;
     }
-  }
-  __syncwarp();
-  for (int m = lane; m < n_mel; m += 32) {
-    const int k0 = fb_start[m], n = fb_len[m];
-    float acc = 0.f;
-    for (int k = k0; k < k0 + n; ++k) acc += pw[k] * fbank[(size_t)k * n_mel + m];
-    o[m] = __logf(fmaxf(acc, eps)) * log_scale;
+    const float2* sp = reinterpret_cast<const float2*>(spec + ((size_t)row * slots + fr) * ld);
+    __syncwarp();  // all lanes have read the previous frame's power
+#pragma unroll 8
+    for (int j = lane; j < n_fft / 2; j += 32) {
+      const float2 v = sp[j];
+      if (j == 0) {
+        pw[0] = v.x * v.x;
+        pw[n_fft / 2] = v.y * v.y;
+      } else {
+        pw[j] = v.x * v.x + v.y * v.y;
+      }
+    }
+    __syncwarp();
+    for (int m = lane; m < n_mel; m += 32) {
+      const int k0 = fb_start[m], n = fb_len[m];
+      float acc = 0.f;
+      for (int k = 0; k < n; ++k) acc += pw[k0 + k] * ws[k * n_mel + m];
+      o[m] = __logf(fmaxf(acc, eps)) * log_scale;
+    }
   }
 }
 
@@ -142,27 +168,36 @@ mel_from_spectrum_kernel(const float* __restrict__ spec, int ld, int slots, int 
 
 RB_EXPORT int rb200_split_hi_lo_fp16(const float* audio, int rows, long long T, long long Tp, long long total, void* hi, void* lo, cudaStream_t stream) {
   if (total <= 0) return RB_OK;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+  if (Tp % 8 || total % 8 || ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15)) {
+    rb_set_error("split_hi_lo: Tp=%lld and total=%lld must be multiples of 8, the outputs 16-byte aligned", Tp, total);
+    return RB_ERR_ARG;
+  }
+  const int blocks = (int)std::min<long long>((total / 8 + 255) / 256, 148LL * 8);
   split_hi_lo_kernel<<<blocks, 256, 0, stream>>>(audio, rows, T, Tp, total, reinterpret_cast<__half*>(hi), reinterpret_cast<__half*>(lo));
   return rb_check_launch("split_hi_lo");
 }
 
 RB_EXPORT int rb200_mel_from_spectrum(const float* spec, int ld, int rows, int slots, int n_frames_max, const int* lens, long long T, int window, int step,
-                                      int n_fft, const float* fbank, const int* fb_start, const int* fb_len, int n_mel, float log_scale, float eps,
-                                      float* out, cudaStream_t stream) {
+                                      int n_fft, const float* weights, int max_len, const int* fb_start, const int* fb_len, int n_mel, float log_scale,
+                                      float eps, float* out, cudaStream_t stream) {
   if (rows <= 0 || n_frames_max <= 0) return RB_OK;
   if ((ld % 2) || n_fft < 2 || (reinterpret_cast<uintptr_t>(spec) & 7)) {
     rb_set_error("mel_from_spectrum: ld=%d must be even and the spectrum 8-byte aligned", ld);
     return RB_ERR_ARG;
   }
-  const size_t smem = (size_t)kMelWarps * (n_fft / 2 + 1) * sizeof(float);
-  if (smem > 48 * 1024) {
-    rb_set_error("mel_from_spectrum: n_fft=%d too large", n_fft);
+  const size_t smem = ((size_t)kMelWarps * (n_fft / 2 + 1) + (size_t)max_len * n_mel) * sizeof(float);
+  if ((size_t)kMelWarps * (n_fft / 2 + 1) * sizeof(float) > 48 * 1024 || smem > 220 * 1024) {
+    rb_set_error("mel_from_spectrum: n_fft=%d or the longest filter (%d bins, %d filters) too large", n_fft, max_len, n_mel);
     return RB_ERR_UNSUPPORTED;
   }
-  dim3 grid((n_frames_max + kMelWarps - 1) / kMelWarps, rows);
-  mel_from_spectrum_kernel<<<grid, kMelWarps * 32, smem, stream>>>(spec, ld, slots, n_frames_max, lens, T, window, step, n_fft, fbank, fb_start, fb_len,
-                                                                 n_mel, log_scale, eps, out);
+  const cudaError_t e = cudaFuncSetAttribute(mel_from_spectrum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  if (e != cudaSuccess) {
+    rb_set_error("mel_from_spectrum: %s", cudaGetErrorString(e));
+    return RB_ERR_LAUNCH;
+  }
+  dim3 grid((n_frames_max + kMelWarps * kMelFrames - 1) / (kMelWarps * kMelFrames), rows);
+  mel_from_spectrum_kernel<<<grid, kMelWarps * 32, smem, stream>>>(spec, ld, slots, n_frames_max, lens, T, window, step, n_fft, weights, max_len, fb_start,
+                                                                 fb_len, n_mel, log_scale, eps, out);
   return rb_check_launch("mel_from_spectrum");
 }
 

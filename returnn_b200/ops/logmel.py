@@ -14,11 +14,13 @@ from __future__ import annotations
 from typing import Optional
 import ctypes
 import math
+import os
 import torch
 from . import _lib
 
 _vp, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 _cache = {}
+_PAIR_KERNEL_OFF = os.environ.get("RETURNN_B200_GEMM_2CTA", "")[:1] == "0"
 
 
 def available() -> bool:
@@ -45,7 +47,7 @@ def _tables(device, sampling_rate, window, n_fft, n_mel, f_min, f_max):
 
 def _dft_tables(device, window: int, n_fft: int, win: torch.Tensor, fb: torch.Tensor):
     """
-    (table_hi, table_lo) fp16 [window, n_fft]: column 2j = win * cos(2 pi j n / n_fft), 2j + 1 = -win * sin(..) for 0 < j < n_fft/2,
+    (table_hi, table_lo) fp16 [window, n_fft], one behind the other in memory: column 2j = win * cos(2 pi j n / n_fft), 2j + 1 = -win * sin(..) for 0 < j < n_fft/2,
     column 0 = win (X_0) and column 1 = win * (-1)^n (X_{n_fft/2}); and the non-zero bin range of every mel filter.
     """
     key = ("dft", str(device), window, n_fft, win.data_ptr(), fb.data_ptr())
@@ -69,13 +71,24 @@ def _dft_tables(device, window: int, n_fft: int, win: torch.Tensor, fb: torch.Te
         end = torch.where(nz, idx + 1, torch.zeros_like(idx)).max(dim=0).values
         length = torch.clamp(end - start, min=0)
         start = torch.where(length > 0, start, torch.zeros_like(start))
-        t = (hi.to(device).contiguous(), lo.to(device).contiguous(), start.to(device, torch.int32).contiguous(), length.to(device, torch.int32).contiguous())
+        both = torch.stack([hi, lo]).to(device)
+        t = (both[0], both[1], start.to(device, torch.int32).contiguous(), length.to(device, torch.int32).contiguous())
         _cache[key] = t
     return t
 
 
+def _mel_weights(fb: torch.Tensor, start: torch.Tensor, length: torch.Tensor) -> torch.Tensor:
+    """the non-zero part of every mel filter, [longest filter, n_mel] fp32: entry i of filter m is ``fb[start[m] + i, m]``"""
+    key = ("weights", str(fb.device), fb.data_ptr())
+    t = _cache.get(key)
+    if t is None:
+        i = torch.arange(max(int(length.max()), 1), device=fb.device)[:, None]
+        idx = torch.clamp(start.long()[None] + i, max=fb.shape[0] - 1)
+        t = _cache[key] = (torch.gather(fb, 0, idx) * (i < length[None])).contiguous()
+    return t
+
+
 def _gemm_form_wanted(flat: torch.Tensor, window: int, step: int, n_fft: int) -> bool:
-    import os
     from . import gemm as G
 
     mode = os.environ.get("RETURNN_B200_LOGMEL", "auto")
@@ -95,22 +108,30 @@ def _log_mel_gemm(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, f
     dev = flat.device
     slots = -(-T // step)
     Tp = slots * step
-    total = rows * Tp + ((window + 7) // 8) * 8  # the last slots read up to `window` samples past the last row
-    hi = torch.empty(total, dtype=torch.float16, device=dev)
-    lo = torch.empty(total, dtype=torch.float16, device=dev)
+    total = -(-(rows * Tp + window) // step) * step  # the last slots read up to `window` samples past the last row
+    parts = torch.empty(2, total, dtype=torch.float16, device=dev)  # the high and the low part, a whole number of slots apart
+    hi, lo = parts[0], parts[1]
     fn = _lib.bind("rb200_split_hi_lo_fp16", [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp])
     _lib.check(fn(flat.data_ptr(), rows, T, Tp, total, hi.data_ptr(), lo.data_ptr(), _lib.stream_ptr()), "split_hi_lo")
     t_hi, t_lo, fb_start, fb_len = _dft_tables(dev, window, n_fft, win, fb)
+    weights = _mel_weights(fb, fb_start, fb_len)
     m = rows * slots
-    a_hi = torch.as_strided(hi, (m, window), (step, 1))
-    a_lo = torch.as_strided(lo, (m, window), (step, 1))
     spec = torch.empty(m, n_fft, dtype=torch.float32, device=dev)
-    G.gemm(a_hi, t_hi, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec)
-    G.gemm(a_hi, t_lo, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec, accumulate=True)
-    G.gemm(a_lo, t_hi, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec, accumulate=True)
-    fn = _lib.bind("rb200_mel_from_spectrum", [_vp, _i32, _i32, _i32, _i32, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _f32, _f32, _vp, _vp])
-    _lib.check(fn(spec.data_ptr(), n_fft, rows, slots, n_frames, l32.data_ptr() if l32 is not None else None, T, window, step, n_fft, fb.data_ptr(),
-                  fb_start.data_ptr(), fb_len.data_ptr(), n_mel, scale, 1e-10, out.data_ptr(), _lib.stream_ptr()), "mel_from_spectrum")
+    if m > 128 and n_fft > 128 and m + total // step < 2 ** 31 and not _PAIR_KERNEL_OFF:
+        # hi*lo + lo*hi + hi*hi summed in one accumulator: the spectrum is written once
+        fn = _lib.bind("rb200_gemm_fp16_split", [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp])
+        _lib.check(fn(parts.data_ptr(), t_hi.data_ptr(), spec.data_ptr(), m, n_fft, window, step, n_fft, n_fft, total // step, window,
+                      G.status_tensor(dev).data_ptr(), _lib.stream_ptr()), "gemm_fp16_split")
+        _lib.count_launch()
+    else:
+        a_hi = torch.as_strided(hi, (m, window), (step, 1))
+        a_lo = torch.as_strided(lo, (m, window), (step, 1))
+        G.gemm(a_hi, t_hi, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec)
+        G.gemm(a_hi, t_lo, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec, accumulate=True)
+        G.gemm(a_lo, t_hi, m=m, n=n_fft, k=window, a_mn_major=False, b_mn_major=True, out=spec, accumulate=True)
+    fn = _lib.bind("rb200_mel_from_spectrum", [_vp, _i32, _i32, _i32, _i32, _vp, _i64, _i32, _i32, _i32, _vp, _i32, _vp, _vp, _i32, _f32, _f32, _vp, _vp])
+    _lib.check(fn(spec.data_ptr(), n_fft, rows, slots, n_frames, l32.data_ptr() if l32 is not None else None, T, window, step, n_fft,
+                  weights.data_ptr(), weights.shape[0], fb_start.data_ptr(), fb_len.data_ptr(), n_mel, scale, 1e-10, out.data_ptr(), _lib.stream_ptr()), "mel_from_spectrum")
     _lib.count_launch(2)
 
 

@@ -188,3 +188,28 @@ def test_linear_backward_before_the_products(m, n, act):
     for g, r in zip(got, want):
         # z and dz are rounded to bf16 (2^-9 each), and dx again
         assert (g.double() - r).norm() <= 8e-3 * r.norm() + 1e-6
+
+
+@gpu
+@pytest.mark.parametrize("m,n,k", [(129, 136, 64), (700, 512, 400), (300, 256, 72)])
+def test_split_operand_product_keeps_fp32_precision(m, n, k):
+    """(hi + lo)(hi + lo) without lo * lo in one accumulator; A as an overlapping strided view, as the feature extraction passes it"""
+    import ctypes
+    from returnn_b200.ops import _lib, gemm as G
+
+    torch.manual_seed(m)
+    step = 40
+    rows = -(-(m * step + k) // step)
+    x = torch.randn(rows * step, device="cuda")
+    t = torch.randn(k, n, device="cuda")
+    parts = torch.stack([x.half(), (x - x.half().float()).half()])
+    table = torch.stack([t.half(), (t - t.half().float()).half()])
+    out = torch.empty(m, n, device="cuda")
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    fn = _lib.bind("rb200_gemm_fp16_split", [vp, vp, vp] + [i32] * 8 + [vp, vp])
+    _lib.check(fn(parts.data_ptr(), table.data_ptr(), out.data_ptr(), m, n, k, step, n, n, rows, k, G.status_tensor(x.device).data_ptr(),
+                  _lib.stream_ptr()), "gemm_fp16_split")
+    G.check_status()
+    want = torch.as_strided(x, (m, k), (step, 1)).double() @ t.double()
+    # 22 mantissa bits per factor, fp32 sums over k
+    assert (out.double() - want).norm() <= 4e-6 * want.norm()
