@@ -89,6 +89,48 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+template <typename S, int NOUT>
+__device__ __forceinline__ void store_partials(float (&acc)[S::MT][NOUT / 8][4], int m_tiles, float* __restrict__ red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  // The partial sums of the warps meet in shared memory without atomics (warps adding 48 values per lane onto the
+  // same words was the largest batch-dependent part of a forward step): the upper half of the warps store theirs into slot warp - W/2, the
+  // lower half add their own onto that slot, the caller sums the W/2 slots (red_sum). Row pitch NOUT + 8 floats: the 8-byte accesses
+  // of a half warp fall on distinct banks.
+  constexpr int RP = NOUT + kRedPad;
+  float* slot = red + (warp & (S::Slots - 1)) * (S::Rows * RP);
+  if (warp >= S::Slots) {
+#pragma unroll
+    for (int m = 0; m < S::MT; ++m) {
+      if (m >= m_tiles) continue;
+      const int r0 = m * 16 + g, r1 = r0 + 8;
+#pragma unroll
+      for (int n = 0; n < NOUT / 8; ++n) {
+        const int c = n * 8 + 2 * t;
+        *reinterpret_cast<float2*>(&slot[r0 * RP + c]) = make_float2(acc[m][n][0], acc[m][n][1]);
+        *reinterpret_cast<float2*>(&slot[r1 * RP + c]) = make_float2(acc[m][n][2], acc[m][n][3]);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < S::Slots) {
+#pragma unroll
+    for (int m = 0; m < S::MT; ++m) {
+      if (m >= m_tiles) continue;
+      const int r0 = m * 16 + g, r1 = r0 + 8;
+#pragma unroll
+      for (int n = 0; n < NOUT / 8; ++n) {
+        const int c = n * 8 + 2 * t;
+        float2* q0 = reinterpret_cast<float2*>(&slot[r0 * RP + c]);
+        float2* q1 = reinterpret_cast<float2*>(&slot[r1 * RP + c]);
+        const float2 v0 = *q0, v1 = *q1;
+        *q0 = make_float2(v0.x + acc[m][n][0], v0.y + acc[m][n][1]);
+        *q1 = make_float2(v1.x + acc[m][n][2], v1.y + acc[m][n][3]);
+      }
+    }
+  }
+}
+
 // red[row][n] += sum_k A[row][k] * Bs[n][k] for rows < n_rows; A in global (written by other CTAs: read through L2), Bs resident
 // in shared memory with row pitch K + kPad. The contraction is cut into blocks of 32 k; the warp w of S::W takes the blocks
 // [w*nblk/W, (w+1)*nblk/W).
@@ -146,42 +188,7 @@ __device__ __forceinline__ void step_matmul(const bf16* __restrict__ A, int n_ro
       }
     }
   }
-  // The partial sums of the warps meet in shared memory without atomics (warps adding 48 values per lane onto the
-  // same words was the largest batch-dependent part of a forward step): the upper half of the warps store theirs into slot warp - W/2, the
-  // lower half add their own onto that slot, the caller sums the W/2 slots (red_sum). Row pitch NOUT + 8 floats: the 8-byte accesses
-  // of a half warp fall on distinct banks.
-  constexpr int RP = NOUT + kRedPad;
-  float* slot = red + (warp & (S::Slots - 1)) * (S::Rows * RP);
-  if (warp >= S::Slots) {
-#pragma unroll
-    for (int m = 0; m < S::MT; ++m) {
-      if (m >= m_tiles) continue;
-      const int r0 = m * 16 + g, r1 = r0 + 8;
-#pragma unroll
-      for (int n = 0; n < NOUT / 8; ++n) {
-        const int c = n * 8 + 2 * t;
-        *reinterpret_cast<float2*>(&slot[r0 * RP + c]) = make_float2(acc[m][n][0], acc[m][n][1]);
-        *reinterpret_cast<float2*>(&slot[r1 * RP + c]) = make_float2(acc[m][n][2], acc[m][n][3]);
-      }
-    }
-  }
-  __syncthreads();
-  if (warp < S::Slots) {
-#pragma unroll
-    for (int m = 0; m < S::MT; ++m) {
-      if (m >= m_tiles) continue;
-      const int r0 = m * 16 + g, r1 = r0 + 8;
-#pragma unroll
-      for (int n = 0; n < NOUT / 8; ++n) {
-        const int c = n * 8 + 2 * t;
-        float2* q0 = reinterpret_cast<float2*>(&slot[r0 * RP + c]);
-        float2* q1 = reinterpret_cast<float2*>(&slot[r1 * RP + c]);
-        const float2 v0 = *q0, v1 = *q1;
-        *q0 = make_float2(v0.x + acc[m][n][0], v0.y + acc[m][n][1]);
-        *q1 = make_float2(v1.x + acc[m][n][2], v1.y + acc[m][n][3]);
-      }
-    }
-  }
+  store_partials<S, NOUT>(acc, m_tiles, red);
 }
 
 // sum over the slots that step_matmul leaves (after a __syncthreads)
@@ -211,10 +218,169 @@ struct FwdArgs {
   bf16* hprev_all;      // [T,B,H]
   float *h_final, *c_final;
   bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state
+  uint32_t* hx;         // wide form: [2,B,H] words (step << 16 | bf16 h), zeroed before the launch
   uint32_t* flags;      // one word per CTA, zeroed before the launch
   int* abort_word;      // zeroed before the launch
   int* status;          // receives (5 << 24) | cta when a barrier wait ran out
 };
+
+// The forward exchange without barrier, wide form: a word of the exchanged matrix carries the number of the step that wrote it next to the
+// value, so a warp that needs a word loads it until the number is the right one. One trip through L2 per step (store, load) takes the place of
+// store, fence, flag, poll and load, and a warp waits only for the CTAs whose units it multiplies. A word of step s - 1 may be overwritten in
+// step s + 1: whoever writes there has seen all of step s, which everybody wrote after reading step s - 1.
+// Whether all words of the warp's blocks [b_begin, b_end) arrived; a[..] then holds them as bf16 pairs.
+template <typename S, int kBlocks>
+__device__ __forceinline__ bool fetch_tagged(const uint32_t* __restrict__ X, int n_rows, int K, int b_begin, int b_end, uint32_t tag,
+                                             uint4 (&a)[kBlocks][S::MT][2], int* abort_word, int* status) {
+  const int lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  uint32_t spins = 0;
+  while (true) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {
+#pragma unroll
+      for (int m = 0; m < S::MT; ++m) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int r = m * 16 + q * 8 + g;
+          a[i][m][q] = make_uint4(0u, 0u, 0u, 0u);
+          if (b_begin + i < b_end && r < n_rows) {
+            const uint32_t* src = X + (size_t)r * K + ((b_begin + i) << 5) + 8 * t;
+            uint32_t w[8];
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(src) : "memory");
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src + 4) : "memory");
+            uint32_t bad = 0u;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) bad |= (w[e] >> 16) ^ tag;
+            ok = ok && bad == 0u;
+            a[i][m][q] = make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410), __byte_perm(w[4], w[5], 0x5410),
+                                    __byte_perm(w[6], w[7], 0x5410));
+          }
+        }
+      }
+    }
+    if (__all_sync(0xffffffffu, ok)) return true;
+    ++spins;
+    if (spins > kSpinLimit || ((spins & 255u) == 0 && *reinterpret_cast<volatile int*>(abort_word))) {
+      if (lane == 0) {
+        atomicExch(abort_word, 1);
+        if (status) atomicCAS(status, 0, (5 << 24) | (int)(blockIdx.x & 0xFFFF));
+      }
+      return false;
+    }
+  }
+}
+
+template <typename S>
+__device__ __forceinline__ void fwd_body_tagged(const FwdArgs& p, const int cta) {
+  constexpr int U = S::U, kThreads = S::Threads, NOUT = 4 * U, PF = S::PrefetchFwd;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int H = p.H, B = p.B;
+  const int pitch = H + kPad;
+  bf16* Ws = reinterpret_cast<bf16*>(smem_raw);                      // [4*U][H+kPad]: row q*U+u = W_rec[q*H + j0 + u]
+  float* red = reinterpret_cast<float*>(Ws + (size_t)NOUT * pitch);  // [slots][rows][4*U + kRedPad]
+  const int j0 = cta * U;
+  for (int idx = threadIdx.x; idx < NOUT * (H / 8); idx += kThreads) {
+    const int r = idx / (H / 8), v = idx % (H / 8);
+    const int q = r / U, u = r % U;
+    *reinterpret_cast<uint4*>(Ws + (size_t)r * pitch + v * 8) = *reinterpret_cast<const uint4*>(p.w_rec + ((size_t)q * H + j0 + u) * H + v * 8);
+  }
+  static_assert(S::PerThread == 1, "one (row, unit) pair per thread");
+  const int b = threadIdx.x / U, u = threadIdx.x % U;
+  const bool own = b < B;
+  float cst = 0.f, hst = 0.f;
+  bf16 zin[4];
+  const int len = own && p.lens ? p.lens[b] : p.T;
+  auto publish = [&](int parity, uint32_t tag, float h) {
+    const uint32_t w = (tag << 16) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16(h));
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p.hx + ((size_t)parity * B + b) * H + j0 + u), "r"(w) : "memory");
+  };
+  auto fetch_zin = [&](int t) {
+    if (!own) return;
+    const bf16* z = p.z_in + ((size_t)t * B + b) * 4 * H + j0 + u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) zin[q] = z[(size_t)q * H];
+  };
+  if (own) {
+    hst = __bfloat162float(__float2bfloat16(p.h0[(size_t)b * H + j0 + u]));
+    cst = p.c0[(size_t)b * H + j0 + u];
+    publish(0, 1u, hst);
+  }
+  if (p.T > 0) fetch_zin(p.reverse ? p.T - 1 : 0);
+  __syncthreads();  // the resident slice is in place
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int m_tiles = (B + 15) / 16;
+  const int nblk = H >> 5;
+  const int b_begin = warp * nblk / S::W, b_end = (warp + 1) * nblk / S::W;
+  for (int s = 0; s < p.T; ++s) {
+    const int t = p.reverse ? p.T - 1 - s : s;
+    const uint32_t tag = (uint32_t)(s + 1) & 0xffffu;
+    const uint32_t* X = p.hx + (size_t)(s & 1) * B * H;
+    float acc[S::MT][NOUT / 8][4];
+#pragma unroll
+    for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NOUT / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+    bool ok = true;
+    for (int bc = b_begin; bc < b_end && ok; bc += PF) {
+      uint4 a[PF][S::MT][2];
+      ok = fetch_tagged<S, PF>(X, B, H, bc, b_end, tag, a, p.abort_word, p.status);
+#pragma unroll
+      for (int i = 0; i < PF; ++i) {
+        if (bc + i >= b_end) break;
+        const int k0 = (bc + i) << 5;
+#pragma unroll
+        for (int n = 0; n < NOUT / 8; ++n) {
+          const uint4 w = *reinterpret_cast<const uint4*>(Ws + (size_t)(n * 8 + g) * pitch + k0 + 8 * t4);
+#pragma unroll
+          for (int m = 0; m < S::MT; ++m) {
+            if (m >= m_tiles) continue;
+            const uint32_t f0[4] = {a[i][m][0].x, a[i][m][1].x, a[i][m][0].y, a[i][m][1].y};
+            mma16816(acc[m][n], f0, w.x, w.y);
+            const uint32_t f1[4] = {a[i][m][0].z, a[i][m][1].z, a[i][m][0].w, a[i][m][1].w};
+            mma16816(acc[m][n], f1, w.z, w.w);
+          }
+        }
+      }
+    }
+    store_partials<S, NOUT>(acc, m_tiles, red);
+    if (!__syncthreads_and(ok ? 1 : 0)) break;
+    float gi = 0.f, gf = 0.f, gg = 0.f, go = 0.f;
+    const float hp = hst;
+    if (own) {
+      if (t < len) {
+        gi = sigm(red_sum<S, NOUT>(red, b, u) + __bfloat162float(zin[0]));
+        gf = sigm(red_sum<S, NOUT>(red, b, U + u) + __bfloat162float(zin[1]));
+        gg = tanhf(red_sum<S, NOUT>(red, b, 2 * U + u) + __bfloat162float(zin[2]));
+        go = sigm(red_sum<S, NOUT>(red, b, 3 * U + u) + __bfloat162float(zin[3]));
+        cst = gf * cst + gi * gg;
+        hst = __bfloat162float(__float2bfloat16(go * tanhf(cst)));
+      }
+      publish((s + 1) & 1, (uint32_t)(s + 2) & 0xffffu, hst);
+    }
+    if (s + 1 < p.T) fetch_zin(p.reverse ? p.T - 2 - s : s + 1);
+    if (own) {
+      const size_t o = ((size_t)t * B + b) * H + j0 + u;
+      const size_t zo = ((size_t)t * B + b) * 4 * H + j0 + u;
+      p.hprev_all[o] = __float2bfloat16(hp);
+      p.y[o] = __float2bfloat16(t < len ? hst : 0.f);
+      p.c_all[o] = cst;
+      p.gates[zo] = __float2bfloat16(gi);
+      p.gates[zo + H] = __float2bfloat16(gf);
+      p.gates[zo + 2 * (size_t)H] = __float2bfloat16(gg);
+      p.gates[zo + 3 * (size_t)H] = __float2bfloat16(go);
+    }
+    __syncthreads();  // the partial sums have been read
+  }
+  if (own) {
+    p.h_final[(size_t)b * H + j0 + u] = hst;
+    p.c_final[(size_t)b * H + j0 + u] = cst;
+  }
+}
 
 template <typename S>
 __device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const int n_cta) {
@@ -333,8 +499,13 @@ struct FwdPair {
 template <typename S>
 __global__ void __launch_bounds__(S::Threads, S::U == 8 ? 2 : 1) lstm_persist_fwd_pair_kernel(const __grid_constant__ FwdPair pp) {
   const int half = gridDim.x / 2;
-  if ((int)blockIdx.x < half) fwd_body<S>(pp.d[0], blockIdx.x, half);
-  else fwd_body<S>(pp.d[1], blockIdx.x - half, half);
+  if constexpr (S::U == 16) {
+    if ((int)blockIdx.x < half) fwd_body_tagged<S>(pp.d[0], blockIdx.x);
+    else fwd_body_tagged<S>(pp.d[1], blockIdx.x - half);
+  } else {
+    if ((int)blockIdx.x < half) fwd_body<S>(pp.d[0], blockIdx.x, half);
+    else fwd_body<S>(pp.d[1], blockIdx.x - half, half);
+  }
 }
 
 struct BwdArgs {
@@ -523,7 +694,7 @@ int rb_lstm_persist_fwd(const void* z_in, const void* w_rec, const int* lens, co
   a.z_in = (const bf16*)z_in; a.w_rec = (const bf16*)w_rec; a.lens = lens; a.h0 = h0; a.c0 = c0;
   a.T = T; a.B = B; a.H = H; a.reverse = reverse;
   a.y = (bf16*)y; a.c_all = c_all; a.gates = (bf16*)gates; a.hprev_all = (bf16*)hprev_all; a.h_final = h_final; a.c_final = c_final;
-  a.hbuf = (bf16*)hbuf; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+  a.hbuf = (bf16*)hbuf; a.hx = nullptr; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
   cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   const size_t smem = fwd_smem<Narrow>(H);
   cudaError_t e = cudaFuncSetAttribute(lstm_persist_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -617,7 +788,7 @@ RB_EXPORT int rb200_blstm_supported(int T, int B, int H) { return pair_shape(T, 
 
 // ptrs[d * 11 + i] for direction d (0: forward in time, 1: reversed):
 //   0 z_in [T,B,4H] bf16, 1 w_rec [4H,H] bf16, 2 h0, 3 c0 [B,H] fp32, 4 y [T,B,H] bf16, 5 c_all [T,B,H] fp32, 6 gates [T,B,4H] bf16,
-//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 hbuf (scratch, 2*B*H bf16)
+//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 exchange buffer (scratch, 2*B*H 32-bit words)
 RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, int H, int* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return RB_OK;
   const int shape = pair_shape(T, B, H);
@@ -637,7 +808,9 @@ RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, 
     a.z_in = (const bf16*)q[0]; a.w_rec = (const bf16*)q[1]; a.lens = lens; a.h0 = (const float*)q[2]; a.c0 = (const float*)q[3];
     a.T = T; a.B = B; a.H = H; a.reverse = d;
     a.y = (bf16*)q[4]; a.c_all = (float*)q[5]; a.gates = (bf16*)q[6]; a.hprev_all = (bf16*)q[7]; a.h_final = (float*)q[8]; a.c_final = (float*)q[9];
-    a.hbuf = (bf16*)q[10]; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+    a.hbuf = (bf16*)q[10]; a.hx = (uint32_t*)q[10];
+    if (shape != kNarrow) cudaMemsetAsync(a.hx, 0, (size_t)2 * B * H * sizeof(uint32_t), stream);
+    a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
     cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   }
   const cudaError_t e = shape == kWide1   ? launch_fwd_pair<Wide1>(pp, H, stream)
