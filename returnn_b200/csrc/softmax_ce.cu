@@ -13,6 +13,13 @@ __device__ __forceinline__ float ld(const void* x, int64_t i, int is_bf16) {
   return is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i]) : reinterpret_cast<const float*>(x)[i];
 }
 
+// A row of an odd vocabulary starts anywhere: single elements up to the first 16-byte boundary of the logits, 16-byte accesses from there
+// on, single elements at the end. (With single elements for every such row, 6000 x 10025 took as long as 6000 x 32000.)
+__device__ __forceinline__ int row_head(const void* x, int64_t base, int v, int elem) {
+  const int off = (int)((reinterpret_cast<uintptr_t>(x) + (uint64_t)base * elem) & 15);
+  return min(off ? (16 - off) / elem : 0, v);
+}
+
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
 ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, float* __restrict__ loss, float* __restrict__ lse_out,
@@ -22,10 +29,20 @@ ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, floa
   const int64_t base = row * (int64_t)v;
   float mx = -INFINITY, sum = 0.f, tot = 0.f;
   int bi = 0x7fffffff;  // index of this thread's first maximum
-  const int v8 = ((base & 7) == 0) ? (v & ~7) : 0;  // vector path only when the row start is 16-byte aligned
+  const int head = row_head(logits, base, v, kBf16 ? 2 : 4);
+  const int v8 = head + ((v - head) & ~7);
+  for (int c = threadIdx.x; c < head; c += blockDim.x) {
+    float a = ld(logits, base + c, is_bf16);
+    if (a > mx) bi = c;
+    float nm = fmaxf(mx, a);
+    const float nu = nm == -INFINITY ? 0.f : nm;  // (only classes of score -inf so far)
+    sum = sum * __expf(mx - nu) + __expf(a - nu);
+    mx = nm;
+    tot += a;
+  }
   // four independent 16-byte loads in flight per thread: the running max / sum chain is short, the loads are the latency
 #pragma unroll 4
-  for (int c = threadIdx.x * 8; c < v8; c += blockDim.x * 8) {
+  for (int c = head + threadIdx.x * 8; c < v8; c += blockDim.x * 8) {
     F8 a = load8(logits, base + c, is_bf16);
     float lm = a.v[0];
     int li = 0;
@@ -37,20 +54,22 @@ ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, floa
       }
     if (lm > mx) bi = c + li;
     float nm = fmaxf(mx, lm);
+    const float nu = nm == -INFINITY ? 0.f : nm;
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      s += __expf(a.v[k] - nm);
+      s += __expf(a.v[k] - nu);
       tot += a.v[k];
     }
-    sum = sum * __expf(mx - nm) + s;
+    sum = sum * __expf(mx - nu) + s;
     mx = nm;
   }
   for (int c = v8 + threadIdx.x; c < v; c += blockDim.x) {
     float a = ld(logits, base + c, is_bf16);
     if (a > mx) bi = c;
     float nm = fmaxf(mx, a);
-    sum = sum * __expf(mx - nm) + __expf(a - nm);
+    const float nu = nm == -INFINITY ? 0.f : nm;  // (only classes of score -inf so far)
+    sum = sum * __expf(mx - nu) + __expf(a - nu);
     mx = nm;
     tot += a;
   }
@@ -108,9 +127,11 @@ ce_bwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, cons
   const float dl = valid ? dloss[row] : 0.f;
   const float q_other = smoothing > 0.f ? smoothing / (float)(mode == 1 ? v : v - 1) : 0.f;
   const float q_tgt = 1.f - smoothing + (mode == 1 ? q_other : 0.f);
-  const int v8 = ((base & 7) == 0) ? (v & ~7) : 0;
+  const int head_in = row_head(logits, base, v, kBf16 ? 2 : 4), head_out = row_head(dlogits, base, v, kBf16 ? 2 : 4);
+  const int head = head_in == head_out ? head_in : v;  // (buffers that are aligned differently: single elements)
+  const int v8 = head + ((v - head) & ~7);
 #pragma unroll 4
-  for (int c = threadIdx.x * 8; c < v8; c += blockDim.x * 8) {
+  for (int c = head + threadIdx.x * 8; c < v8; c += blockDim.x * 8) {
     F8 a = load8(logits, base + c, is_bf16);
     F8 o;
 #pragma unroll
@@ -121,7 +142,8 @@ ce_bwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, cons
     }
     store8(dlogits, base + c, o, is_bf16);
   }
-  for (int c = v8 + threadIdx.x; c < v; c += blockDim.x) {
+  for (int i = threadIdx.x; i < v - (v8 - head); i += blockDim.x) {
+    const int c = i < head ? i : i + (v8 - head);
     float p = __expf(ld(logits, base + c, is_bf16) - lse);
     float q = (c == y) ? q_tgt : q_other;
     float o = dl * (p - q);
