@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kBwdAccWarps * 32, 1)
 ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, const void* __restrict__ gamma,
                   const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
                   float* __restrict__ dgamma, float* __restrict__ dbeta, int64_t rows, int n, int w_bf16, int rms,
-                  const __nv_bfloat16* __restrict__ dres) {
+                  const __nv_bfloat16* __restrict__ dres, unsigned int* __restrict__ done, void* __restrict__ gamma_out, void* __restrict__ beta_out) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
   extern __shared__ __align__(16) unsigned char smem_raw[];  // [warps][depth][3][n] bf16, later [warps][2][n] fp32
@@ -354,6 +354,26 @@ ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
       atomicAdd(dbeta + i - n, t);
     }
   }
+  if (!done) return;
+  // the CTA that finishes last turns the sums into the gradients in the type of the parameters (else a fill and two conversions around
+  // this kernel, each of which takes as long as it)
+  __shared__ unsigned int order;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) order = atomicAdd(done, 1u);
+  __syncthreads();
+  if (order + 1 != gridDim.x) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const float tg = __ldcg(dgamma + i), tb = __ldcg(dbeta + i);
+    if (w_bf16) {
+      reinterpret_cast<__nv_bfloat16*>(gamma_out)[i] = __float2bfloat16(tg);
+      if (beta_out) reinterpret_cast<__nv_bfloat16*>(beta_out)[i] = __float2bfloat16(tb);
+    } else {
+      reinterpret_cast<float*>(gamma_out)[i] = tg;
+      if (beta_out) reinterpret_cast<float*>(beta_out)[i] = tb;
+    }
+  }
 }
 
 // partial sums -> dgamma / dbeta. Block = 32 columns x 8 slices of the partials; grid = ceil(n / 32).
@@ -411,6 +431,36 @@ RB_EXPORT int rb200_layer_norm_fwd(const void* x, const void* gamma, const void*
 }
 
 // dres (optional, same layout as dx): added to dx; accumulate: dgamma / dbeta += instead of =
+// one-kernel form (bf16 rows of at most 512 columns): dgamma / dbeta are added to; with `done` (a zeroed counter) the last CTA also writes them
+// as gamma_out / beta_out in the type of the parameters
+static int ln_bwd_acc(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta,
+                      long long rows, int n, int w_bf16, int rms, const void* dres, unsigned int* done, void* gamma_out, void* beta_out,
+                      cudaStream_t stream) {
+  int ctas = (int)((rows + kBwdAccWarps - 1) / kBwdAccWarps);
+  if (ctas > 148) ctas = 148;
+  const size_t sm = (size_t)kBwdAccWarps * kBwdAccDepth * 3 * n * sizeof(__nv_bfloat16);  // >= the [warps][2][n] fp32 it becomes at the end
+  const int ch = (n + 255) / 256;
+  static bool attr_set[2] = {false, false};
+#define LN_ACC(C)                                                                                                                       \
+if (!attr_set[C - 1]) {                                                                                                               \
+  if (cudaFuncSetAttribute(ln_bwd_acc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)kBwdAccWarps * kBwdAccDepth * 3 * 512 * 2)) != cudaSuccess) { \
+    rb_set_error("layer_norm_bwd_acc: cannot reserve shared memory");                                                                 \
+    return RB_ERR_LAUNCH;                                                                                                              \
+  }                                                                                                                                   \
+  attr_set[C - 1] = true;                                                                                                             \
+}                                                                                                                                     \
+rb_launch_pdl(ln_bwd_acc_kernel<C>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, gamma, mean, rstd, \
+                                                               (__nv_bfloat16*)dx, dgamma, dbeta, rows, n, w_bf16, rms,              \
+                                                               (const __nv_bfloat16*)dres, done, gamma_out, beta_out)
+  if (ch <= 1) {
+    LN_ACC(1);
+  } else {
+    LN_ACC(2);
+  }
+#undef LN_ACC
+  return rb_check_launch("layer_norm_bwd_acc");
+}
+
 RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                                       void* dx, float* part, float* dgamma, float* dbeta, long long rows, int n, int n_part,
                                       int x_bf16, int w_bf16, int rms, const void* dres, int accumulate, cudaStream_t stream) {
@@ -419,31 +469,8 @@ RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void*
     return RB_ERR_ARG;
   }
   if (n_part <= 0) return RB_ERR_ARG;
-  if (accumulate && x_bf16 && n <= 512 && rows > 0 && (dgamma || dbeta)) {
-    int ctas = (int)((rows + kBwdAccWarps - 1) / kBwdAccWarps);
-    if (ctas > 148) ctas = 148;
-    const size_t sm = (size_t)kBwdAccWarps * kBwdAccDepth * 3 * n * sizeof(__nv_bfloat16);  // >= the [warps][2][n] fp32 it becomes at the end
-    const int ch = (n + 255) / 256;
-    static bool attr_set[2] = {false, false};
-#define LN_ACC(C)                                                                                                                       \
-  if (!attr_set[C - 1]) {                                                                                                               \
-    if (cudaFuncSetAttribute(ln_bwd_acc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)kBwdAccWarps * kBwdAccDepth * 3 * 512 * 2)) != cudaSuccess) { \
-      rb_set_error("layer_norm_bwd_acc: cannot reserve shared memory");                                                                 \
-      return RB_ERR_LAUNCH;                                                                                                              \
-    }                                                                                                                                   \
-    attr_set[C - 1] = true;                                                                                                             \
-  }                                                                                                                                     \
-  rb_launch_pdl(ln_bwd_acc_kernel<C>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, gamma, mean, rstd, \
-                                                                 (__nv_bfloat16*)dx, dgamma, dbeta, rows, n, w_bf16, rms,              \
-                                                                 (const __nv_bfloat16*)dres)
-    if (ch <= 1) {
-      LN_ACC(1);
-    } else {
-      LN_ACC(2);
-    }
-#undef LN_ACC
-    return rb_check_launch("layer_norm_bwd_acc");
-  }
+  if (accumulate && x_bf16 && n <= 512 && rows > 0 && (dgamma || dbeta))
+    return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, rows, n, w_bf16, rms, dres, nullptr, nullptr, nullptr, stream);
   dim3 grid(n_part), block(kWarpsPerCta * 32);
   size_t smem = (size_t)kWarpsPerCta * 2 * n * sizeof(float);
   int chunks = (n + 255) / 256;
@@ -461,6 +488,22 @@ RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void*
   if (st) return st;
   ln_bwd_reduce_kernel<<<(n + 31) / 32, 256, 0, stream>>>(part, dgamma, dbeta, n, n_part, accumulate);
   return rb_check_launch("layer_norm_bwd_reduce");
+}
+
+// bf16 rows of n <= 512 columns (a multiple of 8): dx, and dgamma / dbeta (may be null) in the type of gamma. work: 2 n + 1 words
+RB_EXPORT int rb200_layer_norm_bwd_typed(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* work,
+                                         void* dgamma, void* dbeta, long long rows, int n, int w_bf16, int rms, cudaStream_t stream) {
+  if (n % 8 != 0 || n <= 0 || n > 512 || rows <= 0) {
+    rb_set_error("layer_norm_bwd_typed: n=%d must be a multiple of 8 and <= 512, rows=%lld positive", n, rows);
+    return RB_ERR_ARG;
+  }
+  const cudaError_t e = cudaMemsetAsync(work, 0, (size_t)(2 * n + 1) * sizeof(float), stream);
+  if (e != cudaSuccess) {
+    rb_set_error("layer_norm_bwd_typed: %s", cudaGetErrorString(e));
+    return RB_ERR_LAUNCH;
+  }
+  return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, work, work + n, rows, n, w_bf16, rms, nullptr, reinterpret_cast<unsigned int*>(work + 2 * n), dgamma, dbeta,
+                    stream);
 }
 
 RB_EXPORT int rb200_layer_norm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
