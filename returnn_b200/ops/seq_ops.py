@@ -117,7 +117,9 @@ def beam_topk(logits: torch.Tensor, prev_scores: torch.Tensor, *, finished: Opti
     if _native(logits, "rb200_beam_topk") and k <= 32 and beam <= 64 and logits.dtype in (torch.float32, torch.bfloat16):
         lg = logits.contiguous()
         ps = prev_scores.float().contiguous()
-        fin = finished.to(torch.uint8).contiguous() if finished is not None else None
+        fin = None
+        if finished is not None:  # the bytes of a bool tensor are the 0 / 1 that the kernel reads
+            fin = finished.contiguous().view(torch.uint8) if finished.dtype == torch.bool else finished.to(torch.uint8).contiguous()
         dev = logits.device
         out_s = torch.empty(B, k, dtype=torch.float32, device=dev)
         out_b = torch.empty(B, k, dtype=torch.int32, device=dev)
