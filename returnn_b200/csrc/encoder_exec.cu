@@ -42,6 +42,12 @@ int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* dk, const 
                         int n_rows, int heads, int dim, int lp, cudaStream_t stream);
 int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, int to_padded,
                           cudaStream_t stream);
+int rb200_rel_flash_band(int lp, int center, int* off, int* width);
+int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const void* o, const void* d_o, void* dqu,
+                        void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch, int heads,
+                        int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream);
+int rb200_rel_flash_slices(long long rows, int width, int heads);
+int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream);
 int rb200_glu_dwconv_fwd(const void* x, const float* filt, const float* bias, const int* row_batch, const int* row_pos, const int* lens,
                          void* y, float* part, int n_rows, int C, int K, cudaStream_t stream);
 int rb200_bn_stats(const float* part, int n_tiles, int C, float count, float eps, float momentum, float* mean, float* rstd,
@@ -186,6 +192,11 @@ struct Geometry {
   size_t pad_rows;     // B * Lp
   size_t score_elems;  // B * H * Lp * Lp
   size_t band_elems;   // H * B * Lp * Rp
+  // head dim 64: one kernel for the score gradients and the query gradients (rel_pos_flash.cu) over a band of its own width. The forward
+  // pass stays with the batched products: its bf16 scores are what a training step is compared by.
+  bool fused_bwd;
+  int band_w, band_off = 0, slices = 1;  // columns of the backward band, that of position 0, slices of the position gradient's product
+  size_t dband_elems;
   unsigned long long site_ff_act, site_ff_out, site_att, site_att_out, site_conv_out, site_ff2_act, site_ff2_out, per_layer;
   explicit Geometry(const RbEncDims& d) {
     keep_wd = d.training && d.p_att > 0.f;
@@ -197,6 +208,13 @@ struct Geometry {
     pad_rows = (size_t)B * Lp;
     score_elems = (size_t)B * H * Lp * Lp;
     band_elems = (size_t)H * B * Lp * Rp;
+    fused_bwd = Dh == 64;
+    band_w = Rp;
+    if (fused_bwd) {
+      rb200_rel_flash_band(Lp, center, &band_off, &band_w);
+      slices = rb200_rel_flash_slices((long long)pad_rows, band_w, H);
+    }
+    dband_elems = (size_t)H * B * Lp * band_w;
     auto r8 = [](unsigned long long v) { return (v + 7ull) & ~7ull; };
     unsigned long long o = 0;
     site_ff_act = o; o += r8((unsigned long long)n * F);
@@ -212,7 +230,7 @@ struct Geometry {
 
 // activations kept from forward to backward, per layer
 struct Saved {
-  bf16 *ln1, *z1, *a1, *x1, *ln2, *qu, *qv, *kk, *vv, *w, *wd, *posp, *att, *x2, *ln3, *g, *y, *zc, *x3, *ln4, *z2, *a2, *x4, *out;
+  bf16 *ln1, *z1, *a1, *x1, *ln2, *qu, *qv, *kk, *vv, *w, *wd, *o_pad, *posp, *att, *x2, *ln3, *g, *y, *zc, *x3, *ln4, *z2, *a2, *x4, *out;
   float *st1, *st2, *st3, *st4, *st5, *bn_ms;
 };
 
@@ -235,6 +253,7 @@ struct SavedLayout {
     s.w = bump.take<bf16>(g.score_elems);
     // the dropped probabilities are kept too (recomputing them in the backward pass costs a full pass over the scores)
     s.wd = g.keep_wd ? bump.take<bf16>(g.score_elems) : s.w;
+    s.o_pad = bump.take<bf16>(g.fused_bwd ? g.pad_rows * HD : 0);
     s.posp = bump.take<bf16>((size_t)g.R * HD);
     s.att = bump.take<bf16>(n * HD); s.x2 = bump.take<bf16>(n * D);
     s.ln3 = bump.take<bf16>(n * D); s.st3 = bump.take<float>(2 * n);
@@ -437,7 +456,7 @@ struct TmpFwd {
     qkv = b.take<bf16>((size_t)g.n * 3 * g.HD);
     s_ac = b.take<float>(g.score_elems);
     band = b.take<float>(g.band_elems);
-    o_pad = b.take<bf16>(g.pad_rows * g.HD);
+    o_pad = b.take<bf16>(g.fused_bwd ? 0 : g.pad_rows * g.HD);
     conv_part = b.take<float>((size_t)((g.n + 31) / 32) * 2 * g.D);
     if (total) *total = b.off + 256;
   }
@@ -446,7 +465,7 @@ struct TmpFwd {
 // scratch of the backward pass
 struct TmpBwd {
   bf16 *dA, *dB, *tD, *tD2, *tD3, *tW, *datt, *do_pad, *ds, *dband, *dqu, *dqv, *dk, *dv, *dpos;
-  float *dwd, *ln_part, *bn_part, *conv_part, *sum_ds, *sum_ds_yh;
+  float *dwd, *dpos_part, *ln_part, *bn_part, *conv_part, *sum_ds, *sum_ds_yh;
   TmpBwd(void* base, const Geometry& g, size_t* total) {
     Bump b(base);
     const size_t n = g.n, D = g.D, HD = g.HD;
@@ -459,13 +478,14 @@ struct TmpBwd {
     datt = b.take<bf16>(n * HD);
     do_pad = b.take<bf16>(g.pad_rows * HD);
     ds = b.take<bf16>(g.score_elems);
-    dband = b.take<bf16>(g.band_elems);
+    dband = b.take<bf16>(g.dband_elems);
     dqu = b.take<bf16>(4 * g.pad_rows * HD);
     dqv = dqu ? dqu + g.pad_rows * HD : nullptr;
     dk = dqu ? dqu + 2 * g.pad_rows * HD : nullptr;
     dv = dqu ? dqu + 3 * g.pad_rows * HD : nullptr;
-    dpos = b.take<bf16>((size_t)g.R * HD);
-    dwd = b.take<float>(g.score_elems);
+    dpos = b.take<bf16>((size_t)(g.fused_bwd ? g.band_w : g.R) * HD);
+    dpos_part = b.take<float>(g.slices > 1 ? (size_t)g.slices * g.band_w * HD : 0);
+    dwd = b.take<float>(g.fused_bwd ? 0 : g.score_elems);
     ln_part = b.take<float>((size_t)ln_parts(g.n) * 2 * D);
     bn_part = b.take<float>((size_t)bn_tiles_a(g.n) * 2 * D);
     conv_part = b.take<float>((size_t)((g.n + 31) / 32) * D * (g.K + 1));
@@ -555,14 +575,15 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
       const long long o2[10] = {Lp, 0, 0, Dh, 0, 0, 0, Dh, (long long)Lp * Rp, (long long)B * Lp * Rp};
       e.bgemm(sv.qv, sv.posp, t.band, Lp, g.R, Dh, 0, 0, HD, HD, Rp, (long long)B * Lp, HD, g.R, HD, o2, B * H, H, lens, 1, 0, 0, d.att_scale, 0);
     }
+    bf16* o_pad = g.fused_bwd ? sv.o_pad : t.o_pad;
     // w and wd need no memset: the softmax kernel zeroes the margin that the GEMMs read beyond each sequence's length
     bf16* wd = p_att > 0.f ? sv.wd : sv.w;
     if (e.ok()) e.run_tagged("att_softmax_fwd_ex", rb200_att_softmax_fwd_ex(t.s_ac, t.band, 1, sv.w, wd, lens, B, H, Lp, Rp, g.center, p_att, seed, lay.att_off + l, stream));
     {
       const long long o3[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(wd, sv.vv, t.o_pad, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o3, B * H, H, lens, 1, 0, 1, 1.f, 0);
+      e.bgemm(wd, sv.vv, o_pad, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o3, B * H, H, lens, 1, 0, 1, 1.f, 0);
     }
-    if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(t.o_pad, sv.att, row_batch, row_pos, n, HD, Lp, 0, stream));
+    if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(o_pad, sv.att, row_batch, row_pos, n, HD, Lp, 0, stream));
     e.linear_fwd(sv.att, l, P_PROJ_W, P_PROJ_B, n, HD, D, sv.x2, nullptr, 0, p_res, e.site(l, g.site_att_out), sv.x1, 1.f);
     // ---- convolution module
     e.layer_norm(sv.x2, l, P_CONV_LN_G, sv.ln3, sv.st3);
@@ -655,30 +676,46 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     e.linear_dgrad(t.tD, l, P_PROJ_W, n, HD, D, t.datt, nullptr, 0, 0.f, 0);
     e.memset0(t.do_pad, g.pad_rows * HD * sizeof(bf16));
     if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(t.datt, t.do_pad, row_batch, row_pos, n, HD, Lp, 1, stream));
-    const bf16* wd = p_att > 0.f ? sv.wd : sv.w;
-    {
-      const long long o4[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
-      e.bgemm(t.do_pad, sv.vv, t.dwd, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o4, B * H, H, lens, 1, 1, 0, 1.f, 0);
-      const long long o5[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(wd, t.do_pad, t.dv, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o5, B * H, H, lens, 1, 0, 1, 1.f, 0);
-    }
-    e.memset0(t.dband, g.band_elems * sizeof(bf16));
-    if (e.ok()) e.run_tagged("att_softmax_bwd_ex", rb200_att_softmax_bwd_ex(sv.w, t.dwd, 1, t.ds, t.dband, lens, B, H, Lp, Rp, g.center, p_att, seed, lay.att_off + l, stream));
+    bf16* wd = p_att > 0.f ? sv.wd : sv.w;
+    e.memset0(t.dband, g.dband_elems * sizeof(bf16));
     e.memset0(t.dqu, 2 * g.pad_rows * HD * sizeof(bf16));  // dqu, dqv: their column sums run over all padded rows
-    {
-      const long long o6[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(t.ds, sv.kk, t.dqu, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o6, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
-      e.bgemm(t.ds, sv.qu, t.dk, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o6, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
-      const long long o8[10] = {Lp, (long long)B * Lp, 0, 0, 0, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(t.dband, sv.posp, t.dqv, Lp, Dh, g.R, 0, 1, Rp, HD, HD, (long long)H * B * Lp, Rp, g.R, HD, o8, B * H, H, lens, 1, 0, 0, d.att_scale, 0);
-      const long long o9[10] = {0, (long long)B * Lp, 0, 0, 0, 0, 0, Dh, 0, Dh};
-      e.bgemm(t.dband, sv.qv, t.dpos, g.R, Dh, B * Lp, 1, 1, Rp, HD, HD, (long long)H * B * Lp, Rp, (long long)B * Lp, HD, o9, H, H, nullptr, 0, 0, 0,
-              d.att_scale, 0);
+    const bf16* dpos = t.dpos;
+    if (g.fused_bwd) {
+      if (e.ok())
+        e.run_tagged("rel_flash_bwd", rb200_rel_flash_bwd(sv.qu, sv.qv, sv.kk, sv.vv, sv.posp, sv.o_pad, t.do_pad, t.dqu, t.dqv, sv.w, wd, t.ds, t.dband,
+                                                          nullptr, nullptr, lens, B, H, Lp, g.R, g.center, d.att_scale, p_att, status, stream));
+      const long long o_rows[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
+      e.bgemm(wd, t.do_pad, t.dv, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, 1.f, 0);
+      e.bgemm(t.ds, sv.qu, t.dk, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
+      const int rows = (int)(g.pad_rows / g.slices);
+      const long long o9[10] = {rows, (long long)B * Lp, 0, 0, rows, 0, 0, Dh, (long long)g.band_w * HD, Dh};
+      e.bgemm(t.dband, sv.qv, g.slices > 1 ? (void*)t.dpos_part : t.dpos, g.band_w, Dh, rows, 1, 1, g.band_w, HD, HD, (long long)H * B * Lp, g.band_w,
+              (long long)B * Lp, HD, o9, g.slices * H, H, nullptr, 0, 0, 0, d.att_scale, g.slices > 1);
+      if (g.slices > 1 && e.ok()) e.run_tagged("sum_slices", rb200_sum_slices(t.dpos_part, t.dpos, g.slices, (long long)g.band_w * HD, stream));
+      dpos = t.dpos + (size_t)g.band_off * HD;  // the band's first columns lie before position 0
+    } else {
+      {
+        const long long o4[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
+        e.bgemm(t.do_pad, sv.vv, t.dwd, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o4, B * H, H, lens, 1, 1, 0, 1.f, 0);
+        const long long o5[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
+        e.bgemm(wd, t.do_pad, t.dv, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o5, B * H, H, lens, 1, 0, 1, 1.f, 0);
+      }
+      if (e.ok()) e.run_tagged("att_softmax_bwd_ex", rb200_att_softmax_bwd_ex(sv.w, t.dwd, 1, t.ds, t.dband, lens, B, H, Lp, Rp, g.center, p_att, seed, lay.att_off + l, stream));
+      {
+        const long long o6[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
+        e.bgemm(t.ds, sv.kk, t.dqu, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o6, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
+        e.bgemm(t.ds, sv.qu, t.dk, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o6, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
+        const long long o8[10] = {Lp, (long long)B * Lp, 0, 0, 0, 0, 0, Dh, (long long)Lp * HD, Dh};
+        e.bgemm(t.dband, sv.posp, t.dqv, Lp, Dh, g.R, 0, 1, Rp, HD, HD, (long long)H * B * Lp, Rp, g.R, HD, o8, B * H, H, lens, 1, 0, 0, d.att_scale, 0);
+        const long long o9[10] = {0, (long long)B * Lp, 0, 0, 0, 0, 0, Dh, 0, Dh};
+        e.bgemm(t.dband, sv.qv, t.dpos, g.R, Dh, B * Lp, 1, 1, Rp, HD, HD, (long long)H * B * Lp, Rp, (long long)B * Lp, HD, o9, H, H, nullptr, 0, 0, 0,
+                d.att_scale, 0);
+      }
     }
     if (e.ok()) e.run_tagged("att_pack_dqkv", rb200_att_pack_dqkv(t.dqu, t.dqv, t.dk, t.dv, row_batch, row_pos, t.tW, n, H, Dh, Lp, stream));
     if (e.ok() && e.g32(l, P_POS_U)) e.run_tagged("colsum", colsum(t.dqu, nullptr, e.g32(l, P_POS_U), (int)g.pad_rows, HD, 1.f, 0.f, nullptr, nullptr, 0, stream));
     if (e.ok() && e.g32(l, P_POS_V)) e.run_tagged("colsum", colsum(t.dqv, nullptr, e.g32(l, P_POS_V), (int)g.pad_rows, HD, 1.f, 0.f, nullptr, nullptr, 0, stream));
-    e.linear_wgrad(sinus, t.dpos, l, P_POS_W, -1, g.R, D, HD, false);
+    e.linear_wgrad(sinus, dpos, l, P_POS_W, -1, g.R, D, HD, false);
     e.linear_wgrad(sv.ln2, t.tW, l, P_QKV_W, P_QKV_B, n, D, 3 * HD, true);
     e.linear_dgrad(t.tW, l, P_QKV_W, n, D, 3 * HD, t.tD2, nullptr, 0, 0.f, 0);
     e.layer_norm_bwd(sv.x1, t.tD2, l, P_ATT_LN_G, sv.st2, t.dB, t.dA, t.ln_part);

@@ -1,0 +1,128 @@
+// Building blocks of the fused attention kernels (sdpa_flash.cu, rel_pos_flash.cu): [128, 64] operand tiles in shared memory (128-byte
+// swizzle), products of 64-wide tiles, rows of tensor memory in registers, and the life of a CTA (barriers, tensor memory, abort flag).
+#pragma once
+#include "tcgen05.cuh"
+
+namespace rbf {
+
+using namespace rbt;
+
+constexpr int kRows = 128;   // rows of a CTA
+constexpr int kTile = 64;    // width of a score tile, and the head dim
+constexpr int kBig = kRows * 128;   // bytes of a [128, 64] bf16 tile
+constexpr int kSmall = kTile * 128;  // ... [64, 64]
+constexpr float kLog2e = 1.4426950408889634f;
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ void tmem_ld64(uint32_t addr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  tmem_ld32(addr, r);
+  tmem_ld32(addr + 32, r + 32);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// 64 values -> row `row` of a swizzled [rows, 64] bf16 tile
+__device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float* v) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    *reinterpret_cast<uint4*>(tile + row * 128 + ((c ^ (row & 7)) << 4)) =
+        make_uint4(pack2(v[8 * c], v[8 * c + 1]), pack2(v[8 * c + 2], v[8 * c + 3]), pack2(v[8 * c + 4], v[8 * c + 5]), pack2(v[8 * c + 6], v[8 * c + 7]));
+  }
+}
+
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
+  const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    s = fmaf(__uint_as_float(x[e] << 16), __uint_as_float(y[e] << 16), s);
+    s = fmaf(__uint_as_float(x[e] & 0xffff0000u), __uint_as_float(y[e] & 0xffff0000u), s);
+  }
+  return s;
+}
+
+// D[128, 64] (+)= A[128, 64] B: A K-major; B K-major [n, k] or, `b_mn`, stored [k, n]
+template <bool B_MN>
+__device__ __forceinline__ void mma64(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    umma_f16(d, make_desc(sa + kk * 32, 16, 1024), B_MN ? make_desc(sb + kk * 2048, 8192, 1024) : make_desc(sb + kk * 32, 16, 1024), idesc,
+             (accumulate || kk > 0) ? 1u : 0u);
+  }
+}
+
+// barriers, tensor memory and the abort flag of a CTA
+struct Cta {
+  uint64_t* full;    // [2] loads of a stage
+  uint64_t* done;    // products of an iteration
+  uint64_t* extra;   // one more load
+  uint32_t tmem;
+  volatile int* abort_flag;
+};
+
+// DONE: arrivals that complete a phase of `done`
+template <uint32_t COLS, uint32_t DONE = 1>
+__device__ __forceinline__ Cta cta_begin(uint8_t* tail) {
+  Cta c;
+  c.full = reinterpret_cast<uint64_t*>(tail);
+  c.done = c.full + 2;
+  c.extra = c.full + 3;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(c.full + 4);
+  c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(c.full + i, i == 2 ? DONE : 1);
+    *c.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  c.tmem = *slot;
+  return c;
+}
+
+template <uint32_t COLS>
+__device__ __forceinline__ void cta_end(const Cta& c) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*c.abort_flag && threadIdx.x == 0) {
+    for (uint32_t i = 0; i < (1u << 12); ++i) __nanosleep(256);  // copies still in flight land before the shared memory goes away
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "r"(COLS) : "memory");
+  }
+}
+
+__device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// bounded wait; a wait that gives up marks the CTA and the status word
+__device__ __forceinline__ bool wait_or_abort(const Cta& c, uint64_t* bar, uint32_t parity, int* status, int code) {
+  const bool ok = mbar_wait(bar, parity, c.abort_flag);
+  if (!ok) {
+    *c.abort_flag = 1;
+    if (status) atomicCAS(status, 0, (8 << 24) | code);
+  }
+  return ok;
+}
+
+}  // namespace rbf

@@ -1,0 +1,567 @@
+// Relative-position self-attention for head dim 64, fused: scores, shifted position scores, mask, softmax, dropout and the product with the
+// values in one kernel; in the backward pass the recomputed scores, dP, dS and the query gradients in another.
+//
+// Operands are the zero-padded [B, Lp, H*64] matrices of att_prepare (queries with either bias, keys, values) and the projected positions
+// [R, H*64]: score(i, j) = scale * (qu_i . k_j + qv_i . p_{center + j - i}). For a tile of 128 queries from i0 and W keys from j0 the second
+// term needs the W + 127 position rows from center + j0 - i0 - 127 on: one product [128, W + 128] against a window of the position matrix
+// that TMA reads in place (rows outside it are zero). Row i of the result is needed from column 127 - i on: a thread owns a row, the 32 rows
+// of a warp read a common window of tensor memory, and each lane shifts its registers by 31 - lane places in five conditional steps.
+//
+//   rel_fwd  one CTA per (batch entry, head, 128 queries), W = 128: two groups of 128 threads with 64 keys each, each with its own running
+//            maximum, sum and accumulator, merged at the end (tensor memory: 128 scores + 256 positions + 2 x 64 outputs = all 512 columns)
+//   rel_bwd  the same split, W = 64, two groups with 32 keys each: P and dS go to memory for the two products over queries (dV, dK), dQu
+//            and dQv accumulate in tensor memory; dS shifted back is the A operand of dQv and is added to the band that the position
+//            gradient is a product of (the tiles of one row fill disjoint columns of a zeroed band: a bulk add is a store).
+// What went through memory before: scores and position band written and read in both passes, probabilities, dP.
+#include "flash.cuh"
+
+using namespace rbf;
+
+namespace {
+
+constexpr int kThreads = 256;
+
+struct Rel {
+  const int* lens;
+  float* lse;      // [B*H, lp] log2 of the softmax denominator, maximum included
+  uint32_t* keep;  // [B*H, lp, words] dropout: bit j of word w = key 32 w + j is kept
+  const __nv_bfloat16* w;  // [B*H, lp, lp] (backward, saved form) probabilities
+  __nv_bfloat16 *p, *ds;   // [B*H, lp, lp] (backward) dropped probabilities (saved form: read) and score gradients
+  const long long* seed;
+  const long long* offset;
+  int* status;
+  int batch, heads, lp, tiles, words, center, band_off;
+  float scale, p_drop;
+};
+
+template <uint32_t N>
+__device__ __forceinline__ void mma_n(uint32_t d, const uint8_t* a, const uint8_t* b) {  // D[128, N] = A[128, 64] B[N, 64]^T, both K-major
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) umma_f16(d, make_desc(sa + kk * 32, 16, 1024), make_desc(sb + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
+}
+
+// g[j] <- g[j + shift] for j < N, shift in [0, 31]; g holds N + 31 values
+template <int N, int B>
+__device__ __forceinline__ void shift_step(float* g, int shift) {
+  const bool on = shift & B;
+#pragma unroll
+  for (int j = 0; j < N + B - 1; ++j) g[j] = on ? g[j + B] : g[j];
+}
+template <int N>
+__device__ __forceinline__ void shift_down(float* g, int shift) {
+  shift_step<N, 16>(g, shift);
+  shift_step<N, 8>(g, shift);
+  shift_step<N, 4>(g, shift);
+  shift_step<N, 2>(g, shift);
+  shift_step<N, 1>(g, shift);
+}
+
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+template <bool DROP>
+__global__ void __launch_bounds__(kThreads, 1)
+rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant__ CUtensorMap tm_qv, const __grid_constant__ CUtensorMap tm_k,
+               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_pos, const __grid_constant__ CUtensorMap tm_o,
+               const Rel p) {
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const int z = blockIdx.x / p.tiles;
+  const int q0 = (int)(blockIdx.x % p.tiles) * kRows;
+  const int b = z / p.heads, h = z - b * p.heads;
+  const int len = p.lens[b];
+  if (q0 >= len) return;  // nobody reads the padding rows of the output
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* squ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sqv = squ + kBig;
+  uint8_t* sk = sqv + kBig;        // [2][128 keys]
+  uint8_t* sv = sk + 2 * kBig;     // [2][128 keys]
+  uint8_t* spos = sv + 2 * kBig;   // [2][256 positions]
+  uint8_t* sp = spos + 4 * kBig;   // [2 groups][128 queries][64 keys]
+  const Cta c = cta_begin<512>(sp + 2 * kBig);
+  const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
+  const int row = q0 + r;
+  const int n_tiles = (len + 127) / 128;
+  const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
+  const uint32_t t_s = c.tmem, t_g = c.tmem + 128, t_o = c.tmem + 384;
+  auto load = [&](int t) {
+    const int s = t & 1;
+    tma_load_3d(sk + s * kBig, &tm_k, h * 64, t * 128, b, &c.full[s]);
+    tma_load_3d(sv + s * kBig, &tm_v, h * 64, t * 128, b, &c.full[s]);
+    tma_load_2d(spos + s * 2 * kBig, &tm_pos, h * 64, p.center + t * 128 - q0 - 127, &c.full[s]);
+  };
+  auto scores = [&](int s) {
+    mma_n<128>(t_s, squ, sk + s * kBig);
+    mma_n<256>(t_g, sqv, spos + s * 2 * kBig);
+  };
+  bool ok = true;
+  if (tid == 0) {
+    mbar_expect_tx(&c.full[0], 6 * kBig);
+    tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
+    tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
+    load(0);
+    if (n_tiles > 1) {
+      mbar_expect_tx(&c.full[1], 4 * kBig);
+      load(1);
+    }
+    ok = wait_or_abort(c, &c.full[0], 0, p.status, 21);
+    if (ok) {
+      scores(0);
+      umma_commit(c.done);
+    }
+  }
+  const float cs = p.scale * kLog2e;
+  const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
+  const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
+  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+  float m = -INFINITY, l = 0.f;
+  float acc[64];
+#pragma unroll
+  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+  int it = 0;
+  for (; it < n_tiles; ++it) {
+    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 22);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
+      mbar_expect_tx(&c.full[(it + 1) & 1], 4 * kBig);
+      load(it + 1);
+    }
+    __syncwarp();
+    float s[96];
+    uint32_t* raw = reinterpret_cast<uint32_t*>(s);
+    if (it > 0) {
+      tmem_ld64(t_o + t_lane + wg * 64, s);
+#pragma unroll
+      for (int j = 0; j < 64; ++j) acc[j] += s[j];
+    }
+    // the position scores of this warp's rows: 95 columns from 127 - (its last row) + 64 * group on
+    const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 64);
+    tmem_ld32(g0, raw);
+    tmem_ld32(g0 + 32, raw + 32);
+    tmem_ld32(g0 + 64, raw + 64);
+    tmem_wait_ld();
+    shift_down<64>(s, 31 - lane);
+    const int left = len - (it * 128 + wg * 64);  // keys of this group's half that exist
+    float mx = m;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float a[32];
+      tmem_ld32(t_s + t_lane + wg * 64 + half * 32, reinterpret_cast<uint32_t*>(a));
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int jj = half * 32 + j;
+        s[jj] = jj < left ? (a[j] + s[jj]) * cs : -INFINITY;
+        mx = fmaxf(mx, s[jj]);
+      }
+    }
+    const float mu = mx == -INFINITY ? 0.f : mx;
+    const float corr = ex2(m - mu);
+    m = mx;
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      s[j] = ex2(s[j] - mu);
+      sum += s[j];
+    }
+    l = l * corr + sum;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] *= corr;
+    if constexpr (DROP) {
+      const uint64_t base = off + ((uint64_t)z * p.lp + row) * p.lp + it * 128 + wg * 64;
+      uint32_t bits[2] = {0u, 0u};
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) {
+        const uint64_t ctr = base + j;
+        const uint4 x = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x52u, 0u));
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool k = w[e] >= thresh;
+          s[j + e] = k ? s[j + e] * keep_scale : 0.f;
+          if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        }
+      }
+      if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
+    }
+    store_row64(sp + wg * kBig, r, s);
+    fence_proxy_async_smem();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      uint8_t* v = sv + (it & 1) * kBig;
+      mma64<true>(t_o, sp, v, false);
+      mma64<true>(t_o + 64, sp + kBig, v + kSmall, false);
+      if (it + 1 < n_tiles) {
+        ok = wait_or_abort(c, &c.full[(it + 1) & 1], ((it + 1) >> 1) & 1, p.status, 23);
+        if (ok) scores((it + 1) & 1);
+      }
+      if (ok) umma_commit(c.done);
+    }
+  }
+  if (it == n_tiles) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 24);
+  if (!__syncthreads_or(ok ? 0 : 1)) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float s[64];
+    tmem_ld64(t_o + t_lane + wg * 64, s);
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] += s[j];
+    // merge the two groups through shared memory (the position tiles are not needed any more)
+    float* ex = reinterpret_cast<float*>(spos) + r * 67;
+    if (wg == 1) {
+#pragma unroll
+      for (int j = 0; j < 64; ++j) ex[j] = acc[j];
+      ex[64] = m;
+      ex[65] = l;
+    }
+    __syncthreads();
+    if (wg == 0) {
+      const float m1 = ex[64], mm = fmaxf(m, m1);  // (the first key is always there: m is finite for valid rows)
+      const float e0 = ex2(m - mm), e1 = ex2(m1 - mm);
+      l = l * e0 + ex[65] * e1;
+      const float inv = 1.f / l;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) acc[j] = row < len ? (acc[j] * e0 + ex[j] * e1) * inv : 0.f;
+      store_row64(squ, r, acc);
+      if (row < len) p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&tm_o, h * 64, q0, b, squ);
+      tma_store_commit();
+      tma_store_wait_all();
+    }
+  }
+  cta_end<512>(c);
+}
+
+// SAVED: the probabilities (and, dropped, those of the value product) come from memory, as the forward pass of the encoder executor left them;
+// else they are recomputed and the dropped ones written
+template <bool DROP, bool SAVED>
+__global__ void __launch_bounds__(kThreads, 1)
+rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant__ CUtensorMap tm_qv, const __grid_constant__ CUtensorMap tm_k,
+               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_pos, const __grid_constant__ CUtensorMap tm_o,
+               const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dqu, const __grid_constant__ CUtensorMap tm_dqv,
+               const __grid_constant__ CUtensorMap tm_band, const Rel p) {
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const int z = blockIdx.x / p.tiles;
+  const int q0 = (int)(blockIdx.x % p.tiles) * kRows;
+  const int b = z / p.heads, h = z - b * p.heads;
+  const int len = p.lens[b];
+  if (q0 >= len) return;  // the caller zeroed dQu, dQv and the band
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* squ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sqv = squ + kBig;
+  uint8_t* sdo = sqv + kBig;
+  uint8_t* sk = sdo + kBig;          // [2][64 keys]
+  uint8_t* sv = sk + 2 * kSmall;     // [2][64 keys]
+  uint8_t* spos = sv + 2 * kSmall;   // [2][192 positions]
+  uint8_t* sds = spos + 6 * kSmall;  // [128 queries][64 keys]
+  uint8_t* sdg = sds + kBig;         // [3][128 queries][64 positions]; first the tile of O
+  const Cta c = cta_begin<512, 2>(sdg + 3 * kBig);  // `done`: the products, and the bulk add of the previous iteration has read its tile
+  const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
+  const int row = q0 + r;
+  const int n_tiles = (len + 63) / 64;
+  const int len64 = n_tiles * 64;
+  const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
+  const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_g = c.tmem + 128, t_dqu = c.tmem + 320, t_dqv = c.tmem + 384;
+  const int band_row = (h * p.batch + b) * p.lp + q0;
+  const int n_rows_band = min(kRows, p.lp - q0);
+  auto load = [&](int t) {
+    const int s = t & 1;
+    tma_load_3d(sk + s * kSmall, &tm_k, h * 64, t * 64, b, &c.full[s]);
+    tma_load_3d(sv + s * kSmall, &tm_v, h * 64, t * 64, b, &c.full[s]);
+    tma_load_2d(spos + s * 3 * kSmall, &tm_pos, h * 64, p.center + t * 64 - q0 - 127, &c.full[s]);
+  };
+  auto scores = [&](int s) {
+    mma64<false>(t_dp, sdo, sv + s * kSmall, false);
+    if (SAVED) return;
+    mma64<false>(t_s, squ, sk + s * kSmall, false);
+    mma_n<192>(t_g, sqv, spos + s * 3 * kSmall);
+  };
+  bool ok = true;
+  if (tid == 0) {
+    mbar_expect_tx(&c.full[0], 3 * kBig + 5 * kSmall);
+    tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
+    tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
+    tma_load_3d(sdo, &tm_do, h * 64, q0, b, &c.full[0]);
+    load(0);
+    mbar_expect_tx(c.extra, kBig);
+    tma_load_3d(sdg, &tm_o, h * 64, q0, b, c.extra);
+    if (n_tiles > 1) {
+      mbar_expect_tx(&c.full[1], 5 * kSmall);
+      load(1);
+    }
+    ok = wait_or_abort(c, &c.full[0], 0, p.status, 25);
+    if (ok) {
+      scores(0);
+      umma_commit(c.done);
+      mbar_arrive_local(c.done);
+    }
+  }
+  float lse = INFINITY, delta = 0.f;
+  ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 26) && wait_or_abort(c, c.extra, 0, p.status, 26);
+  if (ok) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int at = r * 128 + ((j ^ (r & 7)) << 4);
+      delta += dot8(*reinterpret_cast<const uint4*>(sdg + at), *reinterpret_cast<const uint4*>(sdo + at));
+    }
+    if (!SAVED && row < len) lse = p.lse[(long long)z * p.lp + row];
+  }
+  __syncthreads();
+  for (int i = tid; i < 3 * kBig / 16; i += kThreads) reinterpret_cast<uint4*>(sdg)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  const float cs = p.scale * kLog2e;
+  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+  int it = 0;
+  for (; it < n_tiles; ++it) {
+    const long long at = ((long long)z * p.lp + row) * p.lp + it * 64 + wg * 32;  // this thread's 32 scores
+    uint4 wv[4], wd[4];
+    if (SAVED && row < len) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        wv[q] = *reinterpret_cast<const uint4*>(p.w + at + 8 * q);
+        if (DROP) wd[q] = *reinterpret_cast<const uint4*>(p.p + at + 8 * q);
+      }
+    }
+    uint32_t bits = 0u;
+    if (DROP && !SAVED && row < len) bits = p.keep[((long long)z * p.lp + row) * p.words + it * 2 + wg];
+    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 27);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
+      mbar_expect_tx(&c.full[(it + 1) & 1], 5 * kSmall);
+      load(it + 1);
+    }
+    __syncwarp();
+    float s[64], a[32], dp[32];
+    if (!SAVED) {
+      const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 32);
+      tmem_ld32(g0, reinterpret_cast<uint32_t*>(s));
+      tmem_ld32(g0 + 32, reinterpret_cast<uint32_t*>(s) + 32);
+      tmem_ld32(t_s + t_lane + wg * 32, reinterpret_cast<uint32_t*>(a));
+    }
+    tmem_ld32(t_dp + t_lane + wg * 32, reinterpret_cast<uint32_t*>(dp));
+    tmem_wait_ld();
+    if (!SAVED) shift_down<32>(s, 31 - lane);
+    const int left = row < len ? len - (it * 64 + wg * 32) : 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const bool vis = j < left;
+      float d = dp[j];
+      if (SAVED) {
+        const uint32_t word = reinterpret_cast<const uint32_t*>(wv)[j >> 1];
+        if (DROP) {  // a dropped probability is zero; where the probability itself is, its gradient is too
+          const uint32_t kept = reinterpret_cast<const uint32_t*>(wd)[j >> 1];
+          d = ((j & 1 ? kept >> 16 : kept) & 0x7fffu) ? d * keep_scale : 0.f;
+        }
+        a[j] = vis ? __uint_as_float(j & 1 ? word & 0xffff0000u : word << 16) * (d - delta) : 0.f;
+      } else {
+        const float pr = vis ? ex2(fmaf(a[j] + s[j], cs, -lse)) : 0.f;
+        float pd = pr;
+        if (DROP) {
+          const bool k = (bits >> j) & 1u;
+          d = k ? d * keep_scale : 0.f;
+          pd = k ? pr * keep_scale : 0.f;
+        }
+        a[j] = vis ? pr * (d - delta) : 0.f;
+        s[j] = pd;
+      }
+    }
+    uint4 pk[4], dk[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (!SAVED) pk[q] = make_uint4(pack2(s[8 * q], s[8 * q + 1]), pack2(s[8 * q + 2], s[8 * q + 3]), pack2(s[8 * q + 4], s[8 * q + 5]), pack2(s[8 * q + 6], s[8 * q + 7]));
+      dk[q] = make_uint4(pack2(a[8 * q], a[8 * q + 1]), pack2(a[8 * q + 2], a[8 * q + 3]), pack2(a[8 * q + 4], a[8 * q + 5]), pack2(a[8 * q + 6], a[8 * q + 7]));
+      *reinterpret_cast<uint4*>(sds + r * 128 + (((wg * 4 + q) ^ (r & 7)) << 4)) = dk[q];
+    }
+    if (row < len64) {  // the products over queries run in blocks of 64 rows: zeros up to there
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!SAVED) *reinterpret_cast<uint4*>(p.p + at + 8 * q) = pk[q];
+        *reinterpret_cast<uint4*>(p.ds + at + 8 * q) = dk[q];
+      }
+    }
+    // shifted back: key j of the tile lies at column 127 - r + j, the same columns of this row in every iteration
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const int col = 127 - r + wg * 32 + j;
+      const uint32_t word = reinterpret_cast<const uint32_t*>(dk)[j >> 1];
+      *reinterpret_cast<unsigned short*>(sdg + (col >> 6) * kBig + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4) + (col & 7) * 2) =
+          (unsigned short)(j & 1 ? word >> 16 : word & 0xffffu);
+    }
+    fence_proxy_async_smem();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int st = it & 1;
+      mma64<true>(t_dqu, sds, sk + st * kSmall, it > 0);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) mma64<true>(t_dqv, sdg + q * kBig, spos + (st * 3 + q) * kSmall, it > 0 || q > 0);
+      if (it + 1 < n_tiles) {
+        ok = wait_or_abort(c, &c.full[st ^ 1], ((it + 1) >> 1) & 1, p.status, 28);
+        if (ok) scores(st ^ 1);
+      }
+      if (ok) {
+        umma_commit(c.done);
+        const int x0 = p.center + it * 64 - q0 - 127 + p.band_off;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+            if (half * 64 < n_rows_band) tma_reduce_add_2d(&tm_band, x0 + 64 * q, band_row + half * 64, sdg + q * kBig + half * kSmall);
+        tma_store_commit();
+        tma_store_wait_read();
+        mbar_arrive_local(c.done);
+      }
+    }
+  }
+  if (it == n_tiles) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 29);
+  if (!__syncthreads_or(ok ? 0 : 1)) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float s[64];
+    tmem_ld64((wg ? t_dqv : t_dqu) + t_lane, s);
+#pragma unroll
+    for (int j = 0; j < 64; ++j) s[j] *= p.scale;
+    store_row64(wg ? sqv : squ, r, s);
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&tm_dqu, h * 64, q0, b, squ);
+      tma_store_3d(&tm_dqv, h * 64, q0, b, sqv);
+      tma_store_commit();
+      tma_store_wait_all();
+    }
+  }
+  cta_end<512>(c);
+}
+
+// sum of the slices of a split product, fp32 [slices][n] -> bf16 [n], n a multiple of 4
+__global__ void __launch_bounds__(256)
+sum_slices_kernel(const float4* __restrict__ x, uint2* __restrict__ y, int slices, long long n4) {
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n4) return;
+  float4 s = x[i];
+  for (int k = 1; k < slices; ++k) {
+    const float4 v = x[k * n4 + i];
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  y[i] = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+}
+
+constexpr int kFwdSmem = 12 * kBig + 64 + 1024;
+constexpr int kBwdSmem = 7 * kBig + 10 * kSmall + 64 + 1024;
+static_assert(kFwdSmem <= 227 * 1024 && kBwdSmem <= 227 * 1024, "shared memory");
+
+// positions [r_rows, HD]: boxes of `box` rows, 64 columns
+int map_pos(CUtensorMap* m, const void* pos, int r_rows, int hd, int box) { return make_map(m, pos, hd, r_rows, hd, 64, box); }
+
+int failed(const char* what, cudaError_t e) {
+  rb_set_error("%s: %s", what, cudaGetErrorString(e));
+  return RB_ERR_LAUNCH;
+}
+
+}  // namespace
+
+// qu, qv, k, v, o: bf16 [B, Lp, H*64] (rows past a sequence's length zero, those of o unspecified); pos [R, H*64]; keep words per row:
+// 4 * ceil(Lp / 128); lse [B*H, Lp]
+RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, void* o, float* lse, void* keep,
+                                  const int* lens, int batch, int heads, int lp, int r_rows, int center, float scale, float p_drop,
+                                  const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
+  if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
+  const int hd = heads * 64;
+  Rel p = {};
+  p.lens = lens; p.lse = lse; p.keep = (uint32_t*)keep; p.seed = seed; p.offset = offset; p.status = status;
+  p.batch = batch; p.heads = heads; p.lp = lp; p.center = center; p.scale = scale; p.p_drop = p_drop;
+  p.tiles = (lp + kRows - 1) / kRows;
+  p.words = 4 * ((lp + 127) / 128);
+  CUtensorMap a, b, c, d, e, f;
+  const long long bp = (long long)lp * hd;
+  int st = make_map_3d(&a, qu, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&b, qv, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 128);
+  if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 128);
+  if (!st) st = map_pos(&e, pos, r_rows, hd, 256);
+  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows);
+  if (st) return st;
+  auto kernel = p_drop > 0.f ? rel_fwd_kernel<true> : rel_fwd_kernel<false>;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
+  if (err != cudaSuccess) return failed("rel_flash_fwd", err);
+  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kFwdSmem, stream, a, b, c, d, e, f, p);
+  return rb_check_launch("rel_flash_fwd");
+}
+
+// Column of the band that position row 0 has, such that every tile's first column is a multiple of 8 and none is negative; *width: columns
+// of the band. (Lp a multiple of 64.)
+RB_EXPORT int rb200_rel_flash_band(int lp, int center, int* off, int* width) {
+  const int tiles = (lp + kRows - 1) / kRows;
+  int o = (tiles - 1) * kRows + 127 - center;
+  if (o < 0) o = 0;
+  while ((center - 127 + o) & 7) ++o;
+  *off = o;
+  *width = (center + lp - 64 - 127 + o + 192 + 63) / 64 * 64;
+  return RB_OK;
+}
+
+// dqu, dqv [B, Lp, H*64] and band [H, B, Lp, band_width] zeroed by the caller; pw, ds [B*H, Lp, Lp]: written for the first
+// 64 * ceil(len / 64) rows and columns of each sequence. With saved probabilities `w` (else null; lse and keep are not read then) pw is read:
+// the dropped probabilities, or anything without dropout
+RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const void* o, const void* d_o,
+                                  void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
+                                  int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
+  if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
+  const int hd = heads * 64;
+  Rel p = {};
+  p.lens = lens; p.lse = lse; p.keep = (uint32_t*)keep; p.status = status; p.w = (const __nv_bfloat16*)w; p.p = (__nv_bfloat16*)pw; p.ds = (__nv_bfloat16*)ds;
+  p.batch = batch; p.heads = heads; p.lp = lp; p.center = center; p.scale = scale; p.p_drop = p_drop;
+  p.tiles = (lp + kRows - 1) / kRows;
+  p.words = 4 * ((lp + 127) / 128);
+  int width = 0;
+  rb200_rel_flash_band(lp, center, &p.band_off, &width);
+  CUtensorMap a, b, c, d, e, f, g, h, i, j;
+  const long long bp = (long long)lp * hd;
+  int st = make_map_3d(&a, qu, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&b, qv, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 64);
+  if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 64);
+  if (!st) st = map_pos(&e, pos, r_rows, hd, 192);
+  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&g, d_o, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&h, dqu, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&i, dqv, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map(&j, band, width, (long long)heads * batch * lp, width, 64, 64);
+  if (st) return st;
+  auto kernel = p_drop > 0.f ? (w ? rel_bwd_kernel<true, true> : rel_bwd_kernel<true, false>) : (w ? rel_bwd_kernel<false, true> : rel_bwd_kernel<false, false>);
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+  if (err != cudaSuccess) return failed("rel_flash_bwd", err);
+  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, p);
+  return rb_check_launch("rel_flash_bwd");
+}
+
+// slices that the product of the position gradient, [band_width, rows] x [rows, 64] per head, is cut into: it has few output tiles and
+// B * Lp rows to sum over (48 tiles of 13824 rows for a full Conformer batch: a third of the SMs for 90 us); two waves of CTAs, equal slices
+// of whole 64-row blocks
+RB_EXPORT int rb200_rel_flash_slices(long long rows, int width, int heads) {
+  const long long blocks = rows / 64, tiles = (long long)((width + 127) / 128) * heads;
+  long long n = 296 / (tiles > 0 ? tiles : 1);
+  if (n > blocks / 4) n = blocks / 4;
+  while (n > 1 && blocks % n) --n;
+  return n > 1 ? (int)n : 1;
+}
+
+RB_EXPORT int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream) {
+  if (n <= 0 || slices <= 0) return RB_OK;
+  if (n % 4) {
+    rb_set_error("sum_slices: n=%lld must be a multiple of 4", n);
+    return RB_ERR_ARG;
+  }
+  rb_launch_pdl(sum_slices_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float4*)x, (uint2*)y, slices, n / 4);
+  return rb_check_launch("sum_slices");
+}

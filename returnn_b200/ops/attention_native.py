@@ -1,7 +1,11 @@
 """
 Relative-position self-attention on packed rows, B200 path.
 
-Stages (forward): ``att_prepare`` (packed qkv -> zero-padded Qu = q+u, Qv = q+v, K, V) -> batched tcgen05 GEMMs
+Head dim 64 (``_RelPosFlash``): ``att_prepare`` (packed qkv -> zero-padded q+u, q+v, K, V), one kernel for scores, shifted position
+scores, softmax, dropout and the product with V, gather back to packed rows; backward: one kernel that recomputes the scores and leaves
+dQu, dQv, P, dS and the position band, batched products for dV, dK and the position gradient, one pack kernel.
+
+Other head dims (``_RelPosAttPacked``), stages (forward): ``att_prepare`` (packed qkv -> zero-padded Qu = q+u, Qv = q+v, K, V) -> batched tcgen05 GEMMs
 ``S_ac = scale * Qu K^T`` and ``G = scale * Qv P^T`` (fp32 out) -> ``att_softmax_fwd`` (shifted bias as an index into G,
 key-length mask, softmax, dropout) -> batched GEMM ``O = Wd V`` -> gather back to packed rows.
 Backward: ``dWd = dO V^T``, ``dV = Wd^T dO``, ``att_softmax_bwd`` (exact delta, un-shift into dG), ``dQu = dS K``,
@@ -191,6 +195,110 @@ class _RelPosAttPacked(torch.autograd.Function):
         return dqkv, dpos, du, dvb, None, None, None, None, None, None, None, None, None
 
 
+class _RelPosFlash(torch.autograd.Function):
+    """head dim 64: scores, softmax and both passes over the keys in one kernel per pass (``csrc/rel_pos_flash.cu``)"""
+
+    @staticmethod
+    def forward(ctx, qkv, pos, u, v, row_batch, row_pos, lens, B, H, max_len, scale, p_drop):
+        dev, bf = qkv.device, torch.bfloat16
+        N, HD = qkv.shape[0], H * 64
+        Lp = (max_len + 63) // 64 * 64
+        R = pos.shape[0]
+        center = (R - 1) // 2
+        assert R <= 2 * Lp and center >= max_len - 1
+        qkv = qkv.contiguous()
+        pos = pos.contiguous()
+        uf = u.float().contiguous() if u is not None else None
+        vf = v.float().contiguous() if v is not None else None
+        pads = torch.zeros(4, B * Lp, HD, dtype=bf, device=dev)  # q + u, q + v, k, v
+        qu, qv, kk, vv = (pads[i].data_ptr() for i in range(4))
+        s = _lib.stream_ptr()
+        fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(qkv.data_ptr(), _p(uf), _p(vf), row_batch.data_ptr(), row_pos.data_ptr(), qu, qv, kk, vv, N, H, 64, Lp, s), "att_prepare")
+        o_pad = torch.empty(B * Lp, HD, dtype=bf, device=dev)
+        lse = torch.empty(B * H * Lp, dtype=torch.float32, device=dev)
+        drop = p_drop > 0.0
+        keep = seed = off = None
+        if drop:
+            keep = torch.empty(B * H * Lp * 4 * ((Lp + 127) // 128), dtype=torch.int32, device=dev)
+            seed = _seed_tensor(dev)
+            off = seed[1:2].clone()
+            seed[1] += B * H * Lp * Lp
+        st = _gemm.status_tensor(dev)
+        fn = _lib.bind("rb200_rel_flash_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _f32, _f32, _vp, _vp, _vp, _vp])
+        _lib.check(fn(qu, qv, kk, vv, pos.data_ptr(), o_pad.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp, R, center, scale, p_drop,
+                      _p(seed), _p(off), st.data_ptr(), s), "rel_flash_fwd")
+        out = torch.empty(N, HD, dtype=bf, device=dev)
+        fn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 0, s), "att_gather")
+        _lib.count_launch(3)
+        ctx.save_for_backward(pads, pos, o_pad, lse, keep, row_batch, row_pos, lens)
+        ctx.dims = (B, H, Lp, R, center, N, scale, p_drop)
+        ctx.u_dtype = u.dtype if u is not None else None
+        ctx.v_dtype = v.dtype if v is not None else None
+        return out
+
+    @staticmethod
+    def backward(ctx, d_out):
+        pads, pos, o_pad, lse, keep, row_batch, row_pos, lens = ctx.saved_tensors
+        B, H, Lp, R, center, N, scale, p_drop = ctx.dims
+        dev, bf = d_out.device, torch.bfloat16
+        HD = H * 64
+        rows = B * Lp
+        d_out = d_out.contiguous()
+        s = _lib.stream_ptr()
+        zeroed = torch.zeros(3, rows, HD, dtype=bf, device=dev)  # dO, dQu, dQv
+        do_pad, dqu, dqv = zeroed[0], zeroed[1], zeroed[2]
+        fn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(d_out.data_ptr(), do_pad.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 1, s), "att_scatter")
+        geo = (ctypes.c_int * 2)()
+        fn = _lib.bind("rb200_rel_flash_band", [_i32, _i32, _vp, _vp])
+        _lib.check(fn(Lp, center, ctypes.addressof(geo), ctypes.addressof(geo) + 4), "rel_flash_band")
+        band_off, width = geo[0], geo[1]
+        band = torch.zeros(H * rows, width, dtype=bf, device=dev)
+        scores = torch.empty(2, B * H * Lp, Lp, dtype=bf, device=dev)
+        pw, ds = scores[0], scores[1]
+        st = _gemm.status_tensor(dev)
+        fn = _lib.bind("rb200_rel_flash_bwd", [_vp] * 16 + [_i32] * 5 + [_f32, _f32, _vp, _vp])
+        _lib.check(fn(pads[0].data_ptr(), pads[1].data_ptr(), pads[2].data_ptr(), pads[3].data_ptr(), pos.data_ptr(), o_pad.data_ptr(), do_pad.data_ptr(),
+                      dqu.data_ptr(), dqv.data_ptr(), None, pw.data_ptr(), ds.data_ptr(), band.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp,
+                      R, center, scale, p_drop, st.data_ptr(), s), "rel_flash_bwd")
+        # dV = Pd^T dO, dK = scale * dS^T Qu
+        dkv = torch.empty(2, rows, HD, dtype=bf, device=dev)
+        for a, b, c, alpha in ((pw, do_pad, dkv[1], 1.0), (ds, pads[0], dkv[0], scale)):
+            _bgemm(a, b, c, m=Lp, n=64, k=Lp, a_mn=True, b_mn=True, lda=Lp, ldb=HD, ldc=HD, a_shape=(B * H * Lp, Lp), b_shape=(rows, HD),
+                   offs=(H * Lp, Lp, 0, 0, Lp, 0, 0, 64, Lp * HD, 64), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=True, alpha=alpha)
+        # dP[h] = scale * band[h]^T Qv[h] over all rows of all sequences, in slices of the rows
+        n = _lib.bind("rb200_rel_flash_slices", [_i64, _i32, _i32])(rows, width, H)
+        part = torch.empty(n, width, HD, dtype=torch.float32 if n > 1 else bf, device=dev)
+        _bgemm(band, pads[1], part, m=width, n=64, k=rows // n, a_mn=True, b_mn=True, lda=width, ldb=HD, ldc=HD, a_shape=(H * rows, width),
+               b_shape=(rows, HD), offs=(rows // n, rows, 0, 0, rows // n, 0, 0, 64, width * HD, 64), batch=n * H, heads=H, lens=None, m_l=False, n_l=False,
+               k_l=False, alpha=scale, out_fp32=n > 1)
+        dpos = part[0]
+        if n > 1:
+            dpos = torch.empty(width, HD, dtype=bf, device=dev)
+            fn = _lib.bind("rb200_sum_slices", [_vp, _vp, _i32, _i64, _vp])
+            _lib.check(fn(part.data_ptr(), dpos.data_ptr(), n, width * HD, s), "sum_slices")
+        dqkv = torch.empty(N, 3 * HD, dtype=bf, device=dev)
+        fn = _lib.bind("rb200_att_pack_dqkv", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(dqu.data_ptr(), dqv.data_ptr(), dkv[0].data_ptr(), dkv[1].data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), dqkv.data_ptr(), N, H,
+                      64, Lp, s), "att_pack_dqkv")
+        _lib.count_launch(4)
+        sums = [None, None]
+        for i, dt in enumerate((ctx.u_dtype, ctx.v_dtype)):
+            if dt is not None:
+                t = torch.zeros(HD, dtype=torch.float32, device=dev)
+                fn = _lib.bind("rb200_colsum_bf16", [_vp, _vp, _i32, _i32, _vp])
+                _lib.check(fn(zeroed[1 + i].data_ptr(), t.data_ptr(), rows, HD, s), "colsum")
+                _lib.count_launch()
+                sums[i] = t.reshape(H, 64).to(dt)
+        return dqkv, dpos[band_off: band_off + R], sums[0], sums[1], None, None, None, None, None, None, None, None
+
+
+def _p(t):
+    return None if t is None else t.data_ptr()
+
+
 def rel_pos_attention_packed(qkv, pos, u, v, pack, *, num_heads: int, head_dim: int, scale: float, dropout_p: float = 0.0):
     """
     :param qkv: [N, H*3*D] bf16, per head grouped (q, k, v)
@@ -198,6 +306,10 @@ def rel_pos_attention_packed(qkv, pos, u, v, pack, *, num_heads: int, head_dim: 
     :param u, v: [H, D] biases (any float dtype) or None
     :return: [N, H*D] bf16
     """
+    if head_dim == 64 and hasattr(_lib.get_lib(), "rb200_rel_flash_fwd"):
+        # the tiles of the fused kernels are one head of 64 columns wide; other head dims take products with a softmax kernel in between
+        return _RelPosFlash.apply(qkv, pos.to(torch.bfloat16), u, v, pack.row_batch, pack.row_pos, pack.lens, pack.batch, num_heads, pack.max_len,
+                                  float(scale), float(dropout_p))
     return _RelPosAttPacked.apply(qkv, pos.to(torch.bfloat16), u, v, pack.row_batch, pack.row_pos, pack.lens, pack.batch, num_heads,
                                   head_dim, pack.max_len, float(scale), float(dropout_p))
 

@@ -1,11 +1,11 @@
 """
-Scaled-dot-product attention (self, causal, cross) on the tcgen05 batched GEMM with a fused mask + softmax + dropout kernel
-between the two products; forward and backward.
+Scaled-dot-product attention (self, causal, cross), forward and backward. Head dim 64: one kernel per pass over the keys
+(``csrc/sdpa_flash.cu``). Other head dims: the tcgen05 batched GEMM with a fused mask + softmax + dropout kernel between the two products.
 
 Inputs are the usual projection outputs viewed as matrices: ``q [B, Tq, H*D]``, ``k, v [B, Tk, H*D]`` (bf16, contiguous); head
 ``h`` is the column block ``h*D .. (h+1)*D``, so no transposition to ``[B, H, T, D]`` is made: the batched GEMM addresses the
-blocks by origin. ``k_lens`` masks padded keys, ``causal`` hides keys after the query position. The scores exist only as
-``[B*H, Tq, Tk]`` buffers (padded to multiples of 64) between the kernels.
+blocks by origin. ``k_lens`` masks padded keys, ``causal`` hides keys after the query position. Only for head dims other
+than 64 do the scores exist as ``[B*H, Tq, Tk]`` buffers (padded to multiples of 64) between the kernels.
 
 Reference semantics: returnn/frontend/_backend.py:1575-1647 (``scaled_dot_product_attention``), used by
 ``rf.SelfAttention``, ``rf.CausalSelfAttention``, ``rf.CrossAttention`` and the Transformer decoder.

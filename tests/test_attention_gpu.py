@@ -77,3 +77,63 @@ def test_rel_pos_attention_dropout_consistent():
     mean = torch.stack(outs).mean(0)
     assert (mean - base).abs().mean() < 0.05
     assert (outs[0] - outs[1]).abs().max() > 1e-3
+
+
+@gpu
+@pytest.mark.parametrize("lens,H,extra", [([1], 1, 0), ([64, 63, 65], 3, 0), ([128, 129, 127, 2], 2, 5), ([512, 300], 1, 0), ([257, 256], 4, 1)])
+def test_rel_pos_attention_head_dim_64_tile_edges(lens, H, extra):
+    """lengths around the tiles of 64 keys and 128 queries, a position table that is longer than the batch needs"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import attention_native as an, gemm
+
+    torch.manual_seed(len(lens) + H)
+    D = 64
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    L = min(pack.max_len + extra, (pack.max_len + 63) // 64 * 64)
+    qkv = torch.randn(pack.n, H * 3 * D, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    pos = torch.randn(2 * L - 1, H * D, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    u = (torch.randn(H, D, device="cuda") * 0.3).requires_grad_(True)
+    v = (torch.randn(H, D, device="cuda") * 0.3).requires_grad_(True)
+    dy = torch.randn(pack.n, H * D, device="cuda").to(torch.bfloat16)
+    out = an.rel_pos_attention_packed(qkv, pos, u, v, pack, num_heads=H, head_dim=D, scale=0.125)
+    got = [out, *torch.autograd.grad(out, [qkv, pos, u, v], dy)]
+    gemm.check_status()
+    x = [t.detach().double().requires_grad_(True) for t in (qkv, pos, u, v)]
+    ref = _reference(*x, pack, H, D, 0.125)
+    want = [ref, *torch.autograd.grad(ref, x, dy.double())]
+    for a, b in zip(got, want):
+        # bf16 operands, probabilities and score gradients: 2^-9 each
+        assert (a.double() - b).norm() <= 1.2e-2 * b.norm() + 1e-3
+
+
+@gpu
+def test_rel_pos_attention_head_dim_64_dropout_gradients():
+    """with the identity as values the output is the dropped probabilities: they give the mask, which the backward pass has to use as well"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import attention_native as an
+    from returnn_b200.ops.elementwise import _seed_tensor
+
+    torch.manual_seed(3)
+    T, H, D, p = 64, 2, 64, 0.25
+    pack = PackInfo(torch.tensor([T], dtype=torch.int32), torch.device("cuda"))
+    qkv = torch.randn(T, H, 3, D, device="cuda").to(torch.bfloat16)
+    pos = torch.randn(2 * T - 1, H * D, device="cuda").to(torch.bfloat16)
+    eye = qkv.clone()
+    eye[:, :, 2] = torch.eye(T, device="cuda", dtype=torch.bfloat16)[:, None]
+    seed = _seed_tensor(qkv.device)
+    state = seed.clone()
+    run = lambda x, ps: an.rel_pos_attention_packed(x.reshape(T, -1), ps, None, None, pack, num_heads=H, head_dim=D, scale=0.125, dropout_p=p)  # noqa: E731
+    mask = (run(eye, pos).view(T, H, T).transpose(0, 1) > 0).double()
+    assert abs(mask.mean().item() - (1 - p)) < 0.03
+    seed.copy_(state)
+    x, ps = qkv.clone().requires_grad_(True), pos.clone().requires_grad_(True)
+    dy = torch.randn(T, H * D, device="cuda").to(torch.bfloat16)
+    got = torch.autograd.grad(run(x, ps), [x, ps], dy)
+    xr, pr = qkv.double().requires_grad_(True), pos.double().requires_grad_(True)
+    q, k, v = (xr[:, :, i].transpose(0, 1) for i in range(3))
+    band = q @ pr.view(-1, H, D).permute(1, 2, 0)
+    at = torch.arange(T, device="cuda")
+    s = (q @ k.transpose(1, 2) + torch.gather(band, 2, (at[None] - at[:, None] + T - 1).expand(H, T, T))) * 0.125
+    out = ((torch.softmax(s, -1) * mask / (1 - p)) @ v).transpose(0, 1).reshape(T, -1)
+    for a, b in zip(got, torch.autograd.grad(out, [xr, pr], dy.double())):
+        assert (a.double() - b).norm() <= 1.2e-2 * b.norm()
