@@ -17,6 +17,7 @@ __device__ __forceinline__ float score_f(__nv_bfloat16 x) { return __bfloat162fl
 
 constexpr int kMaxPerLane = 16;  // 32 lanes * 16 = 512 keys
 
+template <typename I>  // index type: 32 bits where the groups fit (the division is a large part of these copies)
 __global__ void __launch_bounds__(256)
 att_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ u, const float* __restrict__ v,
                    const int* __restrict__ row_batch, const int* __restrict__ row_pos, __nv_bfloat16* __restrict__ qu,
@@ -27,10 +28,10 @@ att_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restric
   // one thread per 8 consecutive elements of one of q/k/v of one head of one row
   const int groups_per_part = dim / 8;
   const int groups_per_row = heads * 3 * groups_per_part;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (long long)n_rows * groups_per_row) return;
-  const int row = (int)(gid / groups_per_row);
-  int g = (int)(gid % groups_per_row);
+  const I gid = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (I)n_rows * (I)groups_per_row) return;
+  const int row = (int)(gid / (I)groups_per_row);
+  int g = (int)(gid % (I)groups_per_row);
   const int h = g / (3 * groups_per_part);
   g -= h * 3 * groups_per_part;
   const int part = g / groups_per_part;
@@ -375,6 +376,7 @@ att_redrop_kernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict
   }
 }
 
+template <typename I>  // index type: 32 bits where the groups fit (the division is a large part of these copies)
 __global__ void __launch_bounds__(256)
 att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16* __restrict__ dqv, const __nv_bfloat16* __restrict__ dk,
                      const __nv_bfloat16* __restrict__ dv, const int* __restrict__ row_batch, const int* __restrict__ row_pos,
@@ -383,10 +385,10 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
   rb_pdl_launch();
   const int groups_per_part = dim / 8;
   const int groups_per_row = heads * 3 * groups_per_part;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (long long)n_rows * groups_per_row) return;
-  const int row = (int)(gid / groups_per_row);
-  int g = (int)(gid % groups_per_row);
+  const I gid = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (I)n_rows * (I)groups_per_row) return;
+  const int row = (int)(gid / (I)groups_per_row);
+  int g = (int)(gid % (I)groups_per_row);
   const int h = g / (3 * groups_per_part);
   g -= h * 3 * groups_per_part;
   const int part = g / groups_per_part;
@@ -407,16 +409,17 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
 }
 
 // rows [B*Lp, HD] padded <-> packed [N, HD]
+template <typename I>  // index type: 32 bits where the groups fit (the division is a large part of these copies)
 __global__ void __launch_bounds__(256)
 att_rows_gather_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, const int* __restrict__ row_batch,
                        const int* __restrict__ row_pos, int n_rows, int width, int lp, int to_padded) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
   const int groups = width / 8;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (long long)n_rows * groups) return;
-  const int row = (int)(gid / groups);
-  const int c0 = (int)(gid % groups) * 8;
+  const I gid = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (I)n_rows * (I)groups) return;
+  const int row = (int)(gid / (I)groups);
+  const int c0 = (int)(gid % (I)groups) * 8;
   const long long padded = ((long long)row_batch[row] * lp + row_pos[row]) * width + c0;
   const long long packed = (long long)row * width + c0;
   if (to_padded) store8(dst, padded, load8(src, packed, 1), 1);
@@ -433,7 +436,7 @@ RB_EXPORT int rb200_att_prepare(const void* qkv, const float* u, const float* v,
     return RB_ERR_ARG;
   }
   long long total = (long long)n_rows * heads * 3 * (dim / 8);
-  rb_launch_pdl(att_prepare_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, 
+  rb_launch_pdl(total < (1LL << 31) ? att_prepare_kernel<uint32_t> : att_prepare_kernel<unsigned long long>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, 
       (const __nv_bfloat16*)qkv, u, v, row_batch, row_pos, (__nv_bfloat16*)qu, (__nv_bfloat16*)qv, (__nv_bfloat16*)k, (__nv_bfloat16*)vv,
       n_rows, heads, dim, lp);
   return rb_check_launch("att_prepare");
@@ -496,7 +499,7 @@ RB_EXPORT int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* 
                                   void* dqkv, int n_rows, int heads, int dim, int lp, cudaStream_t stream) {
   if (n_rows <= 0) return RB_OK;
   long long total = (long long)n_rows * heads * 3 * (dim / 8);
-  rb_launch_pdl(att_pack_dqkv_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, 
+  rb_launch_pdl(total < (1LL << 31) ? att_pack_dqkv_kernel<uint32_t> : att_pack_dqkv_kernel<unsigned long long>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, 
       (const __nv_bfloat16*)dqu, (const __nv_bfloat16*)dqv, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, row_batch, row_pos,
       (__nv_bfloat16*)dqkv, n_rows, heads, dim, lp);
   return rb_check_launch("att_pack_dqkv");
@@ -507,7 +510,7 @@ RB_EXPORT int rb200_att_rows_gather(const void* src, void* dst, const int* row_b
   if (n_rows <= 0) return RB_OK;
   if (width % 8) return RB_ERR_ARG;
   long long total = (long long)n_rows * (width / 8);
-  rb_launch_pdl(att_rows_gather_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (const __nv_bfloat16*)src, (__nv_bfloat16*)dst, row_batch, row_pos,
+  rb_launch_pdl(total < (1LL << 31) ? att_rows_gather_kernel<uint32_t> : att_rows_gather_kernel<unsigned long long>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (const __nv_bfloat16*)src, (__nv_bfloat16*)dst, row_batch, row_pos,
                                                                               n_rows, width, lp, to_padded);
   return rb_check_launch("att_rows_gather");
 }

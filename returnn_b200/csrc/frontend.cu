@@ -15,6 +15,7 @@ namespace {
 typedef __nv_bfloat16 bf16;
 
 // ---- conv1: x [B, T, F] bf16 (one input channel), w [C, 9] fp32 (kt major, kf minor), bias [C] -> y [B, T, F/2, C] bf16
+template <typename I>
 __global__ void __launch_bounds__(256)
 conv1_relu_pool_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, const int* __restrict__ lens,
                            int B, int T, int F, int C, bf16* __restrict__ y) {
@@ -23,13 +24,13 @@ conv1_relu_pool_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__
   for (int i = threadIdx.x; i < C; i += blockDim.x) sw[C * 9 + i] = bias ? bias[i] : 0.f;
   __syncthreads();
   const int Fp = F / 2, G = C / 8;
-  const long long total = (long long)B * T * Fp * G;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    long long r = i / G;
-    const int fp = (int)(r % Fp);
-    r /= Fp;
-    const int t = (int)(r % T), b = (int)(r / T);
+  const I total = (I)((long long)B * T * Fp * G);
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    const int g = (int)(i % (I)G);
+    I r = i / (I)G;
+    const int fp = (int)(r % (I)Fp);
+    r /= (I)Fp;
+    const int t = (int)(r % (I)T), b = (int)(r / (I)T);
     F8 o;
     const int len = lens[b];
     if (t >= len) {
@@ -62,11 +63,12 @@ conv1_relu_pool_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__
         o.v[k] = fmaxf(fmaxf(a0, a1), 0.f);
       }
     }
-    store8(y, i * 8, o, 1);
+    store8(y, (int64_t)i * 8, o, 1);
   }
 }
 
 // gradient of conv1's filter and bias: recompute the two pre-pool activations, route dy to the larger one if positive
+template <typename I>
 __global__ void __launch_bounds__(256)
 conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, const int* __restrict__ lens,
                            const bf16* __restrict__ dy, int B, int T, int F, int C, float* __restrict__ dw, float* __restrict__ dbias) {
@@ -79,8 +81,8 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
   const int Fp = F / 2, G = C / 8;
   // a thread keeps its channel group for all its positions, so its sums stay in registers
   const int g = threadIdx.x % G;
-  const long long positions = (long long)B * T * Fp;
-  const long long stride = (long long)gridDim.x * (blockDim.x / G);
+  const I positions = (I)((long long)B * T * Fp);
+  const I stride = (I)gridDim.x * (blockDim.x / G);
   float gw[8][9], gb[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -88,10 +90,10 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
 #pragma unroll
     for (int j = 0; j < 9; ++j) gw[k][j] = 0.f;
   }
-  for (long long p = (long long)blockIdx.x * (blockDim.x / G) + threadIdx.x / G; p < positions; p += stride) {
-    const int fp = (int)(p % Fp);
-    const long long r = p / Fp;
-    const int t = (int)(r % T), b = (int)(r / T);
+  for (I p = (I)blockIdx.x * (blockDim.x / G) + threadIdx.x / G; p < positions; p += stride) {
+    const int fp = (int)(p % (I)Fp);
+    const I r = p / (I)Fp;
+    const int t = (int)(r % (I)T), b = (int)(r / (I)T);
     const int len = lens[b];
     if (t >= len) continue;
     float in[3][4];
@@ -104,7 +106,7 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
         in[dt][df] = (tt >= 0 && tt < len && ff >= 0 && ff < F) ? __bfloat162float(x[((size_t)b * T + tt) * F + ff]) : 0.f;
       }
     }
-    F8 d = load8(dy, (p * G + g) * 8, 1);
+    F8 d = load8(dy, ((int64_t)p * G + g) * 8, 1);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int c = g * 8 + k;
@@ -146,50 +148,52 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
 // ---- patch gather (forward): x [B, T, F, C] -> col [rows, 9 * C], K order (kt, kf, c).
 // rows = all (b, to, f) of the padded output (row_batch == null, To given), or the valid output frames only (row_batch / row_pos
 // [n_frames], rows = n_frames * F). Input frames >= lens_in[b] read as zero.
+template <typename I>
 __global__ void __launch_bounds__(256)
 im2col_kernel(const bf16* __restrict__ x, const int* __restrict__ lens_in, int T, int F, int C, int stride_t, int pad_t, int To,
               const int* __restrict__ row_batch, const int* __restrict__ row_pos, long long n_out_frames, bf16* __restrict__ col) {
   const int G = C / 8;
-  const long long total = n_out_frames * F * 9 * G;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    long long r = i / G;
-    const int j = (int)(r % 9);
-    r /= 9;
-    const int f = (int)(r % F);
-    const long long fr = r / F;
+  const I total = (I)(n_out_frames * F * 9 * G);
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    const int g = (int)(i % (I)G);
+    I r = i / (I)G;
+    const int j = (int)(r % 9u);
+    r /= 9u;
+    const int f = (int)(r % (I)F);
+    const I fr = r / (I)F;
     int b, to;
     if (row_batch) {
       b = row_batch[fr];
       to = row_pos[fr];
     } else {
-      b = (int)(fr / To);
-      to = (int)(fr % To);
+      b = (int)(fr / (I)To);
+      to = (int)(fr % (I)To);
     }
     const int tt = to * stride_t - pad_t + j / 3;
     const int ff = f - 1 + j % 3;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (tt >= 0 && tt < lens_in[b] && tt < T && ff >= 0 && ff < F) v = *reinterpret_cast<const uint4*>(x + (((size_t)b * T + tt) * F + ff) * C + g * 8);
-    *reinterpret_cast<uint4*>(col + (r * 9 + j) * C + g * 8) = v;
+    *reinterpret_cast<uint4*>(col + ((size_t)r * 9 + j) * C + g * 8) = v;
   }
 }
 
 // ---- transposed patch gather (backward data): dy [out frames, F, Co] -> colT [B * T * F, 9 * Co], K order (kt, kf, co):
 // colT[(b, t, f), (kt, kf, :)] = dy[(b, to, f + 1 - kf), :] with to = (t + pad_t - kt) / stride_t when that division is exact and
 // to < lens_out[b]; rows with t >= lens_in[b] are zero. dy is a padded batch [B, To, F, Co] (cu == null) or packed frames (frame index = cu[b] + to).
+template <typename I>
 __global__ void __launch_bounds__(256)
 im2col_transposed_kernel(const bf16* __restrict__ dy, const int* __restrict__ lens_out, const int* __restrict__ lens_in, const int* __restrict__ cu,
                          int B, int T, int F, int Co, int stride_t, int pad_t, int To, bf16* __restrict__ col) {
   const int G = Co / 8;
-  const long long total = (long long)B * T * F * 9 * G;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    long long r = i / G;
-    const int j = (int)(r % 9);
-    r /= 9;
-    const int f = (int)(r % F);
-    const long long bt = r / F;
-    const int b = (int)(bt / T), t = (int)(bt % T);
+  const I total = (I)((long long)B * T * F * 9 * G);
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    const int g = (int)(i % (I)G);
+    I r = i / (I)G;
+    const int j = (int)(r % 9u);
+    r /= 9u;
+    const int f = (int)(r % (I)F);
+    const I bt = r / (I)F;
+    const int b = (int)(bt / (I)T), t = (int)(bt % (I)T);
     const int num = t + pad_t - j / 3;
     const int fo = f + 1 - j % 3;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -201,7 +205,7 @@ im2col_transposed_kernel(const bf16* __restrict__ dy, const int* __restrict__ le
         v = *reinterpret_cast<const uint4*>(dy + (frame * F + fo) * Co + g * 8);
       }
     }
-    *reinterpret_cast<uint4*>(col + (r * 9 + j) * Co + g * 8) = v;
+    *reinterpret_cast<uint4*>(col + ((size_t)r * 9 + j) * Co + g * 8) = v;
   }
 }
 
@@ -210,17 +214,18 @@ im2col_transposed_kernel(const bf16* __restrict__ dy, const int* __restrict__ le
 // the input position:  dx[(b, t, f), :] = sum_{kt, kf} dcol[(b, to, f + 1 - kf), (kt, kf, :)]  with to = (t + pad_t - kt) / stride_t
 // where exact and to < lens_out[b]; zero for t >= lens_in[b]; optionally times relu'(z). A gather: no atomics, and the matrix
 // product has out-frames rows (the transposed-patch form above has stride_t times more, most of them zeros).
+template <typename I>
 __global__ void __launch_bounds__(256)
 col2im_kernel(const bf16* __restrict__ dcol, const int* __restrict__ lens_out, const int* __restrict__ lens_in, const int* __restrict__ cu, int B,
               int T, int F, int Ci, int stride_t, int pad_t, int To, const bf16* __restrict__ relu_z, bf16* __restrict__ dx) {
   const int G = Ci / 8;
-  const long long total = (long long)B * T * F * G;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    long long r = i / G;  // (b, t, f)
-    const int f = (int)(r % F);
-    const long long bt = r / F;
-    const int b = (int)(bt / T), t = (int)(bt % T);
+  const I total = (I)((long long)B * T * F * G);
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    const int g = (int)(i % (I)G);
+    I r = i / (I)G;  // (b, t, f)
+    const int f = (int)(r % (I)F);
+    const I bt = r / (I)F;
+    const int b = (int)(bt / (I)T), t = (int)(bt % (I)T);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (t < lens_in[b]) {
       const int lo = lens_out[b];
@@ -246,7 +251,7 @@ col2im_kernel(const bf16* __restrict__ dcol, const int* __restrict__ lens_out, c
         }
       }
       if (relu_z) {
-        const uint4 z = *reinterpret_cast<const uint4*>(relu_z + r * Ci + g * 8);
+        const uint4 z = *reinterpret_cast<const uint4*>(relu_z + (size_t)r * Ci + g * 8);
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&z);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -260,9 +265,14 @@ col2im_kernel(const bf16* __restrict__ dcol, const int* __restrict__ lens_out, c
     __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
     for (int q = 0; q < 4; ++q) oh[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-    *reinterpret_cast<uint4*>(dx + r * Ci + g * 8) = o;
+    *reinterpret_cast<uint4*>(dx + (size_t)r * Ci + g * 8) = o;
   }
 }
+
+// The kernels above take an element apart into (batch, time, frequency, channel group) by divisions: with 32-bit indices where the elements
+// (and one stride of the grid past them) fit. In 64 bits the divisions were the time of the patch gathers: 870 MB in 355 us, as many
+// instructions as the memory could have fed three times over.
+bool index32(long long total) { return total < (1LL << 31); }
 
 int grid_for(long long total) {
   long long g = (total + 255) / 256;
@@ -281,7 +291,8 @@ RB_EXPORT int rb200_conv1_relu_pool_fwd(const void* x, const float* w, const flo
     return RB_ERR_UNSUPPORTED;
   }
   const long long total = (long long)B * T * (F / 2) * (C / 8);
-  conv1_relu_pool_fwd_kernel<<<grid_for(total), 256, (size_t)C * 10 * sizeof(float), stream>>>((const bf16*)x, w, bias, lens, B, T, F, C, (bf16*)y);
+  auto kernel = index32(total) ? conv1_relu_pool_fwd_kernel<uint32_t> : conv1_relu_pool_fwd_kernel<unsigned long long>;
+  kernel<<<grid_for(total), 256, (size_t)C * 10 * sizeof(float), stream>>>((const bf16*)x, w, bias, lens, B, T, F, C, (bf16*)y);
   return rb_check_launch("conv1_relu_pool_fwd");
 }
 
@@ -289,7 +300,8 @@ RB_EXPORT int rb200_conv1_relu_pool_bwd(const void* x, const float* w, const flo
                                         float* dw, float* dbias, cudaStream_t stream) {
   if (B <= 0 || T <= 0) return RB_OK;
   if (C % 8 || F % 2 || C > 256 || 256 % (C / 8)) return RB_ERR_UNSUPPORTED;
-  conv1_relu_pool_bwd_kernel<<<148 * 4, 256, (size_t)C * 20 * sizeof(float), stream>>>((const bf16*)x, w, bias, lens, (const bf16*)dy, B, T, F, C, dw,
+  auto kernel = index32((long long)B * T * (F / 2)) ? conv1_relu_pool_bwd_kernel<uint32_t> : conv1_relu_pool_bwd_kernel<unsigned long long>;
+  kernel<<<148 * 4, 256, (size_t)C * 20 * sizeof(float), stream>>>((const bf16*)x, w, bias, lens, (const bf16*)dy, B, T, F, C, dw,
                                                                                       dbias);
   return rb_check_launch("conv1_relu_pool_bwd");
 }
@@ -298,7 +310,9 @@ RB_EXPORT int rb200_im2col_3x3(const void* x, const int* lens_in, int T, int F, 
                                const int* row_pos, long long n_out_frames, void* col, cudaStream_t stream) {
   if (n_out_frames <= 0) return RB_OK;
   if (C % 8) return RB_ERR_UNSUPPORTED;
-  im2col_kernel<<<grid_for(n_out_frames * F * 9 * (C / 8)), 256, 0, stream>>>((const bf16*)x, lens_in, T, F, C, stride_t, pad_t, To, row_batch, row_pos,
+  const long long total = n_out_frames * F * 9 * (C / 8);
+  auto kernel = index32(total) ? im2col_kernel<uint32_t> : im2col_kernel<unsigned long long>;
+  kernel<<<grid_for(total), 256, 0, stream>>>((const bf16*)x, lens_in, T, F, C, stride_t, pad_t, To, row_batch, row_pos,
                                                                                n_out_frames, (bf16*)col);
   return rb_check_launch("im2col_3x3");
 }
@@ -307,7 +321,9 @@ RB_EXPORT int rb200_im2col_3x3_transposed(const void* dy, const int* lens_out, c
                                           int To, void* col, cudaStream_t stream) {
   if (B <= 0 || T <= 0) return RB_OK;
   if (Co % 8) return RB_ERR_UNSUPPORTED;
-  im2col_transposed_kernel<<<grid_for((long long)B * T * F * 9 * (Co / 8)), 256, 0, stream>>>((const bf16*)dy, lens_out, lens_in, cu, B, T, F, Co,
+  const long long total = (long long)B * T * F * 9 * (Co / 8);
+  auto kernel = index32(total) ? im2col_transposed_kernel<uint32_t> : im2col_transposed_kernel<unsigned long long>;
+  kernel<<<grid_for(total), 256, 0, stream>>>((const bf16*)dy, lens_out, lens_in, cu, B, T, F, Co,
                                                                                               stride_t, pad_t, To, (bf16*)col);
   return rb_check_launch("im2col_3x3_transposed");
 }
@@ -317,7 +333,9 @@ RB_EXPORT int rb200_col2im_3x3(const void* dcol, const int* lens_out, const int*
                                int pad_t, int To, const void* relu_z, void* dx, cudaStream_t stream) {
   if (B <= 0 || T <= 0) return RB_OK;
   if (Ci % 8) return RB_ERR_UNSUPPORTED;
-  col2im_kernel<<<grid_for((long long)B * T * F * (Ci / 8)), 256, 0, stream>>>((const bf16*)dcol, lens_out, lens_in, cu, B, T, F, Ci, stride_t, pad_t,
+  const long long total = (long long)B * T * F * (Ci / 8);
+  auto kernel = index32(total) ? col2im_kernel<uint32_t> : col2im_kernel<unsigned long long>;
+  kernel<<<grid_for(total), 256, 0, stream>>>((const bf16*)dcol, lens_out, lens_in, cu, B, T, F, Ci, stride_t, pad_t,
                                                                                 To, (const bf16*)relu_z, (bf16*)dx);
   return rb_check_launch("col2im_3x3");
 }
