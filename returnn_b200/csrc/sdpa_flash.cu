@@ -29,7 +29,7 @@ struct Flash {
   const long long* seed;
   const long long* offset;
   int* status;
-  int heads, tq, tk, causal, shift, tiles, hq, hk, hv, hdo, words, tqp, tkp;
+  int heads, bh, tq, tk, causal, shift, tiles, hq, hk, hv, hdo, words, tqp, tkp;
   float scale, p_drop;
 };
 
@@ -52,8 +52,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
-  const int z = blockIdx.x / p.tiles;
-  const int q0 = (p.tiles - 1 - (int)(blockIdx.x % p.tiles)) * kRows;  // causal: the long rows first
+  // the tiles of all heads side by side, causal the ones with the most keys first: the last wave of CTAs is then made of the short ones
+  const int z = blockIdx.x % p.bh;
+  const int q0 = (p.tiles - 1 - (int)(blockIdx.x / p.bh)) * kRows;
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
   const int row = q0 + tid;
@@ -193,8 +194,8 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
-  const int z = blockIdx.x / p.tiles;
-  const int q0 = (p.tiles - 1 - (int)(blockIdx.x % p.tiles)) * kRows;
+  const int z = blockIdx.x % p.bh;
+  const int q0 = (p.tiles - 1 - (int)(blockIdx.x / p.bh)) * kRows;
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
   const int row = q0 + tid;
@@ -321,8 +322,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
-  const int z = blockIdx.x / p.tiles;
-  const int k0 = (int)(blockIdx.x % p.tiles) * kRows;
+  const int z = blockIdx.x % p.bh;
+  const int k0 = (int)(blockIdx.x / p.bh) * kRows;  // causal: the first keys have the most queries
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
   const int key = k0 + tid;
@@ -464,7 +465,7 @@ Flash make_params(const int* g, const int* k_lens, float* lse, float* delta, voi
                   const long long* offset, int* status) {
   Flash p = {};
   p.k_lens = k_lens; p.lse = lse; p.delta = delta; p.keep = (uint32_t*)keep; p.seed = seed; p.offset = offset; p.status = status;
-  p.heads = g[G_H]; p.tq = g[G_TQ]; p.tk = g[G_TK]; p.causal = g[G_CAUSAL]; p.shift = g[G_SHIFT];
+  p.heads = g[G_H]; p.bh = g[G_B] * g[G_H]; p.tq = g[G_TQ]; p.tk = g[G_TK]; p.causal = g[G_CAUSAL]; p.shift = g[G_SHIFT];
   p.hq = g[G_HQ]; p.hk = g[G_HK]; p.hv = g[G_HV]; p.hdo = g[G_HDO]; p.words = g[G_WORDS]; p.tqp = g[G_TQP]; p.tkp = g[G_TKP];
   p.scale = scale; p.p_drop = p_drop;
   return p;
