@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant__ CUtensorMap tm_qv, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_pos, const __grid_constant__ CUtensorMap tm_o,
                const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dqu, const __grid_constant__ CUtensorMap tm_dqv,
-               const __grid_constant__ CUtensorMap tm_band, const Rel p) {
+               const __grid_constant__ CUtensorMap tm_band, const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_ds,
+               const Rel p) {
   rb_pdl_wait();
   rb_pdl_launch();
   const int z = blockIdx.x / p.tiles;
@@ -262,7 +263,8 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* spos = sv + 2 * kSmall;   // [2][192 positions]
   uint8_t* sds = spos + 6 * kSmall;  // [128 queries][64 keys]
   uint8_t* sdg = sds + kBig;         // [3][128 queries][64 positions]; first the tile of O
-  const Cta c = cta_begin<512, 2>(sdg + 3 * kBig);  // `done`: the products, and the bulk add of the previous iteration has read its tile
+  uint8_t* sp = sdg + 3 * kBig;      // [128 queries][64 keys] dropped probabilities
+  const Cta c = cta_begin<512, 2>(sp + kBig);  // `done`: the products, and the bulk stores of the previous iteration have read their tiles
   const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
   const int row = q0 + r;
   const int n_tiles = (len + 63) / 64;
@@ -377,14 +379,9 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     for (int q = 0; q < 4; ++q) {
       if (!SAVED) pk[q] = make_uint4(pack2(s[8 * q], s[8 * q + 1]), pack2(s[8 * q + 2], s[8 * q + 3]), pack2(s[8 * q + 4], s[8 * q + 5]), pack2(s[8 * q + 6], s[8 * q + 7]));
       dk[q] = make_uint4(pack2(a[8 * q], a[8 * q + 1]), pack2(a[8 * q + 2], a[8 * q + 3]), pack2(a[8 * q + 4], a[8 * q + 5]), pack2(a[8 * q + 6], a[8 * q + 7]));
-      *reinterpret_cast<uint4*>(sds + r * 128 + (((wg * 4 + q) ^ (r & 7)) << 4)) = dk[q];
-    }
-    if (row < len64) {  // the products over queries run in blocks of 64 rows: zeros up to there
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (!SAVED) *reinterpret_cast<uint4*>(p.p + at + 8 * q) = pk[q];
-        *reinterpret_cast<uint4*>(p.ds + at + 8 * q) = dk[q];
-      }
+      const int slot = r * 128 + (((wg * 4 + q) ^ (r & 7)) << 4);
+      *reinterpret_cast<uint4*>(sds + slot) = dk[q];
+      if (!SAVED) *reinterpret_cast<uint4*>(sp + slot) = pk[q];
     }
     // shifted back: key j of the tile lies at column 127 - r + j, the same columns of this row in every iteration
 #pragma unroll
@@ -415,6 +412,13 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
 #pragma unroll
           for (int half = 0; half < 2; ++half)
             if (half * 64 < n_rows_band) tma_reduce_add_2d(&tm_band, x0 + 64 * q, band_row + half * 64, sdg + q * kBig + half * kSmall);
+        // P and dS: the products over queries run in blocks of 64 rows, zeros up to there
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (q0 + half * 64 >= len64) break;
+          tma_store_2d(&tm_ds, it * 64, z * p.lp + q0 + half * 64, sds + half * kSmall);
+          if (!SAVED) tma_store_2d(&tm_p, it * 64, z * p.lp + q0 + half * 64, sp + half * kSmall);
+        }
         tma_store_commit();
         tma_store_wait_read();
         mbar_arrive_local(c.done);
@@ -457,7 +461,7 @@ sum_slices_kernel(const float4* __restrict__ x, uint2* __restrict__ y, int slice
 }
 
 constexpr int kFwdSmem = 12 * kBig + 64 + 1024;
-constexpr int kBwdSmem = 7 * kBig + 10 * kSmall + 64 + 1024;
+constexpr int kBwdSmem = 8 * kBig + 10 * kSmall + 64 + 1024;
 static_assert(kFwdSmem <= 227 * 1024 && kBwdSmem <= 227 * 1024, "shared memory");
 
 // positions [r_rows, HD]: boxes of `box` rows, 64 columns
@@ -525,7 +529,7 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   p.words = 4 * ((lp + 127) / 128);
   int width = 0;
   rb200_rel_flash_band(lp, center, &p.band_off, &width);
-  CUtensorMap a, b, c, d, e, f, g, h, i, j;
+  CUtensorMap a, b, c, d, e, f, g, h, i, j, map_p, map_ds;
   const long long bp = (long long)lp * hd;
   int st = make_map_3d(&a, qu, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&b, qv, hd, lp, batch, hd, bp, kRows);
@@ -537,11 +541,13 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   if (!st) st = make_map_3d(&h, dqu, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&i, dqv, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map(&j, band, width, (long long)heads * batch * lp, width, 64, 64);
+  if (!st) st = make_map(&map_p, pw, lp, (long long)batch * heads * lp, lp, 64, 64);
+  if (!st) st = make_map(&map_ds, ds, lp, (long long)batch * heads * lp, lp, 64, 64);
   if (st) return st;
   auto kernel = p_drop > 0.f ? (w ? rel_bwd_kernel<true, true> : rel_bwd_kernel<true, false>) : (w ? rel_bwd_kernel<false, true> : rel_bwd_kernel<false, false>);
   const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
   if (err != cudaSuccess) return failed("rel_flash_bwd", err);
-  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, p);
+  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, map_p, map_ds, p);
   return rb_check_launch("rel_flash_bwd");
 }
 
