@@ -196,6 +196,7 @@ def test_lstm_input_width_off_the_pitch_rule_and_training_through_the_fallback()
             assert float((g.float() - t.grad).abs().max()) / (float(t.grad.abs().max()) + 1e-6) < 0.06
 
 
+@gpu
 @pytest.mark.parametrize("T,B,H", [(1, 1, 128), (7, 16, 256), (6, 17, 128), (9, 32, 384), (5, 33, 128)])
 def test_blstm_batch_sizes_around_the_row_tiles(T, B, H):
     """16 and 32 rows are the capacities of the two wide forms of the recurrence, 33 takes the narrow one; ragged lengths, initial states"""
