@@ -356,6 +356,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
       const bool vis = j < left;
       float d = dp[j];
       if (SAVED) {
+        d = __bfloat162float(__float2bfloat16(d));  // as the batched product left it
         const uint32_t word = reinterpret_cast<const uint32_t*>(wv)[j >> 1];
         if (DROP) {  // a dropped probability is zero; where the probability itself is, its gradient is too
           const uint32_t kept = reinterpret_cast<const uint32_t*>(wd)[j >> 1];
