@@ -193,7 +193,7 @@ struct Geometry {
   size_t score_elems;  // B * H * Lp * Lp
   size_t band_elems;   // H * B * Lp * Rp
   // head dim 64: one kernel for the score gradients and the query gradients (rel_pos_flash.cu) over a band of its own width. The forward
-  // pass stays with the batched products: its bf16 scores are what a training step is compared by.
+  // pass stays with the batched products: scores that are not rounded to bf16 move the logits of a 12-layer stack as far as bf16 itself does.
   bool fused_bwd;
   int band_w, band_off = 0, slices = 1;  // columns of the backward band, that of position 0, slices of the position gradient's product
   size_t dband_elems;
