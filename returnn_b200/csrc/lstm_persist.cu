@@ -2,15 +2,15 @@
 // keeps the rows of W_rec that produce the four gates of its hidden units in shared memory (forward), or the columns
 // that those units feed (backward), for the whole sequence. Per step a CTA multiplies the small [B, K] activation matrix (read
 // from L2, where the other CTAs wrote it in the previous step) with its resident slice on the tensor cores, applies the cell
-// for its units, publishes its slice of h_t (or dz_t) and meets the other CTAs at a grid barrier. The per-step executor in
-// lstm.cu needs two launches of latency-bound kernels per step (about 22 us); here a step is a barrier plus about 100 KB of L2
-// reads per CTA.
+// for its units, publishes its slice of h_t (or dz_t) and waits for those of the others. The per-step executor in lstm.cu needs two
+// launches of latency-bound kernels per step (about 22 us); here a step of both directions takes 4.2 us forward and 5.4 us backward
+// (16 rows, H = 1024; 17.5 us together with 128 narrow CTAs per direction that met at a counter after storing what the backward pass keeps).
 //
 // The step product has only B <= 48 rows: the warp-level mma (m16n8k16, bf16 -> fp32) fits this shape (three 16-row tiles);
-// a tcgen05 tile is at least 64 rows by one CTA and its operands would have to be re-staged through TMA every step. The eight
+// a tcgen05 tile is at least 64 rows by one CTA and its operands would have to be re-staged through TMA every step. The
 // warps of a CTA split the contraction; their partial sums meet in shared memory.
 //
-// Launched cooperatively (all CTAs resident). Every barrier wait is bounded: a CTA that gives up raises the abort word, all
+// Launched cooperatively (all CTAs resident). Every wait is bounded: a CTA that gives up raises the abort word, all
 // CTAs leave the time loop, and the host reports RB_ERR_TIMEOUT.
 //
 // Semantics, gate order (i, f, g, o), masking and the tensors saved for backward are those of lstm.cu
