@@ -479,7 +479,11 @@ int map_of(CUtensorMap* m, const void* base, const int* g, int t, int row_pitch,
 
 RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse, void* keep, const int* k_lens, const int* g, float scale,
                               float p_drop, const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
-  if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0 || g[G_TK] <= 0) return RB_OK;
+  if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0) return RB_OK;
+  if (g[G_TK] <= 0) {
+    rb_set_error("flash_fwd: no keys for %d queries", g[G_TQ]);
+    return RB_ERR_ARG;
+  }
   Flash p = make_params(g, k_lens, lse, nullptr, keep, scale, p_drop, seed, offset, status);
   p.tiles = (p.tq + kRows - 1) / kRows;
   const long long ctas = (long long)p.tiles * g[G_B] * g[G_H];
@@ -503,7 +507,11 @@ RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void*
 
 RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, void* dq, void* dk, void* dv, float* lse,
                               float* delta, void* keep, const int* k_lens, const int* g, float scale, float p_drop, int* status, cudaStream_t stream) {
-  if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0 || g[G_TK] <= 0) return RB_OK;
+  if (g[G_B] <= 0 || g[G_H] <= 0 || (g[G_TQ] <= 0 && g[G_TK] <= 0)) return RB_OK;
+  if (g[G_TQ] <= 0 || g[G_TK] <= 0) {
+    rb_set_error("flash_bwd: %d queries, %d keys", g[G_TQ], g[G_TK]);
+    return RB_ERR_ARG;
+  }
   Flash p = make_params(g, k_lens, lse, delta, keep, scale, p_drop, nullptr, nullptr, status);
   const int hd = g[G_H] * kTile;
   const int tiles_q = (p.tq + kRows - 1) / kRows, tiles_k = (p.tk + kRows - 1) / kRows;

@@ -138,3 +138,18 @@ def test_sdpa_head_dim_64_dropout_gradients(T):
     torch.testing.assert_close(out.float(), ref, atol=2e-2, rtol=2e-2)
     for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
         assert (got.float() - want).norm() / want.norm() < 1e-2  # bf16 probabilities and results: 2^-9 each per element
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_sdpa_without_keys_or_queries_is_refused(D):
+    """no keys: nothing to attend to; no queries: no gradient of the keys. Both are errors for every head dim, not results without values"""
+    from returnn_b200.ops import sdpa as S
+
+    q, none = torch.zeros(2, 3, 2, D, device="cuda", dtype=torch.bfloat16), torch.zeros(2, 0, 2, D, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        S.sdpa_heads(q, none, none)
+    k, v = q.clone().requires_grad_(True), q.clone().requires_grad_(True)
+    out = S.sdpa_heads(none, k, v)
+    assert out.shape == (2, 0, 2, D)
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(out, [k, v], out.detach())
