@@ -484,6 +484,10 @@ RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void*
     rb_set_error("flash_fwd: no keys for %d queries", g[G_TQ]);
     return RB_ERR_ARG;
   }
+  if (p_drop > 0.f && (!seed || !offset || !keep || !(p_drop < 1.f))) {
+    rb_set_error("flash_fwd: dropout of %f needs seed, offset and a buffer for its decisions, and a rate below 1", p_drop);
+    return RB_ERR_ARG;
+  }
   Flash p = make_params(g, k_lens, lse, nullptr, keep, scale, p_drop, seed, offset, status);
   p.tiles = (p.tq + kRows - 1) / kRows;
   const long long ctas = (long long)p.tiles * g[G_B] * g[G_H];
@@ -510,6 +514,10 @@ RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const
   if (g[G_B] <= 0 || g[G_H] <= 0 || (g[G_TQ] <= 0 && g[G_TK] <= 0)) return RB_OK;
   if (g[G_TQ] <= 0 || g[G_TK] <= 0) {
     rb_set_error("flash_bwd: %d queries, %d keys", g[G_TQ], g[G_TK]);
+    return RB_ERR_ARG;
+  }
+  if (p_drop > 0.f && (!keep || !(p_drop < 1.f))) {
+    rb_set_error("flash_bwd: dropout of %f needs the decisions of the forward pass and a rate below 1", p_drop);
     return RB_ERR_ARG;
   }
   Flash p = make_params(g, k_lens, lse, delta, keep, scale, p_drop, nullptr, nullptr, status);

@@ -153,3 +153,13 @@ def test_sdpa_without_keys_or_queries_is_refused(D):
     assert out.shape == (2, 0, 2, D)
     with pytest.raises(RuntimeError):
         torch.autograd.grad(out, [k, v], out.detach())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("p", [1.0, 1.5])
+def test_sdpa_dropout_rate_of_one_or_more_is_refused(D, p):
+    from returnn_b200.ops import sdpa as S
+
+    q = torch.zeros(1, 3, 2, D, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        S.sdpa_heads(q, q, q, dropout_p=p)
