@@ -12,7 +12,9 @@
 // dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
 // The kernels are bound by the per-row exponentials and that chain, not by memory.
 //
-// Visible keys, dropout and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per score.
+// Visible keys, the dropout rate and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per
+// score. They come from a stream of the generator of their own (tag 0x53; sdpa.cu and attention.cu draw from 0x51, rel_pos_flash.cu from
+// 0x52): the counter here steps in scores, theirs in groups of four, so that on one tag a later site would draw these words again.
 #include "flash.cuh"
 
 using namespace rbf;
@@ -131,7 +133,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
       for (int j = 0; j < 64; j += 4) {
         const uint64_t ctr = base + j;
-        const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x51u, 0u));
+        const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x53u, 0u));
         const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {

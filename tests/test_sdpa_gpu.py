@@ -163,3 +163,24 @@ def test_sdpa_dropout_rate_of_one_or_more_is_refused(D, p):
     q = torch.zeros(1, 3, 2, D, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(RuntimeError):
         S.sdpa_heads(q, q, q, dropout_p=p)
+
+
+def test_sdpa_dropout_streams_of_the_two_forms_are_apart():
+    """
+    the fused kernels (head dim 64) count in scores and the softmax kernels (128) in groups of four: if both drew from one stream, group c of
+    the latter would repeat the decisions of the former at score c. With the identity as values the outputs show the decisions.
+    """
+    from returnn_b200.ops import sdpa as S
+    from returnn_b200.ops.elementwise import _seed_tensor
+
+    dev, p, kept = torch.zeros(1, device="cuda").device, 0.3, {}
+    seed = _seed_tensor(dev)
+    for T in (64, 128):
+        seed[1] = 0  # the same position of the generator for both
+        zero = torch.zeros(1, T, 1, T, device=dev, dtype=torch.bfloat16)
+        eye = torch.eye(T, device=dev, dtype=torch.bfloat16)[None, :, None]
+        kept[T] = (S.sdpa_heads(zero, zero, eye, dropout_p=p)[0, :, 0] > 0).view(-1, 4)
+    n = 64 * 64 // 4
+    same = (kept[64][:n] == kept[128][torch.arange(n, device=dev) * 4]).float().mean().item()
+    # independent decisions agree with probability p^2 + (1-p)^2 = 0.58; 4096 of them scatter by 0.008
+    assert abs(same - (p * p + (1 - p) * (1 - p))) < 0.04
