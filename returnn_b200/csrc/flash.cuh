@@ -40,6 +40,33 @@ __device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float*
   }
 }
 
+// 64 values -> row `row` of two swizzled [rows, 32] fp32 tiles of kBig bytes, one behind the other (columns 0 .. 31 and 32 .. 63)
+__device__ __forceinline__ void store_row64_f32(uint8_t* tile, int row, const float* v) {
+#pragma unroll
+  for (int c = 0; c < 16; ++c)
+    *reinterpret_cast<float4*>(tile + (c >> 3) * kBig + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+
+// product of row `row` of two such fp32 tiles with that of a bf16 tile, both [rows, 64]
+__device__ __forceinline__ float dot_row64(const uint8_t* f32, const uint8_t* bf, int row) {
+  float s = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint4 b = *reinterpret_cast<const uint4*>(bf + row * 128 + ((j ^ (row & 7)) << 4));
+    const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int c = (2 * j + half) & 7;
+      const float4 a = *reinterpret_cast<const float4*>(f32 + (j >> 2) * kBig + row * 128 + ((c ^ (row & 7)) << 4));
+      s = fmaf(a.x, __uint_as_float(w[2 * half] << 16), s);
+      s = fmaf(a.y, __uint_as_float(w[2 * half] & 0xffff0000u), s);
+      s = fmaf(a.z, __uint_as_float(w[2 * half + 1] << 16), s);
+      s = fmaf(a.w, __uint_as_float(w[2 * half + 1] & 0xffff0000u), s);
+    }
+  }
+  return s;
+}
+
 __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
   const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
   float s = 0.f;

@@ -8,7 +8,7 @@
 // A CTA has 128 threads = the 128 lanes of tensor memory: a thread owns one row of the score tile (a query; in flash_bwd_kv a key) and
 // needs no exchange with others for maximum and sum. Thread 0 also issues the TMA loads (two stages) and the tcgen05.mma. The chain load ->
 // product -> softmax -> product of one CTA is serial; three (backward: two) CTAs per SM fill each other's gaps. That is why the tiles are
-// 64 wide: 128 TMEM columns and 66 KB of shared memory per CTA (backward 256 columns and 82 / 98 KB). The two-pass backward (dQ apart from
+// 64 wide: 128 TMEM columns and 67 KB of shared memory per CTA (backward 256 columns and 99 / 102 KB). The two-pass backward (dQ apart from
 // dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
 // The kernels are bound by the per-row exponentials and that chain, not by memory.
 //
@@ -32,6 +32,7 @@ struct Flash {
   const long long* offset;
   int* status;
   int heads, bh, tq, tk, causal, shift, tiles, hq, hk, hv, hdo, words, tqp, tkp;
+  int save;  // (forward) the output is kept in 32 bits for the backward pass
   float scale, p_drop;
 };
 
@@ -44,7 +45,7 @@ __device__ __forceinline__ int visible(const Flash& p, int i, int klen) {
 template <bool DROP>
 __global__ void __launch_bounds__(kThreads, 3)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const __grid_constant__ CUtensorMap tm_o, const Flash p) {
+                 const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_o32, const Flash p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sk = sq + kBig;
@@ -169,11 +170,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int j = 0; j < 64; ++j) acc[j] = n > 0 ? (acc[j] + s[j]) * inv : 0.f;
     }
     store_row64(sq, tid, acc);
+    if (p.save) store_row64_f32(sk, tid, acc);  // the tiles of keys and values are not needed any more
     if (row < p.tq) p.lse[(long long)z * p.tq + row] = n > 0 ? m + __log2f(l) : INFINITY;
     fence_proxy_async_smem();
     __syncthreads();
     if (tid == 0) {
       tma_store_3d(&tm_o, h * kTile, q0, b, sq);
+      if (p.save) {
+        tma_store_3d(&tm_o32, h * kTile, q0, b, sk);
+        tma_store_3d(&tm_o32, h * kTile + 32, q0, b, sk + kBig);
+      }
       tma_store_commit();
       tma_store_wait_all();
     }
@@ -184,15 +190,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 template <bool DROP>
 __global__ void __launch_bounds__(kThreads, 2)
 flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                   const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
+                   const __grid_constant__ CUtensorMap tm_o32, const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
                    const Flash p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sdo = sq + kBig;
   uint8_t* sk = sdo + kBig;
   uint8_t* sv = sk + 2 * kSmall;
-  uint8_t* sds = sv + 2 * kSmall;  // first the tile of O
-  const Cta c = cta_begin<256>(sds + kBig);
+  uint8_t* sds = sv + 2 * kSmall;  // first, with the kBig bytes behind it, the tile of O in 32 bits
+  const Cta c = cta_begin<256>(sds + 2 * kBig);
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
@@ -216,8 +222,9 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
     tma_load_3d(sdo, &tm_do, h * p.hdo, q0, b, &c.full[0]);
     load_kv(0);
-    mbar_expect_tx(c.extra, kBig);
-    tma_load_3d(sds, &tm_o, h * kTile, q0, b, c.extra);
+    mbar_expect_tx(c.extra, 2 * kBig);
+    tma_load_3d(sds, &tm_o32, h * kTile, q0, b, c.extra);
+    tma_load_3d(sds + kBig, &tm_o32, h * kTile + 32, q0, b, c.extra);
     if (n_tiles > 1) {
       mbar_expect_tx(&c.full[1], 2 * kSmall);
       load_kv(1);
@@ -233,11 +240,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (n_tiles > 0) {
     ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 6) && wait_or_abort(c, c.extra, 0, p.status, 6);
     if (ok) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int at = tid * 128 + ((j ^ (tid & 7)) << 4);
-        delta += dot8(*reinterpret_cast<const uint4*>(sds + at), *reinterpret_cast<const uint4*>(sdo + at));
-      }
+      delta = dot_row64(sds, sdo, tid);
       if (row < p.tq) {
         lse = p.lse[(long long)z * p.tq + row];
         p.delta[(long long)z * p.tq + row] = delta;
@@ -452,7 +455,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 }
 
 constexpr int kFwdSmem = 2 * kBig + 4 * kSmall + 64 + 1024;
-constexpr int kBwdQSmem = 3 * kBig + 4 * kSmall + 64 + 1024;
+constexpr int kBwdQSmem = 4 * kBig + 4 * kSmall + 64 + 1024;
 constexpr int kBwdKvSmem = 4 * kBig + 4 * kSmall + 1024 + 2048 + 64 + 1024;
 
 int launch_failed(const char* what, cudaError_t e) {
@@ -479,7 +482,10 @@ int map_of(CUtensorMap* m, const void* base, const int* g, int t, int row_pitch,
 
 }  // namespace
 
-RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse, void* keep, const int* k_lens, const int* g, float scale,
+// o [B, Tq, H * 64] bf16; o32 (null: no backward pass follows) the same in fp32, for the row sums dO . O of the backward pass: from the 16-bit
+// values those are off by 2^-9 of |dO| |O| in one direction for a whole row of dS, which is far more than dS where the values share an offset
+// (512 keys, values 24 + n(0, 1), keys 4 + n(0, 1): error of dQ 3.07, from 32 bits 0.11; a training pass over 250 x 100 x 8 heads 164 -> 176 us)
+RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, void* keep, const int* k_lens, const int* g, float scale,
                               float p_drop, const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
   if (g[G_B] <= 0 || g[G_H] <= 0 || g[G_TQ] <= 0) return RB_OK;
   if (g[G_TK] <= 0) {
@@ -498,20 +504,23 @@ RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void*
     return RB_ERR_ARG;
   }
   const int hd = g[G_H] * kTile;
-  CUtensorMap tq, tk, tv, to;
+  p.save = o32 != nullptr;
+  CUtensorMap tq, tk, tv, to, to32;
   int st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kRows);
   if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kTile);
   if (!st) st = map_of(&tv, v, g, p.tk, g[G_RV], g[G_HV], kTile);
   if (!st) st = map_of(&to, o, g, p.tq, hd, kTile, kRows);
+  to32 = to;
+  if (!st && o32) st = make_map_3d(&to32, o32, hd, p.tq, g[G_B], hd, (long long)p.tq * hd, kRows, true);
   if (st) return st;
   auto kernel = p_drop > 0.f ? flash_fwd_kernel<true> : flash_fwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
   if (e != cudaSuccess) return launch_failed("flash_fwd", e);
-  rb_launch_pdl(kernel, dim3((unsigned)ctas), dim3(kThreads), kFwdSmem, stream, tq, tk, tv, to, p);
+  rb_launch_pdl(kernel, dim3((unsigned)ctas), dim3(kThreads), kFwdSmem, stream, tq, tk, tv, to, to32, p);
   return rb_check_launch("flash_fwd");
 }
 
-RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, void* dq, void* dk, void* dv, float* lse,
+RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const float* o32, const void* d_o, void* dq, void* dk, void* dv, float* lse,
                               float* delta, void* keep, const int* k_lens, const int* g, float scale, float p_drop, int* status, cudaStream_t stream) {
   if (g[G_B] <= 0 || g[G_H] <= 0 || (g[G_TQ] <= 0 && g[G_TK] <= 0)) return RB_OK;
   if (g[G_TQ] <= 0 || g[G_TK] <= 0) {
@@ -534,7 +543,7 @@ RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const
   int st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kRows);
   if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kTile);
   if (!st) st = map_of(&tv, v, g, p.tk, g[G_RV], g[G_HV], kTile);
-  if (!st) st = map_of(&to, o, g, p.tq, hd, kTile, kRows);
+  if (!st) st = make_map_3d(&to, o32, hd, p.tq, g[G_B], hd, (long long)p.tq * hd, kRows, true);
   if (!st) st = map_of(&td, d_o, g, p.tq, g[G_RDO], g[G_HDO], kRows);
   if (!st) st = map_of(&tg, dq, g, p.tq, hd, kTile, kRows);
   if (st) return st;

@@ -165,21 +165,22 @@ inline CUresult encode_in_context(Encode encode) {
 
 // 3-D bf16 tensor map with the 128-byte swizzle: `rows` rows of `inner` contiguous elements, `row_pitch` elements apart, in each of
 // `batch` entries that are `batch_pitch` elements apart; boxes of 64 x box_rows within one entry, so that a tile that reaches past an
-// entry's last row reads zeros and writes nothing there
+// entry's last row reads zeros and writes nothing there (fp32 = true: 4-byte elements, boxes of 32 x box_rows)
 inline int make_map_3d(CUtensorMap* map, const void* base, long long inner, long long rows, long long batch, long long row_pitch,
-                       long long batch_pitch, int box_rows) {
+                       long long batch_pitch, int box_rows, bool fp32 = false) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) {
     rb_set_error("cuTensorMapEncodeTiled not available");
     return RB_ERR_UNSUPPORTED;
   }
   cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)batch};
-  cuuint64_t strides[2] = {(cuuint64_t)row_pitch * 2, (cuuint64_t)batch_pitch * 2};
-  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  const int size = fp32 ? 4 : 2;
+  cuuint64_t strides[2] = {(cuuint64_t)row_pitch * size, (cuuint64_t)batch_pitch * size};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / size), (cuuint32_t)box_rows, 1};
   cuuint32_t elem[3] = {1, 1, 1};
   const CUresult r = encode_in_context([&]() {
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   });
   if (r != CUDA_SUCCESS) {
     rb_set_error("cuTensorMapEncodeTiled failed (%d): base %p inner %lld rows %lld batch %lld pitches %lld %lld", (int)r, base, inner, rows, batch,

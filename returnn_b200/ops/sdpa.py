@@ -173,6 +173,8 @@ class _FlashFn(torch.autograd.Function):
         words = (Tk + 127) // 128 * 4
         o = torch.empty(B, Tq, H, D, dtype=torch.bfloat16, device=dev)
         lse = torch.empty(B * H * Tq, dtype=torch.float32, device=dev)
+        # the backward pass takes row sums of the output: from a copy of its own in 32 bits, so that the caller may change the result in place
+        o32 = torch.empty(B, Tq, H, D, dtype=torch.float32, device=dev) if any(ctx.needs_input_grad[:3]) else None
         drop = p_drop > 0.0
         keep = seed = off = None
         if drop:
@@ -182,17 +184,17 @@ class _FlashFn(torch.autograd.Function):
             seed[1] += B * H * Tqp * Tkp
         geom = (B, H, Tq, Tk, int(causal), Tk - Tq, rq, hq, rk, hk, rv, hv, 0, 0, Tqp, Tkp, words)
         st = _gemm.status_tensor(dev)
-        fn = _lib.bind("rb200_flash_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp, _vp, _vp])
-        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), scale,
-                      p_drop, _p(seed), _p(off), st.data_ptr(), _lib.stream_ptr()), "flash_fwd")
+        fn = _lib.bind("rb200_flash_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp, _vp, _vp])
+        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o.data_ptr(), _p(o32), lse.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom),
+                      scale, p_drop, _p(seed), _p(off), st.data_ptr(), _lib.stream_ptr()), "flash_fwd")
         _lib.count_launch()
-        ctx.save_for_backward(q2, k2, v2, o, lse, keep, k_lens)
+        ctx.save_for_backward(q2, k2, v2, o32, lse, keep, k_lens)
         ctx.geom, ctx.scale, ctx.p_drop, ctx.in_dtype = geom, scale, p_drop, q.dtype
         return o if q.dtype == torch.bfloat16 else o.to(q.dtype)
 
     @staticmethod
     def backward(ctx, d_out):
-        q2, k2, v2, o, lse, keep, k_lens = ctx.saved_tensors
+        q2, k2, v2, o32, lse, keep, k_lens = ctx.saved_tensors
         B, H, Tq, Tk = ctx.geom[:4]
         dev, bf = d_out.device, torch.bfloat16
         do2, rdo, hdo = _rows(d_out)
@@ -203,7 +205,7 @@ class _FlashFn(torch.autograd.Function):
         dv = torch.empty(B, Tk, H, 64, dtype=bf, device=dev)
         st = _gemm.status_tensor(dev)
         fn = _lib.bind("rb200_flash_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp])
-        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o.data_ptr(), do2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o32.data_ptr(), do2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                       lse.data_ptr(), delta.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), ctx.scale, ctx.p_drop, st.data_ptr(),
                       _lib.stream_ptr()), "flash_bwd")
         _lib.count_launch(2)

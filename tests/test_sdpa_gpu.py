@@ -184,3 +184,42 @@ def test_sdpa_dropout_streams_of_the_two_forms_are_apart():
     same = (kept[64][:n] == kept[128][torch.arange(n, device=dev) * 4]).float().mean().item()
     # independent decisions agree with probability p^2 + (1-p)^2 = 0.58; 4096 of them scatter by 0.008
     assert abs(same - (p * p + (1 - p) * (1 - p))) < 0.04
+
+
+def test_sdpa_result_of_the_fused_kernels_may_be_changed_in_place():
+    from returnn_b200.ops import sdpa as S
+
+    torch.manual_seed(4)
+    D = 64
+    q, k, v = (torch.randn(2, 70, 2, D, device="cuda", dtype=torch.bfloat16).requires_grad_(True) for _ in range(3))
+    w = torch.randn(2, 70, 2, D, device="cuda", dtype=torch.bfloat16)
+    want = torch.autograd.grad(S.sdpa_heads(q, k, v), [q, k, v], w * 2)
+    out = S.sdpa_heads(q, k, v)
+    out.mul_(2)
+    for a, b in zip(torch.autograd.grad(out, [q, k, v], w), want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,causal", [(512, False), (300, True)])
+def test_sdpa_query_gradient_where_values_share_an_offset(T, causal):
+    """
+    An offset common to all keys or all values leaves the query gradient as it is: the rows of dS sum to zero. That holds as far as the row
+    sums of P * dP are known, here 24 |dO| = 24 * 8, where dS itself is 8 P. What remains is the 16-bit rounding of the n probabilities in
+    the output, 24 * 8 * 0.0009 / sqrt(n) per row, times the common key 4, against 8 / sqrt(n): 0.09 for every n (row sums from the output
+    in 16 bits: 24 * 8 * 0.0009 * 4 against 8 / sqrt(n), 2 at n = 512).
+    """
+    from returnn_b200.ops import sdpa as S
+
+    torch.manual_seed(6)
+    D = 64
+    dev = torch.device("cuda")
+    q = (torch.randn(1, T, 2, D, device=dev) * 0.02).to(torch.bfloat16)
+    k = (torch.randn(1, T, 2, D, device=dev) + 4).to(torch.bfloat16)
+    v = (torch.randn(1, T, 2, D, device=dev) + 24).to(torch.bfloat16)
+    dy = torch.randn(1, T, 2, D, device=dev, dtype=torch.bfloat16)
+    x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    got = torch.autograd.grad(S.sdpa_heads(*x, causal=causal), x[:1], dy)[0]
+    r = [t.double().requires_grad_(True) for t in (q, k, v)]
+    want = torch.autograd.grad(S.sdpa_reference(*(t.flatten(2) for t in r), num_heads=2, causal=causal), r[:1], dy.float().flatten(2))[0]
+    err = ((got.double() - want).norm() / want.norm()).item()
+    assert err <= 0.2, err
