@@ -408,10 +408,10 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
   store8(dqkv, (long long)row * 3 * hd + (long long)h * 3 * dim + part * dim + d0, x, 1);
 }
 
-// rows [B*Lp, HD] padded <-> packed [N, HD]
-template <typename I>  // index type: 32 bits where the groups fit (the division is a large part of these copies)
+// rows [B*Lp, HD] padded <-> packed [N, HD]; F32: the source rows are fp32
+template <typename I, bool F32>  // index type: 32 bits where the groups fit (the division is a large part of these copies)
 __global__ void __launch_bounds__(256)
-att_rows_gather_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, const int* __restrict__ row_batch,
+att_rows_gather_kernel(const void* __restrict__ src, __nv_bfloat16* __restrict__ dst, const int* __restrict__ row_batch,
                        const int* __restrict__ row_pos, int n_rows, int width, int lp, int to_padded) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
@@ -422,8 +422,8 @@ att_rows_gather_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __r
   const int c0 = (int)(gid % (I)groups) * 8;
   const long long padded = ((long long)row_batch[row] * lp + row_pos[row]) * width + c0;
   const long long packed = (long long)row * width + c0;
-  if (to_padded) store8(dst, padded, load8(src, packed, 1), 1);
-  else store8(dst, packed, load8(src, padded, 1), 1);
+  if (to_padded) store8(dst, padded, load8(src, packed, !F32), 1);
+  else store8(dst, packed, load8(src, padded, !F32), 1);
 }
 
 }  // namespace
@@ -510,7 +510,18 @@ RB_EXPORT int rb200_att_rows_gather(const void* src, void* dst, const int* row_b
   if (n_rows <= 0) return RB_OK;
   if (width % 8) return RB_ERR_ARG;
   long long total = (long long)n_rows * (width / 8);
-  rb_launch_pdl(total < (1LL << 31) ? att_rows_gather_kernel<uint32_t> : att_rows_gather_kernel<unsigned long long>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (const __nv_bfloat16*)src, (__nv_bfloat16*)dst, row_batch, row_pos,
-                                                                              n_rows, width, lp, to_padded);
+  rb_launch_pdl(total < (1LL << 31) ? att_rows_gather_kernel<uint32_t, false> : att_rows_gather_kernel<unsigned long long, false>,
+                dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, src, (__nv_bfloat16*)dst, row_batch, row_pos, n_rows, width, lp, to_padded);
   return rb_check_launch("att_rows_gather");
+}
+
+// padded fp32 rows -> packed bf16 rows
+RB_EXPORT int rb200_att_rows_gather_f32(const float* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp,
+                                        cudaStream_t stream) {
+  if (n_rows <= 0) return RB_OK;
+  if (width % 8) return RB_ERR_ARG;
+  long long total = (long long)n_rows * (width / 8);
+  rb_launch_pdl(total < (1LL << 31) ? att_rows_gather_kernel<uint32_t, true> : att_rows_gather_kernel<unsigned long long, true>,
+                dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (const void*)src, (__nv_bfloat16*)dst, row_batch, row_pos, n_rows, width, lp, 0);
+  return rb_check_launch("att_rows_gather_f32");
 }

@@ -42,8 +42,9 @@ int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* dk, const 
                         int n_rows, int heads, int dim, int lp, cudaStream_t stream);
 int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, int to_padded,
                           cudaStream_t stream);
+int rb200_att_rows_gather_f32(const float* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, cudaStream_t stream);
 int rb200_rel_flash_band(int lp, int center, int* off, int* width);
-int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const void* o, const void* d_o, void* dqu,
+int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o, void* dqu,
                         void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch, int heads,
                         int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream);
 int rb200_rel_flash_slices(long long rows, int width, int heads);
@@ -230,8 +231,8 @@ struct Geometry {
 
 // activations kept from forward to backward, per layer
 struct Saved {
-  bf16 *ln1, *z1, *a1, *x1, *ln2, *qu, *qv, *kk, *vv, *w, *wd, *o_pad, *posp, *att, *x2, *ln3, *g, *y, *zc, *x3, *ln4, *z2, *a2, *x4, *out;
-  float *st1, *st2, *st3, *st4, *st5, *bn_ms;
+  bf16 *ln1, *z1, *a1, *x1, *ln2, *qu, *qv, *kk, *vv, *w, *wd, *posp, *att, *x2, *ln3, *g, *y, *zc, *x3, *ln4, *z2, *a2, *x4, *out;
+  float *st1, *st2, *st3, *st4, *st5, *bn_ms, *o_pad;
 };
 
 struct SavedLayout {
@@ -253,7 +254,7 @@ struct SavedLayout {
     s.w = bump.take<bf16>(g.score_elems);
     // the dropped probabilities are kept too (recomputing them in the backward pass costs a full pass over the scores)
     s.wd = g.keep_wd ? bump.take<bf16>(g.score_elems) : s.w;
-    s.o_pad = bump.take<bf16>(g.fused_bwd ? g.pad_rows * HD : 0);
+    s.o_pad = bump.take<float>(g.fused_bwd ? g.pad_rows * HD : 0);
     s.posp = bump.take<bf16>((size_t)g.R * HD);
     s.att = bump.take<bf16>(n * HD); s.x2 = bump.take<bf16>(n * D);
     s.ln3 = bump.take<bf16>(n * D); s.st3 = bump.take<float>(2 * n);
@@ -575,15 +576,16 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
       const long long o2[10] = {Lp, 0, 0, Dh, 0, 0, 0, Dh, (long long)Lp * Rp, (long long)B * Lp * Rp};
       e.bgemm(sv.qv, sv.posp, t.band, Lp, g.R, Dh, 0, 0, HD, HD, Rp, (long long)B * Lp, HD, g.R, HD, o2, B * H, H, lens, 1, 0, 0, d.att_scale, 0);
     }
-    bf16* o_pad = g.fused_bwd ? sv.o_pad : t.o_pad;
+    void* o_pad = g.fused_bwd ? (void*)sv.o_pad : t.o_pad;  // (the fused backward pass takes it in 32 bits)
     // w and wd need no memset: the softmax kernel zeroes the margin that the GEMMs read beyond each sequence's length
     bf16* wd = p_att > 0.f ? sv.wd : sv.w;
     if (e.ok()) e.run_tagged("att_softmax_fwd_ex", rb200_att_softmax_fwd_ex(t.s_ac, t.band, 1, sv.w, wd, lens, B, H, Lp, Rp, g.center, p_att, seed, lay.att_off + l, stream));
     {
       const long long o3[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(wd, sv.vv, o_pad, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o3, B * H, H, lens, 1, 0, 1, 1.f, 0);
+      e.bgemm(wd, sv.vv, o_pad, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o3, B * H, H, lens, 1, 0, 1, 1.f, g.fused_bwd);
     }
-    if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(o_pad, sv.att, row_batch, row_pos, n, HD, Lp, 0, stream));
+    if (e.ok() && g.fused_bwd) e.run_tagged("att_rows_gather", rb200_att_rows_gather_f32(sv.o_pad, sv.att, row_batch, row_pos, n, HD, Lp, stream));
+    else if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(o_pad, sv.att, row_batch, row_pos, n, HD, Lp, 0, stream));
     e.linear_fwd(sv.att, l, P_PROJ_W, P_PROJ_B, n, HD, D, sv.x2, nullptr, 0, p_res, e.site(l, g.site_att_out), sv.x1, 1.f);
     // ---- convolution module
     e.layer_norm(sv.x2, l, P_CONV_LN_G, sv.ln3, sv.st3);

@@ -67,17 +67,6 @@ __device__ __forceinline__ float dot_row64(const uint8_t* f32, const uint8_t* bf
   return s;
 }
 
-__device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
-  const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
-  float s = 0.f;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    s = fmaf(__uint_as_float(x[e] << 16), __uint_as_float(y[e] << 16), s);
-    s = fmaf(__uint_as_float(x[e] & 0xffff0000u), __uint_as_float(y[e] & 0xffff0000u), s);
-  }
-  return s;
-}
-
 // D[128, 64] (+)= A[128, 64] B: A K-major; B K-major [n, k] or, `b_mn`, stored [k, n]
 template <bool B_MN>
 __device__ __forceinline__ void mma64(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {

@@ -224,13 +224,14 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
       const float inv = 1.f / l;
 #pragma unroll
       for (int j = 0; j < 64; ++j) acc[j] = row < len ? (acc[j] * e0 + ex[j] * e1) * inv : 0.f;
-      store_row64(squ, r, acc);
+      store_row64_f32(squ, r, acc);  // (over both query tiles)
       if (row < len) p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
     }
     fence_proxy_async_smem();
     __syncthreads();
     if (tid == 0) {
       tma_store_3d(&tm_o, h * 64, q0, b, squ);
+      tma_store_3d(&tm_o, h * 64 + 32, q0, b, squ + kBig);
       tma_store_commit();
       tma_store_wait_all();
     }
@@ -262,7 +263,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* sv = sk + 2 * kSmall;     // [2][64 keys]
   uint8_t* spos = sv + 2 * kSmall;   // [2][192 positions]
   uint8_t* sds = spos + 6 * kSmall;  // [128 queries][64 keys]
-  uint8_t* sdg = sds + kBig;         // [3][128 queries][64 positions]; first the tile of O
+  uint8_t* sdg = sds + kBig;         // [3][128 queries][64 positions]; first the tile of O in 32 bits
   uint8_t* sp = sdg + 3 * kBig;      // [128 queries][64 keys] dropped probabilities
   const Cta c = cta_begin<512, 2>(sp + kBig);  // `done`: the products, and the bulk stores of the previous iteration have read their tiles
   const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
@@ -292,8 +293,9 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
     tma_load_3d(sdo, &tm_do, h * 64, q0, b, &c.full[0]);
     load(0);
-    mbar_expect_tx(c.extra, kBig);
+    mbar_expect_tx(c.extra, 2 * kBig);
     tma_load_3d(sdg, &tm_o, h * 64, q0, b, c.extra);
+    tma_load_3d(sdg + kBig, &tm_o, h * 64 + 32, q0, b, c.extra);
     if (n_tiles > 1) {
       mbar_expect_tx(&c.full[1], 5 * kSmall);
       load(1);
@@ -308,11 +310,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   float lse = INFINITY, delta = 0.f;
   ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 26) && wait_or_abort(c, c.extra, 0, p.status, 26);
   if (ok) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int at = r * 128 + ((j ^ (r & 7)) << 4);
-      delta += dot8(*reinterpret_cast<const uint4*>(sdg + at), *reinterpret_cast<const uint4*>(sdo + at));
-    }
+    delta = dot_row64(sdg, sdo, r);
     if (!SAVED && row < len) lse = p.lse[(long long)z * p.lp + row];
   }
   __syncthreads();
@@ -356,7 +354,6 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
       const bool vis = j < left;
       float d = dp[j];
       if (SAVED) {
-        d = __bfloat162float(__float2bfloat16(d));  // as the batched product left it
         const uint32_t word = reinterpret_cast<const uint32_t*>(wv)[j >> 1];
         if (DROP) {  // a dropped probability is zero; where the probability itself is, its gradient is too
           const uint32_t kept = reinterpret_cast<const uint32_t*>(wd)[j >> 1];
@@ -475,9 +472,11 @@ int failed(const char* what, cudaError_t e) {
 
 }  // namespace
 
-// qu, qv, k, v, o: bf16 [B, Lp, H*64] (rows past a sequence's length zero, those of o unspecified); pos [R, H*64]; keep words per row:
-// 4 * ceil(Lp / 128); lse [B*H, Lp]
-RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, void* o, float* lse, void* keep,
+// qu, qv, k, v: bf16 [B, Lp, H*64], rows past a sequence's length zero; pos [R, H*64]; keep words per row: 4 * ceil(Lp / 128); lse [B*H, Lp];
+// o: fp32 [B, Lp, H*64], rows past a sequence's length unspecified. In 32 bits because the row sums dO . O of the backward pass are taken from
+// it: the rounding of 16-bit values would be the same for a whole row of dS, which is far more than dS where the values share an offset
+// (300 frames, values 24 + n(0, 1), keys 4 + n(0, 1): error of dQ 2.40, from 32 bits 0.12, as from the sums over P * dP; a training pass 398 -> 401 us at 36 x 333 x 8 heads)
+RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, float* o, float* lse, void* keep,
                                   const int* lens, int batch, int heads, int lp, int r_rows, int center, float scale, float p_drop,
                                   const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
   if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
@@ -494,7 +493,7 @@ RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k,
   if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 128);
   if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 128);
   if (!st) st = map_pos(&e, pos, r_rows, hd, 256);
-  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows, true);
   if (st) return st;
   auto kernel = p_drop > 0.f ? rel_fwd_kernel<true> : rel_fwd_kernel<false>;
   const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
@@ -518,7 +517,7 @@ RB_EXPORT int rb200_rel_flash_band(int lp, int center, int* off, int* width) {
 // dqu, dqv [B, Lp, H*64] and band [H, B, Lp, band_width] zeroed by the caller; pw, ds [B*H, Lp, Lp]: written for the first
 // 64 * ceil(len / 64) rows and columns of each sequence. With saved probabilities `w` (else null; lse and keep are not read then) pw is read:
 // the dropped probabilities, or anything without dropout
-RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const void* o, const void* d_o,
+RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
                                   void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
                                   int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
   if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
@@ -537,7 +536,7 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 64);
   if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 64);
   if (!st) st = map_pos(&e, pos, r_rows, hd, 192);
-  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows);
+  if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows, true);
   if (!st) st = make_map_3d(&g, d_o, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&h, dqu, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&i, dqv, hd, lp, batch, hd, bp, kRows);

@@ -215,7 +215,7 @@ class _RelPosFlash(torch.autograd.Function):
         s = _lib.stream_ptr()
         fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
         _lib.check(fn(qkv.data_ptr(), _p(uf), _p(vf), row_batch.data_ptr(), row_pos.data_ptr(), qu, qv, kk, vv, N, H, 64, Lp, s), "att_prepare")
-        o_pad = torch.empty(B * Lp, HD, dtype=bf, device=dev)
+        o_pad = torch.empty(B * Lp, HD, dtype=torch.float32, device=dev)  # (the backward pass takes row sums of it)
         lse = torch.empty(B * H * Lp, dtype=torch.float32, device=dev)
         drop = p_drop > 0.0
         keep = seed = off = None
@@ -229,8 +229,8 @@ class _RelPosFlash(torch.autograd.Function):
         _lib.check(fn(qu, qv, kk, vv, pos.data_ptr(), o_pad.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp, R, center, scale, p_drop,
                       _p(seed), _p(off), st.data_ptr(), s), "rel_flash_fwd")
         out = torch.empty(N, HD, dtype=bf, device=dev)
-        fn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 0, s), "att_gather")
+        fn = _lib.bind("rb200_att_rows_gather_f32", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        _lib.check(fn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, s), "att_gather")
         _lib.count_launch(3)
         ctx.save_for_backward(pads, pos, o_pad, lse, keep, row_batch, row_pos, lens)
         ctx.dims = (B, H, Lp, R, center, N, scale, p_drop)

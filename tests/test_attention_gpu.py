@@ -137,3 +137,84 @@ def test_rel_pos_attention_head_dim_64_dropout_gradients():
     out = ((torch.softmax(s, -1) * mask / (1 - p)) @ v).transpose(0, 1).reshape(T, -1)
     for a, b in zip(got, torch.autograd.grad(out, [xr, pr], dy.double())):
         assert (a.double() - b).norm() <= 1.2e-2 * b.norm()
+
+
+@gpu
+def test_rel_pos_attention_query_gradient_where_values_share_an_offset():
+    """
+    An offset common to all keys or all values leaves the query gradient as it is, as far as the row sums of P * dP are known: here
+    24 |dO| = 24 * 8, where dS itself is 8 P. What remains is the 16-bit rounding of the n probabilities in the output,
+    24 * 8 * 0.0009 / sqrt(n) per row, times the common key 4, against 8 / sqrt(n): 0.09 (row sums from the output in 16 bits: 1 to 2).
+    """
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import attention_native as an
+
+    torch.manual_seed(8)
+    T, H, D = 300, 2, 64
+    pack = PackInfo(torch.tensor([T], dtype=torch.int32), torch.device("cuda"))
+    qkv = torch.randn(T, H, 3, D, device="cuda") * torch.tensor([0.02, 1.0, 1.0], device="cuda")[:, None]
+    qkv = (qkv + torch.tensor([0.0, 4.0, 24.0], device="cuda")[:, None]).to(torch.bfloat16).reshape(T, -1)
+    pos = (torch.randn(2 * T - 1, H * D, device="cuda") * 0.02).to(torch.bfloat16)
+    u = torch.zeros(H, D, device="cuda")
+    dy = torch.randn(T, H * D, device="cuda").to(torch.bfloat16)
+    x = qkv.clone().requires_grad_(True)
+    got = torch.autograd.grad(an.rel_pos_attention_packed(x, pos, u, u, pack, num_heads=H, head_dim=D, scale=0.125), x, dy)[0]
+    xr = qkv.double().requires_grad_(True)
+    want = torch.autograd.grad(_reference(xr, pos.double(), u.double(), u.double(), pack, H, D, 0.125), xr, dy.double())[0]
+    got, want = (t.double().view(T, H, 3, D)[:, :, 0] for t in (got, want))
+    assert (got - want).norm() <= 0.2 * want.norm(), ((got - want).norm() / want.norm()).item()
+
+
+@gpu
+@pytest.mark.parametrize("lens,H,p", [([150, 192, 40], 2, 0.0), ([150, 192, 40], 2, 0.25), ([321, 257], 1, 0.1), ([64, 1], 3, 0.1)])
+def test_rel_flash_bwd_on_saved_probabilities(lens, H, p):
+    """
+    the form of the backward kernel that the encoder executor takes: probabilities, dropped probabilities and output as a forward pass left
+    them; the score gradients, both query gradients and the band against the definition in 64 bits
+    """
+    import ctypes
+    from returnn_b200.ops import _lib, gemm as G
+
+    torch.manual_seed(len(lens) + H)
+    dev, B, L = "cuda", len(lens), max(lens)
+    Lp, HD, scale = (L + 63) // 64 * 64, H * 64, 0.125
+    R = 2 * L - 1
+    bf = lambda *s: torch.randn(*s, device=dev).to(torch.bfloat16)  # noqa: E731
+    valid = (torch.arange(Lp, device=dev)[None] < torch.tensor(lens, device=dev)[:, None])
+    qu, qv, k, v, do = (bf(B, Lp, HD) * valid[:, :, None] for _ in range(5))
+    pos = bf(R, HD)
+    heads = lambda t: t.view(B, -1, H, 64).transpose(1, 2).double()  # noqa: E731
+    ok = valid[:, None, :, None] & valid[:, None, None, :]
+    at = torch.arange(Lp, device=dev)
+    rel = L - 1 + at[None] - at[:, None]  # position row of (query, key)
+    inside = (rel >= 0) & (rel < R)
+    posh = pos.view(R, H, 64).transpose(0, 1).double()
+    s = heads(qu) @ heads(k).transpose(2, 3)
+    s = s + torch.gather(heads(qv) @ posh.transpose(1, 2), 3, rel.clamp(0, R - 1).expand(B, H, Lp, Lp))
+    w = torch.nan_to_num(torch.softmax((s * scale).masked_fill(~ok, float("-inf")), -1)).to(torch.bfloat16)
+    keep = (torch.rand(B, H, Lp, Lp, device=dev) >= p).double()
+    wd = (w.double() * keep / (1 - p)).to(torch.bfloat16)
+    o = (wd.double() @ heads(v)).transpose(1, 2).reshape(B, Lp, HD).float()
+    # the definition
+    dp = heads(do) @ heads(v).transpose(2, 3) * keep / (1 - p)
+    ds = w.double() * (dp - (heads(do) * heads(o)).sum(-1, keepdim=True))
+    dqu = ds @ heads(k) * scale
+    band = torch.zeros(B, H, Lp, R, device=dev, dtype=torch.float64).scatter_add(3, rel.clamp(0, R - 1).expand(B, H, Lp, Lp), ds * inside)
+    dqv = band @ posh * scale
+    # the kernel
+    geo = (ctypes.c_int * 2)()
+    vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    _lib.check(_lib.bind("rb200_rel_flash_band", [i32, i32, vp, vp])(Lp, L - 1, ctypes.addressof(geo), ctypes.addressof(geo) + 4), "band")
+    got_qu, got_qv = (torch.zeros(B, Lp, HD, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    got_band = torch.zeros(H, B, Lp, geo[1], device=dev, dtype=torch.bfloat16)
+    got_ds = torch.zeros(B, H, Lp, Lp, device=dev, dtype=torch.bfloat16)
+    lens_t = torch.tensor(lens, dtype=torch.int32, device=dev)
+    fn = _lib.bind("rb200_rel_flash_bwd", [vp] * 16 + [i32] * 5 + [f32, f32, vp, vp])
+    _lib.check(fn(qu.data_ptr(), qv.data_ptr(), k.data_ptr(), v.data_ptr(), pos.data_ptr(), o.data_ptr(), do.data_ptr(), got_qu.data_ptr(),
+                  got_qv.data_ptr(), w.data_ptr(), wd.data_ptr(), got_ds.data_ptr(), got_band.data_ptr(), None, None, lens_t.data_ptr(), B, H, Lp, R, L - 1,
+                  scale, p, G.status_tensor(lens_t.device).data_ptr(), _lib.stream_ptr()), "rel_flash_bwd")
+    G.check_status()
+    unheads = lambda t: t.transpose(1, 2).reshape(B, Lp, HD)  # noqa: E731
+    for got, want in ((got_ds, ds), (got_band[..., geo[0]: geo[0] + R].transpose(0, 1), band), (got_qu, unheads(dqu)), (got_qv, unheads(dqv))):
+        # dS is rounded to bf16 (2^-9), the query gradients once more
+        assert (got.double() - want).norm() <= 2 * 2 ** -9 * want.norm() + 1e-6
