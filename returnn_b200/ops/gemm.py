@@ -156,11 +156,12 @@ def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], d
 
 class _LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x2, weight, bias, act):
+    def forward(ctx, x2, weight, bias, act, differentiable):
         w = weight.to(torch.bfloat16).contiguous()
         m, k = x2.shape
         n = w.shape[1]
-        need_z = act is not None and (x2.requires_grad or weight.requires_grad)
+        # (a parameter says that it requires a gradient under no_grad as well)
+        need_z = act is not None and differentiable and (x2.requires_grad or weight.requires_grad)
         if need_z:
             z, y = gemm(x2, w, m=m, n=n, k=k, a_mn_major=False, b_mn_major=True, bias=bias, act=act, want_act_output=True)
         else:
@@ -193,7 +194,7 @@ class _LinearFn(torch.autograd.Function):
                 dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out=torch.zeros(k, n, dtype=torch.float32, device=dy.device), atomic=True)
             else:
                 dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True).to(ctx.w_dtype)
-        return dx, dw, db.to(ctx.bias_dtype) if db is not None else None, None
+        return dx, dw, db.to(ctx.bias_dtype) if db is not None else None, None, None
 
 
 class _ArenaLinearFn(torch.autograd.Function):
@@ -365,5 +366,5 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     x2 = x.reshape(-1, x.shape[-1])
     if not x2.is_contiguous():
         x2 = x2.contiguous()
-    y = _LinearFn.apply(x2, weight, bias, activation)
+    y = _LinearFn.apply(x2, weight, bias, activation, torch.is_grad_enabled())
     return y.reshape(*x.shape[:-1], weight.shape[1])

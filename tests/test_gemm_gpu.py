@@ -213,3 +213,25 @@ def test_split_operand_product_keeps_fp32_precision(m, n, k):
     want = torch.as_strided(x, (m, k), (step, 1)).double() @ t.double()
     # 22 mantissa bits per factor, fp32 sums over k
     assert (out.double() - want).norm() <= 4e-6 * want.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_linear_leaves_no_pre_activation_where_no_gradient_is_wanted(monkeypatch, dtype):
+    """the pre-activation is a second output of the product for the backward pass only (CPU: the product replaced)"""
+    from returnn_b200.ops import gemm as G
+
+    second = []
+
+    def product(a, b, *, m, n, want_act_output=False, **_kwargs):
+        second.append(want_act_output)
+        y = a.new_zeros(m, n)
+        return (y, y.clone()) if want_act_output else y
+
+    monkeypatch.setattr(G, "gemm", product)
+    x, w = torch.zeros(3, 8, dtype=torch.bfloat16), torch.zeros(8, 16, dtype=dtype, requires_grad=True)
+    with torch.no_grad():
+        G.linear_bf16(x, w, None, "silu")
+    G.linear_bf16(x, w.detach(), None, "silu")
+    G.linear_bf16(x, w, None, None)
+    assert G.linear_bf16(x, w, None, "silu").requires_grad
+    assert second == [False, False, False, True]
