@@ -287,10 +287,8 @@ class _RelPosFlash(torch.autograd.Function):
         sums = [None, None]
         for i, dt in enumerate((ctx.u_dtype, ctx.v_dtype)):
             if dt is not None:
-                t = torch.zeros(HD, dtype=torch.float32, device=dev)
-                fn = _lib.bind("rb200_colsum_bf16", [_vp, _vp, _i32, _i32, _vp])
-                _lib.check(fn(zeroed[1 + i].data_ptr(), t.data_ptr(), rows, HD, s), "colsum")
-                _lib.count_launch()
+                t = torch.empty(HD, dtype=torch.float32, device=dev)
+                _gemm._grad_pre(zeroed[1 + i], None, None, t)
                 sums[i] = t.reshape(H, 64).to(dt)
         return dqkv, dpos[band_off: band_off + R], sums[0], sums[1], None, None, None, None, None, None, None, None
 

@@ -131,9 +131,10 @@ def _act_grad(z: torch.Tensor, dy: torch.Tensor, act: str) -> torch.Tensor:
     raise ValueError(act)
 
 
-def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], db: Optional[torch.Tensor]) -> torch.Tensor:
+def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], db: Optional[torch.Tensor], accumulate: bool = False) -> torch.Tensor:
     """
-    gradient before the activation, ``dy * act'(z)``, with its column sums added to ``db`` (fp32, None: not wanted), in one kernel
+    gradient before the activation, ``dy * act'(z)``, with its column sums in ``db`` (fp32, None: not wanted): the same in every run, or with
+    ``accumulate`` added to what is there, in any order
 
     :param dy: [m, n] bf16, contiguous
     """
@@ -143,14 +144,22 @@ def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], d
     # 16-byte accesses: a gradient that starts off that alignment takes the elementwise form
     if dy.dtype == torch.bfloat16 and n % 8 == 0 and dy.data_ptr() % 16 == 0 and (z is None or z.data_ptr() % 16 == 0):
         dz = torch.empty_like(dy) if act is not None else dy
-        fn = _lib.bind("rb200_act_grad_colsum", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        work = None
+        if db is not None and not accumulate:
+            words = _lib.bind("rb200_act_grad_colsum_work", [_i32, _i32])
+            work = torch.empty(words(m, n), dtype=torch.float32, device=dy.device)
+        fn = _lib.bind("rb200_act_grad_colsum", [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
         _lib.check(fn(z.data_ptr() if act is not None else None, dy.data_ptr(), dz.data_ptr() if act is not None else None,
-                      db.data_ptr() if db is not None else None, m, n, _ACT[act], _lib.stream_ptr()), "act_grad_colsum")
-        _lib.count_launch()
+                      db.data_ptr() if db is not None else None, work.data_ptr() if work is not None else None, m, n, _ACT[act],
+                      _lib.stream_ptr()), "act_grad_colsum")
+        _lib.count_launch(1 if work is None else 2)
         return dz
     dz = _act_grad(z, dy, act) if act is not None else dy
     if db is not None:
-        db += dz.float().sum(dim=0)
+        if accumulate:
+            db += dz.float().sum(dim=0)
+        else:
+            torch.sum(dz.float(), dim=0, out=db)
     return dz
 
 
@@ -181,7 +190,7 @@ class _LinearFn(torch.autograd.Function):
         dy = dy.contiguous()
         dx = dw = db = None
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = torch.zeros(n, dtype=torch.float32, device=dy.device)
+            db = torch.empty(n, dtype=torch.float32, device=dy.device)
         dy = _grad_pre(dy, z, ctx.act, db)
         if ctx.needs_input_grad[0]:
             # dX[m,k] = dY[m,n] · W[k,n]^T : contraction over n, W rows are contiguous in n -> "K-major" B
@@ -222,7 +231,7 @@ class _ArenaLinearFn(torch.autograd.Function):
         m, k = x2.shape
         n = w16.shape[1]
         dy = dy.contiguous()
-        dy = _grad_pre(dy, z, ctx.act, ctx.gb32)
+        dy = _grad_pre(dy, z, ctx.act, ctx.gb32, accumulate=True)
         dx = gemm(dy, w16, m=m, n=k, k=n, a_mn_major=False, b_mn_major=False) if ctx.needs_input_grad[0] else None
         if ctx.gw32 is not None:
             gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out=ctx.gw32, atomic=True)

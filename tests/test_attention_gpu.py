@@ -218,3 +218,19 @@ def test_rel_flash_bwd_on_saved_probabilities(lens, H, p):
     for got, want in ((got_ds, ds), (got_band[..., geo[0]: geo[0] + R].transpose(0, 1), band), (got_qu, unheads(dqu)), (got_qv, unheads(dqv))):
         # dS is rounded to bf16 (2^-9), the query gradients once more
         assert (got.double() - want).norm() <= 2 * 2 ** -9 * want.norm() + 1e-6
+
+
+@gpu
+def test_rel_pos_attention_gradients_are_the_same_in_every_run():
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import attention_native as an
+
+    torch.manual_seed(2)
+    H, D = 4, 64
+    pack = PackInfo(torch.tensor([300, 257, 40] * 4, dtype=torch.int32), torch.device("cuda"))
+    x = [torch.randn(*s, device="cuda").to(dt).requires_grad_(True) for s, dt in (
+        ((pack.n, H * 3 * D), torch.bfloat16), ((599, H * D), torch.bfloat16), ((H, D), torch.float32), ((H, D), torch.float32))]
+    dy = torch.randn(pack.n, H * D, device="cuda").to(torch.bfloat16)
+    runs = [torch.autograd.grad(an.rel_pos_attention_packed(*x, pack, num_heads=H, head_dim=D, scale=0.125), x, dy) for _ in range(8)]
+    for r in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(r, runs[0]))

@@ -235,3 +235,19 @@ def test_linear_leaves_no_pre_activation_where_no_gradient_is_wanted(monkeypatch
     G.linear_bf16(x, w, None, None)
     assert G.linear_bf16(x, w, None, "silu").requires_grad
     assert second == [False, False, False, True]
+
+
+@gpu
+@pytest.mark.parametrize("m,k,n,act", [(5000, 64, 1032, "silu"), (6656, 512, 512, None), (700, 512, 64, "relu")])
+def test_linear_gradients_are_the_same_in_every_run(m, k, n, act):
+    """without an arena no gradient is a sum of atomic adds, whose order differs from run to run"""
+    from returnn_b200.ops.linear import linear
+
+    torch.manual_seed(n)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    w = (torch.randn(k, n, device="cuda") * 0.1).requires_grad_(True)
+    b = torch.randn(n, device="cuda").requires_grad_(True)
+    dy = torch.randn(m, n, device="cuda").to(torch.bfloat16)
+    runs = [torch.autograd.grad(linear(x, w, b, act), [x, b], dy) for _ in range(8)]
+    for r in runs[1:]:
+        assert all(torch.equal(a, c) for a, c in zip(r, runs[0]))
