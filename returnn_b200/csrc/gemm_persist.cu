@@ -363,3 +363,23 @@ RB_EXPORT int rb200_gemm_fp16_split(const void* a, const void* b, void* c, int m
   }
   return rb_gemm(g, stream);
 }
+
+RB_EXPORT int rb200_sum_slices_f32(const float* x, float* y, int slices, long long n, cudaStream_t stream);
+
+// dw [k][n] (fp32) = x^T dy, x [m][k], dy [m][n] bf16: one product per slice of `rows` rows into part [ceil(m / rows)][k][n], then their sum in
+// the order of the slices
+RB_EXPORT int rb200_weight_grad_sliced(const void* x, const void* dy, float* part, float* dw, int m, int k, int n, int rows, int* status,
+                                       cudaStream_t stream) {
+  if (m <= 0 || rows <= 0) {
+    rb_set_error("weight_grad_sliced: m=%d rows=%d", m, rows);
+    return RB_ERR_ARG;
+  }
+  RbGemm g;
+  g.a = x; g.b = dy; g.c = part; g.m = k; g.n = n; g.k = rows; g.lda = k; g.ldb = n; g.ldc = n;
+  g.a_mn_major = 1; g.b_mn_major = 1; g.out_fp32 = 1; g.status = status;
+  g.batch = (m + rows - 1) / rows; g.heads = 1;
+  g.a_rb = rows; g.b_rb = rows; g.c_sb = (long long)k * n;
+  g.a_rows = m; g.a_cols = k; g.b_rows = m; g.b_cols = n;
+  const int st = rb_gemm(g, stream);
+  return st ? st : rb200_sum_slices_f32(part, dw, g.batch, (long long)k * n, stream);
+}

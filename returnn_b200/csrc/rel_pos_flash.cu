@@ -443,9 +443,13 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   cta_end<512>(c);
 }
 
-// sum of the slices of a split product, fp32 [slices][n] -> bf16 [n], n a multiple of 4
+// sum of the slices of a split product in their order, fp32 [slices][n] -> bf16 or fp32 [n], n a multiple of 4
+__device__ __forceinline__ void store4(uint2* y, const float4& s) { *y = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w)); }
+__device__ __forceinline__ void store4(float4* y, const float4& s) { *y = s; }
+
+template <typename Out>
 __global__ void __launch_bounds__(256)
-sum_slices_kernel(const float4* __restrict__ x, uint2* __restrict__ y, int slices, long long n4) {
+sum_slices_kernel(const float4* __restrict__ x, Out* __restrict__ y, int slices, long long n4) {
   rb_pdl_wait();
   rb_pdl_launch();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -455,7 +459,18 @@ sum_slices_kernel(const float4* __restrict__ x, uint2* __restrict__ y, int slice
     const float4 v = x[k * n4 + i];
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
   }
-  y[i] = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+  store4(y + i, s);
+}
+
+template <typename Out>
+int sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream) {
+  if (n <= 0 || slices <= 0) return RB_OK;
+  if (n % 4) {
+    rb_set_error("sum_slices: n=%lld must be a multiple of 4", n);
+    return RB_ERR_ARG;
+  }
+  rb_launch_pdl(sum_slices_kernel<Out>, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float4*)x, (Out*)y, slices, n / 4);
+  return rb_check_launch("sum_slices");
 }
 
 constexpr int kFwdSmem = 12 * kBig + 64 + 1024;
@@ -562,12 +577,7 @@ RB_EXPORT int rb200_rel_flash_slices(long long rows, int width, int heads) {
   return n > 1 ? (int)n : 1;
 }
 
-RB_EXPORT int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream) {
-  if (n <= 0 || slices <= 0) return RB_OK;
-  if (n % 4) {
-    rb_set_error("sum_slices: n=%lld must be a multiple of 4", n);
-    return RB_ERR_ARG;
-  }
-  rb_launch_pdl(sum_slices_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float4*)x, (uint2*)y, slices, n / 4);
-  return rb_check_launch("sum_slices");
+RB_EXPORT int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream) { return sum_slices<uint2>(x, y, slices, n, stream); }
+RB_EXPORT int rb200_sum_slices_f32(const float* x, float* y, int slices, long long n, cudaStream_t stream) {
+  return sum_slices<float4>(x, y, slices, n, stream);
 }

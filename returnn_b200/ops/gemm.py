@@ -163,6 +163,35 @@ def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], d
     return dz
 
 
+def _weight_grad(x: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
+    """
+    ``x^T dy`` in fp32, the same in every run: where the result has few tiles and the contraction is long, it is cut into slices of the rows
+    whose products are added in their order.
+
+    :param x: [m, k] bf16
+    :param dy: [m, n] bf16
+    :return: [k, n]
+    """
+    (m, k), n = x.shape, dy.shape[1]
+    # One CTA per tile of 128 x 256 and slice, all of them at once; at least 256 rows per slice (shorter ones gain less than the sum of the
+    # slices costs); no more than 12, from where the slices that are written and read again cost more than shorter products save.
+    # 6656 x 512 x 512: 12 slices 16 us, one 42; 25000 x 512 x 512: 26 and 138; 6656 x 512 x 2048: 4 slices 24 us, one 43 (slices that add
+    # onto one result by atomics, in any order: 13, 19 and 21 us); 600 x 512 x 512: 2 slices 12.5, one 11.2
+    tiles = -(-k // 128) * -(-n // 256)
+    slices = min(148 // tiles, 12, m // 256)
+    if slices <= 1:
+        return gemm(x, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out_dtype=torch.float32)
+    rows = (-(-m // slices) + 63) // 64 * 64  # (rows past the last one are read as zeros)
+    slices = -(-m // rows)
+    part = torch.empty(slices, k, n, dtype=torch.float32, device=x.device)
+    dw = torch.empty(k, n, dtype=torch.float32, device=x.device)
+    fn = _lib.bind("rb200_weight_grad_sliced", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp])
+    _lib.check(fn(x.data_ptr(), dy.data_ptr(), part.data_ptr(), dw.data_ptr(), m, k, n, rows, status_tensor(x.device).data_ptr(), _lib.stream_ptr()),
+               "weight_grad_sliced")
+    _lib.count_launch(2)
+    return dw
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x2, weight, bias, act, differentiable):
@@ -198,9 +227,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             # dW[k,n] = X[m,k]^T · dY[m,n] : contraction over m, both operands contiguous in their output dim
             if ctx.w_dtype == torch.float32:
-                # few output tiles and a long contraction: the sum over the rows is split over the SMs into the fp32 gradient of the
-                # fp32 weight (one slice per tile is the plain product)
-                dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out=torch.zeros(k, n, dtype=torch.float32, device=dy.device), atomic=True)
+                dw = _weight_grad(x2, dy)
             else:
                 dw = gemm(x2, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True).to(ctx.w_dtype)
         return dx, dw, db.to(ctx.bias_dtype) if db is not None else None, None, None

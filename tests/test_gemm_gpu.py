@@ -238,7 +238,8 @@ def test_linear_leaves_no_pre_activation_where_no_gradient_is_wanted(monkeypatch
 
 
 @gpu
-@pytest.mark.parametrize("m,k,n,act", [(5000, 64, 1032, "silu"), (6656, 512, 512, None), (700, 512, 64, "relu")])
+@pytest.mark.parametrize("m,k,n,act", [(5000, 64, 1032, "silu"), (6656, 512, 512, None), (700, 512, 64, "relu"), (513, 136, 264, None),
+                                        (3073, 8, 72, "silu"), (1000, 512, 10000, None)])
 def test_linear_gradients_are_the_same_in_every_run(m, k, n, act):
     """without an arena no gradient is a sum of atomic adds, whose order differs from run to run"""
     from returnn_b200.ops.linear import linear
@@ -248,6 +249,10 @@ def test_linear_gradients_are_the_same_in_every_run(m, k, n, act):
     w = (torch.randn(k, n, device="cuda") * 0.1).requires_grad_(True)
     b = torch.randn(n, device="cuda").requires_grad_(True)
     dy = torch.randn(m, n, device="cuda").to(torch.bfloat16)
-    runs = [torch.autograd.grad(linear(x, w, b, act), [x, b], dy) for _ in range(8)]
+    runs = [torch.autograd.grad(linear(x, w, b, act), [x, w, b], dy) for _ in range(8)]
     for r in runs[1:]:
         assert all(torch.equal(a, c) for a, c in zip(r, runs[0]))
+    if act is None:  # (else dy is rounded on its way)
+        # sums of m products in fp32, in slices that do not divide the rows too
+        want = x.detach().double().t() @ dy.double()
+        assert (runs[0][1].double() - want).norm() <= 2e-5 * want.norm()
