@@ -122,11 +122,8 @@ int colsum_splits(int rows, int cols) {
 
 }  // namespace
 
-// words of workspace for ordered column sums
-RB_EXPORT int rb200_act_grad_colsum_work(int rows, int cols) { return colsum_splits(rows, cols) * cols; }
-
 // act: 0 none (dz unused), 1 relu, 2 silu, 3 gelu; cols a multiple of 8, 16-byte aligned rows. db (may be null): with work
-// (rb200_act_grad_colsum_work words) written, in an order of its own; without added to, by atomics
+// (4 * 148 * 64 + cols words, the most that colsum_splits * cols comes to) written, the sums in order; without added to, by atomics
 RB_EXPORT int rb200_act_grad_colsum(const void* z, const void* dy, void* dz, float* db, float* work, int rows, int cols, int act, cudaStream_t stream) {
   if (cols <= 0 || (!db && act == 0) || (rows <= 0 && !(db && work))) return RB_OK;
   if (cols % 8 || act < 0 || act > 3) {

@@ -146,8 +146,7 @@ def _grad_pre(dy: torch.Tensor, z: Optional[torch.Tensor], act: Optional[str], d
         dz = torch.empty_like(dy) if act is not None else dy
         work = None
         if db is not None and not accumulate:
-            words = _lib.bind("rb200_act_grad_colsum_work", [_i32, _i32])
-            work = torch.empty(words(m, n), dtype=torch.float32, device=dy.device)
+            work = torch.empty(4 * 148 * 64 + n, dtype=torch.float32, device=dy.device)
         fn = _lib.bind("rb200_act_grad_colsum", [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
         _lib.check(fn(z.data_ptr() if act is not None else None, dy.data_ptr(), dz.data_ptr() if act is not None else None,
                       db.data_ptr() if db is not None else None, work.data_ptr() if work is not None else None, m, n, _ACT[act],
