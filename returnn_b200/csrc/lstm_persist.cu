@@ -57,20 +57,37 @@ __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
 // step number into its own flag word (no atomic: adds of all CTAs onto one counter are served one after the other), does what the others
 // need not wait for, and then waits for all flags, one thread per flag. Only the exchanged slice is stored before the announcement, so the
 // fence in it does not wait for the tensors that are kept for the backward pass.
-__device__ __forceinline__ void barrier_arrive(uint32_t* flags, int cta, uint32_t step) {
+// Narrow form with more than kFlagCtas CTAs (H > 512): all CTAs add onto one counter instead, and one thread of each looks at it with pauses.
+// 128 threads in each of up to 256 CTAs that read flags all the time take the issue slots of the other CTA of their SM and the L2 requests of
+// the operand loads: H = 1024, T = 100, one direction, 16 rows, forward 760 us with flags, 566 with the counter; both directions, 33 rows,
+// training 3409 and 2480. Up to 64 CTAs the flags are ahead: one direction, H = 512, 16 rows, forward 428 and 460.
+constexpr int kFlagCtas = 64;
+
+template <typename S>
+__device__ __forceinline__ bool counts(int n_cta) {
+  return S::U == 8 && n_cta > kFlagCtas;
+}
+
+template <typename S>
+__device__ __forceinline__ void barrier_arrive(uint32_t* flags, int cta, int n_cta, uint32_t step) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flags + cta), "r"(step) : "memory");
+    if (counts<S>(n_cta)) atomicAdd(flags, 1u);
+    else asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flags + cta), "r"(step) : "memory");
   }
 }
 // false (for every thread of every CTA, eventually) when someone timed out
+template <typename S>
 __device__ __forceinline__ bool barrier_wait(uint32_t* flags, int n_cta, uint32_t step, int* abort_word, int* status) {
+  const bool count = counts<S>(n_cta);
+  const uint32_t target = count ? step * (uint32_t)n_cta : step;
   int ok = 1;
-  if ((int)threadIdx.x < n_cta) {
+  if ((int)threadIdx.x < (count ? 1 : n_cta)) {
     uint32_t spins = 0;
-    while ((int32_t)(ld_relaxed_gpu(flags + threadIdx.x) - step) < 0) {
+    while ((int32_t)(ld_relaxed_gpu(flags + threadIdx.x) - target) < 0) {
       ++spins;
+      if (count) __nanosleep(64);
       if (spins > kSpinLimit || ((spins & 255u) == 0 && *reinterpret_cast<volatile int*>(abort_word))) {
         ok = 0;
         atomicExch(abort_word, 1);
@@ -219,7 +236,7 @@ struct FwdArgs {
   float *h_final, *c_final;
   bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state
   uint32_t* hx;         // wide form: [2,B,H] words (step << 16 | bf16 h), zeroed before the launch
-  uint32_t* flags;      // one word per CTA, zeroed before the launch
+  uint32_t* flags;      // one word per CTA (or the counter), zeroed before the launch
   int* abort_word;      // zeroed before the launch
   int* status;          // receives (5 << 24) | cta when a barrier wait ran out
 };
@@ -431,9 +448,9 @@ __device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const 
     }
   };
   uint32_t n_bar = 1;
-  barrier_arrive(p.flags, cta, n_bar);
+  barrier_arrive<S>(p.flags, cta, n_cta, n_bar);
   if (p.T > 0) fetch_zin(p.reverse ? p.T - 1 : 0);
-  bool ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);
+  bool ok = barrier_wait<S>(p.flags, n_cta, n_bar, p.abort_word, p.status);
   for (int s = 0; s < p.T && ok; ++s) {
     const int t = p.reverse ? p.T - 1 - s : s;
     const bf16* h_cur = p.hbuf + (size_t)(s & 1) * B * H;
@@ -460,7 +477,7 @@ __device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const 
       }
       h_nxt[(size_t)b * H + j0 + u] = __float2bfloat16(hst[i]);
     }
-    barrier_arrive(p.flags, cta, ++n_bar);
+    barrier_arrive<S>(p.flags, cta, n_cta, ++n_bar);
     if (s + 1 < p.T) fetch_zin(p.reverse ? p.T - 2 - s : s + 1);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -475,7 +492,7 @@ __device__ __forceinline__ void fwd_body(const FwdArgs& p, const int cta, const 
 #pragma unroll
       for (int q = 0; q < 4; ++q) p.gates[zo + (size_t)q * H] = __float2bfloat16(gates[i][q]);
     }
-    ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);
+    ok = barrier_wait<S>(p.flags, n_cta, n_bar, p.abort_word, p.status);
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -600,11 +617,11 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const 
       dcs[i] = dc * gf;
       dhs[i] = 0.f;
     }
-    barrier_arrive(p.flags, cta, ++n_bar);
+    barrier_arrive<S>(p.flags, cta, n_cta, ++n_bar);
 #pragma unroll
     for (int i = 0; i < N; ++i) c_t[i] = c_p[i];
     if (s > 0) fetch(s - 1);
-    ok = barrier_wait(p.flags, n_cta, n_bar, p.abort_word, p.status);  // all slices of dz_t are written
+    ok = barrier_wait<S>(p.flags, n_cta, n_bar, p.abort_word, p.status);  // all slices of dz_t are written
     if (!ok) break;
     step_matmul<S, U, S::PrefetchBwd>(dz_t, B, K, Wt, red);
     __syncthreads();
@@ -762,7 +779,9 @@ bool pair_fits(int H) {
 
 enum { kNoPair = 0, kNarrow = 1, kWide1 = 2, kWide2 = 3 };
 
-// the shape that runs a bidirectional layer
+// The shape that runs a bidirectional layer. Training, T = 100, wide / narrow, us (at H = 1024 the narrow form is timed with the counter of 33
+// rows): H = 1024: 1 row 1130 / 2150, 16: 1360 / 2410, 17: 1800 / 2490, 32: 2110 / 2705; H = 512: 850 / 1114, 930 / 1250, 1170 / 1293,
+// 1355 / 1420. At H <= 256 the forms are within 7 % of each other with 17 to 32 rows (256, 32 rows: 1155 / 1100), and the wide one is ahead below.
 int pair_shape(int T, int B, int H) {
   if (!rb_lstm_persist_supported(T, B, H)) return kNoPair;
   if (B <= 16 && pair_fits<Wide1>(H)) return kWide1;

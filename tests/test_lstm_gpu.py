@@ -221,3 +221,33 @@ def test_blstm_batch_sizes_around_the_row_tiles(T, B, H):
     for a, b in zip([t for d in got for t in d] + list(g), [t for d in ref for t in d] + list(r)):
         # bf16 operands, states and gates: 2^-9 per factor, a few of them per step
         assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-4
+
+
+@gpu
+@pytest.mark.parametrize("both", [False, True])
+@pytest.mark.parametrize("T,B,H", [(6, 34, 512), (7, 40, 640), (9, 48, 1024), (2, 1, 1152)])
+def test_recurrence_around_the_number_of_ctas_that_meet_at_flags(T, B, H, both):
+    """8 units per CTA: 64 CTAs (512 units) still announce by flags of their own, more of them by one counter; one and both directions"""
+    from returnn_b200.ops import lstm as L, gemm
+
+    torch.manual_seed(H)
+    dev, I = "cuda", 32
+    x = (torch.randn(T, B, I, device=dev) * 0.5).requires_grad_(True)
+    par = [(torch.randn(*s, device=dev) * s[-1] ** -0.5).requires_grad_(True) for s in ((4 * H, I), (4 * H, H), (4 * H,)) * 2]
+    st = [(torch.randn(B, H, device=dev) * 0.3).requires_grad_(True) for _ in range(4)]
+    lens = torch.randint(1, T + 1, (B,), dtype=torch.int32)
+    w = torch.randn(2, T, B, H, device=dev)
+
+    def run(one):
+        return [one(x, lens, *par[3 * d: 3 * d + 3], st[2 * d], st[2 * d + 1], reverse=d == 1) for d in range(2)]
+
+    def gradients(dirs):
+        return torch.autograd.grad(sum((y.float() * w[d]).sum() + h.sum() - c.sum() for d, (y, h, c) in enumerate(dirs)), [x, *par, *st])
+
+    got = list(L.blstm(x, lens, tuple(par[:3]), tuple(par[3:]), *st)) if both else run(L.lstm)
+    g = gradients(got)
+    gemm.check_status()
+    ref = run(L.lstm_reference)
+    for a, b in zip([t for d in got for t in d] + list(g), [t for d in ref for t in d] + list(gradients(ref))):
+        # bf16 operands, states and gates: 2^-9 per factor, a few of them per step
+        assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-4
