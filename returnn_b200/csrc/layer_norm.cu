@@ -367,10 +367,10 @@ ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const float tg = __ldcg(dgamma + i), tb = __ldcg(dbeta + i);
     if (w_bf16) {
-      reinterpret_cast<__nv_bfloat16*>(gamma_out)[i] = __float2bfloat16(tg);
+      if (gamma_out) reinterpret_cast<__nv_bfloat16*>(gamma_out)[i] = __float2bfloat16(tg);
       if (beta_out) reinterpret_cast<__nv_bfloat16*>(beta_out)[i] = __float2bfloat16(tb);
     } else {
-      reinterpret_cast<float*>(gamma_out)[i] = tg;
+      if (gamma_out) reinterpret_cast<float*>(gamma_out)[i] = tg;
       if (beta_out) reinterpret_cast<float*>(beta_out)[i] = tb;
     }
   }
@@ -430,7 +430,6 @@ RB_EXPORT int rb200_layer_norm_fwd(const void* x, const void* gamma, const void*
   return rb_check_launch("layer_norm_fwd");
 }
 
-// dres (optional, same layout as dx): added to dx; accumulate: dgamma / dbeta += instead of =
 // one-kernel form (bf16 rows of at most 512 columns): dgamma / dbeta are added to; with `done` (a zeroed counter) the last CTA also writes them
 // as gamma_out / beta_out in the type of the parameters
 static int ln_bwd_acc(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta,
@@ -461,6 +460,7 @@ rb_launch_pdl(ln_bwd_acc_kernel<C>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, str
   return rb_check_launch("layer_norm_bwd_acc");
 }
 
+// dres (optional, same layout as dx): added to dx; accumulate: dgamma / dbeta += instead of =
 RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                                       void* dx, float* part, float* dgamma, float* dbeta, long long rows, int n, int n_part,
                                       int x_bf16, int w_bf16, int rms, const void* dres, int accumulate, cudaStream_t stream) {
@@ -490,7 +490,7 @@ RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void*
   return rb_check_launch("layer_norm_bwd_reduce");
 }
 
-// bf16 rows of n <= 512 columns (a multiple of 8): dx, and dgamma / dbeta (may be null) in the type of gamma. work: 2 n + 1 words
+// bf16 rows of n <= 512 columns (a multiple of 8): dx, and dgamma / dbeta (either may be null) in the type of gamma. work: 2 n + 1 words
 RB_EXPORT int rb200_layer_norm_bwd_typed(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* work,
                                          void* dgamma, void* dbeta, long long rows, int n, int w_bf16, int rms, cudaStream_t stream) {
   if (n % 8 != 0 || n <= 0 || n > 512 || rows <= 0) {

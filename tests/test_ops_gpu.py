@@ -368,3 +368,34 @@ def test_linear_with_output_width_off_the_pitch_rule_runs_on_the_own_gemm():
     torch.testing.assert_close(y.float(), ref, atol=0.05, rtol=0.02)
     for a, r in zip(got, (xf.grad, wf.grad, bf_.grad)):
         assert float((a - r).abs().max()) / (float(r.abs().max()) + 1e-6) < 0.02
+
+
+@gpu
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("skip", ["gamma", "beta"])
+def test_layer_norm_backward_entry_without_one_of_the_parameter_gradients(w_dtype, skip):
+    """the entry that leaves typed gradients takes a null pointer for either of them"""
+    import ctypes
+    from returnn_b200.ops import _lib
+
+    torch.manual_seed(0)
+    rows, n = 37, 264
+    x, dy = (torch.randn(rows, n, device="cuda").to(torch.bfloat16) for _ in range(2))
+    gamma = torch.rand(n, device="cuda").to(w_dtype) + 0.5
+    mean, rstd = x.float().mean(-1), (x.float().var(-1, unbiased=False) + 1e-6).rsqrt()
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    fn = _lib.bind("rb200_layer_norm_bwd_typed", [vp] * 9 + [ctypes.c_longlong, i32, i32, i32, vp])
+
+    def call(gamma_out, beta_out):
+        dx, work = torch.empty_like(x), torch.empty(2 * n + 1, device="cuda")
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        _lib.check(fn(ptr(x), ptr(dy), ptr(gamma), ptr(mean), ptr(rstd), ptr(dx), ptr(work), ptr(gamma_out), ptr(beta_out), rows, n,
+                      1 if w_dtype == torch.bfloat16 else 0, 0, _lib.stream_ptr()), "layer_norm_bwd_typed")
+        return dx
+
+    both = [torch.empty_like(gamma), torch.empty_like(gamma)]
+    want = call(*both)
+    one = torch.empty_like(gamma)
+    assert torch.equal(call(*((None, one) if skip == "gamma" else (one, None))), want)
+    # (sums of 37 rows by atomics: fp32 rounding in another order)
+    torch.testing.assert_close(one, both[1 if skip == "gamma" else 0], atol=1e-4, rtol=1e-2)
