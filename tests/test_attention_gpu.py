@@ -234,3 +234,46 @@ def test_rel_pos_attention_gradients_are_the_same_in_every_run():
     runs = [torch.autograd.grad(an.rel_pos_attention_packed(*x, pack, num_heads=H, head_dim=D, scale=0.125), x, dy) for _ in range(8)]
     for r in runs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(r, runs[0]))
+
+
+@gpu
+@pytest.mark.parametrize("D,T", [(64, 270), (64, 150), (128, 200)])
+def test_rel_pos_attention_dropout_gradients_over_several_tiles(D, T):
+    """the decisions of all tiles, read out block by block: with the identity on a block of keys as values the output is the kept probabilities"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import attention_native as an
+    from returnn_b200.ops.elementwise import _seed_tensor
+
+    torch.manual_seed(9)
+    H, p = 2, 0.2
+    lens = [T, 40]
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    qkv = (torch.randn(pack.n, H, 3, D, device="cuda") * 0.7).to(torch.bfloat16)
+    pos = (torch.randn(2 * T - 1, H * D, device="cuda") * 0.7).to(torch.bfloat16)
+    seed = _seed_tensor(qkv.device)
+    state = seed.clone()
+
+    def run(x, ps):
+        seed.copy_(state)
+        return an.rel_pos_attention_packed(x.reshape(pack.n, -1), ps, None, None, pack, num_heads=H, head_dim=D, scale=D ** -0.5, dropout_p=p)
+
+    mask = torch.zeros(H, T, T, device="cuda", dtype=torch.float64)
+    for j in range(0, T, D):
+        x, n = qkv.clone(), min(D, T - j)
+        x[:, :, 2] = 0
+        x[j: j + n, :, 2, :n] = torch.eye(n, device="cuda", dtype=torch.bfloat16)[:, None]
+        mask[..., j: j + n] = (run(x, pos)[:T].view(T, H, D)[..., :n] > 0).transpose(0, 1).double()
+    assert abs(mask.mean().item() - (1 - p)) < 0.02
+    x, ps = qkv.clone().requires_grad_(True), pos.clone().requires_grad_(True)
+    dy = torch.randn(pack.n, H * D, device="cuda").to(torch.bfloat16)
+    dy[T:] = 0  # (the second sequence only shares the launch)
+    got = torch.autograd.grad(run(x, ps), [x, ps], dy)
+    xr, pr = qkv[:T].double().requires_grad_(True), pos.double().requires_grad_(True)
+    q, k, v = (xr[:, :, i].transpose(0, 1) for i in range(3))
+    band = q @ pr.view(-1, H, D).permute(1, 2, 0)
+    at = torch.arange(T, device="cuda")
+    s = (q @ k.transpose(1, 2) + torch.gather(band, 2, (at[None] - at[:, None] + T - 1).expand(H, T, T))) * D ** -0.5
+    out = ((torch.softmax(s, -1) * mask / (1 - p)) @ v).transpose(0, 1).reshape(T, -1)
+    for a, b in zip((got[0][:T], got[1]), torch.autograd.grad(out, [xr, pr], dy[:T].double())):
+        assert (a.double() - b).norm() <= 1.2e-2 * b.norm()
+    assert float(got[0][T:].abs().max()) == 0.0

@@ -184,3 +184,30 @@ def test_native_encoder_against_fp32_rf_oracle():
         elif e >= 0.1:
             bad.append("%s: rel. max err %.4f (scale %.3g)" % (s.name, e, sc))
     assert not bad, "parameter gradients differ from the fp32 oracle:\n" + "\n".join(bad)
+
+
+@gpu
+def test_native_encoder_with_another_head_dim_matches_per_op_path():
+    """one head of 128: attention by batched products and softmax kernels in both passes of the executor, no fused kernel"""
+    from returnn_b200.models import conformer_native
+
+    model, pt, arena = _make(heads=1)
+    assert conformer_native.get_plan(model.encoder) is not None
+    torch.manual_seed(2)
+    lens = torch.tensor([600, 431, 577, 90], dtype=torch.int32)
+    feats = torch.randn(4, 600, 80, device="cuda")
+    wgt = torch.randn(600, 128, device="cuda")
+    o1, _, gp1 = _run(model, arena, feats, lens, wgt, native=True)
+    o2, _, gp2 = _run(model, arena, feats, lens, wgt, native=False)
+    assert torch.isfinite(o1).all() and torch.isfinite(gp1).all()
+    torch.testing.assert_close(o1, o2, atol=0.08, rtol=0.05)
+    bad = []
+    for s in arena.slots:
+        if s.name.endswith("depthwise_conv.bias"):
+            continue  # a bias in front of BatchNorm has an exactly zero gradient: both paths only produce rounding noise
+        a, b = gp1[s.offset: s.offset + s.numel], gp2[s.offset: s.offset + s.numel]
+        scale = float(b.abs().max()) + 1e-6
+        err = float((a - b).abs().max()) / scale
+        if err >= 0.08:  # bf16 paths that differ in the order of their roundings
+            bad.append("%s: rel. max err %.4f (scale %.3g)" % (s.name, err, scale))
+    assert not bad, "parameter gradients differ:\n" + "\n".join(bad)

@@ -399,3 +399,26 @@ def test_layer_norm_backward_entry_without_one_of_the_parameter_gradients(w_dtyp
     assert torch.equal(call(*((None, one) if skip == "gamma" else (one, None))), want)
     # (sums of 37 rows by atomics: fp32 rounding in another order)
     torch.testing.assert_close(one, both[1 if skip == "gamma" else 0], atol=1e-4, rtol=1e-2)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("v,n_inf", [(1001, 1), (1003, 700), (4096, 4000), (20, 19)])
+def test_softmax_cross_entropy_with_leading_classes_of_minus_infinity(dtype, v, n_inf):
+    """classes that a model rules out: whole vectors and threads of the row pass see nothing but -inf"""
+    from returnn_b200.ops import softmax_ce as ce
+
+    torch.manual_seed(v)
+    logits = torch.randn(5, v, device="cuda").to(dtype)
+    logits[:, :n_inf] = float("-inf")
+    logits.requires_grad_(True)
+    tgt = torch.randint(n_inf, v, (5,), device="cuda")
+    loss, best = ce.softmax_cross_entropy(logits, tgt, with_argmax=True)
+    (grad,) = torch.autograd.grad(loss, [logits], torch.ones_like(loss))
+    ref_in = logits.detach().double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(ref_in, tgt, reduction="none")
+    (want,) = torch.autograd.grad(ref, [ref_in], torch.ones_like(ref))
+    assert torch.equal(best.long(), logits.detach().float().argmax(-1))
+    torch.testing.assert_close(loss.double(), ref.detach(), atol=1e-5, rtol=1e-5)
+    # the gradient leaves in the type of the logits: 2^-9 of a value up to 1
+    torch.testing.assert_close(grad.double(), want, atol=4e-3 if dtype == torch.bfloat16 else 1e-6, rtol=0)

@@ -36,11 +36,23 @@ def _case(B, H, D, Tq, Tk, causal, with_lens, seed=0):
     (2, 2, 64, 17, 130, False, True),    # cross attention: short queries, long padded keys
     (1, 1, 128, 1, 65, True, False),     # one decoding step against a cache (the query is the last position)
     (2, 8, 64, 128, 192, False, False),  # sizes on tile boundaries
-    (2, 2, 64, 40, 300, False, True),    # key rows of two register chunks per lane
-    (1, 2, 64, 64, 600, False, True),    # ... and of four
-    (2, 2, 64, 200, 200, True, True),    # causal with padding, a whole warp per row
+    (2, 2, 64, 40, 300, False, True),    # several tiles of keys
+    (1, 2, 64, 64, 600, False, True),
+    (2, 2, 64, 200, 200, True, True),    # causal with padding
 ])
 def test_sdpa_matches_reference(B, H, D, Tq, Tk, causal, with_lens):
+    _case(B, H, D, Tq, Tk, causal, with_lens)
+
+
+@pytest.mark.parametrize("B,H,D,Tq,Tk,causal,with_lens", [
+    (2, 2, 128, 30, 50, False, True),    # the softmax kernels between two products: eight lanes per row of keys
+    (2, 1, 128, 70, 100, False, True),   # sixteen
+    (2, 2, 128, 200, 200, True, True),   # causal with padding, a whole warp per row
+    (2, 2, 128, 40, 300, False, True),   # rows of two register chunks per lane
+    (1, 2, 192, 64, 600, False, True),   # ... and of four
+    (1, 1, 128, 33, 1100, True, True),   # scores in 32 bits
+])
+def test_sdpa_matches_reference_for_other_head_dims(B, H, D, Tq, Tk, causal, with_lens):
     _case(B, H, D, Tq, Tk, causal, with_lens)
 
 
@@ -223,3 +235,36 @@ def test_sdpa_query_gradient_where_values_share_an_offset(T, causal):
     want = torch.autograd.grad(S.sdpa_reference(*(t.flatten(2) for t in r), num_heads=2, causal=causal), r[:1], dy.float().flatten(2))[0]
     err = ((got.double() - want).norm() / want.norm()).item()
     assert err <= 0.2, err
+
+
+@pytest.mark.parametrize("D,Tq,Tk,causal", [(64, 300, 300, True), (64, 150, 270, False), (64, 129, 200, True), (128, 140, 140, True), (128, 40, 300, False)])
+def test_sdpa_dropout_gradients_over_several_tiles(D, Tq, Tk, causal):
+    """the decisions of all tiles, read out block by block: with the identity on a block of keys as values the output is the kept probabilities"""
+    from returnn_b200.ops import sdpa as S
+    from returnn_b200.ops.elementwise import _seed_tensor
+
+    torch.manual_seed(7)
+    B, H, p = 2, 2, 0.2
+    q, k, v = ((torch.randn(B, t, H, D, device="cuda") * 0.7).to(torch.bfloat16).requires_grad_(True) for t in (Tq, Tk, Tk))
+    seed = _seed_tensor(q.device)
+    state = seed.clone()
+    mask = torch.zeros(B, H, Tq, Tk, device="cuda")
+    for j in range(0, Tk, D):
+        block = torch.zeros(B, Tk, H, D, device="cuda", dtype=torch.bfloat16)
+        n = min(D, Tk - j)
+        block[:, j: j + n, :, :n] = torch.eye(n, device="cuda", dtype=torch.bfloat16)[:, None]
+        seed.copy_(state)
+        mask[..., j: j + n] = (S.sdpa_heads(q.detach(), k.detach(), block, causal=causal, dropout_p=p)[..., :n] > 0).transpose(1, 2).float()
+    seen = torch.ones(Tq, Tk, device="cuda").tril(Tk - Tq) if causal else torch.ones(Tq, Tk, device="cuda")
+    assert abs((mask.sum() / (seen.sum() * B * H)).item() - (1 - p)) < 0.02
+    seed.copy_(state)
+    out = S.sdpa_heads(q, k, v, causal=causal, dropout_p=p)
+    w = torch.randn_like(out)
+    got = torch.autograd.grad(out, [q, k, v], w)
+    r = [t.detach().double().requires_grad_(True) for t in (q, k, v)]
+    s = (torch.einsum("bihd,bjhd->bhij", r[0], r[1]) * D ** -0.5).masked_fill(seen == 0, float("-inf"))
+    ref = torch.einsum("bhij,bjhd->bihd", torch.softmax(s, -1) * mask / (1 - p), r[2])
+    assert (out.double() - ref).norm() <= 1e-2 * ref.norm()
+    for a, b in zip(got, torch.autograd.grad(ref, r, w.double())):
+        # fused: probabilities, dS and results rounded to bf16, 2^-9 each; other head dims: scores and dP as well
+        assert (a.double() - b).norm() <= (1e-2 if D == 64 else 2e-2) * b.norm()
