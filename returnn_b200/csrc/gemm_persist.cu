@@ -349,6 +349,13 @@ RB_EXPORT int rb200_gemm_fp16_ex(const void* a, const void* b, void* c, void* c2
                  offset, drop_site, resid, res_scale, split_k, status, 1, stream);
 }
 
+// whether rb200_gemm_fp16_split takes a product of this size (the CTA-pair kernel can be switched off by the environment)
+RB_EXPORT int rb200_gemm_fp16_split_supported(int m, int n) {
+  RbGemm g;
+  g.m = m; g.n = n;
+  return rb_gemm_pair_wanted(g) ? 1 : 0;
+}
+
 // c[m,n] (fp32) = A·B with fp16 operands split in two: A = hi + lo, hi stored [m][k] at `a` and lo a_lo_rows rows further on, B likewise
 // stored [k][n]; the product of the two lo parts (2^-22 of the result) is left out. RB_ERR_UNSUPPORTED: not a shape of the CTA-pair kernel.
 RB_EXPORT int rb200_gemm_fp16_split(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc, int a_lo_rows, int b_lo_rows,

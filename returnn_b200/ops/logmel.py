@@ -20,7 +20,6 @@ from . import _lib
 
 _vp, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 _cache = {}
-_PAIR_KERNEL_OFF = os.environ.get("RETURNN_B200_GEMM_2CTA", "")[:1] == "0"
 
 
 def available() -> bool:
@@ -117,7 +116,7 @@ def _log_mel_gemm(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, f
     weights = _mel_weights(fb, fb_start, fb_len)
     m = rows * slots
     spec = torch.empty(m, n_fft, dtype=torch.float32, device=dev)
-    if m > 128 and n_fft > 128 and m + total // step < 2 ** 31 and not _PAIR_KERNEL_OFF:
+    if m + total // step < 2 ** 31 and _lib.bind("rb200_gemm_fp16_split_supported", [_i32, _i32])(m, n_fft):
         # hi*lo + lo*hi + hi*hi summed in one accumulator: the spectrum is written once
         fn = _lib.bind("rb200_gemm_fp16_split", [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp])
         _lib.check(fn(parts.data_ptr(), t_hi.data_ptr(), spec.data_ptr(), m, n_fft, window, step, n_fft, n_fft, total // step, window,

@@ -422,3 +422,24 @@ def test_softmax_cross_entropy_with_leading_classes_of_minus_infinity(dtype, v, 
     torch.testing.assert_close(loss.double(), ref.detach(), atol=1e-5, rtol=1e-5)
     # the gradient leaves in the type of the logits: 2^-9 of a value up to 1
     torch.testing.assert_close(grad.double(), want, atol=4e-3 if dtype == torch.bfloat16 else 1e-6, rtol=0)
+
+
+@gpu
+def test_log_mel_follows_the_switch_of_the_pair_kernel_whenever_it_is_set():
+    """the kernel library looks at the switch with its first product, which may come after the import of the feature extraction"""
+    import subprocess
+    import sys
+
+    code = """
+import os, torch
+from returnn_b200.ops import logmel
+os.environ["RETURNN_B200_GEMM_2CTA"] = "0"
+os.environ["RETURNN_B200_LOGMEL"] = "gemm"
+x = torch.randn(2, 40000, device="cuda") * 0.1
+kw = dict(sampling_rate=16000, window=400, step=160, n_fft=512, n_mel=80, f_min=0.0, f_max=8000.0)
+a = logmel.log_mel(x, **kw)
+os.environ["RETURNN_B200_LOGMEL"] = "direct"
+b = logmel.log_mel(x, **kw)
+assert (a - b).abs().max() < 1e-3, float((a - b).abs().max())
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
