@@ -10,7 +10,8 @@
 // product -> softmax -> product of one CTA is serial; three (backward: two) CTAs per SM fill each other's gaps. That is why the tiles are
 // 64 wide: 128 TMEM columns and 67 KB of shared memory per CTA (backward 256 columns and 99 / 102 KB). The two-pass backward (dQ apart from
 // dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
-// The kernels are bound by the per-row exponentials and that chain, not by memory.
+// The kernels are bound by that chain: no unit is saturated (8 x 1000 causal, 8 heads: tensor pipe 15 to 19 % of active cycles, special
+// functions 19 to 30 %), and the warps wait for tensor-memory loads and at the barrier. 37 + 41 + 54 us there, 40 + 51 + 68 at 250 x 100.
 //
 // Visible keys, the dropout rate and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per
 // score. They come from a stream of the generator of their own (tag 0x53; sdpa.cu and attention.cu draw from 0x51, rel_pos_flash.cu from
