@@ -268,3 +268,22 @@ def test_sdpa_dropout_gradients_over_several_tiles(D, Tq, Tk, causal):
     for a, b in zip(got, torch.autograd.grad(ref, r, w.double())):
         # fused: probabilities, dS and results rounded to bf16, 2^-9 each; other head dims: scores and dP as well
         assert (a.double() - b).norm() <= (1e-2 if D == 64 else 2e-2) * b.norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_sdpa_sequence_without_visible_keys(D, causal):
+    """a length of zero in the batch: zeros for its queries, no gradient into its keys and values, nothing of it in the other entries"""
+    from returnn_b200.ops import sdpa as S
+
+    torch.manual_seed(11)
+    lens = torch.tensor([0, 70, 0], device="cuda", dtype=torch.int32)
+    x = [torch.randn(3, 90, 2, D, device="cuda").to(torch.bfloat16).requires_grad_(True) for _ in range(3)]
+    w = torch.randn(3, 90, 2, D, device="cuda").to(torch.bfloat16)
+    out = S.sdpa_heads(*x, k_lens=lens, causal=causal)
+    got = torch.autograd.grad(out, x, w)
+    one = [t.detach()[1:2].clone().requires_grad_(True) for t in x]
+    want_out = S.sdpa_heads(*one, k_lens=lens[1:2].clone(), causal=causal)
+    want = torch.autograd.grad(want_out, one, w[1:2])
+    for a, b in zip((out, *got), (want_out, *want)):
+        assert torch.equal(a[1:2], b) and float(a[0].abs().max()) == 0.0 and float(a[2].abs().max()) == 0.0
