@@ -3,11 +3,12 @@ Log-mel frontend on own kernels (``csrc/mel.cu``): framing, Hann window, DFT, po
 The window and the filterbank are built once per configuration with the same formulas as the RF path
 (:mod:`returnn_b200.frontend.audio.mel`, :func:`returnn_b200.frontend.signal.stft`), so both give the same features.
 
-Two forms. Large inputs run the DFT on the tensor cores: all frames times the windowed cos / sin table is one matrix product on the
+Three forms. Transform lengths of 256, 512 and 1024 run as an fp32 FFT, from audio to features in one kernel (``csrc/mel_fft.cu``).
+Other lengths of large inputs run the DFT on the tensor cores: all frames times the windowed cos / sin table is one matrix product on the
 tcgen05 GEMM, with the frames read as an overlapping strided view of the audio (no frame matrix in memory), fp32 precision kept by
 splitting both factors into fp16 high and low parts (three accumulating products, 22 mantissa bits per factor), followed by one kernel for power -> mel -> log.
-Small inputs (or a hop size that is not a multiple of 8 samples, which the strided view needs for 16-byte row pitches) run the
-single fp32 kernel that does everything per block of 8 frames.
+The rest (small inputs, or a hop size that is not a multiple of 8 samples, which the strided view needs for 16-byte row pitches) runs the
+single fp32 kernel that does everything per block of 8 frames. ``RETURNN_B200_LOGMEL`` = ``direct`` / ``gemm`` asks for one of the last two.
 """
 
 from __future__ import annotations
@@ -63,6 +64,20 @@ def _dft_tables(device, window: int, n_fft: int, win: torch.Tensor, fb: torch.Te
         table = table.float()
         hi = table.half()
         lo = (table - hi.float()).half()
+        both = torch.stack([hi, lo]).to(device)
+        t = (both[0], both[1], *_mel_weights(device, fb)[1:])
+        _cache[key] = t
+    return t
+
+
+def _mel_weights(device, fb: torch.Tensor):
+    """
+    (weights, start, length): the non-zero part of every mel filter, [longest filter, n_mel] fp32, entry i of filter m is
+    ``fb[start[m] + i, m]``, and the bin ranges [n_mel] int32
+    """
+    key = ("weights", str(device), fb.data_ptr())
+    t = _cache.get(key)
+    if t is None:
         nz = fb.cpu() != 0  # [n_bins, n_mel]
         idx = torch.arange(nz.shape[0])[:, None].expand_as(nz)
         big = nz.shape[0]
@@ -70,20 +85,9 @@ def _dft_tables(device, window: int, n_fft: int, win: torch.Tensor, fb: torch.Te
         end = torch.where(nz, idx + 1, torch.zeros_like(idx)).max(dim=0).values
         length = torch.clamp(end - start, min=0)
         start = torch.where(length > 0, start, torch.zeros_like(start))
-        both = torch.stack([hi, lo]).to(device)
-        t = (both[0], both[1], start.to(device, torch.int32).contiguous(), length.to(device, torch.int32).contiguous())
-        _cache[key] = t
-    return t
-
-
-def _mel_weights(fb: torch.Tensor, start: torch.Tensor, length: torch.Tensor) -> torch.Tensor:
-    """the non-zero part of every mel filter, [longest filter, n_mel] fp32: entry i of filter m is ``fb[start[m] + i, m]``"""
-    key = ("weights", str(fb.device), fb.data_ptr())
-    t = _cache.get(key)
-    if t is None:
-        i = torch.arange(max(int(length.max()), 1), device=fb.device)[:, None]
-        idx = torch.clamp(start.long()[None] + i, max=fb.shape[0] - 1)
-        t = _cache[key] = (torch.gather(fb, 0, idx) * (i < length[None])).contiguous()
+        i = torch.arange(max(int(length.max()), 1))[:, None]
+        weights = torch.gather(fb.cpu(), 0, torch.clamp(start[None] + i, max=big - 1)) * (i < length[None])
+        t = _cache[key] = (weights.to(device).contiguous(), start.to(device, torch.int32).contiguous(), length.to(device, torch.int32).contiguous())
     return t
 
 
@@ -113,7 +117,7 @@ def _log_mel_gemm(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, f
     fn = _lib.bind("rb200_split_hi_lo_fp16", [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp])
     _lib.check(fn(flat.data_ptr(), rows, T, Tp, total, hi.data_ptr(), lo.data_ptr(), _lib.stream_ptr()), "split_hi_lo")
     t_hi, t_lo, fb_start, fb_len = _dft_tables(dev, window, n_fft, win, fb)
-    weights = _mel_weights(fb, fb_start, fb_len)
+    weights = _mel_weights(dev, fb)[0]
     m = rows * slots
     spec = torch.empty(m, n_fft, dtype=torch.float32, device=dev)
     if m + total // step < 2 ** 31 and _lib.bind("rb200_gemm_fp16_split_supported", [_i32, _i32])(m, n_fft):
@@ -134,6 +138,24 @@ def _log_mel_gemm(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, f
     _lib.count_launch(2)
 
 
+def _log_mel_fft(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, fb, scale, n_frames, out) -> bool:
+    """one kernel, where the library has it for these sizes; device time for one utterance of 0.5 s 8 us, 64 of 10 s 56 us (the others: 62, 150)"""
+    if os.environ.get("RETURNN_B200_LOGMEL", "auto") in ("direct", "gemm") or not 0 < window <= n_fft:
+        return False
+    lib = _lib.get_lib()
+    if lib is None or not hasattr(lib, "rb200_log_mel_fft"):
+        return False
+    weights, start, length = _mel_weights(flat.device, fb)
+    if not _lib.bind("rb200_log_mel_fft_supported", [_i32, _i32, _i32])(n_fft, weights.shape[0], n_mel):
+        return False
+    rows, T = flat.shape
+    fn = _lib.bind("rb200_log_mel_fft", [_vp, _vp, _i32, _i64, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _vp, _i32, _f32, _f32, _vp, _vp])
+    _lib.check(fn(flat.data_ptr(), l32.data_ptr() if l32 is not None else None, rows, T, n_frames, window, step, n_fft, win.data_ptr(), weights.data_ptr(),
+                  weights.shape[0], start.data_ptr(), length.data_ptr(), n_mel, scale, 1e-10, out.data_ptr(), _lib.stream_ptr()), "log_mel_fft")
+    _lib.count_launch()
+    return True
+
+
 def log_mel(audio: torch.Tensor, *, sampling_rate: int, window: int, step: int, n_fft: int, n_mel: int, f_min: float, f_max: float,
             log_base: float = 10.0, lens: Optional[torch.Tensor] = None) -> torch.Tensor:
     """
@@ -150,8 +172,11 @@ def log_mel(audio: torch.Tensor, *, sampling_rate: int, window: int, step: int, 
         win, fb = _tables(audio.device, sampling_rate, window, n_fft, n_mel, f_min, f_max)
         l32 = lens.to(audio.device, torch.int32).contiguous() if lens is not None else None
         scale = 1.0 if log_base == math.e else 1.0 / math.log(log_base)
+        kw = dict(window=window, step=step, n_fft=n_fft, n_mel=n_mel, win=win, fb=fb, scale=scale, n_frames=n_frames, out=out)
+        if _log_mel_fft(flat, l32, **kw):
+            return out.reshape(shape[:-1] + [n_frames, n_mel])
         if _gemm_form_wanted(flat, window, step, n_fft):
-            _log_mel_gemm(flat, l32, window=window, step=step, n_fft=n_fft, n_mel=n_mel, win=win, fb=fb, scale=scale, n_frames=n_frames, out=out)
+            _log_mel_gemm(flat, l32, **kw)
             return out.reshape(shape[:-1] + [n_frames, n_mel])
         fn = _lib.bind("rb200_log_mel", [_vp, _vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _i32, _f32, _f32, _vp, _vp])
         _lib.check(fn(flat.data_ptr(), l32.data_ptr() if l32 is not None else None, rows, T, window, step, n_fft, win.data_ptr(), fb.data_ptr(), n_mel,

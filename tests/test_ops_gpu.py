@@ -264,6 +264,45 @@ def test_log_mel_gemm_form_matches_float64():
 
 
 @gpu
+@pytest.mark.parametrize("rows,samples,window,step,n_fft,n_mel", [
+    (1, 400, 400, 160, 512, 80), (3, 5361, 400, 160, 512, 80), (2, 5201, 399, 157, 512, 23), (2, 40000, 512, 8, 512, 1), (5, 16000, 200, 80, 256, 40),
+    (2, 3001, 255, 33, 256, 7), (3, 30011, 1024, 441, 1024, 128), (2, 20000, 800, 320, 1024, 80), (150, 2000, 400, 160, 512, 80), (1, 700, 1, 1, 256, 3)])
+def test_log_mel_fft_form_matches_float64(rows, samples, window, step, n_fft, n_mel):
+    """
+    one kernel per call: tiles with one and with all frames, odd windows, hops and rows, all transform lengths. Noise: a bin's power is off by a few
+    2^-24 of the strongest amplitude (10 butterflies) over its own, down to 1e-2 of it: 2 * 6e-7 / 1e-2 * log10(e) = 5e-5
+    """
+    from returnn_b200.ops import logmel
+
+    gen = torch.Generator().manual_seed(samples)
+    audio = torch.randn(rows, samples, generator=gen) * 0.3
+    lens = torch.randint(0, samples + 1, (rows,), generator=gen, dtype=torch.int32)
+    lens[0] = samples
+    got = logmel.log_mel(audio.cuda(), sampling_rate=16000, window=window, step=step, n_fft=n_fft, n_mel=n_mel, f_min=0.0, f_max=8000.0, lens=lens).cpu()
+    win, fb = logmel._tables(torch.device("cpu"), 16000, window, n_fft, n_mel, 0.0, 8000.0)
+    power = torch.fft.rfft(audio.double().unfold(1, window, step) * win.double(), n=n_fft).abs() ** 2
+    ref = torch.log10(torch.clamp(power @ fb.double(), min=1e-10))
+    for r, n in enumerate(lens.tolist()):
+        ref[r, (n - window) // step + 1 if n >= window else 0:] = 0
+    assert got.shape == ref.shape
+    torch.testing.assert_close(got.double(), ref, atol=1e-4, rtol=0)
+
+
+@gpu
+def test_log_mel_frames_with_nan_do_not_reach_other_frames():
+    from returnn_b200.ops import logmel
+
+    audio = torch.randn(2, 16000, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    kw = dict(sampling_rate=16000, window=400, step=160, n_fft=512, n_mel=80, f_min=0.0, f_max=8000.0)
+    ref = logmel.log_mel(audio, **kw)
+    audio[0, 4000], audio[1, 8000] = float("nan"), float("inf")
+    got = logmel.log_mel(audio, **kw)
+    for r, at in ((0, 4000), (1, 8000)):
+        hit = torch.tensor([f * 160 <= at < f * 160 + 400 for f in range(ref.shape[1])], device="cuda")
+        assert torch.equal(got[r][~hit], ref[r][~hit]) and (got[r][hit] == -10.0).all()
+
+
+@gpu
 @pytest.mark.parametrize("rows,n", [(1, 512), (37, 256), (4100, 512), (9475, 384), (2368 * 5 + 3, 512)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_layer_norm_bwd_accumulating_kernel_matches_fp32(rows, n, with_res):
