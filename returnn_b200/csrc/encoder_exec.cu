@@ -50,7 +50,7 @@ int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const voi
 int rb200_rel_flash_slices(long long rows, int width, int heads);
 int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream);
 int rb200_glu_dwconv_fwd(const void* x, const float* filt, const float* bias, const int* row_batch, const int* row_pos, const int* lens,
-                         void* y, float* part, int n_rows, int C, int K, cudaStream_t stream);
+                         void* y, float* part, int n_rows, int n_seqs, int C, int K, cudaStream_t stream);
 int rb200_bn_stats(const float* part, int n_tiles, int C, float count, float eps, float momentum, float* mean, float* rstd,
                    float* running_mean, float* running_var, cudaStream_t stream);
 int rb200_bn_silu_fwd(const void* y, const float* mean, const float* rstd, const float* gamma, const float* beta, void* z, long long n_rows,
@@ -59,7 +59,7 @@ int rb200_bn_silu_bwd_ex(const void* y, const void* dz, const float* mean, const
                          float* part, int n_tiles, float* sum_ds, float* sum_ds_yh, long long n_rows, int C, int training, float* dgamma_acc,
                          float* dbeta_acc, cudaStream_t stream);
 int rb200_glu_dwconv_bwd_ex(const void* x, const void* dy, const float* filt, const int* row_batch, const int* row_pos, const int* lens,
-                            void* dx, float* part, float* dfilt, float* dbias, int n_rows, int C, int K, int accumulate, cudaStream_t stream);
+                            void* dx, float* part, float* dfilt, float* dbias, int n_rows, int n_seqs, int C, int K, int accumulate, cudaStream_t stream);
 }
 
 // dimensions and hyper-parameters of one call (mirrored by a ctypes.Structure on the Python side)
@@ -274,9 +274,9 @@ inline int ln_parts(int n) {
   if (p < 1) p = 1;
   return p;
 }
-inline int bn_tiles_a(int n) {  // 16 rows per CTA: a few hundred CTAs for the batches of a training step
+inline int bn_tiles_a(int n) {  // at least 16 rows per CTA, as many CTAs as are resident
   int t = (n + 15) / 16;
-  if (t > 592) t = 592;
+  if (t > 296) t = 296;
   if (t < 1) t = 1;
   return t;
 }
@@ -590,7 +590,7 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
     // ---- convolution module
     e.layer_norm(sv.x2, l, P_CONV_LN_G, sv.ln3, sv.st3);
     e.linear_fwd(sv.ln3, l, P_PW1_W, P_PW1_B, n, D, 2 * D, sv.g, nullptr, 0, 0.f, 0, nullptr, 1.f);
-    if (e.ok()) e.run_tagged("glu_dwconv_fwd", rb200_glu_dwconv_fwd(sv.g, e.p32(l, P_DW_F), e.p32(l, P_DW_B), row_batch, row_pos, lens, sv.y, t.conv_part, n, D, g.K, stream));
+    if (e.ok()) e.run_tagged("glu_dwconv_fwd", rb200_glu_dwconv_fwd(sv.g, e.p32(l, P_DW_F), e.p32(l, P_DW_B), row_batch, row_pos, lens, sv.y, t.conv_part, n, g.B, D, g.K, stream));
     if (e.ok()) {
       const bool upd = d.training != 0;
       if (d.training) {
@@ -665,7 +665,7 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
       e.launches += 2;
     }
     if (e.ok()) {
-      e.run_tagged("glu_dwconv_bwd_ex", rb200_glu_dwconv_bwd_ex(sv.g, t.tD3, e.p32(l, P_DW_F), row_batch, row_pos, lens, t.tW, t.conv_part, e.g32(l, P_DW_F), e.g32(l, P_DW_B), n, D,
+      e.run_tagged("glu_dwconv_bwd_ex", rb200_glu_dwconv_bwd_ex(sv.g, t.tD3, e.p32(l, P_DW_F), row_batch, row_pos, lens, t.tW, t.conv_part, e.g32(l, P_DW_F), e.g32(l, P_DW_B), n, g.B, D,
                                     g.K, 1, stream));
       e.launches += 1;
     }

@@ -71,3 +71,68 @@ def test_conv_module_fwd_bwd(lens, C, K):
     for n, g, r, t in zip(names, got, ref, tols):
         torch.testing.assert_close(g, r.float(), atol=t, rtol=5e-2, msg=lambda s, n=n: "%s: %s" % (n, s))
     torch.testing.assert_close(rm_native, bn2.running_mean.raw_tensor, atol=1e-2, rtol=1e-2)
+
+
+@gpu
+@pytest.mark.parametrize("lens,C,K", [
+    ([1], 64, 32), ([31, 1, 32, 33, 0, 64], 64, 32), ([3] * 150, 128, 31), ([2000, 5], 64, 17), ([20] * 40 + [600], 256, 16), ([65, 7, 64], 512, 7),
+    ([333, 100, 200, 40], 1024, 2), ([1] * 70, 64, 15), ([90, 120], 64, 33)])
+@pytest.mark.parametrize("training", [True, False])
+def test_conv_module_windows_against_float64(lens, C, K, training):
+    """
+    pieces and steps of the sliding-window kernels: short and empty sequences, pieces of one step and of many, both tap counts, and the old
+    kernel beyond 32 taps. bf16 rounds the convolution, its gradient and the results once each: 2^-9 apiece, twice that in the sums over them
+    """
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import conv_module as cm
+
+    gen = torch.Generator("cuda").manual_seed(sum(lens) + K)
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    n = pack.n
+    x = torch.randn(n, 2 * C, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    filt = (torch.randn(C, 1, K, device="cuda", generator=gen) * K ** -0.5).requires_grad_(True)
+    bias = (torch.randn(C, device="cuda", generator=gen) * 0.1).requires_grad_(not training)  # its gradient under batch statistics is 0
+    bn = _BN(C, "cuda")
+    dz = torch.randn(n, C, device="cuda", generator=gen).bfloat16()
+    z = cm.glu_dwconv_bn_silu(x, filt, bias, bn, pack, training=training)
+    leaves = [x, filt, bn.gamma.raw_tensor, bn.beta.raw_tensor] + ([] if training else [bias])
+    got = [z, *torch.autograd.grad(z, leaves, dz)]
+    x64, f64, g64, b64, c64 = (t.detach().double().requires_grad_(True) for t in (x, filt, bn.gamma.raw_tensor, bn.beta.raw_tensor, bias))
+    h = x64[:, :C] * torch.sigmoid(x64[:, C:])
+    ys, lo = [], 0
+    for m in lens:
+        if m:
+            p = torch.nn.functional.pad(h[lo: lo + m].t()[None], ((K - 1) // 2, K - 1 - (K - 1) // 2))
+            ys.append(torch.nn.functional.conv1d(p, f64, c64, groups=C)[0].t())
+        lo += m
+    y = torch.cat(ys)
+    if training:
+        y = (y - y.mean(0)) * torch.rsqrt(y.var(0, unbiased=False) + bn.eps)
+    else:
+        y = y * (1.0 + bn.eps) ** -0.5  # running statistics 0 and 1
+    ref = torch.nn.functional.silu(y * g64 + b64)
+    refs = [ref, *torch.autograd.grad(ref, [x64, f64, g64, b64] + ([] if training else [c64]), dz.double())]
+    for name, a, b in zip(["z", "dx", "dfilt", "dgamma", "dbeta", "dbias"], got, refs):
+        if training and n < 8:
+            continue  # differences of a few rows from their mean: rounding of y is not small against them
+        a = a.detach()
+        assert float((a.double() - b).norm()) <= 8e-3 * float(b.norm()), (name, float((a.double() - b).norm() / b.norm()))
+
+
+@gpu
+def test_conv_module_sequences_do_not_see_each_other():
+    """not even through the zeros that fill up the taps: a NaN stays in its sequence"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import conv_module as cm
+
+    lens, C = [40, 3, 70], 64
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    for K in (2, 7, 16, 31):
+        x = torch.randn(sum(lens), 2 * C, device="cuda").bfloat16()
+        x[41] = float("nan")
+        x.requires_grad_(True)
+        filt = torch.randn(C, 1, K, device="cuda")
+        z = cm.glu_dwconv_bn_silu(x, filt, None, _BN(C, "cuda"), pack, training=False)
+        (dx,) = torch.autograd.grad(z, [x], torch.ones_like(z))
+        for t in (z, dx):
+            assert bool(torch.isfinite(t[:40]).all()) and bool(torch.isfinite(t[43:]).all())
