@@ -2,10 +2,10 @@
 CTC loss with fused log-softmax.
 
 ``ctc_loss`` takes padded logits ``[B, T, V]``; ``ctc_loss_packed`` takes packed logits ``[N, V]`` with ``cu_seqlens``.
-On B200 (``csrc/ctc.cu``): one CTA per sequence computes the per-frame log-sum-exp, runs the alpha and beta recursions
-in shared memory over the extended label sequence and writes ``dlogits = softmax - posterior`` in the logits dtype, so
-the ``[T, V]`` log-probabilities are never materialised. Scratch memory (global): per-frame log-sum-exp and the alpha
-lattice ``[T, 2S+1]`` per sequence. Otherwise ``torch.nn.functional.ctc_loss`` in fp32.
+On B200 (``csrc/ctc.cu``): one CTA per frame computes the log-sum-exp and writes the softmax, one CTA per sequence runs the alpha and
+beta recursions over the extended label sequence, and the entries of the label classes are then corrected to ``dlogits = softmax -
+posterior`` in the logits dtype, so the ``[T, V]`` log-probabilities are never materialised. Scratch memory (global): the label
+probabilities and the alpha and beta lattices ``[T, 2S+1]`` per sequence. Otherwise ``torch.nn.functional.ctc_loss`` in fp32.
 """
 
 from __future__ import annotations
@@ -30,7 +30,7 @@ def supports(logits, targets) -> bool:
 
 
 def max_target_len() -> int:
-    """longest label sequence the kernels handle (the gradient kernel keeps 16 * (2S+1) floats in shared memory)"""
+    """longest label sequence the kernels handle (the gradient kernel keeps 16 * (2S+1) values in shared memory)"""
     return 1500
 
 
@@ -49,7 +49,7 @@ class _CtcFn(torch.autograd.Function):
         need_grad = logits_rows.requires_grad
         grad = torch.empty_like(logits_rows) if need_grad else None
         s_ext = 2 * max_s + 1
-        scratch = torch.empty(n * (1 + 3 * s_ext) + b, dtype=torch.float32, device=logits_rows.device)
+        scratch = torch.empty(n * (2 + 6 * (s_ext + 1)) + b * (4 + s_ext), dtype=torch.float32, device=logits_rows.device)
         fn = _lib.bind("rb200_ctc_loss", [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i64, _vp])
         _lib.check(fn(logits_rows.data_ptr(), 1 if logits_rows.dtype == torch.bfloat16 else 0, cu.data_ptr(), row_batch.data_ptr(),
                       targets.data_ptr(), tgt_lens.data_ptr(), loss.data_ptr(), grad.data_ptr() if grad is not None else None,

@@ -44,3 +44,79 @@ def test_ctc_loss_packed(lens, tlens, V, dtype):
     torch.testing.assert_close(loss, ref, atol=tol, rtol=1e-3)
     gtol = 2e-2 if dtype == torch.bfloat16 else 1e-4
     torch.testing.assert_close(logits.grad.float(), l32.grad, atol=gtol, rtol=1e-2)
+
+
+def _ctc_float64(x, pack, targets, tl, blank, w):
+    """loss and gradient of every sequence in 64 bits"""
+    x = x.detach().double().requires_grad_(True)
+    lp, res, lo = torch.log_softmax(x, dim=-1), [], 0
+    for b, (n, s) in enumerate(zip(pack.lens_host.tolist(), tl.tolist())):
+        res.append(torch.nn.functional.ctc_loss(lp[lo: lo + n, None], targets[b: b + 1, :s].long(), torch.tensor([n]), torch.tensor([s]), blank=blank,
+                                                reduction="none", zero_infinity=True))
+        lo += n
+    loss = torch.cat(res)
+    return loss.detach(), torch.autograd.grad((loss * w.double()).sum(), [x])[0]
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,tlens,V,scale", [
+    ([1, 2, 9, 17], [0, 1, 4, 8], 5, 2.0),              # one frame; a group of frames and one more
+    ([120, 49, 150], [24, 24, 30], 1001, 10.0),         # one warp per recursion, and the first state of the second
+    ([300, 260, 400], [125, 128, 65], 80, 40.0),        # several warps, widely different probabilities
+    ([500, 31], [240, 15], 2049, 1.0),                  # four states per lane
+    ([1300], [620], 37, 3.0),                           # eight
+    ([40, 60], [7, 11], 33001, 2.0),                    # more vectors than a thread keeps; rows that start anywhere
+    ([25, 30], [5, 9], 10240, 2.0),
+])
+def test_ctc_recursions_against_float64(lens, tlens, V, scale, dtype):
+    """fp32 sums of a few hundred to a thousand products (2^-24 each, the exponent held apart): 2e-5; the bf16 gradient is rounded twice: 2^-8"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import ctc
+
+    gen = torch.Generator("cuda").manual_seed(V)
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    targets = torch.randint(0, V - 1, (len(lens), max(tlens)), device="cuda", dtype=torch.int32, generator=gen)
+    repeat = torch.rand(targets.shape, device="cuda", generator=gen) < 0.2
+    targets[:, 1:] = torch.where(repeat[:, 1:], targets[:, :-1], targets[:, 1:])
+    tl = torch.tensor(tlens, dtype=torch.int32)
+    logits = (torch.randn(pack.n, V, device="cuda", generator=gen) * scale).to(dtype).requires_grad_(True)
+    w = torch.rand(len(lens), device="cuda", generator=gen) + 0.5
+    loss = ctc.ctc_loss_packed(logits, pack, targets, tl, blank_index=V - 1)
+    (grad,) = torch.autograd.grad((loss * w).sum(), [logits])
+    ref, ref_grad = _ctc_float64(logits, pack, targets, tl, V - 1, w)
+    torch.testing.assert_close(loss.detach().double(), ref, atol=1e-4, rtol=2e-6)
+    assert float((grad.double() - ref_grad).norm()) <= (2e-5 if dtype == torch.float32 else 2.0 ** -8) * float(ref_grad.norm())
+    with torch.no_grad():
+        assert torch.equal(ctc.ctc_loss_packed(logits.detach(), pack, targets, tl, blank_index=V - 1), loss.detach())
+
+
+@gpu
+@pytest.mark.parametrize("value", [float("-inf"), -3.0e38, -1e9, -1e5])
+def test_ctc_masked_classes(value):
+    """classes masked by -inf or a large negative number: not in the labels, and in them (the second sequence then has no alignment, or a huge loss)"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import ctc
+
+    gen = torch.Generator("cuda").manual_seed(1)
+    pack = PackInfo(torch.tensor([12, 9, 20], dtype=torch.int32), torch.device("cuda"))
+    logits = torch.randn(pack.n, 30, device="cuda", generator=gen)
+    logits[:, 21:25] = value
+    targets = torch.randint(0, 20, (3, 4), device="cuda", dtype=torch.int32, generator=gen)
+    tl = torch.tensor([4, 3, 2], dtype=torch.int32)
+    for label in (None, 22):
+        if label is not None:
+            targets[1, 1] = label
+        x = logits.clone().requires_grad_(True)
+        loss = ctc.ctc_loss_packed(x, pack, targets, tl, blank_index=29)
+        (grad,) = torch.autograd.grad(loss.sum(), [x])
+        # log_softmax of -inf has no gradient: e^-1e5 is 0 in 64 bits as well
+        ref, ref_grad = _ctc_float64(torch.clamp(x, min=-1e5) if value == float("-inf") else x, pack, targets, tl, 29, torch.ones(3, device="cuda"))
+        if value == float("-inf") and label is not None:
+            ref[1] = 0.0
+        torch.testing.assert_close(loss.detach().double(), ref, atol=1e-4, rtol=1e-6)
+        rows = slice(0, 12) if label is not None else slice(0, pack.n)  # a loss of 1e9 has no digits left for the alignment
+        torch.testing.assert_close(grad[rows].double(), ref_grad[rows], atol=1e-5, rtol=0)
+        assert bool(torch.isfinite(grad).all())
+        if label is not None and value == float("-inf"):
+            assert float(loss[1].detach()) == 0.0 and float(grad[12:21].abs().max()) == 0.0
