@@ -30,8 +30,8 @@ int rb200_gemm_bf16_batched(const void* a, const void* b, void* c, const void* b
                             long long b_cols, int lda, int ldb, int ldc, int m, int n, int k, int a_mn_major, int b_mn_major, int bias_bf16,
                             int act, int out_fp32, int accumulate, float alpha, int batch, int heads, const long long* offs, const int* lens,
                             int m_from_lens, int n_from_lens, int k_from_lens, int* status, cudaStream_t stream);
-int rb200_att_prepare(const void* qkv, const float* u, const float* v, const int* row_batch, const int* row_pos, void* qu, void* qv, void* k,
-                      void* vv, int n_rows, int heads, int dim, int lp, cudaStream_t stream);
+int rb200_att_prepare(const void* qkv, const float* u, const float* v, const int* lens, void* qu, void* qv, void* k, void* vv, int batch, int heads,
+                      int dim, int lp, cudaStream_t stream);
 int rb200_att_softmax_fwd_ex(const void* s_ac, const void* g, int scores_bf16, void* w, void* wd, const int* lens, int batch, int heads, int lp, int rp,
                              int center, float p_drop, const long long* seed, const long long* offset, cudaStream_t stream);
 int rb200_att_softmax_bwd_ex(const void* w, const void* dwd, int dwd_bf16, void* ds, void* dg, const int* lens, int batch, int heads, int lp, int rp,
@@ -40,8 +40,9 @@ int rb200_att_redrop(const void* w, void* wd, const int* lens, int batch, int he
                      const long long* offset, cudaStream_t stream);
 int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* dk, const void* dv, const int* row_batch, const int* row_pos, void* dqkv,
                         int n_rows, int heads, int dim, int lp, cudaStream_t stream);
-int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, int to_padded,
+int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp,
                           cudaStream_t stream);
+int rb200_att_rows_pad(const void* src, void* dst, const int* lens, int batch, int width, int lp, cudaStream_t stream);
 int rb200_att_rows_gather_f32(const float* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, cudaStream_t stream);
 int rb200_rel_flash_band(int lp, int center, int* off, int* width);
 int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o, void* dqu,
@@ -247,7 +248,7 @@ struct SavedLayout {
     s.ln1 = bump.take<bf16>(n * D); s.st1 = bump.take<float>(2 * n);
     s.z1 = bump.take<bf16>(n * F); s.a1 = bump.take<bf16>(n * F); s.x1 = bump.take<bf16>(n * D);
     s.ln2 = bump.take<bf16>(n * D); s.st2 = bump.take<float>(2 * n);
-    s.qu = bump.take<bf16>(4 * g.pad_rows * HD);  // qu, qv, kk, vv back to back: one memset
+    s.qu = bump.take<bf16>(4 * g.pad_rows * HD);  // qu, qv, kk, vv back to back
     s.qv = s.qu ? s.qu + g.pad_rows * HD : nullptr;
     s.kk = s.qu ? s.qu + 2 * g.pad_rows * HD : nullptr;
     s.vv = s.qu ? s.qu + 3 * g.pad_rows * HD : nullptr;
@@ -566,8 +567,7 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
     e.layer_norm(sv.x1, l, P_ATT_LN_G, sv.ln2, sv.st2);
     e.linear_fwd(sv.ln2, l, P_QKV_W, P_QKV_B, n, D, 3 * HD, t.qkv, nullptr, 0, 0.f, 0, nullptr, 1.f);
     e.linear_fwd(sinus, l, P_POS_W, -1, g.R, D, HD, sv.posp, nullptr, 0, 0.f, 0, nullptr, 1.f);
-    e.memset0(sv.qu, 4 * g.pad_rows * HD * sizeof(bf16));
-    if (e.ok()) e.run_tagged("att_prepare", rb200_att_prepare(t.qkv, e.p32(l, P_POS_U), e.p32(l, P_POS_V), row_batch, row_pos, sv.qu, sv.qv, sv.kk, sv.vv, n, H, Dh, Lp, stream));
+    if (e.ok()) e.run_tagged("att_prepare", rb200_att_prepare(t.qkv, e.p32(l, P_POS_U), e.p32(l, P_POS_V), lens, sv.qu, sv.qv, sv.kk, sv.vv, B, H, Dh, Lp, stream));
     {
       const long long o1[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
       // scores and bias band in bf16, like the matmul outputs of the reference under autocast: halves the traffic of this stage
@@ -585,7 +585,7 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
       e.bgemm(wd, sv.vv, o_pad, Lp, Dh, Lp, 0, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o3, B * H, H, lens, 1, 0, 1, 1.f, g.fused_bwd);
     }
     if (e.ok() && g.fused_bwd) e.run_tagged("att_rows_gather", rb200_att_rows_gather_f32(sv.o_pad, sv.att, row_batch, row_pos, n, HD, Lp, stream));
-    else if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(o_pad, sv.att, row_batch, row_pos, n, HD, Lp, 0, stream));
+    else if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(o_pad, sv.att, row_batch, row_pos, n, HD, Lp, stream));
     e.linear_fwd(sv.att, l, P_PROJ_W, P_PROJ_B, n, HD, D, sv.x2, nullptr, 0, p_res, e.site(l, g.site_att_out), sv.x1, 1.f);
     // ---- convolution module
     e.layer_norm(sv.x2, l, P_CONV_LN_G, sv.ln3, sv.st3);
@@ -676,11 +676,8 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     branch_in(t.dA, t.tD, l, P_PROJ_B, 1.f, p_res, e.site(l, g.site_att_out));
     e.linear_wgrad(sv.att, t.tD, l, P_PROJ_W, P_PROJ_B, n, HD, D, false);
     e.linear_dgrad(t.tD, l, P_PROJ_W, n, HD, D, t.datt, nullptr, 0, 0.f, 0);
-    e.memset0(t.do_pad, g.pad_rows * HD * sizeof(bf16));
-    if (e.ok()) e.run_tagged("att_rows_gather", rb200_att_rows_gather(t.datt, t.do_pad, row_batch, row_pos, n, HD, Lp, 1, stream));
+    if (e.ok()) e.run_tagged("att_rows_pad", rb200_att_rows_pad(t.datt, t.do_pad, lens, B, HD, Lp, stream));
     bf16* wd = p_att > 0.f ? sv.wd : sv.w;
-    e.memset0(t.dband, g.dband_elems * sizeof(bf16));
-    e.memset0(t.dqu, 2 * g.pad_rows * HD * sizeof(bf16));  // dqu, dqv: their column sums run over all padded rows
     const bf16* dpos = t.dpos;
     if (g.fused_bwd) {
       if (e.ok())
@@ -696,6 +693,8 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
       if (g.slices > 1 && e.ok()) e.run_tagged("sum_slices", rb200_sum_slices(t.dpos_part, t.dpos, g.slices, (long long)g.band_w * HD, stream));
       dpos = t.dpos + (size_t)g.band_off * HD;  // the band's first columns lie before position 0
     } else {
+      e.memset0(t.dband, g.dband_elems * sizeof(bf16));
+      e.memset0(t.dqu, 2 * g.pad_rows * HD * sizeof(bf16));  // dqu, dqv: their column sums run over all padded rows
       {
         const long long o4[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
         e.bgemm(t.do_pad, sv.vv, t.dwd, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o4, B * H, H, lens, 1, 1, 0, 1.f, 0);

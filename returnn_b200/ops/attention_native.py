@@ -85,13 +85,9 @@ class _RelPosAttPacked(torch.autograd.Function):
         uf = u.float().contiguous() if u is not None else None
         vf = v.float().contiguous() if v is not None else None
         bf = torch.bfloat16
-        qu = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
-        qv = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
-        kk = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
-        vv = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
-        fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(qkv.data_ptr(), uf.data_ptr() if uf is not None else None, vf.data_ptr() if vf is not None else None,
-                      row_batch.data_ptr(), row_pos.data_ptr(), qu.data_ptr(), qv.data_ptr(), kk.data_ptr(), vv.data_ptr(), N, H, D, Lp,
+        qu, qv, kk, vv = torch.empty(4, B * Lp, HD, dtype=bf, device=dev)
+        fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(qkv.data_ptr(), _p(uf), _p(vf), lens.data_ptr(), qu.data_ptr(), qv.data_ptr(), kk.data_ptr(), vv.data_ptr(), B, H, D, Lp,
                       _lib.stream_ptr()), "att_prepare")
         _lib.count_launch()
         # P padded to Rp rows so that tile reads stay inside the tensor
@@ -123,8 +119,8 @@ class _RelPosAttPacked(torch.autograd.Function):
         _bgemm(wd, vv, o_pad, m=Lp, n=D, k=Lp, a_mn=False, b_mn=True, lda=Lp, ldb=HD, ldc=HD, a_shape=(B * H * Lp, Lp), b_shape=(B * Lp, HD),
                offs=(H * Lp, Lp, 0, 0, Lp, 0, 0, D, Lp * HD, D), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=True)
         out = torch.empty(N, HD, dtype=bf, device=dev)
-        gfn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(gfn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 0, _lib.stream_ptr()), "att_gather")
+        gfn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        _lib.check(gfn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, _lib.stream_ptr()), "att_gather")
         _lib.count_launch()
         ctx.save_for_backward(qu, qv, kk, vv, w, pos_p, row_batch, row_pos, lens, off)
         ctx.dims = (B, H, D, Lp, Rp, R, center, N, scale, p_drop)
@@ -140,9 +136,9 @@ class _RelPosAttPacked(torch.autograd.Function):
         HD = H * D
         bf = torch.bfloat16
         d_out = d_out.contiguous()
-        do_pad = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
-        gfn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(gfn(d_out.data_ptr(), do_pad.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 1, _lib.stream_ptr()), "att_scatter")
+        do_pad = torch.empty(B * Lp, HD, dtype=bf, device=dev)
+        gfn = _lib.bind("rb200_att_rows_pad", [_vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        _lib.check(gfn(d_out.data_ptr(), do_pad.data_ptr(), lens.data_ptr(), B, HD, Lp, _lib.stream_ptr()), "att_rows_pad")
         _lib.count_launch()
         drop = p_drop > 0.0
         seed = _seed_tensor(dev)
@@ -210,11 +206,11 @@ class _RelPosFlash(torch.autograd.Function):
         pos = pos.contiguous()
         uf = u.float().contiguous() if u is not None else None
         vf = v.float().contiguous() if v is not None else None
-        pads = torch.zeros(4, B * Lp, HD, dtype=bf, device=dev)  # q + u, q + v, k, v
+        pads = torch.empty(4, B * Lp, HD, dtype=bf, device=dev)  # q + u, q + v, k, v
         qu, qv, kk, vv = (pads[i].data_ptr() for i in range(4))
         s = _lib.stream_ptr()
-        fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(qkv.data_ptr(), _p(uf), _p(vf), row_batch.data_ptr(), row_pos.data_ptr(), qu, qv, kk, vv, N, H, 64, Lp, s), "att_prepare")
+        fn = _lib.bind("rb200_att_prepare", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+        _lib.check(fn(qkv.data_ptr(), _p(uf), _p(vf), lens.data_ptr(), qu, qv, kk, vv, B, H, 64, Lp, s), "att_prepare")
         o_pad = torch.empty(B * Lp, HD, dtype=torch.float32, device=dev)  # (the backward pass takes row sums of it)
         lse = torch.empty(B * H * Lp, dtype=torch.float32, device=dev)
         drop = p_drop > 0.0
@@ -247,15 +243,15 @@ class _RelPosFlash(torch.autograd.Function):
         rows = B * Lp
         d_out = d_out.contiguous()
         s = _lib.stream_ptr()
-        zeroed = torch.zeros(3, rows, HD, dtype=bf, device=dev)  # dO, dQu, dQv
-        do_pad, dqu, dqv = zeroed[0], zeroed[1], zeroed[2]
-        fn = _lib.bind("rb200_att_rows_gather", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(d_out.data_ptr(), do_pad.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, 1, s), "att_scatter")
+        padded = torch.empty(3, rows, HD, dtype=bf, device=dev)  # dO, dQu, dQv
+        do_pad, dqu, dqv = padded[0], padded[1], padded[2]
+        fn = _lib.bind("rb200_att_rows_pad", [_vp, _vp, _vp, _i32, _i32, _i32, _vp])
+        _lib.check(fn(d_out.data_ptr(), do_pad.data_ptr(), lens.data_ptr(), B, HD, Lp, s), "att_rows_pad")
         geo = (ctypes.c_int * 2)()
         fn = _lib.bind("rb200_rel_flash_band", [_i32, _i32, _vp, _vp])
         _lib.check(fn(Lp, center, ctypes.addressof(geo), ctypes.addressof(geo) + 4), "rel_flash_band")
         band_off, width = geo[0], geo[1]
-        band = torch.zeros(H * rows, width, dtype=bf, device=dev)
+        band = torch.empty(H * rows, width, dtype=bf, device=dev)
         scores = torch.empty(2, B * H * Lp, Lp, dtype=bf, device=dev)
         pw, ds = scores[0], scores[1]
         st = _gemm.status_tensor(dev)
@@ -288,7 +284,7 @@ class _RelPosFlash(torch.autograd.Function):
         for i, dt in enumerate((ctx.u_dtype, ctx.v_dtype)):
             if dt is not None:
                 t = torch.empty(HD, dtype=torch.float32, device=dev)
-                _gemm._grad_pre(zeroed[1 + i], None, None, t)
+                _gemm._grad_pre(padded[1 + i], None, None, t)
                 sums[i] = t.reshape(H, 64).to(dt)
         return dqkv, dpos[band_off: band_off + R], sums[0], sums[1], None, None, None, None, None, None, None, None
 

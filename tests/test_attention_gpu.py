@@ -277,3 +277,45 @@ def test_rel_pos_attention_dropout_gradients_over_several_tiles(D, T):
     for a, b in zip((got[0][:T], got[1]), torch.autograd.grad(out, [xr, pr], dy[:T].double())):
         assert (a.double() - b).norm() <= 1.2e-2 * b.norm()
     assert float(got[0][T:].abs().max()) == 0.0
+
+
+@gpu
+@pytest.mark.parametrize("lens,H", [([150, 192, 40], 2), ([64, 1], 1), ([65, 129, 0, 320], 3), ([512], 1)])
+@pytest.mark.parametrize("saved", [True, False])
+def test_rel_flash_bwd_writes_the_padding(lens, H, saved):
+    """buffers full of NaN come back with the values of zeroed ones: every column and row that no tile of keys fills is written as zero"""
+    import ctypes
+    from returnn_b200.ops import _lib, gemm as G
+
+    dev, bf, HD, B, L = "cuda", torch.bfloat16, H * 64, len(lens), max(lens)
+    Lp, R = (L + 63) // 64 * 64, 2 * L - 1
+    torch.manual_seed(5)
+    lens_t = torch.tensor(lens, dtype=torch.int32, device=dev)
+    valid = (torch.arange(Lp, device=dev)[None] < lens_t[:, None])
+    qu, qv, k, v, do = ((torch.randn(B, Lp, HD, device=dev) * valid[..., None]).to(bf) for _ in range(5))
+    pos, o = torch.randn(R, HD, device=dev).to(bf), torch.randn(B, Lp, HD, device=dev)
+    w = torch.rand(B, H, Lp, Lp, device=dev).to(bf) * 0.01
+    lse = torch.full((B, H, Lp), 12.0, device=dev)
+    vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    geo = (ctypes.c_int * 2)()
+    _lib.check(_lib.bind("rb200_rel_flash_band", [i32, i32, vp, vp])(Lp, L - 1, ctypes.addressof(geo), ctypes.addressof(geo) + 4), "band")
+    fn = _lib.bind("rb200_rel_flash_bwd", [vp] * 16 + [i32] * 5 + [f32, f32, vp, vp])
+    res = []
+    for fill in (0.0, float("nan")):
+        dqu, dqv, band = (torch.full(s, fill, device=dev, dtype=bf) for s in ((B, Lp, HD), (B, Lp, HD), (H, B, Lp, geo[1])))
+        pw, ds = w.clone(), torch.zeros(B, H, Lp, Lp, device=dev, dtype=bf)
+        _lib.check(fn(qu.data_ptr(), qv.data_ptr(), k.data_ptr(), v.data_ptr(), pos.data_ptr(), o.data_ptr(), do.data_ptr(), dqu.data_ptr(), dqv.data_ptr(),
+                      w.data_ptr() if saved else None, pw.data_ptr(), ds.data_ptr(), band.data_ptr(), lse.data_ptr(), None, lens_t.data_ptr(), B, H, Lp, R,
+                      L - 1, 0.125, 0.0, G.status_tensor(lens_t.device).data_ptr(), _lib.stream_ptr()), "rel_flash_bwd")
+        G.check_status()
+        res.append((dqu, dqv, band))
+    for a, b in zip(*res):
+        assert torch.isfinite(b).all() and torch.equal(a, b)
+    dqu, dqv, band = res[1]
+    assert not dqu[~valid].any() and not dqv[~valid].any() and not band[:, ~valid].any()
+    # row i of the band holds dS[i, j] at column center + j - i + offset, nothing else
+    i, j = torch.arange(Lp, device=dev)[:, None], torch.arange(Lp, device=dev)[None]
+    col = (L - 1 + j - i + geo[0]).clamp(0, geo[1] - 1)
+    inside = (valid[:, None, :, None] & valid[:, None, None, :]).expand(B, H, Lp, Lp)
+    want = torch.zeros_like(band.transpose(0, 1)).scatter_add(3, col.expand(B, H, Lp, Lp), ds * inside)
+    assert torch.equal(band.transpose(0, 1), want)
