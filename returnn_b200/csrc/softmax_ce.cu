@@ -20,10 +20,40 @@ __device__ __forceinline__ int row_head(const void* x, int64_t base, int v, int 
   return min(off ? (16 - off) / elem : 0, v);
 }
 
+// kArg: the arg max is wanted, kTot: the plain sum of the row is (label smoothing in the loss). Every class costs an exponential, and the
+// instructions around it are what kept the pass from the rate of its reads: with the position of the maximum searched and the sum taken for
+// every caller, 6001 x 32000 bf16 took 89 us (4.3 TB/s). The maximum of a group comes from packed 16-bit comparisons, and its position is
+// looked up only in batches that hold a new one; a batch of 32 classes changes the running maximum once.
+//
+// 16 bytes: 8 bf16 or 4 fp32 values
 template <bool kBf16>
+struct Chunk {
+  static constexpr int kN = kBf16 ? 8 : 4;
+  uint4 u;
+  __device__ __forceinline__ void load(const void* x, int64_t at) {
+    u = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(x) + at * (kBf16 ? 2 : 4));
+  }
+  __device__ __forceinline__ void fill_neg_inf() { u.x = u.y = u.z = u.w = kBf16 ? 0xff80ff80u : 0xff800000u; }
+  __device__ __forceinline__ float at(int i) const {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&u);
+    if (kBf16) return __uint_as_float(i & 1 ? w[i >> 1] & 0xffff0000u : w[i >> 1] << 16);
+    return __uint_as_float(w[i]);
+  }
+  __device__ __forceinline__ float max() const {
+    if (kBf16) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+      const float2 m = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+      return fmaxf(m.x, m.y);
+    }
+    return fmaxf(fmaxf(at(0), at(1)), fmaxf(at(2), at(3)));
+  }
+};
+constexpr int kBatch = 4;  // chunks that a thread has in flight
+
+template <bool kBf16, bool kArg, bool kTot>
 __global__ void __launch_bounds__(256)
 ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, float* __restrict__ loss, float* __restrict__ lse_out,
-              int v, float smoothing, int mode, int* __restrict__ argmax_out) {
+              int v, float smoothing, int* __restrict__ argmax_out) {
   constexpr int is_bf16 = kBf16 ? 1 : 0;
   const int64_t row = blockIdx.x;
   const int64_t base = row * (int64_t)v;
@@ -33,54 +63,65 @@ ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, floa
   const int v8 = head + ((v - head) & ~7);
   for (int c = threadIdx.x; c < head; c += blockDim.x) {
     float a = ld(logits, base + c, is_bf16);
-    if (a > mx) bi = c;
+    if (kArg && a > mx) bi = c;
     float nm = fmaxf(mx, a);
     const float nu = nm == -INFINITY ? 0.f : nm;  // (only classes of score -inf so far)
     sum = sum * __expf(mx - nu) + __expf(a - nu);
     mx = nm;
-    tot += a;
+    if (kTot) tot += a;
   }
-  // four independent 16-byte loads in flight per thread: the running max / sum chain is short, the loads are the latency
-#pragma unroll 4
-  for (int c = head + threadIdx.x * 8; c < v8; c += blockDim.x * 8) {
-    F8 a = load8(logits, base + c, is_bf16);
-    float lm = a.v[0];
-    int li = 0;
+  constexpr int kN = Chunk<kBf16>::kN;
+  for (int c0 = head + threadIdx.x * kN; c0 < v8; c0 += kBatch * 256 * kN) {
+    Chunk<kBf16> a[kBatch];
 #pragma unroll
-    for (int k = 1; k < 8; ++k)
-      if (a.v[k] > lm) {
-        lm = a.v[k];
-        li = k;
-      }
-    if (lm > mx) bi = c + li;
-    float nm = fmaxf(mx, lm);
+    for (int q = 0; q < kBatch; ++q) {
+      const int c = c0 + q * 256 * kN;
+      if (c < v8) a[q].load(logits, base + c);
+      else a[q].fill_neg_inf();
+    }
+    float lm = a[0].max();
+#pragma unroll
+    for (int q = 1; q < kBatch; ++q) lm = fmaxf(lm, a[q].max());
+    if (kArg && lm > mx) {
+#pragma unroll
+      for (int q = kBatch - 1; q >= 0; --q)
+#pragma unroll
+        for (int k = kN - 1; k >= 0; --k)
+          if (a[q].at(k) == lm) bi = c0 + q * 256 * kN + k;
+    }
+    const float nm = fmaxf(mx, lm);
     const float nu = nm == -INFINITY ? 0.f : nm;
     float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      s += __expf(a.v[k] - nu);
-      tot += a.v[k];
+    for (int q = 0; q < kBatch; ++q) {
+#pragma unroll
+      for (int k = 0; k < kN; ++k) s += __expf(a[q].at(k) - nu);
+      if (kTot && c0 + q * 256 * kN < v8) {
+#pragma unroll
+        for (int k = 0; k < kN; ++k) tot += a[q].at(k);
+      }
     }
     sum = sum * __expf(mx - nu) + s;
     mx = nm;
   }
   for (int c = v8 + threadIdx.x; c < v; c += blockDim.x) {
     float a = ld(logits, base + c, is_bf16);
-    if (a > mx) bi = c;
+    if (kArg && a > mx) bi = c;
     float nm = fmaxf(mx, a);
     const float nu = nm == -INFINITY ? 0.f : nm;  // (only classes of score -inf so far)
     sum = sum * __expf(mx - nu) + __expf(a - nu);
     mx = nm;
-    tot += a;
+    if (kTot) tot += a;
   }
   __shared__ float sh_m[8], sh_s[8], sh_t[8];
   __shared__ int sh_i[8];
   float wm = warp_max(mx);
   int wi = (mx == wm) ? bi : 0x7fffffff;
+  if (kArg)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) wi = min(wi, __shfl_xor_sync(0xffffffffu, wi, o));
+    for (int o = 16; o > 0; o >>= 1) wi = min(wi, __shfl_xor_sync(0xffffffffu, wi, o));
   float ws = warp_sum(mx == -INFINITY ? 0.f : sum * __expf(mx - wm));
-  float wt = warp_sum(tot);
+  float wt = kTot ? warp_sum(tot) : 0.f;
   if ((threadIdx.x & 31) == 0) {
     sh_m[threadIdx.x >> 5] = wm;
     sh_s[threadIdx.x >> 5] = ws;
@@ -98,13 +139,13 @@ ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, floa
       t += sh_t[w];
       if (sh_m[w] == m) am = min(am, sh_i[w]);
     }
-    if (argmax_out) argmax_out[row] = am < v ? am : 0;
+    if (kArg) argmax_out[row] = am < v ? am : 0;
     float lse = m + logf(s);
     int y = tgt[row];
     float xy = (y >= 0 && y < v) ? ld(logits, base + y, is_bf16) : 0.f;
     float nll = lse - xy;
     float l = nll;
-    if (smoothing > 0.f && mode == 0) {
+    if (kTot) {
       // other = mean over the v-1 non-target classes of (lse - x_c)
       float other = ((float)v * lse - t - nll) / (float)(v - 1);
       l = (1.f - smoothing) * nll + smoothing * other;
@@ -158,8 +199,12 @@ RB_EXPORT int rb200_softmax_ce_fwd(const void* logits, const int* tgt, float* lo
                                    int is_bf16, int mode, int* argmax_out, cudaStream_t stream) {
   if (rows <= 0) return RB_OK;
   if (v < 2) return RB_ERR_ARG;
-  if (is_bf16) ce_fwd_kernel<true><<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, loss, lse, v, smoothing, mode, argmax_out);
-  else ce_fwd_kernel<false><<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, loss, lse, v, smoothing, mode, argmax_out);
+  const bool arg = argmax_out != nullptr, tot = smoothing > 0.f && mode == 0;
+  auto kernel = is_bf16 ? (arg ? (tot ? ce_fwd_kernel<true, true, true> : ce_fwd_kernel<true, true, false>)
+                               : (tot ? ce_fwd_kernel<true, false, true> : ce_fwd_kernel<true, false, false>))
+                        : (arg ? (tot ? ce_fwd_kernel<false, true, true> : ce_fwd_kernel<false, true, false>)
+                               : (tot ? ce_fwd_kernel<false, false, true> : ce_fwd_kernel<false, false, false>));
+  kernel<<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, loss, lse, v, smoothing, argmax_out);
   return rb_check_launch("softmax_ce_fwd");
 }
 

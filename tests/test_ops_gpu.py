@@ -482,3 +482,37 @@ b = logmel.log_mel(x, **kw)
 assert (a - b).abs().max() < 1e-3, float((a - b).abs().max())
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+@gpu
+@pytest.mark.parametrize("v", [2, 7, 9, 33, 2049, 8191, 8192, 8200, 10025, 32000])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("smoothing,grad_only,with_argmax", [(0.0, False, False), (0.1, False, True), (0.1, True, True), (0.1, False, False)])
+def test_softmax_ce_forward_forms(v, dtype, smoothing, grad_only, with_argmax):
+    """every form of the forward kernel around its 16-byte pieces and batches; odd rows start off the 16-byte grid; ties, one row at the type's lowest value"""
+    from returnn_b200.ops.softmax_ce import softmax_cross_entropy
+
+    torch.manual_seed(v)
+    rows = 5
+    x = (torch.randn(rows, v, device="cuda") * 3).to(dtype)
+    x[1, v // 2] = x[1, v - 1] = 30.0  # a tie: the first index counts
+    x[2] = torch.finfo(dtype).min
+    x[3, : v // 2] = -torch.inf
+    t = torch.randint(v // 2, v, (rows,), device="cuda")
+    if smoothing and not grad_only:
+        x[3, : v // 2] = -50.0  # (classes of score -inf have no finite smoothed loss)
+        x[2] = -100.0
+    got = softmax_cross_entropy(x, t, smoothing, grad_only_smoothing=grad_only, with_argmax=with_argmax)
+    loss = got[0] if with_argmax else got
+    lp = torch.log_softmax(x.double(), -1)
+    want = -lp.gather(1, t[:, None])[:, 0]
+    if smoothing and not grad_only:
+        want = (1 - smoothing) * want + smoothing * (-lp.sum(-1) - want) / (v - 1)
+    # 32-bit sums over v classes; the smoothed loss is a difference of sums of v scores
+    # (at the type's lowest value the log of the sum is below the resolution of 32 bits: finite is all that can be asked)
+    assert torch.isfinite(loss).all()
+    loss, want = loss[[0, 1, 3, 4]], want[[0, 1, 3, 4]]
+    scale = lp[torch.isfinite(lp)].abs().max() if smoothing and not grad_only else want.abs().clamp(min=1.0)
+    assert ((loss.double() - want).abs() <= 2e-5 * scale + 1e-5).all()
+    if with_argmax:
+        assert torch.equal(got[1].long(), x.float().argmax(-1))
