@@ -26,6 +26,9 @@ int rb200_layer_norm_fwd(const void* x, const void* gamma, const void* beta, voi
 int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* part,
                             float* dgamma, float* dbeta, long long rows, int n, int n_part, int x_bf16, int w_bf16, int rms,
                             const void* dres, int accumulate, cudaStream_t stream);
+int rb200_layer_norm_bwd_branch(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* dgamma,
+                                float* dbeta, long long rows, int n, int w_bf16, int rms, const void* dres, void* out, float* sum, float scale,
+                                float p_drop, const long long* seed, const long long* offset, unsigned long long site, cudaStream_t stream);
 int rb200_gemm_bf16_batched(const void* a, const void* b, void* c, const void* bias, long long a_rows, long long a_cols, long long b_rows,
                             long long b_cols, int lda, int ldb, int ldc, int m, int n, int k, int a_mn_major, int b_mn_major, int bias_bf16,
                             int act, int out_fp32, int accumulate, float alpha, int batch, int heads, const long long* offs, const int* lens,
@@ -637,28 +640,37 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
   const float p_res = e.pdrop(d.p_res), p_ff = e.pdrop(d.p_ff), p_att = e.pdrop(d.p_att);
   const int n = g.n, D = g.D, F = g.F, HD = g.HD, Lp = g.Lp, Rp = g.Rp, B = g.B, H = g.H, Dh = g.Dh;
 
-  // dropout(residual-branch) backward + bias gradient:  dy = mask * scale * dx_total;  db += colsum(dy)
-  auto branch_in = [&](const void* dxt, void* dy, int l, int bi, float scale, float p, unsigned long long site_) {
-    if (!e.ok()) return;
-    e.run_tagged("colsum_dropout", colsum(dxt, dy, bi >= 0 ? e.g32(l, bi) : nullptr, n, D, scale, p, seed, offset, site_, stream));
+  // backward of a layer norm (dx, plus the residual gradient dres), and of the residual branch that takes dx as the gradient of its output:
+  // mask * scale * dx, returned (dx itself where that is the same), and the bias gradient of the branch's last linear layer
+  auto layer_norm_branch = [&](const void* x, const void* dy, int l, int gi, const float* stats, void* dx_, const void* dres, int bi, float scale,
+                               unsigned long long site_) -> const void* {
+    if (!e.ok()) return dx_;
+    void* out = p_res > 0.f || scale != 1.f ? t.tD : nullptr;
+    float* sum = e.g32(l, bi);
+    if (D <= 512 && e.g32(l, gi) && (out || sum)) {
+      e.run_tagged("layer_norm_bwd", rb200_layer_norm_bwd_branch(x, dy, e.p32(l, gi), stats, stats + n, dx_, e.g32(l, gi), e.g32(l, gi + 1), n, D, 0, 0, dres,
+                                                                 out, sum, scale, p_res, seed, offset, site_, stream));
+    } else {
+      e.layer_norm_bwd(x, dy, l, gi, stats, dx_, dres, t.ln_part);
+      if (out || sum) e.run_tagged("colsum_dropout", colsum(dx_, out, sum, n, D, scale, p_res, seed, offset, site_, stream));
+    }
+    return out ? out : dx_;
   };
 
   for (int l = layer_hi - 1; l >= layer_lo && e.ok(); --l) {
     const Saved& sv = sv_all[l];
     const void* x0 = l == 0 ? x_in : (const void*)sv_all[l - 1].out;
     // ---- final LayerNorm: dx (d out) -> dA (d x4)
-    e.layer_norm_bwd(sv.x4, dx, l, P_FIN_LN_G, sv.st5, t.dA, nullptr, t.ln_part);
+    const void* dy = layer_norm_branch(sv.x4, dx, l, P_FIN_LN_G, sv.st5, t.dA, nullptr, P_FF2_B2, d.ff_res_scale, e.site(l, g.site_ff2_out));
     // ---- feed-forward 2: dA -> dB (d x3)
-    branch_in(t.dA, t.tD, l, P_FF2_B2, d.ff_res_scale, p_res, e.site(l, g.site_ff2_out));
-    e.linear_wgrad(sv.a2, t.tD, l, P_FF2_W2, P_FF2_B2, n, F, D, false);
-    e.linear_dgrad(t.tD, l, P_FF2_W2, n, F, D, t.tW, sv.z2, 2, p_ff, e.site(l, g.site_ff2_act));
+    e.linear_wgrad(sv.a2, dy, l, P_FF2_W2, P_FF2_B2, n, F, D, false);
+    e.linear_dgrad(dy, l, P_FF2_W2, n, F, D, t.tW, sv.z2, 2, p_ff, e.site(l, g.site_ff2_act));
     e.linear_wgrad(sv.ln4, t.tW, l, P_FF2_W1, P_FF2_B1, n, D, F, true);
     e.linear_dgrad(t.tW, l, P_FF2_W1, n, D, F, t.tD2, nullptr, 0, 0.f, 0);
-    e.layer_norm_bwd(sv.x3, t.tD2, l, P_FF2_LN_G, sv.st4, t.dB, t.dA, t.ln_part);
+    dy = layer_norm_branch(sv.x3, t.tD2, l, P_FF2_LN_G, sv.st4, t.dB, t.dA, P_PW2_B, 1.f, e.site(l, g.site_conv_out));
     // ---- convolution module: dB -> dA (d x2)
-    branch_in(t.dB, t.tD, l, P_PW2_B, 1.f, p_res, e.site(l, g.site_conv_out));
-    e.linear_wgrad(sv.zc, t.tD, l, P_PW2_W, P_PW2_B, n, D, D, false);
-    e.linear_dgrad(t.tD, l, P_PW2_W, n, D, D, t.tD2, nullptr, 0, 0.f, 0);
+    e.linear_wgrad(sv.zc, dy, l, P_PW2_W, P_PW2_B, n, D, D, false);
+    e.linear_dgrad(dy, l, P_PW2_W, n, D, D, t.tD2, nullptr, 0, 0.f, 0);
     if (e.ok()) {
       e.run_tagged("bn_silu_bwd_ex", rb200_bn_silu_bwd_ex(sv.y, t.tD2, sv.bn_ms, sv.bn_ms + D, e.p32(l, P_BN_G), e.p32(l, P_BN_B), t.tD3, t.bn_part, bn_tiles_a(n), t.sum_ds,
                                  t.sum_ds_yh, n, D, 1, e.g32(l, P_BN_G), e.g32(l, P_BN_B), stream));
@@ -671,11 +683,10 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     }
     e.linear_wgrad(sv.ln3, t.tW, l, P_PW1_W, P_PW1_B, n, D, 2 * D, true);
     e.linear_dgrad(t.tW, l, P_PW1_W, n, D, 2 * D, t.tD2, nullptr, 0, 0.f, 0);
-    e.layer_norm_bwd(sv.x2, t.tD2, l, P_CONV_LN_G, sv.st3, t.dA, t.dB, t.ln_part);
+    dy = layer_norm_branch(sv.x2, t.tD2, l, P_CONV_LN_G, sv.st3, t.dA, t.dB, P_PROJ_B, 1.f, e.site(l, g.site_att_out));
     // ---- self-attention: dA -> dB (d x1)
-    branch_in(t.dA, t.tD, l, P_PROJ_B, 1.f, p_res, e.site(l, g.site_att_out));
-    e.linear_wgrad(sv.att, t.tD, l, P_PROJ_W, P_PROJ_B, n, HD, D, false);
-    e.linear_dgrad(t.tD, l, P_PROJ_W, n, HD, D, t.datt, nullptr, 0, 0.f, 0);
+    e.linear_wgrad(sv.att, dy, l, P_PROJ_W, P_PROJ_B, n, HD, D, false);
+    e.linear_dgrad(dy, l, P_PROJ_W, n, HD, D, t.datt, nullptr, 0, 0.f, 0);
     if (e.ok()) e.run_tagged("att_rows_pad", rb200_att_rows_pad(t.datt, t.do_pad, lens, B, HD, Lp, stream));
     bf16* wd = p_att > 0.f ? sv.wd : sv.w;
     const bf16* dpos = t.dpos;
@@ -719,11 +730,10 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     e.linear_wgrad(sinus, dpos, l, P_POS_W, -1, g.R, D, HD, false);
     e.linear_wgrad(sv.ln2, t.tW, l, P_QKV_W, P_QKV_B, n, D, 3 * HD, true);
     e.linear_dgrad(t.tW, l, P_QKV_W, n, D, 3 * HD, t.tD2, nullptr, 0, 0.f, 0);
-    e.layer_norm_bwd(sv.x1, t.tD2, l, P_ATT_LN_G, sv.st2, t.dB, t.dA, t.ln_part);
+    dy = layer_norm_branch(sv.x1, t.tD2, l, P_ATT_LN_G, sv.st2, t.dB, t.dA, P_FF1_B2, d.ff_res_scale, e.site(l, g.site_ff_out));
     // ---- feed-forward 1: dB -> dx (d x0)
-    branch_in(t.dB, t.tD, l, P_FF1_B2, d.ff_res_scale, p_res, e.site(l, g.site_ff_out));
-    e.linear_wgrad(sv.a1, t.tD, l, P_FF1_W2, P_FF1_B2, n, F, D, false);
-    e.linear_dgrad(t.tD, l, P_FF1_W2, n, F, D, t.tW, sv.z1, 2, p_ff, e.site(l, g.site_ff_act));
+    e.linear_wgrad(sv.a1, dy, l, P_FF1_W2, P_FF1_B2, n, F, D, false);
+    e.linear_dgrad(dy, l, P_FF1_W2, n, F, D, t.tW, sv.z1, 2, p_ff, e.site(l, g.site_ff_act));
     e.linear_wgrad(sv.ln1, t.tW, l, P_FF1_W1, P_FF1_B1, n, D, F, true);
     e.linear_dgrad(t.tW, l, P_FF1_W1, n, D, F, t.tD2, nullptr, 0, 0.f, 0);
     e.layer_norm_bwd(x0, t.tD2, l, P_FF1_LN_G, sv.st1, dx, t.dB, t.ln_part);

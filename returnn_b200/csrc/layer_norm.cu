@@ -213,6 +213,11 @@ ln_bwd_kernel(const void* __restrict__ x, const void* __restrict__ dy, const voi
 // exactly the 16-byte pieces it reads back itself (no barrier between fetch and use), with the rows' mean / rstd parked in the
 // lanes of the warp. The 16 warps' column sums meet in the same shared memory afterwards and leave as one atomic per column and
 // CTA: no partials buffer and no second kernel.
+//
+// BRANCH: in a residual stack the gradient that this layer norm leaves is also that of the next residual branch's output: the kernel then
+// writes out = dropout mask * scale * dx as well (null: the branch takes dx as it is) and adds the column sums of that to `sum`, the bias
+// gradient of the linear layer that ends the branch. As a kernel of its own that read dx back (7.4 us at 6740 x 512, 48 times in a 12-layer
+// Conformer pass).
 constexpr int kBwdAccWarps = 16;
 constexpr int kBwdAccDepth = 4;
 
@@ -225,26 +230,43 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int CHUNKS>
+struct LnBranch {
+  __nv_bfloat16* out;
+  float* sum;
+  float scale, p_drop;
+  const long long *seed, *offset;
+  unsigned long long site;
+};
+
+template <int CHUNKS, bool BRANCH>
 __global__ void __launch_bounds__(kBwdAccWarps * 32, 1)
 ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, const void* __restrict__ gamma,
                   const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
                   float* __restrict__ dgamma, float* __restrict__ dbeta, int64_t rows, int n, int w_bf16, int rms,
-                  const __nv_bfloat16* __restrict__ dres, unsigned int* __restrict__ done, void* __restrict__ gamma_out, void* __restrict__ beta_out) {
+                  const __nv_bfloat16* __restrict__ dres, unsigned int* __restrict__ done, void* __restrict__ gamma_out, void* __restrict__ beta_out,
+                  const LnBranch br) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
-  extern __shared__ __align__(16) unsigned char smem_raw[];  // [warps][depth][3][n] bf16, later [warps][2][n] fp32
+  extern __shared__ __align__(16) unsigned char smem_raw[];  // [warps][depth][3][n] bf16, later [warps][2 or 3][n] fp32
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(smem_raw) + (size_t)warp * kBwdAccDepth * 3 * n;
-  F8 g[CHUNKS], acc_g[CHUNKS], acc_b[CHUNKS];
+  F8 g[CHUNKS], acc_g[CHUNKS], acc_b[CHUNKS], acc_y[BRANCH ? CHUNKS : 1];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
     const int col = (c * 32 + lane) * 8;
     if (col < n) g[c] = load8(gamma, col, w_bf16);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc_g[c].v[i] = acc_b[c].v[i] = 0.f;
+    for (int i = 0; i < 8; ++i) {
+      acc_g[c].v[i] = acc_b[c].v[i] = 0.f;
+      if (BRANCH) acc_y[c].v[i] = 0.f;
+    }
   }
+  const bool drop = BRANCH && br.p_drop > 0.f;
+  const uint64_t sd = drop ? (uint64_t)br.seed[0] : 0, off = drop ? (uint64_t)br.offset[0] + br.site : 0;
+  const uint2 key = make_uint2((uint32_t)sd, (uint32_t)(sd >> 32));
+  const uint32_t thresh = drop ? rb_dropout_thresh16(br.p_drop) : 0u;
+  const float keep = drop ? br.scale / (1.f - br.p_drop) : br.scale;
   const int64_t stride = (int64_t)gridDim.x * kBwdAccWarps;
   const int64_t row0 = (int64_t)blockIdx.x * kBwdAccWarps + warp;
   float my_mean = 0.f, my_rstd = 0.f;  // of the row in ring slot `lane` (lanes < depth)
@@ -285,14 +307,15 @@ ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
     const float mean = __shfl_sync(0xffffffffu, my_mean, slot), rstd = __shfl_sync(0xffffffffu, my_rstd, slot);
     const int64_t base = row * (int64_t)n;
     const __nv_bfloat16* src = ring + (size_t)slot * 3 * n;
-    F8 xh[CHUNKS], d[CHUNKS], res[CHUNKS];
+    F8 xh[CHUNKS];
+    uint4 d_raw[CHUNKS], res[CHUNKS];  // unpacked where they are used: registers
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
       const int col = (c * 32 + lane) * 8;
       if (col < n) {
         unpack(*reinterpret_cast<const uint4*>(src + col), xh[c]);
-        unpack(*reinterpret_cast<const uint4*>(src + n + col), d[c]);
-        if (dres) unpack(*reinterpret_cast<const uint4*>(src + 2 * n + col), res[c]);
+        d_raw[c] = *reinterpret_cast<const uint4*>(src + n + col);
+        if (dres) res[c] = *reinterpret_cast<const uint4*>(src + 2 * n + col);
       }
     }
     fetch(row + (int64_t)kBwdAccDepth * stride, slot);  // the slot is in registers now
@@ -301,14 +324,16 @@ ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
     for (int c = 0; c < CHUNKS; ++c) {
       const int col = (c * 32 + lane) * 8;
       if (col < n) {
+        F8 d;
+        unpack(d_raw[c], d);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           xh[c].v[i] = (xh[c].v[i] - mean) * rstd;
-          const float gd = g[c].v[i] * d[c].v[i];
+          const float gd = g[c].v[i] * d.v[i];
           s1 += gd;
           s2 += gd * xh[c].v[i];
-          acc_g[c].v[i] += d[c].v[i] * xh[c].v[i];
-          acc_b[c].v[i] += d[c].v[i];
+          acc_g[c].v[i] += d.v[i] * xh[c].v[i];
+          acc_b[c].v[i] += d.v[i];
         }
       }
     }
@@ -318,40 +343,68 @@ ln_bwd_acc_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
     for (int c = 0; c < CHUNKS; ++c) {
       const int col = (c * 32 + lane) * 8;
       if (col < n) {
-        F8 o;
+        F8 o, d;
+        unpack(d_raw[c], d);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          o.v[i] = rstd * (g[c].v[i] * d[c].v[i] - s1 - xh[c].v[i] * s2);
-          if (dres) o.v[i] += res[c].v[i];
+        for (int i = 0; i < 8; ++i) o.v[i] = rstd * (g[c].v[i] * d.v[i] - s1 - xh[c].v[i] * s2);
+        if (dres) {
+          F8 rs;
+          unpack(res[c], rs);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o.v[i] += rs.v[i];
         }
         store8(dx, base + col, o, 1);
+        if (BRANCH) {  // from the rounded values, which are the operands of the products that follow
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o.v[i] = __bfloat162float(__float2bfloat16(o.v[i]));
+          if (br.out) {
+            if (drop) {
+              rb_dropout_apply8(key, off + (uint64_t)(base + col), thresh, keep, o.v);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o.v[i] *= keep;
+            }
+            store8(br.out, base + col, o, 1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o.v[i] = __bfloat162float(__float2bfloat16(o.v[i]));
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc_y[c].v[i] += o.v[i];
+        }
       }
     }
     slot = slot + 1 == kBwdAccDepth ? 0 : slot + 1;
   }
   cp_async_wait<0>();
-  __syncthreads();  // every warp is done with its ring: the memory becomes [warps][2][n] fp32
+  __syncthreads();  // every warp is done with its ring: the memory becomes [warps][kSums][n] fp32
+  constexpr int kSums = BRANCH ? 3 : 2;
   float* sums = reinterpret_cast<float*>(smem_raw);
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
     const int col = (c * 32 + lane) * 8;
     if (col < n) {
-      float* pg = sums + (size_t)(warp * 2) * n + col;
+      float* pg = sums + (size_t)(warp * kSums) * n + col;
       *reinterpret_cast<float4*>(pg) = make_float4(acc_g[c].v[0], acc_g[c].v[1], acc_g[c].v[2], acc_g[c].v[3]);
       *reinterpret_cast<float4*>(pg + 4) = make_float4(acc_g[c].v[4], acc_g[c].v[5], acc_g[c].v[6], acc_g[c].v[7]);
       *reinterpret_cast<float4*>(pg + n) = make_float4(acc_b[c].v[0], acc_b[c].v[1], acc_b[c].v[2], acc_b[c].v[3]);
       *reinterpret_cast<float4*>(pg + n + 4) = make_float4(acc_b[c].v[4], acc_b[c].v[5], acc_b[c].v[6], acc_b[c].v[7]);
+      if (BRANCH) {
+        *reinterpret_cast<float4*>(pg + 2 * n) = make_float4(acc_y[c].v[0], acc_y[c].v[1], acc_y[c].v[2], acc_y[c].v[3]);
+        *reinterpret_cast<float4*>(pg + 2 * n + 4) = make_float4(acc_y[c].v[4], acc_y[c].v[5], acc_y[c].v[6], acc_y[c].v[7]);
+      }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) {  // i < n: dgamma column i, else dbeta column i - n
+  for (int i = threadIdx.x; i < kSums * n; i += blockDim.x) {  // i < n: dgamma column i, else dbeta column i - n, then the branch's sums
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < kBwdAccWarps; ++w) t += sums[(size_t)w * 2 * n + i];
+    for (int w = 0; w < kBwdAccWarps; ++w) t += sums[(size_t)w * kSums * n + i];
     if (i < n) {
       if (dgamma) atomicAdd(dgamma + i, t);
-    } else if (dbeta) {
-      atomicAdd(dbeta + i - n, t);
+    } else if (i < 2 * n) {
+      if (dbeta) atomicAdd(dbeta + i - n, t);
+    } else if (br.sum) {
+      atomicAdd(br.sum + i - 2 * n, t);
     }
   }
   if (!done) return;
@@ -434,28 +487,28 @@ RB_EXPORT int rb200_layer_norm_fwd(const void* x, const void* gamma, const void*
 // as gamma_out / beta_out in the type of the parameters
 static int ln_bwd_acc(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta,
                       long long rows, int n, int w_bf16, int rms, const void* dres, unsigned int* done, void* gamma_out, void* beta_out,
-                      cudaStream_t stream) {
+                      const LnBranch* branch, cudaStream_t stream) {
   int ctas = (int)((rows + kBwdAccWarps - 1) / kBwdAccWarps);
   if (ctas > 148) ctas = 148;
-  const size_t sm = (size_t)kBwdAccWarps * kBwdAccDepth * 3 * n * sizeof(__nv_bfloat16);  // >= the [warps][2][n] fp32 it becomes at the end
+  const size_t sm = (size_t)kBwdAccWarps * kBwdAccDepth * 3 * n * sizeof(__nv_bfloat16);  // >= the [warps][3][n] fp32 it becomes at the end
   const int ch = (n + 255) / 256;
-  static bool attr_set[2] = {false, false};
-#define LN_ACC(C)                                                                                                                       \
-if (!attr_set[C - 1]) {                                                                                                               \
-  if (cudaFuncSetAttribute(ln_bwd_acc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)kBwdAccWarps * kBwdAccDepth * 3 * 512 * 2)) != cudaSuccess) { \
-    rb_set_error("layer_norm_bwd_acc: cannot reserve shared memory");                                                                 \
-    return RB_ERR_LAUNCH;                                                                                                              \
-  }                                                                                                                                   \
-  attr_set[C - 1] = true;                                                                                                             \
-}                                                                                                                                     \
-rb_launch_pdl(ln_bwd_acc_kernel<C>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, gamma, mean, rstd, \
-                                                               (__nv_bfloat16*)dx, dgamma, dbeta, rows, n, w_bf16, rms,              \
-                                                               (const __nv_bfloat16*)dres, done, gamma_out, beta_out)
-  if (ch <= 1) {
-    LN_ACC(1);
-  } else {
-    LN_ACC(2);
-  }
+  static bool attr_set[2][2] = {{false, false}, {false, false}};
+#define LN_ACC(C, B)                                                                                                                    \
+  do {                                                                                                                                  \
+    if (!attr_set[C - 1][B]) {                                                                                                          \
+      if (cudaFuncSetAttribute(ln_bwd_acc_kernel<C, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)kBwdAccWarps * kBwdAccDepth * 3 * 512 * 2)) != cudaSuccess) { \
+        rb_set_error("layer_norm_bwd_acc: cannot reserve shared memory");                                                               \
+        return RB_ERR_LAUNCH;                                                                                                           \
+      }                                                                                                                                 \
+      attr_set[C - 1][B] = true;                                                                                                        \
+    }                                                                                                                                   \
+    rb_launch_pdl(ln_bwd_acc_kernel<C, B>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, gamma, mean, rstd, \
+                  (__nv_bfloat16*)dx, dgamma, dbeta, rows, n, w_bf16, rms, (const __nv_bfloat16*)dres, done, gamma_out, beta_out, branch ? *branch : LnBranch{});     \
+  } while (0)
+  if (ch <= 1 && branch) LN_ACC(1, true);
+  else if (ch <= 1) LN_ACC(1, false);
+  else if (branch) LN_ACC(2, true);
+  else LN_ACC(2, false);
 #undef LN_ACC
   return rb_check_launch("layer_norm_bwd_acc");
 }
@@ -470,7 +523,7 @@ RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void*
   }
   if (n_part <= 0) return RB_ERR_ARG;
   if (accumulate && x_bf16 && n <= 512 && rows > 0 && (dgamma || dbeta))
-    return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, rows, n, w_bf16, rms, dres, nullptr, nullptr, nullptr, stream);
+    return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, rows, n, w_bf16, rms, dres, nullptr, nullptr, nullptr, nullptr, stream);
   dim3 grid(n_part), block(kWarpsPerCta * 32);
   size_t smem = (size_t)kWarpsPerCta * 2 * n * sizeof(float);
   int chunks = (n + 255) / 256;
@@ -490,6 +543,20 @@ RB_EXPORT int rb200_layer_norm_bwd_ex(const void* x, const void* dy, const void*
   return rb_check_launch("layer_norm_bwd_reduce");
 }
 
+// rb200_layer_norm_bwd_ex on bf16 rows of n <= 512 columns with sums that are added to, for a layer norm whose dx is the gradient of a residual
+// branch's output too: out (bf16, may be null: the branch takes dx) = dropout mask * scale * dx, sum[c] (may be null) += its column sums
+RB_EXPORT int rb200_layer_norm_bwd_branch(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* dgamma,
+                                          float* dbeta, long long rows, int n, int w_bf16, int rms, const void* dres, void* out, float* sum, float scale,
+                                          float p_drop, const long long* seed, const long long* offset, unsigned long long site, cudaStream_t stream) {
+  if (n % 8 != 0 || n <= 0 || n > 512) {
+    rb_set_error("layer_norm_bwd_branch: n=%d must be a multiple of 8 and <= 512", n);
+    return RB_ERR_ARG;
+  }
+  if (rows <= 0) return RB_OK;
+  const LnBranch br = {(__nv_bfloat16*)out, sum, scale, p_drop, seed, offset, site};
+  return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, rows, n, w_bf16, rms, dres, nullptr, nullptr, nullptr, &br, stream);
+}
+
 // bf16 rows of n <= 512 columns (a multiple of 8): dx, and dgamma / dbeta (either may be null) in the type of gamma. work: 2 n + 1 words
 RB_EXPORT int rb200_layer_norm_bwd_typed(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, float* work,
                                          void* dgamma, void* dbeta, long long rows, int n, int w_bf16, int rms, cudaStream_t stream) {
@@ -503,7 +570,7 @@ RB_EXPORT int rb200_layer_norm_bwd_typed(const void* x, const void* dy, const vo
     return RB_ERR_LAUNCH;
   }
   return ln_bwd_acc(x, dy, gamma, mean, rstd, dx, work, work + n, rows, n, w_bf16, rms, nullptr, reinterpret_cast<unsigned int*>(work + 2 * n), dgamma, dbeta,
-                    stream);
+                    nullptr, stream);
 }
 
 RB_EXPORT int rb200_layer_norm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,

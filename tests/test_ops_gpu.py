@@ -516,3 +516,48 @@ def test_softmax_ce_forward_forms(v, dtype, smoothing, grad_only, with_argmax):
     assert ((loss.double() - want).abs() <= 2e-5 * scale + 1e-5).all()
     if with_argmax:
         assert torch.equal(got[1].long(), x.float().argmax(-1))
+
+
+@gpu
+@pytest.mark.parametrize("rows,n", [(1, 8), (37, 256), (33, 264), (2368 * 2 + 5, 512)])
+@pytest.mark.parametrize("scale,p,with_out,with_sum", [(1.0, 0.0, False, True), (0.5, 0.0, True, True), (0.5, 0.25, True, True), (1.0, 0.1, True, False)])
+def test_layer_norm_bwd_with_the_branch(rows, n, scale, p, with_out, with_sum):
+    """the layer norm of a residual stack: dx and the sums as without a branch, the branch's gradient and its column sums from the rounded dx"""
+    import ctypes
+    from returnn_b200.ops import _lib
+
+    torch.manual_seed(rows + n)
+    dev, bf = "cuda", torch.bfloat16
+    x, dy, dres = (torch.randn(rows, n, device=dev).to(bf) for _ in range(3))
+    gam = torch.randn(n, device=dev) * 0.5 + 1.0
+    mean, rstd = x.float().mean(1).contiguous(), (x.float().var(1, unbiased=False) + 1e-6).rsqrt().contiguous()
+    seed = torch.tensor([1234, 96], dtype=torch.int64, device=dev)
+    vp, i32, i64, f32, u64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_ulonglong
+    s = _lib.stream_ptr()
+    dx0, dx, out = (torch.empty_like(x) for _ in range(3))
+    g0, b0, g1, b1 = (torch.zeros(n, device=dev) for _ in range(4))
+    sums = torch.ones(n, device=dev)
+    part = torch.empty(2 * 592 * n, device=dev)
+    fn = _lib.bind("rb200_layer_norm_bwd_ex", [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, vp, i32, vp])
+    _lib.check(fn(x.data_ptr(), dy.data_ptr(), gam.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx0.data_ptr(), part.data_ptr(), g0.data_ptr(),
+                  b0.data_ptr(), rows, n, 416, 1, 0, 0, dres.data_ptr(), 1, s), "ln_bwd")
+    fn = _lib.bind("rb200_layer_norm_bwd_branch", [vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, vp, vp, vp, f32, f32, vp, vp, u64, vp])
+    _lib.check(fn(x.data_ptr(), dy.data_ptr(), gam.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(), g1.data_ptr(), b1.data_ptr(), rows, n, 0, 0,
+                  dres.data_ptr(), out.data_ptr() if with_out else None, sums.data_ptr() if with_sum else None, scale, p, seed.data_ptr(),
+                  seed[1:].data_ptr(), 64, s), "ln_bwd_branch")
+    assert torch.equal(dx, dx0)
+    torch.testing.assert_close(g1, g0, atol=1e-5 * rows, rtol=1e-4)  # (sums of atomics in another order)
+    torch.testing.assert_close(b1, b0, atol=1e-5 * rows, rtol=1e-4)
+    branch = dx
+    if with_out:
+        kept = out != 0
+        if p:
+            assert abs(kept.float().mean().item() - (1 - p)) < 0.02 + 2 / (rows * n) ** 0.5
+        want = torch.where(kept, dx.float() * (scale / (1 - p)), torch.zeros((), device=dev)).to(bf)
+        torch.testing.assert_close(out, want, atol=0, rtol=2 ** -7)
+        branch = out
+    if with_sum:
+        want = branch.double().sum(0) + 1.0
+        assert ((sums.double() - want).abs() <= 1e-6 * branch.double().abs().sum(0) + 1e-6).all()
+    else:
+        assert (sums == 1).all()
