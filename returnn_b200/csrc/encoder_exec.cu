@@ -42,7 +42,7 @@ int rb200_att_softmax_bwd_ex(const void* w, const void* dwd, int dwd_bf16, void*
 int rb200_att_redrop(const void* w, void* wd, const int* lens, int batch, int heads, int lp, float p_drop, const long long* seed,
                      const long long* offset, cudaStream_t stream);
 int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* dk, const void* dv, const int* row_batch, const int* row_pos, void* dqkv,
-                        int n_rows, int heads, int dim, int lp, cudaStream_t stream);
+                        float* sum_qkv, float* sum_u, float* sum_v, int n_rows, int heads, int dim, int lp, int accumulate, cudaStream_t stream);
 int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp,
                           cudaStream_t stream);
 int rb200_att_rows_pad(const void* src, void* dst, const int* lens, int batch, int width, int lp, cudaStream_t stream);
@@ -705,7 +705,6 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
       dpos = t.dpos + (size_t)g.band_off * HD;  // the band's first columns lie before position 0
     } else {
       e.memset0(t.dband, g.dband_elems * sizeof(bf16));
-      e.memset0(t.dqu, 2 * g.pad_rows * HD * sizeof(bf16));  // dqu, dqv: their column sums run over all padded rows
       {
         const long long o4[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
         e.bgemm(t.do_pad, sv.vv, t.dwd, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o4, B * H, H, lens, 1, 1, 0, 1.f, 0);
@@ -724,11 +723,10 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
                 d.att_scale, 0);
       }
     }
-    if (e.ok()) e.run_tagged("att_pack_dqkv", rb200_att_pack_dqkv(t.dqu, t.dqv, t.dk, t.dv, row_batch, row_pos, t.tW, n, H, Dh, Lp, stream));
-    if (e.ok() && e.g32(l, P_POS_U)) e.run_tagged("colsum", colsum(t.dqu, nullptr, e.g32(l, P_POS_U), (int)g.pad_rows, HD, 1.f, 0.f, nullptr, nullptr, 0, stream));
-    if (e.ok() && e.g32(l, P_POS_V)) e.run_tagged("colsum", colsum(t.dqv, nullptr, e.g32(l, P_POS_V), (int)g.pad_rows, HD, 1.f, 0.f, nullptr, nullptr, 0, stream));
+    if (e.ok()) e.run_tagged("att_pack_dqkv", rb200_att_pack_dqkv(t.dqu, t.dqv, t.dk, t.dv, row_batch, row_pos, t.tW,
+                                                                e.g32(l, P_QKV_B), e.g32(l, P_POS_U), e.g32(l, P_POS_V), n, H, Dh, Lp, 1, stream));
     e.linear_wgrad(sinus, dpos, l, P_POS_W, -1, g.R, D, HD, false);
-    e.linear_wgrad(sv.ln2, t.tW, l, P_QKV_W, P_QKV_B, n, D, 3 * HD, true);
+    e.linear_wgrad(sv.ln2, t.tW, l, P_QKV_W, P_QKV_B, n, D, 3 * HD, false);
     e.linear_dgrad(t.tW, l, P_QKV_W, n, D, 3 * HD, t.tD2, nullptr, 0, 0.f, 0);
     dy = layer_norm_branch(sv.x1, t.tD2, l, P_ATT_LN_G, sv.st2, t.dB, t.dA, P_FF1_B2, d.ff_res_scale, e.site(l, g.site_ff_out));
     // ---- feed-forward 1: dB -> dx (d x0)

@@ -490,6 +490,7 @@ sum_slices_kernel(const float4* __restrict__ x, Out* __restrict__ y, int slices,
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n4) return;
   float4 s = x[i];
+#pragma unroll 8  // (loads ahead of the sums, which keep their order)
   for (int k = 1; k < slices; ++k) {
     const float4 v = x[k * n4 + i];
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;

@@ -69,6 +69,31 @@ def _bgemm(a, b, c, *, m, n, k, a_mn, b_mn, lda, ldb, ldc, a_shape, b_shape, off
     _lib.count_launch()
 
 
+def _pack_dqkv(dqu, dqv, dk, dv, row_batch, row_pos, N, H, D, Lp, u_dtype, v_dtype):
+    """packed dqkv and the gradients of the two position biases (None without a dtype), ordered sums over the rows"""
+    dev, HD = dqu.device, H * D
+    s = _lib.stream_ptr()
+    dqkv = torch.empty(N, 3 * HD, dtype=torch.bfloat16, device=dev)
+    biases = N > 0 and (u_dtype is not None or v_dtype is not None)
+    slices = _lib.bind("rb200_att_pack_slices", [_i32, _i32, _i32])(N, H, D) if biases else 0
+    part = torch.empty(slices, 2, HD, dtype=torch.float32, device=dev) if biases else None
+    fn = _lib.bind("rb200_att_pack_dqkv", [_vp] * 10 + [_i32] * 5 + [_vp])
+    _lib.check(fn(dqu.data_ptr(), dqv.data_ptr(), dk.data_ptr(), dv.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), dqkv.data_ptr(), None, _p(part),
+                  None, N, H, D, Lp, 0, s), "att_pack_dqkv")
+    _lib.count_launch()
+    if not biases:
+        zeros = [None if dt is None else torch.zeros(H, D, dtype=dt, device=dev) for dt in (u_dtype, v_dtype)]
+        return dqkv, zeros[0], zeros[1]
+    sums = part[0]
+    if slices > 1:
+        sums = torch.empty(2, HD, dtype=torch.float32, device=dev)
+        fn = _lib.bind("rb200_sum_slices_f32", [_vp, _vp, _i32, _i64, _vp])
+        _lib.check(fn(part.data_ptr(), sums.data_ptr(), slices, 2 * HD, s), "sum_slices")
+        _lib.count_launch()
+    du, dvb = (None if dt is None else sums[i].reshape(H, D).to(dt) for i, dt in enumerate((u_dtype, v_dtype)))
+    return dqkv, du, dvb
+
+
 class _RelPosAttPacked(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, pos, u, v, row_batch, row_pos, lens, B, H, D, max_len, scale, p_drop):
@@ -166,7 +191,7 @@ class _RelPosAttPacked(torch.autograd.Function):
         _lib.count_launch()
         del dwd
         # 6. dQu = scale * dS K
-        dqu = torch.zeros(B * Lp, HD, dtype=bf, device=dev)  # zero tails: the column sums below run over all rows
+        dqu = torch.empty(B * Lp, HD, dtype=bf, device=dev)
         _bgemm(ds, kk, dqu, m=Lp, n=D, k=Lp, a_mn=False, b_mn=True, lda=Lp, ldb=HD, ldc=HD, a_shape=(B * H * Lp, Lp), b_shape=(B * Lp, HD),
                offs=(H * Lp, Lp, 0, 0, Lp, 0, 0, D, Lp * HD, D), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=True, alpha=scale)
         # 7. dK = scale * dS^T Qu
@@ -174,20 +199,14 @@ class _RelPosAttPacked(torch.autograd.Function):
         _bgemm(ds, qu, dk_pad, m=Lp, n=D, k=Lp, a_mn=True, b_mn=True, lda=Lp, ldb=HD, ldc=HD, a_shape=(B * H * Lp, Lp), b_shape=(B * Lp, HD),
                offs=(H * Lp, Lp, 0, 0, Lp, 0, 0, D, Lp * HD, D), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=True, alpha=scale)
         # 8. dQv = scale * dG P
-        dqv = torch.zeros(B * Lp, HD, dtype=bf, device=dev)
+        dqv = torch.empty(B * Lp, HD, dtype=bf, device=dev)
         _bgemm(dg, pos_p, dqv, m=Lp, n=D, k=R, a_mn=False, b_mn=True, lda=Rp, ldb=HD, ldc=HD, a_shape=(H * B * Lp, Rp), b_shape=(R, HD),
                offs=(Lp, B * Lp, 0, 0, 0, 0, 0, D, Lp * HD, D), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=False, alpha=scale)
         # 9. dP[h] = scale * dG[h]^T Qv[h] over all rows of all sequences
         dpos = torch.empty(R, HD, dtype=bf, device=dev)
         _bgemm(dg, qv, dpos, m=R, n=D, k=B * Lp, a_mn=True, b_mn=True, lda=Rp, ldb=HD, ldc=HD, a_shape=(H * B * Lp, Rp), b_shape=(B * Lp, HD),
                offs=(0, B * Lp, 0, 0, 0, 0, 0, D, 0, D), batch=H, heads=H, lens=None, m_l=False, n_l=False, k_l=False, alpha=scale)
-        dqkv = torch.empty(N, 3 * HD, dtype=bf, device=dev)
-        pfn = _lib.bind("rb200_att_pack_dqkv", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(pfn(dqu.data_ptr(), dqv.data_ptr(), dk_pad.data_ptr(), dv_pad.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(),
-                       dqkv.data_ptr(), N, H, D, Lp, _lib.stream_ptr()), "att_pack_dqkv")
-        _lib.count_launch()
-        du = dqu.float().sum(dim=0).reshape(H, D).to(ctx.u_dtype) if ctx.u_dtype is not None else None
-        dvb = dqv.float().sum(dim=0).reshape(H, D).to(ctx.v_dtype) if ctx.v_dtype is not None else None
+        dqkv, du, dvb = _pack_dqkv(dqu, dqv, dk_pad, dv_pad, row_batch, row_pos, N, H, D, Lp, ctx.u_dtype, ctx.v_dtype)
         return dqkv, dpos, du, dvb, None, None, None, None, None, None, None, None, None
 
 
@@ -275,18 +294,9 @@ class _RelPosFlash(torch.autograd.Function):
             dpos = torch.empty(width, HD, dtype=bf, device=dev)
             fn = _lib.bind("rb200_sum_slices", [_vp, _vp, _i32, _i64, _vp])
             _lib.check(fn(part.data_ptr(), dpos.data_ptr(), n, width * HD, s), "sum_slices")
-        dqkv = torch.empty(N, 3 * HD, dtype=bf, device=dev)
-        fn = _lib.bind("rb200_att_pack_dqkv", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(dqu.data_ptr(), dqv.data_ptr(), dkv[0].data_ptr(), dkv[1].data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), dqkv.data_ptr(), N, H,
-                      64, Lp, s), "att_pack_dqkv")
-        _lib.count_launch(4)
-        sums = [None, None]
-        for i, dt in enumerate((ctx.u_dtype, ctx.v_dtype)):
-            if dt is not None:
-                t = torch.empty(HD, dtype=torch.float32, device=dev)
-                _gemm._grad_pre(padded[1 + i], None, None, t)
-                sums[i] = t.reshape(H, 64).to(dt)
-        return dqkv, dpos[band_off: band_off + R], sums[0], sums[1], None, None, None, None, None, None, None, None
+        dqkv, du, dvb = _pack_dqkv(dqu, dqv, dkv[0], dkv[1], row_batch, row_pos, N, H, 64, Lp, ctx.u_dtype, ctx.v_dtype)
+        _lib.count_launch(3)
+        return dqkv, dpos[band_off: band_off + R], du, dvb, None, None, None, None, None, None, None, None
 
 
 def _p(t):

@@ -319,3 +319,39 @@ def test_rel_flash_bwd_writes_the_padding(lens, H, saved):
     inside = (valid[:, None, :, None] & valid[:, None, None, :]).expand(B, H, Lp, Lp)
     want = torch.zeros_like(band.transpose(0, 1)).scatter_add(3, col.expand(B, H, Lp, Lp), ds * inside)
     assert torch.equal(band.transpose(0, 1), want)
+
+
+@gpu
+@pytest.mark.parametrize("lens,H,D", [([1], 1, 64), ([63, 2], 3, 64), ([128, 1, 0, 64], 8, 128), ([500, 300, 411], 8, 64)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_att_pack_dqkv_leaves_the_column_sums(lens, H, D, accumulate):
+    import ctypes
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import _lib
+
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    dev, bf, N, B, HD = "cuda", torch.bfloat16, pack.n, pack.batch, H * D
+    Lp = (pack.max_len + 63) // 64 * 64
+    torch.manual_seed(N)
+    dqu, dqv, dk, dv = (torch.randn(B, Lp, HD, device=dev).to(bf) for _ in range(4))
+    valid = torch.arange(Lp, device=dev)[None] < pack.lens[:, None]
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    slices = _lib.bind("rb200_att_pack_slices", [i32, i32, i32])(N, H, D)
+    got = torch.empty(N, 3 * HD, device=dev, dtype=bf)
+    sq = torch.ones(3 * HD, device=dev)
+    su = torch.ones(HD, device=dev) if accumulate else torch.full((slices, 2, HD), float("nan"), device=dev)
+    sv = torch.ones(HD, device=dev)
+    fn = _lib.bind("rb200_att_pack_dqkv", [vp] * 10 + [i32] * 5 + [vp])
+    _lib.check(fn(dqu.data_ptr(), dqv.data_ptr(), dk.data_ptr(), dv.data_ptr(), pack.row_batch.data_ptr(), pack.row_pos.data_ptr(), got.data_ptr(),
+                  sq.data_ptr(), su.data_ptr(), sv.data_ptr(), N, H, D, Lp, accumulate, _lib.stream_ptr()), "att_pack_dqkv")
+    u, v, k, w = (t[valid].view(N, H, D) for t in (dqu, dqv, dk, dv))
+    want = torch.stack([(u.float() + v.float()).to(bf), k, w], 2).reshape(N, 3 * HD)
+    assert torch.equal(got, want)
+    if not accumulate:
+        assert (sq == 1).all() and (sv == 1).all()
+        su, sv = su.sum(0) + 1
+    else:
+        assert ((sq.double() - 1 - want.double().sum(0)).abs() <= 1e-6 * want.double().abs().sum(0) + 1e-6).all()
+    for s, t in ((su, u), (sv, v)):
+        t = t.reshape(N, HD).double()
+        assert ((s.double() - 1 - t.sum(0)).abs() <= 1e-6 * t.abs().sum(0) + 1e-6).all()
