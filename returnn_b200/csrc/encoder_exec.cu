@@ -402,16 +402,19 @@ struct Exec {
     q.resid = resid; q.res_scale = res_scale; q.status = status;
     run(rb_gemm(q, s), "gemm_fwd");
   }
-  // dx = (dy·W^T) [* act'(z)] [* dropout mask]
+  // dx = (dy·W^T) [* act'(z)] [* dropout mask]; bi >= 0: dx is the output gradient of the layer with that bias, whose gradient is its column sums
   void linear_dgrad(const void* dy, int l, int wi, int m, int in, int out, void* dx, const void* z, int act, float p_drop,
-                    unsigned long long site_) {
+                    unsigned long long site_, int bi = -1) {
     if (!ok()) return;
     RbGemm q;
     q.a = dy; q.b = p16(l, wi); q.c = dx; q.m = m; q.n = in; q.k = out; q.lda = out; q.ldb = out; q.ldc = in;
     q.a_mn_major = 0; q.b_mn_major = 0;
     q.dact_z = z; q.act = z ? act : 0;
     q.drop_p = p_drop; q.seed = seed; q.offset = offset; q.drop_site = site_; q.status = status;
+    float* sum = bi >= 0 ? g32(l, bi) : nullptr;
+    if (sum && rb_gemm_column_sums(q)) q.colsum = sum;
     run(rb_gemm(q, s), "gemm_dgrad");
+    if (sum && !q.colsum && ok()) run(colsum(dx, nullptr, sum, m, in, 1.f, 0.f, nullptr, nullptr, 0, s), "colsum_bias");
   }
   // dW += x^T·dy (fp32, atomics, contraction split over CTAs); db += column sums of dy
   void linear_wgrad(const void* x, const void* dy, int l, int wi, int bi, int m, int in, int out, bool bias_sum) {
@@ -664,8 +667,8 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     const void* dy = layer_norm_branch(sv.x4, dx, l, P_FIN_LN_G, sv.st5, t.dA, nullptr, P_FF2_B2, d.ff_res_scale, e.site(l, g.site_ff2_out));
     // ---- feed-forward 2: dA -> dB (d x3)
     e.linear_wgrad(sv.a2, dy, l, P_FF2_W2, P_FF2_B2, n, F, D, false);
-    e.linear_dgrad(dy, l, P_FF2_W2, n, F, D, t.tW, sv.z2, 2, p_ff, e.site(l, g.site_ff2_act));
-    e.linear_wgrad(sv.ln4, t.tW, l, P_FF2_W1, P_FF2_B1, n, D, F, true);
+    e.linear_dgrad(dy, l, P_FF2_W2, n, F, D, t.tW, sv.z2, 2, p_ff, e.site(l, g.site_ff2_act), P_FF2_B1);
+    e.linear_wgrad(sv.ln4, t.tW, l, P_FF2_W1, P_FF2_B1, n, D, F, false);
     e.linear_dgrad(t.tW, l, P_FF2_W1, n, D, F, t.tD2, nullptr, 0, 0.f, 0);
     dy = layer_norm_branch(sv.x3, t.tD2, l, P_FF2_LN_G, sv.st4, t.dB, t.dA, P_PW2_B, 1.f, e.site(l, g.site_conv_out));
     // ---- convolution module: dB -> dA (d x2)
@@ -731,8 +734,8 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     dy = layer_norm_branch(sv.x1, t.tD2, l, P_ATT_LN_G, sv.st2, t.dB, t.dA, P_FF1_B2, d.ff_res_scale, e.site(l, g.site_ff_out));
     // ---- feed-forward 1: dB -> dx (d x0)
     e.linear_wgrad(sv.a1, dy, l, P_FF1_W2, P_FF1_B2, n, F, D, false);
-    e.linear_dgrad(dy, l, P_FF1_W2, n, F, D, t.tW, sv.z1, 2, p_ff, e.site(l, g.site_ff_act));
-    e.linear_wgrad(sv.ln1, t.tW, l, P_FF1_W1, P_FF1_B1, n, D, F, true);
+    e.linear_dgrad(dy, l, P_FF1_W2, n, F, D, t.tW, sv.z1, 2, p_ff, e.site(l, g.site_ff_act), P_FF1_B1);
+    e.linear_wgrad(sv.ln1, t.tW, l, P_FF1_W1, P_FF1_B1, n, D, F, false);
     e.linear_dgrad(t.tW, l, P_FF1_W1, n, D, F, t.tD2, nullptr, 0, 0.f, 0);
     e.layer_norm_bwd(x0, t.tD2, l, P_FF1_LN_G, sv.st1, dx, t.dB, t.ln_part);
   }

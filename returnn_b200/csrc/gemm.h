@@ -25,6 +25,7 @@ struct RbGemm {
   unsigned long long drop_site = 0;
   const void* resid = nullptr;   // bf16 [m][ldc]: final = resid + res_scale * v
   float res_scale = 1.f;
+  float* colsum = nullptr;       // [n] += the column sums of the stored bf16 values; only where rb_gemm_column_sums says so
   int split_k = 0;               // 0: chosen by the launcher (> 1 only with accumulate == 2)
   // batched form (batch > 0): problem z = b * heads + h reads A from the stored origin (b*a_rb + h*a_rh, b*a_cb + h*a_ch),
   // B likewise, and writes at element offset b*c_sb + h*c_sh. m / n / k are fixed or lens[b] where the *_from_lens flag is set;
@@ -42,6 +43,10 @@ struct RbGemm {
 
 // returns an RB_* status code; the launch is asynchronous on `stream`
 int rb_gemm(const RbGemm& g, cudaStream_t stream);
+
+// whether the epilogue of this problem's kernel can leave column sums (`colsum`): the full epilogue of the CTA-pair kernel with one bf16 output
+// that leaves through bulk stores
+bool rb_gemm_column_sums(const RbGemm& g);
 
 // CTA-pair kernel (gemm_2cta.cu): rb_gemm routes to it when rb_gemm_pair_wanted says so
 bool rb_gemm_pair_wanted(const RbGemm& g);

@@ -278,7 +278,31 @@ bool rb_gemm_pair_wanted(const RbGemm& g) {
   return enabled && g.batch == 0 && g.m > 128 && g.n > 128;
 }
 
+static bool tma_store_on() {
+  static int enabled = -1;
+  if (enabled < 0) {
+    const char* e = getenv("RETURNN_B200_GEMM_TMA_STORE");
+    enabled = (e && e[0] == '0') ? 0 : 1;
+  }
+  return enabled != 0;
+}
+
+static bool full_epilogue(const RbGemm& g) { return g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr; }
+
+static bool aligned_outputs(const RbGemm& g) {
+  auto al16 = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  return (g.ldc % 8 == 0) && al16(g.c) && al16(g.c2) && al16(g.resid) && al16(g.dact_z);
+}
+
+bool rb_gemm_column_sums(const RbGemm& g) {
+  return rb_gemm_pair_wanted(g) && tma_store_on() && full_epilogue(g) && aligned_outputs(g) && g.c != nullptr && g.c2 == nullptr && !g.out_fp32;
+}
+
 int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
+  if (g.colsum && !rb_gemm_column_sums(g)) {
+    rb_set_error("gemm (pair): this problem's epilogue leaves no column sums");
+    return RB_ERR_ARG;
+  }
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
@@ -308,17 +332,11 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   p.kb_per_split = (p.num_kb + split - 1) / split;
   p.split = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
   p.units = tiles * p.split;
-  auto al16 = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  p.vec_ok = (g.ldc % 8 == 0) && al16(g.c) && al16(g.c2) && al16(g.resid) && al16(g.dact_z);
-  p.bias_vec = g.bias != nullptr && !g.bias_bf16 && al16(g.bias);
-  const bool full = g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr;
-  static int tma_store_enabled = -1;
-  if (tma_store_enabled < 0) {
-    const char* e = getenv("RETURNN_B200_GEMM_TMA_STORE");
-    tma_store_enabled = (e && e[0] == '0') ? 0 : 1;
-  }
+  p.vec_ok = aligned_outputs(g);
+  p.bias_vec = g.bias != nullptr && !g.bias_bf16 && (reinterpret_cast<uintptr_t>(g.bias) & 15) == 0;
+  const bool full = full_epilogue(g);
   // bulk tensor stores need what a tensor map needs: 16-byte aligned base, row pitch a multiple of 16 bytes
-  p.tma_store = tma_store_enabled && p.vec_ok && g.c != nullptr && (g.out_fp32 ? true : (g.ldc % 8 == 0));
+  p.tma_store = tma_store_on() && p.vec_ok && g.c != nullptr && (g.out_fp32 ? true : (g.ldc % 8 == 0));
   CUtensorMap tm_a, tm_b, tm_c, tm_c2;
   memset(&tm_c, 0, sizeof(tm_c));
   memset(&tm_c2, 0, sizeof(tm_c2));

@@ -211,3 +211,24 @@ def test_native_encoder_with_another_head_dim_matches_per_op_path():
         if err >= 0.08:  # bf16 paths that differ in the order of their roundings
             bad.append("%s: rel. max err %.4f (scale %.3g)" % (s.name, err, scale))
     assert not bad, "parameter gradients differ:\n" + "\n".join(bad)
+
+
+@gpu
+@pytest.mark.parametrize("frames,ff", [(768, 256), (774, 200), (1530, 136), (1542, 264)])
+def test_native_encoder_bias_gradients_from_the_epilogue(frames, ff):
+    """rows and widths around the epilogue's boxes of 32 x 64: the bias of the first feed-forward layer against column sums on the per-op path"""
+    model, pt, arena = _make(num_layers=1, ff=ff)
+    lens = torch.tensor([frames], dtype=torch.int32)
+    torch.manual_seed(frames)
+    feats = torch.randn(1, frames, 80, device="cuda")
+    wgt = torch.randn(frames // 6 + 2, 128, device="cuda")
+    _, _, got = _run(model, arena, feats, lens, wgt, native=True)
+    _, _, want = _run(model, arena, feats, lens, wgt, native=False)
+    seen = 0
+    for s in arena.slots:
+        if s.name.endswith("linear_ff.bias"):
+            a, b = got[s.offset: s.offset + s.numel], want[s.offset: s.offset + s.numel]
+            # two bf16 paths through one layer: each rounds the gradient of the pre-activation (2^-9 of its size per row)
+            assert float((a - b).norm()) <= 0.02 * float(b.norm()), (s.name, float((a - b).norm()), float(b.norm()))
+            seen += 1
+    assert seen == 2
