@@ -27,44 +27,59 @@ __device__ __forceinline__ int seq_start(const int* __restrict__ lens, int b) {
 }
 
 // The two kernels that fill padded buffers write the padding too: fills of the buffers in front of them took as long as the copies (17 us for
-// the 85 MB of a batch of 36 x 333 frames with 8 heads, 13 us for 42 MB). A CTA belongs to one sequence, `ctas` to each.
+// the 85 MB of a batch of 36 x 333 frames with 8 heads, 13 us for 42 MB). A CTA owns kPadRows padded rows of one sequence, so that a full batch is
+// one wave of CTAs, and a thread has four 16-byte loads in flight (one item per thread and ten thousand CTAs: 28 us, now 23).
+constexpr int kPadRows = 16;
+constexpr int kPadLoads = 4;
 
-// one thread per 8 consecutive elements of one of q/k/v of one head of one padded row
+// item: 8 consecutive elements of one of q/k/v of one head of one padded row
 __global__ void __launch_bounds__(256)
 att_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ u, const float* __restrict__ v,
                    const int* __restrict__ lens, __nv_bfloat16* __restrict__ qu, __nv_bfloat16* __restrict__ qv, __nv_bfloat16* __restrict__ kk,
                    __nv_bfloat16* __restrict__ vv, int heads, int dim, int lp, int ctas) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
-  const int groups_per_part = dim / 8;
+  const uint32_t groups_per_part = dim / 8;
   const uint32_t groups_per_row = heads * 3 * groups_per_part;
   const int b = blockIdx.x / ctas;
-  const uint32_t gid = (blockIdx.x - b * ctas) * blockDim.x + threadIdx.x;
-  const int start = seq_start(lens, b);
-  const int pos = (int)(gid / groups_per_row);
-  if (pos >= lp) return;
-  int g = (int)(gid - pos * groups_per_row);
-  const int h = g / (3 * groups_per_part);
-  g -= h * 3 * groups_per_part;
-  const int part = g / groups_per_part;
-  const int d0 = (g - part * groups_per_part) * 8;
+  const int row0 = (blockIdx.x - b * ctas) * kPadRows;
   const int hd = heads * dim;
-  const bool valid = pos < lens[b];
-  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-  if (valid) raw = *reinterpret_cast<const uint4*>(qkv + (long long)(start + pos) * 3 * hd + (long long)h * 3 * dim + part * dim + d0);
-  const long long dst = ((long long)b * lp + pos) * hd + h * dim + d0;
-  if (part == 0) {
-    F8 a, c;
-    const F8 x = load8(&raw, 0, 1);
+  const int len = lens[b];
+  const __nv_bfloat16* src = qkv + ((long long)seq_start(lens, b) + row0) * 3 * hd;
+  const long long dst0 = ((long long)b * lp + row0) * hd;
+  const uint32_t items = min(kPadRows, lp - row0) * groups_per_row;
+  for (uint32_t it0 = threadIdx.x; it0 < items; it0 += kPadLoads * 256) {
+    uint4 raw[kPadLoads];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      a.v[i] = valid ? x.v[i] + (u ? u[h * dim + d0 + i] : 0.f) : 0.f;
-      c.v[i] = valid ? x.v[i] + (v ? v[h * dim + d0 + i] : 0.f) : 0.f;
+    for (int k = 0; k < kPadLoads; ++k) {
+      const uint32_t it = it0 + k * 256, r = it / groups_per_row;
+      raw[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (it < items && row0 + (int)r < len) raw[k] = *reinterpret_cast<const uint4*>(src + (long long)it * 8);
     }
-    store8(qu, dst, a, 1);
-    store8(qv, dst, c, 1);
-  } else {
-    *reinterpret_cast<uint4*>((part == 1 ? kk : vv) + dst) = raw;
+#pragma unroll
+    for (int k = 0; k < kPadLoads; ++k) {
+      const uint32_t it = it0 + k * 256;
+      if (it >= items) break;
+      const uint32_t r = it / groups_per_row, g = it - r * groups_per_row;
+      const uint32_t h = g / (3 * groups_per_part), in_head = g - h * 3 * groups_per_part;
+      const uint32_t part = in_head / groups_per_part;
+      const int c0 = h * dim + (in_head - part * groups_per_part) * 8;
+      const bool valid = row0 + (int)r < len;
+      const long long dst = dst0 + (long long)r * hd + c0;
+      if (part == 0) {
+        F8 a, c;
+        const F8 x = load8(&raw[k], 0, 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          a.v[i] = valid ? x.v[i] + (u ? u[c0 + i] : 0.f) : 0.f;
+          c.v[i] = valid ? x.v[i] + (v ? v[c0 + i] : 0.f) : 0.f;
+        }
+        store8(qu, dst, a, 1);
+        store8(qv, dst, c, 1);
+      } else {
+        *reinterpret_cast<uint4*>((part == 1 ? kk : vv) + dst) = raw[k];
+      }
+    }
   }
 }
 
@@ -73,16 +88,26 @@ __global__ void __launch_bounds__(256)
 att_rows_pad_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, const int* __restrict__ lens, int width, int lp, int ctas) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
-  const uint32_t groups = width / 8;
   const int b = blockIdx.x / ctas;
-  const uint32_t gid = (blockIdx.x - b * ctas) * blockDim.x + threadIdx.x;
-  const int start = seq_start(lens, b);
-  const int pos = (int)(gid / groups);
-  if (pos >= lp) return;
-  const int c0 = (int)(gid - pos * groups) * 8;
-  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-  if (pos < lens[b]) raw = *reinterpret_cast<const uint4*>(src + (long long)(start + pos) * width + c0);
-  *reinterpret_cast<uint4*>(dst + ((long long)b * lp + pos) * width + c0) = raw;
+  const int row0 = (blockIdx.x - b * ctas) * kPadRows;
+  const __nv_bfloat16* from = src + ((long long)seq_start(lens, b) + row0) * width;
+  __nv_bfloat16* to = dst + ((long long)b * lp + row0) * width;
+  const uint32_t items = min(kPadRows, lp - row0) * (width / 8);
+  const uint32_t valid = max(0, min(kPadRows, lens[b] - row0)) * (width / 8);  // rows lie one after the other on both sides
+  for (uint32_t it0 = threadIdx.x; it0 < items; it0 += kPadLoads * 256) {
+    uint4 raw[kPadLoads];
+#pragma unroll
+    for (int k = 0; k < kPadLoads; ++k) {
+      const uint32_t it = it0 + k * 256;
+      raw[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (it < valid) raw[k] = *reinterpret_cast<const uint4*>(from + (long long)it * 8);
+    }
+#pragma unroll
+    for (int k = 0; k < kPadLoads; ++k) {
+      const uint32_t it = it0 + k * 256;
+      if (it < items) *reinterpret_cast<uint4*>(to + (long long)it * 8) = raw[k];
+    }
+  }
 }
 
 __device__ __forceinline__ uint32_t rng_u32(uint64_t seed, uint64_t idx) {
@@ -501,17 +526,17 @@ att_rows_gather_kernel(const void* __restrict__ src, __nv_bfloat16* __restrict__
 
 }  // namespace
 
-// CTAs of 256 threads per sequence of lp rows with `groups` threads each; 0: more than a launch or a 32-bit index holds
-static int ctas_per_seq(int batch, int lp, long long groups) {
-  const long long n = ((long long)lp * groups + 255) / 256;
-  return n * 256 < (1LL << 31) && n * batch < (1LL << 31) ? (int)n : 0;
+// CTAs per sequence of lp rows; 0: more than a launch holds
+static int ctas_per_seq(int batch, int lp) {
+  const long long n = (lp + kPadRows - 1) / kPadRows;
+  return n * batch < (1LL << 31) ? (int)n : 0;
 }
 
 // packed qkv [N, H*3*D] -> qu = q + u, qv = q + v, k, v [B*Lp, H*D]; lens (device) of the sequences, back to back in qkv
 RB_EXPORT int rb200_att_prepare(const void* qkv, const float* u, const float* v, const int* lens, void* qu, void* qv, void* k, void* vv, int batch,
                                 int heads, int dim, int lp, cudaStream_t stream) {
   if (batch <= 0 || lp <= 0) return RB_OK;
-  const int ctas = dim % 8 ? 0 : ctas_per_seq(batch, lp, (long long)heads * 3 * (dim / 8));
+  const int ctas = dim % 8 ? 0 : ctas_per_seq(batch, lp);
   if (!ctas) {
     rb_set_error("att_prepare: head dim %d must be a multiple of 8, batch %d x %d rows fit a launch", dim, batch, lp);
     return RB_ERR_ARG;
@@ -617,7 +642,7 @@ RB_EXPORT int rb200_att_rows_gather(const void* src, void* dst, const int* row_b
 // packed bf16 rows [N, width] -> [B*Lp, width], zeros in the padding
 RB_EXPORT int rb200_att_rows_pad(const void* src, void* dst, const int* lens, int batch, int width, int lp, cudaStream_t stream) {
   if (batch <= 0 || lp <= 0) return RB_OK;
-  const int ctas = width % 8 ? 0 : ctas_per_seq(batch, lp, width / 8);
+  const int ctas = width % 8 ? 0 : ctas_per_seq(batch, lp);
   if (!ctas) {
     rb_set_error("att_rows_pad: width %d must be a multiple of 8, batch %d x %d rows fit a launch", width, batch, lp);
     return RB_ERR_ARG;

@@ -52,6 +52,8 @@ int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const voi
                         void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch, int heads,
                         int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream);
 int rb200_rel_flash_slices(long long rows, int width, int heads);
+int rb200_rel_flash_dpos(const void* band, const void* qv, void* part, const int* lens, int batch, int heads, int lp, int center, float scale, int slices,
+                         int* status, cudaStream_t stream);
 int rb200_sum_slices(const float* x, void* y, int slices, long long n, cudaStream_t stream);
 int rb200_glu_dwconv_fwd(const void* x, const float* filt, const float* bias, const int* row_batch, const int* row_pos, const int* lens,
                          void* y, float* part, int n_rows, int n_seqs, int C, int K, cudaStream_t stream);
@@ -579,8 +581,15 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
       // scores and bias band in bf16, like the matmul outputs of the reference under autocast: halves the traffic of this stage
       e.bgemm(sv.qu, sv.kk, t.s_ac, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o1, B * H, H, lens, 1, 1, 0,
               d.att_scale, 0);
-      const long long o2[10] = {Lp, 0, 0, Dh, 0, 0, 0, Dh, (long long)Lp * Rp, (long long)B * Lp * Rp};
-      e.bgemm(sv.qv, sv.posp, t.band, Lp, g.R, Dh, 0, 0, HD, HD, Rp, (long long)B * Lp, HD, g.R, HD, o2, B * H, H, lens, 1, 0, 0, d.att_scale, 0);
+      // the band: of each query's positions only the tiles that its keys refer to
+      RbGemm q;
+      q.a = sv.qv; q.b = sv.posp; q.c = t.band; q.m = Lp; q.n = g.R; q.k = Dh; q.lda = HD; q.ldb = HD; q.ldc = Rp;
+      q.alpha = d.att_scale; q.status = status;
+      q.batch = B * H; q.heads = H;
+      q.a_rb = Lp; q.a_ch = Dh; q.b_ch = Dh; q.c_sb = (long long)Lp * Rp; q.c_sh = (long long)B * Lp * Rp;
+      q.a_rows = (long long)B * Lp; q.a_cols = HD; q.b_rows = g.R; q.b_cols = HD;
+      q.lens = lens; q.m_from_lens = 1; q.win = 1; q.win_center = g.center;
+      if (e.ok()) e.run(rb_gemm(q, stream), "gemm_band");
     }
     void* o_pad = g.fused_bwd ? (void*)sv.o_pad : t.o_pad;  // (the fused backward pass takes it in 32 bits)
     // w and wd need no memset: the softmax kernel zeroes the margin that the GEMMs read beyond each sequence's length
@@ -700,10 +709,9 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
       const long long o_rows[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
       e.bgemm(wd, t.do_pad, t.dv, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, 1.f, 0);
       e.bgemm(t.ds, sv.qu, t.dk, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
-      const int rows = (int)(g.pad_rows / g.slices);
-      const long long o9[10] = {rows, (long long)B * Lp, 0, 0, rows, 0, 0, Dh, (long long)g.band_w * HD, Dh};
-      e.bgemm(t.dband, sv.qv, g.slices > 1 ? (void*)t.dpos_part : t.dpos, g.band_w, Dh, rows, 1, 1, g.band_w, HD, HD, (long long)H * B * Lp, g.band_w,
-              (long long)B * Lp, HD, o9, g.slices * H, H, nullptr, 0, 0, 0, d.att_scale, g.slices > 1);
+      if (e.ok())
+        e.run_tagged("gemm_dpos", rb200_rel_flash_dpos(t.dband, sv.qv, g.slices > 1 ? (void*)t.dpos_part : t.dpos, lens, B, H, Lp, g.center, d.att_scale, g.slices,
+                                                       status, stream));
       if (g.slices > 1 && e.ok()) e.run_tagged("sum_slices", rb200_sum_slices(t.dpos_part, t.dpos, g.slices, (long long)g.band_w * HD, stream));
       dpos = t.dpos + (size_t)g.band_off * HD;  // the band's first columns lie before position 0
     } else {

@@ -35,6 +35,12 @@ struct RbGemm {
   long long a_rows = 0, a_cols = 0, b_rows = 0, b_cols = 0;
   const int* lens = nullptr;
   int m_from_lens = 0, n_from_lens = 0, k_from_lens = 0;
+  // windows of a relative-position band (batched form): row i of a sequence of length len concerns the columns [win_center - i, win_center - i + len).
+  // win = 1: the output is the band, m_from_lens; tiles of it without such a column are not computed (and not written).
+  // win = 2: A, stored [k][m], is the band of sequences of win_lp rows each (a multiple of 64) with lengths win_lens, zero outside the windows;
+  // the contraction leaves out blocks of 64 rows that have no such column among those of the tile. k a multiple of 64.
+  int win = 0, win_center = 0, win_lp = 0;
+  const int* win_lens = nullptr;
   // split operands (CTA-pair kernel only): A and B are sums hi + lo whose parts lie in ONE stored matrix each, the rows of lo seg_a / seg_b
   // rows after those of hi (seg_a > 0). The contraction runs over hi*lo, lo*hi and hi*hi into one accumulator. B is stored [k][n].
   int seg_a = 0, seg_b = 0;

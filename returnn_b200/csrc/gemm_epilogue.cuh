@@ -215,6 +215,7 @@ __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
     w.b_r0 = (int)(zb * g.b_rb + zh * g.b_rh); w.b_c0 = (int)(zb * g.b_cb + zh * g.b_ch);
     w.c_off = (size_t)zb * g.c_sb + (size_t)zh * g.c_sh;
     w.valid = w.m0 < w.M && w.n0 < w.N && w.kb1 > 0;
+    if (g.win == 1) w.valid = w.valid && w.n0 < g.win_center - w.m0 + len && w.n0 + BN > g.win_center - (min(w.m0 + BM, len) - 1);
   } else {
     const int sp = u / tiles, t = u % tiles;
     w.M = g.m; w.N = g.n;
@@ -228,6 +229,29 @@ __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
   }
   return w;
 }
+
+// Walks over the K blocks of a unit whose A is a band (win = 2): which of them have a column of the tile in their window. The first is always
+// taken (it starts the accumulator). Producer and MMA issuer walk alike.
+struct BandWalk {
+  const RbGemm& g;
+  int b, i0, len, m0, m1;
+  __device__ __forceinline__ BandWalk(const RbGemm& g_, const Unit& w, int bm) : g(g_), b(0), i0(0), len(0), m0(w.a_c0 + w.m0), m1(w.a_c0 + w.m0 + bm) {
+    if (g.win != 2) return;
+    const int rows = g.heads > 0 ? (int)(w.a_r0 % ((long long)g.batch / g.heads * g.k)) : 0;  // row within the band of one head
+    b = rows / g.win_lp;
+    i0 = rows - b * g.win_lp - BK;
+    len = g.win_lens[b];
+  }
+  __device__ __forceinline__ bool skip(bool first) {  // called once per K block
+    if (g.win != 2) return false;
+    i0 += BK;
+    if (i0 == g.win_lp) {
+      i0 = 0;
+      len = g.win_lens[++b];
+    }
+    return !first && (i0 >= len || g.win_center - i0 + len <= m0 || g.win_center - min(i0 + BK, len) + 1 >= m1);
+  }
+};
 
 // Epilogue of the accumulator columns [c_begin, c_end) of one 128-row tile by one warp (TMEM lane quarter q), in chunks of 16
 // columns: tcgen05.ld -> registers -> this warp's 2 KB staging area (fp32 rows of 64 bytes, 16-byte chunk index xor-swizzled with

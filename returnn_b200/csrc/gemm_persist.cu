@@ -27,11 +27,11 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int kThreads = kGemmThreads;
-constexpr int kRingBytes = 196608;      // operand ring: 4 stages (BN = 256) or 6 stages (BN = 128)
+constexpr int kRingBytes = 196608;      // operand ring: 4 stages (BN = 256), 6 stages (BN = 128) or 8 stages (BN = 64)
 constexpr int kStagingBytes = kEpilogueWarps * kStagingBytesPerWarp;
 constexpr int kBarrierBytes = 256;
 constexpr int kSmemBytes = kRingBytes + kStagingBytes + kBarrierBytes + 1024;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8;
 
 template <int BN, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -89,9 +89,12 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         const Unit w = decode_unit<BM, BN>(p, u);
         if (!w.valid) continue;
         const int m0 = w.m0, n0 = w.n0;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
+        BandWalk walk(g, w, BM);
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+          if (walk.skip(kb == w.kb0)) continue;
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
+          ++it;
           if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag)) {
             *abort_flag = 1;
             if (g.status) atomicCAS(g.status, 0, (1 << 24) | (kb & 0xFFFFFF));
@@ -137,9 +140,12 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        BandWalk walk(g, w, BM);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (walk.skip(kb == kb0)) continue;
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
+          ++it;
           if (!mbar_wait(&full_bar[s], ph, abort_flag)) {
             *abort_flag = 1;
             if (g.status) atomicCAS(g.status, 0, (2 << 24) | (kb & 0xFFFFFF));
@@ -303,6 +309,11 @@ int rb_gemm(const RbGemm& g, cudaStream_t stream) {
     rb_set_error("gemm: dropout epilogue needs seed/offset pointers, ldc %% 8 == 0 and p < 1 (ldc %d, p %f)", g.ldc, g.drop_p);
     return RB_ERR_ARG;
   }
+  if (g.win && (g.batch <= 0 || g.heads <= 0 || (g.win == 1 ? !g.lens || !g.m_from_lens
+                                                            : !g.a_mn_major || !g.win_lens || g.win_lp <= 0 || g.win_lp % BK || g.k % BK || g.k_from_lens))) {
+    rb_set_error("gemm: windows need the batched form, lengths and blocks of whole sequences");
+    return RB_ERR_ARG;
+  }
   if (g.split_k > 1 && g.accumulate != 2) {
     rb_set_error("gemm: split_k needs accumulate == 2");
     return RB_ERR_ARG;
@@ -312,8 +323,10 @@ int rb_gemm(const RbGemm& g, cudaStream_t stream) {
     return RB_ERR_UNSUPPORTED;
   }
   if (rb_gemm_pair_wanted(g)) return rb_gemm_pair(g, stream);
-  if (g.n > 128) return launch<256>(g, stream);
-  return launch<128>(g, stream);
+  // Narrow tiles where wider ones would load and multiply columns that are not wanted: one head of 64 columns, the windows of a band
+  if (g.n > 128 && g.win != 1) return launch<256>(g, stream);
+  if (g.n > 64) return launch<128>(g, stream);
+  return launch<64>(g, stream);
 }
 
 // C entry points with the full epilogue (see gemm.h for the meaning of the arguments); the second reads A and B as fp16

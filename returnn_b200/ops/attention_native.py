@@ -286,9 +286,9 @@ class _RelPosFlash(torch.autograd.Function):
         # dP[h] = scale * band[h]^T Qv[h] over all rows of all sequences, in slices of the rows
         n = _lib.bind("rb200_rel_flash_slices", [_i64, _i32, _i32])(rows, width, H)
         part = torch.empty(n, width, HD, dtype=torch.float32 if n > 1 else bf, device=dev)
-        _bgemm(band, pads[1], part, m=width, n=64, k=rows // n, a_mn=True, b_mn=True, lda=width, ldb=HD, ldc=HD, a_shape=(H * rows, width),
-               b_shape=(rows, HD), offs=(rows // n, rows, 0, 0, rows // n, 0, 0, 64, width * HD, 64), batch=n * H, heads=H, lens=None, m_l=False, n_l=False,
-               k_l=False, alpha=scale, out_fp32=n > 1)
+        fn = _lib.bind("rb200_rel_flash_dpos", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _i32, _vp, _vp])
+        _lib.check(fn(band.data_ptr(), pads[1].data_ptr(), part.data_ptr(), lens.data_ptr(), B, H, Lp, center, scale, n, st.data_ptr(), s), "rel_flash_dpos")
+        _lib.count_launch()
         dpos = part[0]
         if n > 1:
             dpos = torch.empty(width, HD, dtype=bf, device=dev)

@@ -355,3 +355,34 @@ def test_att_pack_dqkv_leaves_the_column_sums(lens, H, D, accumulate):
     for s, t in ((su, u), (sv, v)):
         t = t.reshape(N, HD).double()
         assert ((s.double() - 1 - t.sum(0)).abs() <= 1e-6 * t.abs().sum(0) + 1e-6).all()
+
+
+@gpu
+@pytest.mark.parametrize("lens,H,slices", [([1], 1, 1), ([64, 65, 0, 128], 2, 4), ([320, 7, 201], 3, 5), ([384, 384], 1, 3), ([512, 1, 1, 511], 2, 1)])
+def test_rel_flash_dpos_leaves_out_empty_blocks(lens, H, slices):
+    """the position gradient against the whole product over a band that is zero outside the windows"""
+    import ctypes
+    from returnn_b200.ops import _lib, gemm as G
+
+    dev, bf, HD, B, L = "cuda", torch.bfloat16, H * 64, len(lens), max(lens)
+    Lp = (L + 63) // 64 * 64
+    vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    geo = (ctypes.c_int * 2)()
+    _lib.check(_lib.bind("rb200_rel_flash_band", [i32, i32, vp, vp])(Lp, L - 1, ctypes.addressof(geo), ctypes.addressof(geo) + 4), "band")
+    off, width = geo[0], geo[1]
+    torch.manual_seed(L)
+    lens_t = torch.tensor(lens, dtype=torch.int32, device=dev)
+    i, x = torch.arange(Lp, device=dev)[:, None], torch.arange(width, device=dev)[None]
+    n = lens_t[:, None, None].long()
+    window = (i < n) & (x >= L - 1 + off - i) & (x < L - 1 + off - i + n)
+    band = (torch.randn(H, B, Lp, width, device=dev) * window).to(bf)
+    qv = torch.randn(B, Lp, HD, device=dev).to(bf)
+    part = torch.full((slices, width, HD), float("nan"), device=dev, dtype=torch.float32 if slices > 1 else bf)
+    st = G.status_tensor(lens_t.device)
+    fn = _lib.bind("rb200_rel_flash_dpos", [vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, vp, vp])
+    _lib.check(fn(band.data_ptr(), qv.data_ptr(), part.data_ptr(), lens_t.data_ptr(), B, H, Lp, L - 1, 0.125, slices, st.data_ptr(), _lib.stream_ptr()), "dpos")
+    G.check_status()
+    want = torch.einsum("hrx,rhd->xhd", band.double().view(H, B * Lp, width), qv.double().view(B * Lp, H, 64)).reshape(width, HD) * 0.125
+    got = part.double().sum(0)
+    # fp32 sums, one slice: the result in bf16
+    assert (got - want).norm() <= (1e-5 if slices > 1 else 2 ** -8) * want.norm() + 1e-6
