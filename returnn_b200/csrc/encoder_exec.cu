@@ -577,10 +577,15 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
     e.linear_fwd(sinus, l, P_POS_W, -1, g.R, D, HD, sv.posp, nullptr, 0, 0.f, 0, nullptr, 1.f);
     if (e.ok()) e.run_tagged("att_prepare", rb200_att_prepare(t.qkv, e.p32(l, P_POS_U), e.p32(l, P_POS_V), lens, sv.qu, sv.qv, sv.kk, sv.vv, B, H, Dh, Lp, stream));
     {
-      const long long o1[10] = {Lp, 0, 0, Dh, Lp, 0, 0, Dh, (long long)H * Lp * Lp, (long long)Lp * Lp};
       // scores and bias band in bf16, like the matmul outputs of the reference under autocast: halves the traffic of this stage
-      e.bgemm(sv.qu, sv.kk, t.s_ac, Lp, Lp, Dh, 0, 0, HD, HD, Lp, (long long)B * Lp, HD, (long long)B * Lp, HD, o1, B * H, H, lens, 1, 1, 0,
-              d.att_scale, 0);
+      RbGemm c;
+      c.a = sv.qu; c.b = sv.kk; c.c = t.s_ac; c.m = c.n = Lp; c.k = Dh; c.lda = HD; c.ldb = HD; c.ldc = Lp;
+      c.alpha = d.att_scale; c.status = status;
+      c.batch = B * H; c.heads = H;
+      c.a_rb = c.b_rb = Lp; c.a_ch = c.b_ch = Dh; c.c_sb = (long long)H * Lp * Lp; c.c_sh = (long long)Lp * Lp;
+      c.a_rows = c.b_rows = (long long)B * Lp; c.a_cols = c.b_cols = HD;
+      c.lens = lens; c.m_from_lens = c.n_from_lens = 1; c.c_rows = (long long)B * H * Lp;
+      if (e.ok()) e.run(rb_gemm(c, stream), "gemm_scores");
       // the band: of each query's positions only the tiles that its keys refer to
       RbGemm q;
       q.a = sv.qv; q.b = sv.posp; q.c = t.band; q.m = Lp; q.n = g.R; q.k = Dh; q.lda = HD; q.ldb = HD; q.ldc = Rp;
@@ -588,7 +593,7 @@ RB_EXPORT int rb200_enc_forward(const RbEncDims* dims, const long long* tab, con
       q.batch = B * H; q.heads = H;
       q.a_rb = Lp; q.a_ch = Dh; q.b_ch = Dh; q.c_sb = (long long)Lp * Rp; q.c_sh = (long long)B * Lp * Rp;
       q.a_rows = (long long)B * Lp; q.a_cols = HD; q.b_rows = g.R; q.b_cols = HD;
-      q.lens = lens; q.m_from_lens = 1; q.win = 1; q.win_center = g.center;
+      q.lens = lens; q.m_from_lens = 1; q.win = 1; q.win_center = g.center; q.c_rows = (long long)H * B * Lp;
       if (e.ok()) e.run(rb_gemm(q, stream), "gemm_band");
     }
     void* o_pad = g.fused_bwd ? (void*)sv.o_pad : t.o_pad;  // (the fused backward pass takes it in 32 bits)

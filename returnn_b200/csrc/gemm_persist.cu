@@ -18,6 +18,7 @@
 // Every mbarrier wait is bounded. A wait that gives up raises the CTA's abort flag and writes a status word; all roles
 // leave their loops, the CTA waits for its TMA copies in flight, frees its tensor memory and returns.
 #include "gemm_epilogue.cuh"
+#include <cstring>
 #include <cstdlib>
 
 using namespace rbt;
@@ -35,13 +36,15 @@ constexpr int kMaxStages = 8;
 
 template <int BN, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const Params p) {
+gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c, const Params p) {
   constexpr int kTileBytesA = BM * BK * 2;
   constexpr int kTileBytesB = BN * BK * 2;
   constexpr int kStageBytes = kTileBytesA + kTileBytesB;
   constexpr int kStages = kRingBytes / kStageBytes;
   static_assert(kStages <= kMaxStages && kStages >= 2, "ring");
   constexpr uint32_t kTmemCols = 2 * BN;
+  // bulk stores: a warp takes 64 columns, so tiles of 128 columns keep half of the warps busy, and the halves take the two accumulators in turn
+  constexpr int kParts = BN / 64, kSets = BN == 256 ? 1 : 2;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -64,7 +67,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], kEpilogueWarps);  // one arrival per epilogue warp
+      mbar_init(&acc_empty[i], p.tma_store ? kEpilogueWarps / kSets : kEpilogueWarps);  // one arrival per epilogue warp of the buffer
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -179,6 +182,10 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (!w.valid) continue;
       const int m0 = w.m0, n0 = w.n0;
       const uint32_t buf = t_local & 1u;
+      if (!FULL && BN == 128 && p.tma_store && (int)buf != ((warp - 2) >> 2) / kParts) {
+        ++t_local;
+        continue;
+      }
       bool ok = mbar_wait(&acc_full[buf], (t_local >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) {
         *abort_flag = 1;
@@ -189,9 +196,13 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
       const int part = (warp - 2) >> 2;  // four warps per lane quarter, each with a quarter of the columns
-      epilogue_columns<FULL>(p, w, m0, n0, t_addr, part * (BN / 4), (part + 1) * (BN / 4), stg, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
+      if (!FULL && BN >= 128 && p.tma_store)
+        epilogue_boxes(p, w, (int)(w.c_off / g.ldc), t_addr, (part % kParts) * 64, reinterpret_cast<uint8_t*>(stg), &tm_c, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
+      else
+        epilogue_columns<FULL>(p, w, m0, n0, t_addr, part * (BN / 4), (part + 1) * (BN / 4), stg, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
       ++t_local;
     }
+    if (!FULL && BN >= 128 && p.tma_store && lane == 0) tma_store_wait_read();  // before the shared memory is handed on
   }
 
   // ---------------- teardown ----------------
@@ -255,8 +266,14 @@ int launch(const RbGemm& g, cudaStream_t stream) {
   p.vec_ok = (g.ldc % 8 == 0) && al16(g.c) && al16(g.c2) && al16(g.resid) && al16(g.dact_z);
   p.bias_vec = g.bias != nullptr && !g.bias_bf16 && al16(g.bias);
   const bool full = g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr;
-  CUtensorMap tm_a, tm_b;
+  CUtensorMap tm_a, tm_b, tm_c;
+  memset(&tm_c, 0, sizeof(tm_c));
   int st;
+  p.tma_store = BN >= 128 && !full && g.batch > 0 && g.c_rows > 0 && !g.out_fp32 && !g.c2 && !g.bias && !g.act && p.vec_ok && g.c_sb % g.ldc == 0 && g.c_sh % g.ldc == 0;
+  if (p.tma_store) {
+    st = make_map(&tm_c, g.c, g.ldc, g.c_rows, g.ldc, 32, 32, false, true);
+    if (st) return st;
+  }
   long long a_rows = g.a_mn_major ? g.k : g.m, a_cols = g.a_mn_major ? g.m : g.k;
   long long b_rows = g.b_mn_major ? g.k : g.n, b_cols = g.b_mn_major ? g.n : g.k;
   if (g.batch > 0) {
@@ -276,8 +293,8 @@ int launch(const RbGemm& g, cudaStream_t stream) {
     }
     if (cap > 0 && grid > cap) grid = cap;
   }
-  if (full) rb_launch_pdl(gemm_persist_kernel<BN, true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, p);
-  else rb_launch_pdl(gemm_persist_kernel<BN, false>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, p);
+  if (full) rb_launch_pdl(gemm_persist_kernel<BN, true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, p);
+  else rb_launch_pdl(gemm_persist_kernel<BN, false>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, p);
   return rb_check_launch("gemm_persist");
 }
 

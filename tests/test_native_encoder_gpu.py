@@ -232,3 +232,20 @@ def test_native_encoder_bias_gradients_from_the_epilogue(frames, ff):
             assert float((a - b).norm()) <= 0.02 * float(b.norm()), (s.name, float((a - b).norm()), float(b.norm()))
             seen += 1
     assert seen == 2
+
+
+@gpu
+@pytest.mark.parametrize("frames", [[1542, 774, 6], [384, 378, 390], [3072, 1536]])
+def test_native_encoder_score_tiles_match_per_op_path(frames):
+    """lengths around the tiles of the score and band products (128 rows, 128 and 256 columns, boxes of 32): the rows of every sequence"""
+    model, pt, arena = _make(num_layers=1)
+    lens = torch.tensor(frames, dtype=torch.int32)
+    torch.manual_seed(len(frames))
+    feats = torch.randn(len(frames), max(frames), 80, device="cuda")
+    wgt = torch.randn(int((lens // 6 + 2).sum()), 128, device="cuda")
+    o1, _, g1 = _run(model, arena, feats, lens, wgt, native=True)
+    o2, _, g2 = _run(model, arena, feats, lens, wgt, native=False)
+    # bf16 scores here, fp32 there: 2^-9 of a score of a few units, through one layer
+    assert float((o1 - o2).norm()) <= 0.02 * float(o2.norm())
+    assert float((o1 - o2).abs().max()) <= 0.2
+    assert float((g1 - g2).norm()) <= 0.04 * float(g2.norm())
