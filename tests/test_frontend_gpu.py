@@ -52,3 +52,32 @@ def test_frontend_native_matches_torch_path(lens):
         errs[n] = (float((g.float() - p.grad).abs().max()) / scale, float(torch.nn.functional.cosine_similarity(g.float().flatten(), p.grad.flatten(), dim=0)))
     # bf16 activations and gradients through three layers against an fp32 reference: direction must agree closely, magnitudes within 10 %
     assert all(e < 0.1 and c > 0.995 for e, c in errs.values()), errs
+
+
+@gpu
+@pytest.mark.parametrize("lens,F,C", [([1], 2, 8), ([7, 8, 9, 0], 6, 32), ([17, 3], 80, 64), ([40, 33], 4, 256)])
+@pytest.mark.parametrize("with_bias", [True, False])
+def test_conv1_relu_pool_backward(lens, F, C, with_bias):
+    """filter and bias gradient of convolution, ReLU and pooling over two features against 64 bits: lengths around the runs of 8 frames"""
+    import ctypes
+    from returnn_b200.ops import _lib
+
+    torch.manual_seed(F + C)
+    dev, bf, B, T = "cuda", torch.bfloat16, len(lens), max(lens)
+    x = torch.randn(B, T, F, device=dev).to(bf)
+    w, b = torch.randn(C, 1, 3, 3, device=dev), torch.randn(C, device=dev) * 0.3
+    dy = torch.randn(B, T, F // 2, C, device=dev).to(bf)
+    n = torch.tensor(lens, dtype=torch.int32, device=dev)
+    dw, db = torch.ones(C, 9, device=dev), torch.ones(C, device=dev)
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    fn = _lib.bind("rb200_conv1_relu_pool_bwd", [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
+    _lib.check(fn(x.data_ptr(), w.data_ptr(), b.data_ptr() if with_bias else None, n.data_ptr(), dy.data_ptr(), B, T, F, C, dw.data_ptr(), db.data_ptr(),
+                  _lib.stream_ptr()), "conv1_relu_pool_bwd")
+    valid = (torch.arange(T, device=dev)[None] < n[:, None]).double()
+    w64, b64 = w.double().requires_grad_(True), (b if with_bias else b * 0).double().requires_grad_(True)
+    y = torch.nn.functional.conv2d(x.double()[:, None] * valid[:, None, :, None], w64, b64, padding=1)
+    y = torch.nn.functional.max_pool2d(torch.relu(y), (1, 2)).permute(0, 2, 3, 1)
+    (y * dy.double() * valid[:, :, None, None]).sum().backward()
+    # 32-bit sums of at most 3000 products; inputs drawn from a continuous distribution: no ties of the two candidates but by chance
+    for got, want in ((dw - 1, w64.grad.view(C, 9)), (db - 1, b64.grad)):
+        assert (got.double() - want).norm() <= 1e-3 * want.norm() + 1e-5
