@@ -476,7 +476,8 @@ __device__ __forceinline__ void stage_filter(float* __restrict__ sf, const float
 
 // map[i] = packed row at row first + i of the wider layout, -1 for the rows between sequences; i < n. Rows ascend in both layouts, the
 // wider one adds `gap` per sequence: a look at every 32nd row that can lie in front of the piece finds where to start reading row_batch.
-__device__ __forceinline__ void stage_map(int* __restrict__ map, int* __restrict__ start, const int* __restrict__ row_batch, int first, int n,
+// Returns whether this thread has found a row of the piece.
+__device__ __forceinline__ bool stage_map(int* __restrict__ map, int* __restrict__ start, const int* __restrict__ row_batch, int first, int n,
                                           int gap, int n_rows, int n_seqs) {
   const int lo = max(0, first - gap * (n_seqs - 1)), hi = min(n_rows, first);
   if (threadIdx.x == 0) *start = lo;
@@ -487,17 +488,23 @@ __device__ __forceinline__ void stage_map(int* __restrict__ map, int* __restrict
     if (r + gap * row_batch[r] < first) at = r;
   if (at > lo) atomicMax(start, at);
   __syncthreads();
+  bool any = false;
   for (int r = *start + threadIdx.x; r < n_rows; r += blockDim.x) {
     const int i = r + gap * row_batch[r] - first;
     if (i >= n) break;
-    if (i >= 0) map[i] = r;
+    if (i >= 0) {
+      map[i] = r;
+      any = true;
+    }
   }
+  return any;
 }
 
-// pieces of the wider layout's rows, a whole number of row groups each: about `ctas` CTAs in all, at most one per 32 packed rows (the size
-// of the scratch for the partial sums) unless the map would not hold a piece
+// pieces of the wider layout's rows, a whole number of row groups each: about `ctas` CTAs in all, at most one per 32 packed rows unless the map
+// would not hold a piece. The rows of the wider layout grow with every sequence, empty ones too: with many of those there are more pieces than
+// 32 packed rows, and the backward kernel's CTAs, `walkers` of them, take several (a partial sum each, in a scratch of one per 32 packed rows).
 struct Pieces {
-  int n, rows;
+  int n, rows, walkers;
 };
 inline Pieces pieces_of(int n_rows, int n_seqs, int C, int K, int ctas) {
   const long long wide = n_rows + (long long)((K <= 16 ? 16 : KM2) - 1) * (n_seqs > 0 ? n_seqs - 1 : 0);
@@ -507,7 +514,8 @@ inline Pieces pieces_of(int n_rows, int n_seqs, int C, int K, int ctas) {
   long long rows = ((wide + most - 1) / most + kRpt - 1) / kRpt * kRpt;
   if (rows < kStep) rows = kStep;
   if (rows > kPieceMax) rows = kPieceMax;
-  return {(int)((wide + rows - 1) / rows), (int)rows};
+  const long long n = (wide + rows - 1) / rows, slots = (n_rows + 31) / 32;
+  return {(int)n, (int)rows, (int)(n < slots ? n : slots)};
 }
 constexpr int kFwdCtas = 3 * 148, kBwdCtas = 2 * 148;  // as many as are resident (80 and 128 registers)
 constexpr size_t kFwd2Smem = (size_t)(kRing * CC + CC * kFiltPitch) * sizeof(float) + (kMap + 1) * sizeof(int);
@@ -628,12 +636,12 @@ bn_part_kernel(const __nv_bfloat16* __restrict__ y, float* __restrict__ part, in
   }
 }
 
-// dfilter / dbias sums stay in registers; partial per CTA [gridDim.x][C][K+1]
+// dfilter / dbias sums stay in registers, over all pieces of a CTA; partial per CTA [gridDim.x][C][K+1]
 template <int KT>
 __global__ void __launch_bounds__(kWinThreads, 2)
 glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, const float* __restrict__ filt,
                        const int* __restrict__ row_batch, __nv_bfloat16* __restrict__ dx, float* __restrict__ part, int n_rows, int n_seqs, int C,
-                       int K, int piece) {
+                       int K, int piece, int pieces) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
   extern __shared__ __align__(16) float smem_f[];
@@ -645,11 +653,9 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   const int tid = threadIdx.x;
   const int left = (K - 1) / 2;
   const int right = K - 1 - left;
-  const int begin = blockIdx.x * piece;
   const int c0 = blockIdx.y * CC;
   const int cg = (tid & 7) * 8;
   stage_filter(sf, filt, c0, K);
-  stage_map(map, map + kMap, row_batch, begin - right, piece + kHalo + kStep + 1, KT - 1, n_rows, n_seqs);
   __syncthreads();
   uint4 pd, pa, pg;
   auto fetch = [&](int staged) {  // rows staged .. staged + 31
@@ -669,7 +675,6 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     ring_store8(ring_h, staged + (tid >> 3), cg, h);
     ring_store8(ring_s, staged + (tid >> 3), cg, s);
   };
-  fetch(0);
   const int c = tid % CC;
   const int rg = tid / CC;
   float fr[KT];  // flipped filter: fr[m] = f[K-1-m]
@@ -679,8 +684,6 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
 #pragma unroll
   for (int k = 0; k < KT; ++k) df[k] = 0.f;
   float dbias = 0.f;
-  place(0);
-  fetch(kHalo);
   const int base = rg * kRpt;
   auto rows = [&](auto off, int at) {
     constexpr int OFF = decltype(off)::value;
@@ -706,18 +709,26 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     for (int i = 0; i < kRpt; ++i) dbias += v[i] = ring_dy[((at + i + right) & (kRing - 1)) * CC + c];
     window_corr<KT, OFF>(ring_h, col, v, df);
   };
-  for (int step = 0; step * kStep < piece; ++step) {
-    __syncthreads();  // the rows that are replaced have been read
-    place(kHalo + step * kStep);
-    if ((step + 1) * kStep < piece) fetch(kHalo + (step + 1) * kStep);
-    __syncthreads();
-    const int at = step * kStep + base;
-    int any = -1;
+  for (int at_piece = blockIdx.x; at_piece < pieces; at_piece += gridDim.x) {
+    if (at_piece != (int)blockIdx.x) __syncthreads();  // the map and the rows of the piece before have been read
+    const bool found = stage_map(map, map + kMap, row_batch, at_piece * piece - right, piece + kHalo + kStep + 1, KT - 1, n_rows, n_seqs);
+    if (!__syncthreads_or(found)) continue;  // empty sequences only
+    fetch(0);
+    place(0);
+    fetch(kHalo);
+    for (int step = 0; step * kStep < piece; ++step) {
+      __syncthreads();  // the rows that are replaced have been read
+      place(kHalo + step * kStep);
+      if ((step + 1) * kStep < piece) fetch(kHalo + (step + 1) * kStep);
+      __syncthreads();
+      const int at = step * kStep + base;
+      int any = -1;
 #pragma unroll
-    for (int i = 0; i < kRpt; ++i) any &= map[at + right + i];  // -1 where all are
-    if (at >= piece || any == -1) continue;
-    if (base & 8) rows(std::integral_constant<int, 8>(), at);
-    else rows(std::integral_constant<int, 0>(), at);
+      for (int i = 0; i < kRpt; ++i) any &= map[at + right + i];  // -1 where all are
+      if (at >= piece || any == -1) continue;
+      if (base & 8) rows(std::integral_constant<int, 8>(), at);
+      else rows(std::integral_constant<int, 0>(), at);
+    }
   }
   // sum the row groups in shared memory, one after the other (the same sum in every run), one partial per CTA
   float* red = ring_h;  // [KT + 1][CC]
@@ -945,10 +956,10 @@ RB_EXPORT int rb200_glu_dwconv_bwd_ex(const void* x, const void* dy, const float
       cudaFuncSetAttribute(glu_dwconv_bwd2_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
       attr2 = true;
     }
-    const Pieces pc = pieces_of(n_rows, n_seqs, C, K, kBwdCtas);  // every CTA leaves one partial
-    row_ctas = pc.n;
-    rb_launch_pdl(K <= 16 ? glu_dwconv_bwd2_kernel<16> : glu_dwconv_bwd2_kernel<32>, dim3(pc.n, C / CC), dim3(kWinThreads), kBwd2Smem, stream,
-                  (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, filt, row_batch, (__nv_bfloat16*)dx, part, n_rows, n_seqs, C, K, pc.rows);
+    const Pieces pc = pieces_of(n_rows, n_seqs, C, K, kBwdCtas);
+    row_ctas = pc.walkers;  // every CTA leaves one partial
+    rb_launch_pdl(K <= 16 ? glu_dwconv_bwd2_kernel<16> : glu_dwconv_bwd2_kernel<32>, dim3(pc.walkers, C / CC), dim3(kWinThreads), kBwd2Smem, stream,
+                  (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, filt, row_batch, (__nv_bfloat16*)dx, part, n_rows, n_seqs, C, K, pc.rows, pc.n);
     int st2 = rb_check_launch("glu_dwconv_bwd2");
     if (st2) return st2;
     rb_launch_pdl(dwconv_bwd_reduce2_kernel, dim3((C * (K + 1) + 31) / 32), dim3(256), 0, stream, part, row_ctas, C, K, dfilt, dbias, accumulate);

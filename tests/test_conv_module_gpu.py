@@ -136,3 +136,42 @@ def test_conv_module_sequences_do_not_see_each_other():
         (dx,) = torch.autograd.grad(z, [x], torch.ones_like(z))
         for t in (z, dx):
             assert bool(torch.isfinite(t[:40]).all()) and bool(torch.isfinite(t[43:]).all())
+
+
+@gpu
+@pytest.mark.parametrize("lens", [[1] + [0] * 70, [5, 3] + [0] * 300, [0] * 200 + [40], [0] * 70 + [30] + [0] * 70 + [300], [2, 1, 5]])
+@pytest.mark.parametrize("C,K", [(64, 7), (512, 32)])
+def test_conv_module_backward_with_many_empty_sequences(lens, C, K):
+    """
+    the zeros between the sequences make more pieces than there are partial sums in the scratch: nothing is written behind it, and the CTAs that
+    take several pieces leave the sums of all. Sums of fp32 products in another order, dx rounded to bf16
+    """
+    import ctypes
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import _lib
+
+    gen = torch.Generator("cuda").manual_seed(len(lens) + K)
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    n = pack.n
+    x = torch.randn(n, 2 * C, device="cuda", generator=gen).bfloat16()
+    dy = torch.randn(n, C, device="cuda", generator=gen).bfloat16()
+    filt = torch.randn(C, K, device="cuda", generator=gen) * K ** -0.5
+    size = (n + 31) // 32 * C * (K + 1)
+    part = torch.full((size + 64 * C * (K + 1),), 77.0, device="cuda")
+    dx, dfilt, dbias = torch.empty_like(x), torch.empty_like(filt), torch.empty(C, device="cuda")
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    fn = _lib.bind("rb200_glu_dwconv_bwd", [vp] * 10 + [i32] * 4 + [vp])
+    _lib.check(fn(x.data_ptr(), dy.data_ptr(), filt.data_ptr(), pack.row_batch.data_ptr(), pack.row_pos.data_ptr(), pack.lens.data_ptr(), dx.data_ptr(),
+                  part.data_ptr(), dfilt.data_ptr(), dbias.data_ptr(), n, pack.batch, C, K, _lib.stream_ptr()), "glu_dwconv_bwd")
+    assert bool((part[size:] == 77.0).all())
+    x64, f64 = x.double().requires_grad_(True), filt.double().requires_grad_(True)
+    h = x64[:, :C] * torch.sigmoid(x64[:, C:])
+    ys, lo = [], 0
+    for m in lens:
+        if m:
+            p = torch.nn.functional.pad(h[lo: lo + m].t()[None], ((K - 1) // 2, K - 1 - (K - 1) // 2))
+            ys.append(torch.nn.functional.conv1d(p, f64[:, None], groups=C)[0].t())
+        lo += m
+    want = torch.autograd.grad(torch.cat(ys), [x64, f64], dy.double())
+    for a, b, tol in ((dx, want[0], 2 ** -8), (dfilt, want[1], 1e-5), (dbias, dy.double().sum(0), 1e-5)):
+        assert float((a.double() - b).norm()) <= tol * float(b.norm()) + 1e-6
