@@ -145,7 +145,10 @@ __device__ __forceinline__ float cta_reduce(float v, float* sh, bool sum) {
 // on (the launch picks both by V); a longer row's rest is read three times. The next row is loaded as soon as the vectors are exponentials, and
 // the chain sequence -> number of states -> class -> logit of the states is one step further with each phase of a row.
 // grad (null: none wanted) receives the softmax.
-// The exponentials are 2^(x log2(e) - c) with a whole number c near the maximum: one rounding, no matter how large the logits are.
+// The exponentials are 2^(x log2(e) - c) with a whole number c near the maximum: one rounding each. (That of the constant, 1.3e-8 of it, moves all
+// exponents of a row alike, by less than half a unit in the last place of the logit.) Where the maximum lies beyond 2^100, as in a row that is filled
+// with the type's lowest value, the product may overflow: such a row is marked (bit 1 of wide) and left to the next kernel. (A factor and an offset
+// chosen by row, to have them right here: 75 us for 65.)
 template <int T, int NV, bool BF16>
 __global__ void __launch_bounds__(T, 768 / T)
 ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict__ row_batch, const int* __restrict__ cu, const int* __restrict__ targets,
@@ -191,6 +194,7 @@ ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict
       for (int k = 0; k < P::N; ++k) mx = fmaxf(mx, v[k]);
     }
     mx = cta_reduce<T>(mx, sh[0], false);
+    const bool huge = fabsf(mx) > 0x1p100f && fabsf(mx) < INFINITY;
     const float c = rintf(mx * kLog2e);
     auto ex = [&](float x) {
       float y;
@@ -229,7 +233,7 @@ ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict
     const int any = __syncthreads_or(far);
     if (tid == 0) {
       lse[r] = l;
-      wide[r] = any;
+      wide[r] = (any ? 1 : 0) + (huge ? 2 : 0);
     }
     if (grad != nullptr) {
       const float inv = 1.f / sum;
@@ -462,12 +466,37 @@ __device__ __forceinline__ Wide ctc_recursion(const Wide* __restrict__ prob, Wid
   return {a.m * pow2i(a.e, top) + z.m * pow2i(z.e, top), top};
 }
 
+// A row whose maximum `mx` is finite and beyond 2^100, by all threads of a CTA: two values there are equal or further apart than any exponent, so
+// the maxima share the row. What is NaN stays NaN.
+__device__ void ctc_huge_row(const void* __restrict__ logits, int is_bf16, size_t base, int V, float* __restrict__ lse, void* __restrict__ grad, float* sh) {
+  float mx = kNegInf, n = 0.f;
+  for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, ldf(logits, base + i, is_bf16));
+  auto all = [&](float v, bool sum) {
+    __syncthreads();
+    v = sum ? warp_sum(v) : warp_max(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = sh[0];
+    for (int i = 1; i < (int)blockDim.x / 32; ++i) v = sum ? v + sh[i] : fmaxf(v, sh[i]);
+    return v;
+  };
+  mx = all(mx, false);
+  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    const float x = ldf(logits, base + i, is_bf16);
+    n += x == mx ? 1.f : x != x ? x : 0.f;
+  }
+  n = all(n, true);
+  if (threadIdx.x == 0) *lse = mx + logf(n);
+  if (grad != nullptr)
+    for (int i = threadIdx.x; i < V; i += blockDim.x) stf(grad, base + i, (ldf(logits, base + i, is_bf16) == mx ? 1.f : 0.f) / n, is_bf16);
+}
+
 // One CTA per sequence, the first half of its warps alpha, the second beta. Dynamic shared memory: SE classes, 4 * SE states, of which a
 // sequence that goes through log space uses the first 2 * SE floats, and the warps' rings. link [B, SE], for the labels: the next state of the same class, 0 if there
 // is none, negative (minus one) where an earlier state has the class or the class is blank.
 template <int K, int D>
 __global__ void __launch_bounds__(K == 8 ? 832 : 512, 1)
-ctc_alpha_beta_kernel(const void* __restrict__ logits, int is_bf16, const float* __restrict__ lse, const int* __restrict__ wide,
+ctc_alpha_beta_kernel(const void* __restrict__ logits, int is_bf16, float* __restrict__ lse, const int* __restrict__ wide, void* __restrict__ grad,
                       const Wide* __restrict__ prob, Wide* __restrict__ al, Wide* __restrict__ be, const int* __restrict__ cu,
                       const int* __restrict__ targets, const int* __restrict__ tgt_lens, SeqInfo* __restrict__ info, int* __restrict__ link,
                       float* __restrict__ loss, int V, int s_pitch, int SE, int blank) {
@@ -516,6 +545,13 @@ ctc_alpha_beta_kernel(const void* __restrict__ logits, int is_bf16, const float*
     }
     return;
   }
+  for (int t0 = 0; t0 < T; t0 += blockDim.x) {
+    const int t = t0 + threadIdx.x;
+    if (!__syncthreads_or(t < T && (wide[r0 + t] & 2))) continue;
+    for (int q = t0; q < min(T, t0 + (int)blockDim.x); ++q)
+      if (wide[r0 + q] & 2) ctc_huge_row(logits, is_bf16, (size_t)(r0 + q) * V, V, lse + r0 + q, grad, reinterpret_cast<float*>(state));
+  }
+  __syncthreads();
   // ---- in log space: alpha, then beta; al and be hold logarithms in place of mantissas
   float* prev = logs;
   float* cur = logs + SE;
@@ -638,8 +674,9 @@ ctc_occupancy_kernel(const void* __restrict__ logits, int is_bf16, const int* __
   }
   blank_sum = warp_sum(blank_sum);
   __syncwarp();
+  const bool huge = fabsf(l) > 0x1p100f;  // the logarithm of the number of maxima is below the last digit of l
   auto rewrite = [&](int c, float x, float total) {
-    if (total != 0.f) stf(grad, base + c, __expf(x - l) - total, is_bf16);
+    if (total != 0.f) stf(grad, base + c, (huge ? ldf(grad, base + c, is_bf16) : __expf(x - l)) - total, is_bf16);
   };
   for (int s = 2 * lane + 1; s < se; s += 64) {
     int q = ln[s];
@@ -715,7 +752,7 @@ RB_EXPORT int rb200_ctc_loss(const void* logits, int is_bf16, const int* cu, con
     if (st) return st;
   }
   if (smem_ab > 48 * 1024) cudaFuncSetAttribute(recursion, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ab);
-  recursion<<<batch, 64 * warps, smem_ab, stream>>>(logits, is_bf16, lse, wide, prob, al, be, cu, targets, tgt_lens, info, link, loss, V, s_pitch, SE,
+  recursion<<<batch, 64 * warps, smem_ab, stream>>>(logits, is_bf16, lse, wide, grad, prob, al, be, cu, targets, tgt_lens, info, link, loss, V, s_pitch, SE,
                                                       blank);
   st = rb_check_launch("ctc_alpha_beta");
   if (st) return st;

@@ -2,6 +2,7 @@
 Fused CTC kernels (log-softmax + alpha/beta + gradient on packed logits) against torch.nn.functional.ctc_loss in fp32.
 """
 
+import math
 import pytest
 import torch
 
@@ -120,3 +121,31 @@ def test_ctc_masked_classes(value):
         assert bool(torch.isfinite(grad).all())
         if label is not None and value == float("-inf"):
             assert float(loss[1].detach()) == 0.0 and float(grad[12:21].abs().max()) == 0.0
+
+
+@gpu
+@pytest.mark.parametrize("dtype,V", [(torch.float32, 30), (torch.bfloat16, 30), (torch.bfloat16, 5003)])
+def test_ctc_frames_filled_with_the_lowest_value(dtype, V):
+    """a frame without information: every class equally likely. (Its log(V) is below the resolution of 32 bits at that size: the loss is short of it)"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import ctc
+
+    gen = torch.Generator("cuda").manual_seed(V)
+    pack = PackInfo(torch.tensor([12, 20], dtype=torch.int32), torch.device("cuda"))
+    logits = torch.randn(pack.n, V, device="cuda", generator=gen).to(dtype)
+    logits[5] = torch.finfo(dtype).min
+    logits[14] = torch.finfo(dtype).max
+    logits[15, 1:] = torch.finfo(dtype).min
+    targets = torch.randint(1, 20, (2, 4), device="cuda", dtype=torch.int32, generator=gen)
+    targets[1, 0] = 0  # frame 15 allows nothing else
+    tl = torch.tensor([4, 3], dtype=torch.int32)
+    x = logits.requires_grad_(True)
+    loss = ctc.ctc_loss_packed(x, pack, targets, tl, blank_index=V - 1)
+    (grad,) = torch.autograd.grad(loss.sum(), [x])
+    flat = logits.detach().float().clone()
+    flat[5], flat[14], flat[15, 1:] = 0.0, 0.0, -1e4
+    ref, ref_grad = _ctc_float64(flat, pack, targets, tl, V - 1, torch.ones(2, device="cuda"))
+    torch.testing.assert_close(loss.detach().double(), ref - math.log(V), atol=1e-4, rtol=1e-5)
+    # frame 15 takes the second sequence through log space: 2^-24 of a loss of about 100 per frame, 20 frames
+    tol = 1e-4 if dtype == torch.float32 else 2.0 ** -8
+    assert float((grad.double() - ref_grad).norm()) <= tol * float(ref_grad.norm())
