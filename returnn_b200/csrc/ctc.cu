@@ -624,7 +624,12 @@ ctc_occupancy_kernel(const void* __restrict__ logits, int is_bf16, const int* __
   const int se = 2 * tgt_lens[b] + 1;
   const size_t base = (size_t)r * V;
   if (seq.logp == kNegInf) {
-    for (int c = lane; c < V; c += 32) stf(grad, base + c, 0.f, is_bf16);
+    const int size = is_bf16 ? 2 : 4;
+    const Row row = is_bf16 ? row_of<true>(grad, nullptr, base, V) : row_of<false>(grad, nullptr, base, V);
+    uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<char*>(grad) + (base + row.head) * size);
+#pragma unroll 4
+    for (int i = lane; i < row.n_vec; i += 32) out[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = lane; i < row.scalars; i += 32) stf(grad, base + (is_bf16 ? scalar_at<true>(row, i) : scalar_at<false>(row, i)), 0.f, is_bf16);
     return;
   }
   const float inv = seq.in_log ? 0.f : 1.f / seq.m;

@@ -149,3 +149,24 @@ def test_ctc_frames_filled_with_the_lowest_value(dtype, V):
     # frame 15 takes the second sequence through log space: 2^-24 of a loss of about 100 per frame, 20 frames
     tol = 1e-4 if dtype == torch.float32 else 2.0 ** -8
     assert float((grad.double() - ref_grad).norm()) <= tol * float(ref_grad.norm())
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [9, 1000, 10001])
+def test_ctc_rows_of_infeasible_sequences_are_cleared(V, dtype):
+    """whole rows, wherever they start, and no others"""
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import ctc
+
+    gen = torch.Generator("cuda").manual_seed(V)
+    pack = PackInfo(torch.tensor([9, 3, 7], dtype=torch.int32), torch.device("cuda"))
+    x = torch.randn(pack.n, V, device="cuda", generator=gen).to(dtype).requires_grad_(True)
+    targets = torch.randint(0, V - 1, (3, 5), device="cuda", dtype=torch.int32, generator=gen)
+    grads = []
+    for tl in ([4, 5, 3], [4, 1, 3]):  # five labels in three frames
+        loss = ctc.ctc_loss_packed(x, pack, targets, torch.tensor(tl, dtype=torch.int32), blank_index=V - 1)
+        grads.append(torch.autograd.grad(loss.sum(), [x])[0])
+        assert (float(loss[1].detach()) == 0.0) == (tl[1] == 5)
+    assert not grads[0][9:12].any() and bool(grads[1][9:12].any(1).all())
+    assert torch.equal(grads[0][:9], grads[1][:9]) and torch.equal(grads[0][12:], grads[1][12:])
