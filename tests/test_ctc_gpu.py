@@ -170,3 +170,39 @@ def test_ctc_rows_of_infeasible_sequences_are_cleared(V, dtype):
         assert (float(loss[1].detach()) == 0.0) == (tl[1] == 5)
     assert not grads[0][9:12].any() and bool(grads[1][9:12].any(1).all())
     assert torch.equal(grads[0][:9], grads[1][:9]) and torch.equal(grads[0][12:], grads[1][12:])
+
+
+@gpu
+@pytest.mark.parametrize("lens,tlens,V", [([40, 1, 7], [9, 0, 3], 50), ([300, 260], [125, 128], 80), ([500, 31], [240, 15], 300), ([1300], [620], 37)])
+def test_ctc_recursions_in_log_space_against_float64(lens, tlens, V):
+    """
+    a label masked by a large finite number in the first frames, which the alignments can do without: every sequence takes the recursions in log
+    space. There a sum is rounded to 2^-24 of the loss per frame, and these errors add up like a random walk: 2^-24 * sqrt(frames) * loss
+    """
+    from returnn_b200.models.packing import PackInfo
+    from returnn_b200.ops import ctc
+
+    gen = torch.Generator("cuda").manual_seed(V)
+    pack = PackInfo(torch.tensor(lens, dtype=torch.int32), torch.device("cuda"))
+    targets = torch.randint(0, V - 2, (len(lens), max(tlens)), device="cuda", dtype=torch.int32, generator=gen)
+    repeat = torch.rand(targets.shape, device="cuda", generator=gen) < 0.2
+    targets[:, 1:] = torch.where(repeat[:, 1:], targets[:, :-1], targets[:, 1:])
+    logits = torch.randn(pack.n, V, device="cuda", generator=gen) * 2
+    lo = 0
+    for b, (n, s) in enumerate(zip(lens, tlens)):
+        if s:
+            targets[b, s - 1] = V - 2  # the last label, nowhere else: masked in a frame that is too early for it
+            logits[lo, V - 2] = -1e9
+        lo += n
+    x = logits.requires_grad_(True)
+    tl = torch.tensor(tlens, dtype=torch.int32)
+    loss = ctc.ctc_loss_packed(x, pack, targets, tl, blank_index=V - 1)
+    (grad,) = torch.autograd.grad(loss.sum(), [x])
+    ref, ref_grad = _ctc_float64(x, pack, targets, tl, V - 1, torch.ones(len(lens), device="cuda"))
+    torch.testing.assert_close(loss.detach().double(), ref, atol=1e-4, rtol=4 * max(lens) ** 0.5 * 2.0 ** -24)
+    bound = 8 * max(lens) ** 0.5 * 2.0 ** -24 * float(ref.max()) + 2e-5
+    assert float((grad.double() - ref_grad).norm()) <= bound * float(ref_grad.norm())
+    with torch.no_grad():  # broken input stays visible there
+        y = logits.detach().clone()
+        y[lens[0] // 2, V - 1] = float("nan")
+        assert bool(torch.isnan(ctc.ctc_loss_packed(y, pack, targets, tl, blank_index=V - 1)[0]))
