@@ -446,13 +446,13 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
   __shared__ float red[32][65];
   const int lane8 = (threadIdx.x & 7) * 8, rl = threadIdx.x >> 3;
   const int hd = heads * dim;
-  const int col = blockIdx.y * 64;  // of dqkv; dim is a multiple of 64: one head, one part
+  const int col0 = blockIdx.y * 64, col = col0 + lane8;  // of dqkv; dim is a multiple of 8: a thread's columns are of one head and one part
   const int h = col / (3 * dim);
   const int part = (col - h * 3 * dim) / dim;
   const int src_col = h * dim + (col - (h * 3 + part) * dim);
-  const __nv_bfloat16* a_src = (part == 0 ? dqu : part == 1 ? dk : dv) + src_col + lane8;
-  const __nv_bfloat16* b_src = dqv + src_col + lane8;
-  const int r_end = min(n_rows, (int)(blockIdx.x + 1) * rows_per_cta);
+  const __nv_bfloat16* a_src = (part == 0 ? dqu : part == 1 ? dk : dv) + src_col;
+  const __nv_bfloat16* b_src = dqv + src_col;
+  const int r_end = col < 3 * hd ? min(n_rows, (int)(blockIdx.x + 1) * rows_per_cta) : 0;
   float s_x[8], s_u[8], s_v[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) s_x[i] = s_u[i] = s_v[i] = 0.f;
@@ -481,30 +481,32 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
           x.v[i] = __bfloat162float(__float2bfloat16(x.v[i] + y.v[i]));
         }
       }
-      store8(dqkv, (long long)r * 3 * hd + col + lane8, x, 1);
+      store8(dqkv, (long long)r * 3 * hd + col, x, 1);
 #pragma unroll
       for (int i = 0; i < 8; ++i) s_x[i] += x.v[i];
     }
   }
-  auto leave = [&](const float* s, float* dst) {  // dst: of this CTA's 64 columns
+  auto leave = [&](const float* s, float* dst, bool queries) {  // dst: of all columns of dqkv, or of those of the queries
     if (dst == nullptr) return;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i) red[rl][lane8 + i] = s[i];
     __syncthreads();
-    if (threadIdx.x < 64) {
+    const int at = col0 + threadIdx.x, head = at / (3 * dim), in_head = at - head * 3 * dim;
+    if (threadIdx.x < 64 && at < 3 * hd && (!queries || in_head < dim)) {
       float t = 0.f;
 #pragma unroll
       for (int k = 0; k < 32; ++k) t += red[k][threadIdx.x];
-      if (ATOMIC) atomicAdd(dst + threadIdx.x, t);
-      else dst[threadIdx.x] = t;
+      dst += queries ? head * dim + in_head : at;
+      if (ATOMIC) atomicAdd(dst, t);
+      else *dst = t;
     }
   };
-  leave(s_x, sum_qkv ? sum_qkv + col : nullptr);
-  if (part == 0) {
+  leave(s_x, sum_qkv, false);
+  if (col0 % (3 * dim) < dim || col0 % (3 * dim) + 63 >= 3 * dim) {  // some of the 64 columns are a query's
     const long long slice = ATOMIC ? 0 : (long long)blockIdx.x * 2 * hd;
-    leave(s_u, sum_u ? sum_u + slice + src_col : nullptr);
-    leave(s_v, sum_v ? sum_v + slice + src_col : nullptr);
+    leave(s_u, sum_u ? sum_u + slice : nullptr, true);
+    leave(s_v, sum_v ? sum_v + slice : nullptr, true);
   }
 }
 
@@ -607,7 +609,7 @@ static int pack_rows_per_cta(int n_rows, int chunks) {
 }
 RB_EXPORT int rb200_att_pack_slices(int n_rows, int heads, int dim) {
   if (n_rows <= 0) return 0;
-  const int per = pack_rows_per_cta(n_rows, 3 * heads * dim / 64);
+  const int per = pack_rows_per_cta(n_rows, (3 * heads * dim + 63) / 64);
   return (n_rows + per - 1) / per;
 }
 
@@ -617,11 +619,11 @@ RB_EXPORT int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* 
                                   void* dqkv, float* sum_qkv, float* sum_u, float* sum_v, int n_rows, int heads, int dim, int lp, int accumulate,
                                   cudaStream_t stream) {
   if (n_rows <= 0) return RB_OK;
-  if (dim % 64 || heads <= 0 || 3LL * heads * dim / 64 > 65535) {
-    rb_set_error("att_pack_dqkv: head dim %d must be a multiple of 64 (%d heads)", dim, heads);
+  if (dim % 8 || dim <= 0 || heads <= 0 || 3LL * heads * dim / 64 >= 65535) {
+    rb_set_error("att_pack_dqkv: head dim %d must be a multiple of 8 (%d heads)", dim, heads);
     return RB_ERR_ARG;
   }
-  const int chunks = 3 * heads * dim / 64, per = pack_rows_per_cta(n_rows, chunks);
+  const int chunks = (3 * heads * dim + 63) / 64, per = pack_rows_per_cta(n_rows, chunks);
   if (!accumulate) sum_v = sum_u ? sum_u + (long long)heads * dim : nullptr;
   rb_launch_pdl(accumulate ? att_pack_dqkv_kernel<true> : att_pack_dqkv_kernel<false>, dim3((n_rows + per - 1) / per, chunks), dim3(256), 0, stream,
                 (const __nv_bfloat16*)dqu, (const __nv_bfloat16*)dqv, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, row_batch, row_pos,

@@ -322,7 +322,8 @@ def test_rel_flash_bwd_writes_the_padding(lens, H, saved):
 
 
 @gpu
-@pytest.mark.parametrize("lens,H,D", [([1], 1, 64), ([63, 2], 3, 64), ([128, 1, 0, 64], 8, 128), ([500, 300, 411], 8, 64)])
+@pytest.mark.parametrize("lens,H,D", [([1], 1, 64), ([63, 2], 3, 64), ([128, 1, 0, 64], 8, 128), ([500, 300, 411], 8, 64), ([70, 9], 3, 8), ([40, 33], 5, 24),
+                                      ([100], 2, 96), ([300, 64], 4, 32)])
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_att_pack_dqkv_leaves_the_column_sums(lens, H, D, accumulate):
     import ctypes
