@@ -58,6 +58,9 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// log(max(x, eps)) of a log-mel feature; NaN stays NaN (the maximum of NaN and eps is eps: broken audio would leave as silence)
+__device__ __forceinline__ float log_floor(float x, float eps) { return __logf(x != x ? x : fmaxf(x, eps)); }
+
 // 8 consecutive elements as floats, from bf16 (16-byte load) or fp32 (two 16-byte loads)
 struct F8 {
   float v[8];

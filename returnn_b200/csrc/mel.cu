@@ -67,7 +67,7 @@ log_mel_kernel(const float* __restrict__ audio, const int* __restrict__ lens, lo
     float acc = 0.f;
     const float* p = spow + f * n_bins;
     for (int k = 0; k < n_bins; ++k) acc += p[k] * fbank[(size_t)k * n_mel + m];
-    const float v = fr < n_frames ? __logf(fmaxf(acc, eps)) * log_scale : 0.f;
+    const float v = fr < n_frames ? log_floor(acc, eps) * log_scale : 0.f;
     out[((size_t)row * n_frames_max + fr) * n_mel + m] = v;
   }
 }
@@ -159,7 +159,7 @@ mel_from_spectrum_kernel(const float* __restrict__ spec, int ld, int slots, int 
       const int k0 = fb_start[m], n = fb_len[m];
       float acc = 0.f;
       for (int k = 0; k < n; ++k) acc += pw[k0 + k] * ws[k * n_mel + m];
-      o[m] = __logf(fmaxf(acc, eps)) * log_scale;
+      o[m] = log_floor(acc, eps) * log_scale;
     }
   }
 }

@@ -285,7 +285,7 @@ log_mel_fft_kernel(const Mel p) {
         acc += pk[2 * kPitch] * w.z;
         acc2 += pk[3 * kPitch] * w.w;
       }
-      feat[lane * feat_pitch + m] = on ? __logf(fmaxf(acc + acc2, p.eps)) * p.log_scale : 0.f;
+      feat[lane * feat_pitch + m] = on ? log_floor(acc + acc2, p.eps) * p.log_scale : 0.f;
     }
     __syncthreads();  // the features are complete, and the power array is free for the next tile
     const int n_here = min(kTile, p.n_frames_max - f0) * p.n_mel;
