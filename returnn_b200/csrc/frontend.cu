@@ -32,7 +32,7 @@ conv1_relu_pool_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__
     r /= (I)Fp;
     const int t = (int)(r % (I)T), b = (int)(r / (I)T);
     F8 o;
-    const int len = lens[b];
+    const int len = min(lens[b], T);
     if (t >= len) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) o.v[k] = 0.f;
@@ -101,7 +101,7 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
     const int fp = (int)(p % (I)Fp);
     const I r = p / (I)Fp;
     const int t0 = (int)(r % (I)runs) * kRun, b = (int)(r / (I)runs);
-    const int len = lens[b], t1 = min(t0 + kRun, len);
+    const int len = min(lens[b], T), t1 = min(t0 + kRun, len);
     if (t0 >= t1) continue;
     const bf16* xb = x + (size_t)b * T * F + 2 * fp;
     const bool lo = fp > 0, hi = 2 * fp + 2 < F;

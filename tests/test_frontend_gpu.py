@@ -81,3 +81,32 @@ def test_conv1_relu_pool_backward(lens, F, C, with_bias):
     # 32-bit sums of at most 3000 products; inputs drawn from a continuous distribution: no ties of the two candidates but by chance
     for got, want in ((dw - 1, w64.grad.view(C, 9)), (db - 1, b64.grad)):
         assert (got.double() - want).norm() <= 1e-3 * want.norm() + 1e-5
+
+
+@gpu
+def test_conv1_lengths_beyond_the_batch_count_as_its_length():
+    """forward and backward of the first convolution read no frames behind those that are there"""
+    import ctypes
+    from returnn_b200.ops import _lib
+
+    torch.manual_seed(1)
+    dev, bf, B, T, F, C = "cuda", torch.bfloat16, 2, 13, 6, 32
+    x = torch.randn(B + 1, T, F, device=dev).to(bf)
+    dy = torch.randn(B + 1, T, F // 2, C, device=dev).to(bf)
+    x[B], dy[B] = float("nan"), float("nan")  # what stands behind the batch
+    w, b = torch.randn(C, 9, device=dev), torch.randn(C, device=dev)
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    fwd = _lib.bind("rb200_conv1_relu_pool_fwd", [vp, vp, vp, vp, i32, i32, i32, i32, vp, vp])
+    bwd = _lib.bind("rb200_conv1_relu_pool_bwd", [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
+    res = []
+    for n in (T, T + 5):
+        lens = torch.full((B,), n, dtype=torch.int32, device=dev)
+        y, dw, db = torch.empty(B, T, F // 2, C, device=dev, dtype=bf), torch.zeros(C, 9, device=dev), torch.zeros(C, device=dev)
+        # the second sequence alone: its frames are the last ones
+        _lib.check(fwd(x[1].data_ptr(), w.data_ptr(), b.data_ptr(), lens.data_ptr(), 1, T, F, C, y.data_ptr(), _lib.stream_ptr()), "fwd")
+        _lib.check(bwd(x[1].data_ptr(), w.data_ptr(), b.data_ptr(), lens.data_ptr(), dy[1].data_ptr(), 1, T, F, C, dw.data_ptr(), db.data_ptr(),
+                       _lib.stream_ptr()), "bwd")
+        res.append((y[:1], dw, db))
+    assert torch.equal(res[0][0], res[1][0])
+    for a, c in zip(res[0][1:], res[1][1:]):
+        torch.testing.assert_close(a, c, atol=1e-4, rtol=1e-4)
