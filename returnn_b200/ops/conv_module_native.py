@@ -45,59 +45,56 @@ class _ConvModuleFn(torch.autograd.Function):
         y = torch.empty(N, C, dtype=torch.bfloat16, device=dev)
         own_stats = training or running_mean is None
         part = torch.empty(n_tiles * 2 * C, dtype=torch.float32, device=dev) if own_stats or K > 32 else None
-        s = _lib.stream_ptr()
-        fn = _lib.bind("rb200_glu_dwconv_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(x.data_ptr(), f32.data_ptr(), _p(b32), row_batch.data_ptr(), row_pos.data_ptr(), lens.data_ptr(), y.data_ptr(),
-                      _p(part), N, lens.shape[0], C, K, s), "glu_dwconv_fwd")
-        mean = torch.empty(C, dtype=torch.float32, device=dev)
-        rstd = torch.empty(C, dtype=torch.float32, device=dev)
-        if own_stats:
-            fn = _lib.bind("rb200_bn_stats", [_vp, _i32, _i32, _f32, _f32, _f32, _vp, _vp, _vp, _vp, _vp])
-            upd = training and running_mean is not None
-            _lib.check(fn(part.data_ptr(), n_tiles, C, float(N), float(eps), float(momentum), mean.data_ptr(), rstd.data_ptr(),
-                          running_mean.data_ptr() if upd else None, running_var.data_ptr() if upd else None, s), "bn_stats")
-            _lib.count_launch(2)
-        else:
-            mean.copy_(running_mean.float())
-            rstd.copy_(torch.rsqrt(running_var.float() + eps))
+        stats = torch.empty(2, C, dtype=torch.float32, device=dev)  # mean, 1 / deviation
+        if not own_stats:
+            stats[0].copy_(running_mean.float())
+            stats[1].copy_(torch.rsqrt(running_var.float() + eps))
+        upd = training and running_mean is not None
         z = torch.empty(N, C, dtype=torch.bfloat16, device=dev)
-        fn = _lib.bind("rb200_bn_silu_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp])
-        _lib.check(fn(y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), _p(g32), _p(be32), z.data_ptr(), N, C, s), "bn_silu_fwd")
-        _lib.count_launch(2)
-        ctx.save_for_backward(x, f32, y, mean, rstd, g32, be32, row_batch, row_pos, lens)
+        fn = _lib.bind("rb200_conv_module_fwd", [_vp] * 14 + [_i32] * 5 + [_f32, _f32, _vp])
+        _lib.check(fn(x.data_ptr(), f32.data_ptr(), _p(b32), _p(g32), _p(be32), row_batch.data_ptr(), row_pos.data_ptr(), lens.data_ptr(), y.data_ptr(),
+                      z.data_ptr(), _p(part), stats.data_ptr(), running_mean.data_ptr() if upd else None, running_var.data_ptr() if upd else None,
+                      N, lens.shape[0], C, K, 1 if own_stats else 0, eps, momentum, _lib.stream_ptr()), "conv_module_fwd")
+        _lib.count_launch(2 + (own_stats and (2 if K <= 32 else 1)))
+        ctx.save_for_backward(x, f32, y, stats, g32, be32, row_batch, row_pos, lens)
         ctx.meta = (N, C, K, training, bias is not None, gamma is not None, beta is not None, filt.shape, filt.dtype,
                     bias.dtype if bias is not None else None, gamma.dtype if gamma is not None else None, beta.dtype if beta is not None else None)
         return z
 
     @staticmethod
     def backward(ctx, dz):
-        x, f32, y, mean, rstd, g32, be32, row_batch, row_pos, lens = ctx.saved_tensors
+        x, f32, y, stats, g32, be32, row_batch, row_pos, lens = ctx.saved_tensors
         N, C, K, training, has_bias, has_gamma, has_beta, fshape, fdtype, bdtype, gdtype, bedtype = ctx.meta
         dev = dz.device
         dz = dz.contiguous()
         s = _lib.stream_ptr()
         n_tiles_a = min(296, max(1, (N + 15) // 16))
         ds = torch.empty(N, C, dtype=torch.bfloat16, device=dev)
-        n_tiles = (N + _TT - 1) // _TT
         # the sums of the two passes, one after the other in the same scratch
-        part = torch.empty(max(n_tiles_a * 2 * C, n_tiles * C * (K + 1)), dtype=torch.float32, device=dev)
+        part = torch.empty(max(n_tiles_a * 2 * C, (N + _TT - 1) // _TT * C * (K + 1)), dtype=torch.float32, device=dev)
         sum_ds = torch.empty(C, dtype=torch.float32, device=dev)
         sum_ds_yh = torch.empty(C, dtype=torch.float32, device=dev)
-        fn = _lib.bind("rb200_bn_silu_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _i64, _i32, _i32, _vp])
-        _lib.check(fn(y.data_ptr(), dz.data_ptr(), mean.data_ptr(), rstd.data_ptr(), _p(g32), _p(be32), ds.data_ptr(), part.data_ptr(),
-                      n_tiles_a, sum_ds.data_ptr(), sum_ds_yh.data_ptr(), N, C, 1 if training else 0, s), "bn_silu_bwd")
-        _lib.count_launch(3 if training else 2)
-        if not training:
+        dx = torch.empty_like(x)
+        dfilt = torch.empty(C, K, dtype=torch.float32, device=dev)
+        dbias = torch.empty(C, dtype=torch.float32, device=dev) if has_bias else None
+        if training:
+            fn = _lib.bind("rb200_conv_module_bwd", [_vp] * 12 + [_i32] + [_vp] * 5 + [_i32] * 4 + [_vp])
+            _lib.check(fn(x.data_ptr(), y.data_ptr(), dz.data_ptr(), stats.data_ptr(), f32.data_ptr(), _p(g32), _p(be32), row_batch.data_ptr(),
+                          row_pos.data_ptr(), lens.data_ptr(), ds.data_ptr(), part.data_ptr(), n_tiles_a, sum_ds.data_ptr(), sum_ds_yh.data_ptr(),
+                          dx.data_ptr(), dfilt.data_ptr(), _p(dbias), N, lens.shape[0], C, K, s), "conv_module_bwd")
+            _lib.count_launch(5)
+        else:
+            mean, rstd = stats
+            fn = _lib.bind("rb200_bn_silu_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _i64, _i32, _i32, _vp])
+            _lib.check(fn(y.data_ptr(), dz.data_ptr(), mean.data_ptr(), rstd.data_ptr(), _p(g32), _p(be32), ds.data_ptr(), part.data_ptr(),
+                          n_tiles_a, sum_ds.data_ptr(), sum_ds_yh.data_ptr(), N, C, 0, s), "bn_silu_bwd")
             # eval statistics are constants: dy = gamma * rstd * ds
             scale = rstd * (g32 if g32 is not None else 1.0)
             ds = (ds.float() * scale).to(torch.bfloat16)
-        dx = torch.empty_like(x)
-        dfilt = torch.empty(C, K, dtype=torch.float32, device=dev)
-        dbias = torch.empty(C, dtype=torch.float32, device=dev)
-        fn = _lib.bind("rb200_glu_dwconv_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
-        _lib.check(fn(x.data_ptr(), ds.data_ptr(), f32.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), lens.data_ptr(), dx.data_ptr(),
-                      part.data_ptr(), dfilt.data_ptr(), dbias.data_ptr(), N, lens.shape[0], C, K, s), "glu_dwconv_bwd")
-        _lib.count_launch(2)
+            fn = _lib.bind("rb200_glu_dwconv_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp])
+            _lib.check(fn(x.data_ptr(), ds.data_ptr(), f32.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), lens.data_ptr(), dx.data_ptr(),
+                          part.data_ptr(), dfilt.data_ptr(), _p(dbias), N, lens.shape[0], C, K, s), "glu_dwconv_bwd")
+            _lib.count_launch(4)
         return (dx, dfilt.reshape(fshape).to(fdtype), dbias.to(bdtype) if has_bias else None,
                 sum_ds_yh.to(gdtype) if has_gamma else None, sum_ds.to(bedtype) if has_beta else None,
                 None, None, None, None, None, None, None, None)
