@@ -113,9 +113,10 @@ def test_conv_module_windows_against_float64(lens, C, K, training):
     ref = torch.nn.functional.silu(y * g64 + b64)
     refs = [ref, *torch.autograd.grad(ref, [x64, f64, g64, b64] + ([] if training else [c64]), dz.double())]
     for name, a, b in zip(["z", "dx", "dfilt", "dgamma", "dbeta", "dbias"], got, refs):
-        if training and n < 8:
-            continue  # differences of a few rows from their mean: rounding of y is not small against them
         a = a.detach()
+        if training and n == 1 and name not in ("z", "dbeta"):
+            assert bool(torch.isfinite(a).all()), name  # the one row is its own mean: 0 but for the rounding of ds
+            continue
         assert float((a.double() - b).norm()) <= 8e-3 * float(b.norm()), (name, float((a.double() - b).norm() / b.norm()))
 
 
