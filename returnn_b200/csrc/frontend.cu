@@ -107,7 +107,7 @@ conv1_relu_pool_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__
     const bool lo = fp > 0, hi = 2 * fp + 2 < F;
     auto row = [&](int tt, float (&v)[4]) {
       const bool in = tt >= 0 && tt < len;
-      const bf16* q = xb + (long long)(in ? tt : 0) * F;
+      const bf16* q = xb + (I)(in ? tt : 0) * (I)F;
       v[0] = in && lo ? __bfloat162float(q[-1]) : 0.f;
       v[1] = in ? __bfloat162float(q[0]) : 0.f;
       v[2] = in ? __bfloat162float(q[1]) : 0.f;
