@@ -58,8 +58,14 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// log(max(x, eps)) of a log-mel feature; NaN stays NaN (the maximum of NaN and eps is eps: broken audio would leave as silence)
-__device__ __forceinline__ float log_floor(float x, float eps) { return __logf(x != x ? x : fmaxf(x, eps)); }
+// the larger of two values, NaN if one of them is (fmaxf gives the other one then)
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+// log(max(x, eps)) of a log-mel feature; NaN stays NaN: broken audio does not leave as silence
+__device__ __forceinline__ float log_floor(float x, float eps) { return __logf(max_nan(x, eps)); }
 
 // 8 consecutive elements as floats, from bf16 (16-byte load) or fp32 (two 16-byte loads)
 struct F8 {

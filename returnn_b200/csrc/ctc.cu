@@ -28,11 +28,6 @@ __device__ __forceinline__ void stf(void* x, size_t i, float v, int is_bf16) {
   if (is_bf16) reinterpret_cast<__nv_bfloat16*>(x)[i] = __float2bfloat16(v);
   else reinterpret_cast<float*>(x)[i] = v;
 }
-__device__ __forceinline__ float max_nan(float a, float b) {  // NaN if one of them is
-  float m;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-  return m;
-}
 // log(e^a + e^b + e^c); all three -inf give -inf
 __device__ __forceinline__ float log_add3(float a, float b, float c) {
   const float lo = fminf(a, b), hi = max_nan(a, b), m = max_nan(hi, c);
