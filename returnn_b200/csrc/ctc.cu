@@ -147,9 +147,9 @@ __device__ __forceinline__ float cta_reduce(float v, float* sh, bool sum) {
 // the chain sequence -> number of states -> class -> logit of the states is one step further with each phase of a row.
 // grad (null: none wanted) receives the softmax.
 // The exponentials are 2^(x log2(e) - c) with a whole number c near the maximum: one rounding each. (That of the constant, 1.3e-8 of it, moves all
-// exponents of a row alike, by less than half a unit in the last place of the logit.) Where the maximum lies beyond 2^100, as in a row that is filled
-// with the type's lowest value, the product may overflow: such a row is marked (bit 1 of wide) and left to the next kernel. (A factor and an offset
-// chosen by row, to have them right here: 75 us for 65.)
+// exponents of a row alike, by less than half a unit in the last place of the logit.) Where the maximum lies beyond
+// 2^30, c is off by up to 64 and more, at last the product overflows (a frame that is filled with the type's lowest value): the log-sum-exp is not
+// finite then, and the row is left to the next kernel. (A factor and an offset chosen by row, to have such rows right here: 75 us for 65.)
 template <int T, int NV, bool BF16>
 __global__ void __launch_bounds__(T, 768 / T)
 ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict__ row_batch, const int* __restrict__ cu, const int* __restrict__ targets,
@@ -195,7 +195,6 @@ ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict
       for (int k = 0; k < P::N; ++k) mx = fmaxf(mx, v[k]);
     }
     mx = cta_reduce<T>(mx, sh[0], false);
-    const bool huge = fabsf(mx) > 0x1p100f && fabsf(mx) < INFINITY;
     const float c = rintf(mx * kLog2e);
     auto ex = [&](float x) {
       float y;
@@ -225,7 +224,7 @@ ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict
     sum = cta_reduce<T>(sum, sh[1], true);
     const float l = fmaf(c, 0.693147182464599609375f, fmaf(c, -1.904654323148236e-9f, logf(sum)));  // ln 2 in two parts
     const int clsn = tid < sen ? cls_of(bn, tid) : blank;
-    bool far = false;
+    bool far = !(fabsf(l) < INFINITY);
     for (int s = tid; s < se; s += T) {
       const float lp = (s == tid ? mine : ldf(logits, base + cls_of(b, s), BF16)) - l;
       far |= lp < limit && lp != kNegInf;
@@ -234,7 +233,7 @@ ctc_softmax_gather_kernel(const void* __restrict__ logits, const int* __restrict
     const int any = __syncthreads_or(far);
     if (tid == 0) {
       lse[r] = l;
-      wide[r] = (any ? 1 : 0) + (huge ? 2 : 0);
+      wide[r] = any;
     }
     if (grad != nullptr) {
       const float inv = 1.f / sum;
@@ -467,8 +466,8 @@ __device__ __forceinline__ Wide ctc_recursion(const Wide* __restrict__ prob, Wid
   return {a.m * pow2i(a.e, top) + z.m * pow2i(z.e, top), top};
 }
 
-// A row whose maximum `mx` is finite and beyond 2^100, by all threads of a CTA: two values there are equal or further apart than any exponent, so
-// the maxima share the row. What is NaN stays NaN.
+// A row whose maximum lies beyond 2^30, by all threads of a CTA: two values there are equal or so far apart (2^7) that the maxima share the row.
+// Rows with an infinite maximum, and rows that are not finite because they hold NaN, stay as the pass over the logits has left them.
 __device__ void ctc_huge_row(const void* __restrict__ logits, int is_bf16, size_t base, int V, float* __restrict__ lse, void* __restrict__ grad, float* sh) {
   float mx = kNegInf, n = 0.f;
   for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, ldf(logits, base + i, is_bf16));
@@ -482,6 +481,7 @@ __device__ void ctc_huge_row(const void* __restrict__ logits, int is_bf16, size_
     return v;
   };
   mx = all(mx, false);
+  if (fabsf(mx) <= 0x1p30f || fabsf(mx) == INFINITY) return;
   for (int i = threadIdx.x; i < V; i += blockDim.x) {
     const float x = ldf(logits, base + i, is_bf16);
     n += x == mx ? 1.f : x != x ? x : 0.f;
@@ -548,9 +548,9 @@ ctc_alpha_beta_kernel(const void* __restrict__ logits, int is_bf16, float* __res
   }
   for (int t0 = 0; t0 < T; t0 += blockDim.x) {
     const int t = t0 + threadIdx.x;
-    if (!__syncthreads_or(t < T && (wide[r0 + t] & 2))) continue;
-    for (int q = t0; q < min(T, t0 + (int)blockDim.x); ++q)
-      if (wide[r0 + q] & 2) ctc_huge_row(logits, is_bf16, (size_t)(r0 + q) * V, V, lse + r0 + q, grad, reinterpret_cast<float*>(state));
+    if (!__syncthreads_or(t < T && !(fabsf(lse[r0 + t]) < INFINITY))) continue;
+    for (int q = r0 + t0; q < r0 + min(T, t0 + (int)blockDim.x); ++q)
+      if (!(fabsf(lse[q]) < INFINITY)) ctc_huge_row(logits, is_bf16, (size_t)q * V, V, lse + q, grad, reinterpret_cast<float*>(state));
   }
   __syncthreads();
   // ---- in log space, alpha and beta at the same time as above; al and be hold logarithms in place of mantissas. States i, i + G, ... per
@@ -701,7 +701,7 @@ ctc_occupancy_kernel(const void* __restrict__ logits, int is_bf16, const int* __
   }
   blank_sum = warp_sum(blank_sum);
   __syncwarp();
-  const bool huge = fabsf(l) > 0x1p100f;  // the logarithm of the number of maxima is below the last digit of l
+  const bool huge = fabsf(l) > 0x1p14f;  // the last digit of l is as coarse as those of the softmax that is there
   auto rewrite = [&](int c, float x, float total) {
     if (total != 0.f) stf(grad, base + c, (huge ? ldf(grad, base + c, is_bf16) : __expf(x - l)) - total, is_bf16);
   };

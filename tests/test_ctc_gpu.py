@@ -125,17 +125,22 @@ def test_ctc_masked_classes(value):
 
 @gpu
 @pytest.mark.parametrize("dtype,V", [(torch.float32, 30), (torch.bfloat16, 30), (torch.bfloat16, 5003)])
-def test_ctc_frames_filled_with_the_lowest_value(dtype, V):
-    """a frame without information: every class equally likely. (Its log(V) is below the resolution of 32 bits at that size: the loss is short of it)"""
+@pytest.mark.parametrize("value", [None, -1e9, -1e10, -1e30])
+def test_ctc_frames_filled_with_the_lowest_value(dtype, V, value):
+    """
+    or another large number: a frame without information, every class equally likely. (Its log(V) is below the resolution of 32 bits at that size:
+    the loss is short of it)
+    """
     from returnn_b200.models.packing import PackInfo
     from returnn_b200.ops import ctc
 
     gen = torch.Generator("cuda").manual_seed(V)
     pack = PackInfo(torch.tensor([12, 20], dtype=torch.int32), torch.device("cuda"))
     logits = torch.randn(pack.n, V, device="cuda", generator=gen).to(dtype)
-    logits[5] = torch.finfo(dtype).min
-    logits[14] = torch.finfo(dtype).max
-    logits[15, 1:] = torch.finfo(dtype).min
+    value = torch.finfo(dtype).min if value is None else value
+    logits[5] = value
+    logits[14] = -value
+    logits[15, 1:] = value
     targets = torch.randint(1, 20, (2, 4), device="cuda", dtype=torch.int32, generator=gen)
     targets[1, 0] = 0  # frame 15 allows nothing else
     tl = torch.tensor([4, 3], dtype=torch.int32)
@@ -203,6 +208,7 @@ def test_ctc_recursions_in_log_space_against_float64(lens, tlens, V):
     bound = 8 * max(lens) ** 0.5 * 2.0 ** -24 * float(ref.max()) + 2e-5
     assert float((grad.double() - ref_grad).norm()) <= bound * float(ref_grad.norm())
     with torch.no_grad():  # broken input stays visible there
-        y = logits.detach().clone()
-        y[lens[0] // 2, V - 1] = float("nan")
-        assert bool(torch.isnan(ctc.ctc_loss_packed(y, pack, targets, tl, blank_index=V - 1)[0]))
+        for value in (float("nan"), float("inf")):
+            y = logits.detach().clone()
+            y[lens[0] // 2, V - 1] = value
+            assert bool(torch.isnan(ctc.ctc_loss_packed(y, pack, targets, tl, blank_index=V - 1)[0]))
