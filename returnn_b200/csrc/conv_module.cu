@@ -124,7 +124,7 @@ __device__ __forceinline__ void load_chan8(const float* __restrict__ p, int c, f
 
 // Rows of 8-channel groups: a thread keeps its channels and their constants (the grid is a whole number of rows) and takes every
 // grid-th row, kRowsInFlight loads at a time. With the constants read once per group of eight values (40 scalar loads for two 16-byte
-// ones) these kernels were bound by the L1: 19.5 (forward) and 23.4 us (backward, second pass) for 6889 x 512, now 6.0 and 6.5.
+// ones) these kernels were bound by the L1: 22 (forward) and 28 us (backward, second pass) for 7900 x 512 in a pass, now 8 and 6.5.
 constexpr int kRowsInFlight = 4;
 __host__ __device__ inline int rows_grid(long long total8, int groups) {
   int a = groups, b = 256;  // CTAs in multiples of groups / gcd(groups, 256): grid * 256 threads are whole rows
@@ -402,8 +402,8 @@ glu_dwconv_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
 // instructions for one product or a second pass, and the rest of the CTA waited). The price is KT - 1 rows of staging per sequence; groups
 // of kRpt rows that hold no packed row are skipped. A CTA owns CC channels and walks over a piece of the rows in steps of kStep: the staged
 // rows stand in a ring, a step brings in the kStep rows that the one before has not seen, and their loads are in flight during the products
-// of that one. (A CTA per 64 rows that stages, synchronises, multiplies and stores: every chain of latencies stands alone.) 6889 x 512 in 36
-// sequences, 32 taps: forward 34 -> 18 us, backward 52 -> 32; the products alone are 3 and 6 at full rate, 55 % of the issue slots are used.
+// of that one. (A CTA per 64 rows that stages, synchronises, multiplies and stores: every chain of latencies stands alone.) 7900 x 512 in 36
+// sequences, 32 taps: forward 28 -> 18 us, backward 47 -> 34; the products alone are 3 and 6 at full rate, 41 % of the issue slots are used.
 constexpr int KM2 = 32;         // most taps (filters with fewer taps are zero-padded to 16 or 32)
 constexpr int kRpt = 8;         // rows per thread
 constexpr int kStep = 32;       // output rows per step: 64 channels x 4 row groups in 256 threads

@@ -1,6 +1,6 @@
 // CTC loss with fused log-softmax on packed logits [N, V] (bf16 or fp32), forward and gradient in three launches:
 //
-//   ctc_softmax_gather   one CTA per frame: the row is read once and kept in registers, log-sum-exp over the vocabulary, the probabilities of
+//   ctc_softmax_gather   1 to 24 warps per frame: the row is read once and kept in registers, log-sum-exp over the vocabulary, the probabilities of
 //                        the 2S+1 extended states (blank, l1, blank, l2, ..., blank), and the softmax straight to the gradient
 //   ctc_alpha_beta       one CTA per sequence: the alpha and the beta recursion run at the same time in the two halves of the CTA, and the
 //                        log-likelihood
@@ -11,9 +11,9 @@
 // lse [N], wide [N], prob, alpha, beta [N, SE + 1] numbers with an exponent of their own (8 bytes), and 4 + SE words per sequence.
 // Infeasible alignments (fewer frames than needed) give loss 0 and zero gradient (zero_infinity semantics).
 //
-// 7900 frames x 10001 classes in 36 sequences of up to 333 frames, 67 labels (bf16): softmax 65 us (read and written once, 316 MB: 48 at the
-// rate of a copy), recursions 53 (333 dependent frames), occupancies 20 (four dependent loads a frame), scaling in the backward pass 48 (at
-// the rate of a copy). Before: log-sum-exp 44, recursions in log space 94, gradient in a pass of its own 94, scaling 49.
+// 7900 frames x 10001 classes in 36 sequences of up to 333 frames, 67 labels (bf16): softmax 64 us (read and written once, 316 MB: 48 at the
+// rate of a copy), recursions 52 (333 dependent frames), occupancies 20 (four dependent loads a frame), scaling in the backward pass 50 (316 MB, near
+// the rate of a copy). Before: log-sum-exp 51, recursions in log space 92, gradient in a pass of its own 93, scaling 54.
 #include <algorithm>
 #include "common.cuh"
 

@@ -9,9 +9,9 @@
 // frame, so the mel sums read one row of the array per bin without bank conflicts and the filter weights as broadcasts (with a lane per
 // filter the lanes' ranges start anywhere: several conflicts per read). The features of a tile are one contiguous piece of the output.
 //
-// Bound by the instructions and the shared-memory accesses of the transform (36 us of 56 at 64 utterances of 10 s, 64 k frames; the mel sums
+// Bound by the instructions and the shared-memory accesses of the transform (36 us of 58 at 64 utterances of 10 s, 64 k frames; the mel sums
 // take 14; DRAM 8 % busy, 61 MB); two or three CTAs per SM make no difference. The transform as a matrix product on the tensor cores (mel.cu)
-// takes 88 GFLOP for fp32 precision there and moves the spectrum through memory twice: 150 us, error 6e-7 against 64 bits, here 1.7e-7.
+// takes 79 GFLOP for fp32 precision there and moves the spectrum through memory twice: 147 us, error 6e-7 against 64 bits, here 1.7e-7.
 #include <algorithm>
 #include "common.cuh"
 

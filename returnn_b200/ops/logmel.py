@@ -139,7 +139,7 @@ def _log_mel_gemm(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, f
 
 
 def _log_mel_fft(flat: torch.Tensor, l32, *, window, step, n_fft, n_mel, win, fb, scale, n_frames, out) -> bool:
-    """one kernel, where the library has it for these sizes; device time for one utterance of 0.5 s 8 us, 64 of 10 s 56 us (the others: 62, 150)"""
+    """one kernel, where the library has it for these sizes; device time for one utterance of 0.5 s 8 us, 64 of 10 s 58 us (the others: 62, 147)"""
     if os.environ.get("RETURNN_B200_LOGMEL", "auto") in ("direct", "gemm") or not 0 < window <= n_fft:
         return False
     lib = _lib.get_lib()
