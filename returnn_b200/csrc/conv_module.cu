@@ -636,8 +636,9 @@ bn_part_kernel(const __nv_bfloat16* __restrict__ y, float* __restrict__ part, in
   }
 }
 
-// dfilter / dbias sums stay in registers, over all pieces of a CTA; partial per CTA [gridDim.x][C][K+1]
-template <int KT>
+// dfilter / dbias sums stay in registers, over all pieces of a CTA; partial per CTA [gridDim.x][C][K+1]. MANY: more pieces than CTAs (the loop
+// around a piece costs 2 % where there is but one)
+template <int KT, bool MANY>
 __global__ void __launch_bounds__(kWinThreads, 2)
 glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, const float* __restrict__ filt,
                        const int* __restrict__ row_batch, __nv_bfloat16* __restrict__ dx, float* __restrict__ part, int n_rows, int n_seqs, int C,
@@ -655,7 +656,10 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   const int right = K - 1 - left;
   const int c0 = blockIdx.y * CC;
   const int cg = (tid & 7) * 8;
+  int at_piece = blockIdx.x;
+  auto piece_map = [&]() { return stage_map(map, map + kMap, row_batch, at_piece * piece - right, piece + kHalo + kStep + 1, KT - 1, n_rows, n_seqs); };
   stage_filter(sf, filt, c0, K);
+  piece_map();
   __syncthreads();
   uint4 pd, pa, pg;
   auto fetch = [&](int staged) {  // rows staged .. staged + 31
@@ -675,6 +679,7 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     ring_store8(ring_h, staged + (tid >> 3), cg, h);
     ring_store8(ring_s, staged + (tid >> 3), cg, s);
   };
+  fetch(0);
   const int c = tid % CC;
   const int rg = tid / CC;
   float fr[KT];  // flipped filter: fr[m] = f[K-1-m]
@@ -709,11 +714,7 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     for (int i = 0; i < kRpt; ++i) dbias += v[i] = ring_dy[((at + i + right) & (kRing - 1)) * CC + c];
     window_corr<KT, OFF>(ring_h, col, v, df);
   };
-  for (int at_piece = blockIdx.x; at_piece < pieces; at_piece += gridDim.x) {
-    if (at_piece != (int)blockIdx.x) __syncthreads();  // the map and the rows of the piece before have been read
-    const bool found = stage_map(map, map + kMap, row_batch, at_piece * piece - right, piece + kHalo + kStep + 1, KT - 1, n_rows, n_seqs);
-    if (!__syncthreads_or(found)) continue;  // empty sequences only
-    fetch(0);
+  auto walk = [&]() {  // over the rows of the piece whose first ones have been fetched
     place(0);
     fetch(kHalo);
     for (int step = 0; step * kStep < piece; ++step) {
@@ -728,6 +729,15 @@ glu_dwconv_bwd2_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
       if (at >= piece || any == -1) continue;
       if (base & 8) rows(std::integral_constant<int, 8>(), at);
       else rows(std::integral_constant<int, 0>(), at);
+    }
+  };
+  walk();
+  if (MANY) {
+    for (at_piece += gridDim.x; at_piece < pieces; at_piece += gridDim.x) {
+      __syncthreads();  // the map and the rows of the piece before have been read
+      if (!__syncthreads_or(piece_map())) continue;  // empty sequences only
+      fetch(0);
+      walk();
     }
   }
   // sum the row groups in shared memory, one after the other (the same sum in every run), one partial per CTA
@@ -952,13 +962,16 @@ RB_EXPORT int rb200_glu_dwconv_bwd_ex(const void* x, const void* dy, const float
   if (K <= KM2) {
     static bool attr2 = false;
     if (!attr2) {
-      cudaFuncSetAttribute(glu_dwconv_bwd2_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
-      cudaFuncSetAttribute(glu_dwconv_bwd2_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
+      for (auto kernel : {glu_dwconv_bwd2_kernel<16, false>, glu_dwconv_bwd2_kernel<32, false>, glu_dwconv_bwd2_kernel<16, true>, glu_dwconv_bwd2_kernel<32, true>})
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
       attr2 = true;
     }
     const Pieces pc = pieces_of(n_rows, n_seqs, C, K, kBwdCtas);
     row_ctas = pc.walkers;  // every CTA leaves one partial
-    rb_launch_pdl(K <= 16 ? glu_dwconv_bwd2_kernel<16> : glu_dwconv_bwd2_kernel<32>, dim3(pc.walkers, C / CC), dim3(kWinThreads), kBwd2Smem, stream,
+    const bool many = pc.walkers < pc.n;
+    auto kernel = K <= 16 ? (many ? glu_dwconv_bwd2_kernel<16, true> : glu_dwconv_bwd2_kernel<16, false>)
+                          : (many ? glu_dwconv_bwd2_kernel<32, true> : glu_dwconv_bwd2_kernel<32, false>);
+    rb_launch_pdl(kernel, dim3(pc.walkers, C / CC), dim3(kWinThreads), kBwd2Smem, stream,
                   (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, filt, row_batch, (__nv_bfloat16*)dx, part, n_rows, n_seqs, C, K, pc.rows, pc.n);
     int st2 = rb_check_launch("glu_dwconv_bwd2");
     if (st2) return st2;
