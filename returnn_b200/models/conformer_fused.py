@@ -129,7 +129,8 @@ def _frontend_native(enc, feats: torch.Tensor, lens_host: torch.Tensor):
     lens2 = -(-lens1 // strides[2][0])
     # the padded lengths of the intermediate tensors follow the padded input length, like the torch path
     pack = PackInfo(lens2.to(torch.int32), feats.device)
-    lens_dev = host_to_device(torch.stack([lens0, lens1, lens2]).to(torch.int32), feats.device)
+    # (a length beyond the batch: no frames behind it)
+    lens_dev = host_to_device(torch.stack([lens0.clamp(max=feats.shape[1]), lens1, lens2]).to(torch.int32), feats.device)
     params = [(c.filter.raw_tensor, c.bias.raw_tensor if c.bias is not None else None) for c in convs]
     x = _fe.conv_subsample_packed(feats.to(torch.bfloat16), lens_dev, pack, params, (strides[1][0], strides[2][0]))
     return x, pack

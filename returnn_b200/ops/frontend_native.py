@@ -165,7 +165,7 @@ def conv_subsample_packed(feats: torch.Tensor, lens_dev: torch.Tensor, pack, con
                           time_strides: Tuple[int, int]) -> torch.Tensor:
     """
     :param feats: [B, T, F] bf16 on the device (frames beyond the lengths may hold anything)
-    :param lens_dev: int32 [3, B] on the device: lengths at the input, after layer 2, after layer 3
+    :param lens_dev: int32 [3, B] on the device: lengths at the input (at most T), after layer 2, after layer 3
     :param pack: PackInfo of the output frames (lengths after layer 3)
     :param conv_params: [(filter [C_out, C_in, 3, 3], bias [C_out] or None)] x 3
     :param time_strides: time strides of layers 2 and 3

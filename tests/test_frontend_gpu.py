@@ -84,29 +84,31 @@ def test_conv1_relu_pool_backward(lens, F, C, with_bias):
 
 
 @gpu
-def test_conv1_lengths_beyond_the_batch_count_as_its_length():
-    """forward and backward of the first convolution read no frames behind those that are there"""
-    import ctypes
-    from returnn_b200.ops import _lib
+def test_frontend_lengths_beyond_the_batch_read_no_frames_behind_it():
+    """rows and parameter gradients as with the batch's own length, for the output frames that do not see its end"""
+    from returnn_b200.tensor import Dim
+    from returnn_b200.frontend.encoder.conformer import ConformerEncoder, ConformerConvSubsample
+    from returnn_b200.torch.frontend.bridge import rf_module_to_pt_module
+    from returnn_b200.models import conformer_fused
+    from returnn_b200.utils.basic import BehaviorVersion
 
-    torch.manual_seed(1)
-    dev, bf, B, T, F, C = "cuda", torch.bfloat16, 2, 13, 6, 32
-    x = torch.randn(B + 1, T, F, device=dev).to(bf)
-    dy = torch.randn(B + 1, T, F // 2, C, device=dev).to(bf)
-    x[B], dy[B] = float("nan"), float("nan")  # what stands behind the batch
-    w, b = torch.randn(C, 9, device=dev), torch.randn(C, device=dev)
-    vp, i32 = ctypes.c_void_p, ctypes.c_int
-    fwd = _lib.bind("rb200_conv1_relu_pool_fwd", [vp, vp, vp, vp, i32, i32, i32, i32, vp, vp])
-    bwd = _lib.bind("rb200_conv1_relu_pool_bwd", [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
+    BehaviorVersion._reset(24)
+    torch.manual_seed(0)
+    f = Dim(80, name="feat")
+    enc = ConformerEncoder(f, Dim(64, name="model"), num_layers=1, num_heads=1, ff_dim=Dim(64, name="ff"), conv_kernel_size=3, dropout=0.0, att_dropout=0.0,
+                           input_layer=ConformerConvSubsample(f, out_dims=[Dim(32, name="c1"), Dim(64, name="c2"), Dim(64, name="c3")],
+                                                              filter_sizes=[(3, 3), (3, 3), (3, 3)], pool_sizes=[(1, 2)], strides=[(1, 1), (3, 1), (2, 1)]))
+    pt = rf_module_to_pt_module(enc).to("cuda")
+    params = [p for n, p in pt.named_parameters() if "input_layer" in n]
+    T = 120
+    feats = torch.randn(2, T, 80, device="cuda")
+    wgt = torch.randn(2, T // 6 - 2, 1, device="cuda")
     res = []
-    for n in (T, T + 5):
-        lens = torch.full((B,), n, dtype=torch.int32, device=dev)
-        y, dw, db = torch.empty(B, T, F // 2, C, device=dev, dtype=bf), torch.zeros(C, 9, device=dev), torch.zeros(C, device=dev)
-        # the second sequence alone: its frames are the last ones
-        _lib.check(fwd(x[1].data_ptr(), w.data_ptr(), b.data_ptr(), lens.data_ptr(), 1, T, F, C, y.data_ptr(), _lib.stream_ptr()), "fwd")
-        _lib.check(bwd(x[1].data_ptr(), w.data_ptr(), b.data_ptr(), lens.data_ptr(), dy[1].data_ptr(), 1, T, F, C, dw.data_ptr(), db.data_ptr(),
-                       _lib.stream_ptr()), "bwd")
-        res.append((y[:1], dw, db))
-    assert torch.equal(res[0][0], res[1][0])
-    for a, c in zip(res[0][1:], res[1][1:]):
-        torch.testing.assert_close(a, c, atol=1e-4, rtol=1e-4)
+    for n in (T, T + 11):
+        x, pack = conformer_fused._frontend_native(enc, feats, torch.tensor([n, n], dtype=torch.int32))
+        rows = x[: pack.n].view(2, -1, x.shape[1])[:, : T // 6 - 2]
+        grads = torch.autograd.grad((rows.float() * wgt).sum(), params, allow_unused=True)
+        res.append((rows.detach(), [g for g in grads if g is not None]))
+    assert float((res[0][0].float() - res[1][0].float()).norm()) <= 1e-3 * float(res[0][0].float().norm()) and len(res[0][1]) >= 6
+    for a, b in zip(res[0][1], res[1][1]):  # 32-bit sums in another order
+        assert float((a - b).norm()) <= 1e-3 * float(a.norm())
