@@ -435,7 +435,8 @@ att_redrop_kernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict
 // dQv (gradients of the position biases). A CTA owns 64 columns of dqkv, 8 threads to a row, and a slice of the rows; each thread has the
 // loads of two rows in flight. As a copy (15.6 us at 6740 x 1536) and three column-sum kernels (27 us) the gradients were read twice.
 // ATOMIC: the sums are added to; else every slice leaves its own in sum_u / sum_v ([slices][2 * heads * dim], sum_v = sum_u + heads * dim).
-template <bool ATOMIC>
+// WHOLE: dim is a multiple of 64, so the CTA's columns are of one head and one part; else of 8, and a thread's columns are.
+template <bool ATOMIC, bool WHOLE>
 __global__ void __launch_bounds__(256)
 att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16* __restrict__ dqv, const __nv_bfloat16* __restrict__ dk,
                      const __nv_bfloat16* __restrict__ dv, const int* __restrict__ row_batch, const int* __restrict__ row_pos,
@@ -446,13 +447,14 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
   __shared__ float red[32][65];
   const int lane8 = (threadIdx.x & 7) * 8, rl = threadIdx.x >> 3;
   const int hd = heads * dim;
-  const int col0 = blockIdx.y * 64, col = col0 + lane8;  // of dqkv; dim is a multiple of 8: a thread's columns are of one head and one part
-  const int h = col / (3 * dim);
-  const int part = (col - h * 3 * dim) / dim;
+  const int col0 = blockIdx.y * 64, col = col0 + lane8;  // of dqkv
+  const int first = WHOLE ? col0 : col;
+  const int h = first / (3 * dim);
+  const int part = (first - h * 3 * dim) / dim;
   const int src_col = h * dim + (col - (h * 3 + part) * dim);
   const __nv_bfloat16* a_src = (part == 0 ? dqu : part == 1 ? dk : dv) + src_col;
   const __nv_bfloat16* b_src = dqv + src_col;
-  const int r_end = col < 3 * hd ? min(n_rows, (int)(blockIdx.x + 1) * rows_per_cta) : 0;
+  const int r_end = WHOLE || col < 3 * hd ? min(n_rows, (int)(blockIdx.x + 1) * rows_per_cta) : 0;
   float s_x[8], s_u[8], s_v[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) s_x[i] = s_u[i] = s_v[i] = 0.f;
@@ -492,8 +494,8 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
 #pragma unroll
     for (int i = 0; i < 8; ++i) red[rl][lane8 + i] = s[i];
     __syncthreads();
-    const int at = col0 + threadIdx.x, head = at / (3 * dim), in_head = at - head * 3 * dim;
-    if (threadIdx.x < 64 && at < 3 * hd && (!queries || in_head < dim)) {
+    const int at = col0 + threadIdx.x, head = WHOLE ? h : at / (3 * dim), in_head = at - head * 3 * dim;
+    if (threadIdx.x < 64 && (WHOLE || (at < 3 * hd && (!queries || in_head < dim)))) {
       float t = 0.f;
 #pragma unroll
       for (int k = 0; k < 32; ++k) t += red[k][threadIdx.x];
@@ -503,7 +505,7 @@ att_pack_dqkv_kernel(const __nv_bfloat16* __restrict__ dqu, const __nv_bfloat16*
     }
   };
   leave(s_x, sum_qkv, false);
-  if (col0 % (3 * dim) < dim || col0 % (3 * dim) + 63 >= 3 * dim) {  // some of the 64 columns are a query's
+  if (WHOLE ? part == 0 : col0 % (3 * dim) < dim || col0 % (3 * dim) + 63 >= 3 * dim) {  // some of the 64 columns are a query's
     const long long slice = ATOMIC ? 0 : (long long)blockIdx.x * 2 * hd;
     leave(s_u, sum_u ? sum_u + slice : nullptr, true);
     leave(s_v, sum_v ? sum_v + slice : nullptr, true);
@@ -625,7 +627,9 @@ RB_EXPORT int rb200_att_pack_dqkv(const void* dqu, const void* dqv, const void* 
   }
   const int chunks = (3 * heads * dim + 63) / 64, per = pack_rows_per_cta(n_rows, chunks);
   if (!accumulate) sum_v = sum_u ? sum_u + (long long)heads * dim : nullptr;
-  rb_launch_pdl(accumulate ? att_pack_dqkv_kernel<true> : att_pack_dqkv_kernel<false>, dim3((n_rows + per - 1) / per, chunks), dim3(256), 0, stream,
+  auto kernel = dim % 64 ? (accumulate ? att_pack_dqkv_kernel<true, false> : att_pack_dqkv_kernel<false, false>)
+                         : (accumulate ? att_pack_dqkv_kernel<true, true> : att_pack_dqkv_kernel<false, true>);
+  rb_launch_pdl(kernel, dim3((n_rows + per - 1) / per, chunks), dim3(256), 0, stream,
                 (const __nv_bfloat16*)dqu, (const __nv_bfloat16*)dqv, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, row_batch, row_pos,
                 (__nv_bfloat16*)dqkv, accumulate ? sum_qkv : nullptr, sum_u, sum_v, n_rows, heads, dim, lp, per);
   return rb_check_launch("att_pack_dqkv");
