@@ -106,6 +106,12 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
 template <typename S, int NOUT>
 __device__ __forceinline__ void store_partials(float (&acc)[S::MT][NOUT / 8][4], int m_tiles, float* __restrict__ red) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -234,50 +240,66 @@ struct FwdArgs {
   bf16* gates;          // [T,B,4H]
   bf16* hprev_all;      // [T,B,H]
   float *h_final, *c_final;
-  bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state
-  uint32_t* hx;         // wide form: [2,B,H] words (step << 16 | bf16 h), zeroed before the launch
+  bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state (wide form: unused, hprev_all is the exchanged matrix)
   uint32_t* flags;      // one word per CTA (or the counter), zeroed before the launch
   int* abort_word;      // zeroed before the launch
   int* status;          // receives (5 << 24) | cta when a barrier wait ran out
 };
 
-// The forward exchange without barrier, wide form: a word of the exchanged matrix carries the number of the step that wrote it next to the
-// value, so a warp that needs a word loads it until the number is the right one. One trip through L2 per step (store, load) takes the place of
-// store, fence, flag, poll and load, and a warp waits only for the CTAs whose units it multiplies. A word of step s - 1 may be overwritten in
-// step s + 1: whoever writes there has seen all of step s, which everybody wrote after reading step s - 1.
-// Whether all words of the warp's blocks [b_begin, b_end) arrived; a[..] then holds them as bf16 pairs.
+// The exchange of the wide forms has no barrier: the matrix of a step has a place of its own in memory (h_t in hprev_all, dz_t in dz, which the
+// passes leave anyway), the launcher fills it with kUnwritten, and a warp that needs values loads them until none of them is that. One trip
+// through L2 per step (store, load) takes the place of store, fence, flag, poll and load, a warp waits only for the CTAs whose units it
+// multiplies, and only vectors that were not complete are loaded again. kUnwritten is a NaN that no conversion gives (theirs is 0x7fff); a value
+// that has these bits all the same is published as another NaN.
+constexpr uint32_t kUnwritten = 0xffffu;
+
+__device__ __forceinline__ uint32_t publishable(float v) { return min((uint32_t)__bfloat16_as_ushort(__float2bfloat16(v)), kUnwritten - 1); }
+__device__ __forceinline__ void publish_word(bf16* dst, uint32_t w) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(dst), "r"(w) : "memory");
+}
+
+// Wait until all values of the warp's blocks [b_begin, b_end) arrived; a[..] then holds them (zeros for rows and blocks that do not exist).
 template <typename S, int kBlocks>
-__device__ __forceinline__ bool fetch_tagged(const uint32_t* __restrict__ X, int n_rows, int K, int b_begin, int b_end, uint32_t tag,
-                                             uint4 (&a)[kBlocks][S::MT][2], int* abort_word, int* status) {
+__device__ __forceinline__ bool fetch_published(const bf16* __restrict__ A, int n_rows, int K, int b_begin, int b_end, uint4 (&a)[kBlocks][S::MT][2],
+                                                int* abort_word, int* status) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
+  static_assert(kBlocks * S::MT * 2 <= 32, "one bit per vector");
+  uint32_t missing = 0u;
+#pragma unroll
+  for (int i = 0; i < kBlocks; ++i)
+#pragma unroll
+    for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        a[i][m][q] = make_uint4(0u, 0u, 0u, 0u);
+        if (b_begin + i < b_end && m * 16 + q * 8 + g < n_rows) missing |= 1u << ((i * S::MT + m) * 2 + q);
+      }
+  const bf16* src = A + (size_t)g * K + (b_begin << 5) + 8 * t;
   uint32_t spins = 0;
   while (true) {
-    bool ok = true;
 #pragma unroll
-    for (int i = 0; i < kBlocks; ++i) {
+    for (int i = 0; i < kBlocks; ++i)
 #pragma unroll
-      for (int m = 0; m < S::MT; ++m) {
+      for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (missing >> ((i * S::MT + m) * 2 + q) & 1u) {
+            uint4& v = a[i][m][q];
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                         : "l"(src + (size_t)(m * 16 + q * 8) * K + (i << 5)) : "memory");
+          }
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i)
+#pragma unroll
+      for (int m = 0; m < S::MT; ++m)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const int r = m * 16 + q * 8 + g;
-          a[i][m][q] = make_uint4(0u, 0u, 0u, 0u);
-          if (b_begin + i < b_end && r < n_rows) {
-            const uint32_t* src = X + (size_t)r * K + ((b_begin + i) << 5) + 8 * t;
-            uint32_t w[8];
-            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(src) : "memory");
-            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src + 4) : "memory");
-            uint32_t bad = 0u;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) bad |= (w[e] >> 16) ^ tag;
-            ok = ok && bad == 0u;
-            a[i][m][q] = make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410), __byte_perm(w[4], w[5], 0x5410),
-                                    __byte_perm(w[6], w[7], 0x5410));
-          }
+          const uint4& v = a[i][m][q];
+          const uint32_t top = max_u16x2(max_u16x2(v.x, v.y), max_u16x2(v.z, v.w));
+          if ((top >> 16) != kUnwritten && (top & 0xffffu) != kUnwritten) missing &= ~(1u << ((i * S::MT + m) * 2 + q));
         }
-      }
-    }
-    if (__all_sync(0xffffffffu, ok)) return true;
+    if (__all_sync(0xffffffffu, missing == 0u)) return true;
     ++spins;
     if (spins > kSpinLimit || ((spins & 255u) == 0 && *reinterpret_cast<volatile int*>(abort_word))) {
       if (lane == 0) {
@@ -289,9 +311,49 @@ __device__ __forceinline__ bool fetch_tagged(const uint32_t* __restrict__ X, int
   }
 }
 
+// acc += A . Bs^T over the warp's blocks of a published matrix (see step_matmul for the order of k in a block); false: gave up waiting
+template <typename S, int NOUT, int kPrefetch>
+__device__ __forceinline__ bool published_matmul(const bf16* __restrict__ A, int n_rows, int K, const bf16* __restrict__ Bs, float (&acc)[S::MT][NOUT / 8][4],
+                                                 int* abort_word, int* status) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int pitch = K + kPad;
+#pragma unroll
+  for (int m = 0; m < S::MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NOUT / 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  const int m_tiles = (n_rows + 15) / 16;
+  const int nblk = K >> 5;
+  const int b_begin = warp * nblk / S::W, b_end = (warp + 1) * nblk / S::W;
+  for (int bc = b_begin; bc < b_end; bc += kPrefetch) {
+    uint4 a[kPrefetch][S::MT][2];
+    if (!fetch_published<S, kPrefetch>(A, n_rows, K, bc, b_end, a, abort_word, status)) return false;
+#pragma unroll
+    for (int i = 0; i < kPrefetch; ++i) {
+      if (bc + i >= b_end) break;
+      const int k0 = (bc + i) << 5;
+#pragma unroll
+      for (int n = 0; n < NOUT / 8; ++n) {
+        const uint4 w = *reinterpret_cast<const uint4*>(Bs + (size_t)(n * 8 + g) * pitch + k0 + 8 * t);
+#pragma unroll
+        for (int m = 0; m < S::MT; ++m) {
+          if (m >= m_tiles) continue;
+          const uint32_t f0[4] = {a[i][m][0].x, a[i][m][1].x, a[i][m][0].y, a[i][m][1].y};
+          mma16816(acc[m][n], f0, w.x, w.y);
+          const uint32_t f1[4] = {a[i][m][0].z, a[i][m][1].z, a[i][m][0].w, a[i][m][1].w};
+          mma16816(acc[m][n], f1, w.z, w.w);
+        }
+      }
+    }
+  }
+  return true;
+}
+
 template <typename S>
-__device__ __forceinline__ void fwd_body_tagged(const FwdArgs& p, const int cta) {
-  constexpr int U = S::U, kThreads = S::Threads, NOUT = 4 * U, PF = S::PrefetchFwd;
+__device__ __forceinline__ void fwd_body_published(const FwdArgs& p, const int cta) {
+  constexpr int U = S::U, kThreads = S::Threads, NOUT = 4 * U;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int H = p.H, B = p.B;
   const int pitch = H + kPad;
@@ -303,15 +365,16 @@ __device__ __forceinline__ void fwd_body_tagged(const FwdArgs& p, const int cta)
     const int q = r / U, u = r % U;
     *reinterpret_cast<uint4*>(Ws + (size_t)r * pitch + v * 8) = *reinterpret_cast<const uint4*>(p.w_rec + ((size_t)q * H + j0 + u) * H + v * 8);
   }
-  static_assert(S::PerThread == 1, "one (row, unit) pair per thread");
+  static_assert(S::PerThread == 1 && U % 2 == 0, "one (row, unit) pair per thread, the units of a word in neighbouring lanes");
   const int b = threadIdx.x / U, u = threadIdx.x % U;
   const bool own = b < B;
   float cst = 0.f, hst = 0.f;
   bf16 zin[4];
   const int len = own && p.lens ? p.lens[b] : p.T;
-  auto publish = [&](int parity, uint32_t tag, float h) {
-    const uint32_t w = (tag << 16) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16(h));
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p.hx + ((size_t)parity * B + b) * H + j0 + u), "r"(w) : "memory");
+  auto publish = [&](int t, float h) {  // (all lanes of the warp) h, the state before frame t
+    const uint32_t v = publishable(h);
+    const uint32_t next = __shfl_down_sync(0xffffffffu, v, 1);
+    if (own && (u & 1) == 0) publish_word(p.hprev_all + ((size_t)t * B + b) * H + j0 + u, v | next << 16);
   };
   auto fetch_zin = [&](int t) {
     if (!own) return;
@@ -322,68 +385,35 @@ __device__ __forceinline__ void fwd_body_tagged(const FwdArgs& p, const int cta)
   if (own) {
     hst = __bfloat162float(__float2bfloat16(p.h0[(size_t)b * H + j0 + u]));
     cst = p.c0[(size_t)b * H + j0 + u];
-    publish(0, 1u, hst);
   }
-  if (p.T > 0) fetch_zin(p.reverse ? p.T - 1 : 0);
+  if (p.T > 0) {
+    publish(p.reverse ? p.T - 1 : 0, hst);
+    fetch_zin(p.reverse ? p.T - 1 : 0);
+  }
   __syncthreads();  // the resident slice is in place
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t4 = lane & 3;
   const int m_tiles = (B + 15) / 16;
-  const int nblk = H >> 5;
-  const int b_begin = warp * nblk / S::W, b_end = (warp + 1) * nblk / S::W;
   for (int s = 0; s < p.T; ++s) {
-    const int t = p.reverse ? p.T - 1 - s : s;
-    const uint32_t tag = (uint32_t)(s + 1) & 0xffffu;
-    const uint32_t* X = p.hx + (size_t)(s & 1) * B * H;
+    const int t = p.reverse ? p.T - 1 - s : s, t_next = p.reverse ? t - 1 : t + 1;
     float acc[S::MT][NOUT / 8][4];
-#pragma unroll
-    for (int m = 0; m < S::MT; ++m)
-#pragma unroll
-      for (int n = 0; n < NOUT / 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
-    bool ok = true;
-    for (int bc = b_begin; bc < b_end && ok; bc += PF) {
-      uint4 a[PF][S::MT][2];
-      ok = fetch_tagged<S, PF>(X, B, H, bc, b_end, tag, a, p.abort_word, p.status);
-#pragma unroll
-      for (int i = 0; i < PF; ++i) {
-        if (bc + i >= b_end) break;
-        const int k0 = (bc + i) << 5;
-#pragma unroll
-        for (int n = 0; n < NOUT / 8; ++n) {
-          const uint4 w = *reinterpret_cast<const uint4*>(Ws + (size_t)(n * 8 + g) * pitch + k0 + 8 * t4);
-#pragma unroll
-          for (int m = 0; m < S::MT; ++m) {
-            if (m >= m_tiles) continue;
-            const uint32_t f0[4] = {a[i][m][0].x, a[i][m][1].x, a[i][m][0].y, a[i][m][1].y};
-            mma16816(acc[m][n], f0, w.x, w.y);
-            const uint32_t f1[4] = {a[i][m][0].z, a[i][m][1].z, a[i][m][0].w, a[i][m][1].w};
-            mma16816(acc[m][n], f1, w.z, w.w);
-          }
-        }
-      }
-    }
+    const bool ok = published_matmul<S, NOUT, S::PrefetchFwd>(p.hprev_all + (size_t)t * B * H, B, H, Ws, acc, p.abort_word, p.status);
     store_partials<S, NOUT>(acc, m_tiles, red);
     if (!__syncthreads_and(ok ? 1 : 0)) break;
     float gi = 0.f, gf = 0.f, gg = 0.f, go = 0.f;
-    const float hp = hst;
-    if (own) {
-      if (t < len) {
-        gi = sigm(red_sum<S, NOUT>(red, b, u) + __bfloat162float(zin[0]));
-        gf = sigm(red_sum<S, NOUT>(red, b, U + u) + __bfloat162float(zin[1]));
-        gg = tanhf(red_sum<S, NOUT>(red, b, 2 * U + u) + __bfloat162float(zin[2]));
-        go = sigm(red_sum<S, NOUT>(red, b, 3 * U + u) + __bfloat162float(zin[3]));
-        cst = gf * cst + gi * gg;
-        hst = __bfloat162float(__float2bfloat16(go * tanhf(cst)));
-      }
-      publish((s + 1) & 1, (uint32_t)(s + 2) & 0xffffu, hst);
+    if (own && t < len) {
+      gi = sigm(red_sum<S, NOUT>(red, b, u) + __bfloat162float(zin[0]));
+      gf = sigm(red_sum<S, NOUT>(red, b, U + u) + __bfloat162float(zin[1]));
+      gg = tanhf(red_sum<S, NOUT>(red, b, 2 * U + u) + __bfloat162float(zin[2]));
+      go = sigm(red_sum<S, NOUT>(red, b, 3 * U + u) + __bfloat162float(zin[3]));
+      cst = gf * cst + gi * gg;
+      hst = __bfloat162float(__float2bfloat16(go * tanhf(cst)));
     }
-    if (s + 1 < p.T) fetch_zin(p.reverse ? p.T - 2 - s : s + 1);
+    if (s + 1 < p.T) {
+      publish(t_next, hst);
+      fetch_zin(t_next);
+    }
     if (own) {
       const size_t o = ((size_t)t * B + b) * H + j0 + u;
       const size_t zo = ((size_t)t * B + b) * 4 * H + j0 + u;
-      p.hprev_all[o] = __float2bfloat16(hp);
       p.y[o] = __float2bfloat16(t < len ? hst : 0.f);
       p.c_all[o] = cst;
       p.gates[zo] = __float2bfloat16(gi);
@@ -517,8 +547,8 @@ template <typename S>
 __global__ void __launch_bounds__(S::Threads, S::U == 8 ? 2 : 1) lstm_persist_fwd_pair_kernel(const __grid_constant__ FwdPair pp) {
   const int half = gridDim.x / 2;
   if constexpr (S::U == 16) {
-    if ((int)blockIdx.x < half) fwd_body_tagged<S>(pp.d[0], blockIdx.x);
-    else fwd_body_tagged<S>(pp.d[1], blockIdx.x - half);
+    if ((int)blockIdx.x < half) fwd_body_published<S>(pp.d[0], blockIdx.x);
+    else fwd_body_published<S>(pp.d[1], blockIdx.x - half);
   } else {
     if ((int)blockIdx.x < half) fwd_body<S>(pp.d[0], blockIdx.x, half);
     else fwd_body<S>(pp.d[1], blockIdx.x - half, half);
@@ -540,6 +570,19 @@ struct BwdArgs {
   int* status;
 };
 
+// the columns of W_rec that a CTA's units feed: Wt[u][n] = W_rec[n][j0 + u], in 16-byte pieces
+template <typename S>
+__device__ __forceinline__ void load_transposed(const bf16* __restrict__ w_rec, int K, int H, int j0, bf16* __restrict__ Wt) {
+  constexpr int U = S::U;
+  for (int idx = threadIdx.x; idx < K * (U / 8); idx += S::Threads) {
+    const int n = idx / (U / 8), piece = idx % (U / 8);
+    const uint4 v = *reinterpret_cast<const uint4*>(w_rec + (size_t)n * H + j0 + piece * 8);
+    const bf16* e = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) Wt[(size_t)(piece * 8 + i) * (K + kPad) + n] = e[i];
+  }
+}
+
 template <typename S>
 __device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const int n_cta) {
   constexpr int U = S::U, kThreads = S::Threads;
@@ -549,14 +592,7 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const 
   bf16* Wt = reinterpret_cast<bf16*>(smem_raw);                    // [U][4H+kPad]: Wt[u][n] = W_rec[n][j0+u]
   float* red = reinterpret_cast<float*>(Wt + (size_t)U * pitch);   // [slots][rows][U + kRedPad]
   const int j0 = cta * U;
-  for (int idx = threadIdx.x; idx < K * (U / 8); idx += kThreads) {
-    // row n of W_rec, units j0 .. j0 + U - 1, in 16-byte pieces
-    const int n = idx / (U / 8), piece = idx % (U / 8);
-    const uint4 v = *reinterpret_cast<const uint4*>(p.w_rec + (size_t)n * H + j0 + piece * 8);
-    const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) Wt[(size_t)(piece * 8 + i) * pitch + n] = e[i];
-  }
+  load_transposed<S>(p.w_rec, K, H, j0, Wt);
   // a thread's (row, unit) pairs: gradients arriving at h_t and c_t, and what the forward pass kept, fetched one step ahead (DRAM)
   constexpr int N = S::PerThread;
   float dhs[N], dcs[N], c_t[N], c_p[N];
@@ -644,6 +680,78 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& p, const int cta, const 
 
 __global__ void __launch_bounds__(Narrow::Threads, 1) lstm_persist_bwd_kernel(BwdArgs p) { bwd_body<Narrow>(p, blockIdx.x, gridDim.x); }
 
+// wide form: dz itself is the exchanged matrix, see fetch_published
+template <typename S>
+__device__ __forceinline__ void bwd_body_published(const BwdArgs& p, const int cta) {
+  constexpr int U = S::U, kThreads = S::Threads;
+  static_assert(S::PerThread == 1 && U % 2 == 0, "one (row, unit) pair per thread, the units of a word in neighbouring lanes");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int H = p.H, B = p.B, K = 4 * p.H;
+  bf16* Wt = reinterpret_cast<bf16*>(smem_raw);                          // [U][4H+kPad]: Wt[u][n] = W_rec[n][j0+u]
+  float* red = reinterpret_cast<float*>(Wt + (size_t)U * (K + kPad));    // [slots][rows][U + kRedPad]
+  const int j0 = cta * U;
+  load_transposed<S>(p.w_rec, K, H, j0, Wt);
+  const int b = threadIdx.x / U, u = threadIdx.x % U;
+  const bool own = b < B;
+  // gradients arriving at h_t and c_t, and what the forward pass kept, fetched one step ahead (DRAM)
+  float dhs = 0.f, dcs = 0.f, c_t = 0.f, c_p = 0.f;
+  bf16 kept[4], dy = __float2bfloat16(0.f);  // as loaded: a conversion next to the load would wait for it
+  const int len = own && p.lens ? p.lens[b] : p.T;
+  auto fetch = [&](int s) {  // gates, dy and the cell state before step s; (the state after it is that of the step after)
+    if (!own) return;
+    const int t = p.reverse ? p.T - 1 - s : s;
+    const int t_prev = p.reverse ? t + 1 : t - 1;
+    const bf16* gt = p.gates + ((size_t)t * B + b) * K + j0 + u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) kept[q] = gt[(size_t)q * H];
+    if (p.dy) dy = p.dy[((size_t)t * B + b) * H + j0 + u];
+    c_p = s > 0 ? p.c_all[((size_t)t_prev * B + b) * H + j0 + u] : p.c0[(size_t)b * H + j0 + u];
+  };
+  if (own) {
+    if (p.dh_final) dhs = p.dh_final[(size_t)b * H + j0 + u];
+    if (p.dc_final) dcs = p.dc_final[(size_t)b * H + j0 + u];
+    if (p.T > 0) c_t = p.c_all[((size_t)(p.reverse ? 0 : p.T - 1) * B + b) * H + j0 + u];
+  }
+  if (p.T > 0) fetch(p.T - 1);
+  __syncthreads();  // the resident slice is in place
+  const int m_tiles = (B + 15) / 16;
+  for (int s = p.T - 1; s >= 0; --s) {
+    const int t = p.reverse ? p.T - 1 - s : s;
+    bf16* dz_t = p.dz + (size_t)t * B * K;
+    uint32_t ifg = 0u, gog = 0u;  // (i, f) and (g, o) of this unit
+    if (own && t < len) {  // else the state was carried: dh and dc pass through
+      const float dh = dhs + __bfloat162float(dy);
+      const float gi = __bfloat162float(kept[0]), gf = __bfloat162float(kept[1]), gg = __bfloat162float(kept[2]), go = __bfloat162float(kept[3]);
+      const float tc = tanhf(c_t);
+      const float dc = dcs + dh * go * (1.f - tc * tc);
+      ifg = publishable(dc * gg * gi * (1.f - gi)) | publishable(dc * c_p * gf * (1.f - gf)) << 16;
+      gog = publishable(dc * gi * (1.f - gg * gg)) | publishable(dh * tc * go * (1.f - go)) << 16;
+      dcs = dc * gf;
+      dhs = 0.f;
+    }
+    // a word holds two units of one gate: the lane of the even unit stores gates i and f of both, that of the odd one g and o
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, (u & 1) ? ifg : gog, 1);
+    if (own) {
+      bf16* dst = dz_t + (size_t)b * K + j0 + (u & ~1) + ((u & 1) ? 2 * H : 0);
+      const uint32_t lo = (u & 1) ? other : ifg, hi = (u & 1) ? gog : other;
+      publish_word(dst, __byte_perm(lo, hi, 0x5410));
+      publish_word(dst + H, __byte_perm(lo, hi, 0x7632));
+    }
+    c_t = c_p;
+    if (s > 0) fetch(s - 1);
+    float acc[S::MT][U / 8][4];
+    const bool ok = published_matmul<S, U, S::PrefetchBwd>(dz_t, B, K, Wt, acc, p.abort_word, p.status);
+    store_partials<S, U>(acc, m_tiles, red);
+    if (!__syncthreads_and(ok ? 1 : 0)) break;
+    if (own) dhs += red_sum<S, U>(red, b, u);
+    __syncthreads();  // the partial sums have been read
+  }
+  if (own) {
+    p.dh0[(size_t)b * H + j0 + u] = dhs;
+    p.dc0[(size_t)b * H + j0 + u] = dcs;
+  }
+}
+
 struct BwdPair {
   BwdArgs d[2];
 };
@@ -651,8 +759,13 @@ struct BwdPair {
 template <typename S>
 __global__ void __launch_bounds__(S::Threads, S::U == 8 ? 2 : 1) lstm_persist_bwd_pair_kernel(const __grid_constant__ BwdPair pp) {
   const int half = gridDim.x / 2;
-  if ((int)blockIdx.x < half) bwd_body<S>(pp.d[0], blockIdx.x, half);
-  else bwd_body<S>(pp.d[1], blockIdx.x - half, half);
+  if constexpr (S::U == 16) {
+    if ((int)blockIdx.x < half) bwd_body_published<S>(pp.d[0], blockIdx.x);
+    else bwd_body_published<S>(pp.d[1], blockIdx.x - half);
+  } else {
+    if ((int)blockIdx.x < half) bwd_body<S>(pp.d[0], blockIdx.x, half);
+    else bwd_body<S>(pp.d[1], blockIdx.x - half, half);
+  }
 }
 
 // barrier words of the calls in flight: 64 slots of (abort word, flags), handed out round robin
@@ -711,7 +824,7 @@ int rb_lstm_persist_fwd(const void* z_in, const void* w_rec, const int* lens, co
   a.z_in = (const bf16*)z_in; a.w_rec = (const bf16*)w_rec; a.lens = lens; a.h0 = h0; a.c0 = c0;
   a.T = T; a.B = B; a.H = H; a.reverse = reverse;
   a.y = (bf16*)y; a.c_all = c_all; a.gates = (bf16*)gates; a.hprev_all = (bf16*)hprev_all; a.h_final = h_final; a.c_final = c_final;
-  a.hbuf = (bf16*)hbuf; a.hx = nullptr; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
+  a.hbuf = (bf16*)hbuf; a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
   cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   const size_t smem = fwd_smem<Narrow>(H);
   cudaError_t e = cudaFuncSetAttribute(lstm_persist_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -807,7 +920,7 @@ RB_EXPORT int rb200_blstm_supported(int T, int B, int H) { return pair_shape(T, 
 
 // ptrs[d * 11 + i] for direction d (0: forward in time, 1: reversed):
 //   0 z_in [T,B,4H] bf16, 1 w_rec [4H,H] bf16, 2 h0, 3 c0 [B,H] fp32, 4 y [T,B,H] bf16, 5 c_all [T,B,H] fp32, 6 gates [T,B,4H] bf16,
-//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 exchange buffer (scratch, 2*B*H 32-bit words)
+//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 exchange buffer (scratch, 2*B*H bf16)
 RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, int H, int* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return RB_OK;
   const int shape = pair_shape(T, B, H);
@@ -827,8 +940,8 @@ RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, 
     a.z_in = (const bf16*)q[0]; a.w_rec = (const bf16*)q[1]; a.lens = lens; a.h0 = (const float*)q[2]; a.c0 = (const float*)q[3];
     a.T = T; a.B = B; a.H = H; a.reverse = d;
     a.y = (bf16*)q[4]; a.c_all = (float*)q[5]; a.gates = (bf16*)q[6]; a.hprev_all = (bf16*)q[7]; a.h_final = (float*)q[8]; a.c_final = (float*)q[9];
-    a.hbuf = (bf16*)q[10]; a.hx = (uint32_t*)q[10];
-    if (shape != kNarrow) cudaMemsetAsync(a.hx, 0, (size_t)2 * B * H * sizeof(uint32_t), stream);
+    a.hbuf = (bf16*)q[10];
+    if (shape != kNarrow) cudaMemsetAsync(a.hprev_all, 0xff, (size_t)T * B * H * sizeof(bf16), stream);  // kUnwritten
     a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
     cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   }
@@ -864,6 +977,7 @@ RB_EXPORT int rb200_blstm_bwd(void* const* ptrs, const int* lens, int T, int B, 
     a.dy = (const bf16*)q[0]; a.dh_final = (const float*)q[1]; a.dc_final = (const float*)q[2]; a.w_rec = (const bf16*)q[3]; a.lens = lens;
     a.gates = (const bf16*)q[4]; a.c_all = (const float*)q[5]; a.c0 = (const float*)q[6]; a.T = T; a.B = B; a.H = H; a.reverse = d;
     a.dz = (bf16*)q[8]; a.dh0 = (float*)q[10]; a.dc0 = (float*)q[11];
+    if (shape != kNarrow) cudaMemsetAsync(a.dz, 0xff, (size_t)T * B * 4 * H * sizeof(bf16), stream);  // kUnwritten
     a.flags = sync_words + 32; a.abort_word = reinterpret_cast<int*>(sync_words); a.status = status;
     cudaMemsetAsync(sync_words, 0, kSyncWords * sizeof(unsigned int), stream);
   }

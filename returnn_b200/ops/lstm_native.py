@@ -139,7 +139,7 @@ class _BlstmRecFn(torch.autograd.Function):
             hprev = torch.empty(T, B, H, dtype=bf, device=dev)
             h_fin = torch.empty(B, H, dtype=torch.float32, device=dev)
             c_fin = torch.empty(B, H, dtype=torch.float32, device=dev)
-            hbuf = torch.empty(2, B, H, dtype=torch.int32, device=dev)
+            hbuf = torch.empty(2, B, H, dtype=bf, device=dev)
             h0f, c0f = h0.float().contiguous(), c0.float().contiguous()
             for i, t in enumerate((z16, w16, h0f, c0f, y, c_all, gates, hprev, h_fin, c_fin, hbuf)):
                 ptrs[d * 11 + i] = t.data_ptr()
