@@ -40,8 +40,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// Orders execution only: what the CTAs share goes through mbarriers (their initialisation through fence.mbarrier_init). With .release the arrival
+// waits for all stores before it, 0.7 us at the end of every product.
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // address of the same shared-memory offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
@@ -49,8 +51,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+// Relaxed: what is handed over is tensor memory, which tcgen05.wait::ld and tcgen05.fence order; .release took 1100 cycles per tile and warp.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster_addr) {
   asm volatile(
@@ -73,7 +76,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-template <bool FULL>
+template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
                  const __grid_constant__ CUtensorMap tm_c2, const Params p) {
@@ -105,6 +108,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       mbar_init(&acc_empty[i], 2 * kEpilogueWarps);  // leader: the epilogue warps of both CTAs
     }
     *abort_flag = 0;
+    prefetch_map(&tm_a);
+    prefetch_map(&tm_b);
+    if (p.tma_store) prefetch_map(&tm_c);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -210,7 +216,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // ---------------- epilogue: this CTA's 128 rows ----------------
     const int q = warp & 3;
     uint8_t* box = reinterpret_cast<uint8_t*>(staging) + (warp - 2) * kStoreBoxBytesPerWarp;
-    float* stg = reinterpret_cast<float*>(box);
+    const EpiRng rng = EpiRng::load<KIND>(g);
     uint32_t t_local = 0;
     for (int u = pair; u < p.units; u += n_pairs) {
       const Unit w = decode_unit<BM, BN>(p, u);
@@ -221,7 +227,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       // the epilogue's global input of this lane's row (first 16 columns) is requested before the wait: it arrives while the tile is
       // still multiplied
       uint4 in_a = make_uint4(0u, 0u, 0u, 0u), in_b = in_a;
-      const bool prefetched = FULL && p.tma_store && (g.dact_z != nullptr || g.resid != nullptr);
+      const bool prefetched = epi_has_input(KIND) || (KIND == kEpiAny && p.tma_store && (g.dact_z != nullptr || g.resid != nullptr));
       if (prefetched) epilogue_prefetch16(p, w.M, w.N, m0 + q * 32 + lane, n0 + part * (BN / 4), in_a, in_b);
       bool ok = mbar_wait(&acc_full[buf], (t_local >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) {
@@ -232,9 +238,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-      auto release = [&]() { mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0)); };
-      if (p.tma_store) epilogue_rows_tma<FULL>(p, w, m0, n0, t_addr, part * (BN / 4), box, &tm_c, &tm_c2, lane, q, release, in_a, in_b, prefetched);
-      else epilogue_columns<FULL>(p, w, m0, n0, t_addr, part * (BN / 4), (part + 1) * (BN / 4), stg, lane, q, release);
+      // (nobody waits for the buffers of the last two units: no arrival is on its way to the leader when the CTAs end)
+      const bool reused = u + 2 * n_pairs < p.units;
+      auto release = [&]() {
+        if (reused) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
+      };
+      if constexpr (!epi_generic(KIND))
+        epilogue_kind_tma<KIND>(p, w, m0, n0, t_addr, part * (BN / 4), box, &tm_c, &tm_c2, lane, q, release, in_a, in_b, rng);
+      else if (p.tma_store)
+        epilogue_rows_tma<KIND == kEpiAny>(p, w, m0, n0, t_addr, part * (BN / 4), box, &tm_c, &tm_c2, lane, q, release, in_a, in_b, prefetched);
+      else
+        epilogue_columns<KIND == kEpiAny>(p, w, m0, n0, t_addr, part * (BN / 4), (part + 1) * (BN / 4), reinterpret_cast<float*>(box), lane, q, release);
       ++t_local;
     }
     // the bulk stores read this CTA's shared memory: the reads must have finished before the CTA exits and its shared memory is
@@ -303,13 +317,18 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
     rb_set_error("gemm (pair): this problem's epilogue leaves no column sums");
     return RB_ERR_ARG;
   }
+  using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const Params);
+  static const Kernel kernels[] = {gemm_pair_kernel<kEpiSome>,  gemm_pair_kernel<kEpiAny>,       gemm_pair_kernel<kEpiPlain>, gemm_pair_kernel<kEpiF32>,
+                                   gemm_pair_kernel<kEpiTwo>,   gemm_pair_kernel<kEpiTwoDrop>,   gemm_pair_kernel<kEpiResid>, gemm_pair_kernel<kEpiResidDrop>,
+                                   gemm_pair_kernel<kEpiDact>,  gemm_pair_kernel<kEpiDactDrop>};
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) {
-      rb_set_error("gemm (pair): cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-      return RB_ERR_LAUNCH;
+    for (const Kernel k : kernels) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+      if (e != cudaSuccess) {
+        rb_set_error("gemm (pair): cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+        return RB_ERR_LAUNCH;
+      }
     }
     attr_set = true;
   }
@@ -334,19 +353,21 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   p.units = tiles * p.split;
   p.vec_ok = aligned_outputs(g);
   p.bias_vec = g.bias != nullptr && !g.bias_bf16 && (reinterpret_cast<uintptr_t>(g.bias) & 15) == 0;
-  const bool full = full_epilogue(g);
   // bulk tensor stores need what a tensor map needs: 16-byte aligned base, row pitch a multiple of 16 bytes
   p.tma_store = tma_store_on() && p.vec_ok && g.c != nullptr && (g.out_fp32 ? true : (g.ldc % 8 == 0));
+  const int kind = epilogue_kind(p);
   CUtensorMap tm_a, tm_b, tm_c, tm_c2;
   memset(&tm_c, 0, sizeof(tm_c));
   memset(&tm_c2, 0, sizeof(tm_c2));
   int st;
   if (p.tma_store) {
-    // boxes of 32 rows x 128 bytes: 64 bf16 or 32 fp32 columns; with a second output, 32 rows x 64 bytes (32 bf16 columns) each
+    // boxes of 32 rows x 128 bytes: 64 bf16 or 32 fp32 columns; with a second output, and in the fp32 form, 32 rows x 64 bytes each
     if (g.c2) {
       st = make_map(&tm_c, g.c, g.n, g.m, g.ldc, 32, 32, false, true);
       if (st) return st;
       st = make_map(&tm_c2, g.c2, g.n, g.m, g.ldc, 32, 32, false, true);
+    } else if (kind == kEpiF32) {
+      st = make_map(&tm_c, g.c, g.n, g.m, g.ldc, 16, 32, true, true);
     } else {
       st = make_map(&tm_c, g.c, g.n, g.m, g.ldc, g.out_fp32 ? 32 : 64, 32, g.out_fp32 != 0);
     }
@@ -359,7 +380,6 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   st = g.b_mn_major ? make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, 64, BK) : make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, BK, BN / 2);
   if (st) return st;
   int pairs = p.units < pairs_max ? p.units : pairs_max;
-  if (full) rb_launch_pdl(gemm_pair_kernel<true>, dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, tm_c2, p);
-  else rb_launch_pdl(gemm_pair_kernel<false>, dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, tm_c2, p);
+  rb_launch_pdl(kernels[kind], dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, tm_c2, p);
   return rb_check_launch("gemm_pair");
 }

@@ -401,6 +401,20 @@ __device__ __forceinline__ uint4 pack8_bf16(const float* v) {
   return u;
 }
 
+// Column sums of a box of 64 bf16 columns as it was rounded, added onto `sum`: a lane reads two columns down its rows (the 32 lanes cover a row's 128
+// bytes: no bank conflicts) while the bulk store reads the same memory. As a kernel of its own that read the output again: 14.7 us at 6740 x 2048.
+__device__ __forceinline__ void epilogue_column_sums(const uint8_t* box, int n_rows, int col, int n, float* sum, int lane) {
+  float s0 = 0.f, s1 = 0.f;
+  const uint8_t* at = box + (lane & 3) * 4;
+  for (int i = 0; i < n_rows; ++i) {
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(at + i * 128 + (((lane >> 2) ^ (i & 7)) << 4));
+    s0 += __uint_as_float(u << 16);
+    s1 += __uint_as_float(u & 0xffff0000u);
+  }
+  if (col < n) atomicAdd(sum + col, s0);
+  if (col + 1 < n) atomicAdd(sum + col + 1, s1);
+}
+
 // One warp's share of a tile: rows m0 + q*32 .. +31 (lane = row), accumulator columns [c_begin, c_begin + 64) at TMEM address
 // t_addr (lane quarter already applied). box: this warp's 4 KB of shared memory, 1024-byte aligned. tm_c / tm_c2: tensor maps of the
 // outputs with boxes of 32 rows x 128 bytes (64 bf16 or 32 fp32 columns; with a second output c2: 32 rows x 64 bytes, 64-byte swizzle). `arrive` hands the accumulator buffer back (lane 0).
@@ -483,22 +497,171 @@ __device__ __forceinline__ void epilogue_rows_tma(const Params& p, const Unit& w
         }
         tma_store_commit();
       }
-      if (FULL && g.colsum && ph == 3) {
-        // Column sums of the box as it was rounded: a lane reads two columns down its rows (the 32 lanes cover a row's 128 bytes: no bank
-        // conflicts) while the bulk store reads the same memory. As a kernel of its own that read the output again: 14.7 us at 6740 x 2048.
-        float s0 = 0.f, s1 = 0.f;
-        const int n_rows = min(32, w.M - row0);
-        const uint8_t* at = box + (lane & 3) * 4;
-        for (int i = 0; i < n_rows; ++i) {
-          const uint32_t u = *reinterpret_cast<const uint32_t*>(at + i * 128 + (((lane >> 2) ^ (i & 7)) << 4));
-          s0 += __uint_as_float(u << 16);
-          s1 += __uint_as_float(u & 0xffff0000u);
-        }
-        const int col = col0 + 2 * lane;
-        if (col < w.N) atomicAdd(g.colsum + col, s0);
-        if (col + 1 < w.N) atomicAdd(g.colsum + col + 1, s1);
+      if (FULL && g.colsum && ph == 3) epilogue_column_sums(box, min(32, w.M - row0), col0 + 2 * lane, w.N, g.colsum, lane);
+    }
+  }
+}
+
+// ---- the epilogues that the layers use, each in a form of its own -------------------------------------------------------------------
+// epilogue_rows_tma asks in every group of 8 columns what there is to do, and the 16 warps of a CTA issue all of that: 600 to 840 cycles per
+// phase of 16 columns where the plain form needs about 250 (6912 x 512 x 512: 2.9 us between the last product of a tile and its last store, now
+// 1.2). KIND is chosen by the launcher (epilogue_kind); whatever has no form of its own takes epilogue_rows_tma or epilogue_columns.
+// All: output through bulk tensor stores, n a multiple of 8, fp32 bias on a 16-byte boundary or none.
+enum EpiKind {
+  kEpiSome,      // without activation gradient, dropout, residual: any of the rest
+  kEpiAny,       // anything
+  kEpiPlain,     // bf16: [bias], [activation]
+  kEpiF32,       // fp32, stored or added
+  kEpiTwo,       // pre-activation and activation
+  kEpiTwoDrop,   // ... with dropout on the second
+  kEpiResid,     // residual + res_scale * (value [+ bias])
+  kEpiResidDrop, // ... with dropout on the value
+  kEpiDact,      // value * act'(z), column sums where wanted
+  kEpiDactDrop   // ... with dropout
+};
+constexpr bool epi_generic(int kind) { return kind == kEpiSome || kind == kEpiAny; }
+constexpr bool epi_drops(int kind) { return kind == kEpiTwoDrop || kind == kEpiResidDrop || kind == kEpiDactDrop; }
+constexpr bool epi_has_input(int kind) { return kind == kEpiResid || kind == kEpiResidDrop || kind == kEpiDact || kind == kEpiDactDrop; }
+
+inline int epilogue_kind(const Params& p) {
+  const RbGemm& g = p.g;
+  const bool full = g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr;
+  const int generic = full ? kEpiAny : kEpiSome;
+  if (!p.tma_store || g.n % 8 || (g.bias && !p.bias_vec)) return generic;
+  const bool drop = g.drop_p > 0.f;
+  if (g.out_fp32) return full || g.bias || g.act || g.c2 ? generic : kEpiF32;
+  if (g.dact_z) return g.resid || g.bias || g.c2 ? generic : drop ? kEpiDactDrop : kEpiDact;
+  if (g.resid) return g.act || g.c2 ? generic : drop ? kEpiResidDrop : kEpiResid;
+  if (g.c2) return drop ? kEpiTwoDrop : kEpiTwo;
+  return drop ? generic : kEpiPlain;
+}
+
+// the generator's key and first counter of a product, read once per warp
+struct EpiRng {
+  uint2 key;
+  uint64_t base;
+  uint32_t thresh;
+  float scale;
+  template <int KIND>
+  __device__ __forceinline__ static EpiRng load(const RbGemm& g) {
+    EpiRng r = {};
+    if constexpr (epi_drops(KIND)) {
+      const uint64_t sd = (uint64_t)g.seed[0];
+      r.key = make_uint2((uint32_t)sd, (uint32_t)(sd >> 32));
+      r.base = (uint64_t)g.offset[0] + g.drop_site;
+      r.thresh = rb_dropout_thresh16(g.drop_p);
+      r.scale = 1.f / (1.f - g.drop_p);
+    }
+    return r;
+  }
+};
+
+// Arguments as epilogue_rows_tma. fp32 outputs leave in boxes of 32 rows x 16 columns, two of them in turn in the warp's 4 KB: a bulk add
+// takes about 2000 cycles to read its box, and with one box of 32 columns the second half of a tile waited for that.
+template <int KIND, typename Arrive>
+__device__ __forceinline__ void epilogue_kind_tma(const Params& p, const Unit& w, int m0, int n0, uint32_t t_addr, int c_begin, uint8_t* box,
+                                                  const CUtensorMap* tm_c, const CUtensorMap* tm_c2, int lane, int q, Arrive arrive, uint4 in_a, uint4 in_b,
+                                                  const EpiRng& rng) {
+  constexpr bool F32 = KIND == kEpiF32, TWO = KIND == kEpiTwo || KIND == kEpiTwoDrop, DROP = epi_drops(KIND), INPUT = epi_has_input(KIND);
+  constexpr bool DACT = KIND == kEpiDact || KIND == kEpiDactDrop, RESID = INPUT && !DACT;
+  const RbGemm& g = p.g;
+  const int row0 = m0 + q * 32;
+  const int row = row0 + lane;
+  const int col0 = n0 + c_begin;
+  auto release = [&]() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) arrive();
+  };
+  if (row0 >= w.M || col0 >= w.N) {  // nothing of this warp's box lies inside the matrix (warp-uniform): nothing to read
+    release();
+    return;
+  }
+  const int sw = lane & 7, sw64 = (lane >> 1) & 3;
+  const float alpha = g.alpha;
+  const float* bias = F32 || DACT ? nullptr : reinterpret_cast<const float*>(g.bias);
+#pragma unroll 1
+  for (int ph = 0; ph < 4; ++ph) {
+    const int col = col0 + 16 * ph;
+    uint32_t r[16];
+    tmem_ld16(t_addr + (uint32_t)(c_begin + 16 * ph), r);
+    uint4 nx_a = make_uint4(0u, 0u, 0u, 0u), nx_b = nx_a;
+    if (INPUT && ph < 3) epilogue_prefetch16(p, w.M, w.N, row, col + 16, nx_a, nx_b);
+    float4 b[4];
+    if (bias) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) b[i] = col + 8 * (i >> 1) < w.N ? __ldg(reinterpret_cast<const float4*>(bias + col) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (ph == 3) release();
+    if (F32 || ph == 0 || (TWO && ph == 2)) {  // the box was handed to the TMA unit before: it must have been read
+      if (lane == 0) {
+        if (F32) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        else tma_store_wait_read();
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int gi = 0; gi < 2; ++gi) {
+      float v[8], pre[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * gi + i]) * alpha;
+      if (bias) {
+        const float4 b0 = b[2 * gi], b1 = b[2 * gi + 1];
+        v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+        v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+      }
+      if constexpr (TWO) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) pre[i] = v[i];
+      }
+      if constexpr (DACT) {
+        float z[8];
+        unpack8_bf16(gi == 0 ? in_a : in_b, z);
+        act_grad8(v, z, g.act);
+      } else if constexpr (TWO || KIND == kEpiPlain) {
+        if (g.act) act8(v, g.act);
+      }
+      if constexpr (DROP) rb_dropout_apply8(rng.key, rng.base + (uint64_t)((size_t)row * g.ldc + col + 8 * gi), rng.thresh, rng.scale, v);
+      if constexpr (RESID) {
+        float rs[8];
+        unpack8_bf16(gi == 0 ? in_a : in_b, rs);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = rs[i] + g.res_scale * v[i];
+      }
+      if constexpr (F32) {
+        uint8_t* at = box + (ph & 1) * 2048 + lane * 64;
+        *reinterpret_cast<float4*>(at + (((2 * gi) ^ sw64) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(at + (((2 * gi + 1) ^ sw64) << 4)) = make_float4(v[4], v[5], v[6], v[7]);
+      } else if constexpr (TWO) {
+        uint8_t* at = box + lane * 64 + (((2 * (ph & 1) + gi) ^ sw64) << 4);
+        *reinterpret_cast<uint4*>(at) = pack8_bf16(pre);
+        *reinterpret_cast<uint4*>(at + 2048) = pack8_bf16(v);
+      } else {
+        *reinterpret_cast<uint4*>(box + lane * 128 + (((2 * ph + gi) ^ sw) << 4)) = pack8_bf16(v);
       }
     }
+    if constexpr (INPUT) {
+      in_a = nx_a;
+      in_b = nx_b;
+    }
+    if (F32 || ph == 3 || (TWO && ph == 1)) {
+      const int cbox = F32 ? col : TWO ? col0 + 32 * (ph >> 1) : col0;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (cbox < w.N) {
+          const uint8_t* from = F32 ? box + (ph & 1) * 2048 : box;
+          if (F32 && g.accumulate) tma_reduce_add_2d(tm_c, cbox, row0, from);
+          else tma_store_2d(tm_c, cbox, row0, from);
+          if (TWO) tma_store_2d(tm_c2, cbox, row0, box + 2048);
+        }
+        tma_store_commit();
+      }
+    }
+  }
+  if constexpr (DACT) {
+    if (g.colsum) epilogue_column_sums(box, min(32, w.M - row0), col0 + 2 * lane, w.N, g.colsum, lane);
   }
 }
 
