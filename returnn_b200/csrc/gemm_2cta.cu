@@ -76,6 +76,37 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
+// The units of a pair, one after another: (slice of the contraction, row of tiles, column of tiles), with one division at the start. Divisions per
+// unit left the producer 500 cycles late at every tile.
+struct Walk {
+  const Params& p;
+  int u, sp, mi, ni;
+  __device__ __forceinline__ Walk(const Params& p_, int first) : p(p_), u(first) {
+    const int tiles = p.tiles_m * p.tiles_n;
+    sp = p.split > 1 ? u / tiles : 0;
+    const int t = u - sp * tiles;
+    mi = t / p.tiles_n;
+    ni = t - mi * p.tiles_n;
+  }
+  __device__ __forceinline__ bool more() const { return u < p.units; }
+  __device__ __forceinline__ void next() {
+    u += p.step;
+    sp += p.step_sp;
+    mi += p.step_m;
+    ni += p.step_n;
+    if (ni >= p.tiles_n) {
+      ni -= p.tiles_n;
+      ++mi;
+    }
+    if (mi >= p.tiles_m) {
+      mi -= p.tiles_m;
+      ++sp;
+    }
+  }
+  __device__ __forceinline__ int kb0() const { return sp * p.kb_per_split; }
+  __device__ __forceinline__ int kb1() const { return min(p.num_kb, (sp + 1) * p.kb_per_split); }
+};
+
 template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
@@ -96,7 +127,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
-  const int n_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -122,23 +152,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   cluster_sync();  // barriers of both CTAs are initialised before anyone signals across
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  // everything above touched no global memory: it may overlap the tail of the preceding kernel
-  rb_pdl_wait();
+  // everything above touched no global memory: it may overlap the tail of the preceding kernel. The roles wait for that one themselves, with their
+  // first unit at hand.
   rb_pdl_launch();
 
   if (warp == 0) {
     if (lane == 0) {
       // ---------------- TMA producer (both CTAs) ----------------
-      uint32_t it = 0;
+      const uint32_t full0 = map_to_cta(smem_u32(full_bar), 0);  // the leader's barriers collect both CTAs' bytes
+      uint32_t s = 0, ph = 0;
       bool ok = true;
-      for (int u = pair; u < p.units && ok; u += n_pairs) {
-        const Unit w = decode_unit<BM, BN>(p, u);
-        if (!w.valid) continue;
-        const int m0 = w.m0 + (int)rank * 128;
-        const int n0 = w.n0 + (int)rank * (BN / 2);
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
+      Walk w(p, pair);
+      rb_pdl_wait();
+      for (; w.more() && ok; w.next()) {
+        const int m0 = w.mi * BM + (int)rank * 128;
+        const int n0 = w.ni * BN + (int)rank * (BN / 2);
+        const int kb1 = w.kb1();
+        for (int kb = w.kb0(); kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag)) {
             *abort_flag = 1;
             if (g.status) atomicCAS(g.status, 0, (1 << 24) | (kb & 0xFFFFFF));
@@ -147,7 +177,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
           uint8_t* sa = smem + s * kStageBytes;
           uint8_t* sb = sa + kTileBytesA;
-          const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);  // the leader's barrier collects both CTAs' bytes
+          const uint32_t bar = full0 + s * 8;
           if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
           // split operands: block kb belongs to hi*lo, lo*hi or hi*hi (columns of A past k read zeros, so the rows of B there do not
           // count). The small products come first: additions to a large accumulator are what the tensor core rounds
@@ -166,6 +196,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tm_b, n0 + 64 * j, b_row + k0, bar);
           }
+          if (++s == kStages) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
     }
@@ -175,22 +209,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const uint32_t ab_fmt = g.ab_fp16 ? 0u : 1u;  // operand format field: 0 = fp16, 1 = bf16 (accumulator fp32 either way)
       const uint32_t idesc = (1u << 4) | (ab_fmt << 7) | (ab_fmt << 10) | ((uint32_t)(g.a_mn_major ? 1 : 0) << 15) |
                              ((uint32_t)(g.b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      uint32_t it = 0, t_local = 0;
+      uint32_t s = 0, ph = 0, t_local = 0;
       bool ok = true;
-      for (int u = pair; u < p.units && ok; u += n_pairs) {
-        const Unit w = decode_unit<BM, BN>(p, u);
-        if (!w.valid) continue;
+      for (Walk w(p, pair); w.more() && ok; w.next()) {
         const uint32_t buf = t_local & 1u;
         if (!mbar_wait(&acc_empty[buf], ((t_local >> 1) & 1u) ^ 1u, abort_flag)) {
           *abort_flag = 1;
-          if (g.status) atomicCAS(g.status, 0, (4 << 24) | (u & 0xFFFFFF));
+          if (g.status) atomicCAS(g.status, 0, (4 << 24) | (w.u & 0xFFFFFF));
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
+        const int kb0 = w.kb0(), kb1 = w.kb1();
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[s], ph, abort_flag)) {
             *abort_flag = 1;
             if (g.status) atomicCAS(g.status, 0, (2 << 24) | (kb & 0xFFFFFF));
@@ -204,9 +235,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           for (int kk = 0; kk < BK / 16; ++kk) {
             const uint64_t adesc = g.a_mn_major ? make_desc(sa + kk * 2048, 8192, 1024) : make_desc(sa + kk * 32, 16, 1024);
             const uint64_t bdesc = g.b_mn_major ? make_desc(sb + kk * 2048, 8192, 1024) : make_desc(sb + kk * 32, 16, 1024);
-            umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb > w.kb0 || kk > 0) ? 1u : 0u);
+            umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty_bar[s]);
+          if (++s == kStages) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
         if (ok) umma_commit_pair(&acc_full[buf]);
         ++t_local;
@@ -216,11 +251,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // ---------------- epilogue: this CTA's 128 rows ----------------
     const int q = warp & 3;
     uint8_t* box = reinterpret_cast<uint8_t*>(staging) + (warp - 2) * kStoreBoxBytesPerWarp;
-    const EpiRng rng = EpiRng::load<KIND>(g);
     uint32_t t_local = 0;
-    for (int u = pair; u < p.units; u += n_pairs) {
-      const Unit w = decode_unit<BM, BN>(p, u);
-      if (!w.valid) continue;
+    Walk walk(p, pair);
+    Unit w = {};
+    w.M = g.m;
+    w.N = g.n;
+    rb_pdl_wait();
+    const EpiRng rng = EpiRng::load<KIND>(g);
+    for (; walk.more(); walk.next()) {
+      w.m0 = walk.mi * BM;
+      w.n0 = walk.ni * BN;
       const int m0 = w.m0 + (int)rank * 128, n0 = w.n0;
       const uint32_t buf = t_local & 1u;
       const int part = (warp - 2) >> 2;  // four warps per lane quarter, each with a quarter of the columns
@@ -232,14 +272,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       bool ok = mbar_wait(&acc_full[buf], (t_local >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) {
         *abort_flag = 1;
-        if (g.status) atomicCAS(g.status, 0, (3 << 24) | (u & 0xFFFFFF));
+        if (g.status) atomicCAS(g.status, 0, (3 << 24) | (walk.u & 0xFFFFFF));
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
       // (nobody waits for the buffers of the last two units: no arrival is on its way to the leader when the CTAs end)
-      const bool reused = u + 2 * n_pairs < p.units;
+      const bool reused = walk.u + 2 * p.step < p.units;
       auto release = [&]() {
         if (reused) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
       };
@@ -379,7 +419,11 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   if (st) return st;
   st = g.b_mn_major ? make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, 64, BK) : make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, BK, BN / 2);
   if (st) return st;
-  int pairs = p.units < pairs_max ? p.units : pairs_max;
+  const int pairs = p.units < pairs_max ? p.units : pairs_max;
+  p.step = pairs;
+  p.step_sp = pairs / tiles;
+  p.step_m = pairs % tiles / p.tiles_n;
+  p.step_n = pairs % tiles % p.tiles_n;
   rb_launch_pdl(kernels[kind], dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, tm_c2, p);
   return rb_check_launch("gemm_pair");
 }

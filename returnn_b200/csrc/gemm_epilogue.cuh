@@ -15,6 +15,7 @@ struct Params {
   int vec_ok;    // all epilogue pointers 16-byte aligned and ldc % 8 == 0
   int bias_vec;  // fp32 bias, 16-byte aligned: read as two float4
   int tma_store; // the output leaves through shared memory and bulk tensor stores (tensor maps of c / c2 passed to the kernel)
+  int step, step_sp, step_m, step_n;  // CTA-pair kernel: from a pair's unit to its next, and the same in slices, rows and columns of tiles
   int seg_kb;    // CTA-pair kernel: K blocks per product of split operands (0: not split)
 };
 
