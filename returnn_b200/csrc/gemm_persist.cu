@@ -18,6 +18,7 @@
 // Every mbarrier wait is bounded. A wait that gives up raises the CTA's abort flag and writes a status word; all roles
 // leave their loops, the CTA waits for its TMA copies in flight, frees its tensor memory and returns.
 #include "gemm_epilogue.cuh"
+#include <algorithm>
 #include <cstring>
 #include <cstdlib>
 
@@ -402,6 +403,19 @@ RB_EXPORT int rb200_gemm_fp16_split(const void* a, const void* b, void* c, int m
 }
 
 RB_EXPORT int rb200_sum_slices_f32(const float* x, float* y, int slices, long long n, cudaStream_t stream);
+
+// Rows of x and dy per slice of a weight gradient x^T dy that is the same in every run (rb200_weight_grad_sliced); 0: one product. Where the result
+// has few tiles and the contraction is long, it is cut into slices whose products are added in their order.
+// One CTA per tile of 128 x 256 and slice, all of them at once; at least 256 rows per slice (shorter ones gain less than the sum of the
+// slices costs); no more than 12, from where the slices that are written and read again cost more than shorter products save.
+// 6656 x 512 x 512: 12 slices 16 us, one 42; 25000 x 512 x 512: 26 and 138; 6656 x 512 x 2048: 4 slices 24 us, one 43 (slices that add
+// onto one result by atomics, in any order: 13, 19 and 21 us); 600 x 512 x 512: 2 slices 12.5, one 11.2
+RB_EXPORT int rb200_weight_grad_slices(int m, int k, int n) {
+  const long long tiles = (long long)((k + 127) / 128) * ((n + 255) / 256);
+  if (m <= 0 || tiles <= 0) return 0;
+  const int slices = (int)std::min<long long>({148 / tiles, 12, m / 256});
+  return slices <= 1 ? 0 : ((m + slices - 1) / slices + 63) / 64 * 64;  // (rows past the last one are read as zeros)
+}
 
 // dw [k][n] (fp32) = x^T dy, x [m][k], dy [m][n] bf16: one product per slice of `rows` rows into part [ceil(m / rows)][k][n], then their sum in
 // the order of the slices

@@ -106,7 +106,9 @@ def count_launch(n: int = 1):
 
 def launch_count() -> int:
     """number of native kernel launches so far"""
-    return _launch_count
+    from . import nodes
+
+    return _launch_count + nodes.launches()
 
 
 def check(status: int, what: str):

@@ -3,6 +3,7 @@ Build the native libraries in-tree:
 
 - ``_build/librb200.so``: all CUDA kernels, compiled for sm_100a only
   (``nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo``); nvcc cross-compiles without a GPU.
+- ``_build/_autograd_nodes.so``: autograd nodes in C++ that launch them (g++, against the installed torch).
 - ``_build/librb200_host.so`` and ``_build/librb200_atfork.so``: host-only helpers (g++).
 
 ``python -m returnn_b200.ops.build [--force] [--verbose]``. Sources are compiled in parallel; objects are cached by
@@ -76,7 +77,7 @@ def build_cuda(force: bool = False, verbose: bool = False, ptxas_info: bool = Fa
                 print(o)
     lib = os.path.join(_BUILD, "librb200.so")
     if jobs or force or _newer(lib, objs):
-        _run([nvcc, "-shared", "-o", lib] + objs, verbose)
+        _run([nvcc, "-shared", "-Xlinker", "-soname=librb200.so", "-o", lib] + objs, verbose)
     return lib
 
 
@@ -105,6 +106,9 @@ def build_host(force: bool = False, verbose: bool = False) -> List[str]:
             if force or _newer(lib, [pyext]):
                 _run([gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", inc, "-o", lib, pyext], verbose)
             res.append(lib)
+    nodes = build_nodes(force=force, verbose=verbose)
+    if nodes:
+        res.append(nodes)
     atfork = os.path.join(host_dir, "atfork_patch.cpp")
     if os.path.exists(atfork):
         lib = os.path.join(_BUILD, "librb200_atfork.so")
@@ -112,6 +116,30 @@ def build_host(force: bool = False, verbose: bool = False) -> List[str]:
             _run([gxx, "-O2", "-shared", "-fPIC", "-o", lib, atfork], verbose)
         res.append(lib)
     return res
+
+
+def build_nodes(force: bool = False, verbose: bool = False) -> Optional[str]:
+    """compile the autograd nodes (``csrc/pyext/autograd_nodes.cpp``) against torch and ``librb200.so``; None without a CUDA build of torch"""
+    import sysconfig
+    import torch
+
+    src = os.path.join(_CSRC, "pyext", "autograd_nodes.cpp")
+    kernels = os.path.join(_BUILD, "librb200.so")
+    root = os.path.dirname(torch.__file__)
+    nvcc = _nvcc()
+    if not (torch.version.cuda and nvcc and os.path.exists(src) and os.path.exists(kernels)):
+        return None
+    lib = os.path.join(_BUILD, "_autograd_nodes.so")
+    # (the kernel library is linked by name: its code may change without a new link)
+    if force or _newer(lib, [src, os.path.join(root, "version.py")]):
+        inc = [sysconfig.get_paths()["include"], os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")]
+        libs = os.path.join(root, "lib")
+        cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+               "-D_GLIBCXX_USE_CXX11_ABI=%i" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+        cmd += [x for i in inc for x in ("-isystem", i)] + ["-o", lib, src, kernels, "-L" + libs, "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + libs]
+        _run(cmd + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"], verbose)
+    return lib
 
 
 def build_all(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> List[str]:

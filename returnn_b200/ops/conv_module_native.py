@@ -7,7 +7,7 @@ statistics, dgamma/dbeta, dfilter) live in scratch buffers allocated per call.
 from __future__ import annotations
 import ctypes
 import torch
-from . import _lib
+from . import _lib, nodes
 
 _vp, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 _TT = 32
@@ -106,4 +106,7 @@ def glu_dwconv_bn_silu(x, filt, bias, bn, pack, *, training):
     beta = bn.beta.raw_tensor if bn.affine else None
     rm = bn.running_mean.raw_tensor if bn.running_mean is not None else None
     rv = bn.running_variance.raw_tensor if bn.running_variance is not None else None
+    mod = nodes.active() if training else None
+    if mod is not None:
+        return mod.conv_module(x, filt, bias, gamma, beta, rm, rv, pack.row_batch, pack.row_pos, pack.lens, bn.eps, bn.momentum)
     return _ConvModuleFn.apply(x, filt, bias, gamma, beta, rm, rv, pack.row_batch, pack.row_pos, pack.lens, float(bn.eps), float(bn.momentum), bool(training))

@@ -12,7 +12,7 @@ from typing import Dict, Optional
 import ctypes
 import os
 import torch
-from . import _lib
+from . import _lib, nodes
 from . import status as _status_board
 
 _vp, _i32, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -172,15 +172,9 @@ def _weight_grad(x: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
     :return: [k, n]
     """
     (m, k), n = x.shape, dy.shape[1]
-    # One CTA per tile of 128 x 256 and slice, all of them at once; at least 256 rows per slice (shorter ones gain less than the sum of the
-    # slices costs); no more than 12, from where the slices that are written and read again cost more than shorter products save.
-    # 6656 x 512 x 512: 12 slices 16 us, one 42; 25000 x 512 x 512: 26 and 138; 6656 x 512 x 2048: 4 slices 24 us, one 43 (slices that add
-    # onto one result by atomics, in any order: 13, 19 and 21 us); 600 x 512 x 512: 2 slices 12.5, one 11.2
-    tiles = -(-k // 128) * -(-n // 256)
-    slices = min(148 // tiles, 12, m // 256)
-    if slices <= 1:
+    rows = _lib.bind("rb200_weight_grad_slices", [_i32, _i32, _i32])(m, k, n)
+    if rows == 0:
         return gemm(x, dy, m=k, n=n, k=m, a_mn_major=True, b_mn_major=True, out_dtype=torch.float32)
-    rows = (-(-m // slices) + 63) // 64 * 64  # (rows past the last one are read as zeros)
     slices = -(-m // rows)
     part = torch.empty(slices, k, n, dtype=torch.float32, device=x.device)
     dw = torch.empty(k, n, dtype=torch.float32, device=x.device)
@@ -394,6 +388,9 @@ def linear_arena_padded_out(x: torch.Tensor, weight: torch.Tensor, bias: Optiona
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: Optional[str]) -> torch.Tensor:
     """``x[..., in] @ weight[in, out] (+ bias) (activation)`` with bf16 operands"""
+    mod = nodes.active() if KERNEL != "legacy" else None
+    if mod is not None:
+        return mod.linear(x, weight, bias, _ACT[activation], status_tensor(x.device))
     if x.dtype != torch.bfloat16:
         x = x.to(torch.bfloat16)
     if bias is not None and bias.dtype not in (torch.bfloat16, torch.float32):

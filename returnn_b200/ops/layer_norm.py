@@ -9,7 +9,7 @@ from __future__ import annotations
 from typing import Optional
 import ctypes
 import torch
-from . import _lib
+from . import _lib, nodes
 
 _vp, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -79,14 +79,16 @@ def _native_ok(x: torch.Tensor, gamma: torch.Tensor) -> bool:
 def layer_norm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float) -> torch.Tensor:
     """(x - mean) * rsqrt(var + eps) * gamma + beta over the last axis"""
     if _native_ok(x, gamma):
-        return _LayerNormFn.apply(x, gamma, beta, float(eps), False)
+        n = nodes.active()
+        return n.layer_norm(x, gamma, beta, eps, False) if n is not None else _LayerNormFn.apply(x, gamma, beta, float(eps), False)
     return layer_norm_reference(x, gamma, beta, eps)
 
 
 def rms_norm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float) -> torch.Tensor:
     """x * rsqrt(mean(x^2) + eps) * gamma (+ beta)"""
     if _native_ok(x, gamma):
-        return _LayerNormFn.apply(x, gamma, beta, float(eps), True)
+        n = nodes.active()
+        return n.layer_norm(x, gamma, beta, eps, True) if n is not None else _LayerNormFn.apply(x, gamma, beta, float(eps), True)
     return rms_norm_reference(x, gamma, beta, eps)
 
 

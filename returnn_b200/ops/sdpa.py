@@ -16,7 +16,7 @@ from typing import Optional
 import ctypes
 import math
 import torch
-from . import _lib
+from . import _lib, nodes
 from . import gemm as _gemm
 from .attention_native import _bgemm
 from .elementwise import _seed_tensor
@@ -251,6 +251,9 @@ def sdpa_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, k_lens: Opt
         k_lens = host_to_device(k_lens.to(torch.int32), q.device).contiguous()
     # the fused kernels are written for one 64-column tile per head, the head dim of all configurations here; other dims take the products
     # with a softmax kernel in between
+    mod = nodes.active() if d == 64 else None
+    if mod is not None:
+        return mod.flash(q, k, v, k_lens, causal, scale, dropout_p, _seed_tensor(q.device) if dropout_p > 0.0 else None, _gemm.status_tensor(q.device))
     fn = _FlashFn if d == 64 and hasattr(_lib.get_lib(), "rb200_flash_fwd") else _SdpaFn
     return fn.apply(q, k, v, k_lens, int(num_heads), bool(causal), float(scale), float(dropout_p))
 

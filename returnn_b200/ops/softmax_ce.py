@@ -5,7 +5,7 @@ Softmax cross entropy with label smoothing over a large vocabulary, one online-s
 from __future__ import annotations
 import ctypes
 import torch
-from . import _lib
+from . import _lib, nodes
 
 _vp, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
@@ -64,6 +64,9 @@ def softmax_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, label_smo
     :return: [rows] fp32 loss (, [rows] int32 arg max)
     """
     if logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and _lib.use_native(logits) and available():
+        mod = nodes.active() if not with_argmax else None
+        if mod is not None:
+            return mod.cross_entropy(logits, targets, label_smoothing, grad_only_smoothing)
         return _CeFn.apply(logits, targets, float(label_smoothing), bool(grad_only_smoothing), bool(with_argmax))
     loss = softmax_cross_entropy_reference(logits, targets, label_smoothing, grad_only_smoothing=grad_only_smoothing)
     if with_argmax:
