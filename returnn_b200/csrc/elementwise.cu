@@ -31,43 +31,46 @@ dropout_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ 
 }
 
 // The part of a linear layer's backward pass before its two products, in one pass over the rows: dz = dy * act'(z) (bf16; act 0: dz is
-// dy and is not written) and the bias gradient db[c] += sum_r dz[r][c] of the rounded values. A CTA owns 64 columns (8 threads x 16
-// bytes: whole 128-byte lines) and a slice of the rows; its 32 row lanes take two rows at a time (four loads in flight, two without an
+// dy and is not written) and the bias gradient db[c] += sum_r dz[r][c] of the rounded values. A CTA owns 8 CG columns (CG threads x 16
+// bytes: lines of 128 or pieces of 512 bytes) and a slice of the rows; its 32 row lanes take U rows at a time (2 U loads in flight, U without an
 // activation). Column sums: with `part` every slice leaves its own there, and colsum_slices_kernel adds them up in the order of the slices, so
 // that the gradient of the same inputs is the same in every run; without, one atomic per column and CTA adds them to what is in db (6656 x 2048,
 // silu: 19.3 us ordered, 18.2 by atomics; 6656 x 512, no activation: 5.1 and 2.6).
 // Bound by memory: 6656 x 2048, silu: 82 MB.
-template <int ACT>
-__global__ void __launch_bounds__(256, 4)
+template <int ACT, int CG, int U>
+__global__ void __launch_bounds__(32 * CG, CG == 8 ? 4 : 1)
 act_grad_colsum_kernel(const __nv_bfloat16* __restrict__ z, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dz,
                        float* __restrict__ db, float* __restrict__ part, int rows, int cols, int rows_per_cta) {
   rb_pdl_wait();
   rb_pdl_launch();
-  __shared__ float red[32][65];
-  const int cg = threadIdx.x & 7, rl = threadIdx.x >> 3;
-  const int col = blockIdx.y * 64 + cg * 8;
+  __shared__ float red[32][8 * CG + 1];
+  const int cg = threadIdx.x % CG, rl = threadIdx.x / CG;
+  const int col = (blockIdx.y * CG + cg) * 8;
   const int r_begin = blockIdx.x * rows_per_cta;
   const int r_end = min(rows, r_begin + rows_per_cta);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col < cols) {
-    for (int r0 = r_begin + rl; r0 < r_end; r0 += 64) {
-      F8 d[2], v[2];
+    for (int r0 = r_begin + rl; r0 < r_end; r0 += 32 * U) {
+      uint4 dr[U], vr[U];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < U; ++u) {
         const int r = r0 + u * 32;
         if (r < r_end) {
-          d[u] = load8(dy, (int64_t)r * cols + col, 1);
-          if (ACT) v[u] = load8(z, (int64_t)r * cols + col, 1);
+          dr[u] = *reinterpret_cast<const uint4*>(dy + (int64_t)r * cols + col);
+          if (ACT) vr[u] = *reinterpret_cast<const uint4*>(z + (int64_t)r * cols + col);
         }
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < U; ++u) {
         const int r = r0 + u * 32;
         if (r >= r_end) break;
+        F8 d[1], v[1];
+        d[0] = load8(&dr[u], 0, 1);
+        if (ACT) v[0] = load8(&vr[u], 0, 1);
         if (ACT) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const float x = v[u].v[i];
+            const float x = v[0].v[i];
             float g;
             if (ACT == 1) {
               g = x > 0.f ? 1.f : 0.f;
@@ -77,12 +80,12 @@ act_grad_colsum_kernel(const __nv_bfloat16* __restrict__ z, const __nv_bfloat16*
             } else {
               g = 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * __expf(-0.5f * x * x) * 0.39894228040143268f;
             }
-            d[u].v[i] = __bfloat162float(__float2bfloat16(d[u].v[i] * g));
+            d[0].v[i] = __bfloat162float(__float2bfloat16(d[0].v[i] * g));
           }
-          store8(dz, (int64_t)r * cols + col, d[u], 1);
+          store8(dz, (int64_t)r * cols + col, d[0], 1);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] += d[u].v[i];
+        for (int i = 0; i < 8; ++i) acc[i] += d[0].v[i];
       }
     }
   }
@@ -90,8 +93,8 @@ act_grad_colsum_kernel(const __nv_bfloat16* __restrict__ z, const __nv_bfloat16*
 #pragma unroll
   for (int i = 0; i < 8; ++i) red[rl][cg * 8 + i] = acc[i];
   __syncthreads();
-  const int c = blockIdx.y * 64 + threadIdx.x;
-  if (threadIdx.x < 64 && c < cols) {
+  const int c = blockIdx.y * 8 * CG + threadIdx.x;
+  if (threadIdx.x < 8 * CG && c < cols) {
     float sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 32; ++k) sum += red[k][threadIdx.x];
@@ -136,18 +139,27 @@ RB_EXPORT int rb200_act_grad_colsum(const void* z, const void* dy, void* dz, flo
     rb_launch_pdl(colsum_slices_kernel, dim3(chunks), dim3(256), 0, stream, (const float*)work, db, 0, cols);
     return rb_check_launch("colsum_slices");
   }
-  int splits = colsum_splits(rows, cols);
+  // Wide where the matrices do not stay in the L2 (dz, z and dy of 12 M elements: 72 MB). us, narrow / wide, silu: 6656 x 2048 17.7 / 16.0, 6656 x 4096
+  // 39.1 / 33.6, 25000 x 2048 70.5 / 55.1; below the launch and the start of a CTA of 1024 threads cost more: 2000 x 4096 11.5 / 12.0,
+  // 6656 x 512 7.5 / 8.7, 50 x 512 3.1 / 4.6
+  const bool wide = cols >= 256 && (long long)rows * cols >= 12000000;
+  const int cta_chunks = wide ? (cols + 255) / 256 : chunks;
+  int splits = wide ? max(1, min(148 / cta_chunks, (rows + 31) / 32)) : colsum_splits(rows, cols);
   const int per = (rows + splits - 1) / splits;
   splits = (rows + per - 1) / per;
-  auto kernel = act == 0 ? act_grad_colsum_kernel<0> : act == 1 ? act_grad_colsum_kernel<1> : act == 2 ? act_grad_colsum_kernel<2> : act_grad_colsum_kernel<3>;
+  using Kernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, __nv_bfloat16*, float*, float*, int, int, int);
+  static const Kernel narrow[] = {act_grad_colsum_kernel<0, 8, 2>, act_grad_colsum_kernel<1, 8, 2>, act_grad_colsum_kernel<2, 8, 2>, act_grad_colsum_kernel<3, 8, 2>};
+  static const Kernel wides[] = {act_grad_colsum_kernel<0, 32, 4>, act_grad_colsum_kernel<1, 32, 4>, act_grad_colsum_kernel<2, 32, 4>, act_grad_colsum_kernel<3, 32, 2>};
+  const Kernel kernel = (wide ? wides : narrow)[act];
+  const dim3 grid(splits, cta_chunks), block(wide ? 1024 : 256);
   const __nv_bfloat16 *zp = (const __nv_bfloat16*)z, *dyp = (const __nv_bfloat16*)dy;
   if (!work) {
-    rb_launch_pdl(kernel, dim3(splits, chunks), dim3(256), 0, stream, zp, dyp, (__nv_bfloat16*)dz, db, work, rows, cols, per);
+    rb_launch_pdl(kernel, grid, block, 0, stream, zp, dyp, (__nv_bfloat16*)dz, db, work, rows, cols, per);
     return rb_check_launch("act_grad_colsum");
   }
   // Not launched early: CTAs that come onto the SMs one by one while a product ends do not walk through the rows side by side, and the 64-column
   // pieces of a row are then read far apart in time (6656 x 10000 after a product: 61 us, launched in order 37)
-  kernel<<<dim3(splits, chunks), 256, 0, stream>>>(zp, dyp, (__nv_bfloat16*)dz, db, work, rows, cols, per);
+  kernel<<<grid, block, 0, stream>>>(zp, dyp, (__nv_bfloat16*)dz, db, work, rows, cols, per);
   const int st = rb_check_launch("act_grad_colsum");
   if (st) return st;
   rb_launch_pdl(colsum_slices_kernel, dim3(chunks), dim3(256), 0, stream, (const float*)work, db, splits, cols);

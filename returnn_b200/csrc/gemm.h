@@ -27,6 +27,8 @@ struct RbGemm {
   float res_scale = 1.f;
   float* colsum = nullptr;       // [n] += the column sums of the stored bf16 values; only where rb_gemm_column_sums says so
   int split_k = 0;               // 0: chosen by the launcher (> 1 only with accumulate == 2)
+  int slice_k = 0;               // CTA-pair kernel, fp32 output without the rest of the epilogue, m a multiple of 32: the contraction is cut into slices
+                                 // of this many (a multiple of 64), whose products lie one behind the other in c, [ceil(k / slice_k)][m][ldc]
   // batched form (batch > 0): problem z = b * heads + h reads A from the stored origin (b*a_rb + h*a_rh, b*a_cb + h*a_ch),
   // B likewise, and writes at element offset b*c_sb + h*c_sh. m / n / k are fixed or lens[b] where the *_from_lens flag is set;
   // a problem with an empty extent is skipped. a_rows .. b_cols are the extents of the stored matrices.
@@ -56,6 +58,9 @@ int rb_gemm(const RbGemm& g, cudaStream_t stream);
 // whether the epilogue of this problem's kernel can leave column sums (`colsum`): the full epilogue of the CTA-pair kernel with one bf16 output
 // that leaves through bulk stores
 bool rb_gemm_column_sums(const RbGemm& g);
+
+// whether the CTA-pair kernel takes this problem with slice_k
+bool rb_gemm_slices(const RbGemm& g);
 
 // CTA-pair kernel (gemm_2cta.cu): rb_gemm routes to it when rb_gemm_pair_wanted says so
 bool rb_gemm_pair_wanted(const RbGemm& g);

@@ -261,6 +261,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     for (; walk.more(); walk.next()) {
       w.m0 = walk.mi * BM;
       w.n0 = walk.ni * BN;
+      if (KIND == kEpiF32 && g.slice_k) w.c_r0 = walk.sp * g.m;
       const int m0 = w.m0 + (int)rank * 128, n0 = w.n0;
       const uint32_t buf = t_local & 1u;
       const int part = (warp - 2) >> 2;  // four warps per lane quarter, each with a quarter of the columns
@@ -352,7 +353,16 @@ bool rb_gemm_column_sums(const RbGemm& g) {
   return rb_gemm_pair_wanted(g) && tma_store_on() && full_epilogue(g) && aligned_outputs(g) && g.c != nullptr && g.c2 == nullptr && !g.out_fp32;
 }
 
+bool rb_gemm_slices(const RbGemm& g) {
+  return rb_gemm_pair_wanted(g) && tma_store_on() && aligned_outputs(g) && g.c != nullptr && g.out_fp32 && !g.accumulate && !full_epilogue(g) && !g.bias && !g.act &&
+         !g.c2 && !g.seg_a && g.m % 32 == 0 && g.n % 8 == 0 && g.slice_k > 0 && g.slice_k % BK == 0;
+}
+
 int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
+  if (g.slice_k && !rb_gemm_slices(g)) {
+    rb_set_error("gemm (pair): m=%d n=%d slice_k=%d is not a product in slices", g.m, g.n, g.slice_k);
+    return RB_ERR_ARG;
+  }
   if (g.colsum && !rb_gemm_column_sums(g)) {
     rb_set_error("gemm (pair): this problem's epilogue leaves no column sums");
     return RB_ERR_ARG;
@@ -388,7 +398,7 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
     if (split > max_split) split = max_split;
     if (split < 1) split = 1;
   }
-  p.kb_per_split = (p.num_kb + split - 1) / split;
+  p.kb_per_split = g.slice_k ? g.slice_k / BK : (p.num_kb + split - 1) / split;
   p.split = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
   p.units = tiles * p.split;
   p.vec_ok = aligned_outputs(g);
@@ -407,7 +417,7 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
       if (st) return st;
       st = make_map(&tm_c2, g.c2, g.n, g.m, g.ldc, 32, 32, false, true);
     } else if (kind == kEpiF32) {
-      st = make_map(&tm_c, g.c, g.n, g.m, g.ldc, 16, 32, true, true);
+      st = make_map(&tm_c, g.c, g.n, (long long)g.m * (g.slice_k ? p.split : 1), g.ldc, 16, 32, true, true);
     } else {
       st = make_map(&tm_c, g.c, g.n, g.m, g.ldc, g.out_fp32 ? 32 : 64, 32, g.out_fp32 != 0);
     }

@@ -191,6 +191,7 @@ __device__ __forceinline__ void epilogue_group(const Params& p, int row, int col
 // one work unit: output tile (m0, n0) of problem z, K blocks [kb0, kb1)
 struct Unit {
   int m0, n0, kb0, kb1, M, N;
+  int c_r0;  // row of the stored output that row 0 of this unit's product is (slices one behind the other)
   int a_r0, a_c0, b_r0, b_c0;
   size_t c_off;
   bool valid;
@@ -200,6 +201,7 @@ template <int BM, int BN>
 __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
   const RbGemm& g = p.g;
   Unit w;
+  w.c_r0 = 0;
   const int tiles = p.tiles_m * p.tiles_n;
   if (g.batch > 0) {
     const int z = u / tiles, t = u % tiles;
@@ -654,7 +656,7 @@ __device__ __forceinline__ void epilogue_kind_tma(const Params& p, const Unit& w
         if (cbox < w.N) {
           const uint8_t* from = F32 ? box + (ph & 1) * 2048 : box;
           if (F32 && g.accumulate) tma_reduce_add_2d(tm_c, cbox, row0, from);
-          else tma_store_2d(tm_c, cbox, row0, from);
+          else tma_store_2d(tm_c, cbox, F32 ? w.c_r0 + row0 : row0, from);
           if (TWO) tma_store_2d(tm_c2, cbox, row0, box + 2048);
         }
         tma_store_commit();

@@ -428,9 +428,17 @@ RB_EXPORT int rb200_weight_grad_sliced(const void* x, const void* dy, float* par
   RbGemm g;
   g.a = x; g.b = dy; g.c = part; g.m = k; g.n = n; g.k = rows; g.lda = k; g.ldb = n; g.ldc = n;
   g.a_mn_major = 1; g.b_mn_major = 1; g.out_fp32 = 1; g.status = status;
-  g.batch = (m + rows - 1) / rows; g.heads = 1;
+  const int slices = (m + rows - 1) / rows;
+  RbGemm pair = g;
+  pair.k = m;
+  pair.slice_k = rows;
+  if (rb_gemm_slices(pair)) {  // the same slices with tiles of 256 x 256 by CTA pairs (6656 x 512 x 2048, four slices: 23 -> 20 us in a profile)
+    const int st = rb_gemm(pair, stream);
+    return st ? st : rb200_sum_slices_f32(part, dw, slices, (long long)k * n, stream);
+  }
+  g.batch = slices; g.heads = 1;
   g.a_rb = rows; g.b_rb = rows; g.c_sb = (long long)k * n;
   g.a_rows = m; g.a_cols = k; g.b_rows = m; g.b_cols = n;
   const int st = rb_gemm(g, stream);
-  return st ? st : rb200_sum_slices_f32(part, dw, g.batch, (long long)k * n, stream);
+  return st ? st : rb200_sum_slices_f32(part, dw, slices, (long long)k * n, stream);
 }

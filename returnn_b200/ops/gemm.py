@@ -388,7 +388,7 @@ def linear_arena_padded_out(x: torch.Tensor, weight: torch.Tensor, bias: Optiona
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: Optional[str]) -> torch.Tensor:
     """``x[..., in] @ weight[in, out] (+ bias) (activation)`` with bf16 operands"""
-    mod = nodes.active() if KERNEL != "legacy" else None
+    mod = nodes.active() if x.is_cuda and KERNEL != "legacy" else None
     if mod is not None:
         return mod.linear(x, weight, bias, _ACT[activation], status_tensor(x.device))
     if x.dtype != torch.bfloat16:

@@ -1,7 +1,7 @@
 """
 Debug harness for the native kernels: out-of-bounds writes and missing stream dependencies, found without a sanitizer.
 
-* :class:`CanaryAllocations`: while active, every tensor that the Python wrappers allocate for a kernel (``torch.empty``,
+* :class:`CanaryAllocations`: while active, every tensor that the wrappers allocate for a kernel (``torch.empty``,
   ``zeros``, ``empty_like``, ``zeros_like``, ``full``: outputs, saved tensors, scratch) sits between two guard regions filled
   with a byte pattern. ``check()`` synchronises and reports every guard that a kernel wrote into, with the offset of the
   first damaged byte. The guards are 4 KB on each side, so the data pointer keeps the 256-byte alignment of the allocator
@@ -117,9 +117,18 @@ class CanaryAllocations:
             self._orig[name] = getattr(torch, name)
         for name in self._FUNCS:
             setattr(torch, name, self._wrap(name))
+        from . import nodes
+
+        self._nodes = nodes.active()
+        if self._nodes is not None:  # the autograd nodes in C++ allocate through the same functions while this is active
+            types = (torch.float32, torch.bfloat16, torch.int32)
+            self._hook = lambda like, shape, code: torch.empty(*shape, dtype=types[code], device=like.device)
+            self._nodes.set_allocator(self._hook)
         return self
 
     def __exit__(self, *exc):
+        if self._nodes is not None:
+            self._nodes.set_allocator(None)
         for name, fn in self._orig.items():
             setattr(torch, name, fn)
         return False
