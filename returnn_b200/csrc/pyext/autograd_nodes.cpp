@@ -44,6 +44,7 @@ int rb200_conv_module_bwd(const void* x, const void* y, const void* dz, const fl
                           void* dx, float* dfilt, float* dbias, int n_rows, int n_seqs, int C, int K, cudaStream_t stream);
 int rb200_flash_fwd(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, void* keep, const int* k_lens, const int* g, float scale,
                     float p_drop, const long long* seed, const long long* offset, int* status, cudaStream_t stream);
+int rb200_flash_bwd_one_kernel(int tq, int tk);
 int rb200_flash_bwd(const void* q, const void* k, const void* v, const float* o32, const void* d_o, void* dq, void* dk, void* dv, float* lse, float* delta,
                     void* keep, const int* k_lens, const int* g, float scale, float p_drop, int* status, cudaStream_t stream);
 int rb200_softmax_ce_fwd(const void* logits, const int* targets, float* loss, float* lse, long long rows, int v, float smoothing, int is_bf16, int grad_only,
@@ -70,7 +71,39 @@ T* ptr(const OptTensor& t) {
   return t.has_value() && t->defined() ? static_cast<T*>(t->data_ptr()) : nullptr;
 }
 bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
-Tensor empty(at::IntArrayRef shape, const Tensor& like, at::ScalarType type) { return at::empty(shape, like.options().dtype(type)); }
+
+// A debugger of the kernels (ops/guard.py) may allocate in our place: hook(like, shape, type) with type 0 fp32, 1 bf16, 2 int32, None: not its concern
+std::atomic<PyObject*> allocator{nullptr};
+
+Tensor hooked(PyObject* hook, at::IntArrayRef shape, const Tensor& like, at::ScalarType type) {
+  const int code = type == at::kFloat ? 0 : type == at::kBFloat16 ? 1 : type == at::kInt ? 2 : -1;
+  Tensor res;
+  if (code >= 0) {
+    const PyGILState_STATE gil = PyGILState_Ensure();
+    PyObject* dims = PyTuple_New((Py_ssize_t)shape.size());
+    for (size_t i = 0; dims && i < shape.size(); ++i) PyTuple_SET_ITEM(dims, (Py_ssize_t)i, PyLong_FromLongLong(shape[i]));
+    PyObject* t = dims ? THPVariable_Wrap(like.detach()) : nullptr;
+    PyObject* r = t ? PyObject_CallFunction(hook, "OOi", t, dims, code) : nullptr;
+    if (r && THPVariable_Check(r)) res = THPVariable_Unpack(r);
+    const bool failed = r == nullptr;
+    Py_XDECREF(r);
+    Py_XDECREF(t);
+    Py_XDECREF(dims);
+    if (failed) PyErr_Clear();
+    PyGILState_Release(gil);
+    TORCH_CHECK(!failed, "the allocation hook failed");
+  }
+  return res;
+}
+
+Tensor fresh(at::IntArrayRef shape, const Tensor& like, at::ScalarType type) {
+  if (PyObject* hook = allocator.load(std::memory_order_acquire)) {
+    const Tensor t = hooked(hook, shape, like, type);
+    if (t.defined()) return t;
+  }
+  return at::empty(shape, like.options().dtype(type));
+}
+Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t, t.scalar_type()); }  // (contiguous)
 
 // ---- layer norm, RMS norm
 struct LayerNorm : Function<LayerNorm> {
@@ -81,8 +114,8 @@ struct LayerNorm : Function<LayerNorm> {
     const int64_t rows = x2.size(0);
     const Tensor g = gamma.contiguous();
     const Tensor b = beta.has_value() ? beta->contiguous() : Tensor();
-    Tensor y = at::empty_like(x2);
-    Tensor mean = empty({rows}, x, at::kFloat), rstd = empty({rows}, x, at::kFloat);
+    Tensor y = fresh_like(x2);
+    Tensor mean = fresh({rows}, x, at::kFloat), rstd = fresh({rows}, x, at::kFloat);
     check(rb200_layer_norm_fwd(ptr(x2), ptr(g), b.defined() ? ptr(b) : nullptr, ptr(y), ptr<float>(mean), ptr<float>(rstd), rows, (int)n, (float)eps, is_bf16(x2),
                                is_bf16(g), rms, stream()),
           "layer_norm_fwd");
@@ -101,11 +134,11 @@ struct LayerNorm : Function<LayerNorm> {
     const auto shape = ctx->saved_data["shape"].toIntVector();
     const int64_t rows = x2.size(0), n = x2.size(1);
     const Tensor dy = grads[0].reshape({rows, n}).contiguous();
-    Tensor dx = at::empty_like(x2);
+    Tensor dx = fresh_like(x2);
     if (is_bf16(x2) && n <= 512 && rows > 0 && is_bf16(dy) && (is_bf16(g) || g.scalar_type() == at::kFloat)) {
       // one kernel, which also leaves the parameter gradients in the type of the parameters
-      Tensor work = empty({2 * n + 1}, x2, at::kFloat);
-      Tensor dgamma = at::empty_like(g), dbeta = has_beta ? at::empty_like(g) : Tensor();
+      Tensor work = fresh({2 * n + 1}, x2, at::kFloat);
+      Tensor dgamma = fresh_like(g), dbeta = has_beta ? fresh_like(g) : Tensor();
       check(rb200_layer_norm_bwd_typed(ptr(x2), ptr(dy), ptr(g), ptr<float>(mean), ptr<float>(rstd), ptr(dx), ptr<float>(work), ptr(dgamma),
                                        has_beta ? ptr(dbeta) : nullptr, rows, (int)n, is_bf16(g), rms, stream()),
             "layer_norm_bwd");
@@ -113,7 +146,7 @@ struct LayerNorm : Function<LayerNorm> {
       return {dx.reshape(shape), dgamma, dbeta, Tensor(), Tensor()};
     }
     const int64_t n_part = std::min<int64_t>(296, std::max<int64_t>(1, (rows + 31) / 32));
-    Tensor part = empty({2, n_part, n}, x2, at::kFloat), dgamma = empty({n}, x2, at::kFloat), dbeta = empty({n}, x2, at::kFloat);
+    Tensor part = fresh({2, n_part, n}, x2, at::kFloat), dgamma = fresh({n}, x2, at::kFloat), dbeta = fresh({n}, x2, at::kFloat);
     check(rb200_layer_norm_bwd(ptr(x2), ptr(dy), ptr(g), ptr<float>(mean), ptr<float>(rstd), ptr(dx), ptr<float>(part), ptr<float>(dgamma), ptr<float>(dbeta), rows,
                                (int)n, (int)n_part, is_bf16(x2), is_bf16(g), rms, stream()),
           "layer_norm_bwd");
@@ -160,10 +193,10 @@ struct Linear : Function<Linear> {
     const c10::cuda::CUDAGuard guard(x2.device());
     const Tensor w = weight.to(at::kBFloat16).contiguous();
     const int64_t m = x2.size(0), k = x2.size(1), n = w.size(1);
-    Tensor y = empty({m, n}, x2, at::kBFloat16), z;
+    Tensor y = fresh({m, n}, x2, at::kBFloat16), z;
     // (a parameter says that it requires a gradient under no_grad as well)
     if (act && differentiable && (x2.requires_grad() || weight.requires_grad())) {
-      z = empty({m, n}, x2, at::kBFloat16);
+      z = fresh({m, n}, x2, at::kBFloat16);
       gemm(x2, w, z, &y, bias, m, n, k, false, true, (int)act, status);
     } else {
       gemm(x2, w, y, nullptr, bias, m, n, k, false, true, (int)act, status);
@@ -185,12 +218,12 @@ struct Linear : Function<Linear> {
     const bool has_bias = ctx->saved_data["has_bias"].toBool();
     const int64_t m = x2.size(0), k = x2.size(1), n = w.size(1);
     Tensor dy = grads[0].contiguous(), dx, dw, db;
-    if (has_bias && ctx->needs_input_grad(2)) db = empty({n}, dy, at::kFloat);
+    if (has_bias && ctx->needs_input_grad(2)) db = fresh({n}, dy, at::kFloat);
     if (act || db.defined()) {
       // 16-byte accesses: a gradient that starts off that alignment takes the elementwise form
       if (is_bf16(dy) && n % 8 == 0 && aligned16(dy) && (!z.defined() || aligned16(z))) {
-        Tensor dz = act ? at::empty_like(dy) : dy, work;
-        if (db.defined()) work = empty({4 * 148 * 64 + n}, dy, at::kFloat);
+        Tensor dz = act ? fresh_like(dy) : dy, work;
+        if (db.defined()) work = fresh({4 * 148 * 64 + n}, dy, at::kFloat);
         check(rb200_act_grad_colsum(act ? ptr(z) : nullptr, ptr(dy), act ? ptr(dz) : nullptr, db.defined() ? ptr<float>(db) : nullptr,
                                     work.defined() ? ptr<float>(work) : nullptr, (int)m, (int)n, act, stream()),
               "act_grad_colsum");
@@ -202,25 +235,25 @@ struct Linear : Function<Linear> {
     }
     if (ctx->needs_input_grad(0)) {
       // dX[m,k] = dY[m,n] W[k,n]^T: contraction over n, W rows are contiguous in n -> "K-major" B
-      dx = empty({m, k}, x2, at::kBFloat16);
+      dx = fresh({m, k}, x2, at::kBFloat16);
       gemm(dy, w, dx, nullptr, std::nullopt, m, k, n, false, false, 0, status);
     }
     if (ctx->needs_input_grad(1)) {
       // dW[k,n] = X[m,k]^T dY[m,n]: contraction over m, both operands contiguous in their output dim
       const auto w_dtype = ctx->saved_data["w_dtype"].toScalarType();
       if (w_dtype == at::kFloat) {
-        dw = empty({k, n}, x2, at::kFloat);
+        dw = fresh({k, n}, x2, at::kFloat);
         const int rows = rb200_weight_grad_slices((int)m, (int)k, (int)n);
         if (rows == 0) {
           gemm(x2, dy, dw, nullptr, std::nullopt, k, n, m, true, true, 0, status);
         } else {
-          Tensor part = empty({(m + rows - 1) / rows, k, n}, x2, at::kFloat);
+          Tensor part = fresh({(m + rows - 1) / rows, k, n}, x2, at::kFloat);
           check(rb200_weight_grad_sliced(ptr(x2), ptr(dy), ptr<float>(part), ptr<float>(dw), (int)m, (int)k, (int)n, rows, ptr<int>(status), stream()),
                 "weight_grad_sliced");
           count(2);
         }
       } else {
-        dw = empty({k, n}, x2, at::kBFloat16);
+        dw = fresh({k, n}, x2, at::kBFloat16);
         gemm(x2, dy, dw, nullptr, std::nullopt, k, n, m, true, true, 0, status);
         dw = dw.to(w_dtype);
       }
@@ -253,8 +286,8 @@ struct ConvModule : Function<ConvModule> {
     auto f32 = [](const OptTensor& t) { return t.has_value() ? t->to(at::kFloat).contiguous() : Tensor(); };
     const Tensor f = filt.reshape({C, K}).to(at::kFloat).contiguous(), b = f32(bias), g = f32(gamma), be = f32(beta);
     auto p = [](const Tensor& t) { return t.defined() ? ptr<float>(t) : nullptr; };
-    Tensor y = empty({N, C}, x, at::kBFloat16), z = empty({N, C}, x, at::kBFloat16);
-    Tensor part = empty({(N + 31) / 32 * 2 * C}, x, at::kFloat), stats = empty({2, C}, x, at::kFloat);  // mean, 1 / deviation
+    Tensor y = fresh({N, C}, x, at::kBFloat16), z = fresh({N, C}, x, at::kBFloat16);
+    Tensor part = fresh({(N + 31) / 32 * 2 * C}, x, at::kFloat), stats = fresh({2, C}, x, at::kFloat);  // mean, 1 / deviation
     check(rb200_conv_module_fwd(ptr(x), ptr<float>(f), p(b), p(g), p(be), ptr<int>(row_batch), ptr<int>(row_pos), ptr<int>(lens), ptr(y), ptr(z), ptr<float>(part),
                                 ptr<float>(stats), ptr<float>(running_mean), ptr<float>(running_var), (int)N, (int)lens.size(0), (int)C, (int)K, 1, (float)eps,
                                 (float)momentum, stream()),
@@ -277,12 +310,12 @@ struct ConvModule : Function<ConvModule> {
     const int64_t N = x.size(0), C = x.size(1) / 2, K = f.size(1);
     const Tensor dz = grads[0].contiguous();
     const int64_t tiles = std::min<int64_t>(296, std::max<int64_t>(1, (N + 15) / 16));
-    Tensor ds = empty({N, C}, x, at::kBFloat16);
+    Tensor ds = fresh({N, C}, x, at::kBFloat16);
     // the sums of the two passes, one after the other in the same scratch
-    Tensor part = empty({std::max(tiles * 2 * C, (N + 31) / 32 * C * (K + 1))}, x, at::kFloat);
-    Tensor sum_ds = empty({C}, x, at::kFloat), sum_ds_yh = empty({C}, x, at::kFloat), dx = at::empty_like(x), df = empty({C, K}, x, at::kFloat);
+    Tensor part = fresh({std::max(tiles * 2 * C, (N + 31) / 32 * C * (K + 1))}, x, at::kFloat);
+    Tensor sum_ds = fresh({C}, x, at::kFloat), sum_ds_yh = fresh({C}, x, at::kFloat), dx = fresh_like(x), df = fresh({C, K}, x, at::kFloat);
     const bool has_bias = d.count("bdtype") > 0, has_gamma = d.count("gdtype") > 0, has_beta = d.count("bedtype") > 0;
-    Tensor db = has_bias ? empty({C}, x, at::kFloat) : Tensor();
+    Tensor db = has_bias ? fresh({C}, x, at::kFloat) : Tensor();
     auto p = [](const Tensor& t) { return t.defined() ? ptr<float>(t) : nullptr; };
     check(rb200_conv_module_bwd(ptr(x), ptr(y), ptr(dz), ptr<float>(stats), ptr<float>(f), p(g), p(be), ptr<int>(row_batch), ptr<int>(row_pos), ptr<int>(lens),
                                 ptr(ds), ptr<float>(part), (int)tiles, ptr<float>(sum_ds), ptr<float>(sum_ds_yh), ptr(dx), ptr<float>(df), p(db), (int)N,
@@ -330,11 +363,12 @@ struct Flash : Function<Flash> {
     const int64_t Tqp = (Tq + 63) / 64 * 64, Tkp = (Tk + 63) / 64 * 64, words = (Tk + 127) / 128 * 4;
     geom[0] = B; geom[1] = H; geom[2] = Tq; geom[3] = Tk; geom[4] = causal; geom[5] = Tk - Tq;
     geom[14] = Tqp; geom[15] = Tkp; geom[16] = words;
-    Tensor o = empty({B, Tq, H, 64}, q, at::kBFloat16), lse = empty({B * H * Tq}, q, at::kFloat), o32, keep, off;
+    Tensor o = fresh({B, Tq, H, 64}, q, at::kBFloat16), lse = fresh({B * H * Tq}, q, at::kFloat), o32, keep, off;
     // the backward pass takes row sums of the output: from a copy of its own in 32 bits, so that the caller may change the result in place
-    if (q.requires_grad() || k.requires_grad() || v.requires_grad()) o32 = empty({B, Tq, H, 64}, q, at::kFloat);
+    // (the one kernel of short sequences takes them from the probabilities)
+    if ((q.requires_grad() || k.requires_grad() || v.requires_grad()) && !rb200_flash_bwd_one_kernel((int)Tq, (int)Tk)) o32 = fresh({B, Tq, H, 64}, q, at::kFloat);
     if (p_drop > 0.) {
-      keep = empty({B * H * Tq * words}, q, at::kInt);
+      keep = fresh({B * H * Tq * words}, q, at::kInt);
       off = seed->slice(0, 1, 2).clone();
       seed->select(0, 1).add_(B * H * Tqp * Tkp);
     }
@@ -361,14 +395,15 @@ struct Flash : Function<Flash> {
     auto geom = d["geom"].toIntVector();
     const Tensor d_o = rows_of(grads[0], geom[12], geom[13]), status = d["status"].toTensor();
     const int64_t B = geom[0], H = geom[1], Tq = geom[2], Tk = geom[3];
-    Tensor delta = at::empty_like(lse), dq = empty({B, Tq, H, 64}, q2, at::kBFloat16), dk = empty({B, Tk, H, 64}, q2, at::kBFloat16),
-           dv = empty({B, Tk, H, 64}, q2, at::kBFloat16);
+    Tensor delta = o32.defined() ? fresh_like(lse) : Tensor(), dq = fresh({B, Tq, H, 64}, q2, at::kBFloat16), dk = fresh({B, Tk, H, 64}, q2, at::kBFloat16),
+           dv = fresh({B, Tk, H, 64}, q2, at::kBFloat16);
     const std::vector<int> g(geom.begin(), geom.end());
-    check(rb200_flash_bwd(ptr(q2), ptr(k2), ptr(v2), ptr<float>(o32), ptr(d_o), ptr(dq), ptr(dk), ptr(dv), ptr<float>(lse), ptr<float>(delta),
+    check(rb200_flash_bwd(ptr(q2), ptr(k2), ptr(v2), o32.defined() ? ptr<float>(o32) : nullptr, ptr(d_o), ptr(dq), ptr(dk), ptr(dv), ptr<float>(lse),
+                          delta.defined() ? ptr<float>(delta) : nullptr,
                           keep.defined() ? ptr(keep) : nullptr, k_lens.defined() ? ptr<int>(k_lens) : nullptr, g.data(), (float)d["scale"].toDouble(),
                           (float)d["p_drop"].toDouble(), ptr<int>(status), stream()),
           "flash_bwd");
-    count(2);
+    count(o32.defined() ? 2 : 1);
     const auto dt = d["dtype"].toScalarType();
     const Tensor none;
     return {dq.to(dt), dk.to(dt), dv.to(dt), none, none, none, none, none, none};
@@ -381,7 +416,7 @@ struct CrossEntropy : Function<CrossEntropy> {
     const c10::cuda::CUDAGuard guard(logits_.device());
     const Tensor logits = logits_.contiguous(), tgt = targets.to(at::kInt).contiguous();
     const int64_t rows = logits.size(0), v = logits.size(1);
-    Tensor loss = empty({rows}, logits, at::kFloat), lse = empty({rows}, logits, at::kFloat);
+    Tensor loss = fresh({rows}, logits, at::kFloat), lse = fresh({rows}, logits, at::kFloat);
     check(rb200_softmax_ce_fwd(ptr(logits), ptr<int>(tgt), ptr<float>(loss), ptr<float>(lse), rows, (int)v, (float)smoothing, is_bf16(logits), grad_only, nullptr,
                                stream()),
           "softmax_ce_fwd");
@@ -395,7 +430,7 @@ struct CrossEntropy : Function<CrossEntropy> {
     const auto s = ctx->get_saved_variables();
     const Tensor &logits = s[0], &tgt = s[1], &lse = s[2];
     const c10::cuda::CUDAGuard guard(logits.device());
-    Tensor dlogits = at::empty_like(logits);
+    Tensor dlogits = fresh_like(logits);
     const Tensor dl = grads[0].to(at::kFloat).contiguous();
     check(rb200_softmax_ce_bwd(ptr(logits), ptr<int>(tgt), ptr<float>(lse), ptr<float>(dl), ptr(dlogits), logits.size(0), (int)logits.size(1),
                                (float)ctx->saved_data["smoothing"].toDouble(), is_bf16(logits), ctx->saved_data["grad_only"].toBool(), stream()),
@@ -454,6 +489,10 @@ PyObject* py_flash(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_cross_entropy(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return enter<4>(args, n, [](Args a) { return CrossEntropy::apply(a.tensor(0), a.tensor(1), a.number(2), a.truth(3)); });
 }
+PyObject* py_set_allocator(PyObject*, PyObject* hook) {  // the caller keeps the hook alive until it is replaced
+  allocator.store(hook == Py_None ? nullptr : hook, std::memory_order_release);
+  Py_RETURN_NONE;
+}
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launches.load(std::memory_order_relaxed)); }
 
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
@@ -467,6 +506,7 @@ PyMethodDef methods[] = {
     fast<py_conv_module>("conv_module", "(x, filt, bias, gamma, beta, running_mean, running_var, row_batch, row_pos, lens, eps, momentum) -> z"),
     fast<py_flash>("flash", "(q, k, v, k_lens, causal, scale, p_drop, seed, status) -> o"),
     fast<py_cross_entropy>("cross_entropy", "(logits, targets, smoothing, grad_only) -> loss"),
+    {"set_allocator", py_set_allocator, METH_O, "(hook or None): allocate through hook(like, shape, type); for debugging"},
     {"launches", py_launches, METH_NOARGS, "kernels launched by the nodes so far"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -159,7 +159,7 @@ class _SdpaFn(torch.autograd.Function):
 
 
 class _FlashFn(torch.autograd.Function):
-    """head dim 64: one kernel forward, two backward (``csrc/sdpa_flash.cu``); nothing of size Tq x Tk is kept but the dropout bits"""
+    """head dim 64: one kernel forward, two backward, one up to 128 positions (``csrc/sdpa_flash.cu``); nothing of size Tq x Tk is kept but the dropout bits"""
 
     @staticmethod
     def forward(ctx, q, k, v, k_lens, H, causal, scale, p_drop):
@@ -174,7 +174,9 @@ class _FlashFn(torch.autograd.Function):
         o = torch.empty(B, Tq, H, D, dtype=torch.bfloat16, device=dev)
         lse = torch.empty(B * H * Tq, dtype=torch.float32, device=dev)
         # the backward pass takes row sums of the output: from a copy of its own in 32 bits, so that the caller may change the result in place
-        o32 = torch.empty(B, Tq, H, D, dtype=torch.float32, device=dev) if any(ctx.needs_input_grad[:3]) else None
+        # (the one kernel of short sequences takes them from the probabilities)
+        one = _lib.bind("rb200_flash_bwd_one_kernel", [_i32, _i32])(Tq, Tk)
+        o32 = torch.empty(B, Tq, H, D, dtype=torch.float32, device=dev) if any(ctx.needs_input_grad[:3]) and not one else None
         drop = p_drop > 0.0
         keep = seed = off = None
         if drop:
@@ -199,16 +201,16 @@ class _FlashFn(torch.autograd.Function):
         dev, bf = d_out.device, torch.bfloat16
         do2, rdo, hdo = _rows(d_out)
         geom = ctx.geom[:12] + (rdo, hdo) + ctx.geom[14:]
-        delta = torch.empty_like(lse)
+        delta = torch.empty_like(lse) if o32 is not None else None
         dq = torch.empty(B, Tq, H, 64, dtype=bf, device=dev)
         dk = torch.empty(B, Tk, H, 64, dtype=bf, device=dev)
         dv = torch.empty(B, Tk, H, 64, dtype=bf, device=dev)
         st = _gemm.status_tensor(dev)
         fn = _lib.bind("rb200_flash_bwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp])
-        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), o32.data_ptr(), do2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                      lse.data_ptr(), delta.data_ptr(), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), ctx.scale, ctx.p_drop, st.data_ptr(),
+        _lib.check(fn(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), _p(o32), do2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                      lse.data_ptr(), _p(delta), _p(keep), _p(k_lens), (_i32 * len(geom))(*geom), ctx.scale, ctx.p_drop, st.data_ptr(),
                       _lib.stream_ptr()), "flash_bwd")
-        _lib.count_launch(2)
+        _lib.count_launch(2 if o32 is not None else 1)
         dt = ctx.in_dtype
         return dq.to(dt), dk.to(dt), dv.to(dt), None, None, None, None, None
 
