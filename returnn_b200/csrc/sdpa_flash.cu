@@ -44,8 +44,98 @@ __device__ __forceinline__ int visible(const Flash& p, int i, int klen) {
   return max(n, 0);
 }
 
+// ---- life of a CTA: four warps of rows and one that issues -----------------------------------------------------------------------------
+// The warp behind the rows' four (one lane of it) issues loads and products; the rows' warps meet it at mbarriers and each other nowhere. Scores
+// are in registers as soon as they are read, so the products of the next tile run while the row work of this one does. With thread 0 issuing
+// between barriers of the whole CTA, a tile was product (1000 to 1400 cycles), row work, barrier (500), one after the other: 3600, 2800 and 4500
+// cycles in the three kernels.
+constexpr int kCta = kThreads + 32;
+
+struct Pipe {
+  Cta c;
+  uint64_t *scores, *out, *taken, *put;  // scores of a tile are there, products with P / dS are done; rows have taken the scores, put P / dS
+};
+template <uint32_t COLS>
+__device__ __forceinline__ Pipe pipe_begin(uint8_t* tail) {
+  Pipe p;
+  p.c.full = reinterpret_cast<uint64_t*>(tail);
+  p.c.extra = p.c.full + 2;
+  p.scores = p.c.full + 3;
+  p.c.done = p.out = p.c.full + 4;
+  p.taken = p.c.full + 5;
+  p.put = p.c.full + 6;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(p.c.full + 7);
+  p.c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 7; ++i) mbar_init(p.c.full + i, i >= 5 ? 4 : 1);
+    *p.c.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  p.c.tmem = *slot;
+  return p;
+}
+__device__ __forceinline__ bool pipe_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
+  const bool ok = wait_or_abort(p.c, bar, phase & 1, status, code);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return ok;
+}
+// a warp of rows is through with its accesses to tensor memory and shared memory (those to the latter made visible by each lane before)
+__device__ __forceinline__ void pipe_arrive(uint64_t* bar) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive_local(bar);
+}
+// all lanes of a warp of rows: the wait of one that gave up is the wait of all (the accesses to tensor memory are made by whole warps)
+__device__ __forceinline__ bool rows_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
+  return __all_sync(0xffffffffu, pipe_wait(p, bar, phase, status, code));
+}
+__device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+               ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+               "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+// The issuing lane, over n tiles: `load(t)` into stage t & 1 (its barrier: full[t & 1]), `first(t)` products that give scores, `second(t)` those with
+// what the rows have put. Tiles 0 and 1 are being loaded.
+template <typename Load, typename First, typename Second>
+__device__ __forceinline__ void pipe_issue(const Pipe& p, int n, int* status, Load load, First first, Second second) {
+  bool ok = pipe_wait(p, &p.c.full[0], 0, status, 1);
+  if (ok) {
+    first(0);
+    umma_commit(p.scores);
+  }
+  for (int t = 0; t < n && ok; ++t) {
+    if (t + 1 < n) {
+      ok = pipe_wait(p, p.taken, t, status, 2) && pipe_wait(p, &p.c.full[(t + 1) & 1], (t + 1) >> 1, status, 3);
+      if (!ok) break;
+      first(t + 1);
+      umma_commit(p.scores);
+    }
+    ok = pipe_wait(p, p.put, t, status, 4);
+    if (!ok) break;
+    second(t);
+    umma_commit(p.out);
+    if (t + 2 < n) {
+      ok = pipe_wait(p, p.out, t, status, 5);  // stage t & 1 has been read
+      if (ok) load(t + 2);
+    }
+  }
+}
+
+// The output stays in tensor memory: the maximum that P refers to grows only when a row's has grown by more than 2^8 (what its values are then, up to
+// 256, costs no precision), and only then a warp takes its rows of the output out, scales them and puts them back.
+constexpr float kSlack = 8.f;
+
 template <bool DROP>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kCta, 3)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                  const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_o32, const Flash p) {
   extern __shared__ uint8_t smem_raw[];
@@ -53,7 +143,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t* sk = sq + kBig;
   uint8_t* sv = sk + 2 * kSmall;
   uint8_t* sp = sv + 2 * kSmall;
-  const Cta c = cta_begin<128>(sp + kBig);
+  const Pipe w = pipe_begin<128>(sp + kBig);
+  const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
@@ -62,135 +153,136 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int q0 = (p.tiles - 1 - (int)(blockIdx.x / p.bh)) * kRows;
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
-  const int row = q0 + tid;
-  const int n = row < p.tq ? visible(p, row, klen) : 0;
   const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
-  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
   const uint32_t t_s = c.tmem, t_o = c.tmem + 64;
-  auto load_kv = [&](int t) {
-    const int s = t & 1;
-    tma_load_3d(sk + s * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[s]);
-    tma_load_3d(sv + s * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[s]);
-  };
-  bool ok = true;
-  if (tid == 0 && n_tiles > 0) {
-    mbar_expect_tx(&c.full[0], kBig + 2 * kSmall);
-    tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
-    load_kv(0);
-    if (n_tiles > 1) {
-      mbar_expect_tx(&c.full[1], 2 * kSmall);
-      load_kv(1);
-    }
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 1);
-    if (ok) {
-      mma64<false>(t_s, sq, sk, false);
-      umma_commit(c.done);
-    }
-  }
-  const float cs = p.scale * kLog2e;
-  const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
-  const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
-  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-  float m = -INFINITY, l = 0.f;
-  float acc[64];
+  if (tid == kThreads) {
+    auto load = [&](int t) {
+      const int st = t & 1;
+      mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? kBig : 0));
+      if (t == 0) tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
+      tma_load_3d(sk + st * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[st]);
+      tma_load_3d(sv + st * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[st]);
+    };
+    if (n_tiles > 0) load(0);
+    if (n_tiles > 1) load(1);
+    if (n_tiles > 0)
+      pipe_issue(w, n_tiles, p.status, load, [&](int t) { mma64<false>(t_s, sq, sk + (t & 1) * kSmall, false); },
+                 [&](int t) { mma64<true>(t_o, sp, sv + (t & 1) * kSmall, t > 0); });
+  } else if (tid < kThreads) {
+    const int row = q0 + tid;
+    const int n = row < p.tq ? visible(p, row, klen) : 0;
+    const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+    const float cs = p.scale * kLog2e;
+    const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
+    const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
+    const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int it = 0; it < n_tiles; ++it) {
+      ok = rows_wait(w, w.scores, it, p.status, 6);
+      if (!ok) break;
+      float s[64];
+      tmem_ld64(t_row, s);
+      pipe_arrive(w.taken);
+      const int left = n - it * kTile;  // visible keys of this row in this tile
+      float mx = -INFINITY;
+      if (__all_sync(0xffffffffu, left >= kTile)) {
 #pragma unroll
-  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
-  int it = 0;
-  for (; it < n_tiles; ++it) {
-    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 2);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {  // the products of the previous iteration are complete: its stage is free
-      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
-      load_kv(it + 1);
-    }
-    __syncwarp();
-    float s[64];
-    if (it > 0) {
-      tmem_ld64(t_row + 64, s);
+        for (int j = 0; j < 64; ++j) {
+          s[j] *= cs;
+          mx = fmaxf(mx, s[j]);
+        }
+      } else {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] += s[j];
-    }
-    tmem_ld64(t_row, s);
-    const int left = n - it * kTile;  // visible keys of this row in this tile
-    float mx = m;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      s[j] = j < left ? s[j] * cs : -INFINITY;
-      mx = fmaxf(mx, s[j]);
-    }
-    const float mu = mx == -INFINITY ? 0.f : mx;
-    const float corr = ex2(m - mu);
-    m = mx;
-    float sum = 0.f;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      s[j] = ex2(s[j] - mu);
-      sum += s[j];
-    }
-    l = l * corr + sum;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] *= corr;
-    if constexpr (DROP) {
-      const uint64_t base = off + ((uint64_t)z * p.tqp + row) * p.tkp + it * kTile;
-      uint32_t bits[2] = {0u, 0u};
-#pragma unroll
-      for (int j = 0; j < 64; j += 4) {
-        const uint64_t ctr = base + j;
-        const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x53u, 0u));
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool k = w[e] >= thresh;
-          s[j + e] = k ? s[j + e] * keep_scale : 0.f;
-          if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        for (int j = 0; j < 64; ++j) {
+          s[j] = j < left ? s[j] * cs : -INFINITY;
+          mx = fmaxf(mx, s[j]);
         }
       }
-      if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
-    }
-    store_row64(sp, tid, s);
-    fence_proxy_async_smem();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or(ok ? 0 : 1)) break;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      mma64<true>(t_o, sp, sv + (it & 1) * kSmall, false);
-      if (it + 1 < n_tiles) {
-        ok = wait_or_abort(c, &c.full[(it + 1) & 1], ((it + 1) >> 1) & 1, p.status, 3);
-        if (ok) mma64<false>(t_s, sq, sk + ((it + 1) & 1) * kSmall, false);
+      const bool grow = mx > m + kSlack;  // (also from -inf to anything)
+      bool read = it == 0;  // the products of the tile before are done
+      if (__any_sync(0xffffffffu, grow)) {
+        const float to = grow ? mx : m;
+        const float corr = grow ? ex2(m - to) : 1.f;
+        m = to;
+        l *= corr;
+        if (!read) {
+          ok = rows_wait(w, w.out, it - 1, p.status, 7);
+          if (!ok) break;
+          read = true;
+#pragma unroll 1
+          for (int part = 0; part < 4; ++part) {
+            uint32_t o[16];
+            tmem_ld16(t_row + 64 + 16 * part, o);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+            tmem_st16(t_row + 64 + 16 * part, o);
+          }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
       }
-      if (ok) umma_commit(c.done);
+      const float mu = m == -INFINITY ? 0.f : m;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) {
+        s[j] = ex2(s[j] - mu);
+        sum += s[j];
+      }
+      l += sum;
+      if constexpr (DROP) {
+        const uint64_t base = off + ((uint64_t)z * p.tqp + row) * p.tkp + it * kTile;
+        uint32_t bits[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 64; j += 4) {
+          const uint64_t ctr = base + j;
+          const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x53u, 0u));
+          const uint32_t x[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const bool k = x[e] >= thresh;
+            s[j + e] = k ? s[j + e] * keep_scale : 0.f;
+            if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+          }
+        }
+        if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
+      }
+      if (!read) {
+        ok = rows_wait(w, w.out, it - 1, p.status, 7);  // P of the tile before has been read
+        if (!ok) break;
+      }
+      store_row64(sp, tid, s);
+      fence_proxy_async_smem();
+      pipe_arrive(w.put);
     }
-  }
-  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 4);
-  if (!__syncthreads_or(ok ? 0 : 1)) {
-    if (n_tiles > 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 8);
+    if (ok) {
       float s[64];
-      tmem_ld64(t_row + 64, s);
+      if (n_tiles > 0) tmem_ld64(t_row + 64, s);
       const float inv = n > 0 ? 1.f / l : 0.f;
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] = n > 0 ? (acc[j] + s[j]) * inv : 0.f;
+      for (int j = 0; j < 64; ++j) s[j] = n > 0 ? s[j] * inv : 0.f;
+      store_row64(sq, tid, s);
+      if (p.save) store_row64_f32(sk, tid, s);  // the tiles of keys and values are not needed any more
+      if (row < p.tq) p.lse[(long long)z * p.tq + row] = n > 0 ? m + __log2f(l) : INFINITY;
+      fence_proxy_async_smem();
     }
-    store_row64(sq, tid, acc);
-    if (p.save) store_row64_f32(sk, tid, acc);  // the tiles of keys and values are not needed any more
-    if (row < p.tq) p.lse[(long long)z * p.tq + row] = n > 0 ? m + __log2f(l) : INFINITY;
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+    rows_sync();
+    if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_o, h * kTile, q0, b, sq);
       if (p.save) {
         tma_store_3d(&tm_o32, h * kTile, q0, b, sk);
         tma_store_3d(&tm_o32, h * kTile + 32, q0, b, sk + kBig);
       }
       tma_store_commit();
-      tma_store_wait_all();
+      tma_store_wait_read();  // (the writes complete like any other store of the grid)
     }
   }
   cta_end<128>(c);
 }
 
 template <bool DROP>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kCta, 2)
 flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_o32, const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
                    const Flash p) {
@@ -200,7 +292,8 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint8_t* sk = sdo + kBig;
   uint8_t* sv = sk + 2 * kSmall;
   uint8_t* sds = sv + 2 * kSmall;  // first, with the kBig bytes behind it, the tile of O in 32 bits
-  const Cta c = cta_begin<256>(sds + 2 * kBig);
+  const Pipe w = pipe_begin<256>(sds + 2 * kBig);
+  const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
@@ -208,111 +301,99 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const int q0 = (p.tiles - 1 - (int)(blockIdx.x / p.bh)) * kRows;
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
-  const int row = q0 + tid;
-  const int n = row < p.tq ? visible(p, row, klen) : 0;
   const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
-  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dq = c.tmem + 128;
-  auto load_kv = [&](int t) {
-    const int s = t & 1;
-    tma_load_3d(sk + s * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[s]);
-    tma_load_3d(sv + s * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[s]);
-  };
-  bool ok = true;
-  if (tid == 0 && n_tiles > 0) {
-    mbar_expect_tx(&c.full[0], 2 * kBig + 2 * kSmall);
-    tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
-    tma_load_3d(sdo, &tm_do, h * p.hdo, q0, b, &c.full[0]);
-    load_kv(0);
-    mbar_expect_tx(c.extra, 2 * kBig);
-    tma_load_3d(sds, &tm_o32, h * kTile, q0, b, c.extra);
-    tma_load_3d(sds + kBig, &tm_o32, h * kTile + 32, q0, b, c.extra);
-    if (n_tiles > 1) {
-      mbar_expect_tx(&c.full[1], 2 * kSmall);
-      load_kv(1);
-    }
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 5);
-    if (ok) {
-      mma64<false>(t_s, sq, sk, false);
-      mma64<false>(t_dp, sdo, sv, false);
-      umma_commit(c.done);
-    }
-  }
-  float lse = INFINITY, delta = 0.f;
-  if (n_tiles > 0) {
-    ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 6) && wait_or_abort(c, c.extra, 0, p.status, 6);
-    if (ok) {
-      delta = dot_row64(sds, sdo, tid);
-      if (row < p.tq) {
-        lse = p.lse[(long long)z * p.tq + row];
-        p.delta[(long long)z * p.tq + row] = delta;
+  if (tid == kThreads) {
+    auto load = [&](int t) {
+      const int st = t & 1;
+      mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? 2 * kBig : 0));
+      if (t == 0) {
+        tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
+        tma_load_3d(sdo, &tm_do, h * p.hdo, q0, b, &c.full[0]);
       }
-    }
-  }
-  const float cs = p.scale * kLog2e;
-  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-  int it = 0;
-  for (; it < n_tiles; ++it) {
-    uint2 bits = make_uint2(0u, 0u);
-    if (DROP && row < p.tq) bits = *reinterpret_cast<const uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2);
-    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 7);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
-      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
-      load_kv(it + 1);
-    }
-    __syncwarp();
-    float s[64], dp[64];
-    tmem_ld64(t_row, s);
-    tmem_ld64(t_row + 64, dp);
-    const int left = n - it * kTile;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      float d = dp[j];
-      if (DROP) d = (((j < 32 ? bits.x : bits.y) >> (j & 31)) & 1u) ? d * keep_scale : 0.f;
-      s[j] = j < left ? ex2(fmaf(s[j], cs, -lse)) * (d - delta) : 0.f;
-    }
-    store_row64(sds, tid, s);
-    fence_proxy_async_smem();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or(ok ? 0 : 1)) break;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      mma64<true>(t_dq, sds, sk + (it & 1) * kSmall, it > 0);
-      if (it + 1 < n_tiles) {
-        const int st = (it + 1) & 1;
-        ok = wait_or_abort(c, &c.full[st], ((it + 1) >> 1) & 1, p.status, 8);
-        if (ok) {
-          mma64<false>(t_s, sq, sk + st * kSmall, false);
-          mma64<false>(t_dp, sdo, sv + st * kSmall, false);
-        }
-      }
-      if (ok) umma_commit(c.done);
-    }
-  }
-  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 9);
-  if (!__syncthreads_or(ok ? 0 : 1)) {
-    float s[64];
+      tma_load_3d(sk + st * kSmall, &tm_k, h * p.hk, t * kTile, b, &c.full[st]);
+      tma_load_3d(sv + st * kSmall, &tm_v, h * p.hv, t * kTile, b, &c.full[st]);
+    };
     if (n_tiles > 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      tmem_ld64(t_row + 128, s);
+      load(0);
+      mbar_expect_tx(c.extra, 2 * kBig);
+      tma_load_3d(sds, &tm_o32, h * kTile, q0, b, c.extra);
+      tma_load_3d(sds + kBig, &tm_o32, h * kTile + 32, q0, b, c.extra);
+      if (n_tiles > 1) load(1);
+      pipe_issue(w, n_tiles, p.status, load,
+                 [&](int t) {
+                   mma64<false>(t_s, sq, sk + (t & 1) * kSmall, false);
+                   mma64<false>(t_dp, sdo, sv + (t & 1) * kSmall, false);
+                 },
+                 [&](int t) { mma64<true>(t_dq, sds, sk + (t & 1) * kSmall, t > 0); });
     }
+  } else if (tid < kThreads) {
+    const int row = q0 + tid;
+    const int n = row < p.tq ? visible(p, row, klen) : 0;
+    const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+    float lse = INFINITY, delta = 0.f;
+    bool ok = true;
+    if (n_tiles > 0) {
+      if (row < p.tq) lse = p.lse[(long long)z * p.tq + row];
+      ok = rows_wait(w, &c.full[0], 0, p.status, 9) && rows_wait(w, c.extra, 0, p.status, 9);
+      if (ok) {
+        delta = dot_row64(sds, sdo, tid);
+        if (row < p.tq) p.delta[(long long)z * p.tq + row] = delta;
+      }
+    }
+    const float cs = p.scale * kLog2e;
+    const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      uint2 bits = make_uint2(0u, 0u);
+      if (DROP && row < p.tq) bits = *reinterpret_cast<const uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2);
+      ok = rows_wait(w, w.scores, it, p.status, 10);
+      if (!ok) break;
+      float s[64], dp[64];
+      tmem_ld64(t_row, s);
+      tmem_ld64(t_row + 64, dp);
+      pipe_arrive(w.taken);
+      const int left = n - it * kTile;
+      auto grad = [&](int j) {
+        float d = dp[j];
+        if (DROP) d = (((j < 32 ? bits.x : bits.y) >> (j & 31)) & 1u) ? d * keep_scale : 0.f;
+        return ex2(fmaf(s[j], cs, -lse)) * (d - delta);
+      };
+      if (__all_sync(0xffffffffu, left >= kTile)) {
 #pragma unroll
-    for (int j = 0; j < 64; ++j) s[j] = n_tiles > 0 ? s[j] * p.scale : 0.f;
-    store_row64(sq, tid, s);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+        for (int j = 0; j < 64; ++j) s[j] = grad(j);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) s[j] = j < left ? grad(j) : 0.f;
+      }
+      if (it > 0) {
+        ok = rows_wait(w, w.out, it - 1, p.status, 11);  // dS of the tile before has been read
+        if (!ok) break;
+      }
+      store_row64(sds, tid, s);
+      fence_proxy_async_smem();
+      pipe_arrive(w.put);
+    }
+    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 12);
+    if (ok) {
+      float s[64];
+      if (n_tiles > 0) tmem_ld64(t_row + 128, s);
+#pragma unroll
+      for (int j = 0; j < 64; ++j) s[j] = n_tiles > 0 ? s[j] * p.scale : 0.f;
+      store_row64(sq, tid, s);
+      fence_proxy_async_smem();
+    }
+    rows_sync();
+    if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_dq, h * kTile, q0, b, sq);
       tma_store_commit();
-      tma_store_wait_all();
+      tma_store_wait_read();
     }
   }
   cta_end<256>(c);
 }
 
 template <bool DROP>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kCta, 2)
 flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                     const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                     const Flash p) {
@@ -323,9 +404,11 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint8_t* sdo = sq + 2 * kSmall;
   uint8_t* sp = sdo + 2 * kSmall;
   uint8_t* sds = sp + kBig;
-  float2* stat = reinterpret_cast<float2*>(sds + kBig);        // [2][64] (log-sum, delta) of the queries of a tile
-  uint4* kept = reinterpret_cast<uint4*>(sds + kBig + 1024);   // [2][64] dropout bits of this CTA's 128 keys
-  const Cta c = cta_begin<256>(sds + kBig + 1024 + 2048);
+  // per warp of rows: (log-sum, delta) of the 64 queries of a tile, and the dropout bits of the warp's 32 keys
+  float2* stat = reinterpret_cast<float2*>(sds + kBig) + (threadIdx.x >> 5) * 64;
+  uint32_t* kept = reinterpret_cast<uint32_t*>(sds + kBig + 2048) + (threadIdx.x >> 5) * 64;
+  const Pipe w = pipe_begin<256>(sds + kBig + 2048 + 1024);
+  const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
   const int tid = threadIdx.x;
@@ -333,124 +416,119 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int k0 = (int)(blockIdx.x / p.bh) * kRows;  // causal: the first keys have the most queries
   const int b = z / p.heads, h = z - b * p.heads;
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
-  const int key = k0 + tid;
   const int first = p.causal ? max(0, k0 - p.shift) / kTile : 0;  // queries before cannot see the first key of the tile
   const int n_tiles = k0 < klen ? max(0, (p.tq + kTile - 1) / kTile - first) : 0;
-  // queries that see this key: [lo, tq)
-  const int lo = key < klen ? (p.causal ? max(0, key - p.shift) : 0) : p.tq;
-  const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dv = c.tmem + 128, t_dk = c.tmem + 192;
-  auto load_q = [&](int t) {
-    const int s = t & 1;
-    tma_load_3d(sq + s * kSmall, &tm_q, h * p.hq, (first + t) * kTile, b, &c.full[s]);
-    tma_load_3d(sdo + s * kSmall, &tm_do, h * p.hdo, (first + t) * kTile, b, &c.full[s]);
-  };
-  auto load_stat = [&](int t) {
-    const int q = (first + t) * kTile + (tid & 63);
-    if (tid < 64) {
-      float2 v = make_float2(INFINITY, 0.f);
-      if (q < p.tq) v = make_float2(p.lse[(long long)z * p.tq + q], p.delta[(long long)z * p.tq + q]);
-      stat[(t & 1) * 64 + tid] = v;
-    } else if (DROP) {
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (q < p.tq) v = *reinterpret_cast<const uint4*>(p.keep + ((long long)z * p.tq + q) * p.words + k0 / 32);
-      kept[(t & 1) * 64 + (tid & 63)] = v;
-    }
-  };
-  bool ok = true;
-  if (n_tiles > 0) load_stat(0);
-  __syncthreads();
-  if (tid == 0 && n_tiles > 0) {
-    mbar_expect_tx(&c.full[0], 2 * kBig + 2 * kSmall);
-    tma_load_3d(sk, &tm_k, h * p.hk, k0, b, &c.full[0]);
-    tma_load_3d(sv, &tm_v, h * p.hv, k0, b, &c.full[0]);
-    load_q(0);
-    if (n_tiles > 1) {
-      mbar_expect_tx(&c.full[1], 2 * kSmall);
-      load_q(1);
-    }
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 10);
-    if (ok) {
-      mma64<false>(t_s, sk, sq, false);
-      mma64<false>(t_dp, sv, sdo, false);
-      umma_commit(c.done);
-    }
-  }
-  const float cs = p.scale * kLog2e;
-  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-  int it = 0;
-  for (; it < n_tiles; ++it) {
-    if (it + 1 < n_tiles) load_stat(it + 1);  // seen by all after this iteration's barrier
-    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 11);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
-      mbar_expect_tx(&c.full[(it + 1) & 1], 2 * kSmall);
-      load_q(it + 1);
-    }
-    __syncwarp();
-    float s[64], dp[64];
-    tmem_ld64(t_row, s);
-    tmem_ld64(t_row + 64, dp);
-    const int q_base = (first + it) * kTile;
-    const float2* st = stat + (it & 1) * 64;
-    const uint32_t* kp = reinterpret_cast<const uint32_t*>(kept + (it & 1) * 64) + (tid >> 5);
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      const float2 ld = st[j];
-      const bool vis = q_base + j >= lo && q_base + j < p.tq;
-      float pr = vis ? ex2(fmaf(s[j], cs, -ld.x)) : 0.f;
-      float d = dp[j];
-      float pd = pr;
-      if (DROP) {
-        const bool k = (kp[j * 4] >> (tid & 31)) & 1u;
-        d = k ? d * keep_scale : 0.f;
-        pd = k ? pr * keep_scale : 0.f;
+  if (tid == kThreads) {
+    auto load = [&](int t) {
+      const int st = t & 1;
+      mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? 2 * kBig : 0));
+      if (t == 0) {
+        tma_load_3d(sk, &tm_k, h * p.hk, k0, b, &c.full[0]);
+        tma_load_3d(sv, &tm_v, h * p.hv, k0, b, &c.full[0]);
       }
-      dp[j] = vis ? pr * (d - ld.y) : 0.f;
-      s[j] = pd;
-    }
-    store_row64(sp, tid, s);
-    store_row64(sds, tid, dp);
-    fence_proxy_async_smem();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or(ok ? 0 : 1)) break;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      mma64<true>(t_dv, sp, sdo + (it & 1) * kSmall, it > 0);
-      mma64<true>(t_dk, sds, sq + (it & 1) * kSmall, it > 0);
-      if (it + 1 < n_tiles) {
-        const int sn = (it + 1) & 1;
-        ok = wait_or_abort(c, &c.full[sn], ((it + 1) >> 1) & 1, p.status, 12);
-        if (ok) {
-          mma64<false>(t_s, sk, sq + sn * kSmall, false);
-          mma64<false>(t_dp, sv, sdo + sn * kSmall, false);
-        }
-      }
-      if (ok) umma_commit(c.done);
-    }
-  }
-  if (it == n_tiles && n_tiles > 0) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 13);
-  if (!__syncthreads_or(ok ? 0 : 1)) {
-    float s[64], dp[64];
+      tma_load_3d(sq + st * kSmall, &tm_q, h * p.hq, (first + t) * kTile, b, &c.full[st]);
+      tma_load_3d(sdo + st * kSmall, &tm_do, h * p.hdo, (first + t) * kTile, b, &c.full[st]);
+    };
     if (n_tiles > 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      tmem_ld64(t_row + 128, s);
-      tmem_ld64(t_row + 192, dp);
+      load(0);
+      if (n_tiles > 1) load(1);
+      pipe_issue(w, n_tiles, p.status, load,
+                 [&](int t) {
+                   mma64<false>(t_s, sk, sq + (t & 1) * kSmall, false);
+                   mma64<false>(t_dp, sv, sdo + (t & 1) * kSmall, false);
+                 },
+                 [&](int t) {
+                   mma64<true>(t_dv, sp, sdo + (t & 1) * kSmall, t > 0);
+                   mma64<true>(t_dk, sds, sq + (t & 1) * kSmall, t > 0);
+                 });
     }
+  } else if (tid < kThreads) {
+    const int key = k0 + tid, lane = tid & 31;
+    // queries that see this key: [lo, tq)
+    const int lo = key < klen ? (p.causal ? max(0, key - p.shift) : 0) : p.tq;
+    const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
+    const float cs = p.scale * kLog2e;
+    const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+    float2 ahead[2];     // of the queries lane and lane + 32 of the next tile
+    uint32_t bits[2];
+    auto fetch = [&](int t) {
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      s[j] = n_tiles > 0 ? s[j] : 0.f;
-      dp[j] = n_tiles > 0 ? dp[j] * p.scale : 0.f;
+      for (int e = 0; e < 2; ++e) {
+        const int q = (first + t) * kTile + lane + 32 * e;
+        const long long at = (long long)z * p.tq + q;
+        ahead[e] = q < p.tq ? make_float2(p.lse[at], p.delta[at]) : make_float2(INFINITY, 0.f);
+        if (DROP) bits[e] = q < p.tq ? p.keep[at * p.words + k0 / 32 + (tid >> 5)] : 0u;
+      }
+    };
+    if (n_tiles > 0) fetch(0);
+    bool ok = true;
+    for (int it = 0; it < n_tiles; ++it) {
+      __syncwarp();  // the statistics of the tile before have been read
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        stat[lane + 32 * e] = ahead[e];
+        if (DROP) kept[lane + 32 * e] = bits[e];
+      }
+      __syncwarp();
+      if (it + 1 < n_tiles) fetch(it + 1);
+      ok = rows_wait(w, w.scores, it, p.status, 13);
+      if (!ok) break;
+      float s[64], dp[64];
+      tmem_ld64(t_row, s);
+      tmem_ld64(t_row + 64, dp);
+      pipe_arrive(w.taken);
+      const int q_base = (first + it) * kTile;
+      auto both = [&](int j, bool vis) {
+        const float2 ld = stat[j];
+        float pr = ex2(fmaf(s[j], cs, -ld.x));
+        float d = dp[j], pd = pr;
+        if (DROP) {
+          const bool k = (kept[j] >> lane) & 1u;
+          d = k ? d * keep_scale : 0.f;
+          pd = k ? pr * keep_scale : 0.f;
+        }
+        dp[j] = vis ? pr * (d - ld.y) : 0.f;
+        s[j] = vis ? pd : 0.f;
+      };
+      if (__all_sync(0xffffffffu, q_base >= lo && q_base + kTile <= p.tq)) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) both(j, true);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) both(j, q_base + j >= lo && q_base + j < p.tq);
+      }
+      if (it > 0) {
+        ok = rows_wait(w, w.out, it - 1, p.status, 18);  // P and dS of the tile before have been read
+        if (!ok) break;
+      }
+      store_row64(sp, tid, s);
+      store_row64(sds, tid, dp);
+      fence_proxy_async_smem();
+      pipe_arrive(w.put);
     }
-    store_row64(sv, tid, s);
-    store_row64(sk, tid, dp);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 19);
+    if (ok) {
+      float s[64], dp[64];
+      if (n_tiles > 0) {
+        tmem_ld64(t_row + 128, s);
+        tmem_ld64(t_row + 192, dp);
+      }
+#pragma unroll
+      for (int j = 0; j < 64; ++j) {
+        s[j] = n_tiles > 0 ? s[j] : 0.f;
+        dp[j] = n_tiles > 0 ? dp[j] * p.scale : 0.f;
+      }
+      store_row64(sv, tid, s);
+      store_row64(sk, tid, dp);
+      fence_proxy_async_smem();
+    }
+    rows_sync();
+    if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_dv, h * kTile, k0, b, sv);
       tma_store_3d(&tm_dk, h * kTile, k0, b, sk);
       tma_store_commit();
-      tma_store_wait_all();
+      tma_store_wait_read();
     }
   }
   cta_end<256>(c);
@@ -634,7 +712,7 @@ flash_bwd_small_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 constexpr int kFwdSmem = 2 * kBig + 4 * kSmall + 64 + 1024;
 constexpr int kBwdQSmem = 4 * kBig + 4 * kSmall + 64 + 1024;
 constexpr int kBwdSmallSmem = 6 * kBig + 64 + 1024;
-constexpr int kBwdKvSmem = 4 * kBig + 4 * kSmall + 1024 + 2048 + 64 + 1024;
+constexpr int kBwdKvSmem = 4 * kBig + 4 * kSmall + 2048 + 1024 + 64 + 1024;
 
 int launch_failed(const char* what, cudaError_t e) {
   rb_set_error("%s: %s", what, cudaGetErrorString(e));
@@ -697,7 +775,7 @@ RB_EXPORT int rb200_flash_fwd(const void* q, const void* k, const void* v, void*
   auto kernel = p_drop > 0.f ? flash_fwd_kernel<true> : flash_fwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
   if (e != cudaSuccess) return launch_failed("flash_fwd", e);
-  rb_launch_pdl(kernel, dim3((unsigned)ctas), dim3(kThreads), kFwdSmem, stream, tq, tk, tv, to, to32, p);
+  rb_launch_pdl(kernel, dim3((unsigned)ctas), dim3(kCta), kFwdSmem, stream, tq, tk, tv, to, to32, p);
   return rb_check_launch("flash_fwd");
 }
 
@@ -753,7 +831,7 @@ RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdKvSmem);
   if (e != cudaSuccess) return launch_failed("flash_bwd", e);
   p.tiles = tiles_q;
-  rb_launch_pdl(kq, dim3((unsigned)(bh * tiles_q)), dim3(kThreads), kBwdQSmem, stream, tq, tk, tv, to, td, tg, p);
+  rb_launch_pdl(kq, dim3((unsigned)(bh * tiles_q)), dim3(kCta), kBwdQSmem, stream, tq, tk, tv, to, td, tg, p);
   st = rb_check_launch("flash_bwd_q");
   if (!st) st = map_of(&tq, q, g, p.tq, g[G_RQ], g[G_HQ], kTile);
   if (!st) st = map_of(&tk, k, g, p.tk, g[G_RK], g[G_HK], kRows);
@@ -763,6 +841,6 @@ RB_EXPORT int rb200_flash_bwd(const void* q, const void* k, const void* v, const
   if (!st) st = map_of(&tg2, dv, g, p.tk, hd, kTile, kRows);
   if (st) return st;
   p.tiles = tiles_k;
-  rb_launch_pdl(kkv, dim3((unsigned)(bh * tiles_k)), dim3(kThreads), kBwdKvSmem, stream, tq, tk, tv, td, tg, tg2, p);
+  rb_launch_pdl(kkv, dim3((unsigned)(bh * tiles_k)), dim3(kCta), kBwdKvSmem, stream, tq, tk, tv, td, tg, tg2, p);
   return rb_check_launch("flash_bwd_kv");
 }
