@@ -61,18 +61,21 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// (one lane of a converged warp, see umma_f16_warp)
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "n"(kDescHi)
       : "memory");
 }
 // arrive on the barrier at this offset in both CTAs once the pair's MMAs issued so far have completed
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
   const uint16_t mask = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask)
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "h"(mask)
                : "memory");
 }
 
@@ -157,33 +160,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   rb_pdl_launch();
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer (both CTAs) ----------------
-      const uint32_t full0 = map_to_cta(smem_u32(full_bar), 0);  // the leader's barriers collect both CTAs' bytes
-      uint32_t s = 0, ph = 0;
-      bool ok = true;
-      Walk w(p, pair);
-      rb_pdl_wait();
-      for (; w.more() && ok; w.next()) {
-        const int m0 = w.mi * BM + (int)rank * 128;
-        const int n0 = w.ni * BN + (int)rank * (BN / 2);
-        const int kb1 = w.kb1();
-        for (int kb = w.kb0(); kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag)) {
-            *abort_flag = 1;
-            if (g.status) atomicCAS(g.status, 0, (1 << 24) | (kb & 0xFFFFFF));
-            ok = false;
-            break;
-          }
-          uint8_t* sa = smem + s * kStageBytes;
-          uint8_t* sb = sa + kTileBytesA;
-          const uint32_t bar = full0 + s * 8;
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
-          // split operands: block kb belongs to hi*lo, lo*hi or hi*hi (columns of A past k read zeros, so the rows of B there do not
-          // count). The small products come first: additions to a large accumulator are what the tensor core rounds
-          const int seg = p.seg_kb ? kb / p.seg_kb : 0;
-          const int k0 = (kb - seg * p.seg_kb) * BK;
-          const int a_row = p.seg_kb && seg == 1 ? g.seg_a : 0, b_row = p.seg_kb && seg == 0 ? g.seg_b : 0;
+    // ---------------- TMA producer (both CTAs): the warp walks, one lane of it issues ----------------
+    const uint32_t full0 = map_to_cta(smem_u32(full_bar), 0);  // the leader's barriers collect both CTAs' bytes
+    uint32_t s = 0, ph = 0;
+    bool ok = true;
+    Walk w(p, pair);
+    rb_pdl_wait();
+    for (; w.more() && ok; w.next()) {
+      const int m0 = w.mi * BM + (int)rank * 128;
+      const int n0 = w.ni * BN + (int)rank * (BN / 2);
+      const int kb1 = w.kb1();
+      for (int kb = w.kb0(); kb < kb1; ++kb) {
+        if (!warp_wait(&empty_bar[s], ph ^ 1u, abort_flag)) {
+          *abort_flag = 1;
+          if (g.status && lane == 0) atomicCAS(g.status, 0, (1 << 24) | (kb & 0xFFFFFF));
+          ok = false;
+          break;
+        }
+        uint8_t* sa = smem + s * kStageBytes;
+        uint8_t* sb = sa + kTileBytesA;
+        const uint32_t bar = full0 + s * 8;
+        const bool issuer = elect_one();
+        if (issuer && leader) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
+        // split operands: block kb belongs to hi*lo, lo*hi or hi*hi (columns of A past k read zeros, so the rows of B there do not
+        // count). The small products come first: additions to a large accumulator are what the tensor core rounds
+        const int seg = p.seg_kb ? kb / p.seg_kb : 0;
+        const int k0 = (kb - seg * p.seg_kb) * BK;
+        const int a_row = p.seg_kb && seg == 1 ? g.seg_a : 0, b_row = p.seg_kb && seg == 0 ? g.seg_b : 0;
+        if (issuer) {
           if (!g.a_mn_major) {
             tma_load_2d_pair(sa, &tm_a, k0, a_row + m0, bar);
           } else {
@@ -196,47 +200,45 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * 8192, &tm_b, n0 + 64 * j, b_row + k0, bar);
           }
-          if (++s == kStages) {
-            s = 0;
-            ph ^= 1u;
-          }
+        }
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
-      // ---------------- MMA issuer (leader CTA only) ----------------
+    if (leader) {
+      // ---------------- MMA issuer (leader CTA only): the warp walks, one lane of it issues ----------------
       const uint32_t ab_fmt = g.ab_fp16 ? 0u : 1u;  // operand format field: 0 = fp16, 1 = bf16 (accumulator fp32 either way)
       const uint32_t idesc = (1u << 4) | (ab_fmt << 7) | (ab_fmt << 10) | ((uint32_t)(g.a_mn_major ? 1 : 0) << 15) |
                              ((uint32_t)(g.b_mn_major ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t a_lo = desc_lo(smem_u32(smem), g.a_mn_major ? 8192 : 16), b_lo = desc_lo(smem_u32(smem) + kTileBytesA, g.b_mn_major ? 8192 : 16);
+      const uint32_t a_step = g.a_mn_major ? 128 : 2, b_step = g.b_mn_major ? 128 : 2;  // 16 of the contraction, in units of 16 bytes
       uint32_t s = 0, ph = 0, t_local = 0;
       bool ok = true;
       for (Walk w(p, pair); w.more() && ok; w.next()) {
         const uint32_t buf = t_local & 1u;
-        if (!mbar_wait(&acc_empty[buf], ((t_local >> 1) & 1u) ^ 1u, abort_flag)) {
+        if (!warp_wait(&acc_empty[buf], ((t_local >> 1) & 1u) ^ 1u, abort_flag)) {
           *abort_flag = 1;
-          if (g.status) atomicCAS(g.status, 0, (4 << 24) | (w.u & 0xFFFFFF));
+          if (g.status && lane == 0) atomicCAS(g.status, 0, (4 << 24) | (w.u & 0xFFFFFF));
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + buf * BN;
         const int kb0 = w.kb0(), kb1 = w.kb1();
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[s], ph, abort_flag)) {
+          if (!warp_wait(&full_bar[s], ph, abort_flag)) {
             *abort_flag = 1;
-            if (g.status) atomicCAS(g.status, 0, (2 << 24) | (kb & 0xFFFFFF));
+            if (g.status && lane == 0) atomicCAS(g.status, 0, (2 << 24) | (kb & 0xFFFFFF));
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sa = smem_u32(smem + s * kStageBytes);
-          const uint32_t sb = sa + kTileBytesA;
+          const uint32_t a = a_lo + s * (kStageBytes >> 4), b = b_lo + s * (kStageBytes >> 4);
+          umma_f16_pair(d_tmem, a, b, idesc, kb > kb0 ? 1u : 0u);
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t adesc = g.a_mn_major ? make_desc(sa + kk * 2048, 8192, 1024) : make_desc(sa + kk * 32, 16, 1024);
-            const uint64_t bdesc = g.b_mn_major ? make_desc(sb + kk * 2048, 8192, 1024) : make_desc(sb + kk * 32, 16, 1024);
-            umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 1; kk < BK / 16; ++kk) umma_f16_pair(d_tmem, a + kk * a_step, b + kk * b_step, idesc, 1u);
           umma_commit_pair(&empty_bar[s]);
           if (++s == kStages) {
             s = 0;

@@ -45,7 +45,7 @@ __device__ __forceinline__ int visible(const Flash& p, int i, int klen) {
 }
 
 // ---- life of a CTA: four warps of rows and one that issues -----------------------------------------------------------------------------
-// The warp behind the rows' four (one lane of it) issues loads and products; the rows' warps meet it at mbarriers and each other nowhere. Scores
+// The warp behind the rows' four issues loads and products; the rows' warps meet it at mbarriers and each other nowhere. Scores
 // are in registers as soon as they are read, so the products of the next tile run while the row work of this one does. With thread 0 issuing
 // between barriers of the whole CTA, a tile was product (1000 to 1400 cycles), row work, barrier (500), one after the other: 3600, 2800 and 4500
 // cycles in the three kernels.
@@ -81,20 +81,26 @@ __device__ __forceinline__ Pipe pipe_begin(uint8_t* tail) {
   p.c.tmem = *slot;
   return p;
 }
+// all lanes of a warp: the wait of one that gave up is the wait of all
 __device__ __forceinline__ bool pipe_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
-  const bool ok = wait_or_abort(p.c, bar, phase & 1, status, code);
+  const bool ok = __all_sync(0xffffffffu, wait_or_abort(p.c, bar, phase & 1, status, code));
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return ok;
+}
+// D[128, 64] (+)= A[128, 64] B as mma64, by one lane of a converged warp
+template <bool B_MN>
+__device__ __forceinline__ void mma64_warp(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  const uint32_t da = desc_lo(smem_u32(a), 16), db = desc_lo(smem_u32(b), B_MN ? 8192 : 16);
+  umma_f16_warp(d, da, db, idesc, accumulate ? 1u : 0u);
+#pragma unroll
+  for (int kk = 1; kk < 4; ++kk) umma_f16_warp(d, da + 2 * kk, db + (B_MN ? 128 : 2) * kk, idesc, 1u);
 }
 // a warp of rows is through with its accesses to tensor memory and shared memory (those to the latter made visible by each lane before)
 __device__ __forceinline__ void pipe_arrive(uint64_t* bar) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive_local(bar);
-}
-// all lanes of a warp of rows: the wait of one that gave up is the wait of all (the accesses to tensor memory are made by whole warps)
-__device__ __forceinline__ bool rows_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
-  return __all_sync(0xffffffffu, pipe_wait(p, bar, phase, status, code));
 }
 __device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* r) {
@@ -103,26 +109,26 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* r) {
                "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
 }
-// The issuing lane, over n tiles: `load(t)` into stage t & 1 (its barrier: full[t & 1]), `first(t)` products that give scores, `second(t)` those with
+// The issuing warp, over n tiles: `load(t)` into stage t & 1 (its barrier: full[t & 1]), `first(t)` products that give scores, `second(t)` those with
 // what the rows have put. Tiles 0 and 1 are being loaded.
 template <typename Load, typename First, typename Second>
 __device__ __forceinline__ void pipe_issue(const Pipe& p, int n, int* status, Load load, First first, Second second) {
   bool ok = pipe_wait(p, &p.c.full[0], 0, status, 1);
   if (ok) {
     first(0);
-    umma_commit(p.scores);
+    umma_commit_warp(p.scores);
   }
   for (int t = 0; t < n && ok; ++t) {
     if (t + 1 < n) {
       ok = pipe_wait(p, p.taken, t, status, 2) && pipe_wait(p, &p.c.full[(t + 1) & 1], (t + 1) >> 1, status, 3);
       if (!ok) break;
       first(t + 1);
-      umma_commit(p.scores);
+      umma_commit_warp(p.scores);
     }
     ok = pipe_wait(p, p.put, t, status, 4);
     if (!ok) break;
     second(t);
-    umma_commit(p.out);
+    umma_commit_warp(p.out);
     if (t + 2 < n) {
       ok = pipe_wait(p, p.out, t, status, 5);  // stage t & 1 has been read
       if (ok) load(t + 2);
@@ -155,8 +161,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
   const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
   const uint32_t t_s = c.tmem, t_o = c.tmem + 64;
-  if (tid == kThreads) {
+  if (tid >= kThreads) {
     auto load = [&](int t) {
+      if (!elect_one()) return;
       const int st = t & 1;
       mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? kBig : 0));
       if (t == 0) tma_load_3d(sq, &tm_q, h * p.hq, q0, b, &c.full[0]);
@@ -166,9 +173,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (n_tiles > 0) load(0);
     if (n_tiles > 1) load(1);
     if (n_tiles > 0)
-      pipe_issue(w, n_tiles, p.status, load, [&](int t) { mma64<false>(t_s, sq, sk + (t & 1) * kSmall, false); },
-                 [&](int t) { mma64<true>(t_o, sp, sv + (t & 1) * kSmall, t > 0); });
-  } else if (tid < kThreads) {
+      pipe_issue(w, n_tiles, p.status, load, [&](int t) { mma64_warp<false>(t_s, sq, sk + (t & 1) * kSmall, false); },
+                 [&](int t) { mma64_warp<true>(t_o, sp, sv + (t & 1) * kSmall, t > 0); });
+  } else {
     const int row = q0 + tid;
     const int n = row < p.tq ? visible(p, row, klen) : 0;
     const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
@@ -179,7 +186,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
-      ok = rows_wait(w, w.scores, it, p.status, 6);
+      ok = pipe_wait(w, w.scores, it, p.status, 6);
       if (!ok) break;
       float s[64];
       tmem_ld64(t_row, s);
@@ -207,7 +214,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         m = to;
         l *= corr;
         if (!read) {
-          ok = rows_wait(w, w.out, it - 1, p.status, 7);
+          ok = pipe_wait(w, w.out, it - 1, p.status, 7);
           if (!ok) break;
           read = true;
 #pragma unroll 1
@@ -248,14 +255,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
       }
       if (!read) {
-        ok = rows_wait(w, w.out, it - 1, p.status, 7);  // P of the tile before has been read
+        ok = pipe_wait(w, w.out, it - 1, p.status, 7);  // P of the tile before has been read
         if (!ok) break;
       }
       store_row64(sp, tid, s);
       fence_proxy_async_smem();
       pipe_arrive(w.put);
     }
-    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 8);
+    if (ok && n_tiles > 0) ok = pipe_wait(w, w.out, n_tiles - 1, p.status, 8);
     if (ok) {
       float s[64];
       if (n_tiles > 0) tmem_ld64(t_row + 64, s);
@@ -303,8 +310,9 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const int klen = p.k_lens ? min(p.k_lens[b], p.tk) : p.tk;
   const int n_tiles = (visible(p, min(q0 + kRows, p.tq) - 1, klen) + kTile - 1) / kTile;
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dq = c.tmem + 128;
-  if (tid == kThreads) {
+  if (tid >= kThreads) {
     auto load = [&](int t) {
+      if (!elect_one()) return;
       const int st = t & 1;
       mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? 2 * kBig : 0));
       if (t == 0) {
@@ -316,18 +324,20 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     };
     if (n_tiles > 0) {
       load(0);
-      mbar_expect_tx(c.extra, 2 * kBig);
-      tma_load_3d(sds, &tm_o32, h * kTile, q0, b, c.extra);
-      tma_load_3d(sds + kBig, &tm_o32, h * kTile + 32, q0, b, c.extra);
+      if (elect_one()) {
+        mbar_expect_tx(c.extra, 2 * kBig);
+        tma_load_3d(sds, &tm_o32, h * kTile, q0, b, c.extra);
+        tma_load_3d(sds + kBig, &tm_o32, h * kTile + 32, q0, b, c.extra);
+      }
       if (n_tiles > 1) load(1);
       pipe_issue(w, n_tiles, p.status, load,
                  [&](int t) {
-                   mma64<false>(t_s, sq, sk + (t & 1) * kSmall, false);
-                   mma64<false>(t_dp, sdo, sv + (t & 1) * kSmall, false);
+                   mma64_warp<false>(t_s, sq, sk + (t & 1) * kSmall, false);
+                   mma64_warp<false>(t_dp, sdo, sv + (t & 1) * kSmall, false);
                  },
-                 [&](int t) { mma64<true>(t_dq, sds, sk + (t & 1) * kSmall, t > 0); });
+                 [&](int t) { mma64_warp<true>(t_dq, sds, sk + (t & 1) * kSmall, t > 0); });
     }
-  } else if (tid < kThreads) {
+  } else {
     const int row = q0 + tid;
     const int n = row < p.tq ? visible(p, row, klen) : 0;
     const uint32_t t_row = c.tmem + ((uint32_t)(tid & ~31) << 16);
@@ -335,7 +345,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
     if (n_tiles > 0) {
       if (row < p.tq) lse = p.lse[(long long)z * p.tq + row];
-      ok = rows_wait(w, &c.full[0], 0, p.status, 9) && rows_wait(w, c.extra, 0, p.status, 9);
+      ok = pipe_wait(w, &c.full[0], 0, p.status, 9) && pipe_wait(w, c.extra, 0, p.status, 9);
       if (ok) {
         delta = dot_row64(sds, sdo, tid);
         if (row < p.tq) p.delta[(long long)z * p.tq + row] = delta;
@@ -346,7 +356,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int it = 0; it < n_tiles && ok; ++it) {
       uint2 bits = make_uint2(0u, 0u);
       if (DROP && row < p.tq) bits = *reinterpret_cast<const uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2);
-      ok = rows_wait(w, w.scores, it, p.status, 10);
+      ok = pipe_wait(w, w.scores, it, p.status, 10);
       if (!ok) break;
       float s[64], dp[64];
       tmem_ld64(t_row, s);
@@ -366,14 +376,14 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int j = 0; j < 64; ++j) s[j] = j < left ? grad(j) : 0.f;
       }
       if (it > 0) {
-        ok = rows_wait(w, w.out, it - 1, p.status, 11);  // dS of the tile before has been read
+        ok = pipe_wait(w, w.out, it - 1, p.status, 11);  // dS of the tile before has been read
         if (!ok) break;
       }
       store_row64(sds, tid, s);
       fence_proxy_async_smem();
       pipe_arrive(w.put);
     }
-    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 12);
+    if (ok && n_tiles > 0) ok = pipe_wait(w, w.out, n_tiles - 1, p.status, 12);
     if (ok) {
       float s[64];
       if (n_tiles > 0) tmem_ld64(t_row + 128, s);
@@ -419,8 +429,9 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int first = p.causal ? max(0, k0 - p.shift) / kTile : 0;  // queries before cannot see the first key of the tile
   const int n_tiles = k0 < klen ? max(0, (p.tq + kTile - 1) / kTile - first) : 0;
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_dv = c.tmem + 128, t_dk = c.tmem + 192;
-  if (tid == kThreads) {
+  if (tid >= kThreads) {
     auto load = [&](int t) {
+      if (!elect_one()) return;
       const int st = t & 1;
       mbar_expect_tx(&c.full[st], 2 * kSmall + (t == 0 ? 2 * kBig : 0));
       if (t == 0) {
@@ -435,15 +446,15 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (n_tiles > 1) load(1);
       pipe_issue(w, n_tiles, p.status, load,
                  [&](int t) {
-                   mma64<false>(t_s, sk, sq + (t & 1) * kSmall, false);
-                   mma64<false>(t_dp, sv, sdo + (t & 1) * kSmall, false);
+                   mma64_warp<false>(t_s, sk, sq + (t & 1) * kSmall, false);
+                   mma64_warp<false>(t_dp, sv, sdo + (t & 1) * kSmall, false);
                  },
                  [&](int t) {
-                   mma64<true>(t_dv, sp, sdo + (t & 1) * kSmall, t > 0);
-                   mma64<true>(t_dk, sds, sq + (t & 1) * kSmall, t > 0);
+                   mma64_warp<true>(t_dv, sp, sdo + (t & 1) * kSmall, t > 0);
+                   mma64_warp<true>(t_dk, sds, sq + (t & 1) * kSmall, t > 0);
                  });
     }
-  } else if (tid < kThreads) {
+  } else {
     const int key = k0 + tid, lane = tid & 31;
     // queries that see this key: [lo, tq)
     const int lo = key < klen ? (p.causal ? max(0, key - p.shift) : 0) : p.tq;
@@ -472,7 +483,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       __syncwarp();
       if (it + 1 < n_tiles) fetch(it + 1);
-      ok = rows_wait(w, w.scores, it, p.status, 13);
+      ok = pipe_wait(w, w.scores, it, p.status, 13);
       if (!ok) break;
       float s[64], dp[64];
       tmem_ld64(t_row, s);
@@ -499,7 +510,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int j = 0; j < 64; ++j) both(j, q_base + j >= lo && q_base + j < p.tq);
       }
       if (it > 0) {
-        ok = rows_wait(w, w.out, it - 1, p.status, 18);  // P and dS of the tile before have been read
+        ok = pipe_wait(w, w.out, it - 1, p.status, 18);  // P and dS of the tile before have been read
         if (!ok) break;
       }
       store_row64(sp, tid, s);
@@ -507,7 +518,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       fence_proxy_async_smem();
       pipe_arrive(w.put);
     }
-    if (ok && n_tiles > 0) ok = rows_wait(w, w.out, n_tiles - 1, p.status, 19);
+    if (ok && n_tiles > 0) ok = pipe_wait(w, w.out, n_tiles - 1, p.status, 19);
     if (ok) {
       float s[64], dp[64];
       if (n_tiles > 0) {
