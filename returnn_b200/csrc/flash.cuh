@@ -141,4 +141,109 @@ __device__ __forceinline__ bool wait_or_abort(const Cta& c, uint64_t* bar, uint3
   return ok;
 }
 
+// ---- life of a CTA with warps of rows and one that issues ---------------------------------------------------------------------------
+// The warp behind those of the rows issues loads and products; the rows' warps meet it at mbarriers and each other nowhere. Scores
+// are in registers as soon as they are read, so the products of the next tile run while the row work of this one does. With thread 0 issuing
+// between barriers of the whole CTA, a tile was product (1000 to 1400 cycles), row work, barrier (500), one after the other: 3600, 2800 and 4500
+// cycles in the three kernels.
+struct Pipe {
+  Cta c;
+  uint64_t *scores, *out, *taken, *put;  // scores of a tile are there, products with P / dS are done; rows have taken the scores, put P / dS
+};
+// WARPS: of rows; OUT: arrivals that complete a phase of `out`
+template <uint32_t COLS, int WARPS, int OUT = 1>
+__device__ __forceinline__ Pipe pipe_begin(uint8_t* tail) {
+  Pipe p;
+  p.c.full = reinterpret_cast<uint64_t*>(tail);
+  p.c.extra = p.c.full + 2;
+  p.scores = p.c.full + 3;
+  p.c.done = p.out = p.c.full + 4;
+  p.taken = p.c.full + 5;
+  p.put = p.c.full + 6;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(p.c.full + 7);
+  p.c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 7; ++i) mbar_init(p.c.full + i, i >= 5 ? WARPS : i == 4 ? OUT : 1);
+    *p.c.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  p.c.tmem = *slot;
+  return p;
+}
+// all lanes of a warp: the wait of one that gave up is the wait of all
+__device__ __forceinline__ bool pipe_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
+  const bool ok = __all_sync(0xffffffffu, wait_or_abort(p.c, bar, phase & 1, status, code));
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return ok;
+}
+// D[128, 64] (+)= A[128, 64] B as mma64, by one lane of a converged warp
+template <bool B_MN>
+__device__ __forceinline__ void mma64_warp(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  const uint32_t da = desc_lo(smem_u32(a), 16), db = desc_lo(smem_u32(b), B_MN ? 8192 : 16);
+  umma_f16_warp(d, da, db, idesc, accumulate ? 1u : 0u);
+#pragma unroll
+  for (int kk = 1; kk < 4; ++kk) umma_f16_warp(d, da + 2 * kk, db + (B_MN ? 128 : 2) * kk, idesc, 1u);
+}
+// a warp of rows is through with its accesses to tensor memory and shared memory (those to the latter made visible by each lane before)
+__device__ __forceinline__ void pipe_arrive(uint64_t* bar) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive_local(bar);
+}
+template <int THREADS>
+__device__ __forceinline__ void rows_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
+// The issuing warp, over n tiles: `load(t)` into stage t & 1 (its barrier: full[t & 1]), `first(t)` products that give scores, `second(t)` those with
+// what the rows have put, `after(t)` what else is to be done with that. Tiles 0 and 1 are being loaded.
+template <typename Load, typename First, typename Second, typename After>
+__device__ __forceinline__ void pipe_issue(const Pipe& p, int n, int* status, Load load, First first, Second second, After after) {
+  bool ok = pipe_wait(p, &p.c.full[0], 0, status, 1);
+  if (ok) {
+    first(0);
+    umma_commit_warp(p.scores);
+  }
+  for (int t = 0; t < n && ok; ++t) {
+    if (t + 1 < n) {
+      ok = pipe_wait(p, p.taken, t, status, 2) && pipe_wait(p, &p.c.full[(t + 1) & 1], (t + 1) >> 1, status, 3);
+      if (!ok) break;
+      first(t + 1);
+      umma_commit_warp(p.scores);
+    }
+    ok = pipe_wait(p, p.put, t, status, 4);
+    if (!ok) break;
+    second(t);
+    umma_commit_warp(p.out);
+    after(t);
+    if (t + 2 < n) {
+      ok = pipe_wait(p, p.out, t, status, 5);  // stage t & 1 has been read
+      if (ok) load(t + 2);
+    }
+  }
+}
+
+// The output of a forward pass stays in tensor memory: the maximum that P refers to grows only when a row's has grown by more than 2^kSlack (what its
+// values are then, up to 256, costs no precision), and only then a warp takes its rows of the output out, scales them and puts them back.
+constexpr float kSlack = 8.f;
+__device__ __forceinline__ void tmem_scale64(uint32_t addr, float factor) {
+#pragma unroll 1
+  for (int part = 0; part < 4; ++part) {
+    uint32_t o[16];
+    tmem_ld16(addr + 16 * part, o);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * factor);
+    tmem_st16(addr + 16 * part, o);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 }  // namespace rbf

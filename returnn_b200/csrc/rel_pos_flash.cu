@@ -17,6 +17,12 @@
 //            traffic and twelve small products instead of four, and 58 us of fills (a pass at 36 x 333 frames, 8 heads: 403 -> 343 us). The margins of the band, and
 //            the rows of tiles without a valid query, are zeros that this kernel writes while its first loads are under way.
 // What went through memory before: scores and position band written and read in both passes, probabilities, dP.
+//
+// Both are bound by the row work (window reads, shifts, exponentials: issue slots of the eight row warps). Loads, products and bulk stores are issued by
+// a ninth warp, which meets the rows at mbarriers only: with one of the row threads issuing, all 256 waited for it at block barriers, four times a
+// tile. The outputs stay in tensor memory and are rescaled only when a row's maximum grows by more than 2^8 (see kSlack). Kernels within the
+// backward pass of 6912 rows: rel_bwd 98.3 -> 87.3 us; passes alone, forward 36 x 333 frames, 8 heads 92.0 -> 85.9 us, with gradients 323 -> 307
+// (products of dV, dK and positions included), 20 x 500 frames 305 -> 276, 300 x 40 frames 445 -> 407.
 #include "flash.cuh"
 #include "gemm.h"
 
@@ -24,7 +30,8 @@ using namespace rbf;
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;        // rows: two groups of 128
+constexpr int kCta = kThreads + 32;  // and the warp that issues (see Pipe)
 
 struct Rel {
   const int* lens;
@@ -43,9 +50,9 @@ struct Rel {
 template <uint32_t N>
 __device__ __forceinline__ void mma_n(uint32_t d, const uint8_t* a, const uint8_t* b) {  // D[128, N] = A[128, 64] B[N, 64]^T, both K-major
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+  const uint32_t da = desc_lo(smem_u32(a), 16), db = desc_lo(smem_u32(b), 16);
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) umma_f16(d, make_desc(sa + kk * 32, 16, 1024), make_desc(sb + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
+  for (int kk = 0; kk < 4; ++kk) umma_f16_warp(d, da + 2 * kk, db + 2 * kk, idesc, kk > 0 ? 1u : 0u);
 }
 
 // g[j] <- g[j + shift] for j < N, shift in [0, 31]; g holds N + 31 values
@@ -67,7 +74,7 @@ __device__ __forceinline__ void shift_down(float* g, int shift) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 template <bool DROP>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kCta, 1)
 rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant__ CUtensorMap tm_qv, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_pos, const __grid_constant__ CUtensorMap tm_o,
                const Rel p) {
@@ -85,161 +92,153 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* sv = sk + 2 * kBig;     // [2][128 keys]
   uint8_t* spos = sv + 2 * kBig;   // [2][256 positions]
   uint8_t* sp = spos + 4 * kBig;   // [2 groups][128 queries][64 keys]
-  const Cta c = cta_begin<512>(sp + 2 * kBig);
+  const Pipe w = pipe_begin<512, 8>(sp + 2 * kBig);
+  const Cta& c = w.c;
   const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
-  const int row = q0 + r;
   const int n_tiles = (len + 127) / 128;
-  const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
   const uint32_t t_s = c.tmem, t_g = c.tmem + 128, t_o = c.tmem + 384;
-  auto load = [&](int t) {
-    const int s = t & 1;
-    tma_load_3d(sk + s * kBig, &tm_k, h * 64, t * 128, b, &c.full[s]);
-    tma_load_3d(sv + s * kBig, &tm_v, h * 64, t * 128, b, &c.full[s]);
-    tma_load_2d(spos + s * 2 * kBig, &tm_pos, h * 64, p.center + t * 128 - q0 - 127, &c.full[s]);
-  };
-  auto scores = [&](int s) {
-    mma_n<128>(t_s, squ, sk + s * kBig);
-    mma_n<256>(t_g, sqv, spos + s * 2 * kBig);
-  };
-  bool ok = true;
-  if (tid == 0) {
-    mbar_expect_tx(&c.full[0], 6 * kBig);
-    tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
-    tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
-    load(0);
-    if (n_tiles > 1) {
-      mbar_expect_tx(&c.full[1], 4 * kBig);
-      load(1);
-    }
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 21);
-    if (ok) {
-      scores(0);
-      umma_commit(c.done);
-    }
-  }
-  const float cs = p.scale * kLog2e;
-  const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
-  const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
-  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-  float m = -INFINITY, l = 0.f;
-  float acc[64];
-#pragma unroll
-  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
-  int it = 0;
-  for (; it < n_tiles; ++it) {
-    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 22);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
-      mbar_expect_tx(&c.full[(it + 1) & 1], 4 * kBig);
-      load(it + 1);
-    }
-    __syncwarp();
-    float s[96];
-    uint32_t* raw = reinterpret_cast<uint32_t*>(s);
-    if (it > 0) {
-      tmem_ld64(t_o + t_lane + wg * 64, s);
-#pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] += s[j];
-    }
-    // the position scores of this warp's rows: 95 columns from 127 - (its last row) + 64 * group on
-    const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 64);
-    tmem_ld32(g0, raw);
-    tmem_ld32(g0 + 32, raw + 32);
-    tmem_ld32(g0 + 64, raw + 64);
-    tmem_wait_ld();
-    shift_down<64>(s, 31 - lane);
-    const int left = len - (it * 128 + wg * 64);  // keys of this group's half that exist
-    float mx = m;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float a[32];
-      tmem_ld32(t_s + t_lane + wg * 64 + half * 32, reinterpret_cast<uint32_t*>(a));
-      tmem_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int jj = half * 32 + j;
-        s[jj] = jj < left ? (a[j] + s[jj]) * cs : -INFINITY;
-        mx = fmaxf(mx, s[jj]);
+  if (tid >= kThreads) {
+    auto load = [&](int t) {
+      if (!elect_one()) return;
+      const int s = t & 1;
+      mbar_expect_tx(&c.full[s], (t == 0 ? 6 : 4) * kBig);
+      if (t == 0) {
+        tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
+        tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
       }
-    }
-    const float mu = mx == -INFINITY ? 0.f : mx;
-    const float corr = ex2(m - mu);
-    m = mx;
-    float sum = 0.f;
+      tma_load_3d(sk + s * kBig, &tm_k, h * 64, t * 128, b, &c.full[s]);
+      tma_load_3d(sv + s * kBig, &tm_v, h * 64, t * 128, b, &c.full[s]);
+      tma_load_2d(spos + s * 2 * kBig, &tm_pos, h * 64, p.center + t * 128 - q0 - 127, &c.full[s]);
+    };
+    load(0);
+    if (n_tiles > 1) load(1);
+    pipe_issue(w, n_tiles, p.status, load,
+               [&](int t) {
+                 mma_n<128>(t_s, squ, sk + (t & 1) * kBig);
+                 mma_n<256>(t_g, sqv, spos + (t & 1) * 2 * kBig);
+               },
+               [&](int t) {
+                 const uint8_t* v = sv + (t & 1) * kBig;
+                 mma64_warp<true>(t_o, sp, v, t > 0);
+                 mma64_warp<true>(t_o + 64, sp + kBig, v + kSmall, t > 0);
+               },
+               [](int) {});
+  } else {
+    const int row = q0 + r;
+    const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
+    const float cs = p.scale * kLog2e;
+    const uint64_t sd = DROP ? (uint64_t)p.seed[0] : 0, off = DROP ? (uint64_t)p.offset[0] : 0;
+    const uint32_t thresh = DROP ? (uint32_t)(p.p_drop * 4294967296.0) : 0u;
+    const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int it = 0; it < n_tiles; ++it) {
+      ok = pipe_wait(w, w.scores, it, p.status, 22);
+      if (!ok) break;
+      float s[96];
+      uint32_t* raw = reinterpret_cast<uint32_t*>(s);
+      // the position scores of this warp's rows: 95 columns from 127 - (its last row) + 64 * group on
+      const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 64);
+      tmem_ld32(g0, raw);
+      tmem_ld32(g0 + 32, raw + 32);
+      tmem_ld32(g0 + 64, raw + 64);
+      tmem_wait_ld();
+      shift_down<64>(s, 31 - lane);
+      const int left = len - (it * 128 + wg * 64);  // keys of this group's half that exist
+      float mx = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      s[j] = ex2(s[j] - mu);
-      sum += s[j];
-    }
-    l = l * corr + sum;
+      for (int half = 0; half < 2; ++half) {
+        float a[32];
+        tmem_ld32(t_s + t_lane + wg * 64 + half * 32, reinterpret_cast<uint32_t*>(a));
+        tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] *= corr;
-    if constexpr (DROP) {
-      const uint64_t base = off + ((uint64_t)z * p.lp + row) * p.lp + it * 128 + wg * 64;
-      uint32_t bits[2] = {0u, 0u};
-#pragma unroll
-      for (int j = 0; j < 64; j += 4) {
-        const uint64_t ctr = base + j;
-        const uint4 x = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x52u, 0u));
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool k = w[e] >= thresh;
-          s[j + e] = k ? s[j + e] * keep_scale : 0.f;
-          if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        for (int j = 0; j < 32; ++j) {
+          const int jj = half * 32 + j;
+          s[jj] = jj < left ? (a[j] + s[jj]) * cs : -INFINITY;
+          mx = fmaxf(mx, s[jj]);
         }
       }
-      if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
-    }
-    store_row64(sp + wg * kBig, r, s);
-    fence_proxy_async_smem();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or(ok ? 0 : 1)) break;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint8_t* v = sv + (it & 1) * kBig;
-      mma64<true>(t_o, sp, v, false);
-      mma64<true>(t_o + 64, sp + kBig, v + kSmall, false);
-      if (it + 1 < n_tiles) {
-        ok = wait_or_abort(c, &c.full[(it + 1) & 1], ((it + 1) >> 1) & 1, p.status, 23);
-        if (ok) scores((it + 1) & 1);
+      pipe_arrive(w.taken);
+      // the outputs stay in tensor memory, as in sdpa_flash.cu
+      const bool grow = mx > m + kSlack;
+      bool read = it == 0;  // the products of the tile before are done
+      if (__any_sync(0xffffffffu, grow)) {
+        const float to = grow ? mx : m;
+        const float corr = grow ? ex2(m - to) : 1.f;
+        m = to;
+        l *= corr;
+        if (!read) {
+          ok = pipe_wait(w, w.out, it - 1, p.status, 23);
+          if (!ok) break;
+          read = true;
+          tmem_scale64(t_o + t_lane + wg * 64, corr);
+        }
       }
-      if (ok) umma_commit(c.done);
-    }
-  }
-  if (it == n_tiles) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 24);
-  if (!__syncthreads_or(ok ? 0 : 1)) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float s[64];
-    tmem_ld64(t_o + t_lane + wg * 64, s);
+      const float mu = m == -INFINITY ? 0.f : m;
+      float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] += s[j];
-    // merge the two groups through shared memory (the position tiles are not needed any more)
-    float* ex = reinterpret_cast<float*>(spos) + r * 67;
-    if (wg == 1) {
+      for (int j = 0; j < 64; ++j) {
+        s[j] = ex2(s[j] - mu);
+        sum += s[j];
+      }
+      l += sum;
+      if constexpr (DROP) {
+        const uint64_t base = off + ((uint64_t)z * p.lp + row) * p.lp + it * 128 + wg * 64;
+        uint32_t bits[2] = {0u, 0u};
 #pragma unroll
-      for (int j = 0; j < 64; ++j) ex[j] = acc[j];
-      ex[64] = m;
-      ex[65] = l;
-    }
-    __syncthreads();
-    if (wg == 0) {
-      const float m1 = ex[64], mm = fmaxf(m, m1);  // (the first key is always there: m is finite for valid rows)
-      const float e0 = ex2(m - mm), e1 = ex2(m1 - mm);
-      l = l * e0 + ex[65] * e1;
-      const float inv = 1.f / l;
+        for (int j = 0; j < 64; j += 4) {
+          const uint64_t ctr = base + j;
+          const uint4 x = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x52u, 0u));
+          const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] = row < len ? (acc[j] * e0 + ex[j] * e1) * inv : 0.f;
-      store_row64_f32(squ, r, acc);  // (over both query tiles)
-      if (row < len) p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
+          for (int e = 0; e < 4; ++e) {
+            const bool k = w[e] >= thresh;
+            s[j + e] = k ? s[j + e] * keep_scale : 0.f;
+            if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+          }
+        }
+        if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
+      }
+      if (!read) {
+        ok = pipe_wait(w, w.out, it - 1, p.status, 24);  // P of the tile before has been read
+        if (!ok) break;
+      }
+      store_row64(sp + wg * kBig, r, s);
+      fence_proxy_async_smem();
+      pipe_arrive(w.put);
     }
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tma_store_3d(&tm_o, h * 64, q0, b, squ);
-      tma_store_3d(&tm_o, h * 64 + 32, q0, b, squ + kBig);
-      tma_store_commit();
-      tma_store_wait_all();
+    ok = ok && pipe_wait(w, w.out, n_tiles - 1, p.status, 29);
+    rows_sync<kThreads>();
+    if (ok && !*c.abort_flag) {
+      float acc[64];
+      tmem_ld64(t_o + t_lane + wg * 64, acc);
+      // merge the two groups through shared memory (the position tiles are not needed any more)
+      float* ex = reinterpret_cast<float*>(spos) + r * 67;
+      if (wg == 1) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) ex[j] = acc[j];
+        ex[64] = m;
+        ex[65] = l;
+      }
+      rows_sync<kThreads>();
+      if (wg == 0) {
+        const float m1 = ex[64], mm = fmaxf(m, m1);  // (the first key is always there: m is finite for valid rows)
+        const float e0 = ex2(m - mm), e1 = ex2(m1 - mm);
+        l = l * e0 + ex[65] * e1;
+        const float inv = 1.f / l;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) acc[j] = row < len ? (acc[j] * e0 + ex[j] * e1) * inv : 0.f;
+        store_row64_f32(squ, r, acc);  // (over both query tiles)
+        if (row < len) p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
+      }
+      fence_proxy_async_smem();
+      rows_sync<kThreads>();
+      if (tid == 0) {
+        tma_store_3d(&tm_o, h * 64, q0, b, squ);
+        tma_store_3d(&tm_o, h * 64 + 32, q0, b, squ + kBig);
+        tma_store_commit();
+        tma_store_wait_read();
+      }
     }
   }
   cta_end<512>(c);
@@ -248,7 +247,7 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
 // SAVED: the probabilities (and, dropped, those of the value product) come from memory, as the forward pass of the encoder executor left them;
 // else they are recomputed and the dropped ones written
 template <bool DROP, bool SAVED>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kCta, 1)
 rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant__ CUtensorMap tm_qv, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_pos, const __grid_constant__ CUtensorMap tm_o,
                const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dqu, const __grid_constant__ CUtensorMap tm_dqv,
@@ -274,6 +273,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     }
   };
   if (q0 >= len) {  // no valid query
+    if (tid >= kThreads) return;
     band_zeros(0, 0);
     for (int i = tid; i < n_rows_band * 8; i += kThreads) {
       const long long at = ((long long)b * p.lp + q0 + (i >> 3)) * (p.heads * 64) + h * 64 + (i & 7) * 8;
@@ -292,188 +292,180 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* sds = spos + 6 * kSmall;  // [128 queries][64 keys]
   uint8_t* sdg = sds + kBig;         // ring of [4][128 queries][64 positions]; first the tile of O in 32 bits
   uint8_t* sp = sdg + 4 * kBig;      // [128 queries][64 keys] dropped probabilities
-  const Cta c = cta_begin<512, 2>(sp + kBig);  // `done`: the products, and the bulk stores of the previous iteration have read their tiles
+  const Pipe w = pipe_begin<512, 8, 2>(sp + kBig);  // `out`: the products, and the bulk stores have read their tiles
+  const Cta& c = w.c;
   const int row = q0 + r;
   const int len64 = n_tiles * 64;
   const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 64, t_g = c.tmem + 128, t_dqu = c.tmem + 320, t_dqv = c.tmem + 384;
-  auto load = [&](int t) {
-    const int s = t & 1;
-    tma_load_3d(sk + s * kSmall, &tm_k, h * 64, t * 64, b, &c.full[s]);
-    tma_load_3d(sv + s * kSmall, &tm_v, h * 64, t * 64, b, &c.full[s]);
-    tma_load_2d(spos + s * 3 * kSmall, &tm_pos, h * 64, p.center + t * 64 - q0 - 127, &c.full[s]);
-  };
-  auto scores = [&](int s) {
-    mma64<false>(t_dp, sdo, sv + s * kSmall, false);
-    if (SAVED) return;
-    mma64<false>(t_s, squ, sk + s * kSmall, false);
-    mma_n<192>(t_g, sqv, spos + s * 3 * kSmall);
-  };
-  bool ok = true;
-  if (tid == 0) {
-    mbar_expect_tx(&c.full[0], 3 * kBig + 5 * kSmall);
-    tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
-    tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
-    tma_load_3d(sdo, &tm_do, h * 64, q0, b, &c.full[0]);
+  if (tid >= kThreads) {
+    auto load = [&](int t) {
+      if (!elect_one()) return;
+      const int s = t & 1;
+      mbar_expect_tx(&c.full[s], 5 * kSmall + (t == 0 ? 3 * kBig : 0));
+      if (t == 0) {
+        tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
+        tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
+        tma_load_3d(sdo, &tm_do, h * 64, q0, b, &c.full[0]);
+      }
+      tma_load_3d(sk + s * kSmall, &tm_k, h * 64, t * 64, b, &c.full[s]);
+      tma_load_3d(sv + s * kSmall, &tm_v, h * 64, t * 64, b, &c.full[s]);
+      tma_load_2d(spos + s * 3 * kSmall, &tm_pos, h * 64, p.center + t * 64 - q0 - 127, &c.full[s]);
+    };
     load(0);
-    mbar_expect_tx(c.extra, 2 * kBig);
-    tma_load_3d(sdg, &tm_o, h * 64, q0, b, c.extra);
-    tma_load_3d(sdg + kBig, &tm_o, h * 64 + 32, q0, b, c.extra);
-    if (n_tiles > 1) {
-      mbar_expect_tx(&c.full[1], 5 * kSmall);
-      load(1);
+    if (elect_one()) {
+      mbar_expect_tx(c.extra, 2 * kBig);
+      tma_load_3d(sdg, &tm_o, h * 64, q0, b, c.extra);
+      tma_load_3d(sdg + kBig, &tm_o, h * 64 + 32, q0, b, c.extra);
     }
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 25);
+    if (n_tiles > 1) load(1);
+    auto blocks_done = [&](int t) { return t + 1 < n_tiles ? 1 : 3; };  // blocks of the window that are complete
+    pipe_issue(w, n_tiles, p.status, load,
+               [&](int t) {
+                 const int st = t & 1;
+                 mma64_warp<false>(t_dp, sdo, sv + st * kSmall, false);
+                 if (SAVED) return;
+                 mma64_warp<false>(t_s, squ, sk + st * kSmall, false);
+                 mma_n<192>(t_g, sqv, spos + st * 3 * kSmall);
+               },
+               [&](int t) {
+                 const int st = t & 1;
+                 mma64_warp<true>(t_dqu, sds, sk + st * kSmall, t > 0);
+                 for (int q = 0; q < blocks_done(t); ++q) mma64_warp<true>(t_dqv, sdg + ((t + q) & 3) * kBig, spos + (st * 3 + q) * kSmall, t > 0 || q > 0);
+               },
+               [&](int t) {
+                 if (!elect_one()) return;
+                 for (int q = 0; q < blocks_done(t); ++q)
+#pragma unroll
+                   for (int half = 0; half < 2; ++half)
+                     if (half * 64 < n_rows_band)
+                       tma_store_2d(&tm_band, x0 + 64 * (t + q), band_row + half * 64, sdg + ((t + q) & 3) * kBig + half * kSmall);
+                 // P and dS: the products over queries run in blocks of 64 rows, zeros up to there
+#pragma unroll
+                 for (int half = 0; half < 2; ++half) {
+                   if (q0 + half * 64 >= len64) break;
+                   tma_store_2d(&tm_ds, t * 64, z * p.lp + q0 + half * 64, sds + half * kSmall);
+                   if (!SAVED) tma_store_2d(&tm_p, t * 64, z * p.lp + q0 + half * 64, sp + half * kSmall);
+                 }
+                 tma_store_commit();
+                 tma_store_wait_read();
+                 mbar_arrive_local(w.out);
+               });
+  } else {
+    band_zeros(x0, x0 + 64 * (n_tiles + 2));
+    float lse = INFINITY, delta = 0.f;
+    bool ok = pipe_wait(w, &c.full[0], 0, p.status, 26) && pipe_wait(w, c.extra, 0, p.status, 26);
     if (ok) {
-      scores(0);
-      umma_commit(c.done);
-      mbar_arrive_local(c.done);
+      delta = dot_row64(sdg, sdo, r);
+      if (!SAVED && row < len) lse = p.lse[(long long)z * p.lp + row];
     }
-  }
-  band_zeros(x0, x0 + 64 * (n_tiles + 2));
-  float lse = INFINITY, delta = 0.f;
-  ok = ok && wait_or_abort(c, &c.full[0], 0, p.status, 26) && wait_or_abort(c, c.extra, 0, p.status, 26);
-  if (ok) {
-    delta = dot_row64(sdg, sdo, r);
-    if (!SAVED && row < len) lse = p.lse[(long long)z * p.lp + row];
-  }
-  __syncthreads();
-  for (int i = tid; i < 3 * kBig / 16; i += kThreads) reinterpret_cast<uint4*>(sdg)[i] = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();
-  const float cs = p.scale * kLog2e;
-  const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-  int it = 0;
-  for (; it < n_tiles; ++it) {
-    const long long at = ((long long)z * p.lp + row) * p.lp + it * 64 + wg * 32;  // this thread's 32 scores
-    uint4 wv[4], wd[4];
-    if (SAVED && row < len) {
+    rows_sync<kThreads>();
+    for (int i = tid; i < 3 * kBig / 16; i += kThreads) reinterpret_cast<uint4*>(sdg)[i] = make_uint4(0u, 0u, 0u, 0u);
+    rows_sync<kThreads>();
+    const float cs = p.scale * kLog2e;
+    const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      const long long at = ((long long)z * p.lp + row) * p.lp + it * 64 + wg * 32;  // this thread's 32 scores
+      uint4 wv[4], wd[4];
+      if (SAVED && row < len) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          wv[q] = *reinterpret_cast<const uint4*>(p.w + at + 8 * q);
+          if (DROP) wd[q] = *reinterpret_cast<const uint4*>(p.p + at + 8 * q);
+        }
+      }
+      uint32_t bits = 0u;
+      if (DROP && !SAVED && row < len) bits = p.keep[((long long)z * p.lp + row) * p.words + it * 2 + wg];
+      ok = pipe_wait(w, w.scores, it, p.status, 27);
+      if (!ok) break;
+      float s[64], a[32], dp[32];
+      if (!SAVED) {
+        const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 32);
+        tmem_ld32(g0, reinterpret_cast<uint32_t*>(s));
+        tmem_ld32(g0 + 32, reinterpret_cast<uint32_t*>(s) + 32);
+        tmem_ld32(t_s + t_lane + wg * 32, reinterpret_cast<uint32_t*>(a));
+      }
+      tmem_ld32(t_dp + t_lane + wg * 32, reinterpret_cast<uint32_t*>(dp));
+      tmem_wait_ld();
+      pipe_arrive(w.taken);
+      if (!SAVED) shift_down<32>(s, 31 - lane);
+      const int left = row < len ? len - (it * 64 + wg * 32) : 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const bool vis = j < left;
+        float d = dp[j];
+        if (SAVED) {
+          const uint32_t word = reinterpret_cast<const uint32_t*>(wv)[j >> 1];
+          if (DROP) {  // a dropped probability is zero; where the probability itself is, its gradient is too
+            const uint32_t kept = reinterpret_cast<const uint32_t*>(wd)[j >> 1];
+            d = ((j & 1 ? kept >> 16 : kept) & 0x7fffu) ? d * keep_scale : 0.f;
+          }
+          a[j] = vis ? __uint_as_float(j & 1 ? word & 0xffff0000u : word << 16) * (d - delta) : 0.f;
+        } else {
+          const float pr = vis ? ex2(fmaf(a[j] + s[j], cs, -lse)) : 0.f;
+          float pd = pr;
+          if (DROP) {
+            const bool k = (bits >> j) & 1u;
+            d = k ? d * keep_scale : 0.f;
+            pd = k ? pr * keep_scale : 0.f;
+          }
+          a[j] = vis ? pr * (d - delta) : 0.f;
+          s[j] = pd;
+        }
+      }
+      if (it > 0) {
+        ok = pipe_wait(w, w.out, it - 1, p.status, 28);  // what the tile before has put has been read
+        if (!ok) break;
+      }
+      uint4 pk[4], dk[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        wv[q] = *reinterpret_cast<const uint4*>(p.w + at + 8 * q);
-        if (DROP) wd[q] = *reinterpret_cast<const uint4*>(p.p + at + 8 * q);
+        if (!SAVED) pk[q] = make_uint4(pack2(s[8 * q], s[8 * q + 1]), pack2(s[8 * q + 2], s[8 * q + 3]), pack2(s[8 * q + 4], s[8 * q + 5]), pack2(s[8 * q + 6], s[8 * q + 7]));
+        dk[q] = make_uint4(pack2(a[8 * q], a[8 * q + 1]), pack2(a[8 * q + 2], a[8 * q + 3]), pack2(a[8 * q + 4], a[8 * q + 5]), pack2(a[8 * q + 6], a[8 * q + 7]));
+        const int slot = r * 128 + (((wg * 4 + q) ^ (r & 7)) << 4);
+        *reinterpret_cast<uint4*>(sds + slot) = dk[q];
+        if (!SAVED) *reinterpret_cast<uint4*>(sp + slot) = pk[q];
       }
-    }
-    uint32_t bits = 0u;
-    if (DROP && !SAVED && row < len) bits = p.keep[((long long)z * p.lp + row) * p.words + it * 2 + wg];
-    ok = ok && wait_or_abort(c, c.done, it & 1, p.status, 27);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && it > 0 && it + 1 < n_tiles && ok) {
-      mbar_expect_tx(&c.full[(it + 1) & 1], 5 * kSmall);
-      load(it + 1);
-    }
-    __syncwarp();
-    float s[64], a[32], dp[32];
-    if (!SAVED) {
-      const uint32_t g0 = t_g + t_lane + (uint32_t)(96 - (r & ~31) + wg * 32);
-      tmem_ld32(g0, reinterpret_cast<uint32_t*>(s));
-      tmem_ld32(g0 + 32, reinterpret_cast<uint32_t*>(s) + 32);
-      tmem_ld32(t_s + t_lane + wg * 32, reinterpret_cast<uint32_t*>(a));
-    }
-    tmem_ld32(t_dp + t_lane + wg * 32, reinterpret_cast<uint32_t*>(dp));
-    tmem_wait_ld();
-    if (!SAVED) shift_down<32>(s, 31 - lane);
-    const int left = row < len ? len - (it * 64 + wg * 32) : 0;
+      // shifted back: key j of the tile lies at column 127 - r + j of the window. 32 columns from c0 on as pairs; where c0 is odd, the first and
+      // the last by themselves
+      {
+        const uint32_t* d = reinterpret_cast<const uint32_t*>(dk);
+        const int c0 = 127 - r + wg * 32, odd = c0 & 1;
+        uint8_t* base = sdg + r * 128;
+        auto at_col = [&](int col) { return base + ((it + (col >> 6)) & 3) * kBig + ((((col & 63) >> 3) ^ (r & 7)) << 4) + (col & 7) * 2; };
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const bool vis = j < left;
-      float d = dp[j];
-      if (SAVED) {
-        const uint32_t word = reinterpret_cast<const uint32_t*>(wv)[j >> 1];
-        if (DROP) {  // a dropped probability is zero; where the probability itself is, its gradient is too
-          const uint32_t kept = reinterpret_cast<const uint32_t*>(wd)[j >> 1];
-          d = ((j & 1 ? kept >> 16 : kept) & 0x7fffu) ? d * keep_scale : 0.f;
+        for (int j = 0; j < 15; ++j) *reinterpret_cast<uint32_t*>(at_col(c0 + odd + 2 * j)) = odd ? __funnelshift_r(d[j], d[j + 1], 16) : d[j];
+        if (odd) {
+          *reinterpret_cast<unsigned short*>(at_col(c0)) = (unsigned short)(d[0] & 0xffffu);
+          *reinterpret_cast<unsigned short*>(at_col(c0 + 31)) = (unsigned short)(d[15] >> 16);
+        } else {
+          *reinterpret_cast<uint32_t*>(at_col(c0 + 30)) = d[15];
         }
-        a[j] = vis ? __uint_as_float(j & 1 ? word & 0xffff0000u : word << 16) * (d - delta) : 0.f;
-      } else {
-        const float pr = vis ? ex2(fmaf(a[j] + s[j], cs, -lse)) : 0.f;
-        float pd = pr;
-        if (DROP) {
-          const bool k = (bits >> j) & 1u;
-          d = k ? d * keep_scale : 0.f;
-          pd = k ? pr * keep_scale : 0.f;
-        }
-        a[j] = vis ? pr * (d - delta) : 0.f;
-        s[j] = pd;
       }
-    }
-    uint4 pk[4], dk[4];
+      // the block that joins the window with the next tile; the last two are filled in part
+      if (it + 3 >= n_tiles && it + 3 <= n_tiles + 1) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (!SAVED) pk[q] = make_uint4(pack2(s[8 * q], s[8 * q + 1]), pack2(s[8 * q + 2], s[8 * q + 3]), pack2(s[8 * q + 4], s[8 * q + 5]), pack2(s[8 * q + 6], s[8 * q + 7]));
-      dk[q] = make_uint4(pack2(a[8 * q], a[8 * q + 1]), pack2(a[8 * q + 2], a[8 * q + 3]), pack2(a[8 * q + 4], a[8 * q + 5]), pack2(a[8 * q + 6], a[8 * q + 7]));
-      const int slot = r * 128 + (((wg * 4 + q) ^ (r & 7)) << 4);
-      *reinterpret_cast<uint4*>(sds + slot) = dk[q];
-      if (!SAVED) *reinterpret_cast<uint4*>(sp + slot) = pk[q];
-    }
-    // shifted back: key j of the tile lies at column 127 - r + j of the window. 32 columns from c0 on as pairs; where c0 is odd, the first and
-    // the last by themselves
-    {
-      const uint32_t* d = reinterpret_cast<const uint32_t*>(dk);
-      const int c0 = 127 - r + wg * 32, odd = c0 & 1;
-      uint8_t* base = sdg + r * 128;
-      auto at_col = [&](int col) { return base + ((it + (col >> 6)) & 3) * kBig + ((((col & 63) >> 3) ^ (r & 7)) << 4) + (col & 7) * 2; };
-#pragma unroll
-      for (int j = 0; j < 15; ++j) *reinterpret_cast<uint32_t*>(at_col(c0 + odd + 2 * j)) = odd ? __funnelshift_r(d[j], d[j + 1], 16) : d[j];
-      if (odd) {
-        *reinterpret_cast<unsigned short*>(at_col(c0)) = (unsigned short)(d[0] & 0xffffu);
-        *reinterpret_cast<unsigned short*>(at_col(c0 + 31)) = (unsigned short)(d[15] >> 16);
-      } else {
-        *reinterpret_cast<uint32_t*>(at_col(c0 + 30)) = d[15];
+        for (int q = 0; q < kBig / 16 / kThreads; ++q) reinterpret_cast<uint4*>(sdg + ((it + 3) & 3) * kBig)[q * kThreads + tid] = make_uint4(0u, 0u, 0u, 0u);
       }
+      fence_proxy_async_smem();
+      pipe_arrive(w.put);
     }
-    // the block that joins the window with the next tile; the last two are filled in part
-    if (it + 3 >= n_tiles && it + 3 <= n_tiles + 1) {
+    ok = ok && pipe_wait(w, w.out, n_tiles - 1, p.status, 29);
+    rows_sync<kThreads>();
+    if (ok && !*c.abort_flag) {
+      float s[64];
+      tmem_ld64((wg ? t_dqv : t_dqu) + t_lane, s);
 #pragma unroll
-      for (int q = 0; q < kBig / 16 / kThreads; ++q) reinterpret_cast<uint4*>(sdg + ((it + 3) & 3) * kBig)[q * kThreads + tid] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    fence_proxy_async_smem();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or(ok ? 0 : 1)) break;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int st = it & 1;
-      mma64<true>(t_dqu, sds, sk + st * kSmall, it > 0);
-      const int n_done = it + 1 < n_tiles ? 1 : 3;  // blocks of the window that are complete
-      for (int q = 0; q < n_done; ++q) mma64<true>(t_dqv, sdg + ((it + q) & 3) * kBig, spos + (st * 3 + q) * kSmall, it > 0 || q > 0);
-      if (it + 1 < n_tiles) {
-        ok = wait_or_abort(c, &c.full[st ^ 1], ((it + 1) >> 1) & 1, p.status, 28);
-        if (ok) scores(st ^ 1);
-      }
-      if (ok) {
-        umma_commit(c.done);
-        for (int q = 0; q < n_done; ++q)
-#pragma unroll
-          for (int half = 0; half < 2; ++half)
-            if (half * 64 < n_rows_band)
-              tma_store_2d(&tm_band, x0 + 64 * (it + q), band_row + half * 64, sdg + ((it + q) & 3) * kBig + half * kSmall);
-        // P and dS: the products over queries run in blocks of 64 rows, zeros up to there
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (q0 + half * 64 >= len64) break;
-          tma_store_2d(&tm_ds, it * 64, z * p.lp + q0 + half * 64, sds + half * kSmall);
-          if (!SAVED) tma_store_2d(&tm_p, it * 64, z * p.lp + q0 + half * 64, sp + half * kSmall);
-        }
+      for (int j = 0; j < 64; ++j) s[j] *= p.scale;
+      store_row64(wg ? sqv : squ, r, s);
+      fence_proxy_async_smem();
+      rows_sync<kThreads>();
+      if (tid == 0) {
+        tma_store_3d(&tm_dqu, h * 64, q0, b, squ);
+        tma_store_3d(&tm_dqv, h * 64, q0, b, sqv);
         tma_store_commit();
         tma_store_wait_read();
-        mbar_arrive_local(c.done);
       }
-    }
-  }
-  if (it == n_tiles) ok = ok && wait_or_abort(c, c.done, n_tiles & 1, p.status, 29);
-  if (!__syncthreads_or(ok ? 0 : 1)) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float s[64];
-    tmem_ld64((wg ? t_dqv : t_dqu) + t_lane, s);
-#pragma unroll
-    for (int j = 0; j < 64; ++j) s[j] *= p.scale;
-    store_row64(wg ? sqv : squ, r, s);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tma_store_3d(&tm_dqu, h * 64, q0, b, squ);
-      tma_store_3d(&tm_dqv, h * 64, q0, b, sqv);
-      tma_store_commit();
-      tma_store_wait_all();
     }
   }
   cta_end<512>(c);
@@ -550,7 +542,7 @@ RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k,
   auto kernel = p_drop > 0.f ? rel_fwd_kernel<true> : rel_fwd_kernel<false>;
   const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
   if (err != cudaSuccess) return failed("rel_flash_fwd", err);
-  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kFwdSmem, stream, a, b, c, d, e, f, p);
+  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kCta), kFwdSmem, stream, a, b, c, d, e, f, p);
   return rb_check_launch("rel_flash_fwd");
 }
 
@@ -600,7 +592,7 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   auto kernel = p_drop > 0.f ? (w ? rel_bwd_kernel<true, true> : rel_bwd_kernel<true, false>) : (w ? rel_bwd_kernel<false, true> : rel_bwd_kernel<false, false>);
   const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
   if (err != cudaSuccess) return failed("rel_flash_bwd", err);
-  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kThreads), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, map_p, map_ds, p);
+  rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kCta), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, map_p, map_ds, p);
   return rb_check_launch("rel_flash_bwd");
 }
 

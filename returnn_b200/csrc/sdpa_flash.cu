@@ -44,101 +44,7 @@ __device__ __forceinline__ int visible(const Flash& p, int i, int klen) {
   return max(n, 0);
 }
 
-// ---- life of a CTA: four warps of rows and one that issues -----------------------------------------------------------------------------
-// The warp behind the rows' four issues loads and products; the rows' warps meet it at mbarriers and each other nowhere. Scores
-// are in registers as soon as they are read, so the products of the next tile run while the row work of this one does. With thread 0 issuing
-// between barriers of the whole CTA, a tile was product (1000 to 1400 cycles), row work, barrier (500), one after the other: 3600, 2800 and 4500
-// cycles in the three kernels.
-constexpr int kCta = kThreads + 32;
-
-struct Pipe {
-  Cta c;
-  uint64_t *scores, *out, *taken, *put;  // scores of a tile are there, products with P / dS are done; rows have taken the scores, put P / dS
-};
-template <uint32_t COLS>
-__device__ __forceinline__ Pipe pipe_begin(uint8_t* tail) {
-  Pipe p;
-  p.c.full = reinterpret_cast<uint64_t*>(tail);
-  p.c.extra = p.c.full + 2;
-  p.scores = p.c.full + 3;
-  p.c.done = p.out = p.c.full + 4;
-  p.taken = p.c.full + 5;
-  p.put = p.c.full + 6;
-  uint32_t* slot = reinterpret_cast<uint32_t*>(p.c.full + 7);
-  p.c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < 7; ++i) mbar_init(p.c.full + i, i >= 5 ? 4 : 1);
-    *p.c.abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (threadIdx.x < 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  p.c.tmem = *slot;
-  return p;
-}
-// all lanes of a warp: the wait of one that gave up is the wait of all
-__device__ __forceinline__ bool pipe_wait(const Pipe& p, uint64_t* bar, int phase, int* status, int code) {
-  const bool ok = __all_sync(0xffffffffu, wait_or_abort(p.c, bar, phase & 1, status, code));
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  return ok;
-}
-// D[128, 64] (+)= A[128, 64] B as mma64, by one lane of a converged warp
-template <bool B_MN>
-__device__ __forceinline__ void mma64_warp(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  const uint32_t da = desc_lo(smem_u32(a), 16), db = desc_lo(smem_u32(b), B_MN ? 8192 : 16);
-  umma_f16_warp(d, da, db, idesc, accumulate ? 1u : 0u);
-#pragma unroll
-  for (int kk = 1; kk < 4; ++kk) umma_f16_warp(d, da + 2 * kk, db + (B_MN ? 128 : 2) * kk, idesc, 1u);
-}
-// a warp of rows is through with its accesses to tensor memory and shared memory (those to the latter made visible by each lane before)
-__device__ __forceinline__ void pipe_arrive(uint64_t* bar) {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive_local(bar);
-}
-__device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-               ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-               "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-               : "memory");
-}
-// The issuing warp, over n tiles: `load(t)` into stage t & 1 (its barrier: full[t & 1]), `first(t)` products that give scores, `second(t)` those with
-// what the rows have put. Tiles 0 and 1 are being loaded.
-template <typename Load, typename First, typename Second>
-__device__ __forceinline__ void pipe_issue(const Pipe& p, int n, int* status, Load load, First first, Second second) {
-  bool ok = pipe_wait(p, &p.c.full[0], 0, status, 1);
-  if (ok) {
-    first(0);
-    umma_commit_warp(p.scores);
-  }
-  for (int t = 0; t < n && ok; ++t) {
-    if (t + 1 < n) {
-      ok = pipe_wait(p, p.taken, t, status, 2) && pipe_wait(p, &p.c.full[(t + 1) & 1], (t + 1) >> 1, status, 3);
-      if (!ok) break;
-      first(t + 1);
-      umma_commit_warp(p.scores);
-    }
-    ok = pipe_wait(p, p.put, t, status, 4);
-    if (!ok) break;
-    second(t);
-    umma_commit_warp(p.out);
-    if (t + 2 < n) {
-      ok = pipe_wait(p, p.out, t, status, 5);  // stage t & 1 has been read
-      if (ok) load(t + 2);
-    }
-  }
-}
-
-// The output stays in tensor memory: the maximum that P refers to grows only when a row's has grown by more than 2^8 (what its values are then, up to
-// 256, costs no precision), and only then a warp takes its rows of the output out, scales them and puts them back.
-constexpr float kSlack = 8.f;
+constexpr int kCta = kThreads + 32;  // and the warp that issues (see Pipe)
 
 template <bool DROP>
 __global__ void __launch_bounds__(kCta, 3)
@@ -149,7 +55,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t* sk = sq + kBig;
   uint8_t* sv = sk + 2 * kSmall;
   uint8_t* sp = sv + 2 * kSmall;
-  const Pipe w = pipe_begin<128>(sp + kBig);
+  const Pipe w = pipe_begin<128, 4>(sp + kBig);
   const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
@@ -174,7 +80,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (n_tiles > 1) load(1);
     if (n_tiles > 0)
       pipe_issue(w, n_tiles, p.status, load, [&](int t) { mma64_warp<false>(t_s, sq, sk + (t & 1) * kSmall, false); },
-                 [&](int t) { mma64_warp<true>(t_o, sp, sv + (t & 1) * kSmall, t > 0); });
+                 [&](int t) { mma64_warp<true>(t_o, sp, sv + (t & 1) * kSmall, t > 0); }, [](int) {});
   } else {
     const int row = q0 + tid;
     const int n = row < p.tq ? visible(p, row, klen) : 0;
@@ -217,16 +123,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           ok = pipe_wait(w, w.out, it - 1, p.status, 7);
           if (!ok) break;
           read = true;
-#pragma unroll 1
-          for (int part = 0; part < 4; ++part) {
-            uint32_t o[16];
-            tmem_ld16(t_row + 64 + 16 * part, o);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
-            tmem_st16(t_row + 64 + 16 * part, o);
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tmem_scale64(t_row + 64, corr);
         }
       }
       const float mu = m == -INFINITY ? 0.f : m;
@@ -274,7 +171,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (row < p.tq) p.lse[(long long)z * p.tq + row] = n > 0 ? m + __log2f(l) : INFINITY;
       fence_proxy_async_smem();
     }
-    rows_sync();
+    rows_sync<kThreads>();
     if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_o, h * kTile, q0, b, sq);
       if (p.save) {
@@ -299,7 +196,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint8_t* sk = sdo + kBig;
   uint8_t* sv = sk + 2 * kSmall;
   uint8_t* sds = sv + 2 * kSmall;  // first, with the kBig bytes behind it, the tile of O in 32 bits
-  const Pipe w = pipe_begin<256>(sds + 2 * kBig);
+  const Pipe w = pipe_begin<256, 4>(sds + 2 * kBig);
   const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
@@ -335,7 +232,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                    mma64_warp<false>(t_s, sq, sk + (t & 1) * kSmall, false);
                    mma64_warp<false>(t_dp, sdo, sv + (t & 1) * kSmall, false);
                  },
-                 [&](int t) { mma64_warp<true>(t_dq, sds, sk + (t & 1) * kSmall, t > 0); });
+                 [&](int t) { mma64_warp<true>(t_dq, sds, sk + (t & 1) * kSmall, t > 0); }, [](int) {});
     }
   } else {
     const int row = q0 + tid;
@@ -392,7 +289,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       store_row64(sq, tid, s);
       fence_proxy_async_smem();
     }
-    rows_sync();
+    rows_sync<kThreads>();
     if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_dq, h * kTile, q0, b, sq);
       tma_store_commit();
@@ -417,7 +314,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // per warp of rows: (log-sum, delta) of the 64 queries of a tile, and the dropout bits of the warp's 32 keys
   float2* stat = reinterpret_cast<float2*>(sds + kBig) + (threadIdx.x >> 5) * 64;
   uint32_t* kept = reinterpret_cast<uint32_t*>(sds + kBig + 2048) + (threadIdx.x >> 5) * 64;
-  const Pipe w = pipe_begin<256>(sds + kBig + 2048 + 1024);
+  const Pipe w = pipe_begin<256, 4>(sds + kBig + 2048 + 1024);
   const Cta& c = w.c;
   rb_pdl_wait();
   rb_pdl_launch();
@@ -452,7 +349,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                  [&](int t) {
                    mma64_warp<true>(t_dv, sp, sdo + (t & 1) * kSmall, t > 0);
                    mma64_warp<true>(t_dk, sds, sq + (t & 1) * kSmall, t > 0);
-                 });
+                 },
+                 [](int) {});
     }
   } else {
     const int key = k0 + tid, lane = tid & 31;
@@ -534,7 +432,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       store_row64(sk, tid, dp);
       fence_proxy_async_smem();
     }
-    rows_sync();
+    rows_sync<kThreads>();
     if (tid == 0 && ok && !*c.abort_flag) {
       tma_store_3d(&tm_dv, h * kTile, k0, b, sv);
       tma_store_3d(&tm_dk, h * kTile, k0, b, sk);
@@ -582,20 +480,23 @@ flash_bwd_small_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const uint32_t t_s = c.tmem, t_dp = c.tmem + 128, t_dv = c.tmem, t_dq = c.tmem + 64, t_dk = c.tmem + 128;
   bool ok = true;
   const bool any = key_steps > 0;
-  if (tid == 0 && any) {
-    mbar_expect_tx(&c.full[0], 4 * kBig);
-    tma_load_3d(sq, &tm_q, h * p.hq, 0, b, &c.full[0]);
-    tma_load_3d(sk, &tm_k, h * p.hk, 0, b, &c.full[0]);
-    tma_load_3d(sdo, &tm_do, h * p.hdo, 0, b, &c.full[0]);
-    tma_load_3d(sv, &tm_v, h * p.hv, 0, b, &c.full[0]);
-    ok = wait_or_abort(c, &c.full[0], 0, p.status, 14);
+  if (tid < 32 && any) {  // (loads and products: one lane of the first warp)
+    if (elect_one()) {
+      mbar_expect_tx(&c.full[0], 4 * kBig);
+      tma_load_3d(sq, &tm_q, h * p.hq, 0, b, &c.full[0]);
+      tma_load_3d(sk, &tm_k, h * p.hk, 0, b, &c.full[0]);
+      tma_load_3d(sdo, &tm_do, h * p.hdo, 0, b, &c.full[0]);
+      tma_load_3d(sv, &tm_v, h * p.hv, 0, b, &c.full[0]);
+    }
+    __syncwarp();
+    ok = __all_sync(0xffffffffu, wait_or_abort(c, &c.full[0], 0, p.status, 14));
     if (ok) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(16 * key_steps >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) umma_f16(t_s, make_desc(smem_u32(sq) + kk * 32, 16, 1024), make_desc(smem_u32(sk) + kk * 32, 16, 1024), idesc, kk > 0);
+      for (int kk = 0; kk < 4; ++kk) umma_f16_warp(t_s, desc_lo(smem_u32(sq), 16) + 2 * kk, desc_lo(smem_u32(sk), 16) + 2 * kk, idesc, kk > 0);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) umma_f16(t_dp, make_desc(smem_u32(sdo) + kk * 32, 16, 1024), make_desc(smem_u32(sv) + kk * 32, 16, 1024), idesc, kk > 0);
-      umma_commit(c.done);
+      for (int kk = 0; kk < 4; ++kk) umma_f16_warp(t_dp, desc_lo(smem_u32(sdo), 16) + 2 * kk, desc_lo(smem_u32(sv), 16) + 2 * kk, idesc, kk > 0);
+      umma_commit_warp(c.done);
     }
   }
   const float lse = row < p.tq ? p.lse[(long long)z * p.tq + row] : INFINITY;
@@ -640,11 +541,11 @@ flash_bwd_small_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     // contraction over the queries: A [query][key] is M-major in two panels of 64 keys, B [query][64] N-major
     constexpr uint32_t idesc_t = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     constexpr uint32_t idesc_n = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    if (tid == 0 && ok) {
+    const uint32_t x_t = desc_lo(smem_u32(sx), kBig), x_n = desc_lo(smem_u32(sx), 16);
+    if (tid < 32 && ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int kk = 0; kk < query_steps; ++kk)
-        umma_f16(t_dv, make_desc(smem_u32(sx) + kk * 2048, kBig, 1024), make_desc(smem_u32(sdo) + kk * 2048, 8192, 1024), idesc_t, kk > 0);
-      umma_commit(c.done);
+      for (int kk = 0; kk < query_steps; ++kk) umma_f16_warp(t_dv, x_t + 128 * kk, desc_lo(smem_u32(sdo), 8192) + 128 * kk, idesc_t, kk > 0);
+      umma_commit_warp(c.done);
     }
     __syncwarp();
     uint32_t ds[64];
@@ -675,12 +576,11 @@ flash_bwd_small_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     ok = !__syncthreads_or(ok ? 0 : 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0 && ok) {
+    if (tid < 32 && ok) {
       for (int kk = 0; kk < key_steps; ++kk)
-        umma_f16(t_dq, make_desc(smem_u32(sx) + (kk >> 2) * kBig + (kk & 3) * 32, 16, 1024), make_desc(smem_u32(sk) + kk * 2048, 8192, 1024), idesc_n, kk > 0);
-      for (int kk = 0; kk < query_steps; ++kk)
-        umma_f16(t_dk, make_desc(smem_u32(sx) + kk * 2048, kBig, 1024), make_desc(smem_u32(sq) + kk * 2048, 8192, 1024), idesc_t, kk > 0);
-      umma_commit(c.done);
+        umma_f16_warp(t_dq, x_n + (kk >> 2) * (kBig >> 4) + (kk & 3) * 2, desc_lo(smem_u32(sk), 8192) + 128 * kk, idesc_n, kk > 0);
+      for (int kk = 0; kk < query_steps; ++kk) umma_f16_warp(t_dk, x_t + 128 * kk, desc_lo(smem_u32(sq), 8192) + 128 * kk, idesc_t, kk > 0);
+      umma_commit_warp(c.done);
     }
     __syncwarp();
     float o[64];
