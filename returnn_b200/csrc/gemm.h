@@ -38,7 +38,7 @@ struct RbGemm {
   const int* lens = nullptr;
   int m_from_lens = 0, n_from_lens = 0, k_from_lens = 0;
   // batched form, bf16 output without bias or activation: each problem owns whole rows of c, of ldc columns, and its rows up to the next multiple of 32.
-  // c_rows > 0 (rows of the matrix that holds all problems' outputs): the output leaves in boxes of 32 x 32, what lies in them past m and n is unspecified
+  // c_rows > 0 (rows of the matrix that holds all problems' outputs): the output leaves in boxes of 32 x 64, what lies in them past m and n is unspecified
   long long c_rows = 0;
   // windows of a relative-position band (batched form): row i of a sequence of length len concerns the columns [win_center - i, win_center - i + len).
   // win = 1: the output is the band, m_from_lens; tiles of it without such a column are not computed (and not written).

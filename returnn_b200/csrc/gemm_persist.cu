@@ -31,29 +31,39 @@ using namespace rbg;
 namespace {
 
 constexpr int BM = 128;
-constexpr int kThreads = kGemmThreads;
-constexpr int kRingBytes = 196608;      // operand ring: 4 stages (BN = 256), 6 stages (BN = 128) or 8 stages (BN = 64)
-constexpr int kStagingBytes = kEpilogueWarps * kStagingBytesPerWarp;
 constexpr int kBarrierBytes = 256;
-constexpr int kSmemBytes = kRingBytes + kStagingBytes + kBarrierBytes + 1024;
 constexpr int kMaxStages = 8;
 
-template <int BN, bool FULL>
-__global__ void __launch_bounds__(kThreads, 1)
+// What a CTA of the kernel has: one per SM with a long ring and 16 epilogue warps, or two per SM with 8 for batched problems of few K blocks, where a unit
+// is a chain of first load, few products and epilogue that one CTA's two accumulators do not hide. 36 x 333 frames, 8 heads (lengths from half on):
+// dV 16.8 -> 14.7 us, position gradient 24.7 -> 18.0; 20 x 500 frames 17.8 -> 17.4 and 24.9 -> 19.8. Three CTAs with two stages each: 15.2 and 21.3;
+// a CTA per unit, handed out by the hardware: 20.9 and 17.9. Products of whole rows (attention scores and band, one K block) within a pass of 6912
+// rows: 23 and 34 -> 16.7 us each, most of it by boxes of 128-byte rows that are written while the unit after them is multiplied.
+template <int BN, int CTAS>
+struct Layout {
+  static constexpr bool kBoxes = CTAS > 1 && BN == 128;  // (whole rows of the output: bulk stores of 32 rows x 64 columns)
+  static constexpr int kWarps = CTAS > 1 ? 8 : kEpilogueWarps;
+  static constexpr int kThreads = 64 + kWarps * 32;
+  static constexpr int kStageBytes = (BM + BN) * BK * 2;
+  static constexpr int kStages = CTAS == 1 ? 196608 / kStageBytes : BN == 128 ? 2 : 3;
+  static constexpr int kRingBytes = kStages * kStageBytes;
+  static constexpr int kStaging = kBoxes ? kStoreBoxBytesPerWarp : kStagingBytesPerWarp;  // per warp
+  static constexpr int kSmemBytes = kRingBytes + kWarps * kStaging + kBarrierBytes + 1024;
+  static_assert(kStages <= kMaxStages && kStages >= 2 && CTAS * (kSmemBytes + 1024) <= 228 * 1024 && CTAS * 2 * BN <= 512, "layout");
+};
+
+template <int BN, bool FULL, int CTAS>
+__global__ void __launch_bounds__(Layout<BN, CTAS>::kThreads, CTAS)
 gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c, const Params p) {
   constexpr int kTileBytesA = BM * BK * 2;
-  constexpr int kTileBytesB = BN * BK * 2;
-  constexpr int kStageBytes = kTileBytesA + kTileBytesB;
-  constexpr int kStages = kRingBytes / kStageBytes;
-  static_assert(kStages <= kMaxStages && kStages >= 2, "ring");
+  using L = Layout<BN, CTAS>;
+  constexpr int kStageBytes = L::kStageBytes, kStages = L::kStages;
   constexpr uint32_t kTmemCols = 2 * BN;
-  // bulk stores: a warp takes 64 columns, so tiles of 128 columns keep half of the warps busy, and the halves take the two accumulators in turn
-  constexpr int kParts = BN / 64, kSets = BN == 256 ? 1 : 2;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* staging = reinterpret_cast<float*>(smem + kRingBytes);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kRingBytes + kStagingBytes);
+  float* staging = reinterpret_cast<float*>(smem + L::kRingBytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kRingBytes + L::kWarps * L::kStaging);
   uint64_t* empty_bar = full_bar + kMaxStages;
   uint64_t* acc_full = empty_bar + kMaxStages;
   uint64_t* acc_empty = acc_full + 2;
@@ -71,14 +81,17 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], p.tma_store ? kEpilogueWarps / kSets : kEpilogueWarps);  // one arrival per epilogue warp of the buffer
+      mbar_init(&acc_empty[i], L::kWarps);  // one arrival per epilogue warp
     }
     *abort_flag = 0;
     prefetch_map(&tm_a);
     prefetch_map(&tm_b);
-    if (p.tma_store) prefetch_map(&tm_c);
+    if (L::kBoxes) prefetch_map(&tm_c);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // several CTAs per SM: no tensor memory is taken before the kernel in front has given its own back, and none of the next kernel's before this one
+  // has (a CTA of either that waits for tensor memory while it is waited for itself would never get it)
+  if (CTAS > 1) rb_pdl_wait();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -88,7 +101,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   // everything above touched no global memory: it may overlap the tail of the preceding kernel
-  rb_pdl_wait();
+  if (CTAS == 1) rb_pdl_wait();
   rb_pdl_launch();
   if (warp == 0) {
     // ---------------- TMA producer: the warp walks, one lane of it issues ----------------
@@ -177,17 +190,13 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   } else {
     // ---------------- epilogue: warps 2..5, TMEM lane quarter = warp % 4 ----------------
     const int q = warp & 3;
-    float* stg = staging + (warp - 2) * (kStagingBytesPerWarp / 4);
+    float* stg = staging + (warp - 2) * (L::kStaging / 4);
     uint32_t t_local = 0;
     for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
       const Unit w = decode_unit<BM, BN>(p, u);
       if (!w.valid) continue;
       const int m0 = w.m0, n0 = w.n0;
       const uint32_t buf = t_local & 1u;
-      if (!FULL && BN == 128 && p.tma_store && (int)buf != ((warp - 2) >> 2) / kParts) {
-        ++t_local;
-        continue;
-      }
       bool ok = mbar_wait(&acc_full[buf], (t_local >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) {
         *abort_flag = 1;
@@ -197,14 +206,15 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-      const int part = (warp - 2) >> 2;  // four warps per lane quarter, each with a quarter of the columns
-      if (!FULL && BN >= 128 && p.tma_store)
-        epilogue_boxes(p, w, (int)(w.c_off / g.ldc), t_addr, (part % kParts) * 64, reinterpret_cast<uint8_t*>(stg), &tm_c, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
+      const int part = (warp - 2) >> 2;  // four (two) warps per lane quarter, each with a quarter (half) of the columns
+      constexpr int kCols = BN / (L::kWarps / 4);
+      if (L::kBoxes)
+        epilogue_boxes(p, w, (int)(w.c_off / g.ldc), t_addr, part * 64, reinterpret_cast<uint8_t*>(stg), &tm_c, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
       else
-        epilogue_columns<FULL>(p, w, m0, n0, t_addr, part * (BN / 4), (part + 1) * (BN / 4), stg, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
+        epilogue_columns<FULL>(p, w, m0, n0, t_addr, part * kCols, (part + 1) * kCols, stg, lane, q, [&]() { mbar_arrive(&acc_empty[buf]); });
       ++t_local;
     }
-    if (!FULL && BN >= 128 && p.tma_store && lane == 0) tma_store_wait_read();  // before the shared memory is handed on
+    if (L::kBoxes && lane == 0) tma_store_wait_read();  // before the shared memory is handed on
   }
 
   // ---------------- teardown ----------------
@@ -231,12 +241,24 @@ int num_sms() {
   return n;
 }
 
-template <int BN>
+bool epilogue_full(const RbGemm& g) { return g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr; }
+
+bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }  // (also: not there)
+
+// whether the problems of a batch own whole rows of an output that bulk stores can write (see gemm.h)
+bool boxes_ok(const RbGemm& g) {
+  return !epilogue_full(g) && g.batch > 0 && g.c_rows > 0 && !g.out_fp32 && !g.c2 && !g.bias && !g.act && g.ldc % 8 == 0 && aligned16(g.c) &&
+         g.c_sb % g.ldc == 0 && g.c_sh % g.ldc == 0;
+}
+
+template <int BN, int CTAS>
 int launch(const RbGemm& g, cudaStream_t stream) {
+  using L = Layout<BN, CTAS>;
+  constexpr bool kFull = CTAS == 1;  // several CTAs per SM: the plain epilogue only
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_persist_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_persist_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_persist_kernel<BN, false, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
+    if (kFull && e == cudaSuccess) e = cudaFuncSetAttribute(gemm_persist_kernel<BN, kFull, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) {
       rb_set_error("gemm: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return RB_ERR_LAUNCH;
@@ -264,16 +286,14 @@ int launch(const RbGemm& g, cudaStream_t stream) {
     p.split = 1;
     p.units = tiles * g.batch;
   }
-  auto al16 = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  p.vec_ok = (g.ldc % 8 == 0) && al16(g.c) && al16(g.c2) && al16(g.resid) && al16(g.dact_z);
-  p.bias_vec = g.bias != nullptr && !g.bias_bf16 && al16(g.bias);
-  const bool full = g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr;
+  p.vec_ok = (g.ldc % 8 == 0) && aligned16(g.c) && aligned16(g.c2) && aligned16(g.resid) && aligned16(g.dact_z);
+  p.bias_vec = g.bias != nullptr && !g.bias_bf16 && aligned16(g.bias);
   CUtensorMap tm_a, tm_b, tm_c;
   memset(&tm_c, 0, sizeof(tm_c));
   int st;
-  p.tma_store = BN >= 128 && !full && g.batch > 0 && g.c_rows > 0 && !g.out_fp32 && !g.c2 && !g.bias && !g.act && p.vec_ok && g.c_sb % g.ldc == 0 && g.c_sh % g.ldc == 0;
-  if (p.tma_store) {
-    st = make_map(&tm_c, g.c, g.ldc, g.c_rows, g.ldc, 32, 32, false, true);
+  p.tma_store = L::kBoxes;
+  if (L::kBoxes) {
+    st = make_map(&tm_c, g.c, g.ldc, g.c_rows, g.ldc, 64, 32);
     if (st) return st;
   }
   long long a_rows = g.a_mn_major ? g.k : g.m, a_cols = g.a_mn_major ? g.m : g.k;
@@ -285,7 +305,7 @@ int launch(const RbGemm& g, cudaStream_t stream) {
   if (st) return st;
   st = g.b_mn_major ? make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, 64, BK) : make_map(&tm_b, g.b, b_cols, b_rows, g.ldb, BK, BN);
   if (st) return st;
-  int grid = p.units < sms ? p.units : sms;
+  int grid = p.units < CTAS * sms ? p.units : CTAS * sms;
   {
     // tuning knob: cap the number of CTAs (for bandwidth / latency experiments)
     static int cap = -1;
@@ -295,8 +315,8 @@ int launch(const RbGemm& g, cudaStream_t stream) {
     }
     if (cap > 0 && grid > cap) grid = cap;
   }
-  if (full) rb_launch_pdl(gemm_persist_kernel<BN, true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, p);
-  else rb_launch_pdl(gemm_persist_kernel<BN, false>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_a, tm_b, tm_c, p);
+  if (kFull && epilogue_full(g)) rb_launch_pdl(gemm_persist_kernel<BN, kFull, CTAS>, dim3(grid), dim3(L::kThreads), L::kSmemBytes, stream, tm_a, tm_b, tm_c, p);
+  else rb_launch_pdl(gemm_persist_kernel<BN, false, CTAS>, dim3(grid), dim3(L::kThreads), L::kSmemBytes, stream, tm_a, tm_b, tm_c, p);
   return rb_check_launch("gemm_persist");
 }
 
@@ -343,9 +363,13 @@ int rb_gemm(const RbGemm& g, cudaStream_t stream) {
   }
   if (rb_gemm_pair_wanted(g)) return rb_gemm_pair(g, stream);
   // Narrow tiles where wider ones would load and multiply columns that are not wanted: one head of 64 columns, the windows of a band
-  if (g.n > 128 && g.win != 1) return launch<256>(g, stream);
-  if (g.n > 64) return launch<128>(g, stream);
-  return launch<64>(g, stream);
+  if (g.n > 64 && boxes_ok(g)) return launch<128, 2>(g, stream);
+  if (g.n > 128 && g.win != 1) return launch<256, 1>(g, stream);
+  if (g.n > 64) return launch<128, 1>(g, stream);
+  // (with a unit per SM or less there is nothing to overlap, and tensor memory is to be had before the kernel in front has ended: 4 x 50 frames
+  // 4.0 us, with two CTAs per SM 4.5)
+  if (g.batch > 0 && !epilogue_full(g) && (long long)((g.m + BM - 1) / BM) * g.batch > num_sms()) return launch<64, 2>(g, stream);
+  return launch<64, 1>(g, stream);
 }
 
 // C entry points with the full epilogue (see gemm.h for the meaning of the arguments); the second reads A and B as fp16
