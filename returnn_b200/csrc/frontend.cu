@@ -5,6 +5,8 @@
 // length read as zero, and the last layer is produced directly in packed-row form (valid frames only).
 //
 //   conv1 (C_in = 1): direct kernel, fused ReLU + max-pool over feature pairs + time mask        -> [B, T, F/2, C1]
+// 32 or 64 channels on both sides of a later convolution run without patch matrices (conv_implicit.cu); otherwise:
+//
 //   conv k >= 2: im2col  [rows, 9*C_in]  x  W [C_out, 9*C_in]^T  (+bias, ReLU)                    -> [rows, C_out]
 //   backward data: transposed gather of dY [rows_in, 9*C_out]  x  W' [9*C_out, C_in], epilogue * relu'(saved output)
 //   backward weights: patch matrix^T x dY on the split-K GEMM; conv1: direct reduction kernel (recomputes its activations)

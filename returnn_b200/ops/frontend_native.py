@@ -2,7 +2,8 @@
 Conv2d subsampling frontend on B200 (``csrc/frontend.cu`` + the tcgen05 GEMM): 3x3 convolutions over (time, feature) as
 implicit GEMMs with fused bias / ReLU / ReLU-gradient epilogues, the first layer (one input channel) with fused ReLU +
 max-pool, the last layer computed directly for the valid frames only (packed rows). One autograd function covers the whole
-stack; its backward runs transposed gathers + GEMMs for the data gradients and split-K GEMMs for the filter gradients.
+stack. Layers of 32 or 64 channels on both sides read their operands in place in all three products (``csrc/conv_implicit.cu``); others go through
+patch matrices: GEMMs and gathers for the data gradients, split-K GEMMs for the filter gradients.
 
 Handles the layout of :class:`returnn_b200.frontend.encoder.conformer.ConformerConvSubsample` with three 3x3 layers,
 feature stride 1, "same" padding, pool ``(1, 2)`` after the first layer and ReLU; everything else uses the torch path.
@@ -77,6 +78,33 @@ def _col2im(dcol, lens_out, lens_in, cu, B, T, F, Ci, stride, pad, To, relu_z):
     return dx
 
 
+def _implicit(F: int, c: int, n: int) -> bool:
+    """
+    Whether the convolution of ``c`` to ``n`` channels over ``F`` features runs without patch matrices (``csrc/conv_implicit.cu``: 32 or 64 channels,
+    what the frontend of the Conformer configurations has); else its patches are gathered into a matrix.
+    """
+    lib = _lib.get_lib()
+    return bool(hasattr(lib, "rb200_conv3x3") and _lib.bind("rb200_conv3x3_supported", [_i32, _i32, _i32])(F, c, n))
+
+
+def _conv(x, w, bias, relu_z, y, lens_in, lens_out, cu, row_batch, row_pos, B, T, To, F, c, n, stride, pad, n_frames, back):
+    def ptr(t):
+        return t.data_ptr() if t is not None else None
+
+    _call("rb200_conv3x3", [_vp] * 10 + [_i32] * 8 + [_i64, _i32, _vp, _vp], x.data_ptr(), w.data_ptr(), ptr(bias), ptr(relu_z), y.data_ptr(),
+          lens_in.data_ptr(), ptr(lens_out), ptr(cu), ptr(row_batch), ptr(row_pos), B, T, To, F, c, n, stride, pad, n_frames, 1 if back else 0,
+          _gemm.status_tensor(x.device).data_ptr(), _lib.stream_ptr())
+    return y
+
+
+def _conv_wgrad(x, dy, lens_in, row_batch, row_pos, B, T, To, F, c, n, stride, pad, n_frames):
+    dw = torch.zeros(n, 9 * c, dtype=torch.float32, device=x.device)
+    _call("rb200_conv3x3_wgrad", [_vp] * 6 + [_i32] * 8 + [_i64, _vp, _vp], x.data_ptr(), dy.data_ptr(), dw.data_ptr(), lens_in.data_ptr(),
+          row_batch.data_ptr() if row_batch is not None else None, row_pos.data_ptr() if row_pos is not None else None, B, T, To, F, c, n, stride, pad,
+          n_frames, _gemm.status_tensor(x.device).data_ptr(), _lib.stream_ptr())
+    return dw
+
+
 def _colsum(x: torch.Tensor) -> torch.Tensor:
     """column sums of a bf16 [rows, C] matrix in fp32 (bias gradient), one pass on the native kernel"""
     lib = _lib.get_lib()
@@ -107,47 +135,69 @@ class _FrontendFn(torch.autograd.Function):
         # conv2 on the padded batch
         T2 = -(-T // s2)
         pad2 = _same_pad_left(T, 3, s2)
-        col2 = _im2col(out1, lens_dev[0], T, Fp, C1, s2, pad2, T2, None, None, B * T2)
         w2p = w2.permute(0, 2, 3, 1).reshape(C2, 9 * C1).to(bf).contiguous()
-        out2 = _gemm.gemm(col2, w2p, m=col2.shape[0], n=C2, k=9 * C1, a_mn_major=False, b_mn_major=False, bias=b2.float() if b2 is not None else None,
-                          act="relu").view(B, T2, Fp, C2)
+        b2f = b2.float().contiguous() if b2 is not None else None
+        col2 = col3 = None
+        if _implicit(Fp, C1, C2):
+            out2 = _conv(out1, w2p, b2f, None, torch.empty(B, T2, Fp, C2, dtype=bf, device=dev), lens_dev[0], None, None, None, None, B, T, T2, Fp, C1, C2,
+                         s2, pad2, B * T2, False)
+        else:
+            col2 = _im2col(out1, lens_dev[0], T, Fp, C1, s2, pad2, T2, None, None, B * T2)
+            out2 = _gemm.gemm(col2, w2p, m=col2.shape[0], n=C2, k=9 * C1, a_mn_major=False, b_mn_major=False, bias=b2f, act="relu").view(B, T2, Fp, C2)
         # conv3 for the valid output frames only: the result is already in packed-row order
         T3 = -(-T2 // s3)
         pad3 = _same_pad_left(T2, 3, s3)
         n = row_batch.shape[0]
-        col3 = _im2col(out2, lens_dev[1], T2, Fp, C2, s3, pad3, T3, row_batch, row_pos, n)
         w3p = w3.permute(0, 2, 3, 1).reshape(C3, 9 * C2).to(bf).contiguous()
-        out3 = _gemm.gemm(col3, w3p, m=col3.shape[0], n=C3, k=9 * C2, a_mn_major=False, b_mn_major=False, bias=b3.float() if b3 is not None else None,
-                          act="relu")
-        ctx.save_for_backward(x, lens_dev, cu, w1f, b1f, w2, w3, out1, col2, out2, col3, out3)
+        b3f = b3.float().contiguous() if b3 is not None else None
+        if _implicit(Fp, C2, C3):
+            out3 = _conv(out2, w3p, b3f, None, torch.empty(n * Fp, C3, dtype=bf, device=dev), lens_dev[1], None, None, row_batch, row_pos, B, T2, T3, Fp,
+                         C2, C3, s3, pad3, n, False)
+        else:
+            col3 = _im2col(out2, lens_dev[1], T2, Fp, C2, s3, pad3, T3, row_batch, row_pos, n)
+            out3 = _gemm.gemm(col3, w3p, m=col3.shape[0], n=C3, k=9 * C2, a_mn_major=False, b_mn_major=False, bias=b3f, act="relu")
+        ctx.save_for_backward(x, lens_dev, cu, row_batch, row_pos, w1f, b1f, w2, w3, out1, col2, out2, col3, out3)
         ctx.geom = (B, T, F, C1, C2, C3, T2, T3, s2, s3, pad2, pad3, n, b1 is not None, b2 is not None, b3 is not None, w1.dtype)
         return out3.view(n, Fp * C3)
 
     @staticmethod
     def backward(ctx, d_out):
-        x, lens_dev, cu, w1f, b1f, w2, w3, out1, col2, out2, col3, out3 = ctx.saved_tensors
+        x, lens_dev, cu, row_batch, row_pos, w1f, b1f, w2, w3, out1, col2, out2, col3, out3 = ctx.saved_tensors
         B, T, F, C1, C2, C3, T2, T3, s2, s3, pad2, pad3, n, has_b1, has_b2, has_b3, wdtype = ctx.geom
         Fp = F // 2
         dev = d_out.device
         bf = torch.bfloat16
         # ---- layer 3
         dz3 = torch.where(out3 > 0, d_out.reshape(n * Fp, C3).to(bf), torch.zeros((), dtype=bf, device=dev)).contiguous()
-        dw3p = torch.zeros(C3, 9 * C2, dtype=torch.float32, device=dev)
-        _gemm.gemm(dz3, col3, m=C3, n=9 * C2, k=dz3.shape[0], a_mn_major=True, b_mn_major=True, out=dw3p, atomic=True)
         db3 = _colsum(dz3) if has_b3 else None
-        # data gradient of layer 3: patch gradients on the output side, gathered back (times relu'(out2))
-        w3p = w3.permute(0, 2, 3, 1).reshape(C3, 9 * C2).to(bf).contiguous()
-        dcol3 = _gemm.gemm(dz3, w3p, m=dz3.shape[0], n=9 * C2, k=C3, a_mn_major=False, b_mn_major=True)
-        dz2 = _col2im(dcol3, lens_dev[2], lens_dev[1], cu, B, T2, Fp, C2, s3, pad3, T3, out2).view(-1, C2)
-        del dcol3
+        if col3 is None:
+            dw3p = _conv_wgrad(out2, dz3, lens_dev[1], row_batch, row_pos, B, T2, T3, Fp, C2, C3, s3, pad3, n)
+            # data gradient of layer 3 (times relu'(out2)): the convolution with the channels of the filter exchanged
+            w3b = w3.permute(1, 2, 3, 0).reshape(C2, 9 * C3).to(bf).contiguous()
+            dz2 = _conv(dz3, w3b, None, out2, torch.empty(B * T2 * Fp, C2, dtype=bf, device=dev), lens_dev[1], lens_dev[2], cu, None, None, B, T2, T3, Fp,
+                        C3, C2, s3, pad3, n, True)
+        else:
+            dw3p = torch.zeros(C3, 9 * C2, dtype=torch.float32, device=dev)
+            _gemm.gemm(dz3, col3, m=C3, n=9 * C2, k=dz3.shape[0], a_mn_major=True, b_mn_major=True, out=dw3p, atomic=True)
+            # patch gradients on the output side, gathered back
+            w3p = w3.permute(0, 2, 3, 1).reshape(C3, 9 * C2).to(bf).contiguous()
+            dcol3 = _gemm.gemm(dz3, w3p, m=dz3.shape[0], n=9 * C2, k=C3, a_mn_major=False, b_mn_major=True)
+            dz2 = _col2im(dcol3, lens_dev[2], lens_dev[1], cu, B, T2, Fp, C2, s3, pad3, T3, out2).view(-1, C2)
+            del dcol3
         # ---- layer 2
-        dw2p = torch.zeros(C2, 9 * C1, dtype=torch.float32, device=dev)
-        _gemm.gemm(dz2, col2, m=C2, n=9 * C1, k=dz2.shape[0], a_mn_major=True, b_mn_major=True, out=dw2p, atomic=True)
         db2 = _colsum(dz2) if has_b2 else None
-        w2p = w2.permute(0, 2, 3, 1).reshape(C2, 9 * C1).to(bf).contiguous()
-        dcol2 = _gemm.gemm(dz2, w2p, m=dz2.shape[0], n=9 * C1, k=C2, a_mn_major=False, b_mn_major=True)
-        d_out1 = _col2im(dcol2, lens_dev[1], lens_dev[0], None, B, T, Fp, C1, s2, pad2, T2, None)
-        del dcol2
+        if col2 is None:
+            dw2p = _conv_wgrad(out1, dz2, lens_dev[0], None, None, B, T, T2, Fp, C1, C2, s2, pad2, B * T2)
+            w2b = w2.permute(1, 2, 3, 0).reshape(C1, 9 * C2).to(bf).contiguous()
+            d_out1 = _conv(dz2, w2b, None, None, torch.empty(B, T, Fp, C1, dtype=bf, device=dev), lens_dev[0], lens_dev[1], None, None, None, B, T, T2, Fp,
+                           C2, C1, s2, pad2, B * T2, True)
+        else:
+            dw2p = torch.zeros(C2, 9 * C1, dtype=torch.float32, device=dev)
+            _gemm.gemm(dz2, col2, m=C2, n=9 * C1, k=dz2.shape[0], a_mn_major=True, b_mn_major=True, out=dw2p, atomic=True)
+            w2p = w2.permute(0, 2, 3, 1).reshape(C2, 9 * C1).to(bf).contiguous()
+            dcol2 = _gemm.gemm(dz2, w2p, m=dz2.shape[0], n=9 * C1, k=C2, a_mn_major=False, b_mn_major=True)
+            d_out1 = _col2im(dcol2, lens_dev[1], lens_dev[0], None, B, T, Fp, C1, s2, pad2, T2, None)
+            del dcol2
         # ---- layer 1: filter / bias gradient by direct reduction (pool routing and ReLU recomputed)
         dw1 = torch.zeros(C1, 9, dtype=torch.float32, device=dev)
         db1 = torch.zeros(C1, dtype=torch.float32, device=dev) if has_b1 else None
