@@ -32,52 +32,58 @@ __device__ __forceinline__ int seq_start(const int* __restrict__ lens, int b) {
 constexpr int kPadRows = 16;
 constexpr int kPadLoads = 4;
 
-// item: 8 consecutive elements of one of q/k/v of one head of one padded row
+// A thread keeps 8 columns of a row of qkv (one of q/k/v of one head) and goes down the rows, so that the position biases are read once: with items in
+// the order of memory every item of q read 16 numbers of them, 32 bytes apart from lane to lane. 8 heads of 64, 36 sequences, 7865 of 12024 rows:
+// 23.1 -> 15.2 us (out of DRAM 26.8 -> 20.4), all 12024 rows 24.8 -> 17.4, 4 x 50 rows 7.7 -> 5.0. 32 rows to a CTA: 17.6, 18.2 and 8.2 us.
 __global__ void __launch_bounds__(256)
 att_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ u, const float* __restrict__ v,
                    const int* __restrict__ lens, __nv_bfloat16* __restrict__ qu, __nv_bfloat16* __restrict__ qv, __nv_bfloat16* __restrict__ kk,
                    __nv_bfloat16* __restrict__ vv, int heads, int dim, int lp, int ctas) {
   rb_pdl_wait();  // may have been scheduled before the preceding kernel finished
   rb_pdl_launch();
-  const uint32_t groups_per_part = dim / 8;
-  const uint32_t groups_per_row = heads * 3 * groups_per_part;
   const int b = blockIdx.x / ctas;
   const int row0 = (blockIdx.x - b * ctas) * kPadRows;
   const int hd = heads * dim;
-  const int len = lens[b];
+  const int rows = min(kPadRows, lp - row0), valid = min(rows, lens[b] - row0);
   const __nv_bfloat16* src = qkv + ((long long)seq_start(lens, b) + row0) * 3 * hd;
   const long long dst0 = ((long long)b * lp + row0) * hd;
-  const uint32_t items = min(kPadRows, lp - row0) * groups_per_row;
-  for (uint32_t it0 = threadIdx.x; it0 < items; it0 += kPadLoads * 256) {
-    uint4 raw[kPadLoads];
+  for (int g = threadIdx.x; g < 3 * hd / 8; g += blockDim.x) {
+    const int h = g * 8 / (3 * dim), in_head = g * 8 - h * 3 * dim, part = in_head / dim;
+    const int c0 = h * dim + in_head - part * dim;
+    const __nv_bfloat16* from = src + g * 8;
+    float bu[8], bv[8];
 #pragma unroll
-    for (int k = 0; k < kPadLoads; ++k) {
-      const uint32_t it = it0 + k * 256, r = it / groups_per_row;
-      raw[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (it < items && row0 + (int)r < len) raw[k] = *reinterpret_cast<const uint4*>(src + (long long)it * 8);
+    for (int i = 0; i < 8; ++i) {
+      bu[i] = part == 0 && u ? u[c0 + i] : 0.f;
+      bv[i] = part == 0 && v ? v[c0 + i] : 0.f;
     }
+    __nv_bfloat16* to = (part == 0 ? qu : part == 1 ? kk : vv) + dst0 + c0;
+    __nv_bfloat16* to_v = qv + dst0 + c0;
+    for (int r0 = 0; r0 < rows; r0 += kPadLoads) {
+      uint4 raw[kPadLoads];
 #pragma unroll
-    for (int k = 0; k < kPadLoads; ++k) {
-      const uint32_t it = it0 + k * 256;
-      if (it >= items) break;
-      const uint32_t r = it / groups_per_row, g = it - r * groups_per_row;
-      const uint32_t h = g / (3 * groups_per_part), in_head = g - h * 3 * groups_per_part;
-      const uint32_t part = in_head / groups_per_part;
-      const int c0 = h * dim + (in_head - part * groups_per_part) * 8;
-      const bool valid = row0 + (int)r < len;
-      const long long dst = dst0 + (long long)r * hd + c0;
-      if (part == 0) {
-        F8 a, c;
-        const F8 x = load8(&raw[k], 0, 1);
+      for (int k = 0; k < kPadLoads; ++k) {
+        raw[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (r0 + k < valid) raw[k] = *reinterpret_cast<const uint4*>(from + (long long)(r0 + k) * 3 * hd);
+      }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          a.v[i] = valid ? x.v[i] + (u ? u[c0 + i] : 0.f) : 0.f;
-          c.v[i] = valid ? x.v[i] + (v ? v[c0 + i] : 0.f) : 0.f;
+      for (int k = 0; k < kPadLoads; ++k) {
+        if (r0 + k >= rows) break;
+        const long long at = (long long)(r0 + k) * hd;
+        if (part == 0) {
+          const bool in = r0 + k < valid;
+          F8 a, c;
+          const F8 x = load8(&raw[k], 0, 1);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            a.v[i] = in ? x.v[i] + bu[i] : 0.f;
+            c.v[i] = in ? x.v[i] + bv[i] : 0.f;
+          }
+          store8(to, at, a, 1);
+          store8(to_v, at, c, 1);
+        } else {
+          *reinterpret_cast<uint4*>(to + at) = raw[k];
         }
-        store8(qu, dst, a, 1);
-        store8(qv, dst, c, 1);
-      } else {
-        *reinterpret_cast<uint4*>((part == 1 ? kk : vv) + dst) = raw[k];
       }
     }
   }
@@ -545,7 +551,9 @@ RB_EXPORT int rb200_att_prepare(const void* qkv, const float* u, const float* v,
     rb_set_error("att_prepare: head dim %d must be a multiple of 8, batch %d x %d rows fit a launch", dim, batch, lp);
     return RB_ERR_ARG;
   }
-  rb_launch_pdl(att_prepare_kernel, dim3((unsigned)ctas * batch), dim3(256), 0, stream, (const __nv_bfloat16*)qkv, u, v, lens, (__nv_bfloat16*)qu,
+  // as many threads as share the groups of 8 columns evenly
+  const int groups = 3 * heads * dim / 8, passes = (groups + 255) / 256, threads = ((groups + passes - 1) / passes + 31) / 32 * 32;
+  rb_launch_pdl(att_prepare_kernel, dim3((unsigned)ctas * batch), dim3(threads), 0, stream, (const __nv_bfloat16*)qkv, u, v, lens, (__nv_bfloat16*)qu,
                 (__nv_bfloat16*)qv, (__nv_bfloat16*)k, (__nv_bfloat16*)vv, heads, dim, lp, ctas);
   return rb_check_launch("att_prepare");
 }
