@@ -83,7 +83,7 @@ struct Cand {
   int idx;
 };
 
-// Two kernels. (1) One CTA per hypothesis row [V] selects the row's K best logits and computes its log-sum-exp; the candidates
+// (1) One CTA per hypothesis row [V] selects the row's K best logits and computes its log-sum-exp; the candidates
 // leave as (prev + logit - lse, h * V + v), sorted. B * beam CTAs fill the machine where one CTA per batch entry left most SMs idle.
 // Selection by threshold instead of by sorting: the 256 threads form K groups, every group finds the maximum of its elements; the
 // smallest of these K maxima is a lower bound of the row's K-th largest element (K distinct elements are >= it), so only elements
@@ -91,13 +91,19 @@ struct Cand {
 // shared memory and the list is ranked by counting.
 // A row where more than kTopkCap elements pass (many equal values) takes K rounds of a block-wide argmax instead.
 // (2) One warp per batch entry merges the beam sorted lists.
+// Up to 16 hypotheses (the most CTAs of a cluster) are one kernel: the rows of a batch entry are a cluster, whose first CTA fetches the lists of the others
+// from their shared memory. Small rankings are bound by the host's launches first (12 x 10001: 15.6 us on the device, 23.8 a call; in one kernel
+// 17.9), so that is how they run; from 8 M scores on, where the device is the longer, two kernels are ahead (64 x 12 x 32000: 40.8 us, in one
+// 41.5, as the CTAs of a cluster wait for a place together). Five loads of a thread in flight where the rows have an SM each: 15.1 us of the device;
+// more rows have no registers for it (64 x 12 x 1001: 19.1 us, with five 22.7).
 constexpr int kTopkCap = 1024;
 
 __device__ __forceinline__ bool cand_before(float sa, int ia, float sb, int ib) {  // order: score descending, index ascending
   return sa > sb || (sa == sb && ia < ib);
 }
 
-template <typename F>
+// AHEAD: loads of a thread in flight
+template <int AHEAD, typename F>
 __device__ __forceinline__ void for_each_in_row(const void* logits, int is_bf16, size_t row, int V, F&& visit) {
   if (is_bf16) {
     const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(logits) + row * V;
@@ -106,13 +112,21 @@ __device__ __forceinline__ void for_each_in_row(const void* logits, int is_bf16,
     for (int v = threadIdx.x; v < head; v += kTopkThreads) visit(__bfloat162float(p[v]), v);
     const int n_vec = (V - head) >> 3;
     const uint4* pv = reinterpret_cast<const uint4*>(p + head);
-    for (int q = threadIdx.x; q < n_vec; q += kTopkThreads) {
-      const uint4 u = __ldg(pv + q);
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (int q0 = threadIdx.x; q0 < n_vec; q0 += AHEAD * kTopkThreads) {
+      uint4 u[AHEAD];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        visit(__uint_as_float(w[e] << 16), head + q * 8 + 2 * e);
-        visit(__uint_as_float(w[e] & 0xffff0000u), head + q * 8 + 2 * e + 1);
+      for (int a = 0; a < AHEAD; ++a)
+        if (a == 0 || q0 + a * kTopkThreads < n_vec) u[a] = __ldg(pv + q0 + a * kTopkThreads);
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int q = q0 + a * kTopkThreads;
+        if (a > 0 && q >= n_vec) break;
+        const uint32_t w[4] = {u[a].x, u[a].y, u[a].z, u[a].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          visit(__uint_as_float(w[e] << 16), head + q * 8 + 2 * e);
+          visit(__uint_as_float(w[e] & 0xffff0000u), head + q * 8 + 2 * e + 1);
+        }
       }
     }
     for (int v = head + n_vec * 8 + threadIdx.x; v < V; v += kTopkThreads) visit(__bfloat162float(p[v]), v);
@@ -123,20 +137,29 @@ __device__ __forceinline__ void for_each_in_row(const void* logits, int is_bf16,
     for (int v = threadIdx.x; v < head; v += kTopkThreads) visit(p[v], v);
     const int n_vec = (V - head) >> 2;
     const float4* pv = reinterpret_cast<const float4*>(p + head);
-    for (int q = threadIdx.x; q < n_vec; q += kTopkThreads) {
-      const float4 u = __ldg(pv + q);
-      visit(u.x, head + q * 4);
-      visit(u.y, head + q * 4 + 1);
-      visit(u.z, head + q * 4 + 2);
-      visit(u.w, head + q * 4 + 3);
+    for (int q0 = threadIdx.x; q0 < n_vec; q0 += AHEAD * kTopkThreads) {
+      float4 u[AHEAD];
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+        if (a == 0 || q0 + a * kTopkThreads < n_vec) u[a] = __ldg(pv + q0 + a * kTopkThreads);
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a) {
+        const int q = q0 + a * kTopkThreads;
+        if (a > 0 && q >= n_vec) break;
+        visit(u[a].x, head + q * 4);
+        visit(u[a].y, head + q * 4 + 1);
+        visit(u[a].z, head + q * 4 + 2);
+        visit(u[a].w, head + q * 4 + 3);
+      }
     }
     for (int v = head + n_vec * 4 + threadIdx.x; v < V; v += kTopkThreads) visit(p[v], v);
   }
 }
 
-__global__ void __launch_bounds__(kTopkThreads)
-beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalized, const float* __restrict__ prev_scores,
-                     const uint8_t* __restrict__ finished, int beam, int V, int eos, int K, Cand* __restrict__ cands) {
+// by a CTA: the K best of a row, in order (out: global or shared memory)
+template <int AHEAD>
+__device__ __forceinline__ void topk_row(const void* __restrict__ logits, int is_bf16, int normalized, const float* __restrict__ prev_scores,
+                                         const uint8_t* __restrict__ finished, int beam, int V, int eos, int K, Cand* out) {
   __shared__ float sh_m[kTopkThreads / 32], sh_s[kTopkThreads / 32];
   __shared__ float sh_gmax[kTopkMaxK];
   __shared__ Cand sh_c[kTopkCap];
@@ -146,7 +169,6 @@ beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalize
   const int row = blockIdx.x;  // b * beam + h
   const int h = row % beam;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Cand* out = cands + (size_t)row * K;
   const float prev = prev_scores[row];
   if (finished && finished[row]) {  // only continuation: eos at unchanged score
     if (threadIdx.x < K) {
@@ -157,7 +179,7 @@ beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalize
   }
   // pass 1: this thread's maximum, and the log-sum-exp
   float mx = -INFINITY, sum = 0.f;
-  for_each_in_row(logits, is_bf16, (size_t)row, V, [&](float x, int) {
+  for_each_in_row<AHEAD>(logits, is_bf16, (size_t)row, V, [&](float x, int) {
     if (x > mx) {
       sum = sum * __expf(mx - x) + 1.f;
       mx = x;
@@ -199,7 +221,7 @@ beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalize
   float theta = sh_gmax[0];
   for (int j = 1; j < K; ++j) theta = fminf(theta, sh_gmax[j]);
   // pass 2 (the row comes from L1 / L2 now): collect everything >= theta
-  for_each_in_row(logits, is_bf16, (size_t)row, V, [&](float x, int v) {
+  for_each_in_row<AHEAD>(logits, is_bf16, (size_t)row, V, [&](float x, int v) {
     if (x >= theta) {
       const int pos = atomicAdd(&sh_cnt, 1);
       if (pos < kTopkCap) {
@@ -234,7 +256,7 @@ beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalize
   for (int r = 0; r < K; ++r) {
     float bs = -INFINITY;
     int bi = 0x7fffffff;
-    for_each_in_row(logits, is_bf16, (size_t)row, V, [&](float x, int v) {
+    for_each_in_row<1>(logits, is_bf16, (size_t)row, V, [&](float x, int v) {
       const bool after_last = x < last_s || (x == last_s && v > last_i);
       if (after_last && cand_before(x, v, bs, bi)) {
         bs = x;
@@ -274,19 +296,11 @@ beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalize
   }
 }
 
-// one warp per batch entry: lane l owns the sorted lists of hypotheses l and l + 32; k_out rounds of a warp-wide argmax over the heads. The
-// lists are read once, into shared memory, and the heads stay in registers: a round that reads them from global memory is a trip to L2 (beam
-// 12: 9 us in 12 rounds).
-__global__ void __launch_bounds__(32)
-beam_topk_merge_kernel(const Cand* __restrict__ cands, int beam, int K, int V, float* __restrict__ out_scores, int* __restrict__ out_backref,
-                       int* __restrict__ out_label, int k_out) {
-  __shared__ Cand lists[64 * kTopkMaxK];
-  rb_pdl_wait();
-  rb_pdl_launch();
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const Cand* base = cands + (size_t)b * beam * K;
-  for (int i = lane; i < beam * K; i += 32) lists[i] = base[i];
-  __syncwarp();
+// by a warp, for one batch entry: lane l owns the sorted lists (in shared memory) of hypotheses l and l + 32; k_out rounds of a warp-wide argmax over
+// the heads, which stay in registers: a round that reads them from global memory is a trip to L2 (beam 12: 9 us in 12 rounds).
+__device__ __forceinline__ void merge_lists(const Cand* lists, int b, int beam, int K, int V, float* __restrict__ out_scores, int* __restrict__ out_backref,
+                                            int* __restrict__ out_label, int k_out) {
+  const int lane = threadIdx.x & 31;
   int hd0 = 0, hd1 = 0;
   float s0 = -INFINITY, s1 = -INFINITY;
   int i0 = -1, i1 = -1;
@@ -333,6 +347,54 @@ beam_topk_merge_kernel(const Cand* __restrict__ cands, int beam, int K, int V, f
       out_label[(size_t)b * k_out + r] = widx >= 0 ? widx % V : 0;
     }
   }
+}
+
+__global__ void __launch_bounds__(kTopkThreads)
+beam_topk_row_kernel(const void* __restrict__ logits, int is_bf16, int normalized, const float* __restrict__ prev_scores,
+                     const uint8_t* __restrict__ finished, int beam, int V, int eos, int K, Cand* __restrict__ cands) {
+  topk_row<1>(logits, is_bf16, normalized, prev_scores, finished, beam, V, eos, K, cands + (size_t)blockIdx.x * K);
+}
+
+__global__ void __launch_bounds__(32)
+beam_topk_merge_kernel(const Cand* __restrict__ cands, int beam, int K, int V, float* __restrict__ out_scores, int* __restrict__ out_backref,
+                       int* __restrict__ out_label, int k_out) {
+  __shared__ Cand lists[64 * kTopkMaxK];
+  rb_pdl_wait();
+  rb_pdl_launch();
+  const Cand* base = cands + (size_t)blockIdx.x * beam * K;
+  for (int i = threadIdx.x; i < beam * K; i += 32) lists[i] = base[i];
+  __syncwarp();
+  merge_lists(lists, blockIdx.x, beam, K, V, out_scores, out_backref, out_label, k_out);
+}
+
+// the rows of a batch entry are a cluster
+constexpr int kTopkCluster = 16;
+
+template <int AHEAD>
+__global__ void __launch_bounds__(kTopkThreads)
+beam_topk_cluster_kernel(const void* __restrict__ logits, int is_bf16, int normalized, const float* __restrict__ prev_scores,
+                         const uint8_t* __restrict__ finished, int beam, int V, int eos, int K, float* __restrict__ out_scores,
+                         int* __restrict__ out_backref, int* __restrict__ out_label, int k_out) {
+  __shared__ __align__(8) Cand mine[kTopkMaxK];
+  __shared__ Cand lists[kTopkCluster * kTopkMaxK];
+  topk_row<AHEAD>(logits, is_bf16, normalized, prev_scores, finished, beam, V, eos, K, mine);
+  // (release and acquire: the lists are in the other CTAs' shared memory)
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  const bool first = blockIdx.x % beam == 0;
+  if (first && threadIdx.x < 32) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(mine);
+    for (int i = threadIdx.x; i < beam * K; i += 32) {
+      uint32_t from;
+      uint64_t v;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(at + i % K * 8), "r"(i / K));
+      asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(from) : "memory");
+      lists[i].s = __uint_as_float((uint32_t)v);
+      lists[i].idx = (int)(v >> 32);
+    }
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");  // the lists have been read: the others may leave
+  if (first && threadIdx.x < 32) merge_lists(lists, blockIdx.x / beam, beam, K, V, out_scores, out_backref, out_label, k_out);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -464,7 +526,8 @@ RB_EXPORT int rb200_edit_distance(const int* a, const int* a_len, int lda, const
   return rb_check_launch("edit_distance");
 }
 
-// scratch: room for batch * beam * Kt candidates of 8 bytes, Kt = 8 / 16 / 32 for k <= 8 / 16 / 32 (rb200_beam_topk_scratch_bytes)
+// scratch: room for batch * beam * Kt candidates of 8 bytes, Kt = 8 / 16 / 32 for k <= 8 / 16 / 32 (rb200_beam_topk_scratch_bytes). Null, which up to
+// 16 hypotheses allow: the form in one kernel
 RB_EXPORT long long rb200_beam_topk_scratch_bytes(int batch, int beam, int k) {
   const int kt = k <= 8 ? 8 : (k <= 16 ? 16 : 32);
   return (long long)batch * beam * kt * (long long)sizeof(Cand);
@@ -473,13 +536,39 @@ RB_EXPORT long long rb200_beam_topk_scratch_bytes(int batch, int beam, int k) {
 RB_EXPORT int rb200_beam_topk(const void* logits, int is_bf16, int normalized, const float* prev_scores, const void* finished, int batch, int beam, int V,
                               int eos, int k, float* out_scores, int* out_backref, int* out_label, void* scratch, cudaStream_t stream) {
   if (batch <= 0) return RB_OK;
-  if (k < 1 || k > kTopkMaxK || beam < 1 || beam > 64 || (long long)beam * V > 0x7fffffffLL || !scratch) {
+  if (k < 1 || k > kTopkMaxK || beam < 1 || beam > 64 || (long long)beam * V > 0x7fffffffLL || (!scratch && beam > kTopkCluster)) {
     rb_set_error("beam_topk: k=%d (<= %d), beam=%d (<= 64), scratch %p", k, kTopkMaxK, beam, scratch);
     return RB_ERR_UNSUPPORTED;
   }
   Cand* cands = reinterpret_cast<Cand*>(scratch);
   const int rows = batch * beam;
   const int kt = k <= 8 ? 8 : (k <= 16 ? 16 : 32);  // candidates kept per row (the scratch is sized for this)
+  if (!scratch) {
+    static bool attr_set = false;
+    if (!attr_set && beam > 8) {  // (more than 8 CTAs of a cluster have to be asked for)
+      cudaError_t e = cudaFuncSetAttribute(beam_topk_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(beam_topk_cluster_kernel<5>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) {
+        rb_set_error("beam_topk: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+        return RB_ERR_LAUNCH;
+      }
+      attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows);
+    cfg.blockDim = dim3(kTopkThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = beam;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    // (a CTA per SM or fewer: registers for more loads in flight are there)
+    cudaLaunchKernelEx(&cfg, rows <= 148 ? beam_topk_cluster_kernel<5> : beam_topk_cluster_kernel<1>, logits, is_bf16, normalized, prev_scores, (const uint8_t*)finished, beam, V, eos, kt, out_scores,
+                       out_backref, out_label, k);
+    return rb_check_launch("beam_topk");
+  }
   beam_topk_row_kernel<<<rows, kTopkThreads, 0, stream>>>(logits, is_bf16, normalized, prev_scores, (const uint8_t*)finished, beam, V, eos, kt, cands);
   int rc = rb_check_launch("beam_topk rows");
   if (rc != RB_OK) return rc;
