@@ -51,6 +51,8 @@ int rb200_rel_flash_band(int lp, int center, int* off, int* width);
 int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o, void* dqu,
                         void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch, int heads,
                         int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream);
+int rb200_att_dkv(const void* p, const void* d_o, const void* ds, const void* q, void* dv, void* dk, const int* lens, int batch, int heads, int lp, float scale,
+                  int* status, cudaStream_t stream);
 int rb200_rel_flash_slices(long long rows, int width, int heads);
 int rb200_rel_flash_dpos(const void* band, const void* qv, void* part, const int* lens, int batch, int heads, int lp, int center, float scale, int slices,
                          int* status, cudaStream_t stream);
@@ -711,9 +713,7 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
       if (e.ok())
         e.run_tagged("rel_flash_bwd", rb200_rel_flash_bwd(sv.qu, sv.qv, sv.kk, sv.vv, sv.posp, sv.o_pad, t.do_pad, t.dqu, t.dqv, sv.w, wd, t.ds, t.dband,
                                                           nullptr, nullptr, lens, B, H, Lp, g.R, g.center, d.att_scale, p_att, status, stream));
-      const long long o_rows[10] = {(long long)H * Lp, Lp, 0, 0, Lp, 0, 0, Dh, (long long)Lp * HD, Dh};
-      e.bgemm(wd, t.do_pad, t.dv, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, 1.f, 0);
-      e.bgemm(t.ds, sv.qu, t.dk, Lp, Dh, Lp, 1, 1, Lp, HD, HD, (long long)B * H * Lp, Lp, (long long)B * Lp, HD, o_rows, B * H, H, lens, 1, 0, 1, d.att_scale, 0);
+      if (e.ok()) e.run_tagged("gemm_batched", rb200_att_dkv(wd, t.do_pad, t.ds, sv.qu, t.dv, t.dk, lens, B, H, Lp, d.att_scale, status, stream));
       if (e.ok())
         e.run_tagged("gemm_dpos", rb200_rel_flash_dpos(t.dband, sv.qv, g.slices > 1 ? (void*)t.dpos_part : t.dpos, lens, B, H, Lp, g.center, d.att_scale, g.slices,
                                                        status, stream));

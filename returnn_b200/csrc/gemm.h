@@ -40,6 +40,11 @@ struct RbGemm {
   // batched form, bf16 output without bias or activation: each problem owns whole rows of c, of ldc columns, and its rows up to the next multiple of 32.
   // c_rows > 0 (rows of the matrix that holds all problems' outputs): the output leaves in boxes of 32 x 64, what lies in them past m and n is unspecified
   long long c_rows = 0;
+  // batched form, at most 64 columns, no more of the epilogue than alpha: as many problems again, of the same shape and origins, with other operands, another
+  // output and another alpha (one launch, and the units of both share the SMs)
+  const void *a_next = nullptr, *b_next = nullptr;
+  void* c_next = nullptr;
+  float alpha_next = 1.f;
   // windows of a relative-position band (batched form): row i of a sequence of length len concerns the columns [win_center - i, win_center - i + len).
   // win = 1: the output is the band, m_from_lens; tiles of it without such a column are not computed (and not written).
   // win = 2: A, stored [k][m], is the band of sequences of win_lp rows each (a multiple of 64) with lengths win_lens, zero outside the windows;

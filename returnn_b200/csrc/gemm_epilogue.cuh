@@ -17,6 +17,8 @@ struct Params {
   int tma_store; // the output leaves through shared memory and bulk tensor stores (tensor maps of c / c2 passed to the kernel)
   int step, step_sp, step_m, step_n;  // CTA-pair kernel: from a pair's unit to its next, and the same in slices, rows and columns of tiles
   int seg_kb;    // CTA-pair kernel: K blocks per product of split operands (0: not split)
+  long long c_next;   // c_next - c in elements (a_next: g.alpha is 1, and alpha_first that of the first problems)
+  float alpha_first;
 };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -194,7 +196,7 @@ struct Unit {
   int c_r0;  // row of the stored output that row 0 of this unit's product is (slices one behind the other)
   int a_r0, a_c0, b_r0, b_c0;
   size_t c_off;
-  bool valid;
+  bool valid, next;  // next: of the problems a_next, b_next, c_next
 };
 
 template <int BM, int BN>
@@ -202,9 +204,15 @@ __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
   const RbGemm& g = p.g;
   Unit w;
   w.c_r0 = 0;
+  w.next = false;
   const int tiles = p.tiles_m * p.tiles_n;
   if (g.batch > 0) {
-    const int z = u / tiles, t = u % tiles;
+    int z = u / tiles;
+    const int t = u % tiles;
+    if (z >= g.batch) {
+      w.next = true;
+      z -= g.batch;
+    }
     const int zb = z / g.heads, zh = z % g.heads;
     const int len = g.lens ? g.lens[zb] : 0;
     w.M = g.m_from_lens ? len : g.m;
@@ -216,7 +224,7 @@ __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
     w.kb1 = K > 0 ? (K + BK - 1) / BK : 0;
     w.a_r0 = (int)(zb * g.a_rb + zh * g.a_rh); w.a_c0 = (int)(zb * g.a_cb + zh * g.a_ch);
     w.b_r0 = (int)(zb * g.b_rb + zh * g.b_rh); w.b_c0 = (int)(zb * g.b_cb + zh * g.b_ch);
-    w.c_off = (size_t)zb * g.c_sb + (size_t)zh * g.c_sh;
+    w.c_off = (size_t)zb * g.c_sb + (size_t)zh * g.c_sh + (w.next ? (size_t)p.c_next : 0);
     w.valid = w.m0 < w.M && w.n0 < w.N && w.kb1 > 0;
     if (g.win == 1) w.valid = w.valid && w.n0 < g.win_center - w.m0 + len && w.n0 + BN > g.win_center - (min(w.m0 + BM, len) - 1);
   } else {
@@ -262,7 +270,8 @@ struct BandWalk {
 // `arrive` is called by lane 0 once the warp's last read of the accumulator has completed (hands the TMEM buffer back to the
 // MMA issuer). Many narrow warps rather than few wide ones: the epilogue is latency-bound per warp (measured about 6 stall
 // cycles per issued instruction), so its throughput scales with the number of warps the schedulers can switch between.
-template <bool FULL, typename Arrive>
+// NEXT: two sets of problems, each with its alpha.
+template <bool FULL, bool NEXT = false, typename Arrive>
 __device__ __forceinline__ void epilogue_columns(const Params& p, const Unit& w, int m0, int n0, uint32_t t_addr, int c_begin, int c_end, float* stg,
                                                  int lane, int q, Arrive arrive) {
 #pragma unroll 1
@@ -293,6 +302,11 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, const Unit& w,
       const float4 a = rrow[(2 * cg) ^ sr], b = rrow[(2 * cg + 1) ^ sr];
       if (row < w.M && col < w.N) {
         float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        if (NEXT && p.g.a_next) {
+          const float alpha = w.next ? p.g.alpha_next : p.alpha_first;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] *= alpha;
+        }
         epilogue_group<FULL>(p, row, col, w.N, w.c_off, v);
       }
     }

@@ -280,9 +280,10 @@ class _RelPosFlash(torch.autograd.Function):
                       R, center, scale, p_drop, st.data_ptr(), s), "rel_flash_bwd")
         # dV = Pd^T dO, dK = scale * dS^T Qu
         dkv = torch.empty(2, rows, HD, dtype=bf, device=dev)
-        for a, b, c, alpha in ((pw, do_pad, dkv[1], 1.0), (ds, pads[0], dkv[0], scale)):
-            _bgemm(a, b, c, m=Lp, n=64, k=Lp, a_mn=True, b_mn=True, lda=Lp, ldb=HD, ldc=HD, a_shape=(B * H * Lp, Lp), b_shape=(rows, HD),
-                   offs=(H * Lp, Lp, 0, 0, Lp, 0, 0, 64, Lp * HD, 64), batch=B * H, heads=H, lens=lens, m_l=True, n_l=False, k_l=True, alpha=alpha)
+        fn = _lib.bind("rb200_att_dkv", [_vp] * 7 + [_i32] * 3 + [_f32, _vp, _vp])
+        _lib.check(fn(pw.data_ptr(), do_pad.data_ptr(), ds.data_ptr(), pads[0].data_ptr(), dkv[1].data_ptr(), dkv[0].data_ptr(), lens.data_ptr(), B, H, Lp,
+                      scale, st.data_ptr(), s), "att_dkv")
+        _lib.count_launch()
         # dP[h] = scale * band[h]^T Qv[h] over all rows of all sequences, in slices of the rows
         n = _lib.bind("rb200_rel_flash_slices", [_i64, _i32, _i32])(rows, width, H)
         part = torch.empty(n, width, HD, dtype=torch.float32 if n > 1 else bf, device=dev)
