@@ -40,6 +40,7 @@ struct Rel {
   const __nv_bfloat16* w;  // [B*H, lp, lp] (backward, saved form) probabilities
   __nv_bfloat16* p;        // [B*H, lp, lp] (backward) dropped probabilities (saved form: read)
   __nv_bfloat16 *dqu, *dqv, *band;  // (backward) where the zeros of the padding go
+  __nv_bfloat16* out;               // (forward) packed rows, the sequences back to back
   const long long* seed;
   const long long* offset;
   int* status;
@@ -210,6 +211,10 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     ok = ok && pipe_wait(w, w.out, n_tiles - 1, p.status, 29);
     rows_sync<kThreads>();
     if (ok && !*c.abort_flag) {
+      int start = 0;  // first packed row of the sequence
+      for (int i = lane; i < b; i += 32) start += p.lens[i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) start += __shfl_xor_sync(0xffffffffu, start, o);
       float acc[64];
       tmem_ld64(t_o + t_lane + wg * 64, acc);
       // merge the two groups through shared memory (the position tiles are not needed any more)
@@ -229,7 +234,17 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 64; ++j) acc[j] = row < len ? (acc[j] * e0 + ex[j] * e1) * inv : 0.f;
         store_row64_f32(squ, r, acc);  // (over both query tiles)
-        if (row < len) p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
+        if (row < len) {
+          p.lse[(long long)z * p.lp + row] = mm + __log2f(l);
+          __nv_bfloat16* out = p.out + ((long long)start + row) * (p.heads * 64) + h * 64;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            F8 x;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x.v[i] = acc[8 * j + i];
+            store8(out, 8 * j, x, 1);
+          }
+        }
       }
       fence_proxy_async_smem();
       rows_sync<kThreads>();
@@ -520,12 +535,14 @@ int failed(const char* what, cudaError_t e) {
 // o: fp32 [B, Lp, H*64], rows past a sequence's length unspecified. In 32 bits because the row sums dO . O of the backward pass are taken from
 // it: the rounding of 16-bit values would be the same for a whole row of dS, which is far more than dS where the values share an offset
 // (300 frames, values 24 + n(0, 1), keys 4 + n(0, 1): error of dQ 2.40, from 32 bits 0.12, as from the sums over P * dP; a training pass 398 -> 401 us at 36 x 333 x 8 heads)
-RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, float* o, float* lse, void* keep,
+// o [B, Lp, H*64] (fp32): valid rows written, and the last tile's zeros; out [N, H*64] (bf16, 16-byte aligned): the same rows, packed
+RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, float* o, void* out, float* lse, void* keep,
                                   const int* lens, int batch, int heads, int lp, int r_rows, int center, float scale, float p_drop,
                                   const long long* seed, const long long* offset, int* status, cudaStream_t stream) {
   if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
   const int hd = heads * 64;
   Rel p = {};
+  p.out = (__nv_bfloat16*)out;
   p.lens = lens; p.lse = lse; p.keep = (uint32_t*)keep; p.seed = seed; p.offset = offset; p.status = status;
   p.batch = batch; p.heads = heads; p.lp = lp; p.center = center; p.scale = scale; p.p_drop = p_drop;
   p.tiles = (lp + kRows - 1) / kRows;

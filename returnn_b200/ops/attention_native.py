@@ -240,13 +240,11 @@ class _RelPosFlash(torch.autograd.Function):
             off = seed[1:2].clone()
             seed[1] += B * H * Lp * Lp
         st = _gemm.status_tensor(dev)
-        fn = _lib.bind("rb200_rel_flash_fwd", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _f32, _f32, _vp, _vp, _vp, _vp])
-        _lib.check(fn(qu, qv, kk, vv, pos.data_ptr(), o_pad.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp, R, center, scale, p_drop,
-                      _p(seed), _p(off), st.data_ptr(), s), "rel_flash_fwd")
         out = torch.empty(N, HD, dtype=bf, device=dev)
-        fn = _lib.bind("rb200_att_rows_gather_f32", [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp])
-        _lib.check(fn(o_pad.data_ptr(), out.data_ptr(), row_batch.data_ptr(), row_pos.data_ptr(), N, HD, Lp, s), "att_gather")
-        _lib.count_launch(3)
+        fn = _lib.bind("rb200_rel_flash_fwd", [_vp] * 10 + [_i32, _i32, _i32, _i32, _i32, _f32, _f32, _vp, _vp, _vp, _vp])
+        _lib.check(fn(qu, qv, kk, vv, pos.data_ptr(), o_pad.data_ptr(), out.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp, R, center, scale,
+                      p_drop, _p(seed), _p(off), st.data_ptr(), s), "rel_flash_fwd")
+        _lib.count_launch(2)
         ctx.save_for_backward(pads, pos, o_pad, lse, keep, row_batch, row_pos, lens)
         ctx.dims = (B, H, Lp, R, center, N, scale, p_drop)
         ctx.u_dtype = u.dtype if u is not None else None
