@@ -33,7 +33,7 @@ struct Conv {
   const bf16* relu_z;
   const float* bias;
   bf16* y;
-  float* dw;
+  float *dw, *sums;
   int* status;
   int T, To, F, stride, pad, n_frames, src_frames, tiles, nt, groups, fk;
 };
@@ -183,7 +183,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   int* table = reinterpret_cast<int*>(sbias + N);
   const Bars s = bars_at(reinterpret_cast<uint8_t*>(table) + L::kTable);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (!BACK && (int)threadIdx.x < N) sbias[threadIdx.x] = p.bias ? p.bias[threadIdx.x] : 0.f;
+  if ((int)threadIdx.x < N) sbias[threadIdx.x] = !BACK && p.bias ? p.bias[threadIdx.x] : 0.f;  // (data gradient: the column sums)
   const uint32_t tmem = begin<256>(s, L::kStages, 4);
   // What the roles have to know of a tile is looked up by all threads for as many tiles as the table holds: { taps with a frame (none: its rows are zeros), first
   // output frame, frames of it, frames of the operand [3][nt] }. One warp looking up eight tiles ahead waited for its loads and divisions longer
@@ -197,6 +197,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   const int row = q * 32 + lane, fi = row / p.F, f = row - fi * p.F;
   uint8_t* box = staging + (warp - 2) * 32 * L::kPitch;
   uint32_t st = 0, ph = 0;  // (loading and issuing warp) stage of the ring
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // (epilogue of the data gradient) of the eight columns that this lane stores
   bool ok = true;
   if (warp == 0 && elect_one()) {
     mbar_expect_tx(s.extra, 9 * kTap);
@@ -358,10 +359,27 @@ conv_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
             }
           }
           *reinterpret_cast<uint4*>(p.y + (size_t)to[i] * N + lane % kPer * 8) = o;
+          if (BACK && p.sums) {
+            const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sum[j] += __uint_as_float(j & 1 ? ow[j >> 1] & 0xffff0000u : ow[j >> 1] << 16);
+          }
         }
         __syncwarp();
       }
     }
+  }
+  if (BACK && p.sums) {
+    if (warp >= 2) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+#pragma unroll
+        for (int o = 16; o >= N / 8; o >>= 1) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+        if (lane < N / 8) atomicAdd(&sbias[lane * 8 + j], sum[j]);
+      }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < N) atomicAdd(p.sums + threadIdx.x, sbias[threadIdx.x]);
   }
   end<256>(s, tmem);
 }
@@ -558,7 +576,8 @@ RB_EXPORT int rb200_conv3x3_supported(int f, int c, int n) { return channels_ok(
 // back == 1: y [B, T, F, n] = data gradient of that convolution (n its input channels, c its output channels), x = dY, w [n, (kt, kf, c)] the filter with
 //            its channels exchanged; dY [n_frames, F, c]: frame cu[b] + to, or b * To + to (cu null), frames at or past lens_out[b] give nothing;
 //            zeros at or past lens_in[b]; times relu'(relu_z) if that is given.
-RB_EXPORT int rb200_conv3x3(const void* x, const void* w, const float* bias, const void* relu_z, void* y, const int* lens_in, const int* lens_out, const int* cu,
+//            sums (may be null) [n] += the column sums of y.
+RB_EXPORT int rb200_conv3x3(const void* x, const void* w, const float* bias, const void* relu_z, void* y, float* sums, const int* lens_in, const int* lens_out, const int* cu,
                             const int* row_batch, const int* row_pos, int B, int T, int To, int F, int c, int n, int stride, int pad, long long n_frames,
                             int back, int* status, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || To <= 0 || (!back && n_frames <= 0)) return RB_OK;
@@ -576,7 +595,7 @@ RB_EXPORT int rb200_conv3x3(const void* x, const void* w, const float* bias, con
   Conv p;
   memset(&p, 0, sizeof(p));
   p.lens_in = lens_in; p.lens_out = lens_out; p.cu = cu; p.row_batch = row_batch; p.row_pos = row_pos;
-  p.relu_z = (const bf16*)relu_z; p.bias = bias; p.y = (bf16*)y; p.status = status;
+  p.relu_z = (const bf16*)relu_z; p.bias = bias; p.y = (bf16*)y; p.sums = sums; p.status = status;
   p.T = T; p.To = To; p.F = F; p.stride = stride; p.pad = pad; p.n_frames = (int)out_frames; p.src_frames = (int)in_frames;
   p.nt = 128 / F < 10 ? 128 / F : 10;  // (three taps in time of a tile's frames fit a warp)
   p.groups = ((T + stride - 1) / stride + p.nt - 1) / p.nt;

@@ -73,7 +73,8 @@ act_grad_colsum_kernel(const __nv_bfloat16* __restrict__ z, const __nv_bfloat16*
             const float x = v[0].v[i];
             float g;
             if (ACT == 1) {
-              g = x > 0.f ? 1.f : 0.f;
+              if (!(x > 0.f)) d[0].v[i] = 0.f;  // (also where the gradient is not finite)
+              continue;
             } else if (ACT == 2) {
               const float s = 1.f / (1.f + __expf(-x));
               g = s * (1.f + x * (1.f - s));

@@ -87,12 +87,12 @@ def _implicit(F: int, c: int, n: int) -> bool:
     return bool(hasattr(lib, "rb200_conv3x3") and _lib.bind("rb200_conv3x3_supported", [_i32, _i32, _i32])(F, c, n))
 
 
-def _conv(x, w, bias, relu_z, y, lens_in, lens_out, cu, row_batch, row_pos, B, T, To, F, c, n, stride, pad, n_frames, back):
+def _conv(x, w, bias, relu_z, y, lens_in, lens_out, cu, row_batch, row_pos, B, T, To, F, c, n, stride, pad, n_frames, back, sums=None):
     def ptr(t):
         return t.data_ptr() if t is not None else None
 
-    _call("rb200_conv3x3", [_vp] * 10 + [_i32] * 8 + [_i64, _i32, _vp, _vp], x.data_ptr(), w.data_ptr(), ptr(bias), ptr(relu_z), y.data_ptr(),
-          lens_in.data_ptr(), ptr(lens_out), ptr(cu), ptr(row_batch), ptr(row_pos), B, T, To, F, c, n, stride, pad, n_frames, 1 if back else 0,
+    _call("rb200_conv3x3", [_vp] * 11 + [_i32] * 8 + [_i64, _i32, _vp, _vp], x.data_ptr(), w.data_ptr(), ptr(bias), ptr(relu_z), y.data_ptr(),
+          ptr(sums), lens_in.data_ptr(), ptr(lens_out), ptr(cu), ptr(row_batch), ptr(row_pos), B, T, To, F, c, n, stride, pad, n_frames, 1 if back else 0,
           _gemm.status_tensor(x.device).data_ptr(), _lib.stream_ptr())
     return y
 
@@ -168,14 +168,20 @@ class _FrontendFn(torch.autograd.Function):
         dev = d_out.device
         bf = torch.bfloat16
         # ---- layer 3
-        dz3 = torch.where(out3 > 0, d_out.reshape(n * Fp, C3).to(bf), torch.zeros((), dtype=bf, device=dev)).contiguous()
-        db3 = _colsum(dz3) if has_b3 else None
+        dy3 = d_out.reshape(n * Fp, C3).to(bf).contiguous()
+        if dy3.data_ptr() % 16:
+            dy3 = dy3.clone()
+        dz3 = torch.empty_like(dy3)
+        db3 = torch.zeros(C3, dtype=torch.float32, device=dev) if has_b3 else None
+        _call("rb200_act_grad_colsum", [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp], out3.data_ptr(), dy3.data_ptr(), dz3.data_ptr(),
+              db3.data_ptr() if has_b3 else None, None, n * Fp, C3, 1, _lib.stream_ptr())
+        db2 = torch.zeros(C2, dtype=torch.float32, device=dev) if has_b2 else None
         if col3 is None:
             dw3p = _conv_wgrad(out2, dz3, lens_dev[1], row_batch, row_pos, B, T2, T3, Fp, C2, C3, s3, pad3, n)
             # data gradient of layer 3 (times relu'(out2)): the convolution with the channels of the filter exchanged
             w3b = w3.permute(1, 2, 3, 0).reshape(C2, 9 * C3).to(bf).contiguous()
             dz2 = _conv(dz3, w3b, None, out2, torch.empty(B * T2 * Fp, C2, dtype=bf, device=dev), lens_dev[1], lens_dev[2], cu, None, None, B, T2, T3, Fp,
-                        C3, C2, s3, pad3, n, True)
+                        C3, C2, s3, pad3, n, True, db2)
         else:
             dw3p = torch.zeros(C3, 9 * C2, dtype=torch.float32, device=dev)
             _gemm.gemm(dz3, col3, m=C3, n=9 * C2, k=dz3.shape[0], a_mn_major=True, b_mn_major=True, out=dw3p, atomic=True)
@@ -184,8 +190,8 @@ class _FrontendFn(torch.autograd.Function):
             dcol3 = _gemm.gemm(dz3, w3p, m=dz3.shape[0], n=9 * C2, k=C3, a_mn_major=False, b_mn_major=True)
             dz2 = _col2im(dcol3, lens_dev[2], lens_dev[1], cu, B, T2, Fp, C2, s3, pad3, T3, out2).view(-1, C2)
             del dcol3
+            db2 = _colsum(dz2) if has_b2 else None
         # ---- layer 2
-        db2 = _colsum(dz2) if has_b2 else None
         if col2 is None:
             dw2p = _conv_wgrad(out1, dz2, lens_dev[0], None, None, B, T, T2, Fp, C1, C2, s2, pad2, B * T2)
             w2b = w2.permute(1, 2, 3, 0).reshape(C1, 9 * C2).to(bf).contiguous()

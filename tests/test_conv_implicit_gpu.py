@@ -62,12 +62,15 @@ def test_conv3x3(F, c, n, stride, pad, lens, packed):
 
     for z in (None, torch.randn(B, T, F, c, device=dev).to(bf)):
         dx = torch.full((B, T, F, c), float("nan"), device=dev, dtype=bf)
+        sums = torch.ones(c, device=dev)
         fe._conv(dy, w.permute(1, 2, 3, 0).reshape(c, 9 * n).contiguous(), None, z, dx, lens_in, lens_out, cu, None, None, B, T, To, F, n, c, stride, pad,
-                 n_frames, True)
+                 n_frames, True, sums)
         ref, mag = back(full, wf), back(full.abs(), wf.abs())
         if z is not None:
             ref, mag = ref * (z > 0), mag * (z > 0)
         assert ((dx.float() - ref).abs() <= 2.0**-8 * ref.abs() + 9 * n * 2.0**-24 * mag).all()
+        cols = dx.double().view(-1, c)
+        assert ((sums.double() - 1 - cols.sum(0)).abs() <= (cols.shape[0] + 1) * 2.0**-24 * (1 + cols.abs().sum(0))).all()
 
     dyp = torch.zeros(B, To, F, n, device=dev)
     dyp[pick] = dy.float().view(-1, F, n)
