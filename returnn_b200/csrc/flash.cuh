@@ -230,6 +230,34 @@ __device__ __forceinline__ void pipe_issue(const Pipe& p, int n, int* status, Lo
   }
 }
 
+// The same with tile t + 2 being loaded while tile t's rows are at work, not after: what only `first` reads has two places, what `second` reads three.
+template <typename Load, typename First, typename Second, typename After>
+__device__ __forceinline__ void pipe_issue_ahead(const Pipe& p, int n, int* status, Load load, First first, Second second, After after) {
+  bool ok = pipe_wait(p, &p.c.full[0], 0, status, 1);
+  if (ok) {
+    first(0);
+    umma_commit_warp(p.scores);
+  }
+  for (int t = 0; t < n && ok; ++t) {
+    if (t + 1 < n) {
+      ok = pipe_wait(p, p.taken, t, status, 2) && pipe_wait(p, &p.c.full[(t + 1) & 1], (t + 1) >> 1, status, 3);
+      if (!ok) break;
+      first(t + 1);
+      umma_commit_warp(p.scores);
+    }
+    if (t + 2 < n) {  // the products of tile t that give scores and all of tile t - 1 are done
+      ok = t == 0 || pipe_wait(p, p.out, t - 1, status, 5);
+      if (!ok) break;
+      load(t + 2);
+    }
+    ok = pipe_wait(p, p.put, t, status, 4);
+    if (!ok) break;
+    second(t);
+    umma_commit_warp(p.out);
+    after(t);
+  }
+}
+
 // The output of a forward pass stays in tensor memory: the maximum that P refers to grows only when a row's has grown by more than 2^kSlack (what its
 // values are then, up to 256, costs no precision), and only then a warp takes its rows of the output out, scales them and puts them back.
 constexpr float kSlack = 8.f;

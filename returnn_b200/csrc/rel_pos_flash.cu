@@ -20,7 +20,10 @@
 //
 // Both are bound by the row work (window reads, shifts, exponentials: issue slots of the eight row warps). Loads, products and bulk stores are issued by
 // a ninth warp, which meets the rows at mbarriers only: with one of the row threads issuing, all 256 waited for it at block barriers, four times a
-// tile. The outputs stay in tensor memory and are rescaled only when a row's maximum grows by more than 2^8 (see kSlack). Kernels within the
+// tile. The outputs stay in tensor memory and are rescaled only when a row's maximum grows by more than 2^8 (see kSlack). Tile t + 2 is loaded
+// while the rows are at tile t: the windows of consecutive tiles share all but one block of 64 (forward: 128) positions, so that only that block is
+// loaded anew, and a ring of five (three) blocks leaves the room for a third tile of what both products read (rel_bwd at 36 x 333 frames 104 -> 102 us,
+// 20 x 500 frames with gradients 258 -> 252). Kernels within the
 // backward pass of 6912 rows: rel_bwd 98.3 -> 87.3 us; passes alone, forward 36 x 333 frames, 8 heads 92.0 -> 85.9 us, with gradients 323 -> 307
 // (products of dV, dK and positions included), 20 x 500 frames 305 -> 276, 300 x 40 frames 445 -> 407.
 #include "flash.cuh"
@@ -90,9 +93,9 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* squ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sqv = squ + kBig;
   uint8_t* sk = sqv + kBig;        // [2][128 keys]
-  uint8_t* sv = sk + 2 * kBig;     // [2][128 keys]
-  uint8_t* spos = sv + 2 * kBig;   // [2][256 positions]
-  uint8_t* sp = spos + 4 * kBig;   // [2 groups][128 queries][64 keys]
+  uint8_t* sv = sk + 2 * kBig;     // [3][128 keys]
+  uint8_t* spos = sv + 3 * kBig;   // [3][128 positions]: blocks of the windows, tile t's are t and t + 1
+  uint8_t* sp = spos + 3 * kBig;   // [2 groups][128 queries][64 keys]
   const Pipe w = pipe_begin<512, 8>(sp + 2 * kBig);
   const Cta& c = w.c;
   const int tid = threadIdx.x, wg = tid >> 7, r = tid & 127, lane = tid & 31;
@@ -102,28 +105,31 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     auto load = [&](int t) {
       if (!elect_one()) return;
       const int s = t & 1;
-      mbar_expect_tx(&c.full[s], (t == 0 ? 6 : 4) * kBig);
+      const int p0 = p.center - q0 - 127;  // first position of block 0
+      mbar_expect_tx(&c.full[s], (t == 0 ? 6 : 3) * kBig);
       if (t == 0) {
         tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
         tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
+        tma_load_2d(spos, &tm_pos, h * 64, p0, &c.full[0]);
       }
       tma_load_3d(sk + s * kBig, &tm_k, h * 64, t * 128, b, &c.full[s]);
-      tma_load_3d(sv + s * kBig, &tm_v, h * 64, t * 128, b, &c.full[s]);
-      tma_load_2d(spos + s * 2 * kBig, &tm_pos, h * 64, p.center + t * 128 - q0 - 127, &c.full[s]);
+      tma_load_3d(sv + t % 3 * kBig, &tm_v, h * 64, t * 128, b, &c.full[s]);
+      tma_load_2d(spos + (t + 1) % 3 * kBig, &tm_pos, h * 64, p0 + (t + 1) * 128, &c.full[s]);
     };
     load(0);
     if (n_tiles > 1) load(1);
-    pipe_issue(w, n_tiles, p.status, load,
-               [&](int t) {
-                 mma_n<128>(t_s, squ, sk + (t & 1) * kBig);
-                 mma_n<256>(t_g, sqv, spos + (t & 1) * 2 * kBig);
-               },
-               [&](int t) {
-                 const uint8_t* v = sv + (t & 1) * kBig;
-                 mma64_warp<true>(t_o, sp, v, t > 0);
-                 mma64_warp<true>(t_o + 64, sp + kBig, v + kSmall, t > 0);
-               },
-               [](int) {});
+    pipe_issue_ahead(w, n_tiles, p.status, load,
+                     [&](int t) {
+                       mma_n<128>(t_s, squ, sk + (t & 1) * kBig);
+                       mma_n<128>(t_g, sqv, spos + t % 3 * kBig);
+                       mma_n<128>(t_g + 128, sqv, spos + (t + 1) % 3 * kBig);
+                     },
+                     [&](int t) {
+                       const uint8_t* v = sv + t % 3 * kBig;
+                       mma64_warp<true>(t_o, sp, v, t > 0);
+                       mma64_warp<true>(t_o + 64, sp + kBig, v + kSmall, t > 0);
+                     },
+                     [](int) {});
   } else {
     const int row = q0 + r;
     const uint32_t t_lane = (uint32_t)(r & ~31) << 16;
@@ -301,10 +307,10 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
   uint8_t* squ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sqv = squ + kBig;
   uint8_t* sdo = sqv + kBig;
-  uint8_t* sk = sdo + kBig;          // [2][64 keys]
-  uint8_t* sv = sk + 2 * kSmall;     // [2][64 keys]
-  uint8_t* spos = sv + 2 * kSmall;   // [2][192 positions]
-  uint8_t* sds = spos + 6 * kSmall;  // [128 queries][64 keys]
+  uint8_t* sk = sdo + kBig;          // [3][64 keys]
+  uint8_t* sv = sk + 3 * kSmall;     // [2][64 keys]
+  uint8_t* spos = sv + 2 * kSmall;   // [5][64 positions]: blocks of the windows, tile t's are t to t + 2
+  uint8_t* sds = spos + 5 * kSmall;  // [128 queries][64 keys]
   uint8_t* sdg = sds + kBig;         // ring of [4][128 queries][64 positions]; first the tile of O in 32 bits
   uint8_t* sp = sdg + 4 * kBig;      // [128 queries][64 keys] dropped probabilities
   const Pipe w = pipe_begin<512, 8, 2>(sp + kBig);  // `out`: the products, and the bulk stores have read their tiles
@@ -317,15 +323,18 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     auto load = [&](int t) {
       if (!elect_one()) return;
       const int s = t & 1;
-      mbar_expect_tx(&c.full[s], 5 * kSmall + (t == 0 ? 3 * kBig : 0));
+      const int p0 = p.center - q0 - 127;  // first position of block 0
+      mbar_expect_tx(&c.full[s], 3 * kSmall + (t == 0 ? 3 * kBig + 2 * kSmall : 0));
       if (t == 0) {
         tma_load_3d(squ, &tm_qu, h * 64, q0, b, &c.full[0]);
         tma_load_3d(sqv, &tm_qv, h * 64, q0, b, &c.full[0]);
         tma_load_3d(sdo, &tm_do, h * 64, q0, b, &c.full[0]);
+        tma_load_2d(spos, &tm_pos, h * 64, p0, &c.full[0]);
+        tma_load_2d(spos + kSmall, &tm_pos, h * 64, p0 + 64, &c.full[0]);
       }
-      tma_load_3d(sk + s * kSmall, &tm_k, h * 64, t * 64, b, &c.full[s]);
+      tma_load_3d(sk + t % 3 * kSmall, &tm_k, h * 64, t * 64, b, &c.full[s]);
       tma_load_3d(sv + s * kSmall, &tm_v, h * 64, t * 64, b, &c.full[s]);
-      tma_load_2d(spos + s * 3 * kSmall, &tm_pos, h * 64, p.center + t * 64 - q0 - 127, &c.full[s]);
+      tma_load_2d(spos + (t + 2) % 5 * kSmall, &tm_pos, h * 64, p0 + (t + 2) * 64, &c.full[s]);
     };
     load(0);
     if (elect_one()) {
@@ -335,18 +344,16 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     }
     if (n_tiles > 1) load(1);
     auto blocks_done = [&](int t) { return t + 1 < n_tiles ? 1 : 3; };  // blocks of the window that are complete
-    pipe_issue(w, n_tiles, p.status, load,
+    pipe_issue_ahead(w, n_tiles, p.status, load,
                [&](int t) {
-                 const int st = t & 1;
-                 mma64_warp<false>(t_dp, sdo, sv + st * kSmall, false);
+                 mma64_warp<false>(t_dp, sdo, sv + (t & 1) * kSmall, false);
                  if (SAVED) return;
-                 mma64_warp<false>(t_s, squ, sk + st * kSmall, false);
-                 mma_n<192>(t_g, sqv, spos + st * 3 * kSmall);
+                 mma64_warp<false>(t_s, squ, sk + t % 3 * kSmall, false);
+                 for (int q = 0; q < 3; ++q) mma64_warp<false>(t_g + 64 * q, sqv, spos + (t + q) % 5 * kSmall, false);
                },
                [&](int t) {
-                 const int st = t & 1;
-                 mma64_warp<true>(t_dqu, sds, sk + st * kSmall, t > 0);
-                 for (int q = 0; q < blocks_done(t); ++q) mma64_warp<true>(t_dqv, sdg + ((t + q) & 3) * kBig, spos + (st * 3 + q) * kSmall, t > 0 || q > 0);
+                 mma64_warp<true>(t_dqu, sds, sk + t % 3 * kSmall, t > 0);
+                 for (int q = 0; q < blocks_done(t); ++q) mma64_warp<true>(t_dqv, sdg + ((t + q) & 3) * kBig, spos + (t + q) % 5 * kSmall, t > 0 || q > 0);
                },
                [&](int t) {
                  if (!elect_one()) return;
@@ -553,7 +560,7 @@ RB_EXPORT int rb200_rel_flash_fwd(const void* qu, const void* qv, const void* k,
   if (!st) st = make_map_3d(&b, qv, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 128);
   if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 128);
-  if (!st) st = map_pos(&e, pos, r_rows, hd, 256);
+  if (!st) st = map_pos(&e, pos, r_rows, hd, 128);
   if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows, true);
   if (st) return st;
   auto kernel = p_drop > 0.f ? rel_fwd_kernel<true> : rel_fwd_kernel<false>;
@@ -597,7 +604,7 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   if (!st) st = make_map_3d(&b, qv, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&c, k, hd, lp, batch, hd, bp, 64);
   if (!st) st = make_map_3d(&d, v, hd, lp, batch, hd, bp, 64);
-  if (!st) st = map_pos(&e, pos, r_rows, hd, 192);
+  if (!st) st = map_pos(&e, pos, r_rows, hd, 64);
   if (!st) st = make_map_3d(&f, o, hd, lp, batch, hd, bp, kRows, true);
   if (!st) st = make_map_3d(&g, d_o, hd, lp, batch, hd, bp, kRows);
   if (!st) st = make_map_3d(&h, dqu, hd, lp, batch, hd, bp, kRows);
