@@ -48,7 +48,7 @@ int rb200_att_rows_gather(const void* src, void* dst, const int* row_batch, cons
 int rb200_att_rows_pad(const void* src, void* dst, const int* lens, int batch, int width, int lp, cudaStream_t stream);
 int rb200_att_rows_gather_f32(const float* src, void* dst, const int* row_batch, const int* row_pos, int n_rows, int width, int lp, cudaStream_t stream);
 int rb200_rel_flash_band(int lp, int center, int* off, int* width);
-int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o, void* dqu,
+int rb200_rel_flash_bwd_sparse(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o, void* dqu,
                         void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch, int heads,
                         int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream);
 int rb200_att_dkv(const void* p, const void* d_o, const void* ds, const void* q, void* dv, void* dk, const int* lens, int batch, int heads, int lp, float scale,
@@ -711,7 +711,7 @@ RB_EXPORT int rb200_enc_backward(const RbEncDims* dims, const long long* tab, co
     const bf16* dpos = t.dpos;
     if (g.fused_bwd) {
       if (e.ok())
-        e.run_tagged("rel_flash_bwd", rb200_rel_flash_bwd(sv.qu, sv.qv, sv.kk, sv.vv, sv.posp, sv.o_pad, t.do_pad, t.dqu, t.dqv, sv.w, wd, t.ds, t.dband,
+        e.run_tagged("rel_flash_bwd", rb200_rel_flash_bwd_sparse(sv.qu, sv.qv, sv.kk, sv.vv, sv.posp, sv.o_pad, t.do_pad, t.dqu, t.dqv, sv.w, wd, t.ds, t.dband,
                                                           nullptr, nullptr, lens, B, H, Lp, g.R, g.center, d.att_scale, p_att, status, stream));
       if (e.ok()) e.run_tagged("gemm_batched", rb200_att_dkv(wd, t.do_pad, t.ds, sv.qu, t.dv, t.dk, lens, B, H, Lp, d.att_scale, status, stream));
       if (e.ok())

@@ -48,7 +48,7 @@ struct RbGemm {
   // windows of a relative-position band (batched form): row i of a sequence of length len concerns the columns [win_center - i, win_center - i + len).
   // win = 1: the output is the band, m_from_lens; tiles of it without such a column are not computed (and not written).
   // win = 2: A, stored [k][m], is the band of sequences of win_lp rows each (a multiple of 64) with lengths win_lens, zero outside the windows;
-  // the contraction leaves out blocks of 64 rows that have no such column among those of the tile. k a multiple of 64.
+  // the contraction leaves out blocks of 64 rows that have no such column among those of the tile, and does not read them. k a multiple of 64.
   int win = 0, win_center = 0, win_lp = 0;
   const int* win_lens = nullptr;
   // split operands (CTA-pair kernel only): A and B are sums hi + lo whose parts lie in ONE stored matrix each, the rows of lo seg_a / seg_b

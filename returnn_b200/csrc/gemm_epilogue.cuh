@@ -242,10 +242,11 @@ __device__ __forceinline__ Unit decode_unit(const Params& p, int u) {
 }
 
 // Walks over the K blocks of a unit whose A is a band (win = 2): which of them have a column of the tile in their window. The first is always
-// taken (it starts the accumulator). Producer and MMA issuer walk alike.
+// taken (it starts the accumulator), as zeros where it has none. Producer and MMA issuer walk alike.
 struct BandWalk {
   const RbGemm& g;
   int b, i0, len, m0, m1;
+  bool zeros = false;
   __device__ __forceinline__ BandWalk(const RbGemm& g_, const Unit& w, int bm) : g(g_), b(0), i0(0), len(0), m0(w.a_c0 + w.m0), m1(w.a_c0 + w.m0 + bm) {
     if (g.win != 2) return;
     const int rows = g.heads > 0 ? (int)(w.a_r0 % ((long long)g.batch / g.heads * g.k)) : 0;  // row within the band of one head
@@ -260,7 +261,9 @@ struct BandWalk {
       i0 = 0;
       len = g.win_lens[++b];
     }
-    return !first && (i0 >= len || g.win_center - i0 + len <= m0 || g.win_center - min(i0 + BK, len) + 1 >= m1);
+    const bool out = i0 >= len || g.win_center - i0 + len <= m0 || g.win_center - min(i0 + BK, len) + 1 >= m1;
+    zeros = first && out;
+    return !first && out;
   }
 };
 

@@ -129,19 +129,21 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         uint8_t* sa = smem + s * kStageBytes;
         uint8_t* sb = sa + kTileBytesA;
         const int k0 = kb * BK;
+        // (rows past the end of the matrix are read as zeros)
+        const int a_row = walk.zeros ? (int)g.a_rows : w.a_r0 + k0, b_row = walk.zeros ? (int)g.b_rows : w.b_r0 + k0;
         if (elect_one()) {
           mbar_expect_tx(&full_bar[s], kStageBytes);
           if (!g.a_mn_major) {
             tma_load_2d(sa, map_a, w.a_c0 + k0, w.a_r0 + m0, &full_bar[s]);
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, map_a, w.a_c0 + m0 + 64 * j, w.a_r0 + k0, &full_bar[s]);
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, map_a, w.a_c0 + m0 + 64 * j, a_row, &full_bar[s]);
           }
           if (!g.b_mn_major) {
             tma_load_2d(sb, map_b, w.b_c0 + k0, w.b_r0 + n0, &full_bar[s]);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, map_b, w.b_c0 + n0 + 64 * j, w.b_r0 + k0, &full_bar[s]);
+            for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, map_b, w.b_c0 + n0 + 64 * j, b_row, &full_bar[s]);
           }
         }
       }

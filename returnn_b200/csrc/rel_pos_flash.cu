@@ -48,6 +48,7 @@ struct Rel {
   const long long* offset;
   int* status;
   int batch, heads, lp, tiles, words, center, band_off, band_w;
+  int sparse;  // (backward) the padding is written only where the position gradient's product reads it
   float scale, p_drop;
 };
 
@@ -294,7 +295,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     }
   };
   if (q0 >= len) {  // no valid query
-    if (tid >= kThreads) return;
+    if (tid >= kThreads || p.sparse) return;
     band_zeros(0, 0);
     for (int i = tid; i < n_rows_band * 8; i += kThreads) {
       const long long at = ((long long)b * p.lp + q0 + (i >> 3)) * (p.heads * 64) + h * 64 + (i & 7) * 8;
@@ -374,7 +375,15 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
                  mbar_arrive_local(w.out);
                });
   } else {
-    band_zeros(x0, x0 + 64 * (n_tiles + 2));
+    if (p.sparse) {  // up to the next tiles of 128 columns of the product over the band, half a warp to each side
+      const int lo = x0 & ~127, hi = x0 + 64 * (n_tiles + 2), to = min((hi + 127) & ~127, p.band_w);
+      const int x = lane < 16 ? lo + lane * 8 : hi + (lane - 16) * 8;
+      if (x < (lane < 16 ? x0 : to))
+        for (int i = tid >> 5; i < n_rows_band; i += kThreads / 32)
+          *reinterpret_cast<uint4*>(p.band + (long long)(band_row + i) * p.band_w + x) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      band_zeros(x0, x0 + 64 * (n_tiles + 2));
+    }
     float lse = INFINITY, delta = 0.f;
     bool ok = pipe_wait(w, &c.full[0], 0, p.status, 26) && pipe_wait(w, c.extra, 0, p.status, 26);
     if (ok) {
@@ -585,12 +594,13 @@ RB_EXPORT int rb200_rel_flash_band(int lp, int center, int* off, int* width) {
 // dqu, dqv [B, Lp, H*64] and band [H, B, Lp, band_width]: written whole, zeros in the padding; pw, ds [B*H, Lp, Lp]: written for the first
 // 64 * ceil(len / 64) rows and columns of each sequence. With saved probabilities `w` (else null; lse and keep are not read then) pw is read:
 // the dropped probabilities, or anything without dropout
-RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
+static int rel_flash_bwd(int sparse, const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
                                   void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
                                   int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
   if (batch <= 0 || heads <= 0 || lp <= 0) return RB_OK;
   const int hd = heads * 64;
   Rel p = {};
+  p.sparse = sparse;
   p.lens = lens; p.lse = lse; p.keep = (uint32_t*)keep; p.status = status; p.w = (const __nv_bfloat16*)w; p.p = (__nv_bfloat16*)pw;
   p.dqu = (__nv_bfloat16*)dqu; p.dqv = (__nv_bfloat16*)dqv; p.band = (__nv_bfloat16*)band;
   p.batch = batch; p.heads = heads; p.lp = lp; p.center = center; p.scale = scale; p.p_drop = p_drop;
@@ -618,6 +628,21 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
   if (err != cudaSuccess) return failed("rel_flash_bwd", err);
   rb_launch_pdl(kernel, dim3((unsigned)(p.tiles * batch * heads)), dim3(kCta), kBwdSmem, stream, a, b, c, d, e, f, g, h, i, j, map_p, map_ds, p);
   return rb_check_launch("rel_flash_bwd");
+}
+
+RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
+                                  void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
+                                  int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
+  return rel_flash_bwd(0, qu, qv, k, v, pos, o, d_o, dqu, dqv, w, pw, ds, band, lse, keep, lens, batch, heads, lp, r_rows, center, scale, p_drop, status, stream);
+}
+
+// The same, of the padding only what rel_flash_dpos reads of it: the rest of the band and the rows of dqu and dqv in tiles without a valid query are
+// left as they are (zeros there were 100 of 270 MB at 36 x 334 frames of which 57 % are valid, 8 heads; kernel with saved probabilities
+// 87 -> 68 us; with recomputed ones at 36 x 333 frames 102 -> 90)
+RB_EXPORT int rb200_rel_flash_bwd_sparse(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
+                                  void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
+                                  int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
+  return rel_flash_bwd(1, qu, qv, k, v, pos, o, d_o, dqu, dqv, w, pw, ds, band, lse, keep, lens, batch, heads, lp, r_rows, center, scale, p_drop, status, stream);
 }
 
 // slices that the product of the position gradient, [band_width, rows] x [rows, 64] per head, is cut into: it has few output tiles and

@@ -272,7 +272,7 @@ class _RelPosFlash(torch.autograd.Function):
         scores = torch.empty(2, B * H * Lp, Lp, dtype=bf, device=dev)
         pw, ds = scores[0], scores[1]
         st = _gemm.status_tensor(dev)
-        fn = _lib.bind("rb200_rel_flash_bwd", [_vp] * 16 + [_i32] * 5 + [_f32, _f32, _vp, _vp])
+        fn = _lib.bind("rb200_rel_flash_bwd_sparse", [_vp] * 16 + [_i32] * 5 + [_f32, _f32, _vp, _vp])
         _lib.check(fn(pads[0].data_ptr(), pads[1].data_ptr(), pads[2].data_ptr(), pads[3].data_ptr(), pos.data_ptr(), o_pad.data_ptr(), do_pad.data_ptr(),
                       dqu.data_ptr(), dqv.data_ptr(), None, pw.data_ptr(), ds.data_ptr(), band.data_ptr(), lse.data_ptr(), _p(keep), lens.data_ptr(), B, H, Lp,
                       R, center, scale, p_drop, st.data_ptr(), s), "rel_flash_bwd")
