@@ -1,8 +1,9 @@
 // CTA-pair variant of the persistent bf16 GEMM: two CTAs of a cluster (two SMs) compute one 256 x 256 output tile with
 // tcgen05.mma.cta_group::2. Each CTA loads its own 128 rows of A and half of the B tile, so a pair moves 64 KB per K block for
-// 256 x 256 x 64 multiply-adds: two thirds of the L2->SM operand traffic per flop of the one-CTA kernel (128 x 256 tiles, 48 KB per
-// CTA and K block), which is what bounds that kernel (measured: time per K block independent of the tile width, scaling with the
-// number of active SMs).
+// 256 x 256 x 64 multiply-adds: two thirds of the operand traffic per flop of the one-CTA kernel (128 x 256 tiles, 48 KB per
+// CTA and K block). The traffic does not bound it: 148 SMs fetch 19 TB/s by TMA from the L2 (69 bytes per cycle and SM), a pair needs 64 KB per
+// 512 cycles. What does is, beside the multiplication (512 cycles per K block; 612 while one lane on its own issued it), the fixed time of a
+// product (first load 1.3 us, last epilogue 2.9, teardown 1.2, of 7.5 us at 6912 x 512 x 512) and waves of few tiles (54 on 74 pairs for n = 512).
 //
 // Roles per CTA: warp 0 = TMA producer (loads with .cta_group::2 and no multicast; they complete on the *leader's* full barrier,
 // which is armed for the bytes of both CTAs), warp 1 = TMEM allocation, and in the leader CTA (cluster rank 0) the MMA issuer,

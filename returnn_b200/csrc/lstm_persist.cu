@@ -3,8 +3,9 @@
 // that those units feed (backward), for the whole sequence. Per step a CTA multiplies the small [B, K] activation matrix (read
 // from L2, where the other CTAs wrote it in the previous step) with its resident slice on the tensor cores, applies the cell
 // for its units, publishes its slice of h_t (or dz_t) and waits for those of the others. The per-step executor in lstm.cu needs two
-// launches of latency-bound kernels per step (about 22 us); here a step of both directions takes 4.2 us forward and 5.4 us backward
-// (16 rows, H = 1024; 17.5 us together with 128 narrow CTAs per direction that met at a counter after storing what the backward pass keeps).
+// launches of latency-bound kernels per step (about 22 us); here a step of both directions, forward and backward together, takes about 7.4 us
+// (16 rows, H = 1024; 9.6 with flags and a barrier in front of the backward step's fetch, 17.5 with 128 narrow CTAs per direction that met at a
+// counter after storing what the backward pass keeps).
 //
 // The step product has only B <= 48 rows: the warp-level mma (m16n8k16, bf16 -> fp32) fits this shape (three 16-row tiles);
 // a tcgen05 tile is at least 64 rows by one CTA and its operands would have to be re-staged through TMA every step. The

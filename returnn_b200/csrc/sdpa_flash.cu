@@ -6,13 +6,15 @@
 //   flash_bwd_kv  one CTA per (batch entry, head, 128 keys): a loop over tiles of 64 queries, transposed scores, dK and dV
 //   flash_bwd_small  up to 128 queries and keys: both in one
 //
-// A CTA has 128 threads = the 128 lanes of tensor memory: a thread owns one row of the score tile (a query; in flash_bwd_kv a key) and
-// needs no exchange with others for maximum and sum. Thread 0 also issues the TMA loads (two stages) and the tcgen05.mma. The chain load ->
-// product -> softmax -> product of one CTA is serial; three (backward: two) CTAs per SM fill each other's gaps. That is why the tiles are
+// A CTA has 128 row threads = the 128 lanes of tensor memory: a thread owns one row of the score tile (a query; in flash_bwd_kv a key) and
+// needs no exchange with others for maximum and sum. A warp of its own issues the TMA loads (two stages) and the tcgen05.mma and meets the rows
+// at mbarriers only (see Pipe in flash.cuh). The chain product -> softmax -> product of one CTA is serial; three (backward: two) CTAs per SM fill
+// each other's gaps. That is why the tiles are
 // 64 wide: 128 TMEM columns and 67 KB of shared memory per CTA (backward 256 columns and 99 / 102 KB). The two-pass backward (dQ apart from
 // dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
-// The kernels are bound by that chain: no unit is saturated (8 x 1000 causal, 8 heads: tensor pipe 15 to 19 % of active cycles, special
-// functions 19 to 30 %), and the warps wait for tensor-memory loads and at the barrier. 37 + 41 + 54 us there, 40 + 51 + 68 at 250 x 100.
+// The kernels are bound by the row work of a tile (about 1450 to 1750 cycles for 64 columns: issue slots and exponentials; two threads to a row
+// gain nothing) and the length of the chain. 8 x 1000 causal, 8 heads, within a pass: 23 + 37 + 48 us with one of the row threads issuing and block
+// barriers, 19 + 32 + 41 with the issuing warp.
 //
 // Visible keys, the dropout rate and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per
 // score. They come from a stream of the generator of their own (tag 0x53; sdpa.cu and attention.cu draw from 0x51, rel_pos_flash.cu from
