@@ -395,16 +395,17 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     rows_sync<kThreads>();
     const float cs = p.scale * kLog2e;
     const float keep_scale = DROP ? 1.f / (1.f - p.p_drop) : 1.f;
-    for (int it = 0; it < n_tiles && ok; ++it) {
-      const long long at = ((long long)z * p.lp + row) * p.lp + it * 64 + wg * 32;  // this thread's 32 scores
-      uint4 wv[4], wd[4];
-      if (SAVED && row < len) {
+    uint4 wv[4], wd[4];
+    auto fetch_saved = [&](int t) {
+      const long long at = ((long long)z * p.lp + row) * p.lp + t * 64 + wg * 32;  // this thread's 32 scores
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          wv[q] = *reinterpret_cast<const uint4*>(p.w + at + 8 * q);
-          if (DROP) wd[q] = *reinterpret_cast<const uint4*>(p.p + at + 8 * q);
-        }
+      for (int q = 0; q < 4; ++q) {
+        wv[q] = *reinterpret_cast<const uint4*>(p.w + at + 8 * q);
+        if (DROP) wd[q] = *reinterpret_cast<const uint4*>(p.p + at + 8 * q);
       }
+    };
+    if (SAVED && row < len) fetch_saved(0);
+    for (int it = 0; it < n_tiles && ok; ++it) {
       uint32_t bits = 0u;
       if (DROP && !SAVED && row < len) bits = p.keep[((long long)z * p.lp + row) * p.words + it * 2 + wg];
       ok = pipe_wait(w, w.scores, it, p.status, 27);
@@ -444,6 +445,7 @@ rel_bwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
           s[j] = pd;
         }
       }
+      if (SAVED && row < len && it + 1 < n_tiles) fetch_saved(it + 1);  // (on their way until the next tile's scores are there)
       if (it > 0) {
         ok = pipe_wait(w, w.out, it - 1, p.status, 28);  // what the tile before has put has been read
         if (!ok) break;
@@ -638,7 +640,7 @@ RB_EXPORT int rb200_rel_flash_bwd(const void* qu, const void* qv, const void* k,
 
 // The same, of the padding only what rel_flash_dpos reads of it: the rest of the band and the rows of dqu and dqv in tiles without a valid query are
 // left as they are (zeros there were 100 of 270 MB at 36 x 334 frames of which 57 % are valid, 8 heads; kernel with saved probabilities
-// 87 -> 68 us; with recomputed ones at 36 x 333 frames 102 -> 90)
+// 87 -> 68 us, with the probabilities of a tile fetched during the one before 64; with recomputed ones at 36 x 333 frames 102 -> 90)
 RB_EXPORT int rb200_rel_flash_bwd_sparse(const void* qu, const void* qv, const void* k, const void* v, const void* pos, const float* o, const void* d_o,
                                   void* dqu, void* dqv, const void* w, void* pw, void* ds, void* band, float* lse, void* keep, const int* lens, int batch,
                                   int heads, int lp, int r_rows, int center, float scale, float p_drop, int* status, cudaStream_t stream) {
