@@ -6,6 +6,7 @@
 //         (q = (1-s) one-hot + s/V): what an identity with a smoothing backward between log-softmax and the loss computes.
 // The forward kernel optionally writes the arg max of each row (first index among equal maxima).
 #include "common.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -48,10 +49,14 @@ struct Chunk {
     return fmaxf(fmaxf(at(0), at(1)), fmaxf(at(2), at(3)));
   }
 };
-constexpr int kBatch = 4;  // chunks that a thread has in flight
 
-template <bool kBf16, bool kArg, bool kTot>
-__global__ void __launch_bounds__(256)
+// kBatch: chunks that a thread has in flight, kCtas: CTAs of an SM that the registers are limited for. us of a pass over bf16 rows, four chunks (40 to 56
+// registers) / four with eight CTAs / two with eight, with the sum of the row: 6001 x 32000 76.9 / 68.3 / 69.5, 6001 x 10001 41.2 / 33.6 / 31.4, 6000 x 1000
+// 17.0 / 12.1 / 10.8; without 65.0 / 62.9 / 66.4, 33.5 / 30.7 / 29.5, 12.4 / 10.9 / 10.1. As few rows as are resident at once do not gain from room for more:
+// 800 x 32000 12.7 / 13.1 / 13.0. fp32 rows have half the conversions and twice the bytes: 112.5 / 119.2 / 121.4. (Passes one after the other, a third of the
+// largest matrix still in the L2; from memory alone 6001 x 32000 takes 73.2 / 71.8.)
+template <bool kBf16, bool kArg, bool kTot, int kBatch, int kCtas>
+__global__ void __launch_bounds__(256, kCtas)
 ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, float* __restrict__ loss, float* __restrict__ lse_out,
               int v, float smoothing, int* __restrict__ argmax_out) {
   constexpr int is_bf16 = kBf16 ? 1 : 0;
@@ -207,10 +212,18 @@ RB_EXPORT int rb200_softmax_ce_fwd(const void* logits, const int* tgt, float* lo
   if (rows <= 0) return RB_OK;
   if (v < 2) return RB_ERR_ARG;
   const bool arg = argmax_out != nullptr, tot = smoothing > 0.f && mode == 0;
-  auto kernel = is_bf16 ? (arg ? (tot ? ce_fwd_kernel<true, true, true> : ce_fwd_kernel<true, true, false>)
-                               : (tot ? ce_fwd_kernel<true, false, true> : ce_fwd_kernel<true, false, false>))
-                        : (arg ? (tot ? ce_fwd_kernel<false, true, true> : ce_fwd_kernel<false, true, false>)
-                               : (tot ? ce_fwd_kernel<false, false, true> : ce_fwd_kernel<false, false, false>));
+  auto pick = [&](auto bf16, auto batch, auto ctas) {
+    constexpr bool kB = decltype(bf16)::value;
+    constexpr int kN = decltype(batch)::value, kC = decltype(ctas)::value;
+    return arg ? (tot ? ce_fwd_kernel<kB, true, true, kN, kC> : ce_fwd_kernel<kB, true, false, kN, kC>)
+               : (tot ? ce_fwd_kernel<kB, false, true, kN, kC> : ce_fwd_kernel<kB, false, false, kN, kC>);
+  };
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  using Four = std::integral_constant<int, 4>;
+  using Eight = std::integral_constant<int, 8>;
+  auto kernel = !is_bf16 ? pick(std::false_type(), Four(), One()) : v < 16384 ? pick(std::true_type(), Two(), Eight())
+                : rows > 8 * 148 ? pick(std::true_type(), Four(), Eight()) : pick(std::true_type(), Four(), One());
   kernel<<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, loss, lse, v, smoothing, argmax_out);
   return rb_check_launch("softmax_ce_fwd");
 }
