@@ -258,9 +258,10 @@ __device__ __forceinline__ void pipe_issue_ahead(const Pipe& p, int n, int* stat
   }
 }
 
-// The output of a forward pass stays in tensor memory: the maximum that P refers to grows only when a row's has grown by more than 2^kSlack (what its
-// values are then, up to 256, costs no precision), and only then a warp takes its rows of the output out, scales them and puts them back.
-constexpr float kSlack = 8.f;
+// The output of a forward pass stays in tensor memory; where a row's maximum grows, the warp takes its rows of the output out, scales them and puts them
+// back, in every tile and by any amount: P refers to the exact maximum, so that the largest weight of a row is 1 and is not rounded. (A maximum that
+// lags by up to 2^8 spares most of that, but rounds the largest weight too, an error common to the row that the sum of the weights, taken before the
+// rounding, does not have: the output of peaked rows was off by 2^-9, three times as much as with the exact maximum.)
 __device__ __forceinline__ void tmem_scale64(uint32_t addr, float factor) {
 #pragma unroll 1
   for (int part = 0; part < 4; ++part) {

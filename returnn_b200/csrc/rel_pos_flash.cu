@@ -20,7 +20,7 @@
 //
 // Both are bound by the row work (window reads, shifts, exponentials: issue slots of the eight row warps). Loads, products and bulk stores are issued by
 // a ninth warp, which meets the rows at mbarriers only: with one of the row threads issuing, all 256 waited for it at block barriers, four times a
-// tile. The outputs stay in tensor memory and are rescaled only when a row's maximum grows by more than 2^8 (see kSlack). Tile t + 2 is loaded
+// tile. The outputs stay in tensor memory, where they are rescaled with the maximum of a row (see tmem_scale64). Tile t + 2 is loaded
 // while the rows are at tile t: the windows of consecutive tiles share all but one block of 64 (forward: 128) positions, so that only that block is
 // loaded anew, and a ring of five (three) blocks leaves the room for a third tile of what both products read (rel_bwd at 36 x 333 frames 104 -> 102 us,
 // 20 x 500 frames with gradients 258 -> 252). Kernels within the
@@ -167,21 +167,10 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
         }
       }
       pipe_arrive(w.taken);
-      // the outputs stay in tensor memory, as in sdpa_flash.cu
-      const bool grow = mx > m + kSlack;
-      bool read = it == 0;  // the products of the tile before are done
-      if (__any_sync(0xffffffffu, grow)) {
-        const float to = grow ? mx : m;
-        const float corr = grow ? ex2(m - to) : 1.f;
-        m = to;
-        l *= corr;
-        if (!read) {
-          ok = pipe_wait(w, w.out, it - 1, p.status, 23);
-          if (!ok) break;
-          read = true;
-          tmem_scale64(t_o + t_lane + wg * 64, corr);
-        }
-      }
+      const bool grow = mx > m;  // (also from -inf to anything)
+      const float corr = grow ? ex2(m - mx) : 1.f;
+      if (grow) m = mx;
+      l *= corr;
       const float mu = m == -INFINITY ? 0.f : m;
       float sum = 0.f;
 #pragma unroll
@@ -207,9 +196,10 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
         }
         if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
       }
-      if (!read) {
-        ok = pipe_wait(w, w.out, it - 1, p.status, 24);  // P of the tile before has been read
+      if (it > 0) {
+        ok = pipe_wait(w, w.out, it - 1, p.status, 24);  // P of the tile before has been read, its product is in the output
         if (!ok) break;
+        if (__any_sync(0xffffffffu, grow)) tmem_scale64(t_o + t_lane + wg * 64, corr);
       }
       store_row64(sp + wg * kBig, r, s);
       fence_proxy_async_smem();

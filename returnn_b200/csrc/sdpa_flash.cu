@@ -14,7 +14,9 @@
 // dK / dV) repeats two of five products, which cost little here, and needs neither atomics nor an fp32 copy of dQ.
 // The kernels are bound by the row work of a tile (about 1450 to 1750 cycles for 64 columns: issue slots and exponentials; two threads to a row
 // gain nothing) and the length of the chain. 8 x 1000 causal, 8 heads, within a pass: 23 + 37 + 48 us with one of the row threads issuing and block
-// barriers, 19 + 32 + 41 with the issuing warp.
+// barriers, 20 + 32 + 41 with the issuing warp. The forward kernel scales its output in tensor memory, see tmem_scale64: in a row of calls 30.6 us (with
+// the output in registers 37.7). With dropout its decisions are drawn while the scores are multiplied, before those take up the registers: 61 us (after the
+// exponentials, with spills: 90).
 //
 // Visible keys, the dropout rate and the layouts are those of sdpa.cu. The dropout decisions of the forward pass are kept as one bit per
 // score. They come from a stream of the generator of their own (tag 0x53; sdpa.cu and attention.cu draw from 0x51, rel_pos_flash.cu from
@@ -94,6 +96,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
+      uint32_t bits[2] = {0u, 0u};
+      if constexpr (DROP) {  // while the scores are multiplied, and before they take up the registers
+        const uint64_t base = off + ((uint64_t)z * p.tqp + row) * p.tkp + it * kTile;
+#pragma unroll
+        for (int j = 0; j < 64; j += 4) {
+          const uint64_t ctr = base + j;
+          const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x53u, 0u));
+          const uint32_t x[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (x[e] >= thresh) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        }
+        if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
+      }
       ok = pipe_wait(w, w.scores, it, p.status, 6);
       if (!ok) break;
       float s[64];
@@ -114,20 +130,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           mx = fmaxf(mx, s[j]);
         }
       }
-      const bool grow = mx > m + kSlack;  // (also from -inf to anything)
-      bool read = it == 0;  // the products of the tile before are done
-      if (__any_sync(0xffffffffu, grow)) {
-        const float to = grow ? mx : m;
-        const float corr = grow ? ex2(m - to) : 1.f;
-        m = to;
-        l *= corr;
-        if (!read) {
-          ok = pipe_wait(w, w.out, it - 1, p.status, 7);
-          if (!ok) break;
-          read = true;
-          tmem_scale64(t_row + 64, corr);
-        }
-      }
+      const bool grow = mx > m;  // (also from -inf to anything)
+      const float corr = grow ? ex2(m - mx) : 1.f;
+      if (grow) m = mx;
+      l *= corr;
       const float mu = m == -INFINITY ? 0.f : m;
       float sum = 0.f;
 #pragma unroll
@@ -137,25 +143,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       l += sum;
       if constexpr (DROP) {
-        const uint64_t base = off + ((uint64_t)z * p.tqp + row) * p.tkp + it * kTile;
-        uint32_t bits[2] = {0u, 0u};
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) {
-          const uint64_t ctr = base + j;
-          const uint4 r = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x53u, 0u));
-          const uint32_t x[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const bool k = x[e] >= thresh;
-            s[j + e] = k ? s[j + e] * keep_scale : 0.f;
-            if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
-          }
-        }
-        if (row < p.tq) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.tq + row) * p.words + it * 2) = make_uint2(bits[0], bits[1]);
+        for (int j = 0; j < 64; ++j) s[j] = bits[j >> 5] >> (j & 31) & 1u ? s[j] * keep_scale : 0.f;
       }
-      if (!read) {
-        ok = pipe_wait(w, w.out, it - 1, p.status, 7);  // P of the tile before has been read
+      if (it > 0) {
+        ok = pipe_wait(w, w.out, it - 1, p.status, 7);  // P of the tile before has been read, its product is in the output
         if (!ok) break;
+        if (__any_sync(0xffffffffu, grow)) tmem_scale64(t_row + 64, corr);
       }
       store_row64(sp, tid, s);
       fence_proxy_async_smem();
