@@ -194,8 +194,8 @@ struct Linear : Function<Linear> {
     const Tensor w = weight.to(at::kBFloat16).contiguous();
     const int64_t m = x2.size(0), k = x2.size(1), n = w.size(1);
     Tensor y = fresh({m, n}, x2, at::kBFloat16), z;
-    // (a parameter says that it requires a gradient under no_grad as well)
-    if (act && differentiable && (x2.requires_grad() || weight.requires_grad())) {
+    // (a parameter says that it requires a gradient under no_grad as well; that of the bias alone needs the pre-activation too)
+    if (act && differentiable && (x2.requires_grad() || weight.requires_grad() || (bias.has_value() && bias->requires_grad()))) {
       z = fresh({m, n}, x2, at::kBFloat16);
       gemm(x2, w, z, &y, bias, m, n, k, false, true, (int)act, status);
     } else {

@@ -191,8 +191,8 @@ class _LinearFn(torch.autograd.Function):
         w = weight.to(torch.bfloat16).contiguous()
         m, k = x2.shape
         n = w.shape[1]
-        # (a parameter says that it requires a gradient under no_grad as well)
-        need_z = act is not None and differentiable and (x2.requires_grad or weight.requires_grad)
+        # (a parameter says that it requires a gradient under no_grad as well; that of the bias alone needs the pre-activation too)
+        need_z = act is not None and differentiable and any(t is not None and t.requires_grad for t in (x2, weight, bias))
         if need_z:
             z, y = gemm(x2, w, m=m, n=n, k=k, a_mn_major=False, b_mn_major=True, bias=bias, act=act, want_act_output=True)
         else:

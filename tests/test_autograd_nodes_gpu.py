@@ -53,7 +53,8 @@ def test_layer_norm(monkeypatch, shape, dtype, w_dtype, beta, rms):
 @pytest.mark.parametrize("shape,n,w_dtype,bias,act,grads", [
     ((3, 40, 64), 72, torch.float32, torch.float32, "silu", (1, 1, 1)), ((2048, 64), 64, torch.float32, torch.bfloat16, None, (0, 1, 1)),
     ((1, 512), 512, torch.bfloat16, None, "gelu", (1, 0, 0)), ((130, 64), 136, torch.bfloat16, torch.float16, "relu", (1, 1, 0)),
-    ((64, 16), 8, torch.float32, torch.float32, "relu", (0, 0, 0))])
+    ((64, 16), 8, torch.float32, torch.float32, "relu", (0, 0, 0)), ((70, 64), 72, torch.float32, torch.float32, "silu", (0, 0, 1)),
+    ((70, 64), 72, torch.bfloat16, torch.bfloat16, "relu", (0, 0, 1))])
 def test_linear(monkeypatch, shape, n, w_dtype, bias, act, grads):
     from returnn_b200.ops.gemm import linear_bf16
 
