@@ -175,7 +175,7 @@ Tensor grad_pre_elementwise(const Tensor& dy, const Tensor& z, int act, const Te
   if (act) {
     const Tensor zf = z.to(at::kFloat), d = dy.to(at::kFloat);
     if (act == 1) {
-      dz = (d * (zf > 0)).to(dy.scalar_type());
+      dz = at::where(zf > 0, dy, at::zeros({}, dy.options()));  // (also where the gradient is not finite)
     } else if (act == 2) {
       const Tensor s = at::sigmoid(zf);
       dz = (d * (s * (1 + zf * (1 - s)))).to(dy.scalar_type());

@@ -120,7 +120,7 @@ def _ok_operand(t: torch.Tensor) -> bool:
 def _act_grad(z: torch.Tensor, dy: torch.Tensor, act: str) -> torch.Tensor:
     zf = z.float()
     if act == "relu":
-        return (dy.float() * (zf > 0)).to(dy.dtype)
+        return torch.where(zf > 0, dy, torch.zeros((), dtype=dy.dtype, device=dy.device))  # (also where the gradient is not finite)
     if act in ("silu", "swish"):
         s = torch.sigmoid(zf)
         return (dy.float() * (s * (1 + zf * (1 - s)))).to(dy.dtype)

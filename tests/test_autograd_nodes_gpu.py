@@ -64,6 +64,26 @@ def test_linear(monkeypatch, shape, n, w_dtype, bias, act, grads):
     _same(a, b)
 
 
+@pytest.mark.parametrize("start", [0, 1])
+def test_relu_gradient_that_is_not_finite(monkeypatch, start):
+    """zero where the activation is zero, also where the gradient there is not finite, and for gradients off the alignment of the kernel"""
+    from returnn_b200.ops.gemm import linear_bf16
+
+    x, w, b = _rand(40, 64), _rand(64, 72, dtype=torch.float32, seed=1), _rand(72, dtype=torch.float32, seed=2)
+    off = linear_bf16(x, w, b, "relu").detach() == 0
+
+    def grad(bad):
+        dy = torch.zeros(start + off.numel(), dtype=torch.bfloat16, device="cuda")[start:].view_as(off)
+        dy[off] = torch.tensor(bad, dtype=torch.bfloat16, device="cuda").repeat(off.numel())[: int(off.sum())]
+        dy[~off] = 0.5
+        return dy
+
+    res = [_both(monkeypatch, lambda x, w, b: linear_bf16(x, w, b, "relu"), [x, w, b], lambda y: grad(bad))
+           for bad in ([1.0], [float("inf"), float("nan"), float("-inf")])]
+    for a, b in zip(*res):
+        _same(a, b)
+
+
 @pytest.mark.parametrize("lens,taps,affine,stats", [([5, 0, 33], 32, True, True), ([1], 7, False, True), ([40, 41], 33, True, False)])
 def test_conv_module(monkeypatch, lens, taps, affine, stats):
     from types import SimpleNamespace as NS
