@@ -3,7 +3,7 @@ Build the native libraries in-tree:
 
 - ``_build/librb200.so``: all CUDA kernels, compiled for sm_100a only
   (``nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo``); nvcc cross-compiles without a GPU.
-- ``_build/_autograd_nodes.so``: autograd nodes in C++ that launch them (g++, against the installed torch).
+- ``_build/_autograd_nodes-<versions>.so``: autograd nodes in C++ that launch them (g++, against the installed torch, whose version the name carries).
 - ``_build/librb200_host.so`` and ``_build/librb200_atfork.so``: host-only helpers (g++).
 
 ``python -m returnn_b200.ops.build [--force] [--verbose]``. Sources are compiled in parallel; objects are cached by
@@ -122,6 +122,7 @@ def build_nodes(force: bool = False, verbose: bool = False) -> Optional[str]:
     """compile the autograd nodes (``csrc/pyext/autograd_nodes.cpp``) against torch and ``librb200.so``; None without a CUDA build of torch"""
     import sysconfig
     import torch
+    from . import nodes
 
     src = os.path.join(_CSRC, "pyext", "autograd_nodes.cpp")
     kernels = os.path.join(_BUILD, "librb200.so")
@@ -129,7 +130,10 @@ def build_nodes(force: bool = False, verbose: bool = False) -> Optional[str]:
     nvcc = _nvcc()
     if not (torch.version.cuda and nvcc and os.path.exists(src) and os.path.exists(kernels)):
         return None
-    lib = os.path.join(_BUILD, "_autograd_nodes.so")
+    lib = os.path.join(_BUILD, nodes.file_name())
+    for old in glob.glob(os.path.join(glob.escape(_BUILD), "_autograd_nodes*.so")):
+        if old != lib:
+            os.remove(old)
     # (the kernel library is linked by name: its code may change without a new link)
     if force or _newer(lib, [src, os.path.join(root, "version.py")]):
         inc = [sysconfig.get_paths()["include"], os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
