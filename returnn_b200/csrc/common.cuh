@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "per_device.h"
 
 #define RB_EXPORT extern "C" __attribute__((visibility("default")))
 

@@ -519,14 +519,14 @@ int launch_conv(const CUtensorMap& tm_x, const CUtensorMap& tm_run, const void* 
   if (st) return st;
   constexpr int smem = ConvLayout<C, N>::kSmem;
   static_assert(smem <= 227 * 1024, "shared memory");
-  static bool attr_set = false;
-  if (!attr_set) {
+  static RbPerDevice attr_set;
+  if (attr_set.needed()) {
     cudaError_t e = cudaFuncSetAttribute(conv_kernel<C, N, BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {
       rb_set_error("conv3x3: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return RB_ERR_LAUNCH;
     }
-    attr_set = true;
+    attr_set.done();
   }
   const int grid = p.tiles < num_sms() ? p.tiles : num_sms();
   conv_kernel<C, N, BACK><<<grid, kThreads, smem, stream>>>(tm_x, tm_run, tm_w, p);
@@ -535,14 +535,14 @@ int launch_conv(const CUtensorMap& tm_x, const CUtensorMap& tm_run, const void* 
 
 template <int C, int N>
 int launch_wgrad(const CUtensorMap& tm_x, const CUtensorMap& tm_dy, const Conv& p, cudaStream_t stream) {
-  static bool attr_set = false;
-  if (!attr_set) {
+  static RbPerDevice attr_set;
+  if (attr_set.needed()) {
     cudaError_t e = cudaFuncSetAttribute(wgrad_kernel<C, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgradSmem);
     if (e != cudaSuccess) {
       rb_set_error("conv3x3_wgrad: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return RB_ERR_LAUNCH;
     }
-    attr_set = true;
+    attr_set.done();
   }
   const int smem = wgrad_stages(C, N, p.fk) * wgrad_stage(C, N, p.fk) + wgrad_tail(C, N, p.fk) + 2048;
   const int grid = p.n_frames < num_sms() ? p.n_frames : num_sms();

@@ -877,11 +877,11 @@ RB_EXPORT int rb200_glu_dwconv_fwd(const void* x, const float* filt, const float
     return RB_ERR_ARG;
   }
   if (K <= KM2) {
-    static bool attr2 = false;
-    if (!attr2) {
+    static RbPerDevice attr2;
+    if (attr2.needed()) {
       cudaFuncSetAttribute(glu_dwconv_fwd2_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
       cudaFuncSetAttribute(glu_dwconv_fwd2_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
-      attr2 = true;
+      attr2.done();
     }
     const Pieces pc = pieces_of(n_rows, n_seqs, C, K, kFwdCtas);
     rb_launch_pdl(K <= 16 ? glu_dwconv_fwd2_kernel<16> : glu_dwconv_fwd2_kernel<32>, dim3(pc.n, C / CC), dim3(kWinThreads), kFwd2Smem, stream,
@@ -960,11 +960,11 @@ RB_EXPORT int rb200_glu_dwconv_bwd_ex(const void* x, const void* dy, const float
   if (row_ctas > n_tiles) row_ctas = n_tiles;
   dim3 grid(row_ctas, C / CC);
   if (K <= KM2) {
-    static bool attr2 = false;
-    if (!attr2) {
+    static RbPerDevice attr2;
+    if (attr2.needed()) {
       for (auto kernel : {glu_dwconv_bwd2_kernel<16, false>, glu_dwconv_bwd2_kernel<32, false>, glu_dwconv_bwd2_kernel<16, true>, glu_dwconv_bwd2_kernel<32, true>})
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwd2Smem);
-      attr2 = true;
+      attr2.done();
     }
     const Pieces pc = pieces_of(n_rows, n_seqs, C, K, kBwdCtas);
     row_ctas = pc.walkers;  // every CTA leaves one partial
@@ -978,10 +978,10 @@ RB_EXPORT int rb200_glu_dwconv_bwd_ex(const void* x, const void* dy, const float
     rb_launch_pdl(dwconv_bwd_reduce2_kernel, dim3((C * (K + 1) + 31) / 32), dim3(256), 0, stream, part, row_ctas, C, K, dfilt, dbias, accumulate);
     return rb_check_launch("dwconv_bwd_reduce2");
   } else {
-    static bool attr = false;
-    if (!attr) {
+    static RbPerDevice attr;
+    if (attr.needed()) {
       cudaFuncSetAttribute(glu_dwconv_bwd_kernel<KMAX>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      attr = true;
+      attr.done();
     }
     glu_dwconv_bwd_kernel<KMAX><<<grid, kThreads, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, filt, row_batch, row_pos, lens,
                                                                (__nv_bfloat16*)dx, part, n_rows, C, K);

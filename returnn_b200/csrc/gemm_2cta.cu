@@ -374,8 +374,8 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
   static const Kernel kernels[] = {gemm_pair_kernel<kEpiSome>,  gemm_pair_kernel<kEpiAny>,       gemm_pair_kernel<kEpiPlain>, gemm_pair_kernel<kEpiF32>,
                                    gemm_pair_kernel<kEpiTwo>,   gemm_pair_kernel<kEpiTwoDrop>,   gemm_pair_kernel<kEpiResid>, gemm_pair_kernel<kEpiResidDrop>,
                                    gemm_pair_kernel<kEpiDact>,  gemm_pair_kernel<kEpiDactDrop>};
-  static bool attr_set = false;
-  if (!attr_set) {
+  static RbPerDevice attr_set;
+  if (attr_set.needed()) {
     for (const Kernel k : kernels) {
       const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
       if (e != cudaSuccess) {
@@ -383,7 +383,7 @@ int rb_gemm_pair(const RbGemm& g, cudaStream_t stream) {
         return RB_ERR_LAUNCH;
       }
     }
-    attr_set = true;
+    attr_set.done();
   }
   Params p;
   p.g = g;

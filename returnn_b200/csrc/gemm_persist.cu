@@ -260,15 +260,15 @@ template <int BN, int CTAS>
 int launch(const RbGemm& g, cudaStream_t stream) {
   using L = Layout<BN, CTAS>;
   constexpr bool kFull = CTAS == 1;  // several CTAs per SM: the plain epilogue only
-  static bool attr_set = false;
-  if (!attr_set) {
+  static RbPerDevice attr_set;
+  if (attr_set.needed()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_persist_kernel<BN, false, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (kFull && e == cudaSuccess) e = cudaFuncSetAttribute(gemm_persist_kernel<BN, kFull, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) {
       rb_set_error("gemm: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return RB_ERR_LAUNCH;
     }
-    attr_set = true;
+    attr_set.done();
   }
   Params p;
   p.g = g;

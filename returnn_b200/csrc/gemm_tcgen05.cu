@@ -275,14 +275,14 @@ static int launch_gemm(const void* a, const void* b, long long a_rows, long long
     rb_set_error("gemm: accumulate needs fp32 output");
     return RB_ERR_ARG;
   }
-  static bool attr_set = false;
-  if (!attr_set) {
+  static RbPerDevice attr_set;
+  if (attr_set.needed()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) {
       rb_set_error("gemm: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return RB_ERR_LAUNCH;
     }
-    attr_set = true;
+    attr_set.done();
   }
   CUtensorMap tm_a, tm_b;
   int st;

@@ -492,15 +492,15 @@ static int ln_bwd_acc(const void* x, const void* dy, const void* gamma, const fl
   if (ctas > 148) ctas = 148;
   const size_t sm = (size_t)kBwdAccWarps * kBwdAccDepth * 3 * n * sizeof(__nv_bfloat16);  // >= the [warps][3][n] fp32 it becomes at the end
   const int ch = (n + 255) / 256;
-  static bool attr_set[2][2] = {{false, false}, {false, false}};
+  static RbPerDevice attr_set[2][2];
 #define LN_ACC(C, B)                                                                                                                    \
   do {                                                                                                                                  \
-    if (!attr_set[C - 1][B]) {                                                                                                          \
+    if (attr_set[C - 1][B].needed()) {                                                                                                  \
       if (cudaFuncSetAttribute(ln_bwd_acc_kernel<C, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)kBwdAccWarps * kBwdAccDepth * 3 * 512 * 2)) != cudaSuccess) { \
         rb_set_error("layer_norm_bwd_acc: cannot reserve shared memory");                                                               \
         return RB_ERR_LAUNCH;                                                                                                           \
       }                                                                                                                                 \
-      attr_set[C - 1][B] = true;                                                                                                        \
+      attr_set[C - 1][B].done();                                                                                                        \
     }                                                                                                                                   \
     rb_launch_pdl(ln_bwd_acc_kernel<C, B>, dim3(ctas), dim3(kBwdAccWarps * 32), sm, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, gamma, mean, rstd, \
                   (__nv_bfloat16*)dx, dgamma, dbeta, rows, n, w_bf16, rms, (const __nv_bfloat16*)dres, done, gamma_out, beta_out, branch ? *branch : LnBranch{});     \

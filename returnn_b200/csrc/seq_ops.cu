@@ -517,10 +517,10 @@ RB_EXPORT int rb200_edit_distance(const int* a, const int* a_len, int lda, const
   }
   const int warps = 4;
   const size_t smem = (size_t)warps * 2 * (kEdMaxLen + 1) * sizeof(int);
-  static bool attr = false;
-  if (!attr) {
+  static RbPerDevice attr;
+  if (attr.needed()) {
     cudaFuncSetAttribute(edit_distance_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
+    attr.done();
   }
   edit_distance_kernel<<<(batch + warps - 1) / warps, warps * 32, smem, stream>>>(a, a_len, lda, b, b_len, ldb, out, batch);
   return rb_check_launch("edit_distance");
@@ -544,15 +544,15 @@ RB_EXPORT int rb200_beam_topk(const void* logits, int is_bf16, int normalized, c
   const int rows = batch * beam;
   const int kt = k <= 8 ? 8 : (k <= 16 ? 16 : 32);  // candidates kept per row (the scratch is sized for this)
   if (!scratch) {
-    static bool attr_set = false;
-    if (!attr_set && beam > 8) {  // (more than 8 CTAs of a cluster have to be asked for)
+    static RbPerDevice attr_set;
+    if (beam > 8 && attr_set.needed()) {  // (more than 8 CTAs of a cluster have to be asked for)
       cudaError_t e = cudaFuncSetAttribute(beam_topk_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(beam_topk_cluster_kernel<5>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e != cudaSuccess) {
         rb_set_error("beam_topk: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         return RB_ERR_LAUNCH;
       }
-      attr_set = true;
+      attr_set.done();
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows);
