@@ -527,10 +527,46 @@ RB_EXPORT int rb200_edit_distance(const int* a, const int* a_len, int lda, const
 }
 
 // scratch: room for batch * beam * Kt candidates of 8 bytes, Kt = 8 / 16 / 32 for k <= 8 / 16 / 32 (rb200_beam_topk_scratch_bytes). Null, which up to
-// 16 hypotheses allow: the form in one kernel
+// 16 hypotheses allow where rb200_beam_topk_cluster_fits: the form in one kernel
 RB_EXPORT long long rb200_beam_topk_scratch_bytes(int batch, int beam, int k) {
   const int kt = k <= 8 ? 8 : (k <= 16 ? 16 : 32);
   return (long long)batch * beam * kt * (long long)sizeof(Cand);
+}
+
+// the attribute that clusters of more than 8 CTAs need, on the current device
+static cudaError_t allow_large_clusters() {
+  static RbPerDevice set;
+  if (!set.needed()) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(beam_topk_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(beam_topk_cluster_kernel<5>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) set.done();
+  return e;
+}
+
+static cudaLaunchConfig_t cluster_config(int rows, int beam, cudaLaunchAttribute* attr, cudaStream_t stream) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = beam;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows);
+  cfg.blockDim = dim3(kTopkThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// whether the current device can place the clusters of the form in one kernel: beyond 8 CTAs that is not promised (parts of a device, fewer SMs in a
+// group of them). 0 too where it cannot be asked
+RB_EXPORT int rb200_beam_topk_cluster_fits(int beam) {
+  if (beam < 1 || beam > kTopkCluster) return 0;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config(beam, beam, &attr, nullptr);
+  int a = 0, b = 0;
+  const bool ok = (beam <= 8 || allow_large_clusters() == cudaSuccess) && cudaOccupancyMaxActiveClusters(&a, beam_topk_cluster_kernel<1>, &cfg) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&b, beam_topk_cluster_kernel<5>, &cfg) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok && a > 0 && b > 0;
 }
 
 RB_EXPORT int rb200_beam_topk(const void* logits, int is_bf16, int normalized, const float* prev_scores, const void* finished, int batch, int beam, int V,
@@ -544,26 +580,13 @@ RB_EXPORT int rb200_beam_topk(const void* logits, int is_bf16, int normalized, c
   const int rows = batch * beam;
   const int kt = k <= 8 ? 8 : (k <= 16 ? 16 : 32);  // candidates kept per row (the scratch is sized for this)
   if (!scratch) {
-    static RbPerDevice attr_set;
-    if (beam > 8 && attr_set.needed()) {  // (more than 8 CTAs of a cluster have to be asked for)
-      cudaError_t e = cudaFuncSetAttribute(beam_topk_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(beam_topk_cluster_kernel<5>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) {
-        rb_set_error("beam_topk: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        return RB_ERR_LAUNCH;
-      }
-      attr_set.done();
+    const cudaError_t e = beam > 8 ? allow_large_clusters() : cudaSuccess;  // (more than 8 CTAs of a cluster have to be asked for)
+    if (e != cudaSuccess) {
+      rb_set_error("beam_topk: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return RB_ERR_LAUNCH;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(rows);
-    cfg.blockDim = dim3(kTopkThreads);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = beam;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(rows, beam, &attr, stream);
     // (a CTA per SM or fewer: registers for more loads in flight are there)
     cudaLaunchKernelEx(&cfg, rows <= 148 ? beam_topk_cluster_kernel<5> : beam_topk_cluster_kernel<1>, logits, is_bf16, normalized, prev_scores, (const uint8_t*)finished, beam, V, eos, kt, out_scores,
                        out_backref, out_label, k);

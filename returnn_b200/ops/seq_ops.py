@@ -11,6 +11,7 @@ Sequence utility ops with B200 kernels (``csrc/seq_ops.cu``) and plain torch / n
 from __future__ import annotations
 from typing import Dict, List, Optional, Tuple
 import ctypes
+import functools
 import torch
 from . import _lib
 
@@ -105,6 +106,16 @@ def beam_topk_reference(logits, prev_scores, finished, eos: int, k: int, normali
     return top, (idx // V).to(torch.int32), (idx % V).to(torch.int32)
 
 
+@functools.lru_cache(maxsize=None)
+def _beam_cluster_fits(device: int, beam: int) -> bool:
+    """whether the GPU of this index can place clusters of as many CTAs as there are hypotheses; asked once per device and size"""
+    lib = _lib.get_lib()
+    if not hasattr(lib, "rb200_beam_topk_cluster_fits") or not 0 <= device < torch.cuda.device_count():
+        return False
+    with torch.cuda.device(device):
+        return bool(_lib.bind("rb200_beam_topk_cluster_fits", [_i32])(beam))
+
+
 def beam_topk(logits: torch.Tensor, prev_scores: torch.Tensor, *, finished: Optional[torch.Tensor] = None, eos: int = 0, k: int,
               normalized: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """
@@ -127,7 +138,7 @@ def beam_topk(logits: torch.Tensor, prev_scores: torch.Tensor, *, finished: Opti
         kt = 8 if k <= 8 else (16 if k <= 16 else 32)
         # (score, index) per candidate of the per-row stage; without it the stages are one kernel: up to 16 hypotheses, and below the sizes where
         # the device takes longer than the launches
-        one = beam <= 16 and B * beam * V <= 8000000
+        one = beam <= 16 and B * beam * V <= 8000000 and _beam_cluster_fits(torch._C._cuda_getDevice(), beam)
         scratch = None if one else torch.empty(B * beam * kt * 2, dtype=torch.int32, device=dev)
         fn = _lib.bind("rb200_beam_topk", [_vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp])
         _lib.check(fn(lg.data_ptr(), 1 if lg.dtype == torch.bfloat16 else 0, 1 if normalized else 0, ps.data_ptr(),
