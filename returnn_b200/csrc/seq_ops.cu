@@ -91,10 +91,9 @@ struct Cand {
 // shared memory and the list is ranked by counting.
 // A row where more than kTopkCap elements pass (many equal values) takes K rounds of a block-wide argmax instead.
 // (2) One warp per batch entry merges the beam sorted lists.
-// Up to 16 hypotheses (the most CTAs of a cluster) are one kernel: the rows of a batch entry are a cluster, whose first CTA fetches the lists of the others
-// from their shared memory. Small rankings are bound by the host's launches first (12 x 10001: 15.6 us on the device, 23.8 a call; in one kernel
-// 17.9), so that is how they run; from 8 M scores on, where the device is the longer, two kernels are ahead (64 x 12 x 32000: 40.8 us, in one
-// 41.5, as the CTAs of a cluster wait for a place together). Five loads of a thread in flight where the rows have an SM each: 15.1 us of the device;
+// Up to 16 hypotheses (the most CTAs of a cluster) can be one kernel: the rows of a batch entry are a cluster, whose first CTA fetches the lists of the others
+// from their shared memory. It saves a launch and the scratch of rankings that are bound by the host (12 x 10001: 18.7 us a call, now 16.6); which
+// form runs is decided where it is called (ops/seq_ops.py). Five loads of a thread in flight where the rows have an SM each: 15.1 us of the device;
 // more rows have no registers for it (64 x 12 x 1001: 19.1 us, with five 22.7).
 constexpr int kTopkCap = 1024;
 

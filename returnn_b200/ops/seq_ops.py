@@ -116,6 +116,32 @@ def _beam_cluster_fits(device: int, beam: int) -> bool:
         return bool(_lib.bind("rb200_beam_topk_cluster_fits", [_i32])(beam))
 
 
+def _beam_one_kernel(B: int, beam: int, V: int, item: int) -> bool:
+    """
+    Whether a ranking runs as one kernel (a cluster of CTAs per batch entry) or as two. One launch and no scratch save 4 us of the host's time, the
+    bound of small rankings. Clusters are placed as a whole, several CTAs to an SM where single ones would spread, and meet twice: the larger they
+    are and the more rows and scores there are, the sooner the device takes longer than that. us a call, two kernels / one, bf16:
+    beam 4: 32 x 32000 18.6 / 14.6, 64 x 32000 18.6 / 18.7; beam 8: 12 x 32000 18.9 / 16.6, 16 x 32000 19.2 / 20.7, 32 x 10001 18.7 / 14.6,
+    64 x 10001 18.8 / 18.6; beam 12: 4 x 32000 22.8 / 20.7, 12 x 32000 22.8 / 24.8, 8 x 10001 18.9 / 18.6, 24 x 10001 19.2 / 20.7; beam 16: 2 x 32000
+    24.8 / 22.8, 8 x 32000 24.8 / 26.8, 4 x 10001 20.7 / 20.4, 8 x 10001 19.3 / 20.7, 2 x 5001 17.9 / 18.6. Rows of fewer bytes than the threads of a CTA
+    read at once are ranked by counting, which CTAs that share an SM feel: beam 12, 8 x 1001 63 / 97, 4 x 1001 alike.
+    """
+    rows = B * beam
+    if beam > 16 or rows * V > 8000000:
+        return False
+    if beam <= 4 or (rows <= 64 and (beam <= 12 or V >= 10000)):
+        return True
+    return beam <= 12 and V * item >= 4000 and rows * beam ** 2 * max(V, 2048) <= 200000000
+
+
+@functools.lru_cache(maxsize=1024)
+def _beam_one_kernel_on(device: int, B: int, beam: int, V: int, item: int) -> bool:
+    return _beam_one_kernel(B, beam, V, item) and _beam_cluster_fits(device, beam)
+
+
+_BEAM_ARGS = [_vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp]
+
+
 def beam_topk(logits: torch.Tensor, prev_scores: torch.Tensor, *, finished: Optional[torch.Tensor] = None, eos: int = 0, k: int,
               normalized: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """
@@ -135,16 +161,16 @@ def beam_topk(logits: torch.Tensor, prev_scores: torch.Tensor, *, finished: Opti
         out_s = torch.empty(B, k, dtype=torch.float32, device=dev)
         out_b = torch.empty(B, k, dtype=torch.int32, device=dev)
         out_l = torch.empty(B, k, dtype=torch.int32, device=dev)
-        kt = 8 if k <= 8 else (16 if k <= 16 else 32)
-        # (score, index) per candidate of the per-row stage; without it the stages are one kernel: up to 16 hypotheses, and below the sizes where
-        # the device takes longer than the launches
-        one = beam <= 16 and B * beam * V <= 8000000 and _beam_cluster_fits(torch._C._cuda_getDevice(), beam)
-        scratch = None if one else torch.empty(B * beam * kt * 2, dtype=torch.int32, device=dev)
-        fn = _lib.bind("rb200_beam_topk", [_vp, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp])
+        # (score, index) per candidate of the per-row stage; without it the stages are one kernel
+        scratch = None
+        if not _beam_one_kernel_on(dev.index, B, beam, V, lg.element_size()):
+            kt = 8 if k <= 8 else (16 if k <= 16 else 32)
+            scratch = torch.empty(B * beam * kt * 2, dtype=torch.int32, device=dev)
+        fn = _lib.bind("rb200_beam_topk", _BEAM_ARGS)
         _lib.check(fn(lg.data_ptr(), 1 if lg.dtype == torch.bfloat16 else 0, 1 if normalized else 0, ps.data_ptr(),
                       fin.data_ptr() if fin is not None else None, B, beam, V, int(eos), int(k), out_s.data_ptr(), out_b.data_ptr(), out_l.data_ptr(),
-                      None if one else scratch.data_ptr(), _lib.stream_ptr()), "beam_topk")
-        _lib.count_launch(1 if one else 2)
+                      None if scratch is None else scratch.data_ptr(), _lib.stream_ptr()), "beam_topk")
+        _lib.count_launch(1 if scratch is None else 2)
         return out_s, out_b, out_l
     return beam_topk_reference(logits, prev_scores, finished, eos, k, normalized)
 
