@@ -50,13 +50,15 @@ struct Chunk {
   }
 };
 
-// kBatch: chunks that a thread has in flight, kCtas: CTAs of an SM that the registers are limited for. us of a pass over bf16 rows, four chunks (40 to 56
-// registers) / four with eight CTAs / two with eight, with the sum of the row: 6001 x 32000 76.9 / 68.3 / 69.5, 6001 x 10001 41.2 / 33.6 / 31.4, 6000 x 1000
-// 17.0 / 12.1 / 10.8; without 65.0 / 62.9 / 66.4, 33.5 / 30.7 / 29.5, 12.4 / 10.9 / 10.1. As few rows as are resident at once do not gain from room for more:
-// 800 x 32000 12.7 / 13.1 / 13.0. fp32 rows have half the conversions and twice the bytes: 112.5 / 119.2 / 121.4. (Passes one after the other, a third of the
-// largest matrix still in the L2; from memory alone 6001 x 32000 takes 73.2 / 71.8.)
-template <bool kBf16, bool kArg, bool kTot, int kBatch, int kCtas>
-__global__ void __launch_bounds__(256, kCtas)
+// kBatch: chunks of a row that a thread has in flight. Two where four would leave half of the last round of loads empty (up to 4096 classes, and from
+// 9000 to 12288), and up to 16383 with the position of the maximum, whose search goes through all chunks; else four. us, bf16, out of memory, four / two:
+// with the sum of the row 6000 x 1000 12.0 / 11.1, x 4000 18.4 / 17.0, x 6000 21.4 / 22.3, x 8000 24.6 / 25.3, x 10001 33.2 / 31.7, x 14000 37.5 / 38.4,
+// x 32000 68.9 / 72.7; without 11.5 / 10.6, 16.9 / 15.2, 19.2 / 20.8, 22.2 / 23.4, 30.8 / 29.6, 34.2 / 35.7, 64.5 / 68.5; with the position 13.9 / 11.6,
+// 22.6 / 17.9, 25.1 / 25.2, 28.3 / 27.8, 40.9 / 36.1, 44.6 / 44.2, 82.9 / 83.7. Both have eight CTAs on an SM (32 registers).
+// kWide: as many registers as the loads of a batch like (up to 42, six CTAs), for fp32 rows of several batches; 32 registers / that: 6000 x 500 11.7 / 13.9,
+// 6000 x 5000 27.3 / 27.9 (without the sum 27.1 / 25.1), 1500 x 16000 21.4 / 19.0, 6000 x 32000 119.4 / 114.1.
+template <bool kBf16, bool kArg, bool kTot, int kBatch, bool kWide>
+__global__ void __launch_bounds__(256, kWide ? 1 : 0)
 ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, float* __restrict__ loss, float* __restrict__ lse_out,
               int v, float smoothing, int* __restrict__ argmax_out) {
   constexpr int is_bf16 = kBf16 ? 1 : 0;
@@ -166,13 +168,12 @@ ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, floa
   }
 }
 
-template <bool kBf16>
+template <bool kBf16, bool kLastFirst>
 __global__ void __launch_bounds__(256)
 ce_bwd_kernel(const void* __restrict__ logits, const int* __restrict__ tgt, const float* __restrict__ lse_in,
               const float* __restrict__ dloss, void* __restrict__ dlogits, int v, float smoothing, int mode) {
   constexpr int is_bf16 = kBf16 ? 1 : 0;
-  // the last rows first: what the forward pass read last is what the L2 still holds (6001 x 32000 bf16, both passes: 205.8 -> 200.1 us)
-  const int64_t row = gridDim.x - 1 - blockIdx.x;
+  const int64_t row = kLastFirst ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const int64_t base = row * (int64_t)v;
   const float lse = lse_in[row];
   const int y = tgt[row];
@@ -212,18 +213,18 @@ RB_EXPORT int rb200_softmax_ce_fwd(const void* logits, const int* tgt, float* lo
   if (rows <= 0) return RB_OK;
   if (v < 2) return RB_ERR_ARG;
   const bool arg = argmax_out != nullptr, tot = smoothing > 0.f && mode == 0;
-  auto pick = [&](auto bf16, auto batch, auto ctas) {
-    constexpr bool kB = decltype(bf16)::value;
-    constexpr int kN = decltype(batch)::value, kC = decltype(ctas)::value;
-    return arg ? (tot ? ce_fwd_kernel<kB, true, true, kN, kC> : ce_fwd_kernel<kB, true, false, kN, kC>)
-               : (tot ? ce_fwd_kernel<kB, false, true, kN, kC> : ce_fwd_kernel<kB, false, false, kN, kC>);
+  auto pick = [&](auto bf16, auto batch, auto wide) {
+    constexpr bool kB = decltype(bf16)::value, kW = decltype(wide)::value;
+    constexpr int kN = decltype(batch)::value;
+    return arg ? (tot ? ce_fwd_kernel<kB, true, true, kN, kW> : ce_fwd_kernel<kB, true, false, kN, kW>)
+               : (tot ? ce_fwd_kernel<kB, false, true, kN, kW> : ce_fwd_kernel<kB, false, false, kN, kW>);
   };
-  using One = std::integral_constant<int, 1>;
   using Two = std::integral_constant<int, 2>;
   using Four = std::integral_constant<int, 4>;
-  using Eight = std::integral_constant<int, 8>;
-  auto kernel = !is_bf16 ? pick(std::false_type(), Four(), One()) : v < 16384 ? pick(std::true_type(), Two(), Eight())
-                : rows > 8 * 148 ? pick(std::true_type(), Four(), Eight()) : pick(std::true_type(), Four(), One());
+  const std::true_type yes;
+  const std::false_type no;
+  const bool two = v <= 4352 || (v >= 9000 && v <= 12288) || (arg && v < 16384);
+  auto kernel = is_bf16 ? (two ? pick(yes, Two(), no) : pick(yes, Four(), no)) : v < 4096 ? pick(no, Four(), no) : pick(no, Four(), yes);
   kernel<<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, loss, lse, v, smoothing, argmax_out);
   return rb_check_launch("softmax_ce_fwd");
 }
@@ -231,7 +232,12 @@ RB_EXPORT int rb200_softmax_ce_fwd(const void* logits, const int* tgt, float* lo
 RB_EXPORT int rb200_softmax_ce_bwd(const void* logits, const int* tgt, const float* lse, const float* dloss, void* dlogits,
                                    long long rows, int v, float smoothing, int is_bf16, int mode, cudaStream_t stream) {
   if (rows <= 0) return RB_OK;
-  if (is_bf16) ce_bwd_kernel<true><<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, lse, dloss, dlogits, v, smoothing, mode);
-  else ce_bwd_kernel<false><<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, lse, dloss, dlogits, v, smoothing, mode);
+  // The last rows first where the logits and their gradient do not fit the L2 together (126 MB): what the forward pass read last is what it still holds.
+  // Where they do, or all rows are resident at once, the order they are read in is the better one. us of both passes, bf16, first / last rows first, the
+  // logits out of memory: 6000 x 32000 198.3 / 193.3, 1500 x 32000 60.6 / 57.1, 3000 x 16384 55.7 / 54.5; 1500 x 20000 (60 MB) 37.4 / 37.4, 1500 x 16384 29.2 / 29.9,
+  // 800 x 8000 11.3 / 11.7, 1100 x 50000 65.8 / 67.3
+  const bool last_first = rows > 8 * 148 && rows * v * (is_bf16 ? 2 : 4) >= (64LL << 20);
+  auto kernel = is_bf16 ? (last_first ? ce_bwd_kernel<true, true> : ce_bwd_kernel<true, false>) : last_first ? ce_bwd_kernel<false, true> : ce_bwd_kernel<false, false>;
+  kernel<<<(unsigned)rows, 256, 0, stream>>>(logits, tgt, lse, dloss, dlogits, v, smoothing, mode);
   return rb_check_launch("softmax_ce_bwd");
 }

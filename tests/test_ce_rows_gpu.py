@@ -8,7 +8,8 @@ gpu = pytest.mark.gpu
 
 @gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,v", [(3, 2), (1300, 1000), (5, 16383), (1184, 16384), (1185, 16391), (40, 4097), (7, 32000)])
+@pytest.mark.parametrize("rows,v", [(3, 2), (1300, 1000), (5, 16383), (1184, 16384), (1185, 16391), (40, 4097), (7, 32000), (9, 4095), (3, 4096), (3, 4352), (3, 4353), (5, 8999), (5, 9000),
+                                    (3, 12288), (3, 12289)])
 @pytest.mark.parametrize("smoothing,arg", [(0.1, False), (0.0, True)])
 def test_softmax_ce_forward(dtype, rows, v, smoothing, arg):
     import ctypes
@@ -36,3 +37,22 @@ def test_softmax_ce_forward(dtype, rows, v, smoothing, arg):
     assert ((loss[ok].double() - ref[ok]).abs() <= 2.0**-15 + 2.0**-20 * d[ok].abs().sum(1) / v).all()
     if arg:
         assert torch.isfinite(lse).all() and torch.equal(am.long(), x.float().argmax(1))
+
+
+@gpu
+@pytest.mark.parametrize("dtype,rows,v", [(torch.bfloat16, 1185, 28400), (torch.bfloat16, 1184, 28400), (torch.bfloat16, 1300, 1000), (torch.float32, 1185, 14200)])
+def test_softmax_ce_gradient_by_order_of_rows(dtype, rows, v):
+    """more rows than are resident at once and 64 MB of logits: last rows first; each row's gradient is that of its own target and factor"""
+    from returnn_b200.ops.softmax_ce import softmax_cross_entropy
+
+    g = torch.Generator(device="cuda").manual_seed(rows + v)
+    x = (torch.randn(rows, v, generator=g, device="cuda") * 3).to(dtype).requires_grad_(True)
+    t = torch.randint(0, v, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    f = torch.randn(rows, generator=g, device="cuda")
+    (dx,) = torch.autograd.grad(softmax_cross_entropy(x, t), [x], f)
+    at = [0, 1, rows // 2, rows - 2, rows - 1]
+    want = torch.softmax(x[at].detach().double(), 1)
+    want[torch.arange(len(at)), t[at].long()] -= 1.0
+    want *= f[at].double()[:, None]
+    # a rounding to the type and an exponential of 2 ulp of an argument that is rounded to 2^-20
+    assert ((dx[at].double() - want).norm(dim=1) <= (2.0**-8 if dtype == torch.bfloat16 else 2.0**-17) * want.norm(dim=1)).all()
