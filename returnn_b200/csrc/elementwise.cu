@@ -140,18 +140,24 @@ RB_EXPORT int rb200_act_grad_colsum(const void* z, const void* dy, void* dz, flo
     rb_launch_pdl(colsum_slices_kernel, dim3(chunks), dim3(256), 0, stream, (const float*)work, db, 0, cols);
     return rb_check_launch("colsum_slices");
   }
-  // Wide where the matrices do not stay in the L2 (dz, z and dy of 12 M elements: 72 MB). us, narrow / wide, silu: 6656 x 2048 17.7 / 16.0, 6656 x 4096
-  // 39.1 / 33.6, 25000 x 2048 70.5 / 55.1; below the launch and the start of a CTA of 1024 threads cost more: 2000 x 4096 11.5 / 12.0,
-  // 6656 x 512 7.5 / 8.7, 50 x 512 3.1 / 4.6
-  const bool wide = cols >= 256 && (long long)rows * cols >= 12000000;
+  // Wide where the matrices do not stay in the L2 (dz, z and dy of 12 M elements: 72 MB). us out of memory, narrow / wide, silu: 6656 x 2048 28.4 / 20.9,
+  // 25000 x 1024 36.6 / 31.9, 25000 x 512 21.5 / 21.1, 50000 x 256 21.4 / 21.5, 1000 x 36000 50.1 / 40.6, 400 x 60000 37.2 / 36.3; below the launch and the start of
+  // a CTA of 1024 threads cost more: 2000 x 4096 11.5 / 12.0, 6656 x 512 7.5 / 8.7, 50 x 512 3.1 / 4.6. Without an activation one matrix is read, and the wide
+  // form needs rows of several CTAs, all of them resident at once: 6656 x 2048 10.7 / 8.8, 8000 x 1536 9.9 / 9.0, 1000 x 16000 11.1 / 9.5, 700 x 22000 10.9 / 10.6,
+  // 350 x 36000 8.8 / 8.1, but 50000 x 512 13.0 / 13.2, 100000 x 256 13.3 / 13.7, 400 x 40000 9.6 / 13.1
+  const bool wide = (long long)rows * cols >= 12000000 && (act ? cols >= 256 : cols >= 1536 && cols <= 148 * 256);
   const int cta_chunks = wide ? (cols + 255) / 256 : chunks;
   int splits = wide ? max(1, min(148 / cta_chunks, (rows + 31) / 32)) : colsum_splits(rows, cols);
   const int per = (rows + splits - 1) / splits;
   splits = (rows + per - 1) / per;
   using Kernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, __nv_bfloat16*, float*, float*, int, int, int);
+  // Without an activation the narrow form has four rows of a thread in flight where columns are few and each CTA has many rows, or where the CTAs are
+  // more than fit at once anyway; else two, with which five CTAs fit an SM: 6656 x 512 6.4 us with two, 5.7 with four; 20000 x 512 8.8 / 8.3, 25000 x 1024 13.7 / 12.4,
+  // 400 x 60000 14.9 / 12.7; 600 x 2048 4.0 / 4.8, 800 x 8000 6.3 / 7.3, 400 x 40000 9.6 / 11.4
+  const bool ahead = act == 0 && (cols <= 1024 || chunks > 5 * 148);
   static const Kernel narrow[] = {act_grad_colsum_kernel<0, 8, 2>, act_grad_colsum_kernel<1, 8, 2>, act_grad_colsum_kernel<2, 8, 2>, act_grad_colsum_kernel<3, 8, 2>};
   static const Kernel wides[] = {act_grad_colsum_kernel<0, 32, 4>, act_grad_colsum_kernel<1, 32, 4>, act_grad_colsum_kernel<2, 32, 4>, act_grad_colsum_kernel<3, 32, 2>};
-  const Kernel kernel = (wide ? wides : narrow)[act];
+  const Kernel kernel = wide ? wides[act] : ahead ? act_grad_colsum_kernel<0, 8, 4> : narrow[act];
   const dim3 grid(splits, cta_chunks), block(wide ? 1024 : 256);
   const __nv_bfloat16 *zp = (const __nv_bfloat16*)z, *dyp = (const __nv_bfloat16*)dy;
   if (!work) {

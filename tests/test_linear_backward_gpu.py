@@ -24,9 +24,10 @@ def test_weight_gradient_in_slices(m, k, n):
     assert float((dw - ref).abs().max()) <= 2 ** -24 * m ** 0.5 * 32 * float(ref.std())
 
 
-@pytest.mark.parametrize("rows,cols,act", [(6000, 2056, "silu"), (12100, 1000, None), (46900, 256, "relu"), (1201, 10000, "gelu"), (5800, 2056, "silu")])
+@pytest.mark.parametrize("rows,cols,act", [(6000, 2056, "silu"), (12100, 1000, None), (46900, 256, "relu"), (1201, 10000, "gelu"), (5800, 2056, "silu"), (12000, 1536, None), (317, 37888, None),
+                                           (317, 37896, None), (310, 40000, "relu"), (33, 47400, None), (4100, 1024, None), (3, 1032, None)])
 def test_activation_gradient_and_column_sums(rows, cols, act):
-    """the first four are above 12 M elements (wide form, ragged in rows and columns)"""
+    """wide form (ragged in rows and columns, at the ends of its range, more CTAs than are resident at once) and its neighbours in the narrow one"""
     from returnn_b200.ops import gemm as G
 
     g = torch.Generator(device="cuda").manual_seed(rows)
