@@ -551,7 +551,7 @@ inline int epilogue_kind(const Params& p) {
   const bool drop = g.drop_p > 0.f;
   if (g.out_fp32) return full || g.bias || g.act || g.c2 ? generic : kEpiF32;
   if (g.dact_z) return g.resid || g.bias || g.c2 ? generic : drop ? kEpiDactDrop : kEpiDact;
-  if (g.resid) return g.act || g.c2 ? generic : drop ? kEpiResidDrop : kEpiResid;
+  if (g.resid) return g.act || g.c2 || g.colsum ? generic : drop ? kEpiResidDrop : kEpiResid;
   if (g.c2) return drop ? kEpiTwoDrop : kEpiTwo;
   return drop ? generic : kEpiPlain;
 }
