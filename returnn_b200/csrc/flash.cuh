@@ -67,18 +67,6 @@ __device__ __forceinline__ float dot_row64(const uint8_t* f32, const uint8_t* bf
   return s;
 }
 
-// D[128, 64] (+)= A[128, 64] B: A K-major; B K-major [n, k] or, `b_mn`, stored [k, n]
-template <bool B_MN>
-__device__ __forceinline__ void mma64(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  const uint32_t sa = smem_u32(a), sb = smem_u32(b);
-#pragma unroll
-  for (int kk = 0; kk < 4; ++kk) {
-    umma_f16(d, make_desc(sa + kk * 32, 16, 1024), B_MN ? make_desc(sb + kk * 2048, 8192, 1024) : make_desc(sb + kk * 32, 16, 1024), idesc,
-             (accumulate || kk > 0) ? 1u : 0u);
-  }
-}
-
 // barriers, tensor memory and the abort flag of a CTA
 struct Cta {
   uint64_t* full;    // [2] loads of a stage
@@ -88,8 +76,7 @@ struct Cta {
   volatile int* abort_flag;
 };
 
-// DONE: arrivals that complete a phase of `done`
-template <uint32_t COLS, uint32_t DONE = 1>
+template <uint32_t COLS>
 __device__ __forceinline__ Cta cta_begin(uint8_t* tail) {
   Cta c;
   c.full = reinterpret_cast<uint64_t*>(tail);
@@ -98,7 +85,7 @@ __device__ __forceinline__ Cta cta_begin(uint8_t* tail) {
   uint32_t* slot = reinterpret_cast<uint32_t*>(c.full + 4);
   c.abort_flag = reinterpret_cast<volatile int*>(slot + 1);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 4; ++i) mbar_init(c.full + i, i == 2 ? DONE : 1);
+    for (int i = 0; i < 4; ++i) mbar_init(c.full + i, 1);
     *c.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -183,7 +170,7 @@ __device__ __forceinline__ bool pipe_wait(const Pipe& p, uint64_t* bar, int phas
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return ok;
 }
-// D[128, 64] (+)= A[128, 64] B as mma64, by one lane of a converged warp
+// D[128, 64] (+)= A[128, 64] B by one lane of a converged warp: A K-major; B K-major [n, k] or, `B_MN`, stored [k, n]
 template <bool B_MN>
 __device__ __forceinline__ void mma64_warp(uint32_t d, const uint8_t* a, const uint8_t* b, bool accumulate) {
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);

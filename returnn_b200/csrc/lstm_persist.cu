@@ -241,7 +241,7 @@ struct FwdArgs {
   bf16* gates;          // [T,B,4H]
   bf16* hprev_all;      // [T,B,H]
   float *h_final, *c_final;
-  bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state (wide form: unused, hprev_all is the exchanged matrix)
+  bf16* hbuf;           // [2,B,H] exchange buffer of the hidden state (wide form: null, hprev_all is the exchanged matrix)
   uint32_t* flags;      // one word per CTA (or the counter), zeroed before the launch
   int* abort_word;      // zeroed before the launch
   int* status;          // receives (5 << 24) | cta when a barrier wait ran out
@@ -917,11 +917,12 @@ cudaError_t launch_bwd_pair(BwdPair& pp, int H, cudaStream_t stream) {
 }  // namespace
 
 // whether the two-direction kernels take this problem: the single-direction conditions, and both grids co-resident
-RB_EXPORT int rb200_blstm_supported(int T, int B, int H) { return pair_shape(T, B, H) != kNoPair ? 1 : 0; }
+// 0: not supported; 1: the narrow form, which takes an exchange buffer; more: a wide form, which takes none
+RB_EXPORT int rb200_blstm_supported(int T, int B, int H) { return pair_shape(T, B, H); }
 
 // ptrs[d * 11 + i] for direction d (0: forward in time, 1: reversed):
 //   0 z_in [T,B,4H] bf16, 1 w_rec [4H,H] bf16, 2 h0, 3 c0 [B,H] fp32, 4 y [T,B,H] bf16, 5 c_all [T,B,H] fp32, 6 gates [T,B,4H] bf16,
-//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 exchange buffer (scratch, 2*B*H bf16)
+//   7 hprev_all [T,B,H] bf16, 8 h_final, 9 c_final [B,H] fp32, 10 exchange buffer (narrow form: scratch, 2*B*H bf16)
 RB_EXPORT int rb200_blstm_fwd(void* const* ptrs, const int* lens, int T, int B, int H, int* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return RB_OK;
   const int shape = pair_shape(T, B, H);

@@ -128,6 +128,7 @@ class _BlstmRecFn(torch.autograd.Function):
         dev = z_fw.device
         bf = torch.bfloat16
         per_dir = []
+        wide = _lib.bind("rb200_blstm_supported", [_i32, _i32, _i32])(T, B, H) > 1
         ptrs = (ctypes.c_void_p * 22)()
         keep = []
         for d, (z, w, h0, c0) in enumerate(((z_fw, w_fw, h0_fw, c0_fw), (z_bw, w_bw, h0_bw, c0_bw))):
@@ -139,10 +140,10 @@ class _BlstmRecFn(torch.autograd.Function):
             hprev = torch.empty(T, B, H, dtype=bf, device=dev)
             h_fin = torch.empty(B, H, dtype=torch.float32, device=dev)
             c_fin = torch.empty(B, H, dtype=torch.float32, device=dev)
-            hbuf = torch.empty(2, B, H, dtype=bf, device=dev)
+            hbuf = None if wide else torch.empty(2, B, H, dtype=bf, device=dev)
             h0f, c0f = h0.float().contiguous(), c0.float().contiguous()
             for i, t in enumerate((z16, w16, h0f, c0f, y, c_all, gates, hprev, h_fin, c_fin, hbuf)):
-                ptrs[d * 11 + i] = t.data_ptr()
+                ptrs[d * 11 + i] = t.data_ptr() if t is not None else None
             keep.append((z16, hbuf))
             per_dir.append((w16, gates, c_all, c0f, hprev, y, h_fin, c_fin))
         st = _gemm.status_tensor(dev)
