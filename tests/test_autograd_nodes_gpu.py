@@ -165,3 +165,87 @@ def test_traced_programs_record_the_python_function():
     traced = torch.jit.trace(lambda x: layer_norm(x, g, None, 1e-5), (_rand(9, 64, grad=False),), check_trace=False)
     x = _rand(9, 64, grad=False, seed=5)
     assert torch.equal(traced(x), layer_norm(x, g, None, 1e-5))
+
+
+def _chain(x, w, b, g, v):
+    """a layer norm, a linear layer, attention and a cross entropy"""
+    from returnn_b200.ops.gemm import linear_bf16
+    from returnn_b200.ops.layer_norm import layer_norm
+    from returnn_b200.ops.sdpa import sdpa_heads
+    from returnn_b200.ops.softmax_ce import softmax_cross_entropy
+
+    B, T, _ = x.shape
+    qkv = linear_bf16(layer_norm(x, g, None, 1e-5), w, b, "silu").view(B, T, 2, 192)
+    y = sdpa_heads(qkv[..., :64], qkv[..., 64:128], qkv[..., 128:], causal=True).reshape(B * T, 128)
+    return softmax_cross_entropy(linear_bf16(y, v, None, None), torch.arange(B * T, device="cuda") % 96, 0.1)
+
+
+def _chain_inputs(seed):
+    shapes = ((3, 50, 128), torch.bfloat16), ((128, 384), torch.float32), ((384,), torch.float32), ((128,), torch.float32), ((128, 96), torch.float32)
+    return [_rand(*s, dtype=dt, seed=seed + i) for i, (s, dt) in enumerate(shapes)]
+
+
+def _close(a, b):
+    for x, y in zip(a, b):  # (the gradient of gamma is a sum by atomics)
+        torch.testing.assert_close(x.float(), y.float(), rtol=1e-5, atol=1e-4)
+
+
+def test_two_threads_and_streams_of_their_own():
+    import threading
+
+    want = []
+    for t in range(2):
+        x = _chain_inputs(10 * t)
+        loss = _chain(*x)
+        want.append((loss.detach(), *torch.autograd.grad(loss.sum(), x)))
+    torch.cuda.synchronize()
+    got, errors = [[], []], []
+
+    def work(t):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(5):
+                    x = _chain_inputs(10 * t)
+                    loss = _chain(*x)
+                    got[t].append((loss.detach(), *torch.autograd.grad(loss.sum(), x)))
+                torch.cuda.current_stream().synchronize()
+        except BaseException as exc:  # noqa: B902
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for t in range(2):
+        for res in got[t]:
+            _close(res, want[t])
+
+
+def test_second_backward_through_a_retained_graph():
+    x = _chain_inputs(3)
+    loss = _chain(*x)
+    a = torch.autograd.grad(loss.sum(), x, retain_graph=True)
+    b = torch.autograd.grad(loss.sum() * 2, x, retain_graph=True)
+    c = torch.autograd.grad(loss.sum(), x)
+    _close(a, c)
+    for p, q in zip(a, b):  # a factor of two is exact in every rounding on the way
+        torch.testing.assert_close(2 * p.float(), q.float(), rtol=1e-5, atol=2e-4)
+
+
+@pytest.mark.parametrize("python", [False, True])
+def test_function_transforms_are_refused(monkeypatch, python):
+    """torch.func and forward mode: an error from the nodes as from the Python functions, not a result that leaves the operator out"""
+    from returnn_b200.ops import nodes
+    from returnn_b200.ops.layer_norm import layer_norm
+
+    if python:
+        monkeypatch.setattr(nodes, "active", lambda: None)
+    x, g = _rand(4, 64, grad=False), _rand(64, grad=False, seed=1)
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: layer_norm(t, g, None, 1e-5).float().sum())(x)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda t: layer_norm(t, g, None, 1e-5))(x[:, None])
+    with torch.autograd.forward_ad.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        layer_norm(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)), g, None, 1e-5)

@@ -44,9 +44,9 @@ def test_activation_gradient_and_column_sums(rows, cols, act):
 @pytest.mark.parametrize("m,n,k", [(129, 136, 64), (257, 264, 72), (300, 520, 512), (385, 1000, 200)])
 @pytest.mark.parametrize("form", ["plain", "bias", "two", "resid", "dact", "f32", "drop_two", "drop_resid", "drop_dact", "odd"])
 def test_pair_epilogues(m, n, k, form):
-    """every form of the epilogue at ragged sizes; with dropout against the same product without it and the stand-alone dropout kernel"""
+    """every form of the epilogue at ragged sizes; with dropout the mask is that of the stand-alone dropout kernel at the same counters"""
     from returnn_b200.ops import gemm as G
-    from returnn_b200.ops.elementwise import dropout  # noqa: F401  (the generator is the same)
+    from returnn_b200.ops.elementwise import dropout_with_state
 
     g = torch.Generator(device="cuda").manual_seed(m + n)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
@@ -58,6 +58,11 @@ def test_pair_epilogues(m, n, k, form):
     acc = a.double() @ b.double().t()
     second = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
     drop = dict(dropout_p=0.25, dropout_seed=torch.tensor([5], device="cuda"), dropout_offset=torch.tensor([9], device="cuda")) if "drop" in form else {}
+    mask = torch.ones(m, n, dtype=torch.double, device="cuda")
+    if drop:
+        ones = torch.ones(m, n, dtype=torch.bfloat16, device="cuda")
+        mask = (dropout_with_state(ones, 0.25, drop["dropout_seed"], drop["dropout_offset"] + 1000) > 0).double()
+        drop["dropout_site"] = 1000
     s = torch.sigmoid(z.double())
     if form in ("plain", "f32", "odd"):
         ref = acc
@@ -69,30 +74,23 @@ def test_pair_epilogues(m, n, k, form):
         ref = acc + bias
         G.gemm(a, b, bias=bias, act="silu", want_act_output=True, out_act=second, **drop, **kw)
     elif "resid" in form:
-        ref = r.double() + 0.5 * (acc + bias)
+        ref = r.double() + 0.5 * (acc + bias) * mask / (0.75 if drop else 1.0)
         G.gemm(a, b, bias=bias, resid=r, res_scale=0.5, **drop, **kw)
     else:
-        ref = acc * (s * (1 + z.double() * (1 - s)))
+        ref = acc * (s * (1 + z.double() * (1 - s))) * mask / (0.75 if drop else 1.0)
         G.gemm(a, b, dact_z=z, act="silu", **drop, **kw)
     G.check_status()
     assert float((out[m] - 7.0).abs().max()) == 0.0
     y = out[:m].double()
     # tanh.approx of the SiLU forms is within 2^-11 of its result, the rest is one rounding to bf16 (2^-9) of sums of 32 bits
     tol = 2 ** -20 if form == "f32" else 2 ** -8
-    if form in ("drop_resid", "drop_dact"):
-        base = r.double() if form == "drop_resid" else torch.zeros_like(ref)
-        kept = (base + (ref - base) / 0.75 - y).abs() <= 2 ** -7 * (base + (ref - base) / 0.75).abs() + 2 ** -6
-        dropped = (y - base).abs() <= 2 ** -8 * base.abs()
-        assert bool((kept | dropped).all()) and abs(float((~kept).float().mean()) - 0.25) < 0.05
-    else:
-        assert float((y - ref).norm()) <= tol * float(ref.norm())
+    assert float((y - ref).norm()) <= tol * float(ref.norm())
+    if form == "drop_dact":
+        assert bool((y[mask == 0] == 0).all())
     if "two" in form:
-        act = torch.nn.functional.silu(ref)
-        if drop:
-            keep = second != 0  # (the SiLU of values below -12 or so is 0 as well: only positive ones tell what was kept)
-            assert abs(float(keep[ref > 0].float().mean()) - 0.75) < 0.05
-            act = act / 0.75 * keep
+        act = torch.nn.functional.silu(ref) * mask / (0.75 if drop else 1.0)
         assert float((second.double() - act).norm()) <= 2 ** -8 * float(act.norm())
+        assert bool((second[mask == 0] == 0).all())
 
 
 @pytest.mark.parametrize("rows", [3, 20])

@@ -47,20 +47,38 @@ def test_short_sequences(Tq, Tk, causal, lens):
         assert float((a.double() - b).norm()) <= 2e-2 * float(b.norm()) + 1e-4
 
 
-@pytest.mark.parametrize("T", [31, 128])
-def test_dropout_decisions_are_those_of_the_forward_pass(T):
-    """linear in V: with dY = V's gradient direction the pairs (dropped P, V) of both passes agree"""
+@pytest.mark.parametrize("Tq,Tk", [(31, 31), (128, 128), (17, 128), (128, 65)])
+def test_dropout_decisions_are_those_of_the_forward_pass(Tq, Tk):
+    """
+    The decisions, read out of the forward pass (with the identity on a block of keys as values its output is the kept probabilities), and all
+    gradients against the definition with them in 64 bits.
+    """
+    from returnn_b200.ops.elementwise import _seed_tensor
     from returnn_b200.ops.sdpa import sdpa_heads
 
-    g = torch.Generator(device="cuda").manual_seed(T)
-    q, k, v, dy = (torch.randn(2, T, 2, 64, generator=g, device="cuda").bfloat16().requires_grad_(True) for _ in range(4))
-    y = sdpa_heads(q, k, v, dropout_p=0.3)
-    dq, dk, dv = torch.autograd.grad(y, [q, k, v], dy)
-    # <dV, V> = <dY, Y> (Y is linear in V), and sum over keys of dS is 0: <dQ, Q> = <dK, K>
-    for a, b, c, d in ((dv, v, dy, y), (dq, q, dk, k)):
-        x, z = float((a.double() * b.double()).sum()), float((c.double() * d.double()).sum())
-        size = float((a.double() * b.double()).norm()) + float((c.double() * d.double()).norm())
-        assert abs(x - z) <= 4e-2 * size, (x, z, size)
+    g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
+    B, H, p = 2, 2, 0.3
+    q, k, v, dy = ((torch.randn(B, t, H, 64, generator=g, device="cuda") * f).bfloat16().requires_grad_(True)
+                   for t, f in ((Tq, 0.7), (Tk, 0.7), (Tk, 1.0), (Tq, 1.0)))
+    seed = _seed_tensor(q.device)
+    state = seed.clone()
+    mask = torch.zeros(B, H, Tq, Tk, dtype=torch.double, device="cuda")
+    for j in range(0, Tk, 64):
+        n = min(64, Tk - j)
+        block = torch.zeros(B, Tk, H, 64, dtype=torch.bfloat16, device="cuda")
+        block[:, j: j + n, :, :n] = torch.eye(n, device="cuda", dtype=torch.bfloat16)[:, None]
+        seed.copy_(state)
+        mask[..., j: j + n] = (sdpa_heads(q.detach(), k.detach(), block, dropout_p=p)[..., :n] > 0).transpose(1, 2).double()
+    assert abs(float(mask.mean()) - (1 - p)) < 4 * (p * (1 - p) / mask.numel()) ** 0.5
+    seed.copy_(state)
+    y = sdpa_heads(q, k, v, dropout_p=p)
+    got = torch.autograd.grad(y, [q, k, v], dy.detach())
+    r = [t.detach().double().requires_grad_(True) for t in (q, k, v)]
+    w = torch.softmax(torch.einsum("bihd,bjhd->bhij", r[0], r[1]) * 0.125, -1) * mask / (1 - p)
+    want = torch.einsum("bhij,bjhd->bihd", w, r[2])
+    for a, b in zip((y, *got), (want, *torch.autograd.grad(want, r, dy.detach().double()))):
+        # probabilities, dS and results rounded to bf16, 2^-9 each; a decision that differs is an error of sqrt(1 / (1 - p)) of its element
+        assert float((a.double() - b).detach().norm()) <= 1e-2 * float(b.detach().norm())
 
 
 def test_common_offset_of_the_values():
