@@ -26,7 +26,10 @@ static inline int rb_check_launch(const char* what) {
 // one drain, then the next is launched). A kernel launched through rb_launch_pdl may be scheduled while its predecessor
 // still runs: it does the part of its prologue that touches no global memory, then calls rb_pdl_wait(), which returns once
 // the predecessor grid has completed and its writes are visible. Every kernel launched this way MUST call rb_pdl_wait()
-// before its first global-memory access; rb_pdl_launch() (right after it) lets the successor start being scheduled in turn.
+// before its first global-memory access; rb_pdl_launch() lets the successor start being scheduled in turn. Most kernels call it right after the wait.
+// A kernel may call it before, with the waits in the roles of its warps, if its CTA has all the tensor memory it will ever take by then (a successor's
+// CTA must not take what it needs to go on) and every role that touches global memory waits first, also one that finds no work: a grid is complete
+// only when all before it are.
 // Launched the ordinary way, both calls do nothing. RETURNN_B200_PDL=0 turns the attribute off.
 __device__ __forceinline__ void rb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void rb_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -478,16 +478,6 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ C
   end<512>(s, tmem);
 }
 
-int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 // frames of F rows of C channels; boxes of `rows` rows of a frame. run > 1: of as many frames, which are `stride` frames apart (stride > 1: a
 // coordinate more, frames are [frames / stride][stride])
 int frames_map(CUtensorMap* map, const void* base, int c, int f, long long frames, int rows, int run = 1, int stride = 1, bool split = false) {

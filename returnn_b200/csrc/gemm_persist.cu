@@ -2,7 +2,8 @@
 //
 //   D[M,N] = epilogue(alpha * op(A)·op(B)),   fp32 accumulation in tensor memory
 //
-// One CTA per SM walks a list of work units (128 x BN output tile, BN = 256 or 128, optionally one slice of K):
+// One CTA per SM (two for batches of small problems, see Layout) walks a list of work units (128 x BN output tile, BN = 256, 128 or 64, optionally one
+// slice of K):
 //   warp 0   TMA producer: cp.async.bulk.tensor (128-byte swizzle, no cluster multicast) into a shared-memory ring that keeps
 //            running across units, so the loads of the next tile are in flight while the current one is still multiplied
 //   warp 1   MMA issuer: one lane issues tcgen05.mma (cta_group::1, kind::f16, 128 x BN x 16); tcgen05.commit frees the ring
@@ -10,9 +11,9 @@
 //            issues, so that addresses, descriptors and coordinates stay in uniform registers: the batched products of attention, with one to
 //            eight K blocks a tile, are bound by this walk (dV of 36 x 333 frames, 8 heads: 20.1 -> 16.8 us, position gradient 29.4 -> 24.7,
 //            20 x 500 frames 21.6 -> 17.8 and 29.5 -> 24.9)
-//   warps 2-5 epilogue: tcgen05.ld (32x32b) -> registers -> per-warp shared staging (swizzled fp32) -> every lane then owns
-//            8 consecutive columns of one row, so that bias, activation, activation gradient, dropout (counter-based),
-//            residual add and the store are all 16-byte coalesced accesses
+//   the rest epilogue, 16 warps (8 where two CTAs share an SM), a warp for 32 rows and a quarter (half) of the columns: tcgen05.ld (32x32b) -> registers
+//            -> per-warp shared staging (swizzled fp32) -> every lane then owns 8 consecutive columns of one row, so that bias, activation, activation
+//            gradient, dropout (counter-based), residual add and the store are all 16-byte coalesced accesses
 // The accumulator is double-buffered in tensor memory (2 x BN columns): the epilogue of unit i overlaps the MMAs of unit i+1.
 //
 // Split-K: with accumulate == 2 the launcher may cut K into slices; every slice adds its partial tile to the fp32 output
@@ -193,7 +194,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       ++t_local;
     }
   } else {
-    // ---------------- epilogue: warps 2..5, TMEM lane quarter = warp % 4 ----------------
+    // ---------------- epilogue: TMEM lane quarter = warp % 4 ----------------
     const int q = warp & 3;
     float* stg = staging + (warp - 2) * (L::kStaging / 4);
     uint32_t t_local = 0;
@@ -234,16 +235,6 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
-}
-
-int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
 }
 
 bool epilogue_full(const RbGemm& g) { return g.dact_z != nullptr || g.drop_p > 0.f || g.resid != nullptr; }

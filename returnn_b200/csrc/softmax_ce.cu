@@ -50,8 +50,8 @@ struct Chunk {
   }
 };
 
-// kBatch: chunks of a row that a thread has in flight. Two where four would leave half of the last round of loads empty (up to 4096 classes, and from
-// 9000 to 12288), and up to 16383 with the position of the maximum, whose search goes through all chunks; else four. us, bf16, out of memory, four / two:
+// kBatch: chunks of a row that a thread has in flight. Two where four would leave half of the last round of loads empty (up to little more than 4096
+// classes, and from 9000 to 12288), and up to 16383 with the position of the maximum, whose search goes through all chunks; else four. us, bf16, out of memory, four / two:
 // with the sum of the row 6000 x 1000 12.0 / 11.1, x 4000 18.4 / 17.0, x 6000 21.4 / 22.3, x 8000 24.6 / 25.3, x 10001 33.2 / 31.7, x 14000 37.5 / 38.4,
 // x 32000 68.9 / 72.7; without 11.5 / 10.6, 16.9 / 15.2, 19.2 / 20.8, 22.2 / 23.4, 30.8 / 29.6, 34.2 / 35.7, 64.5 / 68.5; with the position 13.9 / 11.6,
 // 22.6 / 17.9, 25.1 / 25.2, 28.3 / 27.8, 40.9 / 36.1, 44.6 / 44.2, 82.9 / 83.7. Both have eight CTAs on an SM (32 registers).
