@@ -141,6 +141,20 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
+      uint32_t bits[2] = {0u, 0u};
+      if constexpr (DROP) {  // while the scores are multiplied (after the exponentials: 36 x 333 frames, 8 heads 110 us for 101, 300 x 40 186 for 162)
+        const uint64_t base = off + ((uint64_t)z * p.lp + row) * p.lp + it * 128 + wg * 64;
+#pragma unroll
+        for (int j = 0; j < 64; j += 4) {
+          const uint64_t ctr = base + j;
+          const uint4 x = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x52u, 0u));
+          const uint32_t r4[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (r4[e] >= thresh) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
+        }
+        if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
+      }
       ok = pipe_wait(w, w.scores, it, p.status, 22);
       if (!ok) break;
       float s[96];
@@ -180,21 +194,8 @@ rel_fwd_kernel(const __grid_constant__ CUtensorMap tm_qu, const __grid_constant_
       }
       l += sum;
       if constexpr (DROP) {
-        const uint64_t base = off + ((uint64_t)z * p.lp + row) * p.lp + it * 128 + wg * 64;
-        uint32_t bits[2] = {0u, 0u};
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) {
-          const uint64_t ctr = base + j;
-          const uint4 x = philox4x32(make_uint2((uint32_t)sd, (uint32_t)(sd >> 32)), make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x52u, 0u));
-          const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const bool k = w[e] >= thresh;
-            s[j + e] = k ? s[j + e] * keep_scale : 0.f;
-            if (k) bits[(j + e) >> 5] |= 1u << ((j + e) & 31);
-          }
-        }
-        if (row < len) *reinterpret_cast<uint2*>(p.keep + ((long long)z * p.lp + row) * p.words + it * 4 + wg * 2) = make_uint2(bits[0], bits[1]);
+        for (int j = 0; j < 64; ++j) s[j] = bits[j >> 5] >> (j & 31) & 1u ? s[j] * keep_scale : 0.f;
       }
       if (it > 0) {
         ok = pipe_wait(w, w.out, it - 1, p.status, 24);  // P of the tile before has been read, its product is in the output
