@@ -93,6 +93,20 @@ def test_pair_epilogues(m, n, k, form):
         assert bool((second[mask == 0] == 0).all())
 
 
+@pytest.mark.parametrize("m,n", [(6336, 6320), (6272, 6368)])
+def test_adding_onto_a_matrix_beyond_the_cache(m, n):
+    """40 M elements on: another epilogue"""
+    from returnn_b200.ops import gemm as G
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b = (torch.randn(r, 72, generator=g, device="cuda").bfloat16() for r in (m, n))
+    out = torch.full((m, n), 2.0, device="cuda")
+    G.gemm(a, b, m=m, n=n, k=72, a_mn_major=False, b_mn_major=False, out=out, atomic=True)
+    G.check_status()
+    # sums of 72 products and of the two terms in 32 bits: 2^-24 of values of up to 64 each
+    assert float((out - 2.0 - a.float() @ b.float().t()).abs().max()) <= 72 * 2 ** -24 * 64
+
+
 @pytest.mark.parametrize("rows", [3, 20])
 def test_blstm_passes_nan_on_without_waiting(rows):
     """NaN in one sequence (every NaN that a conversion can give) stays there, and no wait runs out: what marks unwritten values is another one"""
