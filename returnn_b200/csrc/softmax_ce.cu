@@ -50,7 +50,7 @@ struct Chunk {
   }
 };
 
-// kBatch: chunks of a row that a thread has in flight. Two where four would leave half of the last round of loads empty (up to little more than 4096
+// kBatch: chunks of a row that a thread has in flight. Two where four would leave half of the last batch of loads empty (up to little more than 4096
 // classes, and from 9000 to 12288), and up to 16383 with the position of the maximum, whose search goes through all chunks; else four. us, bf16, out of memory, four / two:
 // with the sum of the row 6000 x 1000 12.0 / 11.1, x 4000 18.4 / 17.0, x 6000 21.4 / 22.3, x 8000 24.6 / 25.3, x 10001 33.2 / 31.7, x 14000 37.5 / 38.4,
 // x 32000 68.9 / 72.7; without 11.5 / 10.6, 16.9 / 15.2, 19.2 / 20.8, 22.2 / 23.4, 30.8 / 29.6, 34.2 / 35.7, 64.5 / 68.5; with the position 13.9 / 11.6,
